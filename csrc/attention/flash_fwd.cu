@@ -1,17 +1,5 @@
-// K6 (forward): causal flash attention on the 5th-generation tensor cores, head_dim = 128, bf16.
-//
-// One CTA = one (batch, head, 128-query block).  Warp roles:
-//   warp 0     TMA producer  — Q once, then K and V tiles of 128 keys into 2-deep smem rings (3-D tensor maps
-//                              over the packed [tokens, heads, 128] activations, 128-byte swizzle)
-//   warp 1     MMA issuer    — S = Q K^T  (UMMA 128x128x16, both operands K-major, accumulator S[j%2] in TMEM)
-//                              O += P V   (UMMA 128x128x16, A = P from smem (K-major), B = V (MN-major), O in TMEM)
-//   warps 2-5  softmax       — thread = query row: tcgen05.ld S, scale / causal mask / running max, exp2,
-//                              P -> bf16 -> swizzled smem, lazy O rescale in TMEM, final normalisation + store
-// S is double buffered in TMEM so Q K^T of block j+1 runs on the tensor core while the softmax warps work on
-// block j.  The running max is only advanced when it grows by more than 8 (log2 units): between rescales the
-// reference stays put and P may reach 2^8, which fp32 accumulation and bf16 P hold exactly as well — this
-// removes almost all TMEM read-modify-write passes over O.
-// Outputs: O [B,S,H,128] bf16 and the row log-sum-exp (natural log, scale included) for the backward pass.
+// K6 (forward): causal flash attention on the 5th-generation tensor cores, bf16: head sizes 64 and 128, sequences of any
+// length.
 //
 // Reference: HF modules choose SDPA/eager attention behind `self.model(**batch)` (reference
 // llmctl/runtime/engine.py:284); the reference's tuner times a naive softmax(QK^T)V (reference
@@ -23,50 +11,59 @@
 namespace llmctl {
 using namespace ptx;
 
-constexpr int kAD = 128;                 // head dim
-constexpr int kABM = 128;                // queries per CTA
-constexpr int kABN = 128;                // keys per tile
-constexpr int kPanel = 128 * 128;        // bytes of one [128 rows x 64 bf16] swizzled panel
-constexpr int kTile = 2 * kPanel;        // 128 x 128 bf16
-constexpr int kAttnSmem = kTile /*Q*/ + 2 * kTile /*K*/ + 2 * kTile /*V*/ + kTile /*P*/ + 1024;
-constexpr int kAttnThreads = 192;
-constexpr float kRescaleThreshold = 8.f;
-
 // =====================================================================================================
-// Tile structure: one work item = one (batch, head, 256-query block) handled as two 128-query tiles A and B that share
-// every K/V tile (half the K/V smem traffic) and ping-pong on the tensor core: while the softmax warpgroup of
-// tile A works on S_A, the MMA warp runs P_B V / Q_B K^T and vice versa.
+// One work item = one (batch, head, 256-query block) handled as two 128-query tiles A and B that share every K/V tile (half
+// the K/V smem traffic) and ping-pong on the tensor core: while the softmax warpgroup of tile A works on S_A, the MMA warp runs
+// P_B V / Q_B K^T and vice versa.
 //   warps 0-3   softmax warpgroup of tile A      warps 4-7  softmax warpgroup of tile B
-//   warp 8      TMA producer (Q_A, Q_B once; K, V rings of 2 x 128 keys)
+//   warp 8      TMA producer (Q_A, Q_B once per item; rings of 128 keys)
 //   warp 9      MMA issuer                       warps 10-11 idle (they complete the third warpgroup so that
-//               setmaxnreg can move its registers to the softmax warpgroups: 216 per softmax thread, enough to
+//               setmaxnreg can move its registers to the softmax warpgroups: 200 per softmax thread, enough to
 //               hold a whole 128-column S row plus the packed P chunk without spilling)
 // TMEM (all 512 columns): S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512).  P never touches shared
 // memory: the softmax thread overwrites the first 64 columns of its own S row with bf16x2 probabilities
 // (tcgen05.st) and P V reads its A operand straight from TMEM.  The tensor pipe executes in issue order, so
 // Q K^T of block j+1 (which overwrites S/P) is simply issued after P V of block j; tcgen05.commit covers every
 // earlier MMA, so "S(j+1) ready" also means "P V(j) has retired" and the O rescale needs no extra barrier.
-// The epilogue stages O through the (now idle) Q tile and writes it with TMA.
-constexpr int kF2Threads = 384;
-// kPolyCount of every kPolyPeriod score pairs can take the FMA-pipe exponential (ptx.cuh ex2_poly2) instead of
-// MUFU.EX2: per 256x128 tile pair the SFU needs 32768 / 16 = 2048 clk, the same as the tensor core.  Measured on
-// B200 (B1 S4096 H32): 0 -> 170 us, 2 of 4 -> 180 us — the softmax warps are bound by dependent-issue latency,
-// not by SFU throughput, so the extra FMA instructions cost more than the SFU time they free.  Default off.
-#ifndef LLMCTL_FLASH_POLY_COUNT
-#define LLMCTL_FLASH_POLY_COUNT 0
-#endif
-constexpr int kPolyPeriod = 4;
-constexpr int kPolyCount = LLMCTL_FLASH_POLY_COUNT;
-constexpr int kF2Smem = 6 * kTile + 1024;
+// A tile's chain (S ready -> softmax -> P V, Q K^T -> S ready) is longer than the two tiles' tensor work (3600 against 2048
+// clocks per block when P was handed over whole), so P is handed over in two halves: the first 64 keys' P V runs while the
+// second half is still being exponentiated.
+// The running max is only advanced when it grows by more than 8 (log2 units): between rescales the reference stays put and
+// P may reach 2^8, which fp32 accumulation and bf16 P hold exactly as well — this removes almost all TMEM read-modify-write
+// passes over O.
+// =====================================================================================================
+namespace ffwd {
+constexpr int kRows = 128;               // queries per tile, keys per tile
+constexpr int kPanel = kRows * 128;      // bytes of one [128 rows x 64 bf16] swizzled panel
+constexpr int kThreads = 384;
+constexpr float kRescaleThreshold = 8.f;
+// Stages of the K and V rings: what 227 KB hold beside the two query tiles (160 KB at D = 64, 192 KB at 128).
+template <int DQK, int DV>
+struct Cfg {
+  static constexpr int kQTile = DQK / 64 * kPanel, kVTile = DV / 64 * kPanel;
+  static constexpr int kKStages = DQK == 64 ? 4 : 2;
+  static constexpr int kVStages = DQK == 64 ? 4 : 2;
+  static constexpr int kKAt = 2 * kQTile, kVAt = kKAt + kKStages * kQTile;
+  static constexpr int kSmem = kVAt + kVStages * kVTile + 1024;
+};
+__device__ unsigned int g_status = 0;    // != 0: a bounded wait of the kernel ran out
 
-// On the diagonal block the mask is resolved per 32-column chunk, which is warp-uniform (warp q owns rows
-// 32q .. 32q+31): chunks left of the diagonal chunk take the plain path, chunks right of it are all masked and
-// cost nothing (no compare, no exponential, P = 0), only chunk q compares its 32 columns against the lane.
-template <bool kDiag>
-__device__ __forceinline__ void softmax_block_v2(uint32_t tS, uint32_t tO, int row, bool first, float scale_log2,
-                                                 float& m_ref, float& l0, float& l1) {
-  const int dq = row >> 5;            // diagonal chunk of this warp
-  const int dl = row & 31;            // lane = row within the chunk
+// One sequence of the batch: its queries are rows [q_row, q_row + n) at positions start + i, its keys (position 0 first) begin
+// at row k_row.
+struct Seq {
+  int q_row, n, start, k_row;
+};
+}  // namespace ffwd
+
+// The mask is resolved per 32-column chunk, which is warp-uniform (warp q owns rows 32q .. 32q+31; row r sees the columns up to
+// off + r): chunks that all its rows see take the plain path, chunks that none sees cost nothing (no compare, no exponential,
+// P = 0), only the chunks in between compare their columns against the lane.
+template <bool kMask, int DV>
+__device__ __forceinline__ void softmax_block(uint32_t tS, uint32_t tO, int q, int lane, int off, bool first, float scale_log2,
+                                              float& m_ref, float& l0, float& l1, uint64_t* bar_p0, uint64_t* bar_p1) {
+  using namespace ffwd;
+  const int w0 = off + q * 32;        // last column that the warp's first row sees
+  const int mine = w0 + lane;         // ... and this row
   // The whole S row (128 fp32) is read from TMEM once and stays in registers for both passes: every
   // tcgen05.ld -> wait round trip removed here is latency the tensor pipe would otherwise sit idle for.
   uint32_t r[128];
@@ -76,28 +73,22 @@ __device__ __forceinline__ void softmax_block_v2(uint32_t tS, uint32_t tO, int r
   tmem_ld_x32(tS + 96, r + 96);
   tmem_ld_wait();
   // pass 1: raw row maximum (the scale is positive, so it commutes with max)
-  float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
+  float m0 = -INFINITY, m1 = -INFINITY;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    if (kDiag && c > dq) continue;                       // fully masked chunk
-    const bool edge = kDiag && c == dq;
+    if (kMask && c * 32 > w0 + 31) continue;             // fully masked chunk
+    if (kMask && c * 32 + 31 > w0) {
+#pragma unroll
+      for (int e = c * 32; e < c * 32 + 32; ++e)
+        if (e > mine) r[e] = 0xff800000u;                // -inf
+    }
 #pragma unroll
     for (int e = c * 32; e < c * 32 + 32; e += 4) {
-      float a = __uint_as_float(r[e]), b2 = __uint_as_float(r[e + 1]), c2 = __uint_as_float(r[e + 2]),
-            d2 = __uint_as_float(r[e + 3]);
-      if (edge) {
-        if ((e & 31) > dl) a = -INFINITY;
-        if ((e & 31) + 1 > dl) b2 = -INFINITY;
-        if ((e & 31) + 2 > dl) c2 = -INFINITY;
-        if ((e & 31) + 3 > dl) d2 = -INFINITY;
-      }
-      m0 = fmaxf(m0, a);
-      m1 = fmaxf(m1, b2);
-      m2 = fmaxf(m2, c2);
-      m3 = fmaxf(m3, d2);
+      m0 = max3(m0, __uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+      m1 = max3(m1, __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]));
     }
   }
-  const float bm = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) * scale_log2;
+  const float bm = fmaxf(m0, m1) * scale_log2;
   // lazy reference update: only move the reference when the block maximum outgrows it by more than 2^8
   const bool need = bm > m_ref + kRescaleThreshold;
   float alpha = 1.f;
@@ -107,43 +98,10 @@ __device__ __forceinline__ void softmax_block_v2(uint32_t tS, uint32_t tO, int r
     l0 *= alpha;
     l1 *= alpha;
   }
-  const bool rescale = !first && __any_sync(0xffffffffu, need);
-  // pass 2: p = 2^(s*scale - m_ref) -> bf16x2 -> back into the first 64 columns of this S row
-  const float neg_m = -m_ref;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    uint32_t pk[16];
-    if (kDiag && c > dq) {                               // fully masked chunk: P = 0, nothing to compute
-#pragma unroll
-      for (int e = 0; e < 16; ++e) pk[e] = 0u;
-      tmem_st_x16(tS + c * 16, pk);
-      continue;
-    }
-    const bool edge = kDiag && c == dq;
-#pragma unroll
-    for (int e = 0; e < 32; e += 2) {
-      float a0, a1;
-      fma2(a0, a1, __uint_as_float(r[c * 32 + e]), __uint_as_float(r[c * 32 + e + 1]), scale_log2, neg_m);
-      if (edge) {
-        if (e > dl) a0 = -INFINITY;
-        if (e + 1 > dl) a1 = -INFINITY;
-      }
-      float p0, p1;
-      if (((e >> 1) % kPolyPeriod) < kPolyCount) {
-        ex2_poly2(p0, p1, a0, a1);         // FMA-pipe exponential for this pair (see ptx.cuh)
-      } else {
-        p0 = ex2_approx(a0);
-        p1 = ex2_approx(a1);
-      }
-      add2(l0, l1, p0, p1);
-      pk[e >> 1] = pack_bf16x2(p0, p1);
-    }
-    tmem_st_x16(tS + c * 16, pk);
-  }
-  if (rescale) {
-    // rare (reference moved by more than 2^8): scale the running O row; P stores above are already in flight
+  if (!first && __any_sync(0xffffffffu, need)) {
+    // rare (reference moved by more than 2^8): scale the running O row
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < DV / 32; ++c) {
       uint32_t o[32];
       tmem_ld_x32(tO + c * 32, o);
       tmem_ld_wait();
@@ -158,7 +116,32 @@ __device__ __forceinline__ void softmax_block_v2(uint32_t tS, uint32_t tO, int r
       tmem_st_x16(tO + c * 32 + 16, o + 16);
     }
   }
-  tmem_st_wait();
+  // pass 2: p = 2^(s*scale - m_ref) -> bf16x2 -> back into the first 64 columns of this S row
+  const float neg_m = -m_ref;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t pk[16];
+    if (kMask && c * 32 > w0 + 31) {                     // fully masked chunk: P = 0, nothing to compute
+#pragma unroll
+      for (int e = 0; e < 16; ++e) pk[e] = 0u;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 32; e += 2) {
+        float a0, a1;
+        fma2(a0, a1, __uint_as_float(r[c * 32 + e]), __uint_as_float(r[c * 32 + e + 1]), scale_log2, neg_m);
+        const float p0 = ex2_approx(a0), p1 = ex2_approx(a1);
+        add2(l0, l1, p0, p1);
+        pk[e >> 1] = pack_bf16x2(p0, p1);
+      }
+    }
+    tmem_st_x16(tS + c * 16, pk);
+    if (c & 1) {                                         // half of P (and the rescaled O) is in place
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(c == 1 ? bar_p0 : bar_p1);
+    }
+  }
 }
 
 // =====================================================================================================
@@ -172,20 +155,23 @@ __device__ __forceinline__ void softmax_block_v2(uint32_t tS, uint32_t tO, int r
 // item's Q tiles as soon as the last Q K^T of the current one has retired, and the MMA warp starts the next
 // item's Q K^T while the softmax warpgroups are still normalising and storing O of the current one (O goes
 // from registers straight to global memory, so no staging buffer blocks the Q prefetch).
-__global__ void __launch_bounds__(kF2Threads, 1)
-flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                  const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ O, long long o_tok_stride,
-                  float* __restrict__ lse, int B, int S, int H, float scale_log2, int causal,
-                  long long* __restrict__ trace) {
+template <int DQK, int DV>
+__global__ void __launch_bounds__(ffwd::kThreads, 1)
+flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                 const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ O, long long o_tok_stride, int o_wide,
+                 float* __restrict__ lse, int B, int max_q, int H, float scale_log2, int causal, long long* __restrict__ trace) {
+  using namespace ffwd;
+  using C = Cfg<DQK, DV>;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t bar_q[2], bar_qfree[2], bar_kfull[2], bar_vfull[2], bar_kempty[2], bar_vempty[2];
-  __shared__ uint64_t bar_s[2], bar_p[2], bar_o[2], bar_ofree[2];
+  __shared__ uint64_t bar_q[2], bar_qfree[2], bar_kfull[C::kKStages], bar_vfull[C::kVStages], bar_kempty[C::kKStages], bar_vempty[C::kVStages];
+  __shared__ uint64_t bar_s[2], bar_p0[2], bar_p1[2], bar_o[2], bar_ofree[2];
   __shared__ uint32_t tmem_base_smem;
+  __shared__ int abort_flag;
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));      // layout: Q_A, Q_B, K[2], V[2]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nqb = (S + 2 * kABM - 1) / (2 * kABM);
+  uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));      // layout: Q_A, Q_B, K ring, V ring
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int nqb = (max_q + 2 * kRows - 1) / (2 * kRows);
   const int per_qb = H * B;
   const int n_items = nqb * per_qb;
 
@@ -193,15 +179,21 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bar_q[i], 1);
       mbar_init(&bar_qfree[i], 1);
-      mbar_init(&bar_kfull[i], 1);
-      mbar_init(&bar_vfull[i], 1);
-      mbar_init(&bar_kempty[i], 1);
-      mbar_init(&bar_vempty[i], 1);
       mbar_init(&bar_s[i], 1);
-      mbar_init(&bar_p[i], 4);
+      mbar_init(&bar_p0[i], 4);
+      mbar_init(&bar_p1[i], 4);
       mbar_init(&bar_o[i], 1);
       mbar_init(&bar_ofree[i], 4);
     }
+    for (int i = 0; i < C::kKStages; ++i) {
+      mbar_init(&bar_kfull[i], 1);
+      mbar_init(&bar_kempty[i], 1);
+    }
+    for (int i = 0; i < C::kVStages; ++i) {
+      mbar_init(&bar_vfull[i], 1);
+      mbar_init(&bar_vempty[i], 1);
+    }
+    abort_flag = 0;
     fence_mbar_init();
   }
   if (warp == 8 && lane == 0) {
@@ -214,10 +206,10 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
+  volatile int* abort = &abort_flag;
 
   // optional event log of CTA 0 (LLMCTL_FLASH_TRACE): per role 127 x (code, clock) pairs after a count word.
-  // roles: 0/1 softmax A/B (codes 1 = S ready, 2 = P written, 3 = O stored), 2 / 4 = MMA issuer of tile A / B (10+t = P seen,
-  // 20+t = issued, 30 = item start), 3 = TMA (40 = item start)
+  // roles: 0/1 softmax A/B (codes 1 = S ready, 2 = P written, 3 = O stored), 3 = TMA (40 = item start)
   const bool tracing = trace != nullptr && blockIdx.x == 0;
   const long long t_start = tracing ? clock64() : 0;
   int n_ev = 0;
@@ -229,133 +221,167 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       trace[role * 256] = n_ev;
     }
   };
-  // item -> (query block pair, head, batch); heavy (late) query blocks first so the tail is made of light items
-  auto decode = [&](int item, int& qb2, int& head, int& b) {
-    qb2 = nqb - 1 - item / per_qb;
+  // The CTA's items: the list is sorted by length, and every other round runs over the CTAs backwards, so that nobody gets the
+  // longest of every round (S = 2048, 40 heads x 2: 40 instead of 48 blocks on the busiest CTA, 39 on average).
+  auto next_item = [&](int r, int& item) {
+    item = r * gridDim.x + ((r & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+    return item < n_items;
+  };
+  // item -> (first query, head, batch, sequence); heavy (late) query blocks first so the tail is made of light items
+  auto decode = [&](int item, int& q0, int& head, int& b, Seq& sq) {
+    q0 = (nqb - 1 - item / per_qb) * 2 * kRows;
     const int rem = item % per_qb;
     head = rem % H;
     b = rem / H;
+    sq = Seq{0, max_q, 0, 0};
+    return q0 < sq.n;
+  };
+  // key blocks of tile t of an item; a tile past the end of its sequence has none
+  auto blocks = [&](const Seq& sq, int q0, int t) {
+    const int qt = q0 + t * kRows;
+    if (qt >= sq.n) return 0;
+    const int all = (sq.start + sq.n + kRows - 1) / kRows;
+    return causal ? min(all, (sq.start + qt + kRows - 1) / kRows + 1) : all;
   };
 
   if (warp >= 8) {
    // register budget: the CTA owns 384 x 168; what warps 8-11 give back ((168-104) x 128) is exactly what the two
-   // softmax warpgroups take ((200-168) x 256) — asking for more than was released blocks forever.  
+   // softmax warpgroups take ((200-168) x 256) — asking for more than was released blocks forever.
    setmaxnreg_dec<104>();
    if (warp == 8) {
     // ------------------------------------ TMA producer ------------------------------------
     if (lane == 0) {
-      uint32_t g = 0;                 // K/V blocks loaded so far (ring position and phase)
+      uint32_t g = 0;                 // K/V blocks so far (ring position and phase)
       uint32_t nA = 0, nB = 0;        // Q_A / Q_B loads so far
-      for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-        int qb2, head, b;
-        decode(item, qb2, head, b);
-        const int q0 = qb2 * 2 * kABM;
-        const bool validB = q0 + kABM < S;
-        const int nblk = causal ? (validB ? 2 * qb2 + 2 : 2 * qb2 + 1) : (S / kABN);
-        const int tok0 = b * S;
+      uint32_t nk = 0, nv = 0;        // K / V loads so far
+      bool ok = true;
+      for (int item, r = 0; ok && next_item(r, item); ++r) {
+        int q0, head, b;
+        Seq sq;
+        if (!decode(item, q0, head, b, sq)) continue;
+        const int nblk = max(blocks(sq, q0, 0), blocks(sq, q0, 1));
+        const bool validB = q0 + kRows < sq.n;
         ev(3, 40);
-        mbar_wait(&bar_qfree[0], (nA & 1u) ^ 1u);        // the previous item's last Q_A K^T has retired
-        mbar_expect_tx(&bar_q[0], kTile);
-        tma_load_3d(smem, &tmQ, &bar_q[0], 0, head, tok0 + q0);
-        tma_load_3d(smem + kPanel, &tmQ, &bar_q[0], 64, head, tok0 + q0);
+        auto load_q = [&](int t, uint32_t done) {
+          if (!mbar_wait_bounded(&bar_qfree[t], (done & 1u) ^ 1u, abort)) return false;      // the previous item's last Q K^T has retired
+          mbar_expect_tx(&bar_q[t], C::kQTile);
+#pragma unroll
+          for (int p = 0; p < DQK / 64; ++p)
+            tma_load_4d(smem + t * C::kQTile + p * kPanel, &tmQ, &bar_q[t], 64 * p, head, sq.q_row + q0 + t * kRows, b);
+          return true;
+        };
+        if (!(ok = load_q(0, nA))) break;
         ++nA;
         for (int j = 0; j < nblk; ++j, ++g) {
-          const int st = g & 1u;
-          const uint32_t ph = (g >> 1) & 1u;
-          uint8_t* sK = smem + 2 * kTile + st * kTile;
-          uint8_t* sV = smem + 4 * kTile + st * kTile;
-          mbar_wait(&bar_kempty[st], ph ^ 1u);
-          mbar_expect_tx(&bar_kfull[st], kTile);
-          tma_load_3d(sK, &tmK, &bar_kfull[st], 0, head, tok0 + j * kABN);
-          tma_load_3d(sK + kPanel, &tmK, &bar_kfull[st], 64, head, tok0 + j * kABN);
+          const uint32_t ks = g % C::kKStages, vs = g % C::kVStages;
+          const int row = sq.k_row + j * kRows;
+          uint8_t* sK = smem + C::kKAt + ks * C::kQTile;
+          uint8_t* sV = smem + C::kVAt + vs * C::kVTile;
+          if (!(ok = mbar_wait_bounded(&bar_kempty[ks], ((g / C::kKStages) & 1u) ^ 1u, abort))) break;
+          mbar_expect_tx(&bar_kfull[ks], C::kQTile);
+          ++nk;
+#pragma unroll
+          for (int p = 0; p < DQK / 64; ++p) tma_load_4d(sK + p * kPanel, &tmK, &bar_kfull[ks], 64 * p, head, row, b);
           if (j == 0 && validB) {
-            mbar_wait(&bar_qfree[1], (nB & 1u) ^ 1u);
-            mbar_expect_tx(&bar_q[1], kTile);
-            tma_load_3d(smem + kTile, &tmQ, &bar_q[1], 0, head, tok0 + q0 + kABM);
-            tma_load_3d(smem + kTile + kPanel, &tmQ, &bar_q[1], 64, head, tok0 + q0 + kABM);
+            if (!(ok = load_q(1, nB))) break;
             ++nB;
           }
-          mbar_wait(&bar_vempty[st], ph ^ 1u);
-          mbar_expect_tx(&bar_vfull[st], kTile);
-          tma_load_3d(sV, &tmV, &bar_vfull[st], 0, head, tok0 + j * kABN);
-          tma_load_3d(sV + kPanel, &tmV, &bar_vfull[st], 64, head, tok0 + j * kABN);
+          if (!(ok = mbar_wait_bounded(&bar_vempty[vs], ((g / C::kVStages) & 1u) ^ 1u, abort))) break;
+          mbar_expect_tx(&bar_vfull[vs], C::kVTile);
+          ++nv;
+#pragma unroll
+          for (int p = 0; p < DV / 64; ++p) tma_load_4d(sV + p * kPanel, &tmV, &bar_vfull[vs], 64 * p, head, row, b);
         }
+      }
+      // Copies still in flight when a wait ran out land before the CTA's shared memory is given back.
+      if (!ok) {
+        int none = 0;
+        if (nA > 0) mbar_wait_bounded(&bar_q[0], (nA - 1) & 1u, &none);
+        none = 0;
+        if (nB > 0) mbar_wait_bounded(&bar_q[1], (nB - 1) & 1u, &none);
+        none = 0;
+        for (uint32_t j = nk > C::kKStages ? nk - C::kKStages : 0; j < nk; ++j, none = 0)
+          mbar_wait_bounded(&bar_kfull[j % C::kKStages], (j / C::kKStages) & 1u, &none);
+        for (uint32_t j = nv > C::kVStages ? nv - C::kVStages : 0; j < nv; ++j, none = 0)
+          mbar_wait_bounded(&bar_vfull[j % C::kVStages], (j / C::kVStages) & 1u, &none);
       }
     }
    } else if (warp == 9) {
     // ------------------------------------ MMA issuer ------------------------------------
-    // One thread issues for both tiles in strict A, B, A, B order: the issue order is what keeps the two tiles in
+    // One warp issues for both tiles in strict A, B, A, B order: the issue order is what keeps the two tiles in
     // anti-phase (one in its softmax while the other owns the tensor pipe).  Measured alternatives (B1 S8192 H32):
     // two issuing warps, one per tile — the tiles drift into lock-step and the exponential unit and the tensor
     // core alternate instead of overlapping, 1010 -> 750 TFLOP/s; issuing the next item's first Q K^T early from
     // inside this loop — the extra live state spills into the issue sequences (or, with more registers here,
-    // starves the softmax warps), 1010 -> 720-830 TFLOP/s.  This thread's issue latency is on the critical path.
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = make_idesc_bf16(kABM, kABN, 0u, 0u);   // A, B K-major
-      constexpr uint32_t idesc_pv = make_idesc_bf16(kABM, kAD, 0u, 1u);    // A from TMEM, B MN-major (V)
-      uint32_t g0 = 0;                 // K/V blocks consumed by earlier items
-      uint32_t nQ[2] = {0, 0};         // items done per tile (Q / O barrier phases)
-      uint32_t nP[2] = {0, 0};         // P V products issued per tile (bar_p phase)
-      for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-        int qb2, head, b;
-        decode(item, qb2, head, b);
-        const int q0 = qb2 * 2 * kABM;
-        const bool validB = q0 + kABM < S;
-        const int nblk_t0 = causal ? (2 * qb2 + 1) : (S / kABN);
-        const int nblk_t1 = validB ? (causal ? (2 * qb2 + 2) : (S / kABN)) : 0;
-        const int nblk = nblk_t1 > nblk_t0 ? nblk_t1 : nblk_t0;
-        auto nblk_of = [&](int t) { return t == 0 ? nblk_t0 : nblk_t1; };
-        auto issue_qk = [&](int t, int j, bool release_k) {
-          const uint32_t g = g0 + j;
-          const int st = g & 1u;
-          mbar_wait(&bar_kfull[st], (g >> 1) & 1u);
-          tc_fence_after();
-          const uint32_t q_addr = smem_base + t * kTile;
-          const uint32_t k_addr = smem_base + 2 * kTile + st * kTile;
+    // starves the softmax warps), 1010 -> 720-830 TFLOP/s.  This warp's issue latency is on the critical path:
+    // the whole warp walks the loop and waits, only the products and commits are issued by one elected lane, so that
+    // addresses and descriptors stay in uniform registers, which the instruction reads.
+    constexpr uint32_t idesc_qk = make_idesc_bf16(kRows, kRows, 0u, 0u);   // A, B K-major
+    constexpr uint32_t idesc_pv = make_idesc_bf16(kRows, DV, 0u, 1u);      // A from TMEM, B MN-major (V)
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort)) != 0; };
+    uint32_t g0 = 0;                 // K/V blocks consumed by earlier items
+    uint32_t nQ0 = 0, nQ1 = 0;       // items done per tile (Q / O barrier phases)
+    uint32_t nP0 = 0, nP1 = 0;       // P V products issued per tile (bar_p phases)
+    bool ok = true;
+    for (int item, r = 0; ok && next_item(r, item); ++r) {
+      int q0, head, b;
+      Seq sq;
+      if (!decode(item, q0, head, b, sq)) continue;
+      const int nblk_t0 = blocks(sq, q0, 0), nblk_t1 = blocks(sq, q0, 1);
+      const int nblk = max(nblk_t0, nblk_t1);
+      auto issue_qk = [&](int t, int j, bool release_k, bool last) {
+        const uint32_t g = g0 + j, st = g % C::kKStages;
+        if (!wait(&bar_kfull[st], (g / C::kKStages) & 1u)) return false;
+        tc_fence_after();
+        const uint64_t qd = make_smem_desc(smem_base + t * C::kQTile, 16, 1024, 2);
+        const uint64_t kd = make_smem_desc(smem_base + C::kKAt + st * C::kQTile, 16, 1024, 2);
+        if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < kAD / 16; ++ks) {
-            const uint32_t off = (ks >> 2) * kPanel + (ks & 3) * 32;
-            umma_ss<1>(tmem_base + t * 128, make_smem_desc(q_addr + off, 16, 1024, 2),
-                       make_smem_desc(k_addr + off, 16, 1024, 2), idesc_qk, ks != 0 ? 1u : 0u);
+          for (int ks = 0; ks < DQK / 16; ++ks) {
+            const uint64_t off = ((ks >> 2) * kPanel + (ks & 3) * 32) >> 4;
+            umma_ss<1>(tmem_base + t * 128, qd + off, kd + off, idesc_qk, ks != 0 ? 1u : 0u);
           }
           umma_commit<1>(&bar_s[t]);
           if (release_k) umma_commit<1>(&bar_kempty[st]);
-          if (j + 1 == nblk_of(t)) umma_commit<1>(&bar_qfree[t]);       // last use of this item's Q_t
-        };
-        mbar_wait(&bar_q[0], nQ[0] & 1u);
-        issue_qk(0, 0, !validB);
-        if (validB) {
-          mbar_wait(&bar_q[1], nQ[1] & 1u);
-          issue_qk(1, 0, true);
+          if (last) umma_commit<1>(&bar_qfree[t]);       // last use of this item's Q_t
         }
-        for (int j = 0; j < nblk; ++j) {
-          const uint32_t g = g0 + j;
-          const int st = g & 1u;
-          for (int t = 0; t < 2; ++t) {
-            if (j >= nblk_of(t)) continue;
-            mbar_wait(&bar_vfull[st], (g >> 1) & 1u);
-            mbar_wait(&bar_p[t], nP[t] & 1u);                  // P_t(j) is in TMEM, O_t rescaled if needed
-            ++nP[t];
-            if (j == 0 && nQ[t] > 0) mbar_wait(&bar_ofree[t], (nQ[t] - 1) & 1u);   // previous item's O_t was read out
-            tc_fence_after();
-            const uint32_t v_addr = smem_base + 4 * kTile + st * kTile;
-            const uint32_t tP = tmem_base + t * 128;
-            const uint32_t tOt = tmem_base + 256 + t * 128;
+        return true;
+      };
+      // P V of tile t and block j, then Q K^T of its block j + 1
+      auto step = [&](int t, int j, int mine, int other, uint32_t nQ, uint32_t nP) {
+        const uint32_t vs = (g0 + j) % C::kVStages;
+        if (!wait(&bar_vfull[vs], ((g0 + j) / C::kVStages) & 1u)) return false;
+        if (!wait(&bar_p0[t], nP & 1u)) return false;    // first half of P_t(j) is in TMEM, O_t rescaled if needed
+        if (j == 0 && nQ > 0 && !wait(&bar_ofree[t], (nQ - 1) & 1u)) return false;   // previous item's O_t was read out
+        tc_fence_after();
+        const uint64_t vd = make_smem_desc(smem_base + C::kVAt + vs * C::kVTile, kPanel, 1024, 2);
+        const uint32_t tP = tmem_base + t * 128;
+        const uint32_t tOt = tmem_base + 256 + t * 128;
+        if (elect_one()) {
 #pragma unroll
-            for (int ks = 0; ks < kABN / 16; ++ks)
-              umma_ts<1>(tOt, tP + ks * 8, make_smem_desc(v_addr + ks * 2048, kPanel, 1024, 2), idesc_pv,
-                         (j | ks) != 0 ? 1u : 0u);
-            if (t == 1 || j >= nblk_t1) umma_commit<1>(&bar_vempty[st]);    // last reader of V(j)
-            if (j + 1 < nblk_of(t))
-              issue_qk(t, j + 1, t == 1 || j + 1 >= nblk_t1);
-            else
-              umma_commit<1>(&bar_o[t]);
-          }
+          for (int ks = 0; ks < kRows / 32; ++ks)
+            umma_ts<1>(tOt, tP + ks * 8, vd + ks * (2048 >> 4), idesc_pv, (j | ks) != 0 ? 1u : 0u);
         }
-        g0 += nblk;
-        ++nQ[0];
-        if (validB) ++nQ[1];
+        if (!wait(&bar_p1[t], nP & 1u)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = kRows / 32; ks < kRows / 16; ++ks)
+            umma_ts<1>(tOt, tP + ks * 8, vd + ks * (2048 >> 4), idesc_pv, 1u);
+          if (t == 1 || j >= other) umma_commit<1>(&bar_vempty[vs]);    // last reader of V(j)
+          if (j + 1 == mine) umma_commit<1>(&bar_o[t]);
+        }
+        return j + 1 < mine ? issue_qk(t, j + 1, t == 1 || j + 1 >= other, j + 2 == mine) : true;
+      };
+      if (!(ok = wait(&bar_q[0], nQ0 & 1u) && issue_qk(0, 0, nblk_t1 == 0, nblk_t0 == 1))) break;
+      if (nblk_t1 > 0 && !(ok = wait(&bar_q[1], nQ1 & 1u) && issue_qk(1, 0, true, nblk_t1 == 1))) break;
+      for (int j = 0; ok && j < nblk; ++j) {
+        if (j < nblk_t0) ok = step(0, j, nblk_t0, nblk_t1, nQ0, nP0++);
+        if (ok && j < nblk_t1) ok = step(1, j, nblk_t1, nblk_t0, nQ1, nP1++);
       }
+      g0 += nblk;
+      ++nQ0;
+      if (nblk_t1 > 0) ++nQ1;
     }
    }
   } else {
@@ -369,63 +395,73 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const uint32_t tOt = tmem_base + 256 + t * 128 + lane_off;
     uint32_t nS = 0;                               // S tiles consumed so far (bar_s phase)
     uint32_t nO = 0;                               // items finished by this tile (bar_o phase)
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-      int qb2, head, b;
-      decode(item, qb2, head, b);
-      const int q0 = qb2 * 2 * kABM;
-      const int qt0 = q0 + t * kABM;
-      if (qt0 >= S) continue;                      // tile B past the end of the sequence: nobody touches its barriers
-      const int nb = causal ? (2 * qb2 + t + 1) : (S / kABN);
-      const int tok0 = b * S;
+    bool ok = true;
+    for (int item, r = 0; ok && next_item(r, item); ++r) {
+      int q0, head, b;
+      Seq sq;
+      if (!decode(item, q0, head, b, sq)) continue;
+      const int nb = blocks(sq, q0, t);
+      if (nb == 0) continue;                       // tile B past the end of the sequence: nobody touches its barriers
+      const int qt0 = q0 + t * kRows;
       float m_ref = -INFINITY, l0 = 0.f, l1 = 0.f;
       for (int j = 0; j < nb; ++j, ++nS) {
-        mbar_wait(&bar_s[t], nS & 1u);
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_s[t], nS & 1u, abort));
+        if (!ok) break;
         tc_fence_after();
         if (q == 0 && lane == 0) ev(t, 1);
-        if (causal && j == nb - 1)
-          softmax_block_v2<true>(tS, tOt, row, j == 0, scale_log2, m_ref, l0, l1);
+        const int off = sq.start + qt0 - j * kRows;      // the tile's first row sees the block's columns up to this one
+        if (causal && off < kRows - 1)
+          softmax_block<true, DV>(tS, tOt, q, lane, off, j == 0, scale_log2, m_ref, l0, l1, &bar_p0[t], &bar_p1[t]);
         else
-          softmax_block_v2<false>(tS, tOt, row, j == 0, scale_log2, m_ref, l0, l1);
-        tc_fence_before();
-        __syncwarp();
+          softmax_block<false, DV>(tS, tOt, q, lane, off, j == 0, scale_log2, m_ref, l0, l1, &bar_p0[t], &bar_p1[t]);
         if (q == 0 && lane == 0) ev(t, 2);
-        if (lane == 0) mbar_arrive(&bar_p[t]);
       }
-      // ---- epilogue: O / l -> bf16 -> global (row per thread), LSE ----
-      mbar_wait(&bar_o[t], nO & 1u);
+      if (!ok) break;
+      // ---- epilogue: O / l -> bf16 -> global (row per thread, whole 32-byte sectors), LSE ----
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_o[t], nO & 1u, abort));
+      if (!ok) break;
       ++nO;
       tc_fence_after();
       const float l = l0 + l1;
       const float inv_l = 1.f / l;
-      __nv_bfloat16* orow = O + (static_cast<long long>(tok0 + qt0 + row)) * o_tok_stride + head * kAD;
+      const bool real = qt0 + row < sq.n;
+      const long long tok = static_cast<long long>(b) * max_q + qt0 + row;
+      __nv_bfloat16* orow = O + tok * o_tok_stride + head * DV;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < DV / 32; ++c) {
         uint32_t r[32];
         tmem_ld_x32(tOt + c * 32, r);
         tmem_ld_wait();
-        if (c == 3) {                              // O_t is in registers: the next item's P V may overwrite it
+        if (c == DV / 32 - 1) {                    // O_t is in registers: the next item's P V may overwrite it
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bar_ofree[t]);
         }
+        if (!real) continue;
 #pragma unroll
-        for (int gq = 0; gq < 4; ++gq) {
-          uint4 w;
-          w.x = pack_bf16x2(__uint_as_float(r[gq * 8 + 0]) * inv_l, __uint_as_float(r[gq * 8 + 1]) * inv_l);
-          w.y = pack_bf16x2(__uint_as_float(r[gq * 8 + 2]) * inv_l, __uint_as_float(r[gq * 8 + 3]) * inv_l);
-          w.z = pack_bf16x2(__uint_as_float(r[gq * 8 + 4]) * inv_l, __uint_as_float(r[gq * 8 + 5]) * inv_l);
-          w.w = pack_bf16x2(__uint_as_float(r[gq * 8 + 6]) * inv_l, __uint_as_float(r[gq * 8 + 7]) * inv_l);
-          *reinterpret_cast<uint4*>(orow + c * 32 + gq * 8) = w;
+        for (int gq = 0; gq < 2; ++gq) {
+          uint32_t w[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            w[e] = pack_bf16x2(__uint_as_float(r[gq * 16 + 2 * e]) * inv_l, __uint_as_float(r[gq * 16 + 2 * e + 1]) * inv_l);
+          __nv_bfloat16* dst = orow + c * 32 + gq * 16;
+          if (o_wide) {
+            st_v8(dst, w);
+          } else {
+            st_v4(dst, make_uint4(w[0], w[1], w[2], w[3]));
+            st_v4(dst + 8, make_uint4(w[4], w[5], w[6], w[7]));
+          }
         }
       }
-      if (lse != nullptr)
-        lse[(static_cast<long long>(b) * H + head) * S + qt0 + row] = (m_ref + log2f(l)) * 0.6931471805599453f;
+      if (lse != nullptr && real)
+        lse[(static_cast<long long>(b) * H + head) * max_q + qt0 + row] = (m_ref + log2f(l)) * 0.6931471805599453f;
       if (q == 0 && lane == 0) ev(t, 3);
     }
   }
 
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && abort_flag) atomicCAS(&g_status, 0u, 1u);
   if (warp == 9) {
     tc_fence_after();
     tmem_dealloc<1>(tmem_base, 512);
@@ -446,6 +482,23 @@ static long long* flash_trace_buffer() {
   return buf;
 }
 
+// Persistent launch: one CTA per SM over a heavy-first item list.
+template <int DQK, int DV>
+static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, void* o, long long o_tok_stride, float* lse,
+                            int B, int max_q, int H, float scale, int causal, cudaStream_t s) {
+  using namespace ffwd;
+  using C = Cfg<DQK, DV>;
+  const cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<DQK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const long long n_items = static_cast<long long>((max_q + 2 * kRows - 1) / (2 * kRows)) * H * B;
+  if (n_items >= (1ll << 31) - 2 * kNumSMs) return static_cast<int>(cudaErrorInvalidValue);
+  const int grid = n_items < kNumSMs ? static_cast<int>(n_items) : kNumSMs;
+  const int wide = o_tok_stride % 16 == 0 && (reinterpret_cast<uintptr_t>(o) & 31) == 0;
+  flash_fwd_kernel<DQK, DV><<<grid, kThreads, C::kSmem, s>>>(q, k, v, (__nv_bfloat16*)o, o_tok_stride, wide, lse, B, max_q, H,
+                                                             scale * 1.4426950408889634f, causal, flash_trace_buffer());
+  return static_cast<int>(cudaGetLastError());
+}
+
 }  // namespace llmctl
 
 using namespace llmctl;
@@ -458,30 +511,38 @@ LLMCTL_API int llmctl_flash_trace_read(long long* host_out) {
   return static_cast<int>(cudaMemcpy(host_out, b, 2048 * sizeof(long long), cudaMemcpyDeviceToHost));
 }
 
-// q,k,v: [B, S, H, 128] bf16 views with a common layout: element (b,s,h,d) at ((b*S+s)*tok_stride + h*128 + d).
-// o: same indexing with o_tok_stride.  lse: fp32 [B, H, S] (may be NULL).  S must be a multiple of 128.
+// 0 unless a bounded wait of the forward kernel ran out since the last clearing call (synchronises the device).
+LLMCTL_API int llmctl_flash_fwd_status(int clear) {
+  unsigned int v = 0;
+  if (cudaMemcpyFromSymbol(&v, ffwd::g_status, sizeof(v)) != cudaSuccess) return -1;
+  if (clear && v != 0) {
+    const unsigned int zero = 0;
+    (void)cudaMemcpyToSymbol(ffwd::g_status, &zero, sizeof(zero));
+  }
+  return static_cast<int>(v);
+}
+
+// q,k,v: [B, S, H, D] bf16 views, D = 64 or 128, with a common layout: element (b,s,h,d) at ((b*S+s)*tok_stride + h*D + d).
+// o: same indexing with o_tok_stride.  lse: fp32 [B, H, S] (may be NULL).  Any S when causal, else a multiple of 128.
 LLMCTL_API int llmctl_flash_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B,
                                      int S, int H, int D, long long q_tok_stride, long long k_tok_stride,
                                      long long v_tok_stride, long long o_tok_stride, float scale, int causal,
                                      void* stream) {
   LLMCTL_BEGIN();
-  LLMCTL_REQUIRE(D == kAD && S % kABM == 0 && B > 0 && H > 0);
+  LLMCTL_REQUIRE((D == 128 || D == 64) && (causal || S % 128 == 0) && B > 0 && S > 0 && H > 0);
   LLMCTL_REQUIRE(q_tok_stride % 8 == 0 && k_tok_stride % 8 == 0 && v_tok_stride % 8 == 0 && o_tok_stride % 8 == 0);
-  CUtensorMap tq, tk, tv;
-  const uint64_t rows = static_cast<uint64_t>(B) * S;
-  int rc = get_tmap_3d_bf16(&tq, q, kAD, H, rows, kAD, q_tok_stride, 64, 1, kABM, 1);
-  if (rc) LLMCTL_FAIL(rc, "tensor map Q");
-  rc = get_tmap_3d_bf16(&tk, k, kAD, H, rows, kAD, k_tok_stride, 64, 1, kABN, 1);
-  if (rc) LLMCTL_FAIL(rc, "tensor map K");
-  rc = get_tmap_3d_bf16(&tv, v, kAD, H, rows, kAD, v_tok_stride, 64, 1, kABN, 1);
-  if (rc) LLMCTL_FAIL(rc, "tensor map V");
   LLMCTL_REQUIRE(scale > 0.f);
-  // persistent kernel: one CTA per SM over a heavy-first item list
-  LLMCTL_CHECK(cudaFuncSetAttribute(flash_fwd3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kF2Smem));
-  const int n_items = ((S + 2 * kABM - 1) / (2 * kABM)) * H * B;
-  const int grid3 = n_items < kNumSMs ? n_items : kNumSMs;
-  flash_fwd3_kernel<<<grid3, kF2Threads, kF2Smem, (cudaStream_t)stream>>>(
-      tq, tk, tv, (__nv_bfloat16*)o, o_tok_stride, lse, B, S, H, scale * 1.4426950408889634f, causal,
-      flash_trace_buffer());
-  LLMCTL_RETURN_LAST();
+  CUtensorMap tq, tk, tv;
+  int rc = 0;
+  auto mkmap = [&](CUtensorMap* m, const void* base, long long tok) {
+    if (!rc) rc = get_tmap_4d_bf16(m, base, D, H, S, B, D, tok, static_cast<uint64_t>(S) * tok, 64, 1, ffwd::kRows, 1, 1);
+  };
+  mkmap(&tq, q, q_tok_stride);
+  mkmap(&tk, k, k_tok_stride);
+  mkmap(&tv, v, v_tok_stride);
+  if (rc) LLMCTL_FAIL(rc, "tensor map Q / K / V");
+  rc = (D == 128 ? flash_fwd_launch<128, 128> : flash_fwd_launch<64, 64>)(tq, tk, tv, o, o_tok_stride, lse, B, S, H, scale, causal,
+                                                                          (cudaStream_t)stream);
+  if (rc) LLMCTL_FAIL(rc, "flash forward");
+  return 0;
 }

@@ -77,6 +77,23 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   }
 }
 
+// Bounded wait of a kernel whose roles share an abort flag in shared memory: false when the wait ran out (the flag is raised for
+// the other roles) or another role gave up.  The clock is read only when the barrier is not there yet.
+constexpr long long kBoundedWaitCycles = 400000000LL;      // ~0.2 s: far beyond any wait of a healthy pipeline
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  for (uint32_t it = 1;; ++it) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((it & 63u) == 0u) {
+      if (*abort) return false;
+      if (clock64() - t0 > kBoundedWaitCycles) break;
+    }
+  }
+  *abort = 1;
+  return false;
+}
+
 // ----------------------------------------------------------------------------------------------
 // TMA
 // ----------------------------------------------------------------------------------------------
@@ -118,6 +135,14 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, "
       "%4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
       "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int32_t c0, int32_t c1,
+                                            int32_t c2, int32_t c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, "
+      "%4, %5, %6}], [%2];" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* smem_src, int32_t c0,
@@ -409,6 +434,12 @@ __device__ __forceinline__ void st_v4(void* p, uint4 v) {
                "r"(v.w)
                : "memory");
 }
+// 32 bytes at a 32-byte boundary: one whole L2 sector per lane.
+__device__ __forceinline__ void st_v8(void* p, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+               "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
 // NVLS: load-reduce 8 bf16 (as 4 x bf16x2) from a multicast address; fp32 accumulation in-switch.
 __device__ __forceinline__ uint4 multimem_ld_reduce_bf16x8(const void* mc_ptr) {
   uint4 r;
@@ -438,6 +469,11 @@ __device__ __forceinline__ void multimem_st_v4(void* mc_ptr, uint4 v) {
 __device__ __forceinline__ float ex2_approx(float x) {     // 2^x on the SFU, flush-to-zero, no range fix-up
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {      // three-input maximum, one instruction on sm_100
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
   return y;
 }
 // Blackwell issues fp32 FMA / ADD on register pairs (FFMA2 / FADD2): half the issue slots of scalar code.
@@ -500,34 +536,6 @@ __device__ __forceinline__ void setmaxnreg_inc() {
 template <int N>
 __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
-}
-// (a0,a1) * (b0,b1) + (c0,c1)
-__device__ __forceinline__ void fma2vv(float& d0, float& d1, float a0, float a1, float b0, float b1, float c0, float c1) {
-  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
-      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
-      "fma.rn.f32x2 rd, ra, rb, rc;\n\t"
-      "mov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d0), "=f"(d1)
-      : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
-}
-// 2^x for two values WITHOUT the SFU: the exponential unit (16 results / clk / SM) is as scarce as the tensor
-// core in attention (one exp per score), so part of the row is evaluated on the FMA pipes instead.
-// Round-to-nearest split x = n + f, |f| <= 0.5 via the 1.5*2^23 trick (n sits in the low mantissa bits of t),
-// cubic minimax 2^f (max relative error 7.5e-5, below bf16 resolution), exponent patched in with one integer
-// multiply-add.  Inputs are clamped to >= -126 (masked scores give ~1e-38, i.e. zero weight).
-__device__ __forceinline__ void ex2_poly2(float& p0, float& p1, float x0, float x1) {
-  constexpr float kMagic = 12582912.f;   // 1.5 * 2^23
-  x0 = fmaxf(x0, -126.f);
-  x1 = fmaxf(x1, -126.f);
-  float t0, t1, r0, r1, f0, f1, q0, q1;
-  add2v(t0, t1, x0, x1, kMagic, kMagic);
-  add2v(r0, r1, t0, t1, -kMagic, -kMagic);
-  fma2v(f0, f1, r0, r1, -1.f, x0, x1);
-  fma2(q0, q1, f0, f1, 0.05517167f, 0.24261112f);
-  fma2vv(q0, q1, q0, q1, f0, f1, 0.69326099f, 0.69326099f);
-  fma2vv(q0, q1, q0, q1, f0, f1, 0.99992807f, 0.99992807f);
-  p0 = __int_as_float(__float_as_int(q0) + (__float_as_int(t0) << 23));
-  p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(t1) << 23));
 }
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");

@@ -30,13 +30,13 @@ static EncodeTiledFn resolve_encode() {
 }
 
 struct Key {
-  uint64_t v[11];
+  uint64_t v[14];
   bool operator==(const Key& o) const { return memcmp(v, o.v, sizeof(v)) == 0; }
 };
 struct KeyHash {
   size_t operator()(const Key& k) const {
     uint64_t h = 1469598103934665603ull;
-    for (int i = 0; i < 11; ++i) {
+    for (int i = 0; i < 14; ++i) {
       h ^= k.v[i];
       h *= 1099511628211ull;
     }
@@ -67,7 +67,7 @@ static int encode_cached(CUtensorMap* out, const Key& key, int rank, const void*
     (void)cudaFree(nullptr);
     ctx_bound = true;
   }
-  cuuint32_t estr[3] = {1, 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims,
                   strides_bytes, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -123,6 +123,21 @@ int get_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d
   cuuint64_t strides[2] = {s1 * 2, s2 * 2};
   cuuint32_t box[3] = {b0, b1, b2};
   return encode_cached(out, key, 3, base, dims, strides, box, swizzle128);
+}
+
+int get_tmap_4d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t d3,
+                     uint64_t s1, uint64_t s2, uint64_t s3, uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3,
+                     int swizzle128) {
+  Key key;
+  memset(&key, 0, sizeof(key));
+  const uint64_t all[13] = {reinterpret_cast<uint64_t>(base), d0, d1, d2, d3, s1, s2, s3, b0, b1, b2, b3,
+                            static_cast<uint64_t>(swizzle128)};
+  memcpy(key.v, all, sizeof(all));
+  key.v[13] = 4;
+  cuuint64_t dims[4] = {d0, d1, d2, d3};
+  cuuint64_t strides[3] = {s1 * 2, s2 * 2, s3 * 2};
+  cuuint32_t box[4] = {b0, b1, b2, b3};
+  return encode_cached(out, key, 4, base, dims, strides, box, swizzle128);
 }
 
 }  // namespace llmctl

@@ -19,4 +19,9 @@ int get_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d
                      uint64_t s1, uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2,
                      int swizzle128);
 
+// 4D bf16 tensor map: dims (inner -> outer) = {d0, d1, d2, d3} with strides (elements) {1, s1, s2, s3}.
+int get_tmap_4d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t d3,
+                     uint64_t s1, uint64_t s2, uint64_t s3, uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3,
+                     int swizzle128);
+
 }  // namespace llmctl

@@ -2,8 +2,8 @@
 
 ``attention(q, k, v)`` takes ``[B, S, H, D]`` views (typically slices of the packed qkv activation) and
 dispatches to the tcgen05 flash-attention kernels (``csrc/attention``) when they are built and the shape is
-supported (bf16, head_dim 128, or 64 zero-padded to 128; causal sequences of any length — ragged ones are padded to the
-128-token tile), else to PyTorch SDPA (other head sizes, non-causal ragged shapes, CPU).
+supported (bf16, head_dim 64 or 128; causal sequences of any length, others of whole 128-token tiles), else to PyTorch
+SDPA (other head sizes, non-causal ragged shapes, CPU).
 
 Reference: the reference never calls attention itself — HF modules pick SDPA/eager behind
 ``self.model(**batch)`` (reference llmctl/runtime/engine.py:284); its tuner benchmarks a naive
@@ -34,18 +34,31 @@ native.register_signature(
     [c_int, c_int, c_int, c_int] + [c_ll] * 5 + [c_float, c_int, c_void_p])
 
 
-def _native_ok(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
-    if not (q.is_cuda and q.dtype == torch.bfloat16 and kernel_config().attention == "native"):
-        return False
-    if not native.has_symbol("llmctl_flash_attn_fwd"):
+def _native_built(q: torch.Tensor) -> bool:
+    return (q.is_cuda and q.dtype == torch.bfloat16 and kernel_config().attention == "native"
+            and native.has_symbol("llmctl_flash_attn_fwd"))
+
+
+def _native_shape(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool) -> bool:
+    """The kernels' tiles end inside a sequence only under the causal mask, which hides the keys past its end."""
+    return q.shape[-1] in (64, 128) and (causal or q.shape[1] % 128 == 0) and k.shape == q.shape and v.shape == q.shape
+
+
+def _native_ok(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = True) -> bool:
+    """The kernels read these views where they lie: heads side by side in a token, whole 16-byte units, sequences back to back."""
+    if not (_native_built(q) and _native_shape(q, k, v, causal)):
         return False
     B, S, H, D = q.shape
-    if D != 128 or S % 128 != 0:
-        return False
     for t in (q, k, v):
-        if t.stride(3) != 1 or t.stride(2) != D or t.stride(0) != S * t.stride(1) or t.stride(1) % 8:
+        if (t.dtype != q.dtype or t.stride(3) != 1 or t.stride(2) != D or (B > 1 and t.stride(0) != S * t.stride(1))
+                or t.stride(1) % 8 or t.data_ptr() % 16):
             return False
     return True
+
+
+def _stats_scratch(B: int, S: int, H: int, device: torch.device) -> torch.Tensor:
+    """Scratch of the backward kernels: two numbers per (head, query), sequences rounded up to whole tiles, and two counters."""
+    return torch.empty(2 * B * H * ((S + 127) // 128 * 128) + 2, dtype=torch.float32, device=device)
 
 
 class _FlashAttnFn(torch.autograd.Function):
@@ -70,7 +83,7 @@ class _FlashAttnFn(torch.autograd.Function):
             # dq|dk|dv packed like the forward's qkv so the following wgrad GEMM sees one tensor
             dqkv = torch.empty(B, S, 3, H, D, dtype=q.dtype, device=q.device)
             dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
-            scratch = torch.empty(B * H * S * (D + 1), dtype=torch.float32, device=q.device)
+            scratch = _stats_scratch(B, S, H, q.device)
             native.call("llmctl_flash_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                         do.data_ptr(), lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                         scratch.data_ptr(), B, S, H, D, q.stride(1), k.stride(1), v.stride(1), o.stride(1),
@@ -93,25 +106,13 @@ def _sdpa(q, k, v, causal, scale):
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = True,
               scale: Optional[float] = None) -> torch.Tensor:
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
-    if _native_ok(q, k, v):
+    if _native_ok(q, k, v, causal):
         return _FlashAttnFn.apply(q, k, v, scale, causal)
-    S = q.shape[1]
-    if (q.shape[-1] == 64 and q.is_cuda and q.dtype == torch.bfloat16 and kernel_config().attention == "native"
-            and native.has_symbol("llmctl_flash_attn_fwd") and (causal or S % 128 == 0)):
-        # head_dim 64 (gpt-125m class models): the kernel's tiles are 128 wide, so the head is zero-padded to 128 —
-        # zero q/k columns add nothing to the scores, zero v columns produce zero outputs that are sliced away.  Twice
-        # the attention work of a native 64-wide kernel, but on the tensor cores and without a second code path.
-        qp, kp, vp = (F.pad(t, (0, 64)) for t in (q, k, v))
-        return attention(qp, kp, vp, causal=causal, scale=scale)[..., :64]
-    if (causal and S % 128 and q.is_cuda and q.dtype == torch.bfloat16 and q.shape[-1] == 128
-            and kernel_config().attention == "native" and native.has_symbol("llmctl_flash_attn_fwd")):
-        # ragged length (every serving prefill): pad the sequence to the kernel's 128-token tile.  Under the causal
-        # mask the zero keys appended at the end are invisible to every real query; the padded queries' rows are
-        # dropped.  (Differentiable: F.pad / slicing carry the gradient.)
-        pad = 128 - S % 128
-        qp, kp, vp = (F.pad(t, (0, 0, 0, 0, 0, pad)) for t in (q, k, v))
-        if _native_ok(qp, kp, vp):
-            return _FlashAttnFn.apply(qp, kp, vp, scale, causal)[:, :S]
+    if _native_built(q) and _native_shape(q, k, v, causal) and k.dtype == v.dtype == q.dtype and (q.shape[-1] == 64 or q.shape[1] % 128):
+        # other strides or an odd address: head_dim 64 and ragged lengths (gpt-125m, every serving prefill) are always copied for
+        # the kernel, whole 128-wide tiles are left to the library
+        q, k, v = (t.clone(memory_format=torch.contiguous_format) for t in (q, k, v))
+        return _FlashAttnFn.apply(q, k, v, scale, causal)
     return _sdpa(q, k, v, causal, scale)
 
 
@@ -200,7 +201,7 @@ class _RopeAttnPackedFn(torch.autograd.Function):
         do4 = do.reshape(B, S, H, D)
         if use_native and native.has_symbol("llmctl_flash_attn_bwd"):
             do4 = do4.contiguous()
-            scratch = torch.empty(B * H * S * (D + 1), dtype=torch.float32, device=qkv.device)
+            scratch = _stats_scratch(B, S, H, qkv.device)
             native.call("llmctl_flash_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do4.data_ptr(),
                         lse.data_ptr(), d5[:, :, 0].data_ptr(), d5[:, :, 1].data_ptr(), d5[:, :, 2].data_ptr(),
                         scratch.data_ptr(), B, S, H, D, q.stride(1), k.stride(1), v.stride(1), o.stride(1),
@@ -236,8 +237,8 @@ def rope_attention_packed(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tenso
         use_native = _native_ok(v5[:, :, 0], v5[:, :, 1], v5[:, :, 2]) and \
             (native.has_symbol("llmctl_flash_attn_bwd") or not torch.is_grad_enabled())
         pos = None if positions is None else positions.to(torch.int32)
-        # shapes the kernel only takes after padding (head_dim 64, ragged length) go through the composed ops below,
-        # where attention() pads them, instead of dropping to the library inside the fused node
+        # views the kernel only takes after a copy (an odd address at head_dim 64 or a ragged length) go through the composed
+        # ops below, where attention() makes it, instead of dropping to the library inside the fused node
         paddable = (not use_native and cfg.attention == "native" and native.has_symbol("llmctl_flash_attn_bwd")
                     and (head_dim == 64 or (head_dim == 128 and seq % 128 != 0)))
         if not paddable:

@@ -112,12 +112,14 @@ int llmctl_gemm_skinny_bf16(const void* X, const void* W, void* C, int Mb, int N
                             long long ldw, long long ldc, float* workspace, long long workspace_elems,
                             unsigned int* counters, int n_counters, int splits, void* stream);
 
-/* ---- K6 causal flash attention, head_dim 128, bf16.  q/k/v/o: [B,S,H,128] views with token strides in
- * elements; lse: fp32 [B,H,S] (natural log).  S % 128 == 0.  Reference: SDPA/eager inside the HF model
- * (engine.py:284); baseline cuDNN SDPA.
- * Forward: 256 queries per CTA as two tiles sharing K/V, S/P/O in TMEM, P never leaves TMEM.
- * Backward: two deterministic kernels (dK/dV on transposed scores, then dQ); scratch >= 2*B*H*S floats
- * (the single-kernel atomic variant selected by LLMCTL_FLASH_BWD_V1 needs B*S*H*129). */
+/* ---- K6 causal flash attention, head_dim 64 or 128, bf16.  q/k/v/o: [B,S,H,D] views with token strides in
+ * elements; lse: fp32 [B,H,S] (natural log).  Any S when causal, else a multiple of 128.  Reference: SDPA/eager inside
+ * the HF model (engine.py:284); baseline cuDNN SDPA.
+ * Forward: 256 queries per work item as two tiles sharing K/V, S/P/O in TMEM, P never leaves TMEM.
+ * Backward: two deterministic kernels (dK/dV on transposed scores, then dQ); scratch: 2*B*H*(S rounded up to 128) + 2 floats.
+ * llmctl_flash_{fwd,bwd}_status: 0 unless a bounded wait ran out since the last clearing call (synchronises the device). */
+int llmctl_flash_fwd_status(int clear);
+int llmctl_flash_bwd_status(int clear);
 int llmctl_flash_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int S, int H,
                           int D, long long q_tok_stride, long long k_tok_stride, long long v_tok_stride,
                           long long o_tok_stride, float scale, int causal, void* stream);

@@ -327,6 +327,40 @@ def test_flash_attention_head_dim_64_uses_the_native_kernel(cuda_device):
         _close(qkv.grad[:, :, i], ref_in.grad[:, :, i], 4e-2, 4e-2, name)
 
 
+# Lengths around the 128-row blocks and the 256-query items, more items than SMs (256 x 3 blocks), several head groups of the
+# backward's item order (S = 2048: 16 heads of 128 to a group), non-causal whole blocks, views at an odd address (copied first).
+@pytest.mark.parametrize("B,S,H,D,causal,shift", [
+    (1, 1, 1, 128, True, 0), (2, 127, 3, 64, True, 0), (1, 128, 2, 64, True, 0), (2, 129, 2, 128, True, 0), (1, 255, 2, 64, True, 0),
+    (2, 257, 3, 128, True, 0), (8, 384, 32, 64, True, 0), (1, 2048, 20, 128, True, 0), (2, 256, 2, 64, False, 0), (1, 384, 2, 128, False, 0),
+    (2, 200, 2, 128, True, 1), (1, 128, 2, 64, True, 1)])
+def test_flash_attention_edges_of_blocks(cuda_device, B, S, H, D, causal, shift):
+    """Forward and backward against float64.  Inputs are exact, P, dS and the outputs are rounded to bf16 (2^-9 each): 3 x 2^-9 in
+    the 2-norm.  At S = 1 dq and dk are zero up to the rounding of o in delta = dO . O."""
+    from llmctl_b200.ops import attention as attn, native
+    torch.manual_seed(S)
+    flat = torch.randn(B * S * 3 * H * D + shift, device=cuda_device).bfloat16()[shift:].view(B, S, 3, H, D)
+    q, k, v = (flat[:, :, i].detach().requires_grad_(True) for i in range(3))
+    assert attn._native_ok(q, k, v, causal) == (shift == 0)
+    do = torch.randn(B, S, H, D, device=cuda_device).bfloat16()
+    before = native.launch_count
+    o = attn.attention(q, k, v, causal=causal)
+    got = (o.detach(), *torch.autograd.grad(o, (q, k, v), do))
+    assert native.launch_count == before + 4
+    assert native.lib().llmctl_flash_fwd_status(1) == 0 and native.lib().llmctl_flash_bwd_status(1) == 0
+    for h in range(H):          # one head at a time: float64 scores of all heads would not be small
+        qd, kd, vd = (t.detach()[:, :, h].double().requires_grad_(True) for t in (q, k, v))
+        s = qd @ kd.transpose(-1, -2) / math.sqrt(D)
+        if causal:
+            s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device=cuda_device).triu(1), float("-inf"))
+        od = torch.softmax(s, -1) @ vd
+        want = (od.detach(), *torch.autograd.grad(od, (qd, kd, vd), do[:, :, h].double()))
+        for name, a, b in zip(("o", "dq", "dk", "dv"), got, want):
+            a = a[:, :, h].double()
+            bound = 3 * 2.0 ** -9 * b.norm() if S > 1 or name in ("o", "dv") else 2.0 ** -8 * do.double().norm() * v.double().norm() * q.double().norm()
+            assert (a - b).norm() <= bound, f"{name} head {h}: {((a - b).norm() / b.norm()).item():.2e}"
+
+
+
 @pytest.mark.parametrize("M,N,K", [(8, 4096, 1376), (8, 4096, 512), (5, 1000, 200), (32, 2752, 4096), (1, 4096, 1384)])
 def test_skinny_gemm_k_tail_and_odd_shapes(cuda_device, M, N, K):
     """Decode GEMM on shapes whose K is not a multiple of the 64-deep k-block (GPT-7B down-projection at TP=8:
