@@ -18,8 +18,10 @@
 // of operands per clock where shared memory gives 128, and started a CTA per item.)  The streamed tiles Q, dO, Q, dO, ... share
 // one ring: with 5 slots beside the two resident tiles (all that 227 KB hold at D = 128) Q(n+1) is fetched as soon as dV(n-2)
 // has retired, a block and a half ahead of its use; rings of two stages each left the pipe waiting 200-1000 clocks per block.
-// Persistent: one CTA per SM claims items, longest of a group first; TMEM, barriers and maps are set up once, and an item's first
-// tiles are fetched while the previous item is still in its softmax and epilogue.
+// P is handed over in two halves, as in the forward.  Persistent: one CTA per SM claims items, longest of a group first; TMEM,
+// barriers and maps are set up once, an item's first tiles are fetched while the previous item is still in its softmax, and a
+// warpgroup of its own reads the accumulators out and stores them meanwhile (a row per thread: 4900 clocks from the last product
+// to the next item's first softmax when the softmax warps did it, against 2900 per block).
 //
 // A ragged sequence ends inside a block: rows past it are zero-filled by TMA, their statistics make P zero, and they are
 // never stored (causal only: keys past the end are then hidden from every real query by the mask).
@@ -35,7 +37,7 @@ using namespace ptx;
 namespace fbwd {
 constexpr int kBlk = 128;                    // rows of a resident or streamed block
 constexpr int kPanel = kBlk * 128;           // bytes of a [128 x 64 bf16] swizzled panel
-constexpr int kThreads = 320;                // TMA, MMA issuer, 2 softmax warpgroups
+constexpr int kThreads = 448;                // TMA, MMA issuer, 2 softmax warpgroups, epilogue warpgroup
 constexpr int kStatBytes = 2 * kBlk * 4;     // -lse * log2e and -delta of 128 queries
 // Items are claimed from a counter by the TMA warp and told to the others through a queue.  It runs at most two items ahead of
 // the softmax warps (the resident tiles are single), so a slot is never overwritten before all have read it.
@@ -53,7 +55,7 @@ struct Cfg {
   static constexpr int kStatSlots = (kSlots - 1) / 2;
   static constexpr int kStatAt = (2 + kSlots) * kTile;                 // behind all tiles: each starts at a multiple of 1024 bytes
   static constexpr int kBarsAt = kStatAt + kStatSlots * kStatBytes;
-  static constexpr int kSmem = kBarsAt + 320;
+  static constexpr int kSmem = kBarsAt + 384;
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
 __device__ unsigned int g_status = 0;        // != 0: a bounded wait of these kernels ran out
@@ -132,12 +134,12 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   using C = Cfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   struct Bars {
-    uint64_t full[C::kSlots], empty[C::kSlots], res, resfree, s, dp, p, ds, acc, accfree, item_full[kQueue];
+    uint64_t full[C::kSlots], empty[C::kSlots], res, resfree, s, dp, p[2], ds, acc[2], accfree[2], item_full[kQueue];
     int item[kQueue];
     uint32_t tmem;
     int abort;
   };
-  static_assert(sizeof(Bars) <= 320, "barriers");
+  static_assert(sizeof(Bars) <= 384, "barriers");
   Bars& bar = *reinterpret_cast<Bars*>(smem + C::kBarsAt);
   const uint32_t smem_base = smem_u32(smem);
   if (smem_base & 1023u) {             // the swizzled tiles would not line up (uniform over the grid)
@@ -157,10 +159,12 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     }
     mbar_init(&bar.s, 1);
     mbar_init(&bar.dp, 1);
-    mbar_init(&bar.p, 8);
     mbar_init(&bar.ds, 8);
-    mbar_init(&bar.acc, 1);
-    mbar_init(&bar.accfree, 8);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar.p[i], 8);
+      mbar_init(&bar.acc[i], 1);
+      mbar_init(&bar.accfree[i], 4);
+    }
     for (int i = 0; i < kQueue; ++i) mbar_init(&bar.item_full[i], 1);
     bar.abort = 0;
     fence_mbar_init();
@@ -275,12 +279,14 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
       }
     };
     // accumulators: 16 of the 128 streamed rows per instruction; the second half of A lies 64 columns on (a softmax
-    // warpgroup writes its half over the columns that it has read itself)
-    auto issue_acc = [&](uint32_t t, uint32_t a, uint32_t sub, uint32_t fresh) {
+    // warpgroup writes its half over the columns that it has read itself).  part 0 / 1: the rows that both warpgroups write
+    // first / last, 2: all.
+    auto issue_acc = [&](uint32_t t, uint32_t a, uint32_t sub, uint32_t fresh, int part) {
       const uint64_t b0 = make_smem_desc(sub, kPanel, 1024, 2);
 #pragma unroll
       for (int ks = 0; ks < kBlk / 16; ++ks)
-        umma_ts<1>(t, a + (ks >> 2) * 64 + (ks & 3) * 8, b0 + ((ks * 2048) >> 4), id_acc, ks == 0 ? 1u - fresh : 1u);
+        if (part == 2 || ((ks >> 1) & 1) == part)
+          umma_ts<1>(t, a + (ks >> 2) * 64 + (ks & 3) * 8, b0 + ((ks * 2048) >> 4), id_acc, ks == 0 ? 1u - fresh : 1u);
     };
     uint32_t g = 0, k = 0;
     bool ok = true;
@@ -307,12 +313,18 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
             if (kDQ) umma_commit<1>(&bar.empty[e1 % C::kSlots]);
           }
         }
-        if (!(ok = wait(&bar.p, g & 1u))) break;           // P(g) written (dKV) / S(g) read (dQ)
-        if (i == 0 && k > 0 && !(ok = wait(&bar.accfree, (k - 1) & 1u))) break;
+        if (!kDQ) {
+          if (!(ok = wait(&bar.p[0], g & 1u))) break;      // half of P(g) is written
+          if (i == 0 && k > 0 && !(ok = wait(&bar.accfree[0], (k - 1) & 1u))) break;
+          tc_fence_after();
+          if (elect_one()) issue_acc(tAcc0, tS, tile_at(e1), fresh, 0);              // dV += P^T dO
+        }
+        if (!(ok = wait(&bar.p[1], g & 1u))) break;        // P(g) written (dKV) / S(g) read (dQ)
         tc_fence_after();
         if (!kDQ && elect_one()) {
-          issue_acc(tAcc0, tS, tile_at(e1), fresh);        // dV += P^T dO
+          issue_acc(tAcc0, tS, tile_at(e1), 0, 1);
           umma_commit<1>(&bar.empty[e1 % C::kSlots]);
+          if (i + 1 == n) umma_commit<1>(&bar.acc[0]);
         }
         if (i + 1 < n) {
           if (!(ok = arrived(e0 + 2))) break;
@@ -323,11 +335,12 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
           }
         }
         if (!(ok = wait(&bar.ds, g & 1u))) break;
+        if (i == 0 && k > 0 && !(ok = wait(&bar.accfree[kDQ ? 0 : 1], (k - 1) & 1u))) break;
         tc_fence_after();
         if (elect_one()) {
-          issue_acc(kDQ ? tAcc0 : tAcc1, tdP, tile_at(e0), fresh);       // dK += dS^T Q  /  dQ += dS K
+          issue_acc(kDQ ? tAcc0 : tAcc1, tdP, tile_at(e0), fresh, 2);    // dK += dS^T Q  /  dQ += dS K
           umma_commit<1>(&bar.empty[e0 % C::kSlots]);
-          if (i + 1 == n) umma_commit<1>(&bar.acc);
+          if (i + 1 == n) umma_commit<1>(&bar.acc[kDQ ? 0 : 1]);
         }
         if (i + 1 < n) {
           if (!(ok = arrived(e1 + 2))) break;
@@ -341,7 +354,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         }
       }
     }
-  } else {
+  } else if (warp < 10) {
     // ------------------- softmax / dS warpgroups: half wg of the streamed columns, all 128 resident rows -------------------
     const int wg = (warp - 2) >> 2;
     const int q4 = warp & 3;
@@ -375,7 +388,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         if (kDQ) {                                        // S is in registers: the next scores may overwrite it
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&bar.p);
+          if (lane == 0) mbar_arrive(&bar.p[1]);
         }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -407,13 +420,15 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
             rs[e + 2] = __float_as_uint(p2);
             rs[e + 3] = __float_as_uint(p3);
           }
-          if (!kDQ) tmem_st_x8(tSb + c * 8, pk);
-        }
-        if (!kDQ) {
-          tmem_st_wait();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bar.p);
+          if (!kDQ) {
+            tmem_st_x8(tSb + c * 8, pk);
+            if (c & 1) {
+              tmem_st_wait();
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bar.p[c >> 1]);
+            }
+          }
         }
         ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar.dp, g & 1u, abort));
         if (!ok) break;
@@ -447,32 +462,42 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar.ds);
       }
-      if (!ok) break;
-      // ---- epilogue: accumulators -> bf16 -> global, a row per thread ----
-      // dKV: warpgroup 0 writes dV (acc0), warpgroup 1 writes scale * dK (acc1).  dQ: each half of acc0's columns.
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar.acc, k & 1u, abort));
-      if (!ok) break;
-      tc_fence_after();
-      constexpr int kCols = kDQ ? D / 2 : D;
-      const int c0 = kDQ ? wg * (D / 2) : 0;
-      const uint32_t tA = ((kDQ || wg == 0) ? tAcc0 : tAcc1) + c0 + lane_off;
-      const float mul = (kDQ || wg == 1) ? scale : 1.f;
+    }
+  } else {
+    // ------------- epilogue warpgroup: accumulators -> registers -> bf16 -> global, a row per thread -------------
+    const int q4 = warp & 3;
+    const int row = q4 * 32 + lane;
+    const uint32_t lane_off = static_cast<uint32_t>(q4 * 32) << 16;
+    uint32_t k = 0;
+    bool ok = true;
+    for (int item; ok && next_item(k, item); ++k) {
+      int rb, bh, first, n;
+      decode(item, rb, bh, first, n);
       const bool real = rb * kBlk + row < S;
-      __nv_bfloat16* dst = ((kDQ || wg == 0) ? out0 : out1) +
-                           (static_cast<long long>(bh / H) * S + rb * kBlk + row) * out_tok + (bh % H) * D + c0;
+      const long long at = (static_cast<long long>(bh / H) * S + rb * kBlk + row) * out_tok + (bh % H) * D;
+#pragma unroll 1
+      for (int a = 0; a < (kDQ ? 1 : 2); ++a) {           // dKV: dV from acc0, then scale * dK from acc1.  dQ: scale * dQ from acc0.
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar.acc[a], k & 1u, abort));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t tA = (a == 0 ? tAcc0 : tAcc1) + lane_off;
+        const float mul = (kDQ || a == 1) ? scale : 1.f;
+        __nv_bfloat16* dst = (a == 0 ? out0 : out1) + at;
 #pragma unroll
-      for (int c = 0; c < kCols; c += 32) {
-        uint32_t r[32];
-        tmem_ld_x32(tA + c, r);
-        tmem_ld_wait();
-        if (c + 32 == kCols) {                            // the accumulators are in registers: the next item may overwrite them
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bar.accfree);
-        }
-        if (real) {
-          fbwd_store16(dst + c, r, mul, out_wide);
-          fbwd_store16(dst + c + 16, r + 16, mul, out_wide);
+        for (int c0 = 0; c0 < D; c0 += 64) {
+          uint32_t r[64];
+          tmem_ld_x32(tA + c0, r);
+          tmem_ld_x32(tA + c0 + 32, r + 32);
+          tmem_ld_wait();
+          if (c0 + 64 == D) {                             // in registers: the next item may overwrite it
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar.accfree[a]);
+          }
+          if (real) {
+#pragma unroll
+            for (int c = 0; c < 64; c += 16) fbwd_store16(dst + c0 + c, r + c, mul, out_wide);
+          }
         }
       }
     }
