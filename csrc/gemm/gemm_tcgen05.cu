@@ -92,15 +92,19 @@ __device__ __forceinline__ void gate_wait_b(const GemmGate& g, int n0, int n_end
 constexpr int kBM = 128;
 constexpr int kBK = 64;  // 64 bf16 = one 128-byte swizzle row
 constexpr int kGemmThreads = 192;
+// Output staging of the epilogue: per warp two buffers of 32 rows x 64 bf16 (128-byte swizzle) that TMA stores read.
+constexpr int kOutBox = 32 * 128;
+constexpr int kOutBytes = 4 * 2 * kOutBox;
 
 template <int BN>
 struct GemmCfg {
-  static constexpr int kStages = (BN == 256) ? 4 : (BN == 192 ? 5 : 6);
+  static constexpr int kStages = (BN == 256 || BN == 192) ? 4 : (BN == 128 ? 6 : 8);
   static constexpr int kABytes = kBM * kBK * 2;
   static constexpr int kBBytes = BN * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024;  // + alignment slack
-  static constexpr int kTmemCols = (2 * BN <= 256) ? 256 : 512;   // power of two >= 2 accumulators of BN columns
+  static constexpr int kOutAt = kStages * kStageBytes;
+  static constexpr int kSmemBytes = kOutAt + kOutBytes + 1024;    // + alignment slack
+  static constexpr int kTmemCols = (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;   // power of two >= 2 accumulators of BN columns
 };
 
 // Epilogue modes
@@ -120,10 +124,90 @@ __device__ __forceinline__ void tile_to_mn(int tile, int num_m, int num_n, int& 
   n_blk = in_group / gsize;
 }
 
+// Epilogue of one tile, one warp: BN accumulator columns of 32 rows (row0 = the warp's first) -> C.
+// bf16 without accumulation goes through shared memory and TMA: 64 columns at a time, each lane packs its row into the swizzled
+// buffer and one lane stores the box, while the next columns are read.  A row per lane straight to global memory touches 32 lines
+// per instruction: an exposed epilogue (the problem is one tile per CTA) took longer than the main loop of K = 768.
+template <int BN, typename OutT>
+__device__ __forceinline__ void gemm_epilogue(uint32_t t_row, uint8_t* out_smem, uint32_t& out_n, const CUtensorMap* tmC,
+                                              OutT* __restrict__ C, long long ldc, int row0, int n0, int M, int N, int beta, int lane) {
+  if constexpr (sizeof(OutT) == 2) {
+    if (!beta) {
+#pragma unroll 1
+      for (int c = 0; c < BN / 64; ++c) {
+        uint32_t r[64];
+        tmem_ld_x32(t_row + c * 64, r);
+        tmem_ld_x32(t_row + c * 64 + 32, r + 32);
+        tmem_ld_wait();
+        if (row0 >= M || n0 + c * 64 >= N) continue;      // uniform over the warp
+        uint8_t* buf = out_smem + (out_n & 1u) * kOutBox;
+        ++out_n;
+        if (lane == 0) tma_store_wait_read<1>();          // the store before the last has left this buffer
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          uint4 w;
+          w.x = pack_bf16x2(__uint_as_float(r[j * 8 + 0]), __uint_as_float(r[j * 8 + 1]));
+          w.y = pack_bf16x2(__uint_as_float(r[j * 8 + 2]), __uint_as_float(r[j * 8 + 3]));
+          w.z = pack_bf16x2(__uint_as_float(r[j * 8 + 4]), __uint_as_float(r[j * 8 + 5]));
+          w.w = pack_bf16x2(__uint_as_float(r[j * 8 + 6]), __uint_as_float(r[j * 8 + 7]));
+          *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) = w;
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(tmC, buf, n0 + c * 64, row0);
+          tma_store_commit();
+        }
+      }
+      return;
+    }
+  }
+  const int row = row0 + lane;
+  OutT* crow = C + static_cast<long long>(row) * ldc + n0;
+#pragma unroll 1
+  for (int c = 0; c < BN / 32; ++c) {
+    uint32_t r[32];
+    tmem_ld_x32(t_row + c * 32, r);
+    tmem_ld_wait();
+    if (row < M) {
+      if constexpr (sizeof(OutT) == 2) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int col = n0 + c * 32 + j * 8;
+          if (col < N) {
+            float f[8], old[8];
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(crow) + c * 32 + j * 8;
+            unpack8(load8(dst), old);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[j * 8 + e]) + old[e];
+            store8(dst, pack8(f));
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int col = n0 + c * 32 + j * 4;
+          if (col < N) {
+            float4 v = make_float4(__uint_as_float(r[j * 4]), __uint_as_float(r[j * 4 + 1]),
+                                   __uint_as_float(r[j * 4 + 2]), __uint_as_float(r[j * 4 + 3]));
+            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(crow) + c * 32 + j * 4);
+            if (beta) {
+              const float4 o = *dst;
+              v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+            }
+            *dst = v;
+          }
+        }
+      }
+    }
+  }
+}
+
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate) {
+                    const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate) {
   using Cfg = GemmCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[Cfg::kStages];
@@ -134,7 +218,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
 
   const int num_m = (M + kBM - 1) / kBM;
@@ -207,48 +291,50 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(kBM, BN, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t aphase = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-        if (gate.grp_tile_expert != nullptr) {
-          int mb_, nb_;
-          tile_to_mn(tile, num_m, num_n, mb_, nb_);
-          if (grouped_b_row(gate, mb_, 0, N) < 0) continue;
-        }
-        mbar_wait(&bar_tempty[acc], aphase ^ 1u);
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        for (int kb = 0; kb < num_kb; ++kb) {
-          mbar_wait(&bar_full[stage], phase);
-          tc_fence_after();
-          const uint32_t a_addr = smem_base + stage * Cfg::kStageBytes;
-          const uint32_t b_addr = a_addr + Cfg::kABytes;
-#pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t da = A_MN ? make_smem_desc(a_addr + k * 2048, 8192, 1024, 2)
-                                     : make_smem_desc(a_addr + k * 32, 16, 1024, 2);
-            const uint64_t db = B_MN ? make_smem_desc(b_addr + k * 2048, 8192, 1024, 2)
-                                     : make_smem_desc(b_addr + k * 32, 16, 1024, 2);
-            umma_ss<1>(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
-          umma_commit<1>(&bar_empty[stage]);  // frees the smem slot once these MMAs retire
-          if (++stage == Cfg::kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
-        }
-        umma_commit<1>(&bar_tfull[acc]);  // accumulator complete -> epilogue
-        acc ^= 1;
-        if (acc == 0) aphase ^= 1u;
+    // The whole warp walks the loop, one elected lane issues: stage addresses and descriptors stay in uniform registers, which
+    // the instruction reads.  From a single lane's branch a product took 85-107 clocks to issue, more than a 128-wide tile's 64.
+    constexpr uint32_t idesc = make_idesc_bf16(kBM, BN, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t aphase = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      if (gate.grp_tile_expert != nullptr) {
+        int mb_, nb_;
+        tile_to_mn(tile, num_m, num_n, mb_, nb_);
+        if (grouped_b_row(gate, mb_, 0, N) < 0) continue;
       }
+      mbar_wait(&bar_tempty[acc], aphase ^ 1u);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        mbar_wait(&bar_full[stage], phase);
+        __syncwarp();
+        tc_fence_after();
+        const uint32_t a_addr = smem_base + stage * Cfg::kStageBytes;
+        const uint64_t da = A_MN ? make_smem_desc(a_addr, 8192, 1024, 2) : make_smem_desc(a_addr, 16, 1024, 2);
+        const uint64_t db = B_MN ? make_smem_desc(a_addr + Cfg::kABytes, 8192, 1024, 2) : make_smem_desc(a_addr + Cfg::kABytes, 16, 1024, 2);
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_ss<1>(d_tmem, da + ((A_MN ? k * 2048 : k * 32) >> 4), db + ((B_MN ? k * 2048 : k * 32) >> 4), idesc, (kb | k) != 0 ? 1u : 0u);
+          umma_commit<1>(&bar_empty[stage]);  // frees the smem slot once these MMAs retire
+          if (kb + 1 == num_kb) umma_commit<1>(&bar_tfull[acc]);  // accumulator complete -> epilogue
+        }
+        if (++stage == Cfg::kStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      acc ^= 1;
+      if (acc == 0) aphase ^= 1u;
     }
   } else {
     // ------------------------------ epilogue (4 warps) ------------------------------
     const int q = warp & 3;  // TMEM lane quadrant this warp may access
+    uint8_t* out_smem = smem + Cfg::kOutAt + q * 2 * kOutBox;
+    uint32_t out_n = 0;
     int acc = 0;
     uint32_t aphase = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
@@ -260,58 +346,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       if (grouped_b_row(gate, mb_, n0, N) < 0) continue;
       mbar_wait(&bar_tfull[acc], aphase);
       tc_fence_after();
-      const int row = m0 + q * 32 + lane;
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
-                             static_cast<uint32_t>(acc * BN);
-      OutT* crow = C + static_cast<long long>(row) * ldc + n0;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_x32(t_row + c * 32, r);
-        tmem_ld_wait();
-        if (row < M) {
-          if constexpr (sizeof(OutT) == 2) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int col = n0 + c * 32 + j * 8;
-              if (col < N) {
-                float f[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[j * 8 + e]);
-                __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(crow) + c * 32 + j * 8;
-                if (beta) {
-                  float old[8];
-                  unpack8(load8(dst), old);
-#pragma unroll
-                  for (int e = 0; e < 8; ++e) f[e] += old[e];
-                }
-                store8(dst, pack8(f));
-              }
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int col = n0 + c * 32 + j * 4;
-              if (col < N) {
-                float4 v = make_float4(__uint_as_float(r[j * 4]), __uint_as_float(r[j * 4 + 1]),
-                                       __uint_as_float(r[j * 4 + 2]), __uint_as_float(r[j * 4 + 3]));
-                float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(crow) + c * 32 + j * 4);
-                if (beta) {
-                  const float4 o = *dst;
-                  v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-                }
-                *dst = v;
-              }
-            }
-          }
-        }
-      }
+      gemm_epilogue<BN, OutT>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN), out_smem, out_n, &tmC, C,
+                              ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_tempty[acc]);
       acc ^= 1;
       if (acc == 0) aphase ^= 1u;
     }
+    if (lane == 0) tma_store_wait_read<0>();      // the staging buffers are read before the CTA gives them back
   }
 
   tc_fence_before();
@@ -343,14 +386,15 @@ struct Gemm2Cfg {
   static constexpr int kABytes = kBM * kBK * 2;          // 128 x 64 per CTA
   static constexpr int kBBytes = (kBN / 2) * kBK * 2;    // (PBN/2) x 64 per CTA
   static constexpr int kStageBytes = kABytes + kBBytes;  // 32 / 24 KB per CTA
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024;
+  static constexpr int kOutAt = kStages * kStageBytes;
+  static constexpr int kSmemBytes = kOutAt + kOutBytes + 1024;
   static constexpr int kTmemCols = 2 * PBN;              // 512 / 256
 };
 
 template <int PBN, bool A_MN, bool B_MN, typename OutT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate) {
+                     const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate) {
   using Cfg = Gemm2Cfg<PBN>;
   constexpr int BN = Cfg::kBN;
   extern __shared__ uint8_t smem_raw[];
@@ -362,7 +406,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const uint32_t cta_rank = cluster_ctarank();   // 0 = leader
   const int pair = blockIdx.x >> 1;
@@ -439,7 +483,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) ------------------------------
-    if (cta_rank == 0 && lane == 0) {
+    if (cta_rank == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(2 * kBM, BN, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
       int stage = 0;
       uint32_t phase = 0;
@@ -447,28 +491,28 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       uint32_t aphase = 0;
       for (int tile = pair; tile < num_tiles; tile += num_pairs) {
         mbar_wait(&bar_tempty[acc], aphase ^ 1u);
+        __syncwarp();
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
         for (int kb = 0; kb < num_kb; ++kb) {
           mbar_wait(&bar_full[stage], phase);
+          __syncwarp();
           tc_fence_after();
           const uint32_t a_addr = smem_base + stage * Cfg::kStageBytes;
-          const uint32_t b_addr = a_addr + Cfg::kABytes;
+          const uint64_t da = A_MN ? make_smem_desc(a_addr, 8192, 1024, 2) : make_smem_desc(a_addr, 16, 1024, 2);
+          const uint64_t db = B_MN ? make_smem_desc(a_addr + Cfg::kABytes, 8192, 1024, 2) : make_smem_desc(a_addr + Cfg::kABytes, 16, 1024, 2);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t da = A_MN ? make_smem_desc(a_addr + k * 2048, 8192, 1024, 2)
-                                     : make_smem_desc(a_addr + k * 32, 16, 1024, 2);
-            const uint64_t db = B_MN ? make_smem_desc(b_addr + k * 2048, 8192, 1024, 2)
-                                     : make_smem_desc(b_addr + k * 32, 16, 1024, 2);
-            umma_ss<2>(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < kBK / 16; ++k)
+              umma_ss<2>(d_tmem, da + ((A_MN ? k * 2048 : k * 32) >> 4), db + ((B_MN ? k * 2048 : k * 32) >> 4), idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_commit_mc2(&bar_empty[stage], 0x3);   // both CTAs' slots are free once these retire
+            if (kb + 1 == num_kb) umma_commit_mc2(&bar_tfull[acc], 0x3);
           }
-          umma_commit_mc2(&bar_empty[stage], 0x3);   // both CTAs' slots are free once these retire
           if (++stage == Cfg::kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        umma_commit_mc2(&bar_tfull[acc], 0x3);
         acc ^= 1;
         if (acc == 0) aphase ^= 1u;
       }
@@ -476,6 +520,8 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   } else {
     // ------------------------------ epilogue (4 warps, both CTAs) ------------------------------
     const int q = warp & 3;
+    uint8_t* out_smem = smem + Cfg::kOutAt + q * 2 * kOutBox;
+    uint32_t out_n = 0;
     int acc = 0;
     uint32_t aphase = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
@@ -486,58 +532,15 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       const int n0 = nb_ * BN;
       mbar_wait(&bar_tfull[acc], aphase);
       tc_fence_after();
-      const int row = m0 + q * 32 + lane;
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
-                             static_cast<uint32_t>(acc * BN);
-      OutT* crow = C + static_cast<long long>(row) * ldc + n0;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_x32(t_row + c * 32, r);
-        tmem_ld_wait();
-        if (row < M) {
-          if constexpr (sizeof(OutT) == 2) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int col = n0 + c * 32 + j * 8;
-              if (col < N) {
-                float f[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[j * 8 + e]);
-                __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(crow) + c * 32 + j * 8;
-                if (beta) {
-                  float old[8];
-                  unpack8(load8(dst), old);
-#pragma unroll
-                  for (int e = 0; e < 8; ++e) f[e] += old[e];
-                }
-                store8(dst, pack8(f));
-              }
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int col = n0 + c * 32 + j * 4;
-              if (col < N) {
-                float4 v = make_float4(__uint_as_float(r[j * 4]), __uint_as_float(r[j * 4 + 1]),
-                                       __uint_as_float(r[j * 4 + 2]), __uint_as_float(r[j * 4 + 3]));
-                float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(crow) + c * 32 + j * 4);
-                if (beta) {
-                  const float4 o = *dst;
-                  v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-                }
-                *dst = v;
-              }
-            }
-          }
-        }
-      }
+      gemm_epilogue<BN, OutT>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN), out_smem, out_n, &tmC, C,
+                              ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(&bar_tempty[acc], 0);   // always the leader's barrier
       acc ^= 1;
       if (acc == 0) aphase ^= 1u;
     }
+    if (lane == 0) tma_store_wait_read<0>();
   }
 
   tc_fence_before();
@@ -578,6 +581,9 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   if (!B_MN) rc = get_tmap_2d_bf16(&tmB, B, static_cast<uint64_t>(N) * (gate.grp_tile_expert ? gate.grp_experts : 1), K, ldb, BN, kBK, 1);
   else rc = get_tmap_2d_bf16(&tmB, B, K, N, ldb, kBK, 64, 1);
   if (rc) LLMCTL_FAIL(rc, "tensor map B");
+  CUtensorMap tmC = tmA;                 // read only by the bf16 epilogue without accumulation
+  if (sizeof(OutT) == 2 && !beta) rc = get_tmap_2d_bf16(&tmC, C, M, N, ldc, 32, 64, 1);
+  if (rc) LLMCTL_FAIL(rc, "tensor map C");
   auto kern = gemm_tcgen05_kernel<BN, A_MN, B_MN, OutT>;
   LLMCTL_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     Cfg::kSmemBytes));
@@ -585,7 +591,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   int grid = num_sms();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (tiles < grid) grid = tiles;
-  kern<<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, (OutT*)C, ldc, M, N, K, beta, gate);
+  kern<<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate);
   LLMCTL_RETURN_LAST();
 }
 
@@ -618,6 +624,9 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
   if (!B_MN) rc = get_tmap_2d_bf16(&tmB, B, N, K, ldb, Cfg::kBN / 2, kBK, 1);
   else rc = get_tmap_2d_bf16(&tmB, B, K, N, ldb, kBK, 64, 1);
   if (rc) LLMCTL_FAIL(rc, "tensor map B");
+  CUtensorMap tmC = tmA;
+  if (sizeof(OutT) == 2 && !beta) rc = get_tmap_2d_bf16(&tmC, C, M, N, ldc, 32, 64, 1);
+  if (rc) LLMCTL_FAIL(rc, "tensor map C");
   auto kern = gemm2_tcgen05_kernel<PBN, A_MN, B_MN, OutT>;
   LLMCTL_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     Cfg::kSmemBytes));
@@ -626,7 +635,7 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
   if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
   if (pairs < 1) pairs = 1;
   if (tiles < pairs) pairs = tiles;
-  kern<<<2 * pairs, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, (OutT*)C, ldc, M, N, K, beta, gate);
+  kern<<<2 * pairs, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate);
   LLMCTL_RETURN_LAST();
 }
 
@@ -645,7 +654,7 @@ static int dispatch_layout2(int a_mn, int b_mn, const void* A, const void* B, vo
 using namespace llmctl;
 
 // D[M,N] = op(A) op(B) (+ D if beta).  a_mn / b_mn select the operand storage (see file header).
-// out_fp32: D is fp32 (else bf16).  tile_n: 0 = auto, 128 / 192 / 256 (1-CTA tiles), 2 = 256x256 CTA-pair tile, 3 = 256x128 CTA-pair tile.  max_ctas: 0 = all SMs
+// out_fp32: D is fp32 (else bf16).  tile_n: 0 = auto, 64 / 128 / 192 / 256 (1-CTA tiles), 2 = 256x256 CTA-pair tile, 3 = 256x128 CTA-pair tile.  max_ctas: 0 = all SMs
 // (a smaller value leaves SMs free for a concurrent communication kernel).
 static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, int K,
                           long long lda, long long ldb, long long ldc, int a_mn, int b_mn,
@@ -657,14 +666,17 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
                  (reinterpret_cast<uintptr_t>(C) & 15) == 0);
   LLMCTL_REQUIRE(out_fp32 ? (ldc % 4 == 0) : (ldc % 8 == 0));
   cudaStream_t s = (cudaStream_t)stream;
-  // auto: the CTA-pair kernel wins whenever the problem has at least one full pair tile in each dimension
-  // (measured on B200: 1.44-1.61 PFLOP/s vs 1.24-1.45 for the single-CTA 128x256 tile on the GPT-7B shapes)
-  // auto: the 256 x 256 CTA-pair tile wins whenever the problem has at least one full pair tile in each dimension
-  // (measured on B200: 1.44-1.61 PFLOP/s vs 1.24-1.45 for the single-CTA 128x256 tile on the GPT-7B shapes).  The
-  // narrower tiles (192, pair 256 x 128) were added for the 1-3 wave problems of a TP=8 shard and measured SLOWER
-  // there too (4096 x 1536 x 4096: 55 us pair-256, 53 us 192, 85 us pair-128, cuBLAS 42 us): the main loop costs about
-  // the same per 64-deep k-block whatever the tile width (operand traffic from L2, not the tensor pipe, sets the pace),
-  // so less work per tile only lowers the rate.  They stay selectable (tile_n = 192 / 3), never chosen automatically.
+  // auto.  A problem of at most one wave of tiles is bound by what one CTA does (fill, K loop at the latency of L2, epilogue), not
+  // by the chip: the narrowest tile that still fits one wave wins (M x N x K, us, pair 256 x 256 / 128 x 128 / 128 x 64:
+  // 777 x 2304 x 768: 9.2 / 6.8 / 9.0, 777 x 768 x 2048: 14.6 / 10.6 / 10.1, 512 x 2048 x 5632: 30.7 / 23.4 / 21.4).
+  // Beyond one wave operand traffic from L2 sets the pace and the 256 x 256 CTA-pair tile moves least of it (4096 x 2048 x 2048:
+  // 26.7 / 33.1 / 49.0, 4096 x 11264 x 2048: 130 / 181 / 276); 128 x 192 and pair 256 x 128 never win by more than a few per cent
+  // and stay selectable (tile_n = 192 / 3).  Gated operands arrive slab by slab and keep the pair tile.
+  if (tile_n == 0 && g.flags == nullptr && g.b_flags == nullptr && max_ctas == 0) {
+    const long long rows = (M + 127) / 128, sms = num_sms();
+    if (rows * ((N + 63) / 64) <= sms) tile_n = 64;
+    else if (rows * ((N + 127) / 128) <= sms) tile_n = 128;
+  }
   if (tile_n == 0 && M > 128 && N > 128) tile_n = 2;
   if (tile_n == 2) {   // 2-CTA pair tile 256 x 256 (cta_group::2)
     if (out_fp32) return dispatch_layout2<256, float>(a_mn, b_mn, A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
@@ -675,13 +687,17 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
     return dispatch_layout2<128, __nv_bfloat16>(a_mn, b_mn, A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
   }
   int bn = tile_n;
-  if (bn != 128 && bn != 192 && bn != 256) {
+  if (bn != 64 && bn != 128 && bn != 192 && bn != 256) {
     const int sms = num_sms();
     const long long t256 = static_cast<long long>((M + 127) / 128) * ((N + 255) / 256);
     const long long t128 = static_cast<long long>((M + 127) / 128) * ((N + 127) / 128);
     const double c256 = static_cast<double>((t256 + sms - 1) / sms) * 2.0;
     const double c128 = static_cast<double>((t128 + sms - 1) / sms) * 1.45;  // measured: a 128-wide tile runs at ~0.7x the rate
     bn = (c128 < c256) ? 128 : 256;
+  }
+  if (bn == 64) {
+    if (out_fp32) return dispatch_layout<64, float>(a_mn, b_mn, A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
+    return dispatch_layout<64, __nv_bfloat16>(a_mn, b_mn, A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
   }
   if (bn == 192) {
     if (out_fp32) return dispatch_layout<192, float>(a_mn, b_mn, A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);

@@ -221,6 +221,29 @@ def test_linear_autograd(cuda_device):
     _close(w.grad, wf.grad, 0.5, 2e-2, "dw")
 
 
+# One wave of 128 x 64 tiles, of 128 x 128 tiles, and beyond (CTA pairs): both sides of each line of the automatic tile choice on
+# 148 SMs, with ragged rows, columns and K, every operand layout and output type.
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (130, 72, 200), (37 * 128, 256, 64), (37 * 128 + 1, 256, 64), (74 * 128 - 3, 256, 72),
+                                   (74 * 128 + 8, 256, 72), (776, 2304, 136)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, False), (False, True), (True, True)])
+def test_gemm_automatic_tiles(cuda_device, M, N, K, a_mn, b_mn):
+    """Against float64; fp32 accumulation of bf16 products: sqrt(K) 2^-24 and the rounding of the output (2^-9 bf16)."""
+    from llmctl_b200.ops import functional as ops
+    if a_mn and M % 8:
+        M = M + 8 - M % 8          # the row pitch of a [K, M] operand is whole 16-byte units
+    torch.manual_seed(M + N)
+    a = torch.randn(K, M, device=cuda_device).bfloat16() if a_mn else torch.randn(M, K, device=cuda_device).bfloat16()
+    b = torch.randn(K, N, device=cuda_device).bfloat16() if b_mn else torch.randn(N, K, device=cuda_device).bfloat16()
+    want = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    for dtype, bound in ((torch.bfloat16, 2.0 ** -9), (torch.float32, 2.0 ** -20)):
+        pool = torch.full((M + 3, N), 7.0, device=cuda_device, dtype=dtype)
+        out = ops.gemm_raw(a, b, a_mn=a_mn, b_mn=b_mn, out=pool[:M])
+        assert (out.double() - want).norm() <= bound * want.norm()
+        assert bool((pool[M:] == 7).all())
+        ops.gemm_raw(a, b, a_mn=a_mn, b_mn=b_mn, out=out, accumulate=True)
+        assert (out.double() - 2 * want).norm() <= 2 * bound * (2 * want).norm()
+
+
 @pytest.mark.parametrize("B,S,H", [(2, 512, 4), (1, 2048, 2), (3, 128, 1), (1, 1024, 8)])
 @pytest.mark.parametrize("packed", [True, False])
 def test_flash_attention_fwd(cuda_device, B, S, H, packed):
