@@ -1,5 +1,7 @@
 // K6 (forward): causal flash attention on the 5th-generation tensor cores, bf16: head sizes 64 and 128, sequences of any
-// length.
+// length; and queries / keys of 192 (128 of each head's own + 64 of the key that all heads share) over values of 128, for batches
+// of sequences of unlike lengths whose queries may begin behind earlier keys (prompts of latent attention with rebuilt keys and
+// values, llmctl_latent_prompt_attention).
 //
 // Reference: HF modules choose SDPA/eager attention behind `self.model(**batch)` (reference
 // llmctl/runtime/engine.py:284); the reference's tuner times a naive softmax(QK^T)V (reference
@@ -37,19 +39,19 @@ constexpr int kRows = 128;               // queries per tile, keys per tile
 constexpr int kPanel = kRows * 128;      // bytes of one [128 rows x 64 bf16] swizzled panel
 constexpr int kThreads = 384;
 constexpr float kRescaleThreshold = 8.f;
-// Stages of the K and V rings: what 227 KB hold beside the two query tiles (160 KB at D = 64, 192 KB at 128).
+// Stages of the K and V rings: what 227 KB hold beside the two query tiles (160 KB at D = 64, 192 KB at 128, 224 KB at 192 / 128).
 template <int DQK, int DV>
 struct Cfg {
   static constexpr int kQTile = DQK / 64 * kPanel, kVTile = DV / 64 * kPanel;
   static constexpr int kKStages = DQK == 64 ? 4 : 2;
-  static constexpr int kVStages = DQK == 64 ? 4 : 2;
+  static constexpr int kVStages = DQK == 64 ? 4 : DQK == 128 ? 2 : 1;
   static constexpr int kKAt = 2 * kQTile, kVAt = kKAt + kKStages * kQTile;
   static constexpr int kSmem = kVAt + kVStages * kVTile + 1024;
 };
 __device__ unsigned int g_status = 0;    // != 0: a bounded wait of the kernel ran out
 
-// One sequence of the batch: its queries are rows [q_row, q_row + n) at positions start + i, its keys (position 0 first) begin
-// at row k_row.
+// One sequence of a batch of unlike lengths: its queries are rows [q_row, q_row + n) of Q and O at positions start + i, its keys
+// (position 0 first) begin at row k_row of K and V.  Rows from its last key to the next multiple of 128 hold zeros.
 struct Seq {
   int q_row, n, start, k_row;
 };
@@ -158,10 +160,11 @@ __device__ __forceinline__ void softmax_block(uint32_t tS, uint32_t tO, int q, i
 template <int DQK, int DV>
 __global__ void __launch_bounds__(ffwd::kThreads, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                 const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ O, long long o_tok_stride, int o_wide,
-                 float* __restrict__ lse, int B, int max_q, int H, float scale_log2, int causal, long long* __restrict__ trace) {
+                 const __grid_constant__ CUtensorMap tmKs, const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ O,
+                 long long o_tok_stride, int o_wide, float* __restrict__ lse, const ffwd::Seq* __restrict__ seqs, int B, int max_q, int H, float scale_log2, int causal, long long* __restrict__ trace) {
   using namespace ffwd;
   using C = Cfg<DQK, DV>;
+  constexpr int kOwn = DQK > 128 ? 2 : DQK / 64;         // panels of K that belong to the head; the last of three is shared by all
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_q[2], bar_qfree[2], bar_kfull[C::kKStages], bar_vfull[C::kVStages], bar_kempty[C::kKStages], bar_vempty[C::kVStages];
   __shared__ uint64_t bar_s[2], bar_p0[2], bar_p1[2], bar_o[2], bar_ofree[2];
@@ -199,6 +202,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 8 && lane == 0) {
     prefetch_tmap(&tmQ);
     prefetch_tmap(&tmK);
+    if (kOwn < DQK / 64) prefetch_tmap(&tmKs);
     prefetch_tmap(&tmV);
   }
   if (warp == 9) tmem_alloc<1>(&tmem_base_smem, 512);
@@ -227,13 +231,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     item = r * gridDim.x + ((r & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
     return item < n_items;
   };
-  // item -> (first query, head, batch, sequence); heavy (late) query blocks first so the tail is made of light items
+  // item -> (first query, head, batch, sequence); heavy (late) query blocks first so the tail is made of light items.
+  // False: a shorter sequence of the batch has no such block.
   auto decode = [&](int item, int& q0, int& head, int& b, Seq& sq) {
     q0 = (nqb - 1 - item / per_qb) * 2 * kRows;
     const int rem = item % per_qb;
     head = rem % H;
     b = rem / H;
-    sq = Seq{0, max_q, 0, 0};
+    if (seqs != nullptr)
+      sq = seqs[b];
+    else
+      sq = Seq{0, max_q, 0, 0};
     return q0 < sq.n;
   };
   // key blocks of tile t of an item; a tile past the end of its sequence has none
@@ -260,6 +268,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         Seq sq;
         if (!decode(item, q0, head, b, sq)) continue;
         const int nblk = max(blocks(sq, q0, 0), blocks(sq, q0, 1));
+        const int bc = seqs != nullptr ? 0 : b;          // batch coordinate of the maps
         const bool validB = q0 + kRows < sq.n;
         ev(3, 40);
         auto load_q = [&](int t, uint32_t done) {
@@ -267,7 +276,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           mbar_expect_tx(&bar_q[t], C::kQTile);
 #pragma unroll
           for (int p = 0; p < DQK / 64; ++p)
-            tma_load_4d(smem + t * C::kQTile + p * kPanel, &tmQ, &bar_q[t], 64 * p, head, sq.q_row + q0 + t * kRows, b);
+            tma_load_4d(smem + t * C::kQTile + p * kPanel, &tmQ, &bar_q[t], 64 * p, head, sq.q_row + q0 + t * kRows, bc);
           return true;
         };
         if (!(ok = load_q(0, nA))) break;
@@ -281,7 +290,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           mbar_expect_tx(&bar_kfull[ks], C::kQTile);
           ++nk;
 #pragma unroll
-          for (int p = 0; p < DQK / 64; ++p) tma_load_4d(sK + p * kPanel, &tmK, &bar_kfull[ks], 64 * p, head, row, b);
+          for (int p = 0; p < kOwn; ++p) tma_load_4d(sK + p * kPanel, &tmK, &bar_kfull[ks], 64 * p, head, row, bc);
+          if (kOwn < DQK / 64) tma_load_4d(sK + kOwn * kPanel, &tmKs, &bar_kfull[ks], 0, 0, row, bc);
           if (j == 0 && validB) {
             if (!(ok = load_q(1, nB))) break;
             ++nB;
@@ -290,7 +300,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           mbar_expect_tx(&bar_vfull[vs], C::kVTile);
           ++nv;
 #pragma unroll
-          for (int p = 0; p < DV / 64; ++p) tma_load_4d(sV + p * kPanel, &tmV, &bar_vfull[vs], 64 * p, head, row, b);
+          for (int p = 0; p < DV / 64; ++p) tma_load_4d(sV + p * kPanel, &tmV, &bar_vfull[vs], 64 * p, head, row, bc);
         }
       }
       // Copies still in flight when a wait ran out land before the CTA's shared memory is given back.
@@ -425,7 +435,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const float l = l0 + l1;
       const float inv_l = 1.f / l;
       const bool real = qt0 + row < sq.n;
-      const long long tok = static_cast<long long>(b) * max_q + qt0 + row;
+      const long long tok = seqs != nullptr ? sq.q_row + qt0 + row : static_cast<long long>(b) * max_q + qt0 + row;
       __nv_bfloat16* orow = O + tok * o_tok_stride + head * DV;
 #pragma unroll
       for (int c = 0; c < DV / 32; ++c) {
@@ -484,8 +494,8 @@ static long long* flash_trace_buffer() {
 
 // Persistent launch: one CTA per SM over a heavy-first item list.
 template <int DQK, int DV>
-static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, void* o, long long o_tok_stride, float* lse,
-                            int B, int max_q, int H, float scale, int causal, cudaStream_t s) {
+static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& ks, const CUtensorMap& v, void* o,
+                            long long o_tok_stride, float* lse, const ffwd::Seq* seqs, int B, int max_q, int H, float scale, int causal, cudaStream_t s) {
   using namespace ffwd;
   using C = Cfg<DQK, DV>;
   const cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<DQK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
@@ -494,7 +504,7 @@ static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CU
   if (n_items >= (1ll << 31) - 2 * kNumSMs) return static_cast<int>(cudaErrorInvalidValue);
   const int grid = n_items < kNumSMs ? static_cast<int>(n_items) : kNumSMs;
   const int wide = o_tok_stride % 16 == 0 && (reinterpret_cast<uintptr_t>(o) & 31) == 0;
-  flash_fwd_kernel<DQK, DV><<<grid, kThreads, C::kSmem, s>>>(q, k, v, (__nv_bfloat16*)o, o_tok_stride, wide, lse, B, max_q, H,
+  flash_fwd_kernel<DQK, DV><<<grid, kThreads, C::kSmem, s>>>(q, k, ks, v, (__nv_bfloat16*)o, o_tok_stride, wide, lse, seqs, B, max_q, H,
                                                              scale * 1.4426950408889634f, causal, flash_trace_buffer());
   return static_cast<int>(cudaGetLastError());
 }
@@ -541,8 +551,30 @@ LLMCTL_API int llmctl_flash_attn_fwd(const void* q, const void* k, const void* v
   mkmap(&tk, k, k_tok_stride);
   mkmap(&tv, v, v_tok_stride);
   if (rc) LLMCTL_FAIL(rc, "tensor map Q / K / V");
-  rc = (D == 128 ? flash_fwd_launch<128, 128> : flash_fwd_launch<64, 64>)(tq, tk, tv, o, o_tok_stride, lse, B, S, H, scale, causal,
-                                                                          (cudaStream_t)stream);
+  rc = (D == 128 ? flash_fwd_launch<128, 128> : flash_fwd_launch<64, 64>)(tq, tk, tk, tv, o, o_tok_stride, lse, nullptr, B, S, H, scale,
+                                                                          causal, (cudaStream_t)stream);
   if (rc) LLMCTL_FAIL(rc, "flash forward");
+  return 0;
+}
+
+// Causal attention of latent-attention prompts whose per-head keys and values have been rebuilt from the cache: q: [tokens, H * 192]
+// (row stride ldq; the last 64 of a head already rotated), kn: [key_rows, H * 128], kr: [key_rows, 64] shared by all heads, v:
+// [key_rows, H * 128], out: [tokens, H * 128].  seqs: int32 [B, 4] on the device = (first query row, queries, position of the first
+// query, first key row; key rows in whole blocks of 128, zeros past the last key); max_q: the most queries of a sequence.
+LLMCTL_API int llmctl_latent_prompt_attention(const void* q, long long ldq, long long tokens, const void* kn, const void* kr, const void* v,
+                                              long long key_rows, const int* seqs, int B, int max_q, int H, void* out, float scale,
+                                              void* stream) {
+  LLMCTL_BEGIN();
+  LLMCTL_REQUIRE(B > 0 && max_q > 0 && H > 0 && tokens > 0 && key_rows > 0 && key_rows % 128 == 0 && ldq % 8 == 0 && scale > 0.f && seqs != nullptr);
+  CUtensorMap tq, tk, tks, tv;
+  int rc = get_tmap_4d_bf16(&tq, q, 192, H, tokens, 1, 192, ldq, ldq * tokens, 64, 1, ffwd::kRows, 1, 1);
+  const uint64_t ld = static_cast<uint64_t>(H) * 128;
+  if (!rc) rc = get_tmap_4d_bf16(&tk, kn, 128, H, key_rows, 1, 128, ld, ld * key_rows, 64, 1, ffwd::kRows, 1, 1);
+  if (!rc) rc = get_tmap_4d_bf16(&tks, kr, 64, 1, key_rows, 1, 64, 64, 64ull * key_rows, 64, 1, ffwd::kRows, 1, 1);
+  if (!rc) rc = get_tmap_4d_bf16(&tv, v, 128, H, key_rows, 1, 128, ld, ld * key_rows, 64, 1, ffwd::kRows, 1, 1);
+  if (rc) LLMCTL_FAIL(rc, "tensor map q / k / v");
+  rc = flash_fwd_launch<192, 128>(tq, tk, tks, tv, out, static_cast<long long>(ld), nullptr, reinterpret_cast<const ffwd::Seq*>(seqs), B, max_q,
+                                  H, scale, 1, (cudaStream_t)stream);
+  if (rc) LLMCTL_FAIL(rc, "latent prompt attention");
   return 0;
 }

@@ -12,6 +12,9 @@ single rotated key part shared by all heads.  Queries go through their own norme
     ol       = attention over the cache rows (ops.latent_attention.latent_attention)   [T, H, R]
     out      = (ol Uv_h^T) Wo^T
 
+Batches with prompt portions rebuild every head's keys and values from the cached latents instead where that is cheaper
+(ops.latent_attention.rebuild_pays, latent_prompt_attention): k = [Uk_h c | kr], v = Uv_h c, ordinary causal attention.
+
 Optional parts of ``LatentAttention`` (fields of its spec): ``sink`` — a learned number per head whose exponential joins
 the softmax denominator (a key without a value, not scaled); ``out_gate`` — the concatenated heads are multiplied element
 by element with the sigmoid of one more projection of the mixer's input (packed into the down-projection GEMM);
@@ -191,6 +194,12 @@ class LatentAttention(nn.Module):
                                   cache if own else None, batch.slots, batch.positions, self.rot_freq, self.rot_mult, self.eps)
         nq = s.heads * (s.dim + s.rot_dim)
         q = ops.linear(cq, self.w_uq) if s.q_rank else d[:, self.q_at:self.q_at + nq]   # [T, H * (dn + dr)]
+        if (not (batch.decode_only or s.sink or s.head_gate or s.window)
+                and lops.rebuild_pays(q, s.dim, s.rot_dim, s.vdim, s.kv_rank, s.heads, batch.key_rows, batch.pairs)):
+            with torch.no_grad():
+                o = lops.latent_prompt_attention(q, s.dim, cache, batch.block_tables, batch.seqs, batch.key_rows, batch.max_tokens,
+                                                 batch.positions, self.rot_freq, self.rot_mult, s.scale, self.w_uk, self.w_uv)
+            return self._project(o, d)
         qn = q.unflatten(1, (s.heads, s.dim + s.rot_dim))[:, :, :s.dim].transpose(0, 1) # [H, T, dn], a view
         # absorbed queries ql[t, h] = Uk_h^T qn[t, h]: fp32, except that the tensor-core attention kernel takes them
         # in bf16 (it multiplies in bf16 anyway); the kernel reads the [H, T, R] product through its strides
@@ -217,6 +226,10 @@ class LatentAttention(nn.Module):
         o = torch.empty(T, s.heads * s.vdim, dtype=ol.dtype, device=ol.device)          # the product lands head by head in place
         with torch.no_grad():
             torch.bmm(ol.transpose(0, 1), self.w_uv.transpose(1, 2), out=o.view(T, s.heads, s.vdim).transpose(0, 1))
+        return self._project(o, d)
+
+    def _project(self, o: torch.Tensor, d: torch.Tensor) -> torch.Tensor:
+        s = self.spec
         if s.out_gate:
             o = sigmoid_gate_(o, d[:, self.gate_at:self.gate_at + s.heads * s.vdim])
         return ops.linear(o, self.w_o)

@@ -32,6 +32,14 @@ native.register_signature("llmctl_latent_attention_t5", [c_void_p, c_int, c_ll, 
                                                           c_void_p])
 native._KERNELS_PER_CALL["llmctl_latent_attention_t5"] = 2
 
+native.register_signature("llmctl_latent_prompt_prepare", [c_void_p, c_ll, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p,
+                                                            c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p])
+native.register_signature("llmctl_latent_prompt_attention", [c_void_p, c_ll, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_void_p, c_int, c_int,
+                                                              c_int, c_void_p, c_float, c_void_p])
+
+KEY_ROWS = 128              # rebuilt keys of a sequence fill whole blocks of this many rows (the flash kernel's key tile)
+REBUILD_PAIRS = 32          # visible pairs per rebuilt key row from which rebuilding pays (see rebuild_pays)
+REBUILD_BYTES = 1 << 30     # most scratch a layer's rebuilt keys and values may take
 WINDOW_ALIGN = 32           # a window's first key tile starts at a multiple of this (kWindowAlign of the kernels)
 ROWS_PER_TILE = 16          # query rows (token, head) a CTA owns; tiles are built by the engine with this limit
 ROWS_PER_TILE_WIDE = 32     # the tensor-core kernel also takes tiles of 32 rows (half the key traffic per row)
@@ -72,6 +80,39 @@ def rows_per_tile(dtype: torch.dtype, R: int, dr: int, cuda: bool, rows_wanted: 
 def key_span(max_context: int, window: int, tile_tokens: int) -> int:
     """Most keys a query tile of ``tile_tokens`` tokens reads."""
     return min(max_context, window + tile_tokens - 1 + WINDOW_ALIGN - 1) if window > 0 else max_context
+
+
+def rebuild_pays(q: torch.Tensor, dn: int, dr: int, dv: int, R: int, heads: int, key_rows: int, pairs: int) -> bool:
+    """Whether a batch's attention runs over keys and values rebuilt from the cache (``latent_prompt_attention``) instead of
+    absorbed queries: head sizes that the flash kernel has, scratch within ``REBUILD_BYTES``, and at least ``REBUILD_PAIRS`` visible
+    (query, key) pairs per rebuilt row.  A pair costs a head 1088 products at the absorbed kernel's rate or 320 at four times that
+    rate, a rebuilt row 131072 at five times that rate: the line is near 26 pairs a row, a prompt of about 64 tokens."""
+    return (q.is_cuda and q.dtype == torch.bfloat16 and (dn, dr, dv) == (128, 64, 128) and R % 8 == 0 and q.stride(1) == 1
+            and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and key_rows > 0 and pairs >= REBUILD_PAIRS * key_rows
+            and 2 * key_rows * (heads * (dn + dv) + R + dr) <= REBUILD_BYTES and native.has_symbol("llmctl_latent_prompt_attention"))
+
+
+def latent_prompt_attention(q: torch.Tensor, dn: int, cache: torch.Tensor, block_tables: torch.Tensor, seqs: torch.Tensor, key_rows: int,
+                            max_tokens: int, positions: torch.Tensor, freq: torch.Tensor, mult: float, scale: float, w_uk: torch.Tensor,
+                            w_uv: torch.Tensor) -> torch.Tensor:
+    """q: [T, H * (dn + dr)] raw queries (the rope part of each head is rotated in place); w_uk: [H, dn, R], w_uv: [H, dv, R];
+    ``seqs``, ``key_rows``, ``max_tokens``: RaggedBatch.  Returns [T, H * dv]: causal attention of every portion over its sequence's cached
+    rows, with each head's keys ``[Uk c | kr]`` and values ``Uv c`` rebuilt in q's type."""
+    from .functional import gemm_raw
+    T, H, R = q.shape[0], w_uk.shape[0], w_uk.shape[2]
+    dr, dv = cache.shape[-1] - R, w_uv.shape[1]
+    assert cache.is_contiguous()
+    c = torch.empty(key_rows, R, dtype=q.dtype, device=q.device)
+    kr = torch.empty(key_rows, dr, dtype=q.dtype, device=q.device)
+    st = native.stream_ptr()
+    native.call("llmctl_latent_prompt_prepare", q.data_ptr(), q.stride(0), T, H, dn, dr, positions.data_ptr(), freq.data_ptr(), float(mult),
+                cache.data_ptr(), R, block_tables.data_ptr(), block_tables.shape[1], cache.shape[1], seqs.data_ptr(), seqs.shape[0], key_rows,
+                c.data_ptr(), kr.data_ptr(), st)
+    kn, v = gemm_raw(c, w_uk.reshape(H * dn, R)), gemm_raw(c, w_uv.reshape(H * dv, R))
+    out = torch.empty(T, H * dv, dtype=q.dtype, device=q.device)
+    native.call("llmctl_latent_prompt_attention", q.data_ptr(), q.stride(0), T, kn.data_ptr(), kr.data_ptr(), v.data_ptr(), key_rows,
+                seqs.data_ptr(), seqs.shape[0], max_tokens, H, out.data_ptr(), float(scale), st)
+    return out
 
 
 def latent_kv_write(d: torch.Tensor, Q: int, R: int, dr: int, wq: Optional[torch.Tensor], wkv: Optional[torch.Tensor],

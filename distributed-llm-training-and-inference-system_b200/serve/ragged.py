@@ -13,7 +13,7 @@ from typing import List, Optional, Sequence as Seq, Tuple
 import numpy as np
 import torch
 
-from ..ops.latent_attention import ROWS_PER_TILE, TILE_WIDTHS
+from ..ops.latent_attention import KEY_ROWS, ROWS_PER_TILE, TILE_WIDTHS
 
 
 @dataclass
@@ -56,15 +56,17 @@ class RaggedBatch:
             n_out = sum(len(p.want) for p in portions)
             ntiles = tuple(sum((len(p.tokens) + w - 1) // w for p in portions) for w in self._tile_tokens)
         # int32 words: tokens(2T) | slots(2T) | out_rows(2 n_out) | positions(T) | block tables(B max_blocks) | tiles(4 n) per width
-        # | block-table row of every token(T) | portions(4 B)
+        # | block-table row of every token(T) | portions(4 B) | sequences(4 B, at a 16-byte boundary)
         sizes = [2 * T, 2 * T, 2 * n_out, T, B * max_blocks] + [4 * n for n in ntiles] + [T, 4 * B]
+        sizes[-2] += -sum(sizes) % 4
+        sizes.append(4 * B)
         offs = np.concatenate([[0], np.cumsum(sizes)])
         self._host = torch.zeros(int(offs[-1]), dtype=torch.int32, pin_memory=device.type == "cuda")
         a = self._host.numpy()
         self._h = (a[offs[0]:offs[1]].view(np.int64), a[offs[1]:offs[2]].view(np.int64), a[offs[2]:offs[3]].view(np.int64),
                    a[offs[3]:offs[4]], tuple(a[offs[5 + k]:offs[6 + k]].reshape(n, 4) for k, n in enumerate(ntiles)),
-                   a[offs[4]:offs[5]].reshape(B, max_blocks), a[offs[5 + len(ntiles)]:offs[6 + len(ntiles)]],
-                   a[offs[6 + len(ntiles)]:offs[7 + len(ntiles)]].reshape(B, 4))
+                   a[offs[4]:offs[5]].reshape(B, max_blocks), a[offs[5 + len(ntiles)]:offs[5 + len(ntiles)] + T],
+                   a[offs[6 + len(ntiles)]:offs[7 + len(ntiles)]].reshape(B, 4), a[offs[7 + len(ntiles)]:].reshape(B, 4))
         dev = torch.empty_like(self._host, device=device) if device.type == "cuda" else self._host
         self._dev = dev
         self.nbytes = self._host.numel() * 4
@@ -75,15 +77,19 @@ class RaggedBatch:
         self.positions = dev[offs[3]:offs[4]]
         self._tiles = {w: dev[offs[5 + k]:offs[6 + k]].view(ntiles[k], 4) for k, w in enumerate(TILE_WIDTHS)}
         self.block_tables = dev[offs[4]:offs[5]].view(B, max_blocks)
-        self.seq_rows = dev[offs[5 + len(ntiles)]:offs[6 + len(ntiles)]]       # int32 [T]: row of block_tables per token
+        self.seq_rows = dev[offs[5 + len(ntiles)]:offs[5 + len(ntiles)] + T]   # int32 [T]: row of block_tables per token
         # int32 [B, 4] = (first token row, tokens, position of the first token, state slot) per portion; row b belongs to
         # block_tables[b] and seq_rows == b (recurrent layers walk a portion's tokens from its slot's state)
         self.portions = dev[offs[6 + len(ntiles)]:offs[7 + len(ntiles)]].view(B, 4)
+        # int32 [B, 4] = (first token row, tokens, position of the first token, first key row) for attention over keys rebuilt from
+        # the cache: every sequence's keys take whole blocks of KEY_ROWS rows of ``key_rows`` in all; ``pairs``: visible (query, key) pairs
+        self.seqs = dev[offs[7 + len(ntiles)]:].view(B, 4)
+        self.key_rows = self.pairs = self.max_tokens = 0
         self.refill(portions)
 
     def refill(self, portions: List[Portion]) -> None:
         """Write the description of ``portions`` into the (same) buffers and copy it to the device."""
-        tokens, slots, out_rows, positions, tiles, tables, seq_rows, prows = self._h
+        tokens, slots, out_rows, positions, tiles, tables, seq_rows, prows, srows = self._h
         block_size = self.block_size
         if self.pad_to is not None:
             assert len(portions) <= self.pad_to[0] and all(len(p.tokens) == 1 for p in portions)
@@ -97,7 +103,9 @@ class RaggedBatch:
                     tl[r] = (r, 1, r, 0)
                 out_rows[r] = r
                 prows[r] = (r, 1, 0, -1)                    # a padding row keeps no state
-        t = o = 0
+                srows[r] = 0
+        t = o = self.key_rows = self.pairs = 0
+        self.max_tokens = max((len(p.tokens) for p in portions), default=0)
         ti = [0] * len(tiles)
         for b, p in enumerate(portions):
             n = len(p.tokens)
@@ -111,6 +119,9 @@ class RaggedBatch:
             tables[b, :len(bt)] = bt
             seq_rows[t:t + n] = b
             prows[b] = (t, n, p.start, p.state_slot)
+            srows[b] = (t, n, p.start, self.key_rows)
+            self.key_rows += (p.start + n + KEY_ROWS - 1) // KEY_ROWS * KEY_ROWS
+            self.pairs += n * p.start + n * (n + 1) // 2
             if self.pad_to is None:
                 for w in p.want:
                     assert 0 <= w < n

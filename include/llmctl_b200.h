@@ -240,6 +240,13 @@ int llmctl_latent_attention(const void* ql, int ql_bf16, long long ql_st, long l
                             const float* sinks /* fp32 [H] or null: exp(sinks[h]) joins head h's softmax denominator */,
                             int window /* 0: every earlier key */, const void* head_gate /* [tokens, H] pre-sigmoid or null */,
                             long long gate_ld, void* stream);
+/* Prompts over keys and values rebuilt from the latent cache: rotate the queries and gather the rows (csrc/attention/latent_prompt.cu),
+ * then, after two GEMMs, causal attention of 192-wide queries / keys over 128-wide values (csrc/attention/flash_fwd.cu). */
+int llmctl_latent_prompt_prepare(void* q, long long ldq, int tokens, int H, int dn, int dr, const int* positions, const float* freq,
+                                 float mult, const void* cache, int R, const int* block_tables, int max_blocks, int block_size,
+                                 const int* seqs, int B, int key_rows, void* c_out, void* kr_out, void* stream);
+int llmctl_latent_prompt_attention(const void* q, long long ldq, long long tokens, const void* kn, const void* kr, const void* v,
+                                   long long key_rows, const int* seqs, int B, int max_q, int H, void* out, float scale, void* stream);
 /* The tcgen05 kernel (128-row query tiles): sizes that qualify, status of its bounded waits, and the launch.
  * qfull: bf16 scratch [tokens, H, R + dr], or null when dr is 0 and ql is bf16 [heads, tokens, R]; cache_rows = blocks x block_size. */
 int llmctl_latent_attention_t5_ok(int R, int dr, int block_size);

@@ -149,6 +149,71 @@ def test_latent_attention_tcgen05(cuda_device, H, dn, dr, R, bs):
             close(out, ref, dt, 4)
 
 
+# (tokens, position of the first) of the batch's portions: one prompt around the 128-key and 256-query blocks, portions behind earlier
+# keys at positions that are and are not multiples of 128, unlike lengths side by side, a single token among them
+@pytest.mark.parametrize("portions", [[(64, 0)], [(127, 0)], [(128, 0)], [(129, 0)], [(257, 0)], [(700, 0)], [(300, 128)], [(300, 1)],
+                                      [(130, 255)], [(600, 0), (1, 500), (90, 77), (256, 256)]])
+@pytest.mark.parametrize("H,R,bs,q_rank", [(3, 512, 64, 24), (1, 64, 16, 0), (4, 136, 48, 16)])
+def test_latent_prompt_over_rebuilt_keys(cuda_device, monkeypatch, portions, H, R, bs, q_rank):
+    """The layer over rebuilt keys and values against float64 and against absorbed queries (both round intermediate results to bf16:
+    the rebuilt path its keys, values, P and heads, the absorbed one its queries, P, latents and heads: 4 x 2^-9 each in the 2-norm,
+    amplified by scores of unit size)."""
+    from llmctl_b200.models.mixers import LatentAttention, LatentAttentionSpec
+    from llmctl_b200.ops import latent_attention as L, native
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+    torch.manual_seed(sum(n for n, _ in portions) + H)
+    W, dn, dr, dv = 64, 128, 64, 128
+    spec = LatentAttentionSpec(heads=H, dim=dn, rot_dim=dr, vdim=dv, kv_rank=R, q_rank=q_rank, scale=(dn + dr) ** -0.5, rot_base=10000.0)
+    layer = LatentAttention(W, spec, 1e-5, torch.bfloat16, "cuda")
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.copy_(torch.randn(p.shape) / p.shape[-1] ** 0.5 if p.dim() > 1 else 1 + 0.1 * torch.randn(p.shape))
+    pages = [(n + s + bs - 1) // bs for n, s in portions]
+    perm = torch.randperm(sum(pages)).tolist()
+    tables = [perm[sum(pages[:i]):sum(pages[:i + 1])] for i in range(len(pages))]
+    first = torch.randn(sum(pages), bs, R + dr).bfloat16().cuda()
+    batch = RaggedBatch([Portion(i, [1] * n, s, [n - 1], t) for i, ((n, s), t) in enumerate(zip(portions, tables))], bs, torch.device("cuda"))
+    h = torch.randn(batch.num_tokens, W).bfloat16().cuda()
+    outs = {}
+    for name, pairs in (("rebuilt", 0), ("absorbed", 1 << 40)):
+        monkeypatch.setattr(L, "REBUILD_PAIRS", pairs)
+        cache, calls = first.clone(), []
+        real = native.call
+        monkeypatch.setattr(native, "call", lambda fn, *a: (calls.append(fn), real(fn, *a))[1])
+        with torch.no_grad():
+            outs[name] = (layer(h, batch, cache), cache)
+        monkeypatch.setattr(native, "call", real)
+        assert ("llmctl_latent_prompt_attention" in calls) == (name == "rebuilt" and not batch.decode_only)
+    assert native.lib().llmctl_flash_fwd_status(1) == 0
+    assert torch.equal(outs["rebuilt"][1], outs["absorbed"][1])
+    # float64 from the rounded cache rows and the projections as the layer rounds them
+    f = lambda t: t.double()
+    d = (h @ layer.w_down.t())
+    if q_rank:
+        cq = f(d[:, :q_rank])
+        q = f((cq * torch.rsqrt(cq.pow(2).mean(-1, keepdim=True) + 1e-5) * f(layer.q_norm)).bfloat16() @ layer.w_uq.t())
+    else:
+        q = f(d[:, layer.q_at:layer.q_at + H * (dn + dr)])
+    q = q.view(-1, H, dn + dr)
+    rows = f(outs["rebuilt"][1]).view(-1, R + dr)
+    want, t = torch.empty(batch.num_tokens, H, dv, dtype=torch.float64, device="cuda"), 0
+    for (n, s), table in zip(portions, tables):
+        j = torch.arange(s + n)
+        kv = rows[torch.tensor(table)[j // bs] * bs + j % bs]
+        ang = torch.outer(torch.arange(s, s + n, device="cuda", dtype=torch.float64), f(layer.rot_freq))
+        c, sn = ang.cos()[:, None], ang.sin()[:, None]
+        u, v = q[t:t + n, :, dn::2], q[t:t + n, :, dn + 1::2]
+        qr = torch.stack([u * c - v * sn, v * c + u * sn], -1).flatten(-2)
+        dark = torch.arange(s + n, device="cuda")[None] > torch.arange(s, s + n, device="cuda")[:, None]
+        for e in range(H):
+            sc = (q[t:t + n, e, :dn] @ f(layer.w_uk[e]) @ kv[:, :R].t() + qr[:, e] @ kv[:, R:].t()) * spec.scale
+            want[t:t + n, e] = torch.softmax(sc.masked_fill(dark, float("-inf")), -1) @ kv[:, :R] @ f(layer.w_uv[e]).t()
+        t += n
+    want = want.reshape(-1, H * dv) @ f(layer.w_o).t()
+    off = {k: ((f(o[0]) - want).norm() / want.norm()).item() for k, o in outs.items()}
+    assert off["rebuilt"] <= 1.5e-2 and off["rebuilt"] <= 1.5 * off["absorbed"] + 1e-3, off
+
+
 @pytest.mark.parametrize("kind", ["fp32", "bf16_rows16", "bf16_rows32", "bf16_tcgen05"])
 def test_far_key_decides_on_every_kernel(cuda_device, kind):
     """One key far back carries a score that stands out (its query and key coordinates are scaled up) and a value unlike
