@@ -55,7 +55,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __shared__ int s_last;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // stream-K: the (tile, k block) space is flattened and cut into equal ranges, one per CTA
   const long long total = static_cast<long long>(n_tiles) * num_kb;
   const long long begin = static_cast<long long>(blockIdx.x) * L;
@@ -105,37 +105,38 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(kBM, MB, 0u, 0u);
-      int stage = 0;
-      uint32_t phase = 0;
-      int seg = 0;
-      for (long long pos = begin; pos < end; ++seg) {
-        const int kb_s = static_cast<int>(pos % num_kb);
-        const long long left = end - pos;
-        const int seg_len = (num_kb - kb_s < left) ? num_kb - kb_s : static_cast<int>(left);
-        const int buf = seg & 1;
-        mbar_wait(&bar_acc_empty[buf], ((seg >> 1) & 1u) ^ 1u);
+    // the whole warp walks the loop, one elected lane issues (descriptors stay in uniform registers, see gemm_tcgen05.cu)
+    constexpr uint32_t idesc = make_idesc_bf16(kBM, MB, 0u, 0u);
+    int stage = 0;
+    uint32_t phase = 0;
+    int seg = 0;
+    for (long long pos = begin; pos < end; ++seg) {
+      const int kb_s = static_cast<int>(pos % num_kb);
+      const long long left = end - pos;
+      const int seg_len = (num_kb - kb_s < left) ? num_kb - kb_s : static_cast<int>(left);
+      const int buf = seg & 1;
+      mbar_wait(&bar_acc_empty[buf], ((seg >> 1) & 1u) ^ 1u);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + buf * 32;
+      for (int i = 0; i < seg_len; ++i) {
+        mbar_wait(&bar_full[stage], phase);
+        __syncwarp();
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * 32;
-        for (int i = 0; i < seg_len; ++i) {
-          mbar_wait(&bar_full[stage], phase);
-          tc_fence_after();
-          const uint32_t w_addr = smem_base + stage * C_::kStageBytes;
-          const uint32_t x_addr = w_addr + kWBytes;
+        const uint32_t w_addr = smem_base + stage * C_::kStageBytes;
+        const uint64_t dw = make_smem_desc(w_addr, 16, 1024, 2), dx = make_smem_desc(w_addr + kWBytes, 16, 1024, 2);
+        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            umma_ss<1>(d_tmem, make_smem_desc(w_addr + k * 32, 16, 1024, 2), make_smem_desc(x_addr + k * 32, 16, 1024, 2),
-                       idesc, (i | k) != 0 ? 1u : 0u);
+          for (int k = 0; k < kBK / 16; ++k) umma_ss<1>(d_tmem, dw + k * 2, dx + k * 2, idesc, (i | k) != 0 ? 1u : 0u);
           umma_commit<1>(&bar_empty[stage]);
-          if (++stage == C_::kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          if (i + 1 == seg_len) umma_commit<1>(&bar_acc_full[buf]);
         }
-        umma_commit<1>(&bar_acc_full[buf]);
-        pos += seg_len;
+        if (++stage == C_::kStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      pos += seg_len;
     }
   } else {
     // ------------------------------ epilogue (4 warps, thread = weight row) ------------------------------
@@ -190,10 +191,27 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           __threadfence();
           if (n < N) {
 #pragma unroll 1
-            for (int m = 0; m < Mb; ++m) {
-              float sum = 0.f;
-              for (int sp = 0; sp < count; ++sp) sum += __ldcg(wt + (static_cast<size_t>(sp) * MB + m) * kBM + row);
-              C[m * ldc + n] = __float2bfloat16(sum);
+            for (int m0 = 0; m0 < Mb; m0 += 8) {
+              // 8 rows x 4 pieces asked for together: one at a time, the L2 round trips of 32 rows x 4 pieces took 20 us
+              float sum[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) sum[j] = 0.f;
+#pragma unroll 1
+              for (int sp = 0; sp < count; sp += 4) {
+                float v[4][8];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                  for (int j = 0; j < 8; ++j)
+                    v[u][j] = (sp + u < count && m0 + j < Mb) ? __ldcg(wt + (static_cast<size_t>(sp + u) * MB + m0 + j) * kBM + row) : 0.f;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) sum[j] += v[u][j];
+              }
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (m0 + j < Mb) C[(m0 + j) * ldc + n] = __float2bfloat16(sum[j]);
             }
           }
           if (threadIdx.x == 64) counters[tile] = 0u;     // ready for the next call on this stream
@@ -253,11 +271,11 @@ LLMCTL_API int llmctl_gemm_skinny_bf16(const void* X, const void* W, void* C, in
   if (rc) LLMCTL_FAIL(rc, "tensor map X");
   cudaStream_t s = (cudaStream_t)stream;
   if (MB == 16) {
-    LLMCTL_CHECK(cudaFuncSetAttribute(gemm_skinny_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, skinny::Cfg<16>::kSmem));
+    LLMCTL_CHECK(allow_smem(gemm_skinny_kernel<16>, skinny::Cfg<16>::kSmem));
     gemm_skinny_kernel<16><<<grid, skinny::kThreads, skinny::Cfg<16>::kSmem, s>>>(
         tw, tx, (__nv_bfloat16*)C, ldc, Mb, N, num_kb, n_tiles, static_cast<int>(L), max_slots, workspace, counters);
   } else {
-    LLMCTL_CHECK(cudaFuncSetAttribute(gemm_skinny_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, skinny::Cfg<32>::kSmem));
+    LLMCTL_CHECK(allow_smem(gemm_skinny_kernel<32>, skinny::Cfg<32>::kSmem));
     gemm_skinny_kernel<32><<<grid, skinny::kThreads, skinny::Cfg<32>::kSmem, s>>>(
         tw, tx, (__nv_bfloat16*)C, ldc, Mb, N, num_kb, n_tiles, static_cast<int>(L), max_slots, workspace, counters);
   }

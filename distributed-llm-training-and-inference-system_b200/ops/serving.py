@@ -14,6 +14,7 @@ native.register_signature("llmctl_kv_append", [c_void_p, c_ll, c_int, c_int, c_v
 native.register_signature("llmctl_paged_attn_decode",
                           [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_ll, c_void_p,
                            c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p])
+native.register_signature("llmctl_paged_attn_scratch_elems", [c_int, c_int, c_int, c_int])
 native.register_signature("llmctl_sample", [c_void_p, c_int, c_ll, c_int, c_int] + [c_void_p] * 6 + [c_void_p])
 
 
@@ -36,7 +37,9 @@ def choose_splits(batch: int, heads: int, max_context: int, block_size: int, sms
     # Decode attention is a latency-bound stream: each CTA walks block table -> K/V rows -> online softmax in a
     # dependent chain, so HBM only fills up with ~8 resident CTAs per SM.  Splits are whole KV blocks of >= 64 tokens;
     # the merge pass costs (head_dim + 2) floats per split, ~3 % of the K/V bytes at 64 tokens per split.
-    want = max(1, (8 * sms + batch * heads - 1) // (batch * heads))
+    # Up to 8 splits a CTA walks at most 512 tokens: with longer walks a full batch of unlike contexts is one and a half waves
+    # of CTAs that end at different times.
+    want = max(1, (8 * sms + batch * heads - 1) // (batch * heads), min(8, (max_context + 511) // 512))
     per_split = max(block_size, (64 // block_size) * block_size) if block_size <= 64 else block_size
     return int(max(1, min(want, max(1, max_context // per_split), 256)))
 
@@ -51,14 +54,16 @@ def paged_attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     if q.is_cuda:
         ns = num_splits or choose_splits(B, H, max_context, block_size)
-        need = B * H * ns * (D + 2)
-        if scratch is None or scratch.numel() < need:
+        need = native.lib().llmctl_paged_attn_scratch_elems(B, H, D, ns)
+        if need and (scratch is None or scratch.numel() < need):
             scratch = torch.empty(need, dtype=torch.float32, device=q.device)
         out = torch.empty(B, H, D, dtype=q.dtype, device=q.device)
         native.call("llmctl_paged_attn_decode", q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
                     block_tables.data_ptr(), block_tables.shape[1], context_lens.data_ptr(), out.data_ptr(),
-                    out.stride(0), scratch.data_ptr(), B, H, D, block_size, int(max_context), ns, float(scale),
+                    out.stride(0), native.ptr(scratch), B, H, D, block_size, int(max_context), ns, float(scale),
                     native.stream_ptr())
+        if need:
+            native.launch_count += 1        # the merge kernel
         return out
     out = torch.zeros(B, H, D, dtype=q.dtype)
     for b in range(B):

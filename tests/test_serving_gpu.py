@@ -27,6 +27,29 @@ def test_paged_decode_attention(cuda_device, B, H, D, ctx, bs, splits):
     assert err < 2e-2, f"max err {err}"
 
 
+# Splits merged in a cluster (up to 8) and through scratch (9), contexts of 0 (a padding row: zeros), 1, less than a split and whole
+@pytest.mark.parametrize("splits", [1, 2, 7, 8, 9])
+@pytest.mark.parametrize("H,D,bs", [(3, 128, 16), (12, 64, 8)])
+def test_paged_decode_attention_splits(cuda_device, H, D, bs, splits):
+    """Against float64 of the same bf16 inputs: fp32 arithmetic, one rounding of the output (2^-9 of a value of order one)."""
+    from llmctl_b200.ops import serving as sops
+    torch.manual_seed(splits)
+    lens = [700, 0, 1, 65, 333]
+    nblk = (max(lens) + bs - 1) // bs
+    kc, vc = (torch.randn(len(lens) * nblk, bs, H, D, device=cuda_device).bfloat16() for _ in range(2))
+    bt = torch.randperm(len(lens) * nblk).view(len(lens), nblk).to(torch.int32).to(cuda_device)
+    q = torch.randn(len(lens), H, D, device=cuda_device).bfloat16()
+    out = sops.paged_attention_decode(q, kc, vc, bt, torch.tensor(lens, dtype=torch.int32, device=cuda_device), 704, num_splits=splits)
+    for b, n in enumerate(lens):
+        if n == 0:
+            assert not out[b].any()
+            continue
+        k, v = (t[bt[b].long()].reshape(-1, H, D)[:n].double() for t in (kc, vc))
+        p = torch.softmax(torch.einsum("hd,nhd->hn", q[b].double(), k) / math.sqrt(D), -1)
+        want = torch.einsum("hn,nhd->hd", p, v)
+        assert (out[b].double() - want).norm() <= 2.0 ** -8.5 * want.norm()
+
+
 def test_kv_append(cuda_device):
     from llmctl_b200.ops import serving as sops
     T, H, D, bs, nb = 37, 4, 128, 16, 10
