@@ -537,8 +537,8 @@ static int flash_bwd_launch(const void* q, const void* k, const void* v, const v
   mkmap(&mv, v, v_tok);
   mkmap(&mdo, d_o, o_tok);
   if (rc) return rc;
-  cudaError_t e = cudaFuncSetAttribute(flash_bwd_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(flash_bwd_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+  cudaError_t e = allow_smem(flash_bwd_kernel<D, false>, C::kSmem);
+  if (e == cudaSuccess) e = allow_smem(flash_bwd_kernel<D, true>, C::kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const float sl2 = scale * 1.4426950408889634f;
   const int n_items = nblk * B * H, grid = n_items < kNumSMs ? n_items : kNumSMs;

@@ -498,7 +498,7 @@ static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CU
                             long long o_tok_stride, float* lse, const ffwd::Seq* seqs, int B, int max_q, int H, float scale, int causal, cudaStream_t s) {
   using namespace ffwd;
   using C = Cfg<DQK, DV>;
-  const cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<DQK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+  const cudaError_t e = allow_smem(flash_fwd_kernel<DQK, DV>, C::kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const long long n_items = static_cast<long long>((max_q + 2 * kRows - 1) / (2 * kRows)) * H * B;
   if (n_items >= (1ll << 31) - 2 * kNumSMs) return static_cast<int>(cudaErrorInvalidValue);

@@ -342,7 +342,7 @@ static int launch_latent_attention(const float* ql, long long ql_st, long long q
 #define LAUNCH(NC)                                                                                                   \
   do {                                                                                                               \
     auto kern = latent_attention_kernel<T, NC>;                                                                      \
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
+    cudaError_t e = allow_smem(kern, static_cast<int>(smem)); \
     if (e != cudaSuccess) return static_cast<int>(e);                                                                \
     kern<<<grid, kAttnThreads, smem, s>>>(ql, ql_st, ql_sh, (const T*)q, ldq, dn, (const T*)cache, block_tables, max_blocks, \
                                           block_size, tiles, positions, freq, mult, scale, H, R, dr, heads_per_tile, \
@@ -606,7 +606,7 @@ static int launch_latent_attention_tc(const TQ* ql, long long ql_st, long long q
 #define LAUNCH_TC(NT, MT)                                                                                            \
   do {                                                                                                               \
     auto kern = latent_attention_tc_kernel<NT, MT, TQ>;                                                              \
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
+    cudaError_t e = allow_smem(kern, static_cast<int>(smem)); \
     if (e != cudaSuccess) return static_cast<int>(e);                                                                \
     kern<<<grid, 256 * MT, smem, s>>>(ql, ql_st, ql_sh, (const __nv_bfloat16*)q, ldq, dn, (const __nv_bfloat16*)cache, \
                                       block_tables, max_blocks, block_size, tiles, positions, freq, mult, scale,     \

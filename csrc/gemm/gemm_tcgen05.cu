@@ -585,8 +585,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   if (sizeof(OutT) == 2 && !beta) rc = get_tmap_2d_bf16(&tmC, C, M, N, ldc, 32, 64, 1);
   if (rc) LLMCTL_FAIL(rc, "tensor map C");
   auto kern = gemm_tcgen05_kernel<BN, A_MN, B_MN, OutT>;
-  LLMCTL_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    Cfg::kSmemBytes));
+  LLMCTL_CHECK(allow_smem(kern, Cfg::kSmemBytes));
   const int tiles = ((M + kBM - 1) / kBM) * ((N + BN - 1) / BN);
   int grid = num_sms();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
@@ -628,8 +627,7 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
   if (sizeof(OutT) == 2 && !beta) rc = get_tmap_2d_bf16(&tmC, C, M, N, ldc, 32, 64, 1);
   if (rc) LLMCTL_FAIL(rc, "tensor map C");
   auto kern = gemm2_tcgen05_kernel<PBN, A_MN, B_MN, OutT>;
-  LLMCTL_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    Cfg::kSmemBytes));
+  LLMCTL_CHECK(allow_smem(kern, Cfg::kSmemBytes));
   const int tiles = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + Cfg::kBN - 1) / Cfg::kBN);
   int pairs = num_sms() / 2;
   if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2;

@@ -107,12 +107,12 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
               scale: Optional[float] = None) -> torch.Tensor:
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
     if _native_ok(q, k, v, causal):
-        return _FlashAttnFn.apply(q, k, v, scale, causal)
+        return native.apply(_FlashAttnFn, q, k, v, scale, causal)
     if _native_built(q) and _native_shape(q, k, v, causal) and k.dtype == v.dtype == q.dtype and (q.shape[-1] == 64 or q.shape[1] % 128):
         # other strides or an odd address: head_dim 64 and ragged lengths (gpt-125m, every serving prefill) are always copied for
         # the kernel, whole 128-wide tiles are left to the library
         q, k, v = (t.clone(memory_format=torch.contiguous_format) for t in (q, k, v))
-        return _FlashAttnFn.apply(q, k, v, scale, causal)
+        return native.apply(_FlashAttnFn, q, k, v, scale, causal)
     return _sdpa(q, k, v, causal, scale)
 
 
@@ -242,7 +242,7 @@ def rope_attention_packed(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tenso
         paddable = (not use_native and cfg.attention == "native" and native.has_symbol("llmctl_flash_attn_bwd")
                     and (head_dim == 64 or (head_dim == 128 and seq % 128 != 0)))
         if not paddable:
-            return _RopeAttnPackedFn.apply(qkv, cos, sin, batch, seq, heads, head_dim, pos, scale, use_native)
+            return native.apply(_RopeAttnPackedFn, qkv, cos, sin, batch, seq, heads, head_dim, pos, scale, use_native)
     qkv = ops.rope_packed(qkv, cos, sin, 2 * heads, head_dim, seq, positions)
     v5 = qkv.view(batch, seq, 3, heads, head_dim)
     o = attention(v5[:, :, 0], v5[:, :, 1], v5[:, :, 2], causal=True, scale=scale)

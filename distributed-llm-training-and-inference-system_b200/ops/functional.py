@@ -138,7 +138,7 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5,
     """Returns ``(y, h)`` with ``h = x + residual`` (``h is x`` when no residual) and
     ``y = h * rsqrt(mean(h^2) + eps) * w``."""
     if _use_native(x, "elementwise"):
-        y, h = _RMSNormFn.apply(x, residual, w, eps)
+        y, h = native.apply(_RMSNormFn, x, residual, w, eps)
         return (y, h) if residual is not None else (y, x)
     h = x if residual is None else x + residual
     hf = h.float()
@@ -189,7 +189,7 @@ class _LayerNormFn(torch.autograd.Function):
 
 def layernorm(x, w, b=None, eps: float = 1e-5, residual=None):
     if _use_native(x, "elementwise"):
-        y, h = _LayerNormFn.apply(x, residual, w, b, eps)
+        y, h = native.apply(_LayerNormFn, x, residual, w, b, eps)
         return (y, h) if residual is not None else (y, x)
     h = x if residual is None else x + residual
     y = F.layer_norm(h.float(), (h.shape[-1],), w.float(), None if b is None else b.float(), eps)
@@ -258,7 +258,7 @@ def rope_packed(x: torch.Tensor, cos, sin, n_rot_heads: int, head_dim: int, seq_
     if _use_native(x, "elementwise"):
         if x.is_leaf and x.requires_grad:
             x = x.clone()   # never rotate a trainable leaf in place (other inputs ARE rotated in place)
-        return _RopeFn.apply(x, cos, sin, n_rot_heads, head_dim, seq_len,
+        return native.apply(_RopeFn, x, cos, sin, n_rot_heads, head_dim, seq_len,
                              None if positions is None else positions.to(torch.int32))
     T = x.shape[0]
     rot = x[:, : n_rot_heads * head_dim].reshape(T, n_rot_heads, head_dim)
@@ -297,7 +297,7 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
         g2 = gate_up.reshape(-1, shape[-1])
         if g2.stride(1) != 1 or g2.stride(0) % 8:
             g2 = g2.contiguous()
-        return _SwiGLUFn.apply(g2).view(*shape[:-1], shape[-1] // 2)
+        return native.apply(_SwiGLUFn, g2).view(*shape[:-1], shape[-1] // 2)
     g, u = gate_up.chunk(2, dim=-1)
     return (F.silu(g.float()) * u.float()).to(gate_up.dtype)
 
@@ -432,7 +432,7 @@ def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
                 and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))):
             return gemm_skinny(x2, w).view(*shape[:-1], w.shape[0])
         if _gemm_ok(x2, w) and w.shape[0] % 8 == 0:
-            return _LinearFn.apply(x2, w).view(*shape[:-1], w.shape[0])
+            return native.apply(_LinearFn, x2, w).view(*shape[:-1], w.shape[0])
     gate = getattr(w, "_k8_gate", None)
     if gate is not None:
         w._k8_gate = None

@@ -90,9 +90,19 @@ def register_signature(name: str, argtypes: list) -> None:
             pass
 
 
+_functions: dict = {}       # entry points of the loaded library by name; the library is loaded once and never replaced
+
+
+def _function(name: str):
+    fn = _functions.get(name)
+    if fn is None:
+        fn = _functions[name] = getattr(lib(), name)
+    return fn
+
+
 def has_symbol(name: str) -> bool:
     try:
-        getattr(lib(), name)
+        _function(name)
         return True
     except (AttributeError, RuntimeError):
         return False
@@ -114,20 +124,53 @@ def stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+_forward_ad = torch.autograd.forward_ad
+_interpreter = torch._C._functorch.peek_interpreter_stack
+_tracing_state = torch._C._get_tracing_state
+
+
+class _NoContext:
+    """Stands in for an autograd context where nothing is recorded: keeps what the forward sets on it and saves nothing."""
+
+    def save_for_backward(self, *tensors) -> None:
+        pass
+
+    def mark_non_differentiable(self, *tensors) -> None:
+        pass
+
+    def mark_dirty(self, *tensors) -> None:
+        for t in tensors:
+            if not t.is_inference():
+                torch.autograd.graph.increment_version(t)
+
+
+def apply(fn, *args):
+    """``fn.apply(*args)`` of an autograd function whose forward is one kernel call.  Where no gradient can be recorded the
+    forward is called itself: the autograd machinery costs about 10 us, twice the launch (model_logits of 12 layers makes 98 such
+    calls).  Forward-mode AD, functorch transforms and tracing still go through ``apply``, which refuses or records them."""
+    if torch.is_grad_enabled():
+        for a in args:
+            if isinstance(a, torch.Tensor) and a.requires_grad:
+                return fn.apply(*args)
+    if _forward_ad._current_level >= 0 or _interpreter() is not None or _tracing_state() is not None:
+        return fn.apply(*args)
+    return fn.forward(_NoContext(), *args)
+
+
 class NativeError(RuntimeError):
     pass
 
 
 #: kernels launched per entry point when it is not exactly one
 _KERNELS_PER_CALL = {"llmctl_rmsnorm_bwd": 2, "llmctl_layernorm_bwd": 3, "llmctl_sumsq": 2, "llmctl_rmsnorm_bwd_noalloc": 2,
-                     "llmctl_flash_attn_bwd": 3, "llmctl_rs_sumsq": 2, "llmctl_ag_gemm": 2, "llmctl_paged_attn_decode": 2,
+                     "llmctl_flash_attn_bwd": 3, "llmctl_rs_sumsq": 2, "llmctl_ag_gemm": 2,
                      "llmctl_comm_watchdog_poll": 0, "llmctl_comm_watchdog_set_timeout_ms": 0}
 
 
 def call(name: str, *args) -> None:
     """Invoke a C entry point and raise on a non-zero status."""
     global launch_count
-    fn = getattr(lib(), name)
+    fn = _functions.get(name) or _function(name)
     if _nvtx.KERNEL_RANGES:
         with _nvtx.nvtx_range(name):
             rc = fn(*args)

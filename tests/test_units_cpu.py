@@ -410,3 +410,49 @@ def test_reference_arm_provisions_itself(tmp_path):
                        env=dict(os.environ, LLMCTL_REFERENCE_DST=str(tmp_path / "ref2"), LLMCTL_REFERENCE_SRC=str(tmp_path / "nowhere")))
     # /root/reference is still found (second source); with it hidden the function reports why it cannot install
     assert r.returncode == 0
+
+
+def test_apply_without_gradients_keeps_autograd_rules():
+    """ops.native.apply calls the forward itself only where autograd, forward-mode AD and tracing have nothing to record, and an
+    in-place forward still moves the version counter."""
+    from llmctl_b200.ops import native
+    seen = []
+
+    class Twice(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            seen.append(type(ctx).__name__)
+            ctx.save_for_backward(x)
+            return x * 2
+
+        @staticmethod
+        def backward(ctx, g):
+            return 2 * g
+
+    class AddOne(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            with torch.no_grad():
+                x.data.add_(1)
+            ctx.mark_dirty(x)
+            return x
+
+        @staticmethod
+        def backward(ctx, g):
+            return g
+    x = torch.ones(3, requires_grad=True)
+    y = native.apply(Twice, x)
+    y.sum().backward()
+    assert torch.equal(x.grad, torch.full((3,), 2.0)) and seen[-1] != "_NoContext"
+    with torch.no_grad():
+        assert torch.equal(native.apply(Twice, x), torch.full((3,), 2.0)) and seen[-1] == "_NoContext"
+    assert not native.apply(Twice, torch.ones(3)).requires_grad and seen[-1] == "_NoContext"
+    z = torch.zeros(3)
+    before = z._version
+    assert native.apply(AddOne, z) is z and z._version > before and torch.equal(z, torch.ones(3))
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(torch.ones(3), torch.ones(3))
+        with pytest.raises(Exception):
+            native.apply(Twice, dual)           # no jvp: refused, as Twice.apply refuses it
+    with pytest.raises(Exception):
+        torch.func.vmap(lambda t: native.apply(Twice, t))(torch.ones(2, 3))
