@@ -180,6 +180,13 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
       : "memory");
 }
 
+// 1D bulk copy shared -> global, tracked by bulk groups (tma_store_commit / tma_store_wait_read).
+__device__ __forceinline__ void bulk_store_1d(void* gdst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(reinterpret_cast<uint64_t>(gdst)),
+               "r"(smem_u32(smem_src)), "r"(bytes)
+               : "memory");
+}
+
 // ----------------------------------------------------------------------------------------------
 // cluster
 // ----------------------------------------------------------------------------------------------

@@ -8,6 +8,7 @@
 //
 // The vocab-parallel variant (logits sharded over TP ranks) splits this into "partial max/sumexp",
 // an all-reduce, and "finalize"; both halves are exposed below.
+#include "../common/ptx.cuh"
 #include "../common/util.cuh"
 
 namespace llmctl {
@@ -80,6 +81,165 @@ ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long l
       }
       store8(p + v * 8, pack8(g));
     }
+  }
+}
+
+// Rows of 8 K to 57 K logits: persistent CTAs with a ring of two or three whole rows in shared memory.  Bound by HBM (the row is read and
+// written once): while a row is reduced and differentiated the next is copied in and the one before is copied out by bulk copies,
+// which a CTA that loads, reduces and stores one row after the other cannot do (4096 x 32000: 204 us, two of them
+// per SM; here 118 us = 4.4 TB/s).  Maximum
+// and sum of exponentials come from one pass per thread and one block reduction of (maximum, sum) pairs, and up to 32 K logits the
+// exponentials are kept for the gradient.
+constexpr int kCERingBytes = 220 * 1024;
+__device__ unsigned int g_ce_status = 0;       // != 0: a bounded wait ran out
+
+template <int kVec>
+__global__ void __launch_bounds__(kCEThreads, 1)
+ce_rows_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long* __restrict__ targets, float* __restrict__ loss_out,
+               float* __restrict__ lse_out, int rows, int V, int stages, long long ignore_index, float host_scale,
+               const float* __restrict__ scale_dev, int write_grad) {
+  using namespace ptx;
+  extern __shared__ __align__(128) uint8_t ring[];
+  __shared__ uint64_t full[3];
+  __shared__ float red_m[2][kCEThreads / 32], red_s[2][kCEThreads / 32];
+  __shared__ int abort_flag;
+  constexpr float kLog2e = 1.4426950408889634f;
+  constexpr bool kKeep = kVec <= 8;      // the exponentials fit the registers: the gradient needs no second ones
+  const int nvec = V >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t row_bytes = static_cast<uint32_t>(V) * 2;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 3; ++i) mbar_init(&full[i], 1);
+    abort_flag = 0;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  auto begin_load = [&](int row, int st) {
+    mbar_expect_tx(&full[st], row_bytes);
+    bulk_load_1d(ring + st * row_bytes, logits + static_cast<long long>(row) * ld, row_bytes, &full[st]);
+  };
+  const int first = blockIdx.x, step = gridDim.x;
+  if (threadIdx.x == 0)
+    for (int i = 0; i < stages - 1 && first + i * step < rows; ++i) begin_load(first + i * step, i);
+  float scale0 = host_scale;
+  if (scale_dev != nullptr) scale0 *= *scale_dev;
+  int i = 0;
+  for (int row = first; row < rows; row += step, ++i) {
+    const int st = i % stages;
+    const long long tgt = targets[row];
+    const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V;
+    const bool ok = mbar_wait_bounded(&full[st], (i / stages) & 1, &abort_flag);
+    if (!__syncthreads_and(ok)) break;
+    __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(ring + st * row_bytes);
+    bf16x8 data[kVec];
+    float m = -INFINITY, se = 0.f;
+#pragma unroll
+    for (int v = 0; v < kVec; ++v) {
+      const int at = v * kCEThreads + threadIdx.x;
+      if (at < nvec) {
+        data[v] = load8(p + at * 8);
+        float a[8];
+        unpack8(data[v], a);
+        m = max3(m, a[0], a[1]);
+        m = max3(m, a[2], a[3]);
+        m = max3(m, a[4], a[5]);
+        m = max3(m, a[6], a[7]);
+      }
+    }
+    const float neg_m = m == -INFINITY ? 0.f : -m;
+    float se1 = 0.f;
+    float ex[kKeep ? kVec * 8 : 1];      // exponentials relative to this thread's maximum
+#pragma unroll
+    for (int v = 0; v < kVec; ++v) {
+      if (v * kCEThreads + threadIdx.x < nvec) {
+        float a[8];
+        unpack8(data[v], a);
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+          float x0, x1;
+          add2v(x0, x1, a[j], a[j + 1], neg_m, neg_m);
+          mul2(x0, x1, x0, x1, kLog2e);
+          const float e0 = ex2_approx(x0), e1 = ex2_approx(x1);
+          add2(se, se1, e0, e1);
+          if (kKeep) {
+            ex[v * 8 + j] = e0;
+            ex[v * 8 + j + 1] = e1;
+          }
+        }
+      }
+    }
+    se += se1;
+    // (maximum, sum) of the warp, then of the block; the rows alternate between two sets of slots
+    const float wm = warp_max(m);
+    se = warp_sum(m == -INFINITY && se == 0.f ? 0.f : se * __expf(m - wm));
+    if (lane == 0) {
+      red_m[i & 1][warp] = wm;
+      red_s[i & 1][warp] = se;
+    }
+    float target_logit = 0.f;
+    if (threadIdx.x == 0 && !ignored) target_logit = __bfloat162float(p[tgt]);
+    __syncthreads();
+    const float pm = lane < kCEThreads / 32 ? red_m[i & 1][lane] : -INFINITY;
+    const float ps = lane < kCEThreads / 32 ? red_s[i & 1][lane] : 0.f;
+    const float mx = warp_max(pm);
+    const float sum = warp_sum(pm == -INFINITY && ps == 0.f ? 0.f : ps * __expf(pm - mx));
+    if (threadIdx.x == 0) {
+      const float lse = mx + __logf(sum);
+      if (lse_out) lse_out[row] = lse;
+      loss_out[row] = ignored ? 0.f : lse - target_logit;
+    }
+    if (write_grad) {
+      const float scale = ignored ? 0.f : scale0, by = scale / sum;
+      const float mine = m == -INFINITY ? 0.f : __expf(m - mx) * by;
+#pragma unroll
+      for (int v = 0; v < kVec; ++v) {
+        const int at = v * kCEThreads + threadIdx.x;
+        if (at < nvec) {
+          float a[8];
+          if (kKeep) {
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) mul2(a[j], a[j + 1], ex[v * 8 + j], ex[v * 8 + j + 1], mine);
+          } else {
+            unpack8(data[v], a);
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+              float x0, x1;
+              add2v(x0, x1, a[j], a[j + 1], -mx, -mx);
+              mul2(x0, x1, x0, x1, kLog2e);
+              mul2(a[j], a[j + 1], ex2_approx(x0), ex2_approx(x1), by);
+            }
+          }
+          if (!ignored && tgt >> 3 == at) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if ((tgt & 7) == j) a[j] -= scale;
+          }
+          store8(p + at * 8, pack8(a));
+        }
+      }
+      fence_proxy_async_smem();
+    }
+    __syncthreads();                     // the row is done with (and, with gradients, whole in shared memory)
+    if (threadIdx.x == 0) {
+      if (write_grad) {
+        bulk_store_1d(logits + static_cast<long long>(row) * ld, p, row_bytes);
+        tma_store_commit();
+      }
+      const int next = row + (stages - 1) * step;
+      if (next < rows) {                 // into the stage of the row before, whose copy out has been read by then
+        tma_store_wait_read<1>();
+        begin_load(next, (i + stages - 1) % stages);
+      }
+    }
+  }
+  if (threadIdx.x == 0) {
+    if (abort_flag) {
+      // let the copies in flight land before the shared memory is given back
+      int none = 0;
+      for (int k = i; k < i + stages - 1 && first + k * step < rows; ++k, none = 0)
+        mbar_wait_bounded(&full[k % stages], (k / stages) & 1, &none);
+      atomicCAS(&g_ce_status, 0u, 1u);
+    }
+    tma_store_wait_read<0>();
   }
 }
 
@@ -214,13 +374,24 @@ LLMCTL_API int llmctl_cross_entropy_fwd_bwd(void* logits, long long ld, const lo
   ce_fwd_bwd_kernel<KV><<<rows, kCEThreads, 0, s>>>((__nv_bfloat16*)logits, ld, targets,        \
                                                     loss_per_row, lse_per_row, V, ignore_index, \
                                                     host_scale, scale_dev, write_grad)
+  const size_t row_bytes = static_cast<size_t>(V) * 2;
+  const int stages = row_bytes * 3 <= kCERingBytes ? 3 : 2;
+  auto rows_launch = [&](auto kern) -> cudaError_t {
+    const cudaError_t e = allow_smem(kern, kCERingBytes);
+    if (e != cudaSuccess) return e;
+    kern<<<rows < kNumSMs ? rows : kNumSMs, kCEThreads, stages * row_bytes, s>>>((__nv_bfloat16*)logits, ld, targets, loss_per_row, lse_per_row, rows,
+                                                                                 V, stages, ignore_index, host_scale, scale_dev, write_grad);
+    return cudaSuccess;
+  };
+  // short rows: several CTAs per SM overlap each other; rows that do not fit the ring twice stream through L2
   if (kv <= 2) LAUNCH(2);
-  else if (kv <= 4) LAUNCH(4);
-  else if (kv <= 8) LAUNCH(8);
-  else
+  else if (row_bytes * 2 > kCERingBytes || (reinterpret_cast<uintptr_t>(logits) & 15) != 0)
     ce_fwd_bwd_stream_kernel<<<rows, kCEThreads, 0, s>>>((__nv_bfloat16*)logits, ld, targets,
                                                          loss_per_row, lse_per_row, V, ignore_index,
                                                          host_scale, scale_dev, write_grad);
+  else if (kv <= 4) LLMCTL_CHECK(rows_launch(ce_rows_kernel<4>));
+  else if (kv <= 8) LLMCTL_CHECK(rows_launch(ce_rows_kernel<8>));
+  else LLMCTL_CHECK(rows_launch(ce_rows_kernel<14>));
 #undef LAUNCH
   LLMCTL_RETURN_LAST();
 }
@@ -248,4 +419,15 @@ LLMCTL_API int llmctl_cross_entropy_finalize(void* logits, long long ld, const l
       (__nv_bfloat16*)logits, ld, targets, lse, V_local, vocab_start, ignore_index, host_scale,
       scale_dev);
   LLMCTL_RETURN_LAST();
+}
+
+// 0 unless a bounded wait of the loss kernel ran out since the last clearing call (synchronises the device).
+LLMCTL_API int llmctl_cross_entropy_status(int clear) {
+  unsigned int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_ce_status, sizeof(v)) != cudaSuccess) return -1;
+  if (clear && v != 0) {
+    const unsigned int zero = 0;
+    (void)cudaMemcpyToSymbol(g_ce_status, &zero, sizeof(zero));
+  }
+  return static_cast<int>(v);
 }

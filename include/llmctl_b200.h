@@ -69,6 +69,8 @@ int llmctl_cross_entropy_fwd_bwd(void* logits, long long ld, const long long* ta
                                  float* loss_per_row, float* lse_per_row, int rows, int V,
                                  long long ignore_index, float host_scale, const float* scale_dev,
                                  int write_grad, void* stream);
+/* 0 unless a bounded wait of the loss kernel ran out since the last clearing call (synchronises the device). */
+int llmctl_cross_entropy_status(int clear);
 int llmctl_cross_entropy_partial(const void* logits, long long ld, const long long* targets,
                                  float* stats, int rows, int V_local, long long vocab_start,
                                  void* stream);
