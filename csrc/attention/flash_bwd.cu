@@ -1,14 +1,14 @@
-// K6 (backward): two deterministic tcgen05 kernels, head sizes 64 and 128, sequences of any length.
+// K6 (backward): one deterministic tcgen05 kernel over two kinds of items, head sizes 64 and 128, sequences of any length.
 //
-//   dKV kernel  — an item = (batch, head, 128-key block): K_j, V_j resident in shared memory, query blocks of 128 rows
+//   dKV items   — an item = (batch, head, 128-key block): K_j, V_j resident in shared memory, query blocks of 128 rows
 //                 streamed.  It works on the TRANSPOSED scores,
 //                     S^T = K_j Q_i^T      dP^T = V_j dO_i^T        (M = 128 keys in TMEM lanes, N = 128 queries)
 //                 so that P^T and dS^T — written back by the softmax threads as bf16 over the very TMEM columns they
 //                 were read from — are directly the A operands of
 //                     dV += P^T dO_i       dK += dS^T Q_i
-//   dQ kernel   — an item = (batch, head, 128-query block): Q_i, dO_i resident, key blocks of 128 streamed;
+//   dQ items    — an item = (batch, head, 128-query block): Q_i, dO_i resident, key blocks of 128 streamed;
 //                     S = Q_i K_j^T    dP = dO_i V_j^T    dS -> TMEM    dQ += dS K_j
-// Recomputing S and dP in the second kernel costs 7 products instead of 5, but needs no fp32 accumulator of dQ in memory and
+// Recomputing S and dP for the second kind costs 7 products instead of 5, but needs no fp32 accumulator of dQ in memory and
 // makes the gradient bit-reproducible.  The 1/sqrt(d) factor of dS is applied once in the dK / dQ epilogues.
 //
 // What bounds it: the tensor pipe (4 / 3 products of 128 x 128 x D per block pair, 2048 / 1536 clocks at D = 128) against
@@ -18,8 +18,9 @@
 // of operands per clock where shared memory gives 128, and started a CTA per item.)  The streamed tiles Q, dO, Q, dO, ... share
 // one ring: with 5 slots beside the two resident tiles (all that 227 KB hold at D = 128) Q(n+1) is fetched as soon as dV(n-2)
 // has retired, a block and a half ahead of its use; rings of two stages each left the pipe waiting 200-1000 clocks per block.
-// P is handed over in two halves, as in the forward.  Persistent: one CTA per SM claims items, longest of a group first; TMEM,
-// barriers and maps are set up once, an item's first tiles are fetched while the previous item is still in its softmax, and a
+// P is handed over in two halves, as in the forward.  Persistent: one CTA per SM claims items, longest of a group first, the dKV items
+// of a group of heads before its dQ items (which read the same tiles again, from L2, and fill the SMs that the last dKV items leave
+// idle: 8 x 512 x 32 x 128 took 94 us in two launches, 88 us in one); TMEM, barriers and maps are set up once, an item's first tiles are fetched while the previous item is still in its softmax, and a
 // warpgroup of its own reads the accumulators out and stores them meanwhile (a row per thread: 4900 clocks from the last product
 // to the next item's first softmax when the softmax warps did it, against 2900 per block).
 //
@@ -27,6 +28,8 @@
 // never stored (causal only: keys past the end are then hidden from every real query by the mask).
 //
 // Reference: autograd through HF attention (reference llmctl/runtime/engine.py:288-291).  Baseline: cuDNN SDPA bwd.
+#include <type_traits>
+
 #include "../common/ptx.cuh"
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
@@ -58,10 +61,12 @@ struct Cfg {
   static constexpr int kSmem = kBarsAt + 384;
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
-__device__ unsigned int g_status = 0;        // != 0: a bounded wait of these kernels ran out
+__device__ unsigned int g_status = 0;        // != 0: a bounded wait of the kernel ran out
+using DKV = std::integral_constant<bool, false>;
+using DQ = std::integral_constant<bool, true>;
 
 struct Maps {
-  CUtensorMap res0, res1, sub0, sub1;        // operand 0 pairs up in the S-like product, operand 1 in the dP-like one
+  CUtensorMap q, k, v, d_o;
 };
 }  // namespace fbwd
 
@@ -72,8 +77,8 @@ template <int D>
 __global__ void __launch_bounds__(256)
 flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO, long long tok_stride,
                       const float* __restrict__ lse, float* __restrict__ nl2, float* __restrict__ ndl, int S, int Sp, int H,
-                      int chunks, int* __restrict__ counters) {
-  if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;       // the item counters of the two kernels that follow
+                      int chunks, int* __restrict__ counter) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;       // the item counter of the kernel that follows
   constexpr int kLanes = D / 8, kGroups = 256 / kLanes, kRows = 4;
   const int g = threadIdx.x / kLanes, li = threadIdx.x % kLanes;
   const int bh = blockIdx.x / chunks, h = bh % H;
@@ -123,13 +128,13 @@ __device__ __forceinline__ void fbwd_store16(__nv_bfloat16* dst, const uint32_t*
   }
 }
 
-// kDQ = false: dKV kernel (resident K, V; streamed Q, dO; out0 = dV, out1 = dK).  kDQ = true: dQ kernel (resident Q, dO; streamed
-// K, V; out0 = dQ).
-template <int D, bool kDQ>
+// dKV items: resident K, V; streamed Q, dO.  dQ items: resident Q, dO; streamed K, V.  Operand 0 of either pair (K / Q) makes the
+// S-like product, operand 1 (V / dO) the dP-like one.
+template <int D>
 __global__ void __launch_bounds__(fbwd::kThreads, 1)
 flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restrict__ nl2, const float* __restrict__ ndl,
-                 __nv_bfloat16* __restrict__ out0, __nv_bfloat16* __restrict__ out1, long long out_tok, int out_wide, int B, int S,
-                 int H, int group, int* __restrict__ counter, float scale_log2, float scale, int causal) {
+                 __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long long out_tok,
+                 int out_wide, int B, int S, int H, int group, int* __restrict__ counter, float scale_log2, float scale, int causal) {
   using namespace fbwd;
   using C = Cfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -148,7 +153,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   }
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int nblk = (S + kBlk - 1) / kBlk, Sp = nblk * kBlk;
-  const int BH = B * H, n_items = nblk * BH;
+  const int BH = B * H, n_items = 2 * nblk * BH;
 
   if (threadIdx.x == 0) {
     mbar_init(&bar.res, 1);
@@ -170,10 +175,10 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     fence_mbar_init();
   }
   if (warp == 0 && lane == 0) {
-    prefetch_tmap(&maps.res0);
-    prefetch_tmap(&maps.res1);
-    prefetch_tmap(&maps.sub0);
-    prefetch_tmap(&maps.sub1);
+    prefetch_tmap(&maps.q);
+    prefetch_tmap(&maps.k);
+    prefetch_tmap(&maps.v);
+    prefetch_tmap(&maps.d_o);
   }
   if (warp == 1) tmem_alloc<1>(&bar.tmem, 512);
   tc_fence_before();
@@ -184,14 +189,17 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tAcc0 = tmem_base + 256, tAcc1 = tmem_base + 384;
   volatile int* abort = &bar.abort;
 
-  // item -> (resident block, batch x head) and the streamed blocks [first, first + n); longest items of a group first
-  auto decode = [&](int item, int& rb, int& bh, int& first, int& n) {
-    const int base = item / (group * nblk) * group, rem = item - base * nblk, heads = min(group, BH - base);
+  // item -> (kind, resident block, batch x head) and the streamed blocks [first, first + n); longest items of a group first
+  auto decode = [&](int item, bool& is_dq, int& rb, int& bh, int& first, int& n) {
+    const int base = item / (2 * group * nblk) * group, heads = min(group, BH - base);
+    int rem = item - 2 * base * nblk;
+    is_dq = rem >= heads * nblk;
+    if (is_dq) rem -= heads * nblk;
     const int k = rem / heads;
     bh = base + rem % heads;
-    rb = kDQ ? nblk - 1 - k : k;
-    first = (!kDQ && causal) ? rb : 0;
-    n = (causal ? (kDQ ? rb + 1 : nblk) : nblk) - first;
+    rb = is_dq ? nblk - 1 - k : k;
+    first = (!is_dq && causal) ? rb : 0;
+    n = (causal ? (is_dq ? rb + 1 : nblk) : nblk) - first;
   };
   // the k-th item of this CTA, as the TMA warp published it; false when a wait ran out or there is none left
   auto next_item = [&](uint32_t k, int& item) {
@@ -228,24 +236,27 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         mbar_arrive(&bar.item_full[k % kQueue]);
         if (item >= n_items) break;
         const int next = gridDim.x + atomicAdd(counter, 1);
+        bool is_dq;
         int rb, bh, first, n;
-        decode(item, rb, bh, first, n);
+        decode(item, is_dq, rb, bh, first, n);
         const int h = bh % H, b = bh / H;
+        const CUtensorMap *res0 = is_dq ? &maps.q : &maps.k, *res1 = is_dq ? &maps.d_o : &maps.v;
+        const CUtensorMap *sub0 = is_dq ? &maps.k : &maps.q, *sub1 = is_dq ? &maps.v : &maps.d_o;
         for (int i = 0; i < n; ++i) {
           const int row = (first + i) * kBlk;
-          if (!(ok = stream(&maps.sub0, h, row, b, nullptr, nullptr))) break;
+          if (!(ok = stream(sub0, h, row, b, nullptr, nullptr))) break;
           if (i == 0) {                // the resident tiles: free once the previous item's last S and dP have retired
             if (!(ok = mbar_wait_bounded(&bar.resfree, (k & 1u) ^ 1u, abort))) break;
             mbar_expect_tx(&bar.res, 2 * C::kTile);
             ++nr;
 #pragma unroll
             for (int p = 0; p < C::kPanels; ++p) {
-              tma_load_4d(smem + p * kPanel, &maps.res0, &bar.res, 64 * p, h, rb * kBlk, b);
-              tma_load_4d(smem + C::kTile + p * kPanel, &maps.res1, &bar.res, 64 * p, h, rb * kBlk, b);
+              tma_load_4d(smem + p * kPanel, res0, &bar.res, 64 * p, h, rb * kBlk, b);
+              tma_load_4d(smem + C::kTile + p * kPanel, res1, &bar.res, 64 * p, h, rb * kBlk, b);
             }
           }
           const long long at = static_cast<long long>(bh) * Sp + row;
-          if (!(ok = stream(&maps.sub1, h, row, b, kDQ ? nullptr : nl2 + at, ndl + at))) break;
+          if (!(ok = stream(sub1, h, row, b, is_dq ? nullptr : nl2 + at, ndl + at))) break;
         }
         if (!ok) break;
         item = next;
@@ -289,11 +300,9 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
           umma_ts<1>(t, a + (ks >> 2) * 64 + (ks & 3) * 8, b0 + ((ks * 2048) >> 4), id_acc, ks == 0 ? 1u - fresh : 1u);
     };
     uint32_t g = 0, k = 0;
-    bool ok = true;
-    for (int item; ok && next_item(k, item); ++k) {
-      int rb, bh, first, n;
-      decode(item, rb, bh, first, n);
-      ok = wait(&bar.res, k & 1u);
+    auto run = [&](auto kind, int n) {
+      constexpr bool kDQ = decltype(kind)::value;
+      bool ok = true;
       for (int i = 0; ok && i < n; ++i, ++g) {
         const uint32_t e0 = 2 * g, e1 = e0 + 1;            // this block's streamed tiles; the next block's are e0 + 2, e1 + 2
         const uint32_t fresh = i == 0 ? 1u : 0u;
@@ -340,7 +349,10 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         if (elect_one()) {
           issue_acc(kDQ ? tAcc0 : tAcc1, tdP, tile_at(e0), fresh, 2);    // dK += dS^T Q  /  dQ += dS K
           umma_commit<1>(&bar.empty[e0 % C::kSlots]);
-          if (i + 1 == n) umma_commit<1>(&bar.acc[kDQ ? 0 : 1]);
+          if (i + 1 == n) {
+            if (kDQ) umma_commit<1>(&bar.acc[0]);
+            umma_commit<1>(&bar.acc[1]);                   // every item completes both, used or not: phases follow the items
+          }
         }
         if (i + 1 < n) {
           if (!(ok = arrived(e1 + 2))) break;
@@ -353,6 +365,15 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
           }
         }
       }
+      return ok;
+    };
+    bool ok = true;
+    for (int item; ok && next_item(k, item); ++k) {
+      bool is_dq;
+      int rb, bh, first, n;
+      decode(item, is_dq, rb, bh, first, n);
+      ok = wait(&bar.res, k & 1u);
+      if (ok) ok = is_dq ? run(DQ{}, n) : run(DKV{}, n);
     }
   } else if (warp < 10) {
     // ------------------- softmax / dS warpgroups: half wg of the streamed columns, all 128 resident rows -------------------
@@ -362,10 +383,9 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     const uint32_t lane_off = static_cast<uint32_t>(q4 * 32) << 16;
     const uint32_t tSb = tS + wg * 64 + lane_off, tPb = tdP + wg * 64 + lane_off;
     uint32_t g = 0, k = 0;
-    bool ok = true;
-    for (int item; ok && next_item(k, item); ++k) {
-      int rb, bh, first, n;
-      decode(item, rb, bh, first, n);
+    auto run = [&](auto kind, int rb, int bh, int first, int n) {
+      constexpr bool kDQ = decltype(kind)::value;
+      bool ok = true;
       float row_nl = 0.f, row_nd = 0.f;                   // dQ kernel: this query row's statistics
       if (kDQ) {
         row_nl = nl2[static_cast<long long>(bh) * Sp + rb * kBlk + row];
@@ -388,7 +408,10 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         if (kDQ) {                                        // S is in registers: the next scores may overwrite it
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&bar.p[1]);
+          if (lane == 0) {
+            mbar_arrive(&bar.p[0]);                       // every block completes both halves: phases follow the blocks
+            mbar_arrive(&bar.p[1]);
+          }
         }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -462,6 +485,14 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar.ds);
       }
+      return ok;
+    };
+    bool ok = true;
+    for (int item; ok && next_item(k, item); ++k) {
+      bool is_dq;
+      int rb, bh, first, n;
+      decode(item, is_dq, rb, bh, first, n);
+      ok = is_dq ? run(DQ{}, rb, bh, first, n) : run(DKV{}, rb, bh, first, n);
     }
   } else {
     // ------------- epilogue warpgroup: accumulators -> registers -> bf16 -> global, a row per thread -------------
@@ -471,18 +502,23 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     uint32_t k = 0;
     bool ok = true;
     for (int item; ok && next_item(k, item); ++k) {
+      bool is_dq;
       int rb, bh, first, n;
-      decode(item, rb, bh, first, n);
+      decode(item, is_dq, rb, bh, first, n);
       const bool real = rb * kBlk + row < S;
       const long long at = (static_cast<long long>(bh / H) * S + rb * kBlk + row) * out_tok + (bh % H) * D;
 #pragma unroll 1
-      for (int a = 0; a < (kDQ ? 1 : 2); ++a) {           // dKV: dV from acc0, then scale * dK from acc1.  dQ: scale * dQ from acc0.
+      for (int a = 0; a < 2; ++a) {                       // dKV: dV from acc0, then scale * dK from acc1.  dQ: scale * dQ from acc0.
         ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar.acc[a], k & 1u, abort));
         if (!ok) break;
+        if (is_dq && a == 1) {                            // nothing there
+          if (lane == 0) mbar_arrive(&bar.accfree[1]);
+          break;
+        }
         tc_fence_after();
         const uint32_t tA = (a == 0 ? tAcc0 : tAcc1) + lane_off;
-        const float mul = (kDQ || a == 1) ? scale : 1.f;
-        __nv_bfloat16* dst = (a == 0 ? out0 : out1) + at;
+        const float mul = (is_dq || a == 1) ? scale : 1.f;
+        __nv_bfloat16* dst = (is_dq ? dq : a == 0 ? dv : dk) + at;
 #pragma unroll
         for (int c0 = 0; c0 < D; c0 += 64) {
           uint32_t r[64];
@@ -505,7 +541,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
 
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && bar.abort) atomicCAS(&g_status, 0u, kDQ ? 2u : 1u);
+  if (threadIdx.x == 0 && bar.abort) atomicCAS(&g_status, 0u, 1u);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc<1>(tmem_base, 512);
@@ -520,13 +556,13 @@ static int flash_bwd_launch(const void* q, const void* k, const void* v, const v
   using C = Cfg<D>;
   const int nblk = (S + kBlk - 1) / kBlk, Sp = nblk * kBlk;
   float *nl2 = scratch, *ndl = scratch + static_cast<long long>(B) * H * Sp;
-  int* counters = reinterpret_cast<int*>(ndl + static_cast<long long>(B) * H * Sp);
+  int* counter = reinterpret_cast<int*>(ndl + static_cast<long long>(B) * H * Sp);
   const long long head_bytes = 4ll * Sp * D * 2, fit = kGroupBytes / head_bytes;
   const int group = static_cast<int>(fit < 1 ? 1 : fit < B * H ? fit : B * H);
   constexpr int kPrepRows = 256 / (D / 8) * 4;
   const int chunks = (Sp + kPrepRows - 1) / kPrepRows;
   flash_bwd_prep_kernel<D><<<chunks * B * H, 256, 0, s>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, o_tok, lse, nl2, ndl, S, Sp,
-                                                          H, chunks, counters);
+                                                          H, chunks, counter);
   CUtensorMap mq, mk, mv, mdo;
   int rc = 0;
   auto mkmap = [&](CUtensorMap* m, const void* base, long long tok) {
@@ -537,18 +573,12 @@ static int flash_bwd_launch(const void* q, const void* k, const void* v, const v
   mkmap(&mv, v, v_tok);
   mkmap(&mdo, d_o, o_tok);
   if (rc) return rc;
-  cudaError_t e = allow_smem(flash_bwd_kernel<D, false>, C::kSmem);
-  if (e == cudaSuccess) e = allow_smem(flash_bwd_kernel<D, true>, C::kSmem);
+  const cudaError_t e = allow_smem(flash_bwd_kernel<D>, C::kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  const float sl2 = scale * 1.4426950408889634f;
-  const int n_items = nblk * B * H, grid = n_items < kNumSMs ? n_items : kNumSMs;
+  const int n_items = 2 * nblk * B * H, grid = n_items < kNumSMs ? n_items : kNumSMs;
   const int wide = dqkv_tok % 16 == 0 && ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 31) == 0;
-  // dKV: S^T = K Q^T, dP^T = V dO^T; dV in accumulator 0, dK in 1
-  flash_bwd_kernel<D, false><<<grid, kThreads, C::kSmem, s>>>(Maps{mk, mv, mq, mdo}, nl2, ndl, (__nv_bfloat16*)dv, (__nv_bfloat16*)dk,
-                                                              dqkv_tok, wide, B, S, H, group, counters, sl2, scale, causal);
-  // dQ: S = Q K^T, dP = dO V^T
-  flash_bwd_kernel<D, true><<<grid, kThreads, C::kSmem, s>>>(Maps{mq, mdo, mk, mv}, nl2, ndl, (__nv_bfloat16*)dq, nullptr, dqkv_tok, wide,
-                                                             B, S, H, group, counters + 1, sl2, scale, causal);
+  flash_bwd_kernel<D><<<grid, kThreads, C::kSmem, s>>>(Maps{mq, mk, mv, mdo}, nl2, ndl, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv,
+                                                       dqkv_tok, wide, B, S, H, group, counter, scale * 1.4426950408889634f, scale, causal);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -558,7 +588,7 @@ using namespace llmctl;
 
 // q,k,v,o,do: [B,S,H,D] bf16 views, D = 64 or 128 (token strides given in elements, a batch S tokens on; do and o share
 // o_tok_stride); dq,dk,dv: outputs with token stride dqkv_tok_stride; lse: fp32 [B,H,S] from the forward;
-// scratch: fp32 [2 * B * H * (S rounded up to 128) + 2]: per-row log-sum-exp and delta, item counters.
+// scratch: fp32 [2 * B * H * (S rounded up to 128) + 2]: per-row log-sum-exp and delta, item counter.
 // Any S when causal, else a multiple of 128.
 LLMCTL_API int llmctl_flash_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                                      const float* lse, void* dq, void* dk, void* dv, float* scratch, int B, int S,
