@@ -124,6 +124,24 @@ __device__ __forceinline__ void tile_to_mn(int tile, int num_m, int num_n, int& 
   n_blk = in_group / gsize;
 }
 
+// One 32-row x 64-column box: `pair(e)` gives columns 2e and 2e + 1 of this lane's row, packed to bf16; buffers alternate.
+template <typename Pair>
+__device__ __forceinline__ void stage_box(uint8_t* out_smem, uint32_t& out_n, const CUtensorMap* tm, int col0, int row0, int lane, Pair pair) {
+  uint8_t* buf = out_smem + (out_n & 1u) * kOutBox;
+  ++out_n;
+  if (lane == 0) tma_store_wait_read<1>();          // the store before the last has left this buffer
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(pair(4 * j), pair(4 * j + 1), pair(4 * j + 2), pair(4 * j + 3));
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    tma_store_2d(tm, buf, col0, row0);
+    tma_store_commit();
+  }
+}
+
 // Epilogue of one tile, one warp: BN accumulator columns of 32 rows (row0 = the warp's first) -> C.
 // bf16 without accumulation goes through shared memory and TMA: 64 columns at a time, each lane packs its row into the swizzled
 // buffer and one lane stores the box, while the next columns are read.  A row per lane straight to global memory touches 32 lines
@@ -140,25 +158,8 @@ __device__ __forceinline__ void gemm_epilogue(uint32_t t_row, uint8_t* out_smem,
         tmem_ld_x32(t_row + c * 64 + 32, r + 32);
         tmem_ld_wait();
         if (row0 >= M || n0 + c * 64 >= N) continue;      // uniform over the warp
-        uint8_t* buf = out_smem + (out_n & 1u) * kOutBox;
-        ++out_n;
-        if (lane == 0) tma_store_wait_read<1>();          // the store before the last has left this buffer
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          uint4 w;
-          w.x = pack_bf16x2(__uint_as_float(r[j * 8 + 0]), __uint_as_float(r[j * 8 + 1]));
-          w.y = pack_bf16x2(__uint_as_float(r[j * 8 + 2]), __uint_as_float(r[j * 8 + 3]));
-          w.z = pack_bf16x2(__uint_as_float(r[j * 8 + 4]), __uint_as_float(r[j * 8 + 5]));
-          w.w = pack_bf16x2(__uint_as_float(r[j * 8 + 6]), __uint_as_float(r[j * 8 + 7]));
-          *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) = w;
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          tma_store_2d(tmC, buf, n0 + c * 64, row0);
-          tma_store_commit();
-        }
+        stage_box(out_smem, out_n, tmC, n0 + c * 64, row0, lane,
+                  [&](int e) { return pack_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])); });
       }
       return;
     }
@@ -204,10 +205,43 @@ __device__ __forceinline__ void gemm_epilogue(uint32_t t_row, uint8_t* out_smem,
   }
 }
 
-template <int BN, bool A_MN, bool B_MN, typename OutT>
+// Gated up-projection (llmctl_gemm_swiglu_bf16): the tile's first half of columns multiplies rows of the gate matrix, the second half the
+// same rows of the up matrix, and the epilogue stores silu(gate) * up, and gate and up beside it when the backward will want them.
+struct SwigluMaps {
+  CUtensorMap w_up, gate, up, act;
+  int keep;                  // gate and up are stored
+};
+template <int BN>
+__device__ __forceinline__ void swiglu_epilogue(uint32_t t_row, uint8_t* out_smem, uint32_t& out_n, const SwigluMaps& maps, int row0, int f0,
+                                                int M, int F, int lane) {
+#pragma unroll 1
+  for (int c = 0; c < BN / 128; ++c) {
+    uint32_t g[64], u[64];
+    tmem_ld_x32(t_row + c * 64, g);
+    tmem_ld_x32(t_row + c * 64 + 32, g + 32);
+    tmem_ld_x32(t_row + BN / 2 + c * 64, u);
+    tmem_ld_x32(t_row + BN / 2 + c * 64 + 32, u + 32);
+    tmem_ld_wait();
+    const int col = f0 + c * 64;
+    if (row0 >= M || col >= F) continue;               // uniform over the warp
+    auto packed = [](const uint32_t* r, int e) { return pack_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])); };
+    if (maps.keep) {
+      stage_box(out_smem, out_n, &maps.gate, col, row0, lane, [&](int e) { return packed(g, e); });
+      stage_box(out_smem, out_n, &maps.up, col, row0, lane, [&](int e) { return packed(u, e); });
+    }
+    auto act = [](uint32_t gv, uint32_t uv) {
+      const float x = __uint_as_float(gv);
+      return x * __uint_as_float(uv) * __fdividef(1.f, 1.f + __expf(-x));
+    };
+    stage_box(out_smem, out_n, &maps.act, col, row0, lane, [&](int e) { return pack_bf16x2(act(g[2 * e], u[2 * e]), act(g[2 * e + 1], u[2 * e + 1])); });
+  }
+}
+
+template <int BN, bool A_MN, bool B_MN, typename OutT, bool kSwiglu = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate) {
+                    const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate,
+                    const __grid_constant__ SwigluMaps sw) {
   using Cfg = GemmCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[Cfg::kStages];
@@ -222,7 +256,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int lane = threadIdx.x & 31;
 
   const int num_m = (M + kBM - 1) / kBM;
-  const int num_n = (N + BN - 1) / BN;
+  constexpr int kCols = kSwiglu ? BN / 2 : BN;         // output columns per tile; with the gate N counts those of one half
+  const int num_n = (N + kCols - 1) / kCols;
   const int num_tiles = num_m * num_n;
   const int num_kb = (K + kBK - 1) / kBK;
 
@@ -257,7 +292,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         tile_to_mn(tile, num_m, num_n, mb_, nb_);
         mb_ = gate_perm(gate, mb_);
         const int m0 = mb_ * kBM;
-        const int n0 = nb_ * BN;
+        const int n0 = nb_ * kCols;
         const int b_row = grouped_b_row(gate, mb_, n0, N);
         if (b_row < 0) continue;
         gate_wait(gate, m0, min(m0 + kBM, M));
@@ -275,7 +310,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int g = 0; g < kBM / 64; ++g)
               tma_load_2d(sA + g * 8192, &tmA, &bar_full[stage], m0 + g * 64, k0);
           }
-          if (!B_MN) {
+          if (kSwiglu) {
+            tma_load_2d(sB, &tmB, &bar_full[stage], k0, n0);
+            tma_load_2d(sB + Cfg::kBBytes / 2, &sw.w_up, &bar_full[stage], k0, n0);
+          } else if (!B_MN) {
             tma_load_2d(sB, &tmB, &bar_full[stage], k0, b_row);
           } else {
 #pragma unroll
@@ -342,12 +380,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       tile_to_mn(tile, num_m, num_n, mb_, nb_);
       mb_ = gate_perm(gate, mb_);
       const int m0 = mb_ * kBM;
-      const int n0 = nb_ * BN;
+      const int n0 = nb_ * kCols;
       if (grouped_b_row(gate, mb_, n0, N) < 0) continue;
       mbar_wait(&bar_tfull[acc], aphase);
       tc_fence_after();
-      gemm_epilogue<BN, OutT>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN), out_smem, out_n, &tmC, C,
-                              ldc, m0 + q * 32, n0, M, N, beta, lane);
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
+      if constexpr (kSwiglu)
+        swiglu_epilogue<BN>(t_row, out_smem, out_n, sw, m0 + q * 32, n0, M, N, lane);
+      else
+        gemm_epilogue<BN, OutT>(t_row, out_smem, out_n, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_tempty[acc]);
@@ -391,10 +432,11 @@ struct Gemm2Cfg {
   static constexpr int kTmemCols = 2 * PBN;              // 512 / 256
 };
 
-template <int PBN, bool A_MN, bool B_MN, typename OutT>
+template <int PBN, bool A_MN, bool B_MN, typename OutT, bool kSwiglu = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate) {
+                     const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate,
+                    const __grid_constant__ SwigluMaps sw) {
   using Cfg = Gemm2Cfg<PBN>;
   constexpr int BN = Cfg::kBN;
   extern __shared__ uint8_t smem_raw[];
@@ -413,7 +455,8 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   const int num_pairs = gridDim.x >> 1;
 
   const int num_m = (M + 2 * kBM - 1) / (2 * kBM);
-  const int num_n = (N + BN - 1) / BN;
+  constexpr int kCols = kSwiglu ? BN / 2 : BN;         // output columns per tile; with the gate N counts those of one half
+  const int num_n = (N + kCols - 1) / kCols;
   const int num_tiles = num_m * num_n;
   const int num_kb = (K + kBK - 1) / kBK;
 
@@ -449,7 +492,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         tile_to_mn(tile, num_m, num_n, mb_, nb_);
         mb_ = gate_perm(gate, mb_);
         const int m0 = mb_ * (2 * kBM) + static_cast<int>(cta_rank) * kBM;
-        const int n0 = nb_ * BN + static_cast<int>(cta_rank) * (BN / 2);
+        const int n0 = kSwiglu ? nb_ * kCols : nb_ * BN + static_cast<int>(cta_rank) * (BN / 2);
         if (m0 < M) gate_wait(gate, m0, min(m0 + kBM, M));
         gate_wait_b<B_MN>(gate, n0, min(n0 + BN / 2, N));
         for (int kb = 0; kb < num_kb; ++kb) {
@@ -468,7 +511,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
               tma_load_2d_cg2(sA + g * 8192, &tmA, full_leader, m0 + g * 64, k0);
           }
           if (!B_MN) {
-            tma_load_2d_cg2(sB, &tmB, full_leader, k0, n0);
+            tma_load_2d_cg2(sB, kSwiglu && cta_rank == 1 ? &sw.w_up : &tmB, full_leader, k0, n0);
           } else {
 #pragma unroll
             for (int g = 0; g < (BN / 2) / 64; ++g)
@@ -529,11 +572,14 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       tile_to_mn(tile, num_m, num_n, mb_, nb_);
       mb_ = gate_perm(gate, mb_);
       const int m0 = mb_ * (2 * kBM) + static_cast<int>(cta_rank) * kBM;
-      const int n0 = nb_ * BN;
+      const int n0 = nb_ * kCols;
       mbar_wait(&bar_tfull[acc], aphase);
       tc_fence_after();
-      gemm_epilogue<BN, OutT>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN), out_smem, out_n, &tmC, C,
-                              ldc, m0 + q * 32, n0, M, N, beta, lane);
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
+      if constexpr (kSwiglu)
+        swiglu_epilogue<BN>(t_row, out_smem, out_n, sw, m0 + q * 32, n0, M, N, lane);
+      else
+        gemm_epilogue<BN, OutT>(t_row, out_smem, out_n, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(&bar_tempty[acc], 0);   // always the leader's barrier
@@ -590,7 +636,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   int grid = num_sms();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (tiles < grid) grid = tiles;
-  kern<<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate);
+  kern<<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate, SwigluMaps{});
   LLMCTL_RETURN_LAST();
 }
 
@@ -633,7 +679,7 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
   if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
   if (pairs < 1) pairs = 1;
   if (tiles < pairs) pairs = tiles;
-  kern<<<2 * pairs, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate);
+  kern<<<2 * pairs, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate, SwigluMaps{});
   LLMCTL_RETURN_LAST();
 }
 
@@ -645,6 +691,37 @@ static int dispatch_layout2(int a_mn, int b_mn, const void* A, const void* B, vo
   if (!a_mn && b_mn) return launch_gemm2<PBN, false, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
   if (a_mn && !b_mn) return launch_gemm2<PBN, true, false, OutT>(A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
   return launch_gemm2<PBN, true, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
+}
+
+template <bool kPair>
+static int launch_swiglu(const void* X, const void* W, void* GU, void* ACT, int M, int F, int K, long long ldx, long long ldw, long long ldgu,
+                         long long ldact, cudaStream_t s) {
+  constexpr int kCols = kPair ? 128 : 64;            // gate rows (and up rows) per tile
+  const __nv_bfloat16 *w = (const __nv_bfloat16*)W, *gu = (const __nv_bfloat16*)GU;
+  CUtensorMap tmA, tmW;
+  SwigluMaps sw;
+  int rc = get_tmap_2d_bf16(&tmA, X, M, K, ldx, kBM, kBK, 1);
+  if (!rc) rc = get_tmap_2d_bf16(&tmW, w, F, K, ldw, kCols, kBK, 1);
+  if (!rc) rc = get_tmap_2d_bf16(&sw.w_up, w + static_cast<long long>(F) * ldw, F, K, ldw, kCols, kBK, 1);
+  if (!rc) rc = get_tmap_2d_bf16(&sw.act, ACT, M, F, ldact, 32, 64, 1);
+  sw.gate = sw.up = sw.act;
+  sw.keep = GU != nullptr;
+  if (!rc && GU != nullptr) rc = get_tmap_2d_bf16(&sw.gate, gu, M, F, ldgu, 32, 64, 1);
+  if (!rc && GU != nullptr) rc = get_tmap_2d_bf16(&sw.up, gu + F, M, F, ldgu, 32, 64, 1);
+  if (rc) LLMCTL_FAIL(rc, "tensor maps");
+  const int tiles = ((M + (kPair ? 2 : 1) * kBM - 1) / ((kPair ? 2 : 1) * kBM)) * ((F + kCols - 1) / kCols);
+  if constexpr (kPair) {
+    auto kern = gemm2_tcgen05_kernel<256, false, false, __nv_bfloat16, true>;
+    LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256>::kSmemBytes));
+    const int pairs = tiles < num_sms() / 2 ? tiles : num_sms() / 2;
+    kern<<<2 * pairs, kGemmThreads, Gemm2Cfg<256>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0, GemmGate{}, sw);
+  } else {
+    auto kern = gemm_tcgen05_kernel<128, false, false, __nv_bfloat16, true>;
+    LLMCTL_CHECK(allow_smem(kern, GemmCfg<128>::kSmemBytes));
+    kern<<<tiles < num_sms() ? tiles : num_sms(), kGemmThreads, GemmCfg<128>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0,
+                                                                                            GemmGate{}, sw);
+  }
+  LLMCTL_RETURN_LAST();
 }
 
 }  // namespace llmctl
@@ -714,6 +791,20 @@ LLMCTL_API int llmctl_gemm_bf16(const void* A, const void* B, void* C, int M, in
                                 int out_fp32, int beta, int tile_n, int max_ctas, void* stream) {
   return gemm_bf16_impl(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, beta, tile_n, max_ctas, stream,
                         GemmGate{});
+}
+
+// ACT[M, F] = silu(X Wg^T) * (X Wu^T) for X [M, K] and the packed W [2F, K] = [Wg ; Wu]; GU [M, 2F] receives the two products (rounded
+// to bf16) unless it is null.  The activation is taken from the fp32 accumulators.  One pass less over the 2F columns and one launch
+// less than the product and llmctl_swiglu_fwd; tiles by the rule of llmctl_gemm_bf16 (128 of the 256 columns of a pair tile are gate
+// columns, 64 of the 128 of a single one).
+LLMCTL_API int llmctl_gemm_swiglu_bf16(const void* X, const void* W, void* GU, void* ACT, int M, int F, int K, long long ldx, long long ldw,
+                                       long long ldgu, long long ldact, void* stream) {
+  LLMCTL_BEGIN();
+  LLMCTL_REQUIRE(M > 0 && F > 0 && K > 0 && F % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && ldact % 8 == 0 && (GU == nullptr || ldgu % 8 == 0));
+  LLMCTL_REQUIRE(((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(GU) |
+                   reinterpret_cast<uintptr_t>(ACT)) & 15) == 0 && static_cast<long long>(ldact) >= F);
+  const bool one_wave = static_cast<long long>((M + kBM - 1) / kBM) * ((F + 63) / 64) <= num_sms();
+  return (one_wave || M <= 128 ? launch_swiglu<false> : launch_swiglu<true>)(X, W, GU, ACT, M, F, K, ldx, ldw, ldgu, ldact, (cudaStream_t)stream);
 }
 
 // Grouped GEMM for mixture-of-experts layers: C[r, :] = A[r, :] W[expert(r)]^T over `max_tiles` blocks of 128 rows of A

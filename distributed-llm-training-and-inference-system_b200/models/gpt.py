@@ -81,6 +81,8 @@ class MLP(nn.Module):
                                           dtype=dtype, device=device, fused_name="mlp_down")
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        if self.gated and not (self.selective_recompute and torch.is_grad_enabled()) and self.up.runs_plain():
+            return self.down(ops.linear_swiglu(x, self.up.weight))
         gu = self.up(x)
         if self.gated and self.selective_recompute and torch.is_grad_enabled():
             # selective activation checkpointing: the SwiGLU product is recomputed in backward

@@ -440,6 +440,65 @@ def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     return F.linear(x, w)
 
 
+def _wgrad(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
+    """dyT x, accumulated straight into ``w.main_grad`` where there is one (then None is returned)."""
+    mg = getattr(w, "main_grad", None)
+    if mg is None:
+        return gemm_raw(dy, x, a_mn=True, b_mn=True)
+    fresh = getattr(w, "_main_grad_fresh", False)
+    gemm_raw(dy, x, a_mn=True, b_mn=True, out=mg, accumulate=not fresh)
+    w._main_grad_fresh = False
+    cb = getattr(w, "_grad_ready_cb", None)
+    if cb is not None:
+        cb(w)
+    return None
+
+
+def _gemm_swiglu(x: torch.Tensor, w: torch.Tensor, keep: bool) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
+    M, K = x.shape
+    Fd = w.shape[0] // 2
+    act = torch.empty(M, Fd, dtype=x.dtype, device=x.device)
+    gu = torch.empty(M, 2 * Fd, dtype=x.dtype, device=x.device) if keep else None
+    native.call("llmctl_gemm_swiglu_bf16", x.data_ptr(), w.data_ptr(), native.ptr(gu), act.data_ptr(), M, Fd, K, x.stride(0), w.stride(0),
+                2 * Fd, Fd, native.stream_ptr())
+    return act, gu
+
+
+class _LinearSwiGLUFn(torch.autograd.Function):
+    """``swiglu(x @ w.T)`` in one kernel; ``gate_up`` is written beside the product only for the backward."""
+
+    @staticmethod
+    def forward(ctx, x, w):
+        act, gu = _gemm_swiglu(x, w, any(ctx.needs_input_grad))
+        ctx.save_for_backward(x, w, gu)
+        return act
+
+    @staticmethod
+    def backward(ctx, dact):
+        x, w, gu = ctx.saved_tensors
+        M, F2 = gu.shape
+        dact = dact.contiguous()
+        dgu = torch.empty_like(gu)
+        native.call("llmctl_swiglu_bwd", dact.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, F2 // 2, gu.stride(0), native.stream_ptr())
+        dx = gemm_raw(dgu, w, b_mn=True) if ctx.needs_input_grad[0] else None
+        dw = _wgrad(dgu, x, w) if ctx.needs_input_grad[1] else None
+        return dx, dw
+
+
+def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """``swiglu(x @ w.T)`` for a packed ``w`` [2F, K] (gate rows first).  Native bf16 products of more than the decode GEMM's rows
+    run as one kernel; everything else composes ``linear`` and ``swiglu``."""
+    if (_use_native(x, "gemm") and _cfg.elementwise == "native" and _cfg.gemm_tile_n == 0 and w.dtype == torch.bfloat16
+            and getattr(w, "_k8_gate", None) is None and w.shape[0] % 16 == 0):
+        shape = x.shape
+        x2 = x.reshape(-1, shape[-1])
+        if not _gemm_ok(x2):
+            x2 = x2.contiguous()
+        if x2.shape[0] > SKINNY_MAX_ROWS and _gemm_ok(x2, w) and native.has_symbol("llmctl_gemm_swiglu_bf16"):
+            return native.apply(_LinearSwiGLUFn, x2, w).view(*shape[:-1], w.shape[0] // 2)
+    return swiglu(linear(x, w))
+
+
 class _SwiGLULinearFn(torch.autograd.Function):
     """``swiglu(gate_up) @ w.T`` that stores only ``gate_up``: the SwiGLU product (the down-projection's input,
     tokens x ffn) is recomputed in backward.  This is the "selective" activation-checkpointing policy."""

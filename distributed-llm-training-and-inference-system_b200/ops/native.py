@@ -43,6 +43,7 @@ _SIGNATURES = {
     "llmctl_cross_entropy_finalize": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_ll, c_ll, c_float, c_void_p, c_void_p],
     "llmctl_gemm_bf16": [c_void_p] * 3 + [c_int] * 3 + [c_ll] * 3 + [c_int] * 6 + [c_void_p],
     "llmctl_gemm_bf16_bgated": [c_void_p] * 3 + [c_int] * 3 + [c_ll] * 3 + [c_int] * 6 + [c_void_p, ctypes.c_uint, c_ll, c_ll, c_void_p],
+    "llmctl_gemm_swiglu_bf16": [c_void_p] * 4 + [c_int] * 3 + [c_ll] * 4 + [c_void_p],
     "llmctl_gemm_skinny_bf16": [c_void_p] * 3 + [c_int] * 3 + [c_ll] * 3 + [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p],
 }
 
@@ -131,6 +132,7 @@ _tracing_state = torch._C._get_tracing_state
 
 class _NoContext:
     """Stands in for an autograd context where nothing is recorded: keeps what the forward sets on it and saves nothing."""
+    needs_input_grad = ()
 
     def save_for_backward(self, *tensors) -> None:
         pass

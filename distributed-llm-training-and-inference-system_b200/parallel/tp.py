@@ -152,6 +152,10 @@ class ColumnParallelLinear(nn.Module):
         self.weight.tp_packed = packed      # rows are `packed` equal groups (q|k|v, gate|up), each sharded
         self.fused_name = fused_name
 
+    def runs_plain(self) -> bool:
+        """Whether the layer is its matrix product and nothing else: one rank, no hooks that a fused caller would pass by."""
+        return get_state().tp == 1 and not (self._forward_hooks or self._forward_pre_hooks or self._backward_hooks or self._backward_pre_hooks)
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         st = get_state()
         if st.tp > 1:

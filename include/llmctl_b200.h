@@ -106,6 +106,10 @@ int llmctl_sample(const void* logits, int logits_is_fp32, long long ld, int rows
                   const float* temperature, const int* top_k, const float* top_p, const float* uniform,
                   long long* out_token, float* out_logprob, void* stream);
 
+/* ACT[M,F] = silu(X Wg^T) * (X Wu^T), W [2F,K] = [Wg ; Wu]; GU [M,2F] = the two products, or NULL. */
+int llmctl_gemm_swiglu_bf16(const void* X, const void* W, void* GU, void* ACT, int M, int F, int K, long long ldx, long long ldw,
+                            long long ldgu, long long ldact, void* stream);
+
 /* ---- K0s skinny (decode) GEMM: C[Mb,N] = X[Mb,K] W[N,K]^T, 1 <= Mb <= 32.  Swap-AB (UMMA M = 128 weight rows,
  * N = 16/32 token rows), split-K over CTAs with a deterministic in-kernel fix-up.  workspace: fp32 scratch;
  * counters: >= ceil(N/128) zeroed uint32 tickets (left zero on return); one call at a time per pair.

@@ -270,6 +270,30 @@ def test_gemm_automatic_tiles(cuda_device, M, N, K, a_mn, b_mn):
         assert (out.double() - 2 * want).norm() <= 2 * bound * (2 * want).norm()
 
 
+# Rows around the decode GEMM's 32 and the tiles of 128 / 256, gate columns around 64 / 128, both tile kernels, ragged K
+@pytest.mark.parametrize("M,F_,K", [(32, 64, 64), (33, 8, 72), (129, 136, 200), (1000, 2048, 768), (300, 5632, 264), (2560, 1032, 128)])
+def test_linear_swiglu(cuda_device, M, F_, K):
+    """Forward and gradients against float64 of the same bf16 inputs.  Forward: one rounding of the output (the composed path rounds
+    gate and up too); backward: gate, up, their gradients and the results are rounded to bf16, 2^-9 each."""
+    from llmctl_b200.ops import functional as ops, native
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device=cuda_device).bfloat16().requires_grad_(True)
+    w = (torch.randn(2 * F_, K, device=cuda_device) / K ** 0.5).bfloat16().requires_grad_(True)
+    dy = torch.randn(M, F_, device=cuda_device).bfloat16()
+    before = native.launch_count
+    y = ops.linear_swiglu(x, w)
+    assert native.launch_count == before + (1 if M > 32 else 2)
+    dx, dw = torch.autograd.grad(y, (x, w), dy)
+    with torch.no_grad():
+        assert (ops.linear_swiglu(x, w).double() - y.double()).norm() <= 2.0 ** -8 * y.double().norm()
+    xd, wd = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    g, u = (xd @ wd.t()).chunk(2, -1)
+    want = F.silu(g) * u
+    gx, gw = torch.autograd.grad(want, (xd, wd), dy.double())
+    assert (y.double() - want).norm() <= (2.0 ** -9 if M > 32 else 2.0 ** -7.5) * want.norm()
+    assert (dx.double() - gx).norm() <= 2.0 ** -7 * gx.norm() and (dw.double() - gw).norm() <= 2.0 ** -7 * gw.norm()
+
+
 @pytest.mark.parametrize("B,S,H", [(2, 512, 4), (1, 2048, 2), (3, 128, 1), (1, 1024, 8)])
 @pytest.mark.parametrize("packed", [True, False])
 def test_flash_attention_fwd(cuda_device, B, S, H, packed):
