@@ -203,9 +203,10 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   };
   // the k-th item of this CTA, as the TMA warp published it; false when a wait ran out or there is none left
   auto next_item = [&](uint32_t k, int& item) {
-    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar.item_full[k % kQueue], (k / kQueue) & 1u, abort))) return false;
+    mbar_wait_or_abort(&bar.item_full[k % kQueue], (k / kQueue) & 1u, abort);
+    __syncwarp();
     item = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&bar.item[k % kQueue]), 0);
-    return item < n_items;
+    return item < n_items && !*abort;
   };
 
   if (warp == 0) {
@@ -278,8 +279,11 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     constexpr uint32_t id_acc = make_idesc_bf16(kBlk, D, 0u, 1u);      // A from TMEM, B MN-major
     const uint64_t kRes0 = make_smem_desc(smem_base, 16, 1024, 2), kRes1 = make_smem_desc(smem_base + C::kTile, 16, 1024, 2);
     auto tile_at = [&](uint32_t e) { return smem_base + (2 + e % C::kSlots) * C::kTile; };
-    auto wait = [&](uint64_t* b, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(b, parity, abort)) != 0; };
-    auto arrived = [&](uint32_t e) { return wait(&bar.full[e % C::kSlots], (e / C::kSlots) & 1u); };
+    auto wait = [&](uint64_t* b, uint32_t parity) {
+      mbar_wait_or_abort(b, parity, abort);
+      __syncwarp();
+    };
+    auto arrived = [&](uint32_t e) { wait(&bar.full[e % C::kSlots], (e / C::kSlots) & 1u); };
     // scores: 16 of the D columns per instruction, a panel of 64 columns every fourth
     auto issue_scores = [&](uint32_t t, uint64_t res, uint32_t sub) {
       const uint64_t b0 = make_smem_desc(sub, 16, 1024, 2);
@@ -302,18 +306,17 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     uint32_t g = 0, k = 0;
     auto run = [&](auto kind, int n) {
       constexpr bool kDQ = decltype(kind)::value;
-      bool ok = true;
-      for (int i = 0; ok && i < n; ++i, ++g) {
+      for (int i = 0; i < n; ++i, ++g) {
         const uint32_t e0 = 2 * g, e1 = e0 + 1;            // this block's streamed tiles; the next block's are e0 + 2, e1 + 2
         const uint32_t fresh = i == 0 ? 1u : 0u;
         if (i == 0) {
-          if (!(ok = arrived(e0))) break;
+          arrived(e0);
           tc_fence_after();
           if (elect_one()) {
             issue_scores(tS, kRes0, tile_at(e0));
             umma_commit<1>(&bar.s);
           }
-          if (!(ok = arrived(e1))) break;
+          arrived(e1);
           tc_fence_after();
           if (elect_one()) {
             issue_scores(tdP, kRes1, tile_at(e1));
@@ -323,12 +326,12 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
           }
         }
         if (!kDQ) {
-          if (!(ok = wait(&bar.p[0], g & 1u))) break;      // half of P(g) is written
-          if (i == 0 && k > 0 && !(ok = wait(&bar.accfree[0], (k - 1) & 1u))) break;
+          wait(&bar.p[0], g & 1u);      // half of P(g) is written
+          if (i == 0 && k > 0) wait(&bar.accfree[0], (k - 1) & 1u);
           tc_fence_after();
           if (elect_one()) issue_acc(tAcc0, tS, tile_at(e1), fresh, 0);              // dV += P^T dO
         }
-        if (!(ok = wait(&bar.p[1], g & 1u))) break;        // P(g) written (dKV) / S(g) read (dQ)
+        wait(&bar.p[1], g & 1u);        // P(g) written (dKV) / S(g) read (dQ)
         tc_fence_after();
         if (!kDQ && elect_one()) {
           issue_acc(tAcc0, tS, tile_at(e1), 0, 1);
@@ -336,15 +339,15 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
           if (i + 1 == n) umma_commit<1>(&bar.acc[0]);
         }
         if (i + 1 < n) {
-          if (!(ok = arrived(e0 + 2))) break;
+          arrived(e0 + 2);
           tc_fence_after();
           if (elect_one()) {
             issue_scores(tS, kRes0, tile_at(e0 + 2));
             umma_commit<1>(&bar.s);
           }
         }
-        if (!(ok = wait(&bar.ds, g & 1u))) break;
-        if (i == 0 && k > 0 && !(ok = wait(&bar.accfree[kDQ ? 0 : 1], (k - 1) & 1u))) break;
+        wait(&bar.ds, g & 1u);
+        if (i == 0 && k > 0) wait(&bar.accfree[kDQ ? 0 : 1], (k - 1) & 1u);
         tc_fence_after();
         if (elect_one()) {
           issue_acc(kDQ ? tAcc0 : tAcc1, tdP, tile_at(e0), fresh, 2);    // dK += dS^T Q  /  dQ += dS K
@@ -355,7 +358,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
           }
         }
         if (i + 1 < n) {
-          if (!(ok = arrived(e1 + 2))) break;
+          arrived(e1 + 2);
           tc_fence_after();
           if (elect_one()) {
             issue_scores(tdP, kRes1, tile_at(e1 + 2));
@@ -365,15 +368,13 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
           }
         }
       }
-      return ok;
     };
-    bool ok = true;
-    for (int item; ok && next_item(k, item); ++k) {
+    for (int item; next_item(k, item); ++k) {
       bool is_dq;
       int rb, bh, first, n;
       decode(item, is_dq, rb, bh, first, n);
-      ok = wait(&bar.res, k & 1u);
-      if (ok) ok = is_dq ? run(DQ{}, n) : run(DKV{}, n);
+      wait(&bar.res, k & 1u);
+      if (is_dq) run(DQ{}, n); else run(DKV{}, n);
     }
   } else if (warp < 10) {
     // ------------------- softmax / dS warpgroups: half wg of the streamed columns, all 128 resident rows -------------------
@@ -385,7 +386,6 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     uint32_t g = 0, k = 0;
     auto run = [&](auto kind, int rb, int bh, int first, int n) {
       constexpr bool kDQ = decltype(kind)::value;
-      bool ok = true;
       float row_nl = 0.f, row_nd = 0.f;                   // dQ kernel: this query row's statistics
       if (kDQ) {
         row_nl = nl2[static_cast<long long>(bh) * Sp + rb * kBlk + row];
@@ -397,9 +397,9 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         const bool diag = causal && first + i == rb;
         // columns a row may see on the diagonal block: dKV key `row` <= query, dQ key <= query `row`
         const int edge = row - wg * 64;
-        ok = (kDQ || mbar_wait_bounded(&bar.full[e1 % C::kSlots], (e1 / C::kSlots) & 1u, abort)) && mbar_wait_bounded(&bar.s, g & 1u, abort);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+        if (!kDQ) mbar_wait_or_abort(&bar.full[e1 % C::kSlots], (e1 / C::kSlots) & 1u, abort);
+        mbar_wait_or_abort(&bar.s, g & 1u, abort);
+        __syncwarp();
         tc_fence_after();
         uint32_t rs[64];
         tmem_ld_x32(tSb, rs);
@@ -453,8 +453,8 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
             }
           }
         }
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar.dp, g & 1u, abort));
-        if (!ok) break;
+        mbar_wait_or_abort(&bar.dp, g & 1u, abort);
+        __syncwarp();
         tc_fence_after();
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
@@ -485,14 +485,12 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar.ds);
       }
-      return ok;
     };
-    bool ok = true;
-    for (int item; ok && next_item(k, item); ++k) {
+    for (int item; next_item(k, item); ++k) {
       bool is_dq;
       int rb, bh, first, n;
       decode(item, is_dq, rb, bh, first, n);
-      ok = is_dq ? run(DQ{}, rb, bh, first, n) : run(DKV{}, rb, bh, first, n);
+      if (is_dq) run(DQ{}, rb, bh, first, n); else run(DKV{}, rb, bh, first, n);
     }
   } else {
     // ------------- epilogue warpgroup: accumulators -> registers -> bf16 -> global, a row per thread -------------
@@ -500,8 +498,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     const int row = q4 * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(q4 * 32) << 16;
     uint32_t k = 0;
-    bool ok = true;
-    for (int item; ok && next_item(k, item); ++k) {
+    for (int item; next_item(k, item); ++k) {
       bool is_dq;
       int rb, bh, first, n;
       decode(item, is_dq, rb, bh, first, n);
@@ -509,8 +506,8 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
       const long long at = (static_cast<long long>(bh / H) * S + rb * kBlk + row) * out_tok + (bh % H) * D;
 #pragma unroll 1
       for (int a = 0; a < 2; ++a) {                       // dKV: dV from acc0, then scale * dK from acc1.  dQ: scale * dQ from acc0.
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar.acc[a], k & 1u, abort));
-        if (!ok) break;
+        mbar_wait_or_abort(&bar.acc[a], k & 1u, abort);
+        __syncwarp();
         if (is_dq && a == 1) {                            // nothing there
           if (lane == 0) mbar_arrive(&bar.accfree[1]);
           break;

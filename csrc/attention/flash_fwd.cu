@@ -229,7 +229,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // longest of every round (S = 2048, 40 heads x 2: 40 instead of 48 blocks on the busiest CTA, 39 on average).
   auto next_item = [&](int r, int& item) {
     item = r * gridDim.x + ((r & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
-    return item < n_items;
+    return item < n_items && !*abort;
   };
   // item -> (first query, head, batch, sequence); heavy (late) query blocks first so the tail is made of light items.
   // False: a shorter sequence of the batch has no such block.
@@ -304,7 +304,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       }
       // Copies still in flight when a wait ran out land before the CTA's shared memory is given back.
-      if (!ok) {
+      if (*abort) {
         int none = 0;
         if (nA > 0) mbar_wait_bounded(&bar_q[0], (nA - 1) & 1u, &none);
         none = 0;
@@ -328,12 +328,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // addresses and descriptors stay in uniform registers, which the instruction reads.
     constexpr uint32_t idesc_qk = make_idesc_bf16(kRows, kRows, 0u, 0u);   // A, B K-major
     constexpr uint32_t idesc_pv = make_idesc_bf16(kRows, DV, 0u, 1u);      // A from TMEM, B MN-major (V)
-    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort)) != 0; };
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      mbar_wait_or_abort(bar, parity, abort);
+      __syncwarp();
+    };
     uint32_t g0 = 0;                 // K/V blocks consumed by earlier items
     uint32_t nQ0 = 0, nQ1 = 0;       // items done per tile (Q / O barrier phases)
     uint32_t nP0 = 0, nP1 = 0;       // P V products issued per tile (bar_p phases)
-    bool ok = true;
-    for (int item, r = 0; ok && next_item(r, item); ++r) {
+    for (int item, r = 0; next_item(r, item); ++r) {
       int q0, head, b;
       Seq sq;
       if (!decode(item, q0, head, b, sq)) continue;
@@ -341,7 +343,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int nblk = max(nblk_t0, nblk_t1);
       auto issue_qk = [&](int t, int j, bool release_k, bool last) {
         const uint32_t g = g0 + j, st = g % C::kKStages;
-        if (!wait(&bar_kfull[st], (g / C::kKStages) & 1u)) return false;
+        wait(&bar_kfull[st], (g / C::kKStages) & 1u);
         tc_fence_after();
         const uint64_t qd = make_smem_desc(smem_base + t * C::kQTile, 16, 1024, 2);
         const uint64_t kd = make_smem_desc(smem_base + C::kKAt + st * C::kQTile, 16, 1024, 2);
@@ -355,14 +357,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (release_k) umma_commit<1>(&bar_kempty[st]);
           if (last) umma_commit<1>(&bar_qfree[t]);       // last use of this item's Q_t
         }
-        return true;
       };
       // P V of tile t and block j, then Q K^T of its block j + 1
       auto step = [&](int t, int j, int mine, int other, uint32_t nQ, uint32_t nP) {
         const uint32_t vs = (g0 + j) % C::kVStages;
-        if (!wait(&bar_vfull[vs], ((g0 + j) / C::kVStages) & 1u)) return false;
-        if (!wait(&bar_p0[t], nP & 1u)) return false;    // first half of P_t(j) is in TMEM, O_t rescaled if needed
-        if (j == 0 && nQ > 0 && !wait(&bar_ofree[t], (nQ - 1) & 1u)) return false;   // previous item's O_t was read out
+        wait(&bar_vfull[vs], ((g0 + j) / C::kVStages) & 1u);
+        wait(&bar_p0[t], nP & 1u);                       // first half of P_t(j) is in TMEM, O_t rescaled if needed
+        if (j == 0 && nQ > 0) wait(&bar_ofree[t], (nQ - 1) & 1u);                    // previous item's O_t was read out
         tc_fence_after();
         const uint64_t vd = make_smem_desc(smem_base + C::kVAt + vs * C::kVTile, kPanel, 1024, 2);
         const uint32_t tP = tmem_base + t * 128;
@@ -372,7 +373,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           for (int ks = 0; ks < kRows / 32; ++ks)
             umma_ts<1>(tOt, tP + ks * 8, vd + ks * (2048 >> 4), idesc_pv, (j | ks) != 0 ? 1u : 0u);
         }
-        if (!wait(&bar_p1[t], nP & 1u)) return false;
+        wait(&bar_p1[t], nP & 1u);
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -381,13 +382,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (t == 1 || j >= other) umma_commit<1>(&bar_vempty[vs]);    // last reader of V(j)
           if (j + 1 == mine) umma_commit<1>(&bar_o[t]);
         }
-        return j + 1 < mine ? issue_qk(t, j + 1, t == 1 || j + 1 >= other, j + 2 == mine) : true;
+        if (j + 1 < mine) issue_qk(t, j + 1, t == 1 || j + 1 >= other, j + 2 == mine);
       };
-      if (!(ok = wait(&bar_q[0], nQ0 & 1u) && issue_qk(0, 0, nblk_t1 == 0, nblk_t0 == 1))) break;
-      if (nblk_t1 > 0 && !(ok = wait(&bar_q[1], nQ1 & 1u) && issue_qk(1, 0, true, nblk_t1 == 1))) break;
-      for (int j = 0; ok && j < nblk; ++j) {
-        if (j < nblk_t0) ok = step(0, j, nblk_t0, nblk_t1, nQ0, nP0++);
-        if (ok && j < nblk_t1) ok = step(1, j, nblk_t1, nblk_t0, nQ1, nP1++);
+      wait(&bar_q[0], nQ0 & 1u);
+      issue_qk(0, 0, nblk_t1 == 0, nblk_t0 == 1);
+      if (nblk_t1 > 0) {
+        wait(&bar_q[1], nQ1 & 1u);
+        issue_qk(1, 0, true, nblk_t1 == 1);
+      }
+      for (int j = 0; j < nblk; ++j) {
+        if (j < nblk_t0) step(0, j, nblk_t0, nblk_t1, nQ0, nP0++);
+        if (j < nblk_t1) step(1, j, nblk_t1, nblk_t0, nQ1, nP1++);
       }
       g0 += nblk;
       ++nQ0;
@@ -405,8 +410,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t tOt = tmem_base + 256 + t * 128 + lane_off;
     uint32_t nS = 0;                               // S tiles consumed so far (bar_s phase)
     uint32_t nO = 0;                               // items finished by this tile (bar_o phase)
-    bool ok = true;
-    for (int item, r = 0; ok && next_item(r, item); ++r) {
+    for (int item, r = 0; next_item(r, item); ++r) {
       int q0, head, b;
       Seq sq;
       if (!decode(item, q0, head, b, sq)) continue;
@@ -415,8 +419,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int qt0 = q0 + t * kRows;
       float m_ref = -INFINITY, l0 = 0.f, l1 = 0.f;
       for (int j = 0; j < nb; ++j, ++nS) {
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_s[t], nS & 1u, abort));
-        if (!ok) break;
+        mbar_wait_or_abort(&bar_s[t], nS & 1u, abort);
+        __syncwarp();
         tc_fence_after();
         if (q == 0 && lane == 0) ev(t, 1);
         const int off = sq.start + qt0 - j * kRows;      // the tile's first row sees the block's columns up to this one
@@ -426,10 +430,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           softmax_block<false, DV>(tS, tOt, q, lane, off, j == 0, scale_log2, m_ref, l0, l1, &bar_p0[t], &bar_p1[t]);
         if (q == 0 && lane == 0) ev(t, 2);
       }
-      if (!ok) break;
       // ---- epilogue: O / l -> bf16 -> global (row per thread, whole 32-byte sectors), LSE ----
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_o[t], nO & 1u, abort));
-      if (!ok) break;
+      mbar_wait_or_abort(&bar_o[t], nO & 1u, abort);
+      __syncwarp();
       ++nO;
       tc_fence_after();
       const float l = l0 + l1;

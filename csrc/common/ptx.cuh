@@ -94,6 +94,26 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// The same for warps that must not vote on the outcome: when the wait runs out (or another role gave up) the flag is raised and the
+// caller goes on with what is there.  Its loops are counted, its accesses do not depend on the data, and it leaves at the next
+// item.  (A vote and a branch after every wait cost an issuing warp a third of its time: 2116 against 1200 clocks for the waits of two
+// attention tiles.)
+__device__ __forceinline__ void mbar_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort) {
+  uint32_t n = 0;
+  long long t0 = 0;
+  while (!mbar_try_wait(bar, parity)) {
+    if ((++n & 255u) == 0u) {
+      if (*abort) return;
+      const long long t = clock64();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > kBoundedWaitCycles) {
+        *abort = 1;
+        return;
+      }
+    }
+  }
+}
+
 // ----------------------------------------------------------------------------------------------
 // TMA
 // ----------------------------------------------------------------------------------------------
