@@ -207,9 +207,12 @@ __device__ __forceinline__ void gemm_epilogue(uint32_t t_row, uint8_t* out_smem,
 
 // Gated up-projection (llmctl_gemm_swiglu_bf16): the tile's first half of columns multiplies rows of the gate matrix, the second half the
 // same rows of the up matrix, and the epilogue stores silu(gate) * up, and gate and up beside it when the backward will want them.
+enum class Gated { kNone, kForward, kBackward };
 struct SwigluMaps {
   CUtensorMap w_up, gate, up, act;
   int keep;                  // gate and up are stored
+  const __nv_bfloat16* gu;   // backward: gate | up as the forward left them; `gate` and `up` take their gradients
+  long long ldgu;
 };
 template <int BN>
 __device__ __forceinline__ void swiglu_epilogue(uint32_t t_row, uint8_t* out_smem, uint32_t& out_n, const SwigluMaps& maps, int row0, int f0,
@@ -237,7 +240,75 @@ __device__ __forceinline__ void swiglu_epilogue(uint32_t t_row, uint8_t* out_sme
   }
 }
 
-template <int BN, bool A_MN, bool B_MN, typename OutT, bool kSwiglu = false>
+// Gradient of the gated activation (llmctl_gemm_swiglu_bwd_bf16): the tile is dL/d(silu(gate) * up).  Gate and up come in whole lines, eight
+// lanes to a row, one box of 64 columns ahead of its use, and turn to a row per lane in the warp's staging buffers, where their gradients
+// replace them.  All of it passes beside the main loop of the next tile, which it must not outlast: read a row per lane straight from
+// global memory (32 lines per load) the 4096 x 5632 x 2048 problem took 94 us, with an IEEE reciprocal on top of that 146.
+template <int BN>
+__device__ __forceinline__ void swiglu_bwd_epilogue(uint32_t t_row, uint8_t* out_smem, const SwigluMaps& maps, int row0, int f0, int M, int F,
+                                                    int lane) {
+  uint4 g[8], u[8];
+  const int sub = lane >> 3, part = lane & 7;
+  auto fetch = [&](int c) {
+    const int col = f0 + c * 64 + part * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = row0 + 4 * i + sub;
+      g[i] = u[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (row < M && col < F) {
+        const __nv_bfloat16* src = maps.gu + static_cast<long long>(row) * maps.ldgu + col;
+        g[i] = *reinterpret_cast<const uint4*>(src);
+        u[i] = *reinterpret_cast<const uint4*>(src + F);
+      }
+    }
+  };
+  uint8_t *gs = out_smem, *us = out_smem + kOutBox;
+  fetch(0);
+#pragma unroll 1
+  for (int c = 0; c < BN / 64; ++c) {
+    const int col = f0 + c * 64;
+    if (row0 >= M || col >= F) break;                  // uniform over the warp
+    if (lane == 0) tma_store_wait_read<0>();
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 4 * i + sub, at = row * 128 + ((part ^ (row & 7)) << 4);
+      *reinterpret_cast<uint4*>(gs + at) = g[i];
+      *reinterpret_cast<uint4*>(us + at) = u[i];
+    }
+    __syncwarp();
+    if (c + 1 < BN / 64) fetch(c + 1);
+    uint32_t r[64];
+    tmem_ld_x32(t_row + c * 64, r);
+    tmem_ld_x32(t_row + c * 64 + 32, r + 32);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int at = lane * 128 + ((j ^ (lane & 7)) << 4);
+      float gv[8], uv[8];
+      unpack8(*reinterpret_cast<const bf16x8*>(gs + at), gv);
+      unpack8(*reinterpret_cast<const bf16x8*>(us + at), uv);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float d = __uint_as_float(r[8 * j + e]);
+        const float sig = __fdividef(1.f, 1.f + __expf(-gv[e])), silu = gv[e] * sig;
+        gv[e] = d * uv[e] * (sig + silu * (1.f - sig));
+        uv[e] = d * silu;
+      }
+      *reinterpret_cast<bf16x8*>(gs + at) = pack8(gv);
+      *reinterpret_cast<bf16x8*>(us + at) = pack8(uv);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(&maps.gate, gs, col, row0);
+      tma_store_2d(&maps.up, us, col, row0);
+      tma_store_commit();
+    }
+  }
+}
+
+template <int BN, bool A_MN, bool B_MN, typename OutT, Gated kGated = Gated::kNone>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate,
@@ -256,6 +327,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int lane = threadIdx.x & 31;
 
   const int num_m = (M + kBM - 1) / kBM;
+  constexpr bool kSwiglu = kGated == Gated::kForward;
   constexpr int kCols = kSwiglu ? BN / 2 : BN;         // output columns per tile; with the gate N counts those of one half
   const int num_n = (N + kCols - 1) / kCols;
   const int num_tiles = num_m * num_n;
@@ -387,6 +459,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
       if constexpr (kSwiglu)
         swiglu_epilogue<BN>(t_row, out_smem, out_n, sw, m0 + q * 32, n0, M, N, lane);
+      else if constexpr (kGated == Gated::kBackward)
+        swiglu_bwd_epilogue<BN>(t_row, out_smem, sw, m0 + q * 32, n0, M, N, lane);
       else
         gemm_epilogue<BN, OutT>(t_row, out_smem, out_n, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
@@ -432,7 +506,7 @@ struct Gemm2Cfg {
   static constexpr int kTmemCols = 2 * PBN;              // 512 / 256
 };
 
-template <int PBN, bool A_MN, bool B_MN, typename OutT, bool kSwiglu = false>
+template <int PBN, bool A_MN, bool B_MN, typename OutT, Gated kGated = Gated::kNone>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate,
@@ -455,6 +529,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   const int num_pairs = gridDim.x >> 1;
 
   const int num_m = (M + 2 * kBM - 1) / (2 * kBM);
+  constexpr bool kSwiglu = kGated == Gated::kForward;
   constexpr int kCols = kSwiglu ? BN / 2 : BN;         // output columns per tile; with the gate N counts those of one half
   const int num_n = (N + kCols - 1) / kCols;
   const int num_tiles = num_m * num_n;
@@ -578,6 +653,8 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
       if constexpr (kSwiglu)
         swiglu_epilogue<BN>(t_row, out_smem, out_n, sw, m0 + q * 32, n0, M, N, lane);
+      else if constexpr (kGated == Gated::kBackward)
+        swiglu_bwd_epilogue<BN>(t_row, out_smem, sw, m0 + q * 32, n0, M, N, lane);
       else
         gemm_epilogue<BN, OutT>(t_row, out_smem, out_n, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
@@ -711,12 +788,12 @@ static int launch_swiglu(const void* X, const void* W, void* GU, void* ACT, int 
   if (rc) LLMCTL_FAIL(rc, "tensor maps");
   const int tiles = ((M + (kPair ? 2 : 1) * kBM - 1) / ((kPair ? 2 : 1) * kBM)) * ((F + kCols - 1) / kCols);
   if constexpr (kPair) {
-    auto kern = gemm2_tcgen05_kernel<256, false, false, __nv_bfloat16, true>;
+    auto kern = gemm2_tcgen05_kernel<256, false, false, __nv_bfloat16, Gated::kForward>;
     LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256>::kSmemBytes));
     const int pairs = tiles < num_sms() / 2 ? tiles : num_sms() / 2;
     kern<<<2 * pairs, kGemmThreads, Gemm2Cfg<256>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0, GemmGate{}, sw);
   } else {
-    auto kern = gemm_tcgen05_kernel<128, false, false, __nv_bfloat16, true>;
+    auto kern = gemm_tcgen05_kernel<128, false, false, __nv_bfloat16, Gated::kForward>;
     LLMCTL_CHECK(allow_smem(kern, GemmCfg<128>::kSmemBytes));
     kern<<<tiles < num_sms() ? tiles : num_sms(), kGemmThreads, GemmCfg<128>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0,
                                                                                             GemmGate{}, sw);
@@ -724,9 +801,47 @@ static int launch_swiglu(const void* X, const void* W, void* GU, void* ACT, int 
   LLMCTL_RETURN_LAST();
 }
 
+// kBN: 64 or 128 (one CTA), 256 (CTA pair).
+template <int kBN>
+static int launch_swiglu_bwd(const void* DY, const void* W, const void* GU, void* DGU, int M, int F, int K, long long lddy, long long ldw,
+                             long long ldgu, cudaStream_t s) {
+  constexpr bool kPair = kBN == 256;
+  constexpr int kRows = (kPair ? 2 : 1) * kBM;
+  CUtensorMap tmA, tmW;
+  SwigluMaps sw;
+  int rc = get_tmap_2d_bf16(&tmA, DY, M, K, lddy, kBM, kBK, 1);
+  if (!rc) rc = get_tmap_2d_bf16(&tmW, W, K, F, ldw, kBK, 64, 1);
+  if (!rc) rc = get_tmap_2d_bf16(&sw.gate, DGU, M, F, ldgu, 32, 64, 1);
+  if (!rc) rc = get_tmap_2d_bf16(&sw.up, (const __nv_bfloat16*)DGU + F, M, F, ldgu, 32, 64, 1);
+  if (rc) LLMCTL_FAIL(rc, "tensor maps");
+  sw.w_up = sw.act = sw.gate;
+  sw.keep = 0;
+  sw.gu = (const __nv_bfloat16*)GU;
+  sw.ldgu = ldgu;
+  const int tiles = ((M + kRows - 1) / kRows) * ((F + kBN - 1) / kBN), most = kPair ? num_sms() / 2 : num_sms();
+  const int grid = tiles < most ? tiles : most;
+  if constexpr (kPair) {
+    auto kern = gemm2_tcgen05_kernel<256, false, true, __nv_bfloat16, Gated::kBackward>;
+    LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256>::kSmemBytes));
+    kern<<<2 * grid, kGemmThreads, Gemm2Cfg<256>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw);
+  } else {
+    auto kern = gemm_tcgen05_kernel<kBN, false, true, __nv_bfloat16, Gated::kBackward>;
+    LLMCTL_CHECK(allow_smem(kern, GemmCfg<kBN>::kSmemBytes));
+    kern<<<grid, kGemmThreads, GemmCfg<kBN>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw);
+  }
+  LLMCTL_RETURN_LAST();
+}
+
 }  // namespace llmctl
 
 using namespace llmctl;
+
+// The narrowest tile with which the problem is still one wave (see gemm_bf16_impl), 0 if there is none.
+static int one_wave_tile(int M, int N) {
+  const long long rows = (M + 127) / 128, sms = num_sms();
+  if (rows * ((N + 63) / 64) <= sms) return 64;
+  return rows * ((N + 127) / 128) <= sms ? 128 : 0;
+}
 
 // D[M,N] = op(A) op(B) (+ D if beta).  a_mn / b_mn select the operand storage (see file header).
 // out_fp32: D is fp32 (else bf16).  tile_n: 0 = auto, 64 / 128 / 192 / 256 (1-CTA tiles), 2 = 256x256 CTA-pair tile, 3 = 256x128 CTA-pair tile.  max_ctas: 0 = all SMs
@@ -747,11 +862,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
   // Beyond one wave operand traffic from L2 sets the pace and the 256 x 256 CTA-pair tile moves least of it (4096 x 2048 x 2048:
   // 26.7 / 33.1 / 49.0, 4096 x 11264 x 2048: 130 / 181 / 276); 128 x 192 and pair 256 x 128 never win by more than a few per cent
   // and stay selectable (tile_n = 192 / 3).  Gated operands arrive slab by slab and keep the pair tile.
-  if (tile_n == 0 && g.flags == nullptr && g.b_flags == nullptr && max_ctas == 0) {
-    const long long rows = (M + 127) / 128, sms = num_sms();
-    if (rows * ((N + 63) / 64) <= sms) tile_n = 64;
-    else if (rows * ((N + 127) / 128) <= sms) tile_n = 128;
-  }
+  if (tile_n == 0 && g.flags == nullptr && g.b_flags == nullptr && max_ctas == 0) tile_n = one_wave_tile(M, N);
   if (tile_n == 0 && M > 128 && N > 128) tile_n = 2;
   if (tile_n == 2) {   // 2-CTA pair tile 256 x 256 (cta_group::2)
     if (out_fp32) return dispatch_layout2<256, float>(a_mn, b_mn, A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
@@ -805,6 +916,21 @@ LLMCTL_API int llmctl_gemm_swiglu_bf16(const void* X, const void* W, void* GU, v
                    reinterpret_cast<uintptr_t>(ACT)) & 15) == 0 && static_cast<long long>(ldact) >= F);
   const bool one_wave = static_cast<long long>((M + kBM - 1) / kBM) * ((F + 63) / 64) <= num_sms();
   return (one_wave || M <= 128 ? launch_swiglu<false> : launch_swiglu<true>)(X, W, GU, ACT, M, F, K, ldx, ldw, ldgu, ldact, (cudaStream_t)stream);
+}
+
+// DGU[M, 2F] = (d gate | d up) of a gated MLP from dy [M, K], the down-projection W [K, F] and the forward's GU [M, 2F] (row stride ldgu for
+// both): the product dy W is never stored.  Against the product and llmctl_swiglu_bwd it saves writing and reading M x F and a launch, and
+// the activation's arithmetic and traffic hide behind the products of the next tile (4096 x 5632 x 2048: 106 us
+// in two, 86 us in one; 16384 rows: 380 / 297; 1000 x 2048 x 2048: 25.6 / 23.4).
+LLMCTL_API int llmctl_gemm_swiglu_bwd_bf16(const void* DY, const void* W, const void* GU, void* DGU, int M, int F, int K, long long lddy,
+                                           long long ldw, long long ldgu, void* stream) {
+  LLMCTL_BEGIN();
+  LLMCTL_REQUIRE(M > 0 && F > 0 && K > 0 && F % 8 == 0 && lddy % 8 == 0 && ldw % 8 == 0 && ldgu % 8 == 0 && ldgu >= 2LL * F);
+  LLMCTL_REQUIRE(((reinterpret_cast<uintptr_t>(DY) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(GU) |
+                   reinterpret_cast<uintptr_t>(DGU)) & 15) == 0);
+  const int bn = one_wave_tile(M, F);
+  auto launch = bn == 64 ? launch_swiglu_bwd<64> : bn == 128 || M <= 128 || F <= 128 ? launch_swiglu_bwd<128> : launch_swiglu_bwd<256>;
+  return launch(DY, W, GU, DGU, M, F, K, lddy, ldw, ldgu, (cudaStream_t)stream);
 }
 
 // Grouped GEMM for mixture-of-experts layers: C[r, :] = A[r, :] W[expert(r)]^T over `max_tiles` blocks of 128 rows of A

@@ -82,6 +82,8 @@ class MLP(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if self.gated and not (self.selective_recompute and torch.is_grad_enabled()) and self.up.runs_plain():
+            if self.down.runs_plain():
+                return ops.swiglu_mlp(x, self.up.weight, self.down.weight)
             return self.down(ops.linear_swiglu(x, self.up.weight))
         gu = self.up(x)
         if self.gated and self.selective_recompute and torch.is_grad_enabled():

@@ -485,18 +485,70 @@ class _LinearSwiGLUFn(torch.autograd.Function):
         return dx, dw
 
 
-def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    """``swiglu(x @ w.T)`` for a packed ``w`` [2F, K] (gate rows first).  Native bf16 products of more than the decode GEMM's rows
-    run as one kernel; everything else composes ``linear`` and ``swiglu``."""
+# Columns of the down-projection from which the fused backward pays: its epilogue takes as long as ~1000 columns of products and hides
+# behind them (us in two launches / in one: 8192 x 3072 x 768 81 / 83, 4096 x 2816 x 1024 48 / 50, 8192 x 4096 x 1024 107 / 97,
+# 4096 x 4096 x 1536 73 / 66, 4096 x 5632 x 2048 106 / 86).
+SWIGLU_BWD_COLS = 1024
+
+
+class _SwiGLUMLPFn(torch.autograd.Function):
+    """``swiglu(x @ w_up.T) @ w_down.T``: the gradient of the product of the two halves goes straight into theirs."""
+
+    @staticmethod
+    def forward(ctx, x, w_up, w_down):
+        act, gu = _gemm_swiglu(x, w_up, True)
+        ctx.save_for_backward(x, w_up, w_down, gu, act)
+        return gemm_raw(act, w_down)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, w_up, w_down, gu, act = ctx.saved_tensors
+        if not _gemm_ok(dy):
+            dy = dy.contiguous()
+        dx = dw_up = dgu = None
+        if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
+            M, F2 = gu.shape
+            dgu = torch.empty_like(gu)
+            native.call("llmctl_gemm_swiglu_bwd_bf16", dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, F2 // 2, dy.shape[1],
+                        dy.stride(0), w_down.stride(0), gu.stride(0), native.stream_ptr())
+        dw_down = _wgrad(dy, act, w_down) if ctx.needs_input_grad[2] else None
+        if ctx.needs_input_grad[0]:
+            dx = gemm_raw(dgu, w_up, b_mn=True)
+        if ctx.needs_input_grad[1]:
+            dw_up = _wgrad(dgu, x, w_up)
+        return dx, dw_up, dw_down
+
+
+def _swiglu_rows(x: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
+    """``x`` as the rows of the kernel that multiplies by the packed gate | up ``w`` and activates, or None where it does not apply."""
     if (_use_native(x, "gemm") and _cfg.elementwise == "native" and _cfg.gemm_tile_n == 0 and w.dtype == torch.bfloat16
             and getattr(w, "_k8_gate", None) is None and w.shape[0] % 16 == 0):
-        shape = x.shape
-        x2 = x.reshape(-1, shape[-1])
+        x2 = x.reshape(-1, x.shape[-1])
         if not _gemm_ok(x2):
             x2 = x2.contiguous()
         if x2.shape[0] > SKINNY_MAX_ROWS and _gemm_ok(x2, w) and native.has_symbol("llmctl_gemm_swiglu_bf16"):
-            return native.apply(_LinearSwiGLUFn, x2, w).view(*shape[:-1], w.shape[0] // 2)
-    return swiglu(linear(x, w))
+            return x2
+    return None
+
+
+def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """``swiglu(x @ w.T)`` for a packed ``w`` [2F, K] (gate rows first).  Native bf16 products of more than the decode GEMM's rows
+    run as one kernel; everything else composes ``linear`` and ``swiglu``."""
+    x2 = _swiglu_rows(x, w)
+    if x2 is None:
+        return swiglu(linear(x, w))
+    return native.apply(_LinearSwiGLUFn, x2, w).view(*x.shape[:-1], w.shape[0] // 2)
+
+
+def swiglu_mlp(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor) -> torch.Tensor:
+    """``swiglu(x @ w_up.T) @ w_down.T``.  Where a gradient will be asked for and the width allows, the backward of the activation runs
+    inside the product that precedes it; everything else composes ``linear_swiglu`` and ``linear``."""
+    fused = w_down.shape[0] >= SWIGLU_BWD_COLS and torch.is_grad_enabled() and (x.requires_grad or w_up.requires_grad)
+    x2 = _swiglu_rows(x, w_up) if fused else None
+    if (x2 is None or w_down.dtype != torch.bfloat16 or getattr(w_down, "_k8_gate", None) is not None or w_down.shape[0] % 8
+            or not _gemm_ok(w_down)):
+        return linear(linear_swiglu(x, w_up), w_down)
+    return native.apply(_SwiGLUMLPFn, x2, w_up, w_down).view(*x.shape[:-1], w_down.shape[0])
 
 
 class _SwiGLULinearFn(torch.autograd.Function):

@@ -136,6 +136,11 @@ def _init_weight(shape, std, dtype, device, seed_offset: int = 0):
     return w
 
 
+def _runs_plain(layer: nn.Module) -> bool:
+    """Whether the layer is its matrix product and nothing else: one rank, no hooks that a fused caller would pass by."""
+    return get_state().tp == 1 and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks)
+
+
 class ColumnParallelLinear(nn.Module):
     """y_local = x @ W_local.T, W sharded on the output dim.  Input is replicated over TP, or — with
     sequence parallelism — sharded on tokens and all-gathered first."""
@@ -153,8 +158,7 @@ class ColumnParallelLinear(nn.Module):
         self.fused_name = fused_name
 
     def runs_plain(self) -> bool:
-        """Whether the layer is its matrix product and nothing else: one rank, no hooks that a fused caller would pass by."""
-        return get_state().tp == 1 and not (self._forward_hooks or self._forward_pre_hooks or self._backward_hooks or self._backward_pre_hooks)
+        return _runs_plain(self)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         st = get_state()
@@ -183,6 +187,9 @@ class RowParallelLinear(nn.Module):
         self.weight = nn.Parameter(_init_weight((out_features, self.in_local), std, dtype, device))
         self.weight.tp_shard_dim = 1
         self.fused_name = fused_name
+
+    def runs_plain(self) -> bool:
+        return _runs_plain(self)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         st = get_state()

@@ -109,6 +109,8 @@ int llmctl_sample(const void* logits, int logits_is_fp32, long long ld, int rows
 /* ACT[M,F] = silu(X Wg^T) * (X Wu^T), W [2F,K] = [Wg ; Wu]; GU [M,2F] = the two products, or NULL. */
 int llmctl_gemm_swiglu_bf16(const void* X, const void* W, void* GU, void* ACT, int M, int F, int K, long long ldx, long long ldw,
                             long long ldgu, long long ldact, void* stream);
+int llmctl_gemm_swiglu_bwd_bf16(const void* DY, const void* W, const void* GU, void* DGU, int M, int F, int K, long long lddy, long long ldw,
+                                long long ldgu, void* stream);
 
 /* ---- K0s skinny (decode) GEMM: C[Mb,N] = X[Mb,K] W[N,K]^T, 1 <= Mb <= 32.  Swap-AB (UMMA M = 128 weight rows,
  * N = 16/32 token rows), split-K over CTAs with a deterministic in-kernel fix-up.  workspace: fp32 scratch;

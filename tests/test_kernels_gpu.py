@@ -294,6 +294,33 @@ def test_linear_swiglu(cuda_device, M, F_, K):
     assert (dx.double() - gx).norm() <= 2.0 ** -7 * gx.norm() and (dw.double() - gw).norm() <= 2.0 ** -7 * gw.norm()
 
 
+# One-wave tiles of 64 and 128 columns and the pair tile, rows and columns that end inside a tile, ragged K
+@pytest.mark.parametrize("M,F_,K,N", [(33, 8, 64, 72), (200, 136, 264, 64), (1000, 2048, 768, 768), (2560, 1032, 128, 200), (2049, 5632, 64, 320)])
+def test_swiglu_mlp(cuda_device, monkeypatch, M, F_, K, N):
+    """Forward and gradients against float64 of the same bf16 inputs: the activation, gate, up, their gradients and the results are
+    rounded to bf16 (2^-9 each); what the down-projection hands to the activation is not."""
+    from llmctl_b200.ops import functional as ops, native
+    monkeypatch.setattr(ops, "SWIGLU_BWD_COLS", 0)
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device=cuda_device).bfloat16().requires_grad_(True)
+    w_up = (torch.randn(2 * F_, K, device=cuda_device) / K ** 0.5).bfloat16().requires_grad_(True)
+    w_down = (torch.randn(N, F_, device=cuda_device) / F_ ** 0.5).bfloat16().requires_grad_(True)
+    dy = torch.randn(M, N, device=cuda_device).bfloat16()
+    before = native.launch_count
+    y = ops.swiglu_mlp(x, w_up, w_down)
+    grads = torch.autograd.grad(y, (x, w_up, w_down), dy)
+    assert native.launch_count == before + 6
+    composed = ops.linear(ops.linear_swiglu(x, w_up), w_down)
+    general = torch.autograd.grad(composed, (x, w_up, w_down), dy)
+    assert torch.equal(y, composed)
+    xd, ud, dd = (t.detach().double().requires_grad_(True) for t in (x, w_up, w_down))
+    g, u = (xd @ ud.t()).chunk(2, -1)
+    want = torch.autograd.grad((F.silu(g) * u) @ dd.t(), (xd, ud, dd), dy.double())
+    for got, old, ref in zip(grads, general, want):
+        err, was = ((t.double() - ref).norm() / ref.norm() for t in (got, old))
+        assert err <= 2.0 ** -7 and err <= 1.02 * was, (float(err), float(was))
+
+
 @pytest.mark.parametrize("B,S,H", [(2, 512, 4), (1, 2048, 2), (3, 128, 1), (1, 1024, 8)])
 @pytest.mark.parametrize("packed", [True, False])
 def test_flash_attention_fwd(cuda_device, B, S, H, packed):
