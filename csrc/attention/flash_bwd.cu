@@ -18,11 +18,12 @@
 // of operands per clock where shared memory gives 128, and started a CTA per item.)  The streamed tiles Q, dO, Q, dO, ... share
 // one ring: with 5 slots beside the two resident tiles (all that 227 KB hold at D = 128) Q(n+1) is fetched as soon as dV(n-2)
 // has retired, a block and a half ahead of its use; rings of two stages each left the pipe waiting 200-1000 clocks per block.
-// P is handed over in two halves, as in the forward.  Persistent: one CTA per SM claims items, longest of a group first, the dKV items
-// of a group of heads before its dQ items (which read the same tiles again, from L2, and fill the SMs that the last dKV items leave
-// idle: 8 x 512 x 32 x 128 took 94 us in two launches, 88 us in one); TMEM, barriers and maps are set up once, an item's first tiles are fetched while the previous item is still in its softmax, and a
-// warpgroup of its own reads the accumulators out and stores them meanwhile (a row per thread: 4900 clocks from the last product
-// to the next item's first softmax when the softmax warps did it, against 2900 per block).
+// P is handed over in two halves, as in the forward.  Persistent: one CTA per SM claims items, longest of a group first, the dKV
+// items of a group of heads before its dQ items.  These read the same tiles again, from L2, and fill the SMs that the last dKV items
+// leave idle (8 x 512 x 32 x 128: 94 us in two launches, 88 us in one).  TMEM, barriers and maps are set up once, an item's first
+// tiles are fetched while the previous item is still in its softmax, and a warpgroup of its own reads the accumulators out and stores
+// them meanwhile (a row per thread: 4900 clocks from the last product to the next item's first softmax when the softmax warps did it,
+// against 2900 per block).
 //
 // A ragged sequence ends inside a block: rows past it are zero-filled by TMA, their statistics make P zero, and they are
 // never stored (causal only: keys past the end are then hidden from every real query by the mask).

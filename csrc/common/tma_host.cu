@@ -103,28 +103,6 @@ int get_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t
   return encode_cached(out, key, 2, base, dims, strides, box, swizzle128);
 }
 
-int get_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
-                     uint64_t s1, uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2,
-                     int swizzle128) {
-  Key key;
-  memset(&key, 0, sizeof(key));
-  key.v[0] = reinterpret_cast<uint64_t>(base);
-  key.v[1] = d0;
-  key.v[2] = d1;
-  key.v[3] = d2;
-  key.v[4] = s1;
-  key.v[5] = s2;
-  key.v[6] = b0;
-  key.v[7] = b1;
-  key.v[8] = b2;
-  key.v[9] = swizzle128;
-  key.v[10] = 3;
-  cuuint64_t dims[3] = {d0, d1, d2};
-  cuuint64_t strides[2] = {s1 * 2, s2 * 2};
-  cuuint32_t box[3] = {b0, b1, b2};
-  return encode_cached(out, key, 3, base, dims, strides, box, swizzle128);
-}
-
 int get_tmap_4d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t d3,
                      uint64_t s1, uint64_t s2, uint64_t s3, uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3,
                      int swizzle128) {

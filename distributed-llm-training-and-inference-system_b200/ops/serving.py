@@ -46,7 +46,7 @@ def choose_splits(batch: int, heads: int, max_context: int, block_size: int, sms
 
 def _launch_splits(batch: int, heads: int, max_context: int, block_size: int, sms: int = 148) -> int:
     # One launch, merged inside clusters of up to 8 splits, while all CTAs (three per SM) are resident together and none walks
-    # more than 768 tokens: one context of 4096, 32 heads of 128: 23 us with 37 splits and a merge kernel, 15 us with 8.  Larger batches
+    # more than 768 tokens: one context of 4096, 32 heads of 128: 23 us with 37 splits and a merge kernel, 18 us with 8.  Larger batches
     # and longer contexts take the finer splits of choose_splits.
     one_wave = max(1, min(8, 3 * sms // (batch * heads)))
     if max_context <= 768 * one_wave:
