@@ -38,7 +38,7 @@ native.register_signature("llmctl_latent_prompt_attention", [c_void_p, c_ll, c_l
                                                               c_int, c_void_p, c_float, c_void_p])
 
 KEY_ROWS = 128              # rebuilt keys of a sequence fill whole blocks of this many rows (the flash kernel's key tile)
-REBUILD_PAIRS = 32          # visible pairs per rebuilt key row from which rebuilding pays (see rebuild_pays)
+REBUILD_PAIRS = 24          # visible pairs per rebuilt key row from which rebuilding pays (see rebuild_pays)
 REBUILD_BYTES = 1 << 30     # most scratch a layer's rebuilt keys and values may take
 WINDOW_ALIGN = 32           # a window's first key tile starts at a multiple of this (kWindowAlign of the kernels)
 ROWS_PER_TILE = 16          # query rows (token, head) a CTA owns; tiles are built by the engine with this limit
@@ -86,7 +86,9 @@ def rebuild_pays(q: torch.Tensor, dn: int, dr: int, dv: int, R: int, heads: int,
     """Whether a batch's attention runs over keys and values rebuilt from the cache (``latent_prompt_attention``) instead of
     absorbed queries: head sizes that the flash kernel has, scratch within ``REBUILD_BYTES``, and at least ``REBUILD_PAIRS`` visible
     (query, key) pairs per rebuilt row.  A pair costs a head 1088 products at the absorbed kernel's rate or 320 at four times that
-    rate, a rebuilt row 131072 at five times that rate: the line is near 26 pairs a row, a prompt of about 64 tokens."""
+    rate, a rebuilt row 131072 at five times that rate: the line is near 26 pairs a row.  Layer of 16 heads, us absorbed / rebuilt: one prompt of
+    48 tokens 74.4 / 74.6, 64 (16 pairs a row) 72.9 / 74.7, 80 (25 pairs) 76.7 / 74.7, 128 97.2 / 74.8, 512 218 / 85, 2 x 2048 937 / 179;
+    behind 4000 cached tokens 24 tokens 181 / 136, 128 232 / 140, 512 519 / 161."""
     return (q.is_cuda and q.dtype == torch.bfloat16 and (dn, dr, dv) == (128, 64, 128) and R % 8 == 0 and q.stride(1) == 1
             and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and key_rows > 0 and pairs >= REBUILD_PAIRS * key_rows
             and 2 * key_rows * (heads * (dn + dv) + R + dr) <= REBUILD_BYTES and native.has_symbol("llmctl_latent_prompt_attention"))
