@@ -81,8 +81,8 @@ class MLP(nn.Module):
                                           dtype=dtype, device=device, fused_name="mlp_down")
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if self.gated and not (self.selective_recompute and torch.is_grad_enabled()) and self.up.runs_plain():
-            if self.down.runs_plain():
+        if self.gated and not (self.selective_recompute and torch.is_grad_enabled()) and tpl.runs_plain(self.up):
+            if tpl.runs_plain(self.down):
                 return ops.swiglu_mlp(x, self.up.weight, self.down.weight)
             return self.down(ops.linear_swiglu(x, self.up.weight))
         gu = self.up(x)

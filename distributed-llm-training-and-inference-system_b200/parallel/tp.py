@@ -136,11 +136,6 @@ def _init_weight(shape, std, dtype, device, seed_offset: int = 0):
     return w
 
 
-def _runs_plain(layer: nn.Module) -> bool:
-    """Whether the layer is its matrix product and nothing else: one rank, no hooks that a fused caller would pass by."""
-    return get_state().tp == 1 and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks)
-
-
 class ColumnParallelLinear(nn.Module):
     """y_local = x @ W_local.T, W sharded on the output dim.  Input is replicated over TP, or — with
     sequence parallelism — sharded on tokens and all-gathered first."""
@@ -156,9 +151,6 @@ class ColumnParallelLinear(nn.Module):
         self.weight.tp_shard_dim = 0
         self.weight.tp_packed = packed      # rows are `packed` equal groups (q|k|v, gate|up), each sharded
         self.fused_name = fused_name
-
-    def runs_plain(self) -> bool:
-        return _runs_plain(self)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         st = get_state()
@@ -188,9 +180,6 @@ class RowParallelLinear(nn.Module):
         self.weight.tp_shard_dim = 1
         self.fused_name = fused_name
 
-    def runs_plain(self) -> bool:
-        return _runs_plain(self)
-
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         st = get_state()
         if st.tp > 1 and st.sequence_parallel:
@@ -205,6 +194,21 @@ class RowParallelLinear(nn.Module):
         if st.tp > 1:
             return reduce_scatter_seq(y_local) if st.sequence_parallel else reduce_from_tp(y_local)
         return y_local
+
+
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+_OWN = ((ColumnParallelLinear.forward, None), (RowParallelLinear.forward, RowParallelLinear.finish))
+
+
+def runs_plain(layer: nn.Module) -> bool:
+    """Whether calling ``layer`` is ``ops.linear(x, layer.weight)`` and nothing else, so that a fused caller may take its weight and pass
+    it by: one rank, one of the two layers above with the ``forward`` that stands there (a subclass, an instance or a module put in its
+    place may do more), and no hook on it or on all modules that would want to see the call."""
+    t, every = type(layer), torch.nn.modules.module
+    return ((getattr(t, "forward", None), getattr(t, "finish", None)) in _OWN
+            and t.__call__ is nn.Module.__call__ and not layer.__dict__.keys() & {"forward", "finish", "__call__"}
+            and getattr(layer, "_compiled_call_impl", None) is None and get_state().tp == 1
+            and not any(getattr(layer, h) or getattr(every, "_global" + h) for h in _HOOKS))
 
 
 class VocabParallelEmbedding(nn.Module):

@@ -456,3 +456,70 @@ def test_apply_without_gradients_keeps_autograd_rules():
             native.apply(Twice, dual)           # no jvp: refused, as Twice.apply refuses it
     with pytest.raises(Exception):
         torch.func.vmap(lambda t: native.apply(Twice, t))(torch.ones(2, 3))
+
+
+@pytest.mark.parametrize("layer", ["up", "down"])
+@pytest.mark.parametrize("change", ["subclass", "finish", "instance", "class", "call", "global_forward", "global_pre", "global_backward", "hook", "module"])
+def test_gated_mlp_calls_its_layers_where_they_are_more_than_their_product(monkeypatch, layer, change):
+    """Subclasses, replaced methods and modules and hooks of any kind see every call of an MLP's two layers, as if nothing were fused."""
+    from torch.nn.modules import module as every
+    from llmctl_b200.models.config import ModelConfig
+    from llmctl_b200.models.gpt import MLP
+    from llmctl_b200.ops import functional as ops
+    from llmctl_b200.parallel import tp
+    cfg = ModelConfig(name="t", layers=1, hidden=16, ffn=24, heads=2, vocab_size=32, max_position_embeddings=8)
+    torch.manual_seed(0)
+    mlp = MLP(cfg, torch.float32, "cpu")
+    x = torch.randn(5, 16, requires_grad=True)
+    seen, factor = [], 1.0
+    assert tp.runs_plain(mlp.up) and tp.runs_plain(mlp.down)
+    old = getattr(mlp, layer)
+    handle = None
+    if change == "subclass":
+        class Doubled(type(old)):
+            def forward(self, x):
+                return 2 * super().forward(x)
+        old.__class__, factor = Doubled, 2.0
+    elif change == "finish":
+        if layer == "up":
+            pytest.skip("only the row-parallel layer has it")
+        old.finish, factor = lambda y: 2 * y, 2.0
+    elif change == "instance":
+        old.forward, factor = lambda x: 2 * x @ old.weight.t(), 2.0
+    elif change == "class":
+        monkeypatch.setattr(type(old), "forward", lambda self, x: 2 * x @ self.weight.t())
+        factor = 2.0
+    elif change == "call":
+        class Called(type(old)):
+            def __call__(self, x):
+                return 2 * super().__call__(x)
+        old.__class__, factor = Called, 2.0
+    elif change == "global_forward":
+        handle = every.register_module_forward_hook(lambda m, i, o: seen.append(m))
+    elif change == "global_pre":
+        handle = every.register_module_forward_pre_hook(lambda m, i: seen.append(m))
+    elif change == "global_backward":
+        handle = every.register_module_full_backward_hook(lambda m, gi, go: seen.append(m))
+    elif change == "hook":
+        old.register_forward_hook(lambda m, i, o: seen.append(m))
+    else:
+        new = torch.nn.Linear(*reversed(old.weight.shape), bias=True)
+        with torch.no_grad():
+            new.weight.copy_(2 * old.weight)
+            new.bias.zero_()
+        setattr(mlp, layer, new)
+        factor = 2.0
+    try:
+        assert not tp.runs_plain(getattr(mlp, layer))
+        y = mlp(x)
+        y.sum().backward()
+    finally:
+        if handle is not None:
+            handle.remove()
+    w_up = old.weight if layer == "up" else mlp.up.weight
+    w_down = old.weight if layer == "down" else mlp.down.weight
+    f_up, f_down = (factor, 1.0) if layer == "up" else (1.0, factor)
+    want = f_down * (ops.swiglu(f_up * x @ w_up.t()) @ w_down.t())
+    assert torch.allclose(y, want, rtol=1e-5, atol=1e-6)
+    if change.startswith("global") or change == "hook":
+        assert old in seen
