@@ -186,6 +186,9 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bar.tmem;
+  // A waiter of an mbarrier sees only the parity of its phase, so no barrier may complete its next phase before everyone has passed the
+  // wait for this one.  acc[a] (product finished) is therefore committed only after accfree[a] (read out) of the use before has been
+  // waited for.  acc[0] is used by every item, acc[1] by dKV items alone, each side counting them.
   // TMEM: S [0,128)  dP [128,256)  acc0 [256,256+D)  acc1 [384,384+D)
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tAcc0 = tmem_base + 256, tAcc1 = tmem_base + 384;
   volatile int* abort = &bar.abort;
@@ -304,7 +307,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         if (part == 2 || ((ks >> 1) & 1) == part)
           umma_ts<1>(t, a + (ks >> 2) * 64 + (ks & 3) * 8, b0 + ((ks * 2048) >> 4), id_acc, ks == 0 ? 1u - fresh : 1u);
     };
-    uint32_t g = 0, k = 0;
+    uint32_t g = 0, k = 0, kv = 0;     // blocks, items and dKV items so far
     auto run = [&](auto kind, int n) {
       constexpr bool kDQ = decltype(kind)::value;
       for (int i = 0; i < n; ++i, ++g) {
@@ -348,15 +351,12 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
           }
         }
         wait(&bar.ds, g & 1u);
-        if (i == 0 && k > 0) wait(&bar.accfree[kDQ ? 0 : 1], (k - 1) & 1u);
+        if (i == 0 && (kDQ ? k : kv) > 0) wait(&bar.accfree[kDQ ? 0 : 1], ((kDQ ? k : kv) - 1) & 1u);
         tc_fence_after();
         if (elect_one()) {
           issue_acc(kDQ ? tAcc0 : tAcc1, tdP, tile_at(e0), fresh, 2);    // dK += dS^T Q  /  dQ += dS K
           umma_commit<1>(&bar.empty[e0 % C::kSlots]);
-          if (i + 1 == n) {
-            if (kDQ) umma_commit<1>(&bar.acc[0]);
-            umma_commit<1>(&bar.acc[1]);                   // every item completes both, used or not: phases follow the items
-          }
+          if (i + 1 == n) umma_commit<1>(&bar.acc[kDQ ? 0 : 1]);
         }
         if (i + 1 < n) {
           arrived(e1 + 2);
@@ -375,7 +375,12 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
       int rb, bh, first, n;
       decode(item, is_dq, rb, bh, first, n);
       wait(&bar.res, k & 1u);
-      if (is_dq) run(DQ{}, n); else run(DKV{}, n);
+      if (is_dq) {
+        run(DQ{}, n);
+      } else {
+        run(DKV{}, n);
+        ++kv;
+      }
     }
   } else if (warp < 10) {
     // ------------------- softmax / dS warpgroups: half wg of the streamed columns, all 128 resident rows -------------------
@@ -498,7 +503,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     const int q4 = warp & 3;
     const int row = q4 * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(q4 * 32) << 16;
-    uint32_t k = 0;
+    uint32_t k = 0, kv = 0;            // items and dKV items so far
     for (int item; next_item(k, item); ++k) {
       bool is_dq;
       int rb, bh, first, n;
@@ -506,13 +511,9 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
       const bool real = rb * kBlk + row < S;
       const long long at = (static_cast<long long>(bh / H) * S + rb * kBlk + row) * out_tok + (bh % H) * D;
 #pragma unroll 1
-      for (int a = 0; a < 2; ++a) {                       // dKV: dV from acc0, then scale * dK from acc1.  dQ: scale * dQ from acc0.
-        mbar_wait_or_abort(&bar.acc[a], k & 1u, abort);
+      for (int a = 0; a < (is_dq ? 1 : 2); ++a) {         // dKV: dV from acc0, then scale * dK from acc1.  dQ: scale * dQ from acc0.
+        mbar_wait_or_abort(&bar.acc[a], (a == 0 ? k : kv) & 1u, abort);
         __syncwarp();
-        if (is_dq && a == 1) {                            // nothing there
-          if (lane == 0) mbar_arrive(&bar.accfree[1]);
-          break;
-        }
         tc_fence_after();
         const uint32_t tA = (a == 0 ? tAcc0 : tAcc1) + lane_off;
         const float mul = (is_dq || a == 1) ? scale : 1.f;
@@ -534,6 +535,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
           }
         }
       }
+      if (!is_dq) ++kv;
     }
   }
 

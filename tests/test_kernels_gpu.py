@@ -460,6 +460,30 @@ def test_flash_attention_edges_of_blocks(cuda_device, B, S, H, D, causal, shift)
             assert (a - b).norm() <= bound, f"{name} head {h}: {((a - b).norm() / b.norm()).item():.2e}"
 
 
+def test_flash_backward_of_short_items_beside_other_work(cuda_device):
+    """One block per sequence: thousands of the shortest items in a row, while copies on another stream slow the stores of the
+    accumulators down.  The gradients are those of an undisturbed run, bit for bit, and no wait runs out."""
+    from llmctl_b200.ops import attention as attn, native
+    torch.manual_seed(3)
+    B, S, H, D = 64, 128, 32, 64
+    q, k, v = (torch.randn(B, S, H, D, device=cuda_device).bfloat16().requires_grad_(True) for _ in range(3))
+    do = torch.randn(B, S, H, D, device=cuda_device).bfloat16()
+    def grads():
+        return torch.autograd.grad(attn.attention(q, k, v), (q, k, v), do)
+    want = grads()
+    side, a = torch.cuda.Stream(), torch.empty(128 << 20, dtype=torch.uint8, device=cuda_device)
+    b = torch.empty_like(a)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        with torch.cuda.stream(side):
+            for _ in range(4):
+                b.copy_(a)
+        got = grads()
+        assert all(torch.equal(x, y) for x, y in zip(got, want))
+    torch.cuda.synchronize()
+    assert native.lib().llmctl_flash_fwd_status(1) == 0 and native.lib().llmctl_flash_bwd_status(1) == 0
+
+
 
 @pytest.mark.parametrize("M,N,K", [(8, 4096, 1376), (8, 4096, 512), (5, 1000, 200), (32, 2752, 4096), (1, 4096, 1384)])
 def test_skinny_gemm_k_tail_and_odd_shapes(cuda_device, M, N, K):

@@ -523,3 +523,55 @@ def test_gated_mlp_calls_its_layers_where_they_are_more_than_their_product(monke
     assert torch.allclose(y, want, rtol=1e-5, atol=1e-6)
     if change.startswith("global") or change == "hook":
         assert old in seen
+
+
+@pytest.mark.parametrize("kinds", ["qq", "kq", "kqq", "qkq", "kkqq", "kqkq", "qqqq"])
+def test_flash_backward_accumulator_handover_orders_its_barriers(kinds):
+    """The issuer and an epilogue warp of csrc/attention/flash_bwd.cu, in every interleaving, over the barriers acc (product finished) and
+    accfree (read out) of the two accumulators.  A waiter sees the parity of a phase only, so a barrier must not complete a phase more
+    while somebody still has to pass the last one; a shared phase count for both kinds (acc[1] committed by dQ items too, which waited for
+    accfree[0] alone) breaks that."""
+    def program(counted):
+        issuer, epilogue, k, kv = [], [], 0, 0
+        for kind in kinds:
+            dkv = kind == "k"
+            n = kv if counted else k                                    # the use of acc[1] / accfree[1]
+            if dkv:
+                issuer += ([("wait", "accfree0", k - 1)] if k else []) + [("done", "acc0")]
+                issuer += ([("wait", "accfree1", n - 1)] if n else []) + [("done", "acc1")]
+            else:
+                issuer += ([("wait", "accfree0", k - 1)] if k else []) + [("done", "acc0")] + ([] if counted else [("done", "acc1")])
+            epilogue += [("wait", "acc0", k), ("done", "accfree0")]
+            if dkv or not counted:
+                epilogue += [("wait", "acc1", n), ("done", "accfree1")]
+            k, kv = k + 1, kv + dkv
+        return issuer, epilogue
+
+    def sound(programs):
+        """Every reachable state: no waiter is a whole phase behind, nobody passes a wait early, both sides end."""
+        seen, todo = set(), [((0, 0), ())]
+        while todo:
+            at, phases = state = todo.pop()
+            if state in seen:
+                continue
+            seen.add(state)
+            done, moved = dict(phases), False
+            for i, ops in enumerate(programs):
+                if at[i] == len(ops):
+                    continue
+                op = ops[at[i]]
+                n = done.get(op[1], 0)
+                if op[0] == "wait":
+                    if n > op[2] + 1 or (n & 1 != op[2] & 1) != (n == op[2] + 1):
+                        return False                                    # the parity no longer tells this phase from another
+                    if n != op[2] + 1:
+                        continue
+                nxt = dict(done, **({op[1]: n + 1} if op[0] == "done" else {}))
+                todo.append((tuple(a + (j == i) for j, a in enumerate(at)), tuple(sorted(nxt.items()))))
+                moved = True
+            if not moved and any(at[i] < len(programs[i]) for i in (0, 1)):
+                return False
+        return True
+
+    assert sound(program(counted=True))
+    assert sound(program(counted=False)) == ("q" not in kinds[1:])
