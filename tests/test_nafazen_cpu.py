@@ -343,3 +343,16 @@ def test_bfloat16_serving_precision_is_close_to_oracle():
     got = run_cut(eng, 1, toks, [25] + [1] * 15)
     err = (got - ref).pow(2).mean().sqrt() / ref.pow(2).mean().sqrt()
     assert err < 0.05, err
+
+
+@pytest.mark.parametrize("R,rebuilds", [(64, True), (144, True), (512, True), (136, False), (152, False), (520, False), (768, False), (1024, False)])
+def test_latent_ranks_of_the_fp32_kernel_keep_it_for_prompts(monkeypatch, R, rebuilds):
+    """Ranks that the tensor-core kernels do not take run with queries and probabilities in fp32, for prompts too; keys and values rebuilt
+    in bf16 are for the others."""
+    from types import SimpleNamespace
+    from llmctl_b200.ops import latent_attention as L
+    monkeypatch.setattr(L.native, "has_symbol", lambda name: True)
+    q = SimpleNamespace(is_cuda=True, dtype=torch.bfloat16, stride=lambda d: (4 * 192, 1)[d], data_ptr=lambda: 256)
+    assert L.uses_tensor_cores(q.dtype, R, 64) == rebuilds
+    assert L.rebuild_pays(q, 128, 64, 128, R, 4, 1024, 1024 * L.REBUILD_PAIRS) == rebuilds
+    assert not L.rebuild_pays(q, 128, 64, 128, R, 4, 1024, 1024 * L.REBUILD_PAIRS - 1)

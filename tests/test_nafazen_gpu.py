@@ -153,7 +153,7 @@ def test_latent_attention_tcgen05(cuda_device, H, dn, dr, R, bs):
 # keys at positions that are and are not multiples of 128, unlike lengths side by side, a single token among them
 @pytest.mark.parametrize("portions", [[(64, 0)], [(127, 0)], [(128, 0)], [(129, 0)], [(257, 0)], [(700, 0)], [(300, 128)], [(300, 1)],
                                       [(130, 255)], [(600, 0), (1, 500), (90, 77), (256, 256)]])
-@pytest.mark.parametrize("H,R,bs,q_rank", [(3, 512, 64, 24), (1, 64, 16, 0), (4, 136, 48, 16)])
+@pytest.mark.parametrize("H,R,bs,q_rank", [(3, 512, 64, 24), (1, 64, 16, 0), (4, 144, 48, 16)])
 def test_latent_prompt_over_rebuilt_keys(cuda_device, monkeypatch, portions, H, R, bs, q_rank):
     """The layer over rebuilt keys and values against float64 and against absorbed queries (both round intermediate results to bf16:
     the rebuilt path its keys, values, P and heads, the absorbed one its queries, P, latents and heads: 4 x 2^-9 each in the 2-norm,
