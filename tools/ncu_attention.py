@@ -1,4 +1,4 @@
-"""One causal attention forward + backward at a fixed shape, for `ncu -k regex:flash` captures."""
+"""One causal attention forward + backward at a fixed shape, for `ncu --clock-control none -k regex:flash` captures."""
 import math
 import sys
 from pathlib import Path

@@ -1,4 +1,4 @@
-"""A few skinny-GEMM launches at the qkv decode shape for `ncu -k regex:gemm_skinny` captures."""
+"""A few skinny-GEMM launches at the qkv decode shape for `ncu --clock-control none -k regex:gemm_skinny` captures."""
 import sys
 from pathlib import Path
 

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Tiny single-GPU launch targets for `ncu --set full` (one kernel family per invocation, a handful of
+"""Tiny single-GPU launch targets for `ncu --clock-control none --set full` (one kernel family per invocation, a handful of
 launches, no timing reported)."""
 import sys
 from pathlib import Path

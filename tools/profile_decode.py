@@ -1,6 +1,6 @@
 """Decode-step kernel breakdown: prefill N prompts, then run a few eager decode steps between
-cudaProfilerStart/Stop so that `ncu --profile-from-start off --metrics gpu__time_duration.sum` lists them.
-    ncu --profile-from-start off --metrics gpu__time_duration.sum --csv --log-file out.csv python tools/profile_decode.py
+cudaProfilerStart/Stop so that `ncu --clock-control none --profile-from-start off --metrics gpu__time_duration.sum` lists them.
+    ncu --clock-control none --profile-from-start off --metrics gpu__time_duration.sum --csv --log-file out.csv python tools/profile_decode.py
 Without ncu it prints per-phase wall times (prefill per request, decode per step) for graph and eager modes."""
 import sys
 import time
