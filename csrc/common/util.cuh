@@ -7,6 +7,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include "smem_limit.h"
+
 #define LLMCTL_API extern "C" __attribute__((visibility("default")))
 
 // Clear any stale (non-sticky) error left behind by another library on this thread, so that the status
@@ -50,26 +52,6 @@ static inline bool llmctl_debug() {
 namespace llmctl {
 
 constexpr int kNumSMs = 148;
-
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize), asked of the runtime once per kernel, device and thread: the call costs about as
-// much host time as a quarter of a launch, and the limit only has to be raised once.
-template <typename Kernel>
-static inline cudaError_t allow_smem(Kernel kernel, int bytes) {
-  struct Entry {
-    const void* f;
-    int device, bytes;
-  };
-  static thread_local Entry seen[64] = {};
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return e;
-  const void* f = reinterpret_cast<const void*>(kernel);
-  Entry& at = seen[(reinterpret_cast<uintptr_t>(f) >> 4) & 63];
-  if (at.f == f && at.device == device && at.bytes >= bytes) return cudaSuccess;
-  e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) at = Entry{f, device, bytes};
-  return e;
-}
 
 struct __align__(16) bf16x8 {
   __nv_bfloat162 v[4];

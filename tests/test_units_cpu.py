@@ -575,3 +575,62 @@ def test_flash_backward_accumulator_handover_orders_its_barriers(kinds):
 
     assert sound(program(counted=True))
     assert sound(program(counted=False)) == ("q" not in kinds[1:])
+
+
+
+def test_shared_memory_limits_are_raised_and_never_lowered(tmp_path):
+    """csrc/common/smem_limit.h with the runtime's two calls replaced: threads that ask for unlike sizes of one kernel leave the largest in
+    place, a device counts by itself, and a call that was refused is asked again."""
+    import shutil
+    import subprocess
+    root = Path(__file__).resolve().parents[1]
+    gxx, cuda = shutil.which("g++"), Path("/usr/local/cuda/include")
+    if gxx is None or not (cuda / "cuda_runtime_api.h").exists():
+        pytest.skip("needs g++ and the CUDA headers")
+    (tmp_path / "t.cpp").write_text(r"""
+#include "common/smem_limit.h"
+#include <atomic>
+#include <thread>
+#include <vector>
+#include <cstdio>
+static thread_local int device = 0;
+static std::atomic<int> limit[2], calls, refuse;
+extern "C" cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
+extern "C" cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int v) {
+  ++calls;
+  if (refuse) return cudaErrorInvalidValue;
+  limit[device] = v;
+  return cudaSuccess;
+}
+static void kernel() {}
+#define EXPECT(c) if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); return 1; }
+int main() {
+  using llmctl::allow_smem;
+  EXPECT(allow_smem(kernel, 200) == cudaSuccess && limit[0] == 200);
+  std::thread([] { allow_smem(kernel, 100); }).join();             // another thread's table is empty
+  EXPECT(limit[0] == 200 && calls == 1);
+  EXPECT(allow_smem(kernel, 200) == cudaSuccess && limit[0] == 200);
+  device = 1;
+  EXPECT(allow_smem(kernel, 100) == cudaSuccess && limit[1] == 100 && limit[0] == 200);
+  refuse = 1;
+  EXPECT(allow_smem(kernel, 300) == cudaErrorInvalidValue);
+  refuse = 0;
+  EXPECT(allow_smem(kernel, 300) == cudaSuccess && limit[1] == 300);
+  device = 0;
+  std::vector<std::thread> ts;
+  std::atomic<int> bad{0};
+  for (int i = 0; i < 8; ++i)
+    ts.emplace_back([&, i] {
+      for (int k = 0; k < 2000; ++k) {
+        const int n = 201 + (k * 7 + i * 13) % 500;
+        if (allow_smem(kernel, n) != cudaSuccess || limit[0] < n) ++bad;
+      }
+    });
+  for (auto& t : ts) t.join();
+  EXPECT(bad == 0 && limit[0] == 700);
+}
+""")
+    exe = tmp_path / "t"
+    subprocess.run([gxx, "-std=c++17", "-O1", "-pthread", "-I", str(root / "csrc"), "-I", str(cuda), str(tmp_path / "t.cpp"), "-o", str(exe)], check=True)
+    done = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert done.returncode == 0, done.stdout
