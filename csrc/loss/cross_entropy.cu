@@ -84,7 +84,7 @@ ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long l
   }
 }
 
-// Rows of 8 K to 57 K logits: persistent CTAs with a ring of two or three whole rows in shared memory.  Bound by HBM (the row is read and
+// Rows of 8 K (8200) to 55 K logits (kCERingBytes / 4 = 56320): persistent CTAs with a ring of two or three whole rows in shared memory.  Bound by HBM (the row is read and
 // written once): while a row is reduced and differentiated the next is copied in and the one before is copied out by bulk copies,
 // which a CTA that loads, reduces and stores one row after the other cannot do (4096 x 32000: 204 us, two of them
 // per SM; here 118 us = 4.4 TB/s).  Maximum
@@ -365,7 +365,7 @@ LLMCTL_API int llmctl_cross_entropy_fwd_bwd(void* logits, long long ld, const lo
                                             int V, long long ignore_index, float host_scale,
                                             const float* scale_dev, int write_grad, void* stream) {
   LLMCTL_BEGIN();
-  LLMCTL_REQUIRE(V % 8 == 0 && ld % 8 == 0 && ld >= V);
+  LLMCTL_REQUIRE(V % 8 == 0 && ld % 8 == 0 && ld >= V && (reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   if (rows == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   const int nvec = V / 8;
@@ -385,7 +385,7 @@ LLMCTL_API int llmctl_cross_entropy_fwd_bwd(void* logits, long long ld, const lo
   };
   // short rows: several CTAs per SM overlap each other; rows that do not fit the ring twice stream through L2
   if (kv <= 2) LAUNCH(2);
-  else if (row_bytes * 2 > kCERingBytes || (reinterpret_cast<uintptr_t>(logits) & 15) != 0)
+  else if (row_bytes * 2 > kCERingBytes)
     ce_fwd_bwd_stream_kernel<<<rows, kCEThreads, 0, s>>>((__nv_bfloat16*)logits, ld, targets,
                                                          loss_per_row, lse_per_row, V, ignore_index,
                                                          host_scale, scale_dev, write_grad);
@@ -400,7 +400,7 @@ LLMCTL_API int llmctl_cross_entropy_partial(const void* logits, long long ld,
                                             const long long* targets, float* stats, int rows,
                                             int V_local, long long vocab_start, void* stream) {
   LLMCTL_BEGIN();
-  LLMCTL_REQUIRE(V_local % 8 == 0 && ld % 8 == 0);
+  LLMCTL_REQUIRE(V_local % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   if (rows == 0) return 0;
   ce_partial_kernel<<<rows, kCEThreads, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)logits, ld, targets, stats, V_local, vocab_start);
@@ -413,7 +413,7 @@ LLMCTL_API int llmctl_cross_entropy_finalize(void* logits, long long ld, const l
                                              float host_scale, const float* scale_dev,
                                              void* stream) {
   LLMCTL_BEGIN();
-  LLMCTL_REQUIRE(V_local % 8 == 0 && ld % 8 == 0);
+  LLMCTL_REQUIRE(V_local % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   if (rows == 0) return 0;
   ce_finalize_kernel<<<rows, kCEThreads, 0, (cudaStream_t)stream>>>(
       (__nv_bfloat16*)logits, ld, targets, lse, V_local, vocab_start, ignore_index, host_scale,

@@ -641,7 +641,9 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int
     V = logits.shape[-1]
     logits2 = logits.reshape(-1, V)
     t = targets.reshape(-1)
-    if _use_native(logits2, "elementwise") and V % 8 == 0 and logits2.stride(1) == 1 and logits2.stride(0) % 8 == 0:
+    # rows of whole 16-byte units at 16-byte boundaries (what is cloned below begins at one)
+    if (_use_native(logits2, "elementwise") and V % 8 == 0 and logits2.stride(1) == 1 and logits2.stride(0) % 8 == 0
+            and (not logits2.requires_grad or logits2.data_ptr() % 16 == 0)):
         cnt = (t != ignore_index).sum().clamp_min(1).to(torch.float32)
         inv = (1.0 / cnt).reshape(1)
         if not logits2.requires_grad:

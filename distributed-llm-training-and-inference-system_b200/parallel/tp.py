@@ -323,6 +323,6 @@ def vocab_parallel_cross_entropy(logits: torch.Tensor, targets: torch.Tensor, ig
     if st.tp == 1:
         return ops.cross_entropy(logits, targets, ignore_index, grad_scale=grad_scale, assume_unit_grad=True)
     if (ops._use_native(logits, "elementwise") and V_local % 8 == 0 and logits.stride(1) == 1
-            and logits.stride(0) % 8 == 0 and not logits.is_leaf):
+            and logits.stride(0) % 8 == 0 and logits.data_ptr() % 16 == 0 and not logits.is_leaf):
         return _VocabParallelCENative.apply(logits, targets.contiguous(), st.tp_rank * V_local, ignore_index, grad_scale)
     return _VocabParallelCE.apply(logits, targets, st.tp_rank * V_local, ignore_index, grad_scale)

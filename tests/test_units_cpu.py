@@ -634,3 +634,21 @@ int main() {
     subprocess.run([gxx, "-std=c++17", "-O1", "-pthread", "-I", str(root / "csrc"), "-I", str(cuda), str(tmp_path / "t.cpp"), "-o", str(exe)], check=True)
     done = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert done.returncode == 0, done.stdout
+
+
+@pytest.mark.parametrize("shift,grad,native_rows", [(0, True, True), (1, True, False), (4, True, False), (8, True, True), (1, False, True)])
+def test_cross_entropy_of_rows_at_odd_addresses_stays_off_the_kernel(monkeypatch, shift, grad, native_rows):
+    """The loss kernels read and write 16-byte units: logits that begin elsewhere take the library path, unless they are copied first."""
+    from llmctl_b200.ops import functional as ops
+    base = torch.randn(4 * 64 + 8).bfloat16().requires_grad_(grad)      # the allocator's boundaries are multiples of 64 bytes
+    logits = base[shift:shift + 256].view(4, 64)
+    assert logits.data_ptr() % 16 == 2 * shift % 16
+    t = torch.tensor([1, -100, 63, 5])
+    calls = []
+    monkeypatch.setattr(ops, "_use_native", lambda *a: True)
+    monkeypatch.setattr(ops._CrossEntropyFn, "apply", lambda x, *a: calls.append(x.data_ptr()) or torch.zeros(()))
+    loss = ops.cross_entropy(logits, t)
+    assert bool(calls) == native_rows and all(p % 16 == 0 for p in calls)
+    if not native_rows:
+        loss.backward()
+        assert torch.equal(loss, torch.nn.functional.cross_entropy(logits.float(), t)) and base.grad is not None
