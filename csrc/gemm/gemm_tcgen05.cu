@@ -232,9 +232,9 @@ __device__ __forceinline__ void swiglu_epilogue(uint32_t t_row, uint8_t* out_sme
       stage_box(out_smem, out_n, &maps.gate, col, row0, lane, [&](int e) { return packed(g, e); });
       stage_box(out_smem, out_n, &maps.up, col, row0, lane, [&](int e) { return packed(u, e); });
     }
-    auto act = [](uint32_t gv, uint32_t uv) {
+    auto act = [](uint32_t gv, uint32_t uv) {          // silu first, as in swiglu.cu: x * up may overflow where silu(x) * up does not
       const float x = __uint_as_float(gv);
-      return x * __uint_as_float(uv) * __fdividef(1.f, 1.f + __expf(-x));
+      return x * __fdividef(1.f, 1.f + __expf(-x)) * __uint_as_float(uv);
     };
     stage_box(out_smem, out_n, &maps.act, col, row0, lane, [&](int e) { return pack_bf16x2(act(g[2 * e], u[2 * e]), act(g[2 * e + 1], u[2 * e + 1])); });
   }

@@ -294,6 +294,24 @@ def test_linear_swiglu(cuda_device, M, F_, K):
     assert (dx.double() - gx).norm() <= 2.0 ** -7 * gx.norm() and (dw.double() - gw).norm() <= 2.0 ** -7 * gw.norm()
 
 
+def test_linear_swiglu_of_extreme_halves(cuda_device):
+    """Gates where the sigmoid is 0 beside halves near the largest bf16: 0 as from the separate kernels, not the NaN of inf * 0; products
+    that overflow by themselves stay infinite."""
+    from llmctl_b200.ops import functional as ops
+    x = torch.zeros(64, 64, device=cuda_device).bfloat16()
+    x[:, 0] = 1
+    gate = torch.tensor([-120.0, -90.0, 0.0, 2.0, 100.0, -3.0, 88.0, 1.0], device=cuda_device)
+    up = torch.tensor([3e38, -3e38, 3e38, 1e38, 3e38, 1e38, -2e38, -1.0], device=cuda_device)
+    w = torch.zeros(16, 64, device=cuda_device).bfloat16()
+    w[:8, 0], w[8:, 0] = gate.bfloat16(), up.bfloat16()
+    got = ops.linear_swiglu(x, w)
+    want = ops.swiglu(ops.linear(x, w))
+    assert torch.equal(got.isinf(), want.isinf()) and not got.isnan().any() and not want.isnan().any()
+    fine = ~want.isinf()
+    assert torch.allclose(got[fine].double(), want[fine].double(), rtol=2.0 ** -8, atol=0)
+    assert (got[:, :2] == 0).all() and got[:, 4].isinf().all()
+
+
 # One-wave tiles of 64 and 128 columns and the pair tile, rows and columns that end inside a tile, ragged K
 @pytest.mark.parametrize("M,F_,K,N", [(33, 8, 64, 72), (200, 136, 264, 64), (1000, 2048, 768, 768), (2560, 1032, 128, 200), (2049, 5632, 64, 320)])
 def test_swiglu_mlp(cuda_device, monkeypatch, M, F_, K, N):
