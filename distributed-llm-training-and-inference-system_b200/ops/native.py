@@ -47,6 +47,7 @@ _SIGNATURES = {
     "llmctl_gemm_swiglu_bwd_bf16": [c_void_p] * 4 + [c_int] * 3 + [c_ll] * 3 + [c_void_p],
     "llmctl_gemm_skinny_bf16": [c_void_p] * 3 + [c_int] * 3 + [c_ll] * 3 + [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p],
 }
+_RESULTS: dict = {}         # result types by name; int for the rest
 
 
 def library_path() -> Path:
@@ -75,18 +76,20 @@ def lib() -> ctypes.CDLL:
                 fn = getattr(l, name)
             except AttributeError:
                 continue
-            fn.restype = c_int
+            fn.restype = _RESULTS.get(name, c_int)
             fn.argtypes = argtypes
         _lib = l
     return _lib
 
 
-def register_signature(name: str, argtypes: list) -> None:
+def register_signature(name: str, argtypes: list, restype=c_int) -> None:
+    """``restype``: what the entry point returns where that is not a status."""
     _SIGNATURES[name] = argtypes
+    _RESULTS[name] = restype
     if _lib is not None:
         try:
             fn = getattr(_lib, name)
-            fn.restype = c_int
+            fn.restype = restype
             fn.argtypes = argtypes
         except AttributeError:
             pass

@@ -14,7 +14,7 @@ native.register_signature("llmctl_kv_append", [c_void_p, c_ll, c_int, c_int, c_v
 native.register_signature("llmctl_paged_attn_decode",
                           [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_ll, c_void_p,
                            c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p])
-native.register_signature("llmctl_paged_attn_scratch_elems", [c_int, c_int, c_int, c_int])
+native.register_signature("llmctl_paged_attn_scratch_elems", [c_int, c_int, c_int, c_int], restype=c_ll)
 native.register_signature("llmctl_sample", [c_void_p, c_int, c_ll, c_int, c_int] + [c_void_p] * 6 + [c_void_p])
 
 

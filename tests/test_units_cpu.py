@@ -652,3 +652,14 @@ def test_cross_entropy_of_rows_at_odd_addresses_stays_off_the_kernel(monkeypatch
     if not native_rows:
         loss.backward()
         assert torch.equal(loss, torch.nn.functional.cross_entropy(logits.float(), t)) and base.grad is not None
+
+
+def test_paged_decode_scratch_is_counted_in_64_bits():
+    """256 sequences of 128 heads in 512 splits want more than 2^31 numbers: the entry point returns them as a long long."""
+    from llmctl_b200.ops import native, serving
+    if not native.available():
+        pytest.skip("kernel library not built")
+    for batch, heads, dim, splits in ((256, 128, 128, 512), (65535, 32, 128, 8), (16, 32, 128, 8), (1, 12, 64, 8), (700, 1, 64, 1)):
+        one_wave = splits == 1 or (splits <= 8 and batch * heads * splits <= 3 * 148)
+        want = 0 if one_wave else batch * heads * splits * (dim + 2)
+        assert native.lib().llmctl_paged_attn_scratch_elems(batch, heads, dim, splits) == want
