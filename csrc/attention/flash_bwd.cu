@@ -34,6 +34,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
+#include "../common/wait_status.h"
 
 namespace llmctl {
 using namespace ptx;
@@ -135,7 +136,8 @@ template <int D>
 __global__ void __launch_bounds__(fbwd::kThreads, 1)
 flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restrict__ nl2, const float* __restrict__ ndl,
                  __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long long out_tok,
-                 int out_wide, int B, int S, int H, int group, int* __restrict__ counter, float scale_log2, float scale, int causal) {
+                 int out_wide, int B, int S, int H, int group, int* __restrict__ counter, float scale_log2, float scale, int causal,
+                 unsigned char* wait_byte) {
   using namespace fbwd;
   using C = Cfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -149,7 +151,10 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   Bars& bar = *reinterpret_cast<Bars*>(smem + C::kBarsAt);
   const uint32_t smem_base = smem_u32(smem);
   if (smem_base & 1023u) {             // the swizzled tiles would not line up (uniform over the grid)
-    if (threadIdx.x == 0) atomicCAS(&g_status, 0u, 16u);
+    if (threadIdx.x == 0) {
+      atomicCAS(&g_status, 0u, 16u);
+      report_wait(wait_byte);
+    }
     return;
   }
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -541,7 +546,10 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
 
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && bar.abort) atomicCAS(&g_status, 0u, 1u);
+  if (threadIdx.x == 0 && bar.abort) {
+    atomicCAS(&g_status, 0u, 1u);
+    report_wait(wait_byte);
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc<1>(tmem_base, 512);
@@ -573,12 +581,14 @@ static int flash_bwd_launch(const void* q, const void* k, const void* v, const v
   mkmap(&mv, v, v_tok);
   mkmap(&mdo, d_o, o_tok);
   if (rc) return rc;
+  unsigned char* const wait_byte = wait_report(kWaitFlashBackward);
+  if (wait_byte == nullptr) return static_cast<int>(cudaErrorMemoryAllocation);
   const cudaError_t e = allow_smem(flash_bwd_kernel<D>, C::kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int n_items = 2 * nblk * B * H, grid = n_items < kNumSMs ? n_items : kNumSMs;
   const int wide = dqkv_tok % 16 == 0 && ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 31) == 0;
   flash_bwd_kernel<D><<<grid, kThreads, C::kSmem, s>>>(Maps{mq, mk, mv, mdo}, nl2, ndl, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv,
-                                                       dqkv_tok, wide, B, S, H, group, counter, scale * 1.4426950408889634f, scale, causal);
+                                                       dqkv_tok, wide, B, S, H, group, counter, scale * 1.4426950408889634f, scale, causal, wait_byte);
   return static_cast<int>(cudaGetLastError());
 }
 

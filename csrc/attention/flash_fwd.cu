@@ -9,6 +9,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
+#include "../common/wait_status.h"
 
 namespace llmctl {
 using namespace ptx;
@@ -161,7 +162,8 @@ template <int DQK, int DV>
 __global__ void __launch_bounds__(ffwd::kThreads, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmKs, const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ O,
-                 long long o_tok_stride, int o_wide, float* __restrict__ lse, const ffwd::Seq* __restrict__ seqs, int B, int max_q, int H, float scale_log2, int causal, long long* __restrict__ trace) {
+                 long long o_tok_stride, int o_wide, float* __restrict__ lse, const ffwd::Seq* __restrict__ seqs, int B, int max_q, int H, float scale_log2, int causal,
+                 unsigned char* wait_byte, long long* __restrict__ trace) {
   using namespace ffwd;
   using C = Cfg<DQK, DV>;
   constexpr int kOwn = DQK > 128 ? 2 : DQK / 64;         // panels of K that belong to the head; the last of three is shared by all
@@ -474,7 +476,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && abort_flag) atomicCAS(&g_status, 0u, 1u);
+  if (threadIdx.x == 0 && abort_flag) {
+    atomicCAS(&g_status, 0u, 1u);
+    report_wait(wait_byte);
+  }
   if (warp == 9) {
     tc_fence_after();
     tmem_dealloc<1>(tmem_base, 512);
@@ -506,9 +511,11 @@ static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CU
   const long long n_items = static_cast<long long>((max_q + 2 * kRows - 1) / (2 * kRows)) * H * B;
   if (n_items >= (1ll << 31) - 2 * kNumSMs) return static_cast<int>(cudaErrorInvalidValue);
   const int grid = n_items < kNumSMs ? static_cast<int>(n_items) : kNumSMs;
+  unsigned char* const wait_byte = wait_report(kWaitFlashForward);
+  if (wait_byte == nullptr) return static_cast<int>(cudaErrorMemoryAllocation);
   const int wide = o_tok_stride % 16 == 0 && (reinterpret_cast<uintptr_t>(o) & 31) == 0;
   flash_fwd_kernel<DQK, DV><<<grid, kThreads, C::kSmem, s>>>(q, k, ks, v, (__nv_bfloat16*)o, o_tok_stride, wide, lse, seqs, B, max_q, H,
-                                                             scale * 1.4426950408889634f, causal, flash_trace_buffer());
+                                                             scale * 1.4426950408889634f, causal, wait_byte, flash_trace_buffer());
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -28,6 +28,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
+#include "../common/wait_status.h"
 #include "../rope/rope_interleaved.cuh"
 
 namespace llmctl {
@@ -86,7 +87,7 @@ latent_attention_t5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
                            const int* __restrict__ tiles, const int* __restrict__ positions, float scale, int H, int R,
                            int dr, int heads_per_tile, int keys_per_split, int nsplit, int q_rows_are_heads,
                            __nv_bfloat16* __restrict__ out, float* __restrict__ partial, const float* __restrict__ sinks, int window,
-                           const __nv_bfloat16* __restrict__ head_gate, long long gate_ld, int q_head_rows) {
+                           const __nv_bfloat16* __restrict__ head_gate, long long gate_ld, int q_head_rows, unsigned char* wait_byte) {
   using namespace t5;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_q, bar_kfull[2], bar_kempty[2], bar_s[2], bar_p, bar_pv;
@@ -115,7 +116,10 @@ latent_attention_t5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
   __shared__ unsigned int seen_status;
   if (threadIdx.x == 0) seen_status = *reinterpret_cast<volatile unsigned int*>(&g_status);
   __syncthreads();
-  if (seen_status != 0u) return;      // an earlier CTA gave up: do not queue up behind it (uniform over the CTA)
+  if (seen_status != 0u) {            // an earlier CTA gave up: do not queue up behind it (uniform over the CTA)
+    if (threadIdx.x == 0) report_wait(wait_byte);
+    return;
+  }
   if (ntile == 0) {        // a split past this tile's context: an empty partial (uniform over the CTA)
     if (partial != nullptr)
       for (int r = threadIdx.x; r < nrows; r += blockDim.x) {
@@ -358,6 +362,7 @@ latent_attention_t5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
 
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && abort_flag) report_wait(wait_byte);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc<1>(tmem_base, t5::kTmemCols);
@@ -429,13 +434,15 @@ LLMCTL_API int llmctl_latent_attention_t5(const void* ql, int ql_bf16, long long
   rc = get_tmap_2d_bf16(&tmK, cache, cache_rows, D, D, t5::kKeys, 64, 1);
   if (rc) LLMCTL_FAIL(rc, "tensor map K");
   const int smem = (t5::kRows + 2 * t5::kKeys) * D * 2 + 1024;
+  unsigned char* const wait_byte = wait_report(kWaitLatentAttention);
+  LLMCTL_REQUIRE(wait_byte != nullptr);
   LLMCTL_CHECK(cudaFuncSetAttribute(latent_attention_t5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int ncg = (R + t5::kColGroup - 1) / t5::kColGroup;
   dim3 grid(ntiles, (H + heads_per_tile - 1) / heads_per_tile, splits * ncg);
   latent_attention_t5_kernel<<<grid, t5::kThreads, smem, s>>>(tmQ, tmK, block_tables, max_blocks, block_size, tiles, positions,
                                                                scale, H, R, dr, heads_per_tile, keys_per_split, splits,
                                                                rows_are_heads, (__nv_bfloat16*)out, splits > 1 ? partial : nullptr, sinks, window,
-                                                               (const __nv_bfloat16*)head_gate, gate_ld, qfull == nullptr ? tokens : 0);
+                                                               (const __nv_bfloat16*)head_gate, gate_ld, qfull == nullptr ? tokens : 0, wait_byte);
   if (splits > 1) {
     rc = launch_latent_attention_merge_bf16(partial, out, R, splits, tokens * H, H, head_gate, gate_ld, s);
     if (rc) LLMCTL_FAIL(rc, "merge");

@@ -10,6 +10,7 @@
 // an all-reduce, and "finalize"; both halves are exposed below.
 #include "../common/ptx.cuh"
 #include "../common/util.cuh"
+#include "../common/wait_status.h"
 
 namespace llmctl {
 
@@ -97,7 +98,7 @@ template <int kVec>
 __global__ void __launch_bounds__(kCEThreads, 1)
 ce_rows_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long* __restrict__ targets, float* __restrict__ loss_out,
                float* __restrict__ lse_out, int rows, int V, int stages, long long ignore_index, float host_scale,
-               const float* __restrict__ scale_dev, int write_grad) {
+               const float* __restrict__ scale_dev, int write_grad, unsigned char* wait_byte) {
   using namespace ptx;
   extern __shared__ __align__(128) uint8_t ring[];
   __shared__ uint64_t full[3];
@@ -238,6 +239,7 @@ ce_rows_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long
       for (int k = i; k < i + stages - 1 && first + k * step < rows; ++k, none = 0)
         mbar_wait_bounded(&full[k % stages], (k / stages) & 1, &none);
       atomicCAS(&g_ce_status, 0u, 1u);
+      report_wait(wait_byte);
     }
     tma_store_wait_read<0>();
   }
@@ -377,10 +379,12 @@ LLMCTL_API int llmctl_cross_entropy_fwd_bwd(void* logits, long long ld, const lo
   const size_t row_bytes = static_cast<size_t>(V) * 2;
   const int stages = row_bytes * 3 <= kCERingBytes ? 3 : 2;
   auto rows_launch = [&](auto kern) -> cudaError_t {
+    unsigned char* const wait_byte = wait_report(kWaitCrossEntropy);
+    if (wait_byte == nullptr) return cudaErrorMemoryAllocation;
     const cudaError_t e = allow_smem(kern, kCERingBytes);
     if (e != cudaSuccess) return e;
     kern<<<rows < kNumSMs ? rows : kNumSMs, kCEThreads, stages * row_bytes, s>>>((__nv_bfloat16*)logits, ld, targets, loss_per_row, lse_per_row, rows,
-                                                                                 V, stages, ignore_index, host_scale, scale_dev, write_grad);
+                                                                                 V, stages, ignore_index, host_scale, scale_dev, write_grad, wait_byte);
     return cudaSuccess;
   };
   // short rows: several CTAs per SM overlap each other; rows that do not fit the ring twice stream through L2

@@ -167,6 +167,37 @@ class NativeError(RuntimeError):
     pass
 
 
+# Kernels whose bounded waits report when they run out (csrc/common/wait_status.h), in the order of their bytes in the host word, with
+# the entry points that read and clear their device-side status.
+_WAITS = (("flash attention forward", "llmctl_flash_fwd_status"), ("flash attention backward", "llmctl_flash_bwd_status"),
+          ("cross-entropy", "llmctl_cross_entropy_status"), ("latent attention", "llmctl_latent_attention_t5_status"))
+_wait_word = ctypes.c_uint32(0)         # the library's word once a kernel has been launched
+_wait_bound = False
+
+
+def _bind_waits() -> None:
+    global _wait_word, _wait_bound
+    register_signature("llmctl_wait_status_word", [], restype=c_void_p)
+    address = _function("llmctl_wait_status_word")()
+    if address:
+        _wait_word = ctypes.c_uint32.from_address(address)
+    _wait_bound = True
+
+
+def check_waits(context: str = "") -> None:
+    """Raise ``NativeError`` if a bounded wait of a kernel has run out since the last report: what that launch and those after it computed
+    is invalid.  Reads a word of host memory, so it costs nothing, and sees what has finished: call it where the device has been waited for."""
+    value = _wait_word.value
+    if value:
+        _wait_word.value = 0
+        names = [name for i, (name, _) in enumerate(_WAITS) if value >> 8 * i & 0xff]
+        for _, status in _WAITS:
+            if has_symbol(status):
+                _function(status)(1)
+        raise NativeError(f"a bounded wait ran out in: {', '.join(names)}{(' (' + context + ')') if context else ''}; "
+                          "results since the last check are invalid")
+
+
 #: kernels launched per entry point when it is not exactly one
 _KERNELS_PER_CALL = {"llmctl_rmsnorm_bwd": 2, "llmctl_layernorm_bwd": 3, "llmctl_sumsq": 2, "llmctl_rmsnorm_bwd_noalloc": 2,
                      "llmctl_flash_attn_bwd": 2, "llmctl_rs_sumsq": 2, "llmctl_ag_gemm": 2,
@@ -176,6 +207,10 @@ _KERNELS_PER_CALL = {"llmctl_rmsnorm_bwd": 2, "llmctl_layernorm_bwd": 3, "llmctl
 def call(name: str, *args) -> None:
     """Invoke a C entry point and raise on a non-zero status."""
     global launch_count
+    if not _wait_bound:
+        _bind_waits()
+    if _wait_word.value:
+        check_waits("found before " + name)
     fn = _functions.get(name) or _function(name)
     if _nvtx.KERNEL_RANGES:
         with _nvtx.nvtx_range(name):

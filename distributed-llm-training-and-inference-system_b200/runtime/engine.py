@@ -35,6 +35,7 @@ from ..io.dataset import TokenLoader, build_dataset
 from ..models.config import ModelConfig, resolve_model
 from ..models.gpt import build_model
 from ..ops import functional as ops
+from ..ops import native
 from ..parallel.pp import PipelineSchedule, partition_layers
 from ..parallel.zero import ZeroOptimizer
 from ..utils.nvtx import nvtx_range
@@ -403,7 +404,7 @@ class TrainingEngine:
                 # the only host sync of the loop: once per logging window
                 loss = self._reduce_scalar(out["loss"])
                 gn = float(out["grad_norm"])
-                self._check_comm_watchdog(f"steps up to {step}")
+                self._check_waits(f"steps up to {step}")
                 self._guard_nonfinite(step, loss, gn)
                 dt = (time.perf_counter() - window_t0) / max(window_steps, 1)
                 if st.world_size > 1:
@@ -452,10 +453,11 @@ class TrainingEngine:
             raise RuntimeError(f"training diverged: {self.nonfinite_windows} consecutive logging windows with non-finite "
                                f"loss or gradient norm (last at step {step}); no checkpoint is written from this state")
 
-    def _check_comm_watchdog(self, context: str) -> None:
-        """Peer-memory kernels give up (instead of hanging the GPU) when a peer's flag never arrives; whatever
-        they produced after that is garbage, so this is checked wherever results leave the device: before a
-        logging window is reported and before a checkpoint is written."""
+    def _check_waits(self, context: str) -> None:
+        """Kernels give up (instead of hanging the GPU) when a wait runs out, peer-memory kernels when a peer's flag never
+        arrives; whatever they produced after that is garbage, so this is checked wherever results leave the device:
+        before a logging window is reported, after an evaluation and before a checkpoint is written."""
+        native.check_waits(context)
         if self.state.device.type == "cuda" and self.state.world_size > 1:
             from ..comms.symm import check_watchdog
             check_watchdog(context)
@@ -501,6 +503,7 @@ class TrainingEngine:
             if losses:
                 total += torch.stack(losses).sum().float()
         loss = self._reduce_scalar(total / n)
+        self._check_waits("this evaluation")
         self.best_eval_loss = min(self.best_eval_loss, loss)
         return {"eval_loss": loss, "perplexity": math.exp(min(loss, 30.0))}
 
@@ -509,7 +512,7 @@ class TrainingEngine:
         c = self.config
         if self.state.device.type == "cuda":
             torch.cuda.synchronize(self.state.device)
-        self._check_comm_watchdog("the steps before this checkpoint")
+        self._check_waits("the steps before this checkpoint")
         return ckpt_io.save_checkpoint(
             c.output_dir, self.global_step, self.model, self.optimizer, epoch=self.epoch, config=c.to_dict(),
             model_config=self.model_config,

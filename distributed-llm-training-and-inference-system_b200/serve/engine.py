@@ -32,6 +32,7 @@ from ..comms.mesh import get_state
 from ..models.config import ModelConfig, resolve_model
 from ..models.gpt import GPTModel, build_model
 from ..ops import functional as ops
+from ..ops import native
 from ..ops import serving as sops
 from .native_host import DECODE, PREFILL, BatchScheduler, KVBlockManager
 from .ragged import Portion, RaggedBatch
@@ -580,7 +581,9 @@ class InferenceEngine:
         if self.st.tp > 1:
             import torch.distributed as dist
             dist.broadcast(u, src=self.st.tp_ranks[0], group=self.st.tp_group)   # same draw on every TP rank
-        return sops.sample(logits, t, k, p, u).tolist()    # the step's only D2H copy
+        tokens = sops.sample(logits, t, k, p, u).tolist()  # the step's only D2H copy
+        native.check_waits("the step of these tokens")
+        return tokens
 
     # ---- one engine step ---------------------------------------------------------------------------------
     def step(self) -> List[Sequence]:

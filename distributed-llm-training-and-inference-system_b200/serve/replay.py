@@ -21,6 +21,8 @@ from typing import Dict, IO, List, Optional
 import numpy as np
 import torch
 
+from ..ops import native
+
 MAX_LIVE_REQUESTS = 4
 PAGE_TOKENS = 64
 
@@ -85,6 +87,7 @@ def run(model: str, dtype: str, out: str, max_tokens: int, device: Optional[str]
         logits = rp.step(obj)
         if logits is not None:
             a = logits.detach().to("cpu", torch.float32).contiguous().numpy().astype("<f4", copy=False)
+            native.check_waits(f"step {obj['step']}")
             tmp = outdir / f".{obj['step']}.part"
             a.tofile(tmp)
             tmp.replace(outdir / f"{obj['step']}.f32")

@@ -516,3 +516,15 @@ def test_skinny_gemm_k_tail_and_odd_shapes(cuda_device, M, N, K):
     y = ops.gemm_skinny(x, w)
     ref = x.float() @ w.float().t()
     assert ((y.float() - ref).abs().max() / ref.abs().max()).item() < 1e-2
+
+
+@pytest.mark.parametrize("which", [0, 1, 2, 3])
+def test_a_wait_reported_on_the_device_is_raised_on_the_host(cuda_device, which):
+    """The byte that a kernel sets when its wait runs out, set by a kernel that does nothing else."""
+    from llmctl_b200.ops import native
+    native.register_signature("llmctl_wait_status_report", [native.c_int, native.c_void_p])
+    native.call("llmctl_wait_status_report", which, native.stream_ptr())
+    torch.cuda.synchronize()
+    with pytest.raises(native.NativeError, match=native._WAITS[which][0]):
+        native.check_waits()
+    native.check_waits()

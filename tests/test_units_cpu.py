@@ -663,3 +663,59 @@ def test_paged_decode_scratch_is_counted_in_64_bits():
         one_wave = splits == 1 or (splits <= 8 and batch * heads * splits <= 3 * 148)
         want = 0 if one_wave else batch * heads * splits * (dim + 2)
         assert native.lib().llmctl_paged_attn_scratch_elems(batch, heads, dim, splits) == want
+
+
+@pytest.mark.parametrize("byte,name", [(0, "flash attention forward"), (1, "flash attention backward"), (2, "cross-entropy"), (3, "latent attention")])
+def test_waits_that_ran_out_are_raised_once_wherever_the_host_looks(monkeypatch, byte, name):
+    """The word that kernels write when a wait runs out, faked: reported by name at a check and before the next launch, then cleared."""
+    import ctypes
+    from llmctl_b200.ops import native
+    word, launched, cleared = ctypes.c_uint32(0), [], []
+    monkeypatch.setattr(native, "_wait_word", word)
+    monkeypatch.setattr(native, "_wait_bound", True)
+    monkeypatch.setattr(native, "_functions", {"llmctl_x": lambda *a: launched.append(a) or 0,
+                                               **{status: cleared.append for _, status in native._WAITS}})
+    native.check_waits("nothing")
+    native.call("llmctl_x", 1)
+    word.value = 1 << 8 * byte
+    with pytest.raises(native.NativeError, match=f"in: {name} \\(this step\\)"):
+        native.check_waits("this step")
+    assert word.value == 0 and cleared == [1, 1, 1, 1]
+    native.check_waits("again")
+    word.value = 1 << 8 * byte
+    with pytest.raises(native.NativeError, match=name):
+        native.call("llmctl_x", 2)
+    native.call("llmctl_x", 3)
+    assert launched == [(1,), (3,)]
+
+
+def test_training_and_serving_report_waits_that_ran_out(monkeypatch, tmp_path):
+    """A wait that ran out during a step ends training before the window is logged or a checkpoint is written, and a served step before its
+    tokens are handed out."""
+    import ctypes
+    from llmctl_b200.comms import mesh
+    from llmctl_b200.ops import native
+    from llmctl_b200.runtime.engine import TrainingEngine, create_training_config
+    from llmctl_b200.serve.engine import InferenceEngine
+    mesh.reset_state()
+    word = ctypes.c_uint32(0)
+    monkeypatch.setattr(native, "_wait_word", word)
+    eng = TrainingEngine(create_training_config(model_name_or_path="gpt-tiny", output_dir=str(tmp_path), batch_size=2, seq_len=16, max_steps=3,
+                                                logging_steps=1, eval_steps=0, kernels="native"))
+    step = eng.train_step
+    monkeypatch.setattr(eng, "train_step", lambda: (step(), setattr(word, "value", 1 << 8))[0])
+    with pytest.raises(native.NativeError, match="flash attention backward"):
+        eng.train()
+    assert eng.global_step == 1 and not list(tmp_path.rglob("*.safetensors"))
+    word.value = 1
+    with pytest.raises(native.NativeError, match="checkpoint"):
+        eng.save_checkpoint()
+    word.value = 1 << 16
+    with pytest.raises(native.NativeError, match="evaluation"):
+        eng.evaluate()
+    serving = InferenceEngine("gpt-tiny", device="cpu", kv_block_size=4, num_kv_blocks=64)
+    seq = serving.add_request([1, 2, 3], 4, 0.0, 1.0, -1)
+    word.value = 1
+    with pytest.raises(native.NativeError, match="tokens"):
+        serving.step()
+    assert seq.generated == []
