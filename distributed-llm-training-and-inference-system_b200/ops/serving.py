@@ -37,20 +37,26 @@ def choose_splits(batch: int, heads: int, max_context: int, block_size: int, sms
     # Decode attention is a latency-bound stream: each CTA walks block table -> K/V rows -> online softmax in a
     # dependent chain, so HBM only fills up with ~8 resident CTAs per SM.  Splits are whole KV blocks of >= 64 tokens;
     # the merge pass costs (head_dim + 2) floats per split, ~3 % of the K/V bytes at 64 tokens per split.
-    # Up to 8 splits a CTA walks at most 512 tokens: with longer walks a full batch of unlike contexts is one and a half waves
-    # of CTAs that end at different times.
-    want = max(1, (8 * sms + batch * heads - 1) // (batch * heads), min(8, (max_context + 511) // 512))
+    # Up to 512 (head, sequence) pairs a CTA walks at most 512 tokens where 8 splits allow it: with longer walks a full batch of unlike
+    # contexts is one and a half waves of CTAs that end at different times (us in ceil(8 sms / pairs) splits / in 8, 32 heads of 128, contexts
+    # from 1 K to 4 K: 16 sequences 154.6 / 140.3).  More pairs fill the waves by themselves, and what each split adds is lost (32 sequences
+    # 242.7 / 246.8, 64: 448 / 472, 256: 1692 / 1912; 64 sequences of up to 2304, 12 heads of 64: 72.9 / 85.0).
+    want = max(1, (8 * sms + batch * heads - 1) // (batch * heads), min(8, (max_context + 511) // 512) if batch * heads <= 512 else 1)
     per_split = max(block_size, (64 // block_size) * block_size) if block_size <= 64 else block_size
     return int(max(1, min(want, max(1, max_context // per_split), 256)))
 
 
-def _launch_splits(batch: int, heads: int, max_context: int, block_size: int, sms: int = 148) -> int:
+def _launch_splits(batch: int, heads: int, head_dim: int, max_context: int, block_size: int, sms: int = 148) -> int:
     # One launch, merged inside clusters of up to 8 splits, while all CTAs (three per SM) are resident together and none walks
-    # more than 768 tokens: one context of 4096, 32 heads of 128: 23 us with 37 splits and a merge kernel, 18 us with 8.  Larger batches
-    # and longer contexts take the finer splits of choose_splits.
-    one_wave = max(1, min(8, 3 * sms // (batch * heads)))
-    if max_context <= 768 * one_wave:
-        return max(1, min(one_wave, max_context // 64))
+    # more than 768 tokens (us in the splits of choose_splits with a merge kernel / in one launch: one context of 4096, 32 heads of 128
+    # 23 / 18; 8 of up to 2304, 4 heads 25.6 / 22.6; 4 of up to 700, 32 heads 25.6 / 20.5; 64 of 500, 4 heads 31.7 / 26.7).  Beyond one
+    # wave a single split without a merge kernel pays for the shortest walks only (64 of 500, 12 heads of 64: 39.9 / 37.0; 32 heads of
+    # 128: 68.6 / 75.8 for 32 of them); larger batches and longer contexts take choose_splits.
+    resident = min(8, 3 * sms // (batch * heads))
+    if max_context <= 768 * resident:
+        return max(1, min(resident, max_context // 64))
+    if resident == 0 and max_context * head_dim <= 512 * 64:
+        return 1
     return choose_splits(batch, heads, max_context, block_size, sms)
 
 
@@ -63,7 +69,7 @@ def paged_attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     block_size = k_cache.shape[1]
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     if q.is_cuda:
-        ns = num_splits or _launch_splits(B, H, max_context, block_size)
+        ns = num_splits or _launch_splits(B, H, D, max_context, block_size)
         need = native.lib().llmctl_paged_attn_scratch_elems(B, H, D, ns)
         if need and (scratch is None or scratch.numel() < need):
             scratch = torch.empty(need, dtype=torch.float32, device=q.device)

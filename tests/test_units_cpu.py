@@ -719,3 +719,15 @@ def test_training_and_serving_report_waits_that_ran_out(monkeypatch, tmp_path):
     with pytest.raises(native.NativeError, match="tokens"):
         serving.step()
     assert seq.generated == []
+
+
+# pairs of 512 / 513 and more: the splits of long contexts; 444 pairs (three CTAs on each of 148 SMs) / 445: one launch or the merge kernel
+@pytest.mark.parametrize("batch,heads,dim,context,splits,launch", [
+    (16, 32, 128, 4096, 8, 8), (16, 32, 128, 512, 3, 3), (19, 27, 128, 4096, 3, 3), (32, 32, 128, 4096, 2, 2), (32, 32, 128, 512, 2, 2),
+    (64, 32, 128, 4096, 1, 1), (256, 32, 128, 4096, 1, 1), (64, 12, 64, 512, 2, 1), (64, 12, 64, 1024, 2, 2), (37, 12, 64, 768, 3, 1),
+    (37, 12, 64, 769, 3, 3), (89, 5, 64, 768, 3, 3), (8, 4, 128, 2304, 36, 8), (1, 32, 128, 4096, 37, 8), (1, 32, 128, 8192, 37, 37),
+    (4, 32, 128, 1024, 10, 3), (64, 4, 128, 512, 5, 1), (1, 1, 64, 10, 1, 1)])
+def test_decode_splits_by_pairs_of_head_and_sequence(batch, heads, dim, context, splits, launch):
+    from llmctl_b200.ops import serving
+    assert serving.choose_splits(batch, heads, context, 16) == splits
+    assert serving._launch_splits(batch, heads, dim, context, 16) == launch
