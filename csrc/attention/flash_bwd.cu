@@ -610,6 +610,9 @@ LLMCTL_API int llmctl_flash_attn_bwd(const void* q, const void* k, const void* v
   LLMCTL_REQUIRE(static_cast<long long>(B) * H * ((S + 31) / 32) < (1ll << 31));
   LLMCTL_REQUIRE(q_tok_stride % 8 == 0 && k_tok_stride % 8 == 0 && v_tok_stride % 8 == 0 && o_tok_stride % 8 == 0 &&
                  dqkv_tok_stride % 8 == 0);
+  LLMCTL_REQUIRE(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(o) |
+                   reinterpret_cast<uintptr_t>(d_o) | reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) |
+                   reinterpret_cast<uintptr_t>(dv) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0);
   const int rc = (D == 128 ? flash_bwd_launch<128> : flash_bwd_launch<64>)(
       q, k, v, o, d_o, lse, dq, dk, dv, scratch, B, S, H, q_tok_stride, k_tok_stride, v_tok_stride, o_tok_stride, dqkv_tok_stride, scale,
       causal, (cudaStream_t)stream);

@@ -551,7 +551,7 @@ LLMCTL_API int llmctl_flash_attn_fwd(const void* q, const void* k, const void* v
   LLMCTL_BEGIN();
   LLMCTL_REQUIRE((D == 128 || D == 64) && (causal || S % 128 == 0) && B > 0 && S > 0 && H > 0);
   LLMCTL_REQUIRE(q_tok_stride % 8 == 0 && k_tok_stride % 8 == 0 && v_tok_stride % 8 == 0 && o_tok_stride % 8 == 0);
-  LLMCTL_REQUIRE(scale > 0.f);
+  LLMCTL_REQUIRE(scale > 0.f && (reinterpret_cast<uintptr_t>(o) & 15) == 0);      // q, k, v: the tensor maps check them
   CUtensorMap tq, tk, tv;
   int rc = 0;
   auto mkmap = [&](CUtensorMap* m, const void* base, long long tok) {

@@ -57,8 +57,14 @@ def _native_ok(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool =
 
 
 def _stats_scratch(B: int, S: int, H: int, device: torch.device) -> torch.Tensor:
-    """Scratch of the backward kernels: two numbers per (head, query), sequences rounded up to whole tiles, and two counters."""
+    """Scratch of the backward: two numbers per (head, query), sequences rounded up to whole tiles, and the item counter (in two words)."""
     return torch.empty(2 * B * H * ((S + 127) // 128 * 128) + 2, dtype=torch.float32, device=device)
+
+
+def _whole_units(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous from a 16-byte boundary, as the backward kernels read it."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 class _FlashAttnFn(torch.autograd.Function):
@@ -79,7 +85,7 @@ class _FlashAttnFn(torch.autograd.Function):
         q, k, v, o, lse = ctx.saved_tensors
         if native.has_symbol("llmctl_flash_attn_bwd"):
             B, S, H, D = q.shape
-            do = do.contiguous()
+            do = _whole_units(do)
             # dq|dk|dv packed like the forward's qkv so the following wgrad GEMM sees one tensor
             dqkv = torch.empty(B, S, 3, H, D, dtype=q.dtype, device=q.device)
             dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
@@ -200,7 +206,7 @@ class _RopeAttnPackedFn(torch.autograd.Function):
         d5 = dqkv.view(B, S, 3, H, D)
         do4 = do.reshape(B, S, H, D)
         if use_native and native.has_symbol("llmctl_flash_attn_bwd"):
-            do4 = do4.contiguous()
+            do4 = _whole_units(do4)
             scratch = _stats_scratch(B, S, H, qkv.device)
             native.call("llmctl_flash_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do4.data_ptr(),
                         lse.data_ptr(), d5[:, :, 0].data_ptr(), d5[:, :, 1].data_ptr(), d5[:, :, 2].data_ptr(),

@@ -478,6 +478,28 @@ def test_flash_attention_edges_of_blocks(cuda_device, B, S, H, D, causal, shift)
             assert (a - b).norm() <= bound, f"{name} head {h}: {((a - b).norm() / b.norm()).item():.2e}"
 
 
+@pytest.mark.parametrize("S,D", [(130, 64), (128, 64), (77, 128), (128, 128)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_flash_attention_gradients_at_odd_addresses(cuda_device, S, D, packed):
+    """The incoming gradient is read in 16-byte units: one that begins elsewhere is copied, and the gradients are those of the copy."""
+    from llmctl_b200.ops import attention as attn, functional as ops
+    torch.manual_seed(S)
+    B, H = 2, 3
+    flat = torch.randn(B * S * H * D + 1, device=cuda_device).bfloat16()
+    odd = flat[1:]
+    assert odd.data_ptr() % 16 == 2
+    leaf = torch.randn(B * S, 3 * H * D, device=cuda_device).bfloat16().requires_grad_(True)
+    cos, sin = ops.rope_tables(D, S, device=cuda_device)
+    def grad(do):
+        x = leaf * 1
+        if packed:
+            o = attn.rope_attention_packed(x, cos, sin, B, S, H, D)
+        else:
+            o = attn.attention(*x.view(B, S, 3, H, D).unbind(2))
+        return torch.autograd.grad(o, leaf, do.view(o.shape))[0]
+    assert torch.equal(grad(odd), grad(odd.clone()))
+
+
 def test_flash_backward_of_short_items_beside_other_work(cuda_device):
     """One block per sequence: thousands of the shortest items in a row, while copies on another stream slow the stores of the
     accumulators down.  The gradients are those of an undisturbed run, bit for bit, and no wait runs out."""
