@@ -182,7 +182,8 @@ ce_rows_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long
     const float pm = lane < kCEThreads / 32 ? red_m[i & 1][lane] : -INFINITY;
     const float ps = lane < kCEThreads / 32 ? red_s[i & 1][lane] : 0.f;
     const float mx = warp_max(pm);
-    const float sum = warp_sum(pm == -INFINITY && ps == 0.f ? 0.f : ps * __expf(pm - mx));
+    float sum = warp_sum(pm == -INFINITY && ps == 0.f ? 0.f : ps * __expf(pm - mx));
+    if (mx == -INFINITY) sum = NAN;      // a row without a finite logit has no distribution: NaN in its loss and gradient, as everywhere else
     if (threadIdx.x == 0) {
       const float lse = mx + __logf(sum);
       if (lse_out) lse_out[row] = lse;
@@ -190,7 +191,7 @@ ce_rows_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long
     }
     if (write_grad) {
       const float scale = ignored ? 0.f : scale0, by = scale / sum;
-      const float mine = m == -INFINITY ? 0.f : __expf(m - mx) * by;
+      const float mine = __expf(m - mx) * by;
 #pragma unroll
       for (int v = 0; v < kVec; ++v) {
         const int at = v * kCEThreads + threadIdx.x;

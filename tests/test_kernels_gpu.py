@@ -550,3 +550,33 @@ def test_a_wait_reported_on_the_device_is_raised_on_the_host(cuda_device, which)
     with pytest.raises(native.NativeError, match=native._WAITS[which][0]):
         native.check_waits()
     native.check_waits()
+
+
+@pytest.mark.parametrize("V", [8192, 8200, 16392, 32000, 40000, 56328])
+def test_cross_entropy_of_rows_that_are_not_finite(cuda_device, V):
+    """Rows without a finite logit, with an infinite one or with a NaN: NaN in the loss and in the whole row's gradient, on every path (short
+    rows in registers, rows in the ring with exponentials kept and without, streamed rows), and nowhere else; parts masked to -inf stay 0."""
+    from llmctl_b200.ops import functional as ops
+    torch.manual_seed(V)
+    inf = float("inf")
+    x = torch.randn(9, V, device=cuda_device).bfloat16()
+    x[0] = -inf
+    x[1, 5] = inf
+    x[2, V - 1] = float("nan")
+    x[3, : V // 2] = -inf
+    x[4, 1:] = -inf
+    x[5] = -inf
+    x[6, 3:V - 3] = -inf
+    t = torch.tensor([0, 7, 9, V - 1, 0, -100, 1, 3, -100], device=cuda_device)
+    ref = x.float().requires_grad_(True)
+    rows = torch.nn.functional.cross_entropy(ref, t, reduction="none")
+    rows.sum().backward()
+    for i in range(9):
+        leaf = x[i:i + 1].clone().requires_grad_(True)
+        loss = ops.cross_entropy(leaf * 1, t[i:i + 1])
+        grad = torch.autograd.grad(loss, leaf)[0]
+        assert torch.equal(grad.isnan(), ref.grad[i:i + 1].isnan()), i
+        assert bool(loss.isnan()) == bool(rows[i].isnan()), i
+        if not ref.grad[i].isnan().any():
+            assert torch.allclose(grad.float(), ref.grad[i:i + 1], rtol=2.0 ** -7, atol=1e-6), i
+            assert torch.allclose(loss, rows[i], rtol=1e-4, atol=1e-5), i
