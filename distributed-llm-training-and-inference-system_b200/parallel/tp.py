@@ -196,19 +196,22 @@ class RowParallelLinear(nn.Module):
         return y_local
 
 
-_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
-_OWN = ((ColumnParallelLinear.forward, None), (RowParallelLinear.forward, RowParallelLinear.finish))
+_CALL, _every = nn.Module.__call__, torch.nn.modules.module
+_OWN = {ColumnParallelLinear: (ColumnParallelLinear.forward, None), RowParallelLinear: (RowParallelLinear.forward, RowParallelLinear.finish)}
 
 
 def runs_plain(layer: nn.Module) -> bool:
     """Whether calling ``layer`` is ``ops.linear(x, layer.weight)`` and nothing else, so that a fused caller may take its weight and pass
-    it by: one rank, one of the two layers above with the ``forward`` that stands there (a subclass, an instance or a module put in its
-    place may do more), and no hook on it or on all modules that would want to see the call."""
-    t, every = type(layer), torch.nn.modules.module
-    return ((getattr(t, "forward", None), getattr(t, "finish", None)) in _OWN
-            and t.__call__ is nn.Module.__call__ and not layer.__dict__.keys() & {"forward", "finish", "__call__"}
-            and getattr(layer, "_compiled_call_impl", None) is None and get_state().tp == 1
-            and not any(getattr(layer, h) or getattr(every, "_global" + h) for h in _HOOKS))
+    it by: one rank, one of the two layers above with the methods that stand there (a subclass, an instance or a module put in its place
+    may do more), and no hook on it or on all modules that would want to see the call."""
+    t, d = type(layer), layer.__dict__
+    own = _OWN.get(t)
+    return (own is not None and t.forward is own[0] and getattr(t, "finish", None) is own[1] and t.__call__ is _CALL
+            and not ("forward" in d or "finish" in d or d.get("_compiled_call_impl")
+                     or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
+                     or _every._global_forward_hooks or _every._global_forward_pre_hooks
+                     or _every._global_backward_hooks or _every._global_backward_pre_hooks)
+            and get_state().tp == 1)
 
 
 class VocabParallelEmbedding(nn.Module):
