@@ -92,18 +92,24 @@ __device__ __forceinline__ void gate_wait_b(const GemmGate& g, int n0, int n_end
 constexpr int kBM = 128;
 constexpr int kBK = 64;  // 64 bf16 = one 128-byte swizzle row
 constexpr int kGemmThreads = 192;
-// Output staging of the epilogue: per warp two buffers of 32 rows x 64 bf16 (128-byte swizzle) that TMA stores read.
+// Output staging of the epilogue: boxes of 32 rows x 64 bf16 (128-byte swizzle) that TMA stores read.  Each of the four warps has one
+// buffer, two with a gated activation.  A second one for the plain product gains nothing (its stores hide behind the next tile's main loop,
+// and a CTA's last tile is staged in the operand ring, see OutStage) and takes the room that the kernels of the communication streams
+// (fused/ag_push.cu, fused/rs_adam.cu) need beside a persistent GEMM, which holds its SM's shared memory to the end: with it one of their
+// CTAs fitted, where their registers allow two; beside a gated activation's 196-209 registers they allow one.
 constexpr int kOutBox = 32 * 128;
-constexpr int kOutBytes = 4 * 2 * kOutBox;
+constexpr int kSmShared = 228 * 1024, kNeighbourShared = 1280;      // of an SM; of such a CTA (static, the reserved KB, rounded up)
+enum class Gated { kNone, kForward, kBackward };
+constexpr int out_bufs(Gated g) { return g == Gated::kNone ? 1 : 2; }
 
-template <int BN>
+template <int BN, Gated kGated = Gated::kNone>
 struct GemmCfg {
   static constexpr int kStages = (BN == 256 || BN == 192) ? 4 : (BN == 128 ? 6 : 8);
   static constexpr int kABytes = kBM * kBK * 2;
   static constexpr int kBBytes = BN * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kOutAt = kStages * kStageBytes;
-  static constexpr int kSmemBytes = kOutAt + kOutBytes + 1024;    // + alignment slack
+  static constexpr int kSmemBytes = kOutAt + 4 * out_bufs(kGated) * kOutBox + 1024;    // + alignment slack
   static constexpr int kTmemCols = (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;   // power of two >= 2 accumulators of BN columns
 };
 
@@ -124,13 +130,30 @@ __device__ __forceinline__ void tile_to_mn(int tile, int num_m, int num_n, int& 
   n_blk = in_group / gsize;
 }
 
-// One 32-row x 64-column box: `pair(e)` gives columns 2e and 2e + 1 of this lane's row, packed to bf16; buffers alternate.
-template <typename Pair>
-__device__ __forceinline__ void stage_box(uint8_t* out_smem, uint32_t& out_n, const CUtensorMap* tm, int col0, int row0, int lane, Pair pair) {
-  uint8_t* buf = out_smem + (out_n & 1u) * kOutBox;
-  ++out_n;
-  if (lane == 0) tma_store_wait_read<1>();          // the store before the last has left this buffer
-  __syncwarp();
+// Where a warp stages its boxes: kBufs buffers in turn, or, for the last tile of a CTA, a buffer per box in the operand ring, which is
+// idle by then (the accumulator is finished, so every load has landed and been read).  Nobody waits for a store there: a problem of one
+// wave is nothing but last tiles, and its epilogue is exposed (2048 x 2048 x 4096: 31.6 us with two buffers, 32.8 with one and no ring).
+template <int kBufs>
+struct OutStage {
+  uint8_t* at;
+  uint32_t n;              // boxes so far
+  bool last;
+  __device__ __forceinline__ void begin(uint8_t* bufs, uint8_t* ring, int q, int boxes, bool last_tile) {
+    last = last_tile;
+    at = last ? ring + q * boxes * kOutBox : bufs + q * kBufs * kOutBox;
+    if (last) n = 0;
+  }
+};
+
+// One 32-row x 64-column box: `pair(e)` gives columns 2e and 2e + 1 of this lane's row, packed to bf16.
+template <int kBufs, typename Pair>
+__device__ __forceinline__ void stage_box(OutStage<kBufs>& out, const CUtensorMap* tm, int col0, int row0, int lane, Pair pair) {
+  uint8_t* buf = out.at + (out.last ? out.n : out.n % kBufs) * kOutBox;
+  ++out.n;
+  if (!out.last) {
+    if (lane == 0) tma_store_wait_read<kBufs - 1>();          // the store that last read this buffer is through
+    __syncwarp();
+  }
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(pair(4 * j), pair(4 * j + 1), pair(4 * j + 2), pair(4 * j + 3));
@@ -147,7 +170,7 @@ __device__ __forceinline__ void stage_box(uint8_t* out_smem, uint32_t& out_n, co
 // buffer and one lane stores the box, while the next columns are read.  A row per lane straight to global memory touches 32 lines
 // per instruction: an exposed epilogue (the problem is one tile per CTA) took longer than the main loop of K = 768.
 template <int BN, typename OutT>
-__device__ __forceinline__ void gemm_epilogue(uint32_t t_row, uint8_t* out_smem, uint32_t& out_n, const CUtensorMap* tmC,
+__device__ __forceinline__ void gemm_epilogue(uint32_t t_row, OutStage<1>& out, const CUtensorMap* tmC,
                                               OutT* __restrict__ C, long long ldc, int row0, int n0, int M, int N, int beta, int lane) {
   if constexpr (sizeof(OutT) == 2) {
     if (!beta) {
@@ -158,7 +181,7 @@ __device__ __forceinline__ void gemm_epilogue(uint32_t t_row, uint8_t* out_smem,
         tmem_ld_x32(t_row + c * 64 + 32, r + 32);
         tmem_ld_wait();
         if (row0 >= M || n0 + c * 64 >= N) continue;      // uniform over the warp
-        stage_box(out_smem, out_n, tmC, n0 + c * 64, row0, lane,
+        stage_box(out, tmC, n0 + c * 64, row0, lane,
                   [&](int e) { return pack_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])); });
       }
       return;
@@ -207,7 +230,6 @@ __device__ __forceinline__ void gemm_epilogue(uint32_t t_row, uint8_t* out_smem,
 
 // Gated up-projection (llmctl_gemm_swiglu_bf16): the tile's first half of columns multiplies rows of the gate matrix, the second half the
 // same rows of the up matrix, and the epilogue stores silu(gate) * up, and gate and up beside it when the backward will want them.
-enum class Gated { kNone, kForward, kBackward };
 struct SwigluMaps {
   CUtensorMap w_up, gate, up, act;
   int keep;                  // gate and up are stored
@@ -215,7 +237,7 @@ struct SwigluMaps {
   long long ldgu;
 };
 template <int BN>
-__device__ __forceinline__ void swiglu_epilogue(uint32_t t_row, uint8_t* out_smem, uint32_t& out_n, const SwigluMaps& maps, int row0, int f0,
+__device__ __forceinline__ void swiglu_epilogue(uint32_t t_row, OutStage<2>& out, const SwigluMaps& maps, int row0, int f0,
                                                 int M, int F, int lane) {
 #pragma unroll 1
   for (int c = 0; c < BN / 128; ++c) {
@@ -229,14 +251,14 @@ __device__ __forceinline__ void swiglu_epilogue(uint32_t t_row, uint8_t* out_sme
     if (row0 >= M || col >= F) continue;               // uniform over the warp
     auto packed = [](const uint32_t* r, int e) { return pack_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])); };
     if (maps.keep) {
-      stage_box(out_smem, out_n, &maps.gate, col, row0, lane, [&](int e) { return packed(g, e); });
-      stage_box(out_smem, out_n, &maps.up, col, row0, lane, [&](int e) { return packed(u, e); });
+      stage_box(out, &maps.gate, col, row0, lane, [&](int e) { return packed(g, e); });
+      stage_box(out, &maps.up, col, row0, lane, [&](int e) { return packed(u, e); });
     }
     auto act = [](uint32_t gv, uint32_t uv) {          // silu first, as in swiglu.cu: x * up may overflow where silu(x) * up does not
       const float x = __uint_as_float(gv);
       return x * __fdividef(1.f, 1.f + __expf(-x)) * __uint_as_float(uv);
     };
-    stage_box(out_smem, out_n, &maps.act, col, row0, lane, [&](int e) { return pack_bf16x2(act(g[2 * e], u[2 * e]), act(g[2 * e + 1], u[2 * e + 1])); });
+    stage_box(out, &maps.act, col, row0, lane, [&](int e) { return pack_bf16x2(act(g[2 * e], u[2 * e]), act(g[2 * e + 1], u[2 * e + 1])); });
   }
 }
 
@@ -313,7 +335,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate,
                     const __grid_constant__ SwigluMaps sw) {
-  using Cfg = GemmCfg<BN>;
+  using Cfg = GemmCfg<BN, kGated>;
+  static_assert(Cfg::kSmemBytes + 1280 + (kGated == Gated::kNone ? 2 : 1) * kNeighbourShared <= kSmShared, "no room for the kernels beside this one");
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[Cfg::kStages];
   __shared__ uint64_t bar_empty[Cfg::kStages];
@@ -443,8 +466,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   } else {
     // ------------------------------ epilogue (4 warps) ------------------------------
     const int q = warp & 3;  // TMEM lane quadrant this warp may access
-    uint8_t* out_smem = smem + Cfg::kOutAt + q * 2 * kOutBox;
-    uint32_t out_n = 0;
+    OutStage<out_bufs(kGated)> out{nullptr, 0u, false};
     int acc = 0;
     uint32_t aphase = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
@@ -457,12 +479,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       mbar_wait(&bar_tfull[acc], aphase);
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
+      out.begin(smem + Cfg::kOutAt, smem, q, BN / 64, kGated == Gated::kNone && tile + static_cast<int>(gridDim.x) >= num_tiles);
       if constexpr (kSwiglu)
-        swiglu_epilogue<BN>(t_row, out_smem, out_n, sw, m0 + q * 32, n0, M, N, lane);
+        swiglu_epilogue<BN>(t_row, out, sw, m0 + q * 32, n0, M, N, lane);
       else if constexpr (kGated == Gated::kBackward)
-        swiglu_bwd_epilogue<BN>(t_row, out_smem, sw, m0 + q * 32, n0, M, N, lane);
+        swiglu_bwd_epilogue<BN>(t_row, out.at, sw, m0 + q * 32, n0, M, N, lane);
       else
-        gemm_epilogue<BN, OutT>(t_row, out_smem, out_n, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
+        gemm_epilogue<BN, OutT>(t_row, out, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_tempty[acc]);
@@ -494,7 +517,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // ================================================================================================
 // PBN = N of the pair tile: 256 (the throughput tile) or 128 (half the work per tile: fills the last wave of the
 // 1-3 wave problems of a TP=8 shard, where a 256 x 256 tile is 26 us of tensor-core time).
-template <int PBN>
+template <int PBN, Gated kGated = Gated::kNone>
 struct Gemm2Cfg {
   static constexpr int kBN = PBN;
   static constexpr int kStages = (PBN == 256) ? 6 : 8;
@@ -502,7 +525,7 @@ struct Gemm2Cfg {
   static constexpr int kBBytes = (kBN / 2) * kBK * 2;    // (PBN/2) x 64 per CTA
   static constexpr int kStageBytes = kABytes + kBBytes;  // 32 / 24 KB per CTA
   static constexpr int kOutAt = kStages * kStageBytes;
-  static constexpr int kSmemBytes = kOutAt + kOutBytes + 1024;
+  static constexpr int kSmemBytes = kOutAt + 4 * out_bufs(kGated) * kOutBox + 1024;
   static constexpr int kTmemCols = 2 * PBN;              // 512 / 256
 };
 
@@ -511,7 +534,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate,
                     const __grid_constant__ SwigluMaps sw) {
-  using Cfg = Gemm2Cfg<PBN>;
+  using Cfg = Gemm2Cfg<PBN, kGated>;
+  static_assert(Cfg::kSmemBytes + 1280 + (kGated == Gated::kNone ? 2 : 1) * kNeighbourShared <= kSmShared, "no room for the kernels beside this one");
   constexpr int BN = Cfg::kBN;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[Cfg::kStages];
@@ -638,8 +662,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   } else {
     // ------------------------------ epilogue (4 warps, both CTAs) ------------------------------
     const int q = warp & 3;
-    uint8_t* out_smem = smem + Cfg::kOutAt + q * 2 * kOutBox;
-    uint32_t out_n = 0;
+    OutStage<out_bufs(kGated)> out{nullptr, 0u, false};
     int acc = 0;
     uint32_t aphase = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
@@ -651,12 +674,13 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       mbar_wait(&bar_tfull[acc], aphase);
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
+      out.begin(smem + Cfg::kOutAt, smem, q, BN / 64, kGated == Gated::kNone && tile + num_pairs >= num_tiles);
       if constexpr (kSwiglu)
-        swiglu_epilogue<BN>(t_row, out_smem, out_n, sw, m0 + q * 32, n0, M, N, lane);
+        swiglu_epilogue<BN>(t_row, out, sw, m0 + q * 32, n0, M, N, lane);
       else if constexpr (kGated == Gated::kBackward)
-        swiglu_bwd_epilogue<BN>(t_row, out_smem, sw, m0 + q * 32, n0, M, N, lane);
+        swiglu_bwd_epilogue<BN>(t_row, out.at, sw, m0 + q * 32, n0, M, N, lane);
       else
-        gemm_epilogue<BN, OutT>(t_row, out_smem, out_n, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
+        gemm_epilogue<BN, OutT>(t_row, out, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(&bar_tempty[acc], 0);   // always the leader's barrier
@@ -789,13 +813,13 @@ static int launch_swiglu(const void* X, const void* W, void* GU, void* ACT, int 
   const int tiles = ((M + (kPair ? 2 : 1) * kBM - 1) / ((kPair ? 2 : 1) * kBM)) * ((F + kCols - 1) / kCols);
   if constexpr (kPair) {
     auto kern = gemm2_tcgen05_kernel<256, false, false, __nv_bfloat16, Gated::kForward>;
-    LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256>::kSmemBytes));
+    LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256, Gated::kForward>::kSmemBytes));
     const int pairs = tiles < num_sms() / 2 ? tiles : num_sms() / 2;
-    kern<<<2 * pairs, kGemmThreads, Gemm2Cfg<256>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0, GemmGate{}, sw);
+    kern<<<2 * pairs, kGemmThreads, Gemm2Cfg<256, Gated::kForward>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0, GemmGate{}, sw);
   } else {
     auto kern = gemm_tcgen05_kernel<128, false, false, __nv_bfloat16, Gated::kForward>;
-    LLMCTL_CHECK(allow_smem(kern, GemmCfg<128>::kSmemBytes));
-    kern<<<tiles < num_sms() ? tiles : num_sms(), kGemmThreads, GemmCfg<128>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0,
+    LLMCTL_CHECK(allow_smem(kern, GemmCfg<128, Gated::kForward>::kSmemBytes));
+    kern<<<tiles < num_sms() ? tiles : num_sms(), kGemmThreads, GemmCfg<128, Gated::kForward>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0,
                                                                                             GemmGate{}, sw);
   }
   LLMCTL_RETURN_LAST();
@@ -822,12 +846,12 @@ static int launch_swiglu_bwd(const void* DY, const void* W, const void* GU, void
   const int grid = tiles < most ? tiles : most;
   if constexpr (kPair) {
     auto kern = gemm2_tcgen05_kernel<256, false, true, __nv_bfloat16, Gated::kBackward>;
-    LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256>::kSmemBytes));
-    kern<<<2 * grid, kGemmThreads, Gemm2Cfg<256>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw);
+    LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256, Gated::kBackward>::kSmemBytes));
+    kern<<<2 * grid, kGemmThreads, Gemm2Cfg<256, Gated::kBackward>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw);
   } else {
     auto kern = gemm_tcgen05_kernel<kBN, false, true, __nv_bfloat16, Gated::kBackward>;
-    LLMCTL_CHECK(allow_smem(kern, GemmCfg<kBN>::kSmemBytes));
-    kern<<<grid, kGemmThreads, GemmCfg<kBN>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw);
+    LLMCTL_CHECK(allow_smem(kern, GemmCfg<kBN, Gated::kBackward>::kSmemBytes));
+    kern<<<grid, kGemmThreads, GemmCfg<kBN, Gated::kBackward>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw);
   }
   LLMCTL_RETURN_LAST();
 }
