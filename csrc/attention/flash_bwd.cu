@@ -397,7 +397,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     uint32_t g = 0, k = 0;
     auto run = [&](auto kind, int rb, int bh, int first, int n) {
       constexpr bool kDQ = decltype(kind)::value;
-      float row_nl = 0.f, row_nd = 0.f;                   // dQ kernel: this query row's statistics
+      float row_nl = 0.f, row_nd = 0.f;                   // dQ items: this query row's statistics
       if (kDQ) {
         row_nl = nl2[static_cast<long long>(bh) * Sp + rb * kBlk + row];
         row_nd = ndl[static_cast<long long>(bh) * Sp + rb * kBlk + row];

@@ -274,7 +274,7 @@ LLMCTL_API int llmctl_kv_append(const void* qkv, long long row_stride, int k_off
 
 // One launch, merged inside clusters: one split, or up to 8 while all CTAs are resident together.  A CTA that ends early waits for
 // its cluster and keeps its place on the SM meanwhile, so beyond one wave of unlike contexts clusters lose (16 contexts of 1200-4096,
-// 32 heads, 8 splits, with the loads in registers: 252 us in clusters, 195 us with a merge kernel; with the ring 131 us with one); below,
+// 32 heads, 8 splits, with the loads in registers: 252 us in clusters, 195 us with a merge kernel; with the ring 127 us with one); below,
 // the second launch is a third of the time (300 keys, 12 heads of 64: 6.0 us in two launches, 4.1 us in one).
 static bool decode_in_clusters(long long batch, int heads, int num_splits) {
   return num_splits == 1 || (num_splits <= kMaxClusterSplits && batch * heads * num_splits <= 3 * kNumSMs);

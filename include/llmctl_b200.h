@@ -69,6 +69,10 @@ int llmctl_cross_entropy_fwd_bwd(void* logits, long long ld, const long long* ta
                                  float* loss_per_row, float* lse_per_row, int rows, int V,
                                  long long ignore_index, float host_scale, const float* scale_dev,
                                  int write_grad, void* stream);
+/* Waits of kernels that ran out (csrc/common/wait_status.h): the host word that they set, one byte per kernel, or NULL; and a kernel that
+ * sets byte `which` and does nothing else. */
+void* llmctl_wait_status_word(void);
+int llmctl_wait_status_report(int which, void* stream);
 /* 0 unless a bounded wait of the loss kernel ran out since the last clearing call (synchronises the device). */
 int llmctl_cross_entropy_status(int clear);
 int llmctl_cross_entropy_partial(const void* logits, long long ld, const long long* targets,
@@ -83,7 +87,8 @@ int llmctl_cross_entropy_finalize(void* logits, long long ld, const long long* t
  * D[M,N] = op(A) op(B) (+ D if beta).  a_mn=0: A is [M,K] row-major; a_mn=1: A stored [K,M].
  * b_mn=0: B is [N,K] row-major (Linear weight); b_mn=1: B stored [K,N].
  * out_fp32: D fp32 else bf16.  tile_n: 0 auto | 64 | 128 | 192 | 256 (single-CTA tiles) | 2 = 256x256 and 3 = 256x128 tile on a CTA pair
- * (cta_group::2); auto picks the 256x256 pair tile whenever M, N > 128.  max_ctas: 0 = all SMs. */
+ * (cta_group::2); auto picks the narrowest of 64 and 128 with which the problem is one wave of tiles, else the 256x256 pair tile
+ * whenever M, N > 128.  max_ctas: 0 = all SMs. */
 int llmctl_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                      long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32, int beta,
                      int tile_n, int max_ctas, void* stream);
@@ -124,7 +129,8 @@ int llmctl_gemm_skinny_bf16(const void* X, const void* W, void* C, int Mb, int N
  * elements; lse: fp32 [B,H,S] (natural log).  Any S when causal, else a multiple of 128.  Reference: SDPA/eager inside
  * the HF model (engine.py:284); baseline cuDNN SDPA.
  * Forward: 256 queries per work item as two tiles sharing K/V, S/P/O in TMEM, P never leaves TMEM.
- * Backward: two deterministic kernels (dK/dV on transposed scores, then dQ); scratch: 2*B*H*(S rounded up to 128) + 2 floats.
+ * Backward: a pass for the rows' statistics, then one deterministic kernel over dK/dV items (transposed scores) and dQ items;
+ * scratch: 2*B*H*(S rounded up to 128) + 2 floats.  All pointers at 16-byte boundaries.
  * llmctl_flash_{fwd,bwd}_status: 0 unless a bounded wait ran out since the last clearing call (synchronises the device). */
 int llmctl_flash_fwd_status(int clear);
 int llmctl_flash_bwd_status(int clear);

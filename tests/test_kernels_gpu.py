@@ -421,7 +421,7 @@ def test_flash_attention_ragged_lengths_use_the_native_kernel(cuda_device, S):
 
 
 def test_flash_attention_head_dim_64_uses_the_native_kernel(cuda_device):
-    """head_dim 64 (gpt-125m): zero-padded to the kernel's 128-wide head, forward and backward vs the fp32 reference."""
+    """head_dim 64 (gpt-125m) at a ragged length: forward and backward vs the fp32 reference."""
     from llmctl_b200.ops import attention as attn, native
     if not native.has_symbol("llmctl_flash_attn_bwd"):
         pytest.skip("flash attention kernels not built")

@@ -51,7 +51,8 @@ elif what == "swiglu":
     for _ in range(4):
         ops.swiglu(gu).sum().backward()
 elif what == "paged":
-    B, H, D, ctx, bs = 8, 4, 128, 2304, 16
+    B, H, ctx = (int(v) for v in sys.argv[2:5]) if len(sys.argv) > 4 else (8, 4, 2304)
+    D, bs = 128, 16
     nb = B * (ctx // bs)
     kc = torch.randn(nb, bs, H, D, device=dev).bfloat16(); vc = torch.randn_like(kc)
     bt = torch.arange(nb, device=dev, dtype=torch.int32).view(B, -1); cl = torch.full((B,), ctx, device=dev, dtype=torch.int32)
