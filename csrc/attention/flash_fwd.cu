@@ -575,7 +575,8 @@ LLMCTL_API int llmctl_latent_prompt_attention(const void* q, long long ldq, long
                                               long long key_rows, const int* seqs, int B, int max_q, int H, void* out, float scale,
                                               void* stream) {
   LLMCTL_BEGIN();
-  LLMCTL_REQUIRE(B > 0 && max_q > 0 && H > 0 && tokens > 0 && key_rows > 0 && key_rows % 128 == 0 && ldq % 8 == 0 && scale > 0.f && seqs != nullptr);
+  LLMCTL_REQUIRE(B > 0 && max_q > 0 && H > 0 && tokens > 0 && key_rows > 0 && key_rows % 128 == 0 && ldq % 8 == 0 && scale > 0.f && seqs != nullptr &&
+                 (reinterpret_cast<uintptr_t>(out) & 15) == 0);
   CUtensorMap tq, tk, tks, tv;
   int rc = get_tmap_4d_bf16(&tq, q, 192, H, tokens, 1, 192, ldq, ldq * tokens, 64, 1, ffwd::kRows, 1, 1);
   const uint64_t ld = static_cast<uint64_t>(H) * 128;
