@@ -11,19 +11,24 @@
 // Recomputing S and dP for the second kind costs 7 products instead of 5, but needs no fp32 accumulator of dQ in memory and
 // makes the gradient bit-reproducible.  The 1/sqrt(d) factor of dS is applied once in the dK / dQ epilogues.
 //
-// What bounds it: the tensor pipe (4 / 3 products of 128 x 128 x D per block pair, 2048 / 1536 clocks at D = 128) against
-// 1024 clocks of exponentials and the hand-overs between them.  S and dP are single buffers of 128 columns, and the order of
-// issue keeps the pipe busy instead: while the softmax warpgroups turn S(n) into P(n) the pipe runs dK(n-1) and dP(n), while
-// they turn dP(n) into dS(n) it runs dV(n) and S(n+1).  (64-row blocks with double buffers, the earlier layout, read 192 bytes
-// of operands per clock where shared memory gives 128, and started a CTA per item.)  The streamed tiles Q, dO, Q, dO, ... share
-// one ring: with 5 slots beside the two resident tiles (all that 227 KB hold at D = 128) Q(n+1) is fetched as soon as dV(n-2)
-// has retired, a block and a half ahead of its use; rings of two stages each left the pipe waiting 200-1000 clocks per block.
-// P is handed over in two halves, as in the forward.  Persistent: one CTA per SM claims items, longest of a group first, the dKV
-// items of a group of heads before its dQ items.  These read the same tiles again, from L2, and fill the SMs that the last dKV items
-// leave idle (8 x 512 x 32 x 128: 94 us in two launches, 88 us in one).  TMEM, barriers and maps are set up once, an item's first
-// tiles are fetched while the previous item is still in its softmax, and a warpgroup of its own reads the accumulators out and stores
-// them meanwhile (a row per thread: 4900 clocks from the last product to the next item's first softmax when the softmax warps did it,
-// against 2900 per block).
+// What bounds it: the softmax warps, 1600 clocks from S to P and 550 from dP to dS for a 128 x 128 block (1024 of exponentials alone), beside
+// 2048 / 1536 clocks of tensor pipe (4 / 3 products of 128 x 128 x D at D = 128): 2740 clocks per dKV block, 2400 per dQ block.  S and dP
+// are single buffers of 128 columns (with the accumulators all of TMEM), and the order of issue keeps the pipe busy instead: while the
+// softmax warpgroups turn S(n) into P(n) the pipe runs dK(n-1) and dP(n), while they turn dP(n) into dS(n) it runs dV(n) and S(n+1).
+// (64-row blocks with double buffers, an earlier layout, read 192 bytes of operands per clock where shared memory gives 128.)  P is handed
+// over in two halves, as in the forward.
+// The blocks of all items make one stream: an item's resident and streamed tiles share six slots that are handed on in the order of
+// their last use, so the next item's first tiles are there and its first scores are made while this one's last block is in its softmax.
+// (With two slots for the resident tiles alone these could only be fetched when the item before had let go of them: 4500 clocks between
+// items, as long as one and a half blocks.)  Two warps issue the products: one could not wait, work out addresses and issue 32 products in
+// the time that they take.  A warpgroup of its own reads the accumulators out, through a seventh slot and TMA stores (a row per
+// thread straight to memory slowed the softmax warps' own loads twofold meanwhile).
+// Persistent: one CTA per SM claims items, longest of a group first, the dKV items of a group of heads before its dQ items.  These
+// read the same tiles again, from L2, and fill the SMs that the last dKV items leave idle.
+// Before / after (one stream of blocks, two issuers, TMA stores): 8 x 512 x 32 x 128 105.6 / 96.3 us with the statistics pass, 2 x 2048 x 40 x 128
+// 282 / 269, 1 x 4096 x 32 x 128 397 / 377, 8 x 512 x 12 x 64 32.7 / 28.1, 1 x 2048 x 33 x 64 110 / 104.
+// Tried: dS^T kept in memory for the dQ items instead of the scores made again (5 products for 7): 399 us for 282, the dQ items wait for
+// the last dKV items of their head.
 //
 // A ragged sequence ends inside a block: rows past it are zero-filled by TMA, their statistics make P zero, and they are
 // never stored (causal only: keys past the end are then hidden from every real query by the mask).
@@ -35,6 +40,7 @@
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
 #include "../common/wait_status.h"
+#include "flash_bwd_slots.cuh"
 
 namespace llmctl {
 using namespace ptx;
@@ -42,11 +48,12 @@ using namespace ptx;
 namespace fbwd {
 constexpr int kBlk = 128;                    // rows of a resident or streamed block
 constexpr int kPanel = kBlk * 128;           // bytes of a [128 x 64 bf16] swizzled panel
-constexpr int kThreads = 448;                // TMA, MMA issuer, 2 softmax warpgroups, epilogue warpgroup
+constexpr int kThreads = 480;                // TMA, issuer A, 2 softmax warpgroups, epilogue warpgroup, issuer B
 constexpr int kStatBytes = 2 * kBlk * 4;     // -lse * log2e and -delta of 128 queries
-// Items are claimed from a counter by the TMA warp and told to the others through a queue.  It runs at most two items ahead of
-// the softmax warps (the resident tiles are single), so a slot is never overwritten before all have read it.
-constexpr int kQueue = 4;
+// Items are claimed from a counter by the TMA warp and told to the others through a queue.  When item m is published all tiles of item
+// m - 1 are on their way, so item m - 3 has handed all of its back and item m - 4 has been read out: everyone has read the slot of item m - 8.
+constexpr int kQueue = 8;
+constexpr int kRing = 16;                    // barriers for loads and for hand-backs
 // Heads are worked through in groups whose q, k, v and dO stay in L2 (126 MB, with the outputs of the group before) while every
 // block of the group streams them again; block by block over all heads, S = 2048 with 80 heads read them from HBM every time.
 constexpr long long kGroupBytes = 32ll << 20;
@@ -54,13 +61,11 @@ template <int D>
 struct Cfg {
   static constexpr int kPanels = D / 64;
   static constexpr int kTile = kPanels * kPanel;
-  static constexpr int kSlots = D == 128 ? 5 : 9;                      // streamed tiles: element 2n = operand 0 of block n, 2n + 1 = operand 1
-  // statistics of block n go with element 2n + 1, whose slot is free only when operand 0 of block n - (kSlots - 1) / 2 is: by
-  // then the softmax is done with that block
-  static constexpr int kStatSlots = (kSlots - 1) / 2;
-  static constexpr int kStatAt = (2 + kSlots) * kTile;                 // behind all tiles: each starts at a multiple of 1024 bytes
+  static constexpr int kOutAt = kTiles * kTile;                       // a tile of gradients on its way out
+  static constexpr int kStatSlots = D == 128 ? 2 : 4;
+  static constexpr int kStatAt = kOutAt + kTile;                       // behind all tiles: each starts at a multiple of 1024 bytes
   static constexpr int kBarsAt = kStatAt + kStatSlots * kStatBytes;
-  static constexpr int kSmem = kBarsAt + 384;
+  static constexpr int kSmem = kBarsAt + 640;
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
 __device__ unsigned int g_status = 0;        // != 0: a bounded wait of the kernel ran out
@@ -68,7 +73,11 @@ using DKV = std::integral_constant<bool, false>;
 using DQ = std::integral_constant<bool, true>;
 
 struct Maps {
-  CUtensorMap q, k, v, d_o;
+  CUtensorMap q, k, v, d_o, dq, dk, dv;
+};
+struct Item {
+  bool dq;
+  int rb, bh, first, n;      // resident block, batch x head, streamed blocks [first, first + n)
 };
 }  // namespace fbwd
 
@@ -117,37 +126,23 @@ flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* 
   }
 }
 
-// 16 columns of an fp32 accumulator row -> 16 bf16 at dst (32 bytes)
-__device__ __forceinline__ void fbwd_store16(__nv_bfloat16* dst, const uint32_t* r, float mul, bool wide) {
-  uint32_t w[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) w[e] = pack_bf16x2(__uint_as_float(r[2 * e]) * mul, __uint_as_float(r[2 * e + 1]) * mul);
-  if (wide) {
-    st_v8(dst, w);
-  } else {
-    st_v4(dst, make_uint4(w[0], w[1], w[2], w[3]));
-    st_v4(dst + 8, make_uint4(w[4], w[5], w[6], w[7]));
-  }
-}
-
 // dKV items: resident K, V; streamed Q, dO.  dQ items: resident Q, dO; streamed K, V.  Operand 0 of either pair (K / Q) makes the
 // S-like product, operand 1 (V / dO) the dP-like one.
 template <int D>
 __global__ void __launch_bounds__(fbwd::kThreads, 1)
 flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restrict__ nl2, const float* __restrict__ ndl,
-                 __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long long out_tok,
-                 int out_wide, int B, int S, int H, int group, int* __restrict__ counter, float scale_log2, float scale, int causal,
+                 int in_step, int out_step, int B, int S, int H, int group, int* __restrict__ counter, float scale_log2, float scale, int causal,
                  unsigned char* wait_byte) {
   using namespace fbwd;
   using C = Cfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   struct Bars {
-    uint64_t full[C::kSlots], empty[C::kSlots], res, resfree, s, dp, p[2], ds, acc[2], accfree[2], item_full[kQueue];
-    int item[kQueue];
+    uint64_t full[kRing], given[kRing], stat_full[C::kStatSlots], stat_free[C::kStatSlots], s, dp, p[2], ds, acc[2], accfree[2], item_full[kQueue];
+    int4 item[kQueue];                 // Item as the TMA warp decoded it; no blocks: the end
     uint32_t tmem;
     int abort;
   };
-  static_assert(sizeof(Bars) <= 384, "barriers");
+  static_assert(sizeof(Bars) <= 640, "barriers");
   Bars& bar = *reinterpret_cast<Bars*>(smem + C::kBarsAt);
   const uint32_t smem_base = smem_u32(smem);
   if (smem_base & 1023u) {             // the swizzled tiles would not line up (uniform over the grid)
@@ -162,11 +157,13 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   const int BH = B * H, n_items = 2 * nblk * BH;
 
   if (threadIdx.x == 0) {
-    mbar_init(&bar.res, 1);
-    mbar_init(&bar.resfree, 1);
-    for (int i = 0; i < C::kSlots; ++i) {
+    for (int i = 0; i < kRing; ++i) {
       mbar_init(&bar.full[i], 1);
-      mbar_init(&bar.empty[i], 1);
+      mbar_init(&bar.given[i], 2);     // e1 is read by both issuers
+    }
+    for (int i = 0; i < C::kStatSlots; ++i) {
+      mbar_init(&bar.stat_full[i], 1);
+      mbar_init(&bar.stat_free[i], 1);
     }
     mbar_init(&bar.s, 1);
     mbar_init(&bar.dp, 1);
@@ -185,6 +182,9 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     prefetch_tmap(&maps.k);
     prefetch_tmap(&maps.v);
     prefetch_tmap(&maps.d_o);
+    prefetch_tmap(&maps.dq);
+    prefetch_tmap(&maps.dk);
+    prefetch_tmap(&maps.dv);
   }
   if (warp == 1) tmem_alloc<1>(&bar.tmem, 512);
   tc_fence_before();
@@ -193,198 +193,211 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   const uint32_t tmem_base = bar.tmem;
   // A waiter of an mbarrier sees only the parity of its phase, so no barrier may complete its next phase before everyone has passed the
   // wait for this one.  acc[a] (product finished) is therefore committed only after accfree[a] (read out) of the use before has been
-  // waited for.  acc[0] is used by every item, acc[1] by dKV items alone, each side counting them.
+  // waited for.  acc[0] is used by dKV items alone, acc[1] by every item, each side counting them.
   // TMEM: S [0,128)  dP [128,256)  acc0 [256,256+D)  acc1 [384,384+D)
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tAcc0 = tmem_base + 256, tAcc1 = tmem_base + 384;
   volatile int* abort = &bar.abort;
 
-  // item -> (kind, resident block, batch x head) and the streamed blocks [first, first + n); longest items of a group first
-  auto decode = [&](int item, bool& is_dq, int& rb, int& bh, int& first, int& n) {
+  // longest items of a group first
+  auto decode = [&](int item) {
+    Item it{};
+    if (item >= n_items) return it;
     const int base = item / (2 * group * nblk) * group, heads = min(group, BH - base);
     int rem = item - 2 * base * nblk;
-    is_dq = rem >= heads * nblk;
-    if (is_dq) rem -= heads * nblk;
+    it.dq = rem >= heads * nblk;
+    if (it.dq) rem -= heads * nblk;
     const int k = rem / heads;
-    bh = base + rem % heads;
-    rb = is_dq ? nblk - 1 - k : k;
-    first = (!is_dq && causal) ? rb : 0;
-    n = (causal ? (is_dq ? rb + 1 : nblk) : nblk) - first;
+    it.bh = base + rem - k * heads;
+    it.rb = it.dq ? nblk - 1 - k : k;
+    it.first = (!it.dq && causal) ? it.rb : 0;
+    it.n = (causal ? (it.dq ? it.rb + 1 : nblk) : nblk) - it.first;
+    return it;
   };
-  // the k-th item of this CTA, as the TMA warp published it; false when a wait ran out or there is none left
-  auto next_item = [&](uint32_t k, int& item) {
+  // the k-th item of this CTA, as the TMA warp published it (decoding takes ~700 clocks of divisions); false when a wait ran out or
+  // there is none left
+  auto next_item = [&](uint32_t k, Item& it) {
     mbar_wait_or_abort(&bar.item_full[k % kQueue], (k / kQueue) & 1u, abort);
+    const int4 w = bar.item[k % kQueue];
     __syncwarp();
-    item = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&bar.item[k % kQueue]), 0);
-    return item < n_items && !*abort;
+    it.dq = __shfl_sync(0xffffffffu, w.x & 1, 0) != 0;
+    it.rb = __shfl_sync(0xffffffffu, w.x >> 1, 0);
+    it.bh = __shfl_sync(0xffffffffu, w.y, 0);
+    it.first = __shfl_sync(0xffffffffu, w.z, 0);
+    it.n = __shfl_sync(0xffffffffu, *abort ? 0 : w.w, 0);
+    return it.n > 0;
   };
 
   if (warp == 0) {
     // ------------------------------------ TMA producer ------------------------------------
     if (lane == 0) {
-      uint32_t e = 0, k = 0;           // streamed tiles / items so far
-      uint32_t nr = 0;                 // resident pairs begun
+      uint32_t l = 0, k = 0, gs = 0;   // loads, items and blocks with statistics so far
       bool ok = true;
-      // the next streamed tile: false when its slot does not become free
-      auto stream = [&](const CUtensorMap* m, int h, int row, int b, const float* st0, const float* st1) {
-        const uint32_t slot = e % C::kSlots;
-        if (!mbar_wait_bounded(&bar.empty[slot], ((e / C::kSlots) & 1u) ^ 1u, abort)) return false;
-        mbar_expect_tx(&bar.full[slot], C::kTile + (st0 != nullptr ? kStatBytes : 0));
-        uint8_t* dst = smem + (2 + slot) * C::kTile;
+      Slots sl;
+      // the next tile: false when its slot is not handed back
+      auto load = [&](uint32_t slot, const CUtensorMap* m, int h, int row, int b) {
+        const uint32_t j = l - kTiles;
+        if (l >= kTiles && !mbar_wait_bounded(&bar.given[j % kRing], (j / kRing) & 1u, abort)) return false;
+        uint64_t* full = &bar.full[l % kRing];
+        mbar_expect_tx(full, C::kTile);
+        uint8_t* dst = smem + slot * C::kTile;
 #pragma unroll
-        for (int p = 0; p < C::kPanels; ++p) tma_load_4d(dst + p * kPanel, m, &bar.full[slot], 64 * p, h, row, b);
-        if (st0 != nullptr) {
-          uint8_t* sStat = smem + C::kStatAt + ((e >> 1) % C::kStatSlots) * kStatBytes;
-          bulk_load_1d(sStat, st0, kBlk * 4, &bar.full[slot]);
-          bulk_load_1d(sStat + kBlk * 4, st1, kBlk * 4, &bar.full[slot]);
-        }
-        ++e;
+        for (int p = 0; p < C::kPanels; ++p) tma_load_4d(dst + p * kPanel, m, full, 64 * p, h, row, b);
+        ++l;
         return true;
       };
-      int item = blockIdx.x;
-      for (;; ++k) {
-        bar.item[k % kQueue] = item;
+      auto load_stats = [&](long long at) {
+        const uint32_t slot = gs % C::kStatSlots;
+        if (!mbar_wait_bounded(&bar.stat_free[slot], ((gs / C::kStatSlots) & 1u) ^ 1u, abort)) return false;
+        mbar_expect_tx(&bar.stat_full[slot], kStatBytes);
+        uint8_t* dst = smem + C::kStatAt + slot * kStatBytes;
+        bulk_load_1d(dst, nl2 + at, kBlk * 4, &bar.stat_full[slot]);
+        bulk_load_1d(dst + kBlk * 4, ndl + at, kBlk * 4, &bar.stat_full[slot]);
+        ++gs;
+        return true;
+      };
+      for (int item = blockIdx.x, next = 0;; ++k, item = next) {
+        const Item it = decode(item);
+        bar.item[k % kQueue] = make_int4(it.rb * 2 + (it.dq ? 1 : 0), it.bh, it.first, it.n);
         mbar_arrive(&bar.item_full[k % kQueue]);
-        if (item >= n_items) break;
-        const int next = gridDim.x + atomicAdd(counter, 1);
-        bool is_dq;
-        int rb, bh, first, n;
-        decode(item, is_dq, rb, bh, first, n);
-        const int h = bh % H, b = bh / H;
-        const CUtensorMap *res0 = is_dq ? &maps.q : &maps.k, *res1 = is_dq ? &maps.d_o : &maps.v;
-        const CUtensorMap *sub0 = is_dq ? &maps.k : &maps.q, *sub1 = is_dq ? &maps.v : &maps.d_o;
-        for (int i = 0; i < n; ++i) {
-          const int row = (first + i) * kBlk;
-          if (!(ok = stream(sub0, h, row, b, nullptr, nullptr))) break;
-          if (i == 0) {                // the resident tiles: free once the previous item's last S and dP have retired
-            if (!(ok = mbar_wait_bounded(&bar.resfree, (k & 1u) ^ 1u, abort))) break;
-            mbar_expect_tx(&bar.res, 2 * C::kTile);
-            ++nr;
-#pragma unroll
-            for (int p = 0; p < C::kPanels; ++p) {
-              tma_load_4d(smem + p * kPanel, res0, &bar.res, 64 * p, h, rb * kBlk, b);
-              tma_load_4d(smem + C::kTile + p * kPanel, res1, &bar.res, 64 * p, h, rb * kBlk, b);
-            }
-          }
-          const long long at = static_cast<long long>(bh) * Sp + row;
-          if (!(ok = stream(sub1, h, row, b, is_dq ? nullptr : nl2 + at, ndl + at))) break;
+        if (it.n == 0) break;
+        const int h = it.bh % H, b = it.bh / H;
+        const CUtensorMap *res0 = it.dq ? &maps.q : &maps.k, *res1 = it.dq ? &maps.d_o : &maps.v;
+        const CUtensorMap *sub0 = it.dq ? &maps.k : &maps.q, *sub1 = it.dq ? &maps.v : &maps.d_o;
+        const int hr0 = it.dq ? h : h + in_step, hr1 = it.dq ? h : h + 2 * in_step, hs0 = it.dq ? h + in_step : h, hs1 = it.dq ? h + 2 * in_step : h;
+        const long long stat = static_cast<long long>(it.bh) * Sp;
+        for (int i = 0; ok && i < it.n; ++i) {
+          const int row = (it.first + i) * kBlk;
+          // claimed as late as its latency can be hidden: what a CTA holds nobody else can begin
+          if (i == max(0, it.n - 2)) next = gridDim.x + atomicAdd(counter, 1);
+          ok = (i > 0 || load(sl.res(0), res0, hr0, it.rb * kBlk, b)) && load(sl.streamed(0, i), sub0, hs0, row, b) &&
+               (i > 0 || load(sl.res(1), res1, hr1, it.rb * kBlk, b)) && load(sl.streamed(1, i), sub1, hs1, row, b) && (it.dq ? i > 0 || load_stats(stat + it.rb * kBlk) : load_stats(stat + row));
         }
         if (!ok) break;
-        item = next;
+        sl.next(it.n);
       }
       // Copies still in flight when a wait ran out land before the CTA's shared memory is given back.
       if (!ok) {
         int none = 0;
-        for (uint32_t j = e > C::kSlots ? e - C::kSlots : 0; j < e; ++j, none = 0)
-          mbar_wait_bounded(&bar.full[j % C::kSlots], (j / C::kSlots) & 1u, &none);
-        if (nr > 0) mbar_wait_bounded(&bar.res, (nr - 1) & 1u, &none);
+        for (uint32_t j = l > kTiles ? l - kTiles : 0; j < l; ++j, none = 0) mbar_wait_bounded(&bar.full[j % kRing], (j / kRing) & 1u, &none);
+        for (uint32_t j = gs > C::kStatSlots ? gs - C::kStatSlots : 0; j < gs; ++j, none = 0)
+          mbar_wait_bounded(&bar.stat_full[j % C::kStatSlots], (j / C::kStatSlots) & 1u, &none);
       }
     }
-  } else if (warp == 1) {
-    // ------------------------------------ MMA issuer ------------------------------------
-    // The whole warp walks the loop and waits; only the products and commits are issued by one elected lane.  Addresses and
-    // descriptors then stay in uniform registers, which the instruction reads; computed in a single lane's branch they are
-    // moved there one by one, and a product of 64 clocks took 85-107 to issue.
+  } else if (warp == 1 || warp == 14) {
+    // ------------------------------------ MMA issuers ------------------------------------
+    // Two warps: A issues S and dV, B dP and dK / dQ.  They share no accumulator and no order: a product waits in its warp for the one
+    // whose operand it writes over.  The tensor pipe takes few products ahead, so what one warp spends on waits, addresses and descriptors
+    // between its products (300-500 clocks) left the pipe idle; now the other warp's products run meanwhile.
+    // A whole warp walks the loop and waits; only the products and commits are issued by one elected lane.
+    const bool is_a = warp == 1;
     constexpr uint32_t id_s = make_idesc_bf16(kBlk, kBlk, 0u, 0u);     // A, B K-major
     constexpr uint32_t id_acc = make_idesc_bf16(kBlk, D, 0u, 1u);      // A from TMEM, B MN-major
-    const uint64_t kRes0 = make_smem_desc(smem_base, 16, 1024, 2), kRes1 = make_smem_desc(smem_base + C::kTile, 16, 1024, 2);
-    auto tile_at = [&](uint32_t e) { return smem_base + (2 + e % C::kSlots) * C::kTile; };
+    const uint32_t tScore = is_a ? tS : tdP, tAcc = is_a ? tAcc0 : tAcc1;
+    const int mine = is_a ? 0 : 1;     // the operand of this warp's scores; its gradients read the other
+    auto tile_at = [&](uint32_t slot) { return smem_base + slot * C::kTile; };
     auto wait = [&](uint64_t* b, uint32_t parity) {
       mbar_wait_or_abort(b, parity, abort);
       __syncwarp();
     };
-    auto arrived = [&](uint32_t e) { wait(&bar.full[e % C::kSlots], (e / C::kSlots) & 1u); };
+    auto arrived = [&](uint32_t l) { wait(&bar.full[l % kRing], (l / kRing) & 1u); };
+    auto given = [&](uint32_t j) { return &bar.given[j % kRing]; };
     // scores: 16 of the D columns per instruction, a panel of 64 columns every fourth
-    auto issue_scores = [&](uint32_t t, uint64_t res, uint32_t sub) {
-      const uint64_t b0 = make_smem_desc(sub, 16, 1024, 2);
+    auto issue_scores = [&](uint32_t res_at, uint32_t sub) {
+      const uint64_t a0 = make_smem_desc(res_at, 16, 1024, 2), b0 = make_smem_desc(sub, 16, 1024, 2);
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
         const uint64_t off = ((ks >> 2) * kPanel + (ks & 3) * 32) >> 4;
-        umma_ss<1>(t, res + off, b0 + off, id_s, ks != 0 ? 1u : 0u);
+        umma_ss<1>(tScore, a0 + off, b0 + off, id_s, ks != 0 ? 1u : 0u);
       }
     };
     // accumulators: 16 of the 128 streamed rows per instruction; the second half of A lies 64 columns on (a softmax
     // warpgroup writes its half over the columns that it has read itself).  part 0 / 1: the rows that both warpgroups write
     // first / last, 2: all.
-    auto issue_acc = [&](uint32_t t, uint32_t a, uint32_t sub, uint32_t fresh, int part) {
+    auto issue_acc = [&](uint32_t sub, uint32_t fresh, int part) {
       const uint64_t b0 = make_smem_desc(sub, kPanel, 1024, 2);
 #pragma unroll
       for (int ks = 0; ks < kBlk / 16; ++ks)
         if (part == 2 || ((ks >> 1) & 1) == part)
-          umma_ts<1>(t, a + (ks >> 2) * 64 + (ks & 3) * 8, b0 + ((ks * 2048) >> 4), id_acc, ks == 0 ? 1u - fresh : 1u);
+          umma_ts<1>(tAcc, tScore + (ks >> 2) * 64 + (ks & 3) * 8, b0 + ((ks * 2048) >> 4), id_acc, ks == 0 ? 1u - fresh : 1u);
     };
-    uint32_t g = 0, k = 0, kv = 0;     // blocks, items and dKV items so far
-    auto run = [&](auto kind, int n) {
-      constexpr bool kDQ = decltype(kind)::value;
-      for (int i = 0; i < n; ++i, ++g) {
-        const uint32_t e0 = 2 * g, e1 = e0 + 1;            // this block's streamed tiles; the next block's are e0 + 2, e1 + 2
-        const uint32_t fresh = i == 0 ? 1u : 0u;
-        if (i == 0) {
-          arrived(e0);
-          tc_fence_after();
-          if (elect_one()) {
-            issue_scores(tS, kRes0, tile_at(e0));
-            umma_commit<1>(&bar.s);
-          }
-          arrived(e1);
-          tc_fence_after();
-          if (elect_one()) {
-            issue_scores(tdP, kRes1, tile_at(e1));
-            umma_commit<1>(&bar.dp);
-            if (n == 1) umma_commit<1>(&bar.resfree);
-            if (kDQ) umma_commit<1>(&bar.empty[e1 % C::kSlots]);
-          }
-        }
-        if (!kDQ) {
+    // The block whose scores are issued next runs ahead of the one whose gradients are, across the ends of items.
+    Item it{};                         // its item, block in it, slots
+    int i = 0;
+    Slots sl;
+    uint32_t k = 0;
+    auto advance = [&]() {
+      if (++i < it.n) return true;
+      if (it.n > 0) sl.next(it.n);
+      i = 0;
+      return next_item(k++, it);
+    };
+    uint32_t at_res = 0, at_sub = 0;
+    auto scores_ready = [&]() {
+      if (i == 0) arrived(sl.load_res(mine));
+      arrived(sl.load_streamed(mine, i));
+      at_res = tile_at(sl.res(mine));
+      at_sub = tile_at(sl.streamed(mine, i));
+    };
+    auto scores = [&]() {              // one lane
+      issue_scores(at_res, at_sub);
+      umma_commit<1>(is_a ? &bar.s : &bar.dp);
+      if (!is_a) {
+        uint64_t* b = given(sl.given_streamed(1, i, it.n));
+        if (it.dq) mbar_arrive(b);     // A has no use for it
+        umma_commit<1>(b);
+      }
+      if (i + 1 == it.n) {
+        uint64_t* b = given(sl.given_res(mine, it.n));
+        mbar_arrive(b);
+        umma_commit<1>(b);
+      }
+    };
+    bool more = advance();
+    if (more) {
+      scores_ready();
+      tc_fence_after();
+      if (elect_one()) scores();
+    }
+    uint32_t uses = 0;                 // of this warp's accumulator
+    for (uint32_t g = 0, gs = 0; more; ++g) {
+      const bool kdq = it.dq, last = i + 1 == it.n;
+      const uint32_t fresh = i == 0 ? 1u : 0u, l1 = sl.load_streamed(1, i), at = tile_at(sl.streamed(1 - mine, i));
+      uint64_t* const back = given(sl.given_streamed(1 - mine, i, it.n));
+      more = advance();
+      if (more) scores_ready();
+      if (is_a) {
+        if (!kdq) {
+          arrived(l1);
+          if (fresh) wait(&bar.accfree[0], (uses & 1u) ^ 1u);
           wait(&bar.p[0], g & 1u);      // half of P(g) is written
-          if (i == 0 && k > 0) wait(&bar.accfree[0], (k - 1) & 1u);
           tc_fence_after();
-          if (elect_one()) issue_acc(tAcc0, tS, tile_at(e1), fresh, 0);              // dV += P^T dO
+          if (elect_one()) issue_acc(at, fresh, 0);                    // dV += P^T dO
         }
         wait(&bar.p[1], g & 1u);        // P(g) written (dKV) / S(g) read (dQ)
         tc_fence_after();
-        if (!kDQ && elect_one()) {
-          issue_acc(tAcc0, tS, tile_at(e1), 0, 1);
-          umma_commit<1>(&bar.empty[e1 % C::kSlots]);
-          if (i + 1 == n) umma_commit<1>(&bar.acc[0]);
-        }
-        if (i + 1 < n) {
-          arrived(e0 + 2);
-          tc_fence_after();
-          if (elect_one()) {
-            issue_scores(tS, kRes0, tile_at(e0 + 2));
-            umma_commit<1>(&bar.s);
+        if (elect_one()) {
+          if (!kdq) {
+            issue_acc(at, 0, 1);
+            umma_commit<1>(back);
+            if (last) umma_commit<1>(&bar.acc[0]);
           }
+          if (more) scores();
         }
+        if (!kdq && last) ++uses;
+      } else {
+        if (fresh) wait(&bar.accfree[1], (uses & 1u) ^ 1u);
         wait(&bar.ds, g & 1u);
-        if (i == 0 && (kDQ ? k : kv) > 0) wait(&bar.accfree[kDQ ? 0 : 1], ((kDQ ? k : kv) - 1) & 1u);
         tc_fence_after();
         if (elect_one()) {
-          issue_acc(kDQ ? tAcc0 : tAcc1, tdP, tile_at(e0), fresh, 2);    // dK += dS^T Q  /  dQ += dS K
-          umma_commit<1>(&bar.empty[e0 % C::kSlots]);
-          if (i + 1 == n) umma_commit<1>(&bar.acc[kDQ ? 0 : 1]);
+          issue_acc(at, fresh, 2);                                     // dK += dS^T Q  /  dQ += dS K
+          mbar_arrive(back);
+          umma_commit<1>(back);
+          if (last) umma_commit<1>(&bar.acc[1]);
+          if (more) scores();
+          if (!kdq || last) mbar_arrive(&bar.stat_free[gs % C::kStatSlots]);     // dS(g) is written: its statistics have been read
         }
-        if (i + 1 < n) {
-          arrived(e1 + 2);
-          tc_fence_after();
-          if (elect_one()) {
-            issue_scores(tdP, kRes1, tile_at(e1 + 2));
-            umma_commit<1>(&bar.dp);
-            if (i + 2 == n) umma_commit<1>(&bar.resfree);
-            if (kDQ) umma_commit<1>(&bar.empty[(e1 + 2) % C::kSlots]);
-          }
-        }
-      }
-    };
-    for (int item; next_item(k, item); ++k) {
-      bool is_dq;
-      int rb, bh, first, n;
-      decode(item, is_dq, rb, bh, first, n);
-      wait(&bar.res, k & 1u);
-      if (is_dq) {
-        run(DQ{}, n);
-      } else {
-        run(DKV{}, n);
-        ++kv;
+        if (!kdq || last) ++gs;
+        if (last) ++uses;
       }
     }
   } else if (warp < 10) {
@@ -394,21 +407,26 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
     const int row = q4 * 32 + lane;                       // resident row == TMEM lane
     const uint32_t lane_off = static_cast<uint32_t>(q4 * 32) << 16;
     const uint32_t tSb = tS + wg * 64 + lane_off, tPb = tdP + wg * 64 + lane_off;
-    uint32_t g = 0, k = 0;
-    auto run = [&](auto kind, int rb, int bh, int first, int n) {
+    uint32_t g = 0, gs = 0, k = 0;     // blocks, blocks with statistics and items so far
+    auto run = [&](auto kind, int rb, int first, int n) {
       constexpr bool kDQ = decltype(kind)::value;
       float row_nl = 0.f, row_nd = 0.f;                   // dQ items: this query row's statistics
       if (kDQ) {
-        row_nl = nl2[static_cast<long long>(bh) * Sp + rb * kBlk + row];
-        row_nd = ndl[static_cast<long long>(bh) * Sp + rb * kBlk + row];
+        const float* stat = reinterpret_cast<const float*>(smem + C::kStatAt + (gs % C::kStatSlots) * kStatBytes);
+        mbar_wait_or_abort(&bar.stat_full[gs % C::kStatSlots], (gs / C::kStatSlots) & 1u, abort);
+        ++gs;
+        row_nl = stat[row];
+        row_nd = stat[kBlk + row];
       }
       for (int i = 0; i < n; ++i, ++g) {
-        const float* stat = reinterpret_cast<const float*>(smem + C::kStatAt + (g % C::kStatSlots) * kStatBytes) + wg * 64;
-        const uint32_t e1 = 2 * g + 1;                    // the statistics came with this streamed tile
+        const float* stat = reinterpret_cast<const float*>(smem + C::kStatAt + (gs % C::kStatSlots) * kStatBytes) + wg * 64;
         const bool diag = causal && first + i == rb;
         // columns a row may see on the diagonal block: dKV key `row` <= query, dQ key <= query `row`
         const int edge = row - wg * 64;
-        if (!kDQ) mbar_wait_or_abort(&bar.full[e1 % C::kSlots], (e1 / C::kSlots) & 1u, abort);
+        if (!kDQ) {
+          mbar_wait_or_abort(&bar.stat_full[gs % C::kStatSlots], (gs / C::kStatSlots) & 1u, abort);
+          ++gs;
+        }
         mbar_wait_or_abort(&bar.s, g & 1u, abort);
         __syncwarp();
         tc_fence_after();
@@ -497,32 +515,27 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         if (lane == 0) mbar_arrive(&bar.ds);
       }
     };
-    for (int item; next_item(k, item); ++k) {
-      bool is_dq;
-      int rb, bh, first, n;
-      decode(item, is_dq, rb, bh, first, n);
-      if (is_dq) run(DQ{}, rb, bh, first, n); else run(DKV{}, rb, bh, first, n);
+    for (Item it; next_item(k, it); ++k) {
+      if (it.dq) run(DQ{}, it.rb, it.first, it.n); else run(DKV{}, it.rb, it.first, it.n);
     }
-  } else {
-    // ------------- epilogue warpgroup: accumulators -> registers -> bf16 -> global, a row per thread -------------
+  } else if (warp < 14) {
+    // ------------- epilogue warpgroup: accumulators -> registers -> bf16 in shared memory -> TMA, a row per thread -------------
     const int q4 = warp & 3;
     const int row = q4 * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(q4 * 32) << 16;
+    uint8_t* out = smem + C::kOutAt;
+    const bool issuer = warp == 10 && lane == 0;
     uint32_t k = 0, kv = 0;            // items and dKV items so far
-    for (int item; next_item(k, item); ++k) {
-      bool is_dq;
-      int rb, bh, first, n;
-      decode(item, is_dq, rb, bh, first, n);
-      const bool real = rb * kBlk + row < S;
-      const long long at = (static_cast<long long>(bh / H) * S + rb * kBlk + row) * out_tok + (bh % H) * D;
+    for (Item it; next_item(k, it); ++k) {
 #pragma unroll 1
-      for (int a = 0; a < (is_dq ? 1 : 2); ++a) {         // dKV: dV from acc0, then scale * dK from acc1.  dQ: scale * dQ from acc0.
-        mbar_wait_or_abort(&bar.acc[a], (a == 0 ? k : kv) & 1u, abort);
+      for (int a = it.dq ? 1 : 0; a < 2; ++a) {           // dKV: dV from acc0, then scale * dK from acc1.  dQ: scale * dQ from acc1.
+        mbar_wait_or_abort(&bar.acc[a], (a == 0 ? kv : k) & 1u, abort);
         __syncwarp();
         tc_fence_after();
         const uint32_t tA = (a == 0 ? tAcc0 : tAcc1) + lane_off;
-        const float mul = (is_dq || a == 1) ? scale : 1.f;
-        __nv_bfloat16* dst = (is_dq ? dq : a == 0 ? dv : dk) + at;
+        const float mul = a == 1 ? scale : 1.f;
+        if (issuer) tma_store_wait_read<0>();             // the tile before is on its way
+        named_bar_sync(1, 128);
 #pragma unroll
         for (int c0 = 0; c0 < D; c0 += 64) {
           uint32_t r[64];
@@ -534,14 +547,29 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar.accfree[a]);
           }
-          if (real) {
 #pragma unroll
-            for (int c = 0; c < 64; c += 16) fbwd_store16(dst + c0 + c, r + c, mul, out_wide);
+          for (int c = 0; c < 8; ++c) {
+            uint4 w;
+            w.x = pack_bf16x2(__uint_as_float(r[8 * c]) * mul, __uint_as_float(r[8 * c + 1]) * mul);
+            w.y = pack_bf16x2(__uint_as_float(r[8 * c + 2]) * mul, __uint_as_float(r[8 * c + 3]) * mul);
+            w.z = pack_bf16x2(__uint_as_float(r[8 * c + 4]) * mul, __uint_as_float(r[8 * c + 5]) * mul);
+            w.w = pack_bf16x2(__uint_as_float(r[8 * c + 6]) * mul, __uint_as_float(r[8 * c + 7]) * mul);
+            *reinterpret_cast<uint4*>(out + c0 / 64 * kPanel + row * 128 + ((c ^ (row & 7)) * 16)) = w;
           }
         }
+        fence_proxy_async_smem();
+        named_bar_sync(1, 128);
+        if (issuer) {
+          const CUtensorMap* m = it.dq ? &maps.dq : a == 0 ? &maps.dv : &maps.dk;
+#pragma unroll
+          for (int p = 0; p < C::kPanels; ++p)
+            tma_store_4d(m, out + p * kPanel, 64 * p, it.bh % H + (it.dq ? 0 : a == 0 ? 2 * out_step : out_step), it.rb * kBlk, it.bh / H);
+          tma_store_commit();
+        }
       }
-      if (!is_dq) ++kv;
+      if (!it.dq) ++kv;
     }
+    if (issuer) tma_store_wait_read<0>();
   }
 
   tc_fence_before();
@@ -571,24 +599,34 @@ static int flash_bwd_launch(const void* q, const void* k, const void* v, const v
   const int chunks = (Sp + kPrepRows - 1) / kPrepRows;
   flash_bwd_prep_kernel<D><<<chunks * B * H, 256, 0, s>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, o_tok, lse, nl2, ndl, S, Sp,
                                                           H, chunks, counter);
-  CUtensorMap mq, mk, mv, mdo;
   int rc = 0;
-  auto mkmap = [&](CUtensorMap* m, const void* base, long long tok) {
-    if (!rc) rc = get_tmap_4d_bf16(m, base, D, H, S, B, D, tok, static_cast<uint64_t>(S) * tok, 64, 1, kBlk, 1, 1);
+  auto mkmap = [&](CUtensorMap* m, const void* base, long long tok, int heads) {
+    if (!rc) rc = get_tmap_4d_bf16(m, base, D, heads, S, B, D, tok, static_cast<uint64_t>(S) * tok, 64, 1, kBlk, 1, 1);
   };
-  mkmap(&mq, q, q_tok);
-  mkmap(&mk, k, k_tok);
-  mkmap(&mv, v, v_tok);
-  mkmap(&mdo, d_o, o_tok);
+  // q | k | v side by side in a token, as one projection leaves them, are one tensor of 3 H heads: one map instead of three (about 1 us of
+  // host time each where the address is a new one)
+  auto three = [&](CUtensorMap* m, const void* a, const void* b, const void* c, long long ta, long long tb, long long tc) {
+    const long long step = 2ll * H * D;
+    const bool packed = static_cast<const char*>(b) - static_cast<const char*>(a) == step && static_cast<const char*>(c) - static_cast<const char*>(b) == step && ta == tb && ta == tc;
+    mkmap(m, a, ta, packed ? 3 * H : H);
+    if (packed) {
+      m[1] = m[2] = m[0];
+    } else {
+      mkmap(m + 1, b, tb, H);
+      mkmap(m + 2, c, tc, H);
+    }
+    return packed ? H : 0;
+  };
+  Maps maps;
+  const int in_step = three(&maps.q, q, k, v, q_tok, k_tok, v_tok), out_step = three(&maps.dq, dq, dk, dv, dqkv_tok, dqkv_tok, dqkv_tok);
+  mkmap(&maps.d_o, d_o, o_tok, H);
   if (rc) return rc;
   unsigned char* const wait_byte = wait_report(kWaitFlashBackward);
   if (wait_byte == nullptr) return static_cast<int>(cudaErrorMemoryAllocation);
   const cudaError_t e = allow_smem(flash_bwd_kernel<D>, C::kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int n_items = 2 * nblk * B * H, grid = n_items < kNumSMs ? n_items : kNumSMs;
-  const int wide = dqkv_tok % 16 == 0 && ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 31) == 0;
-  flash_bwd_kernel<D><<<grid, kThreads, C::kSmem, s>>>(Maps{mq, mk, mv, mdo}, nl2, ndl, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv,
-                                                       dqkv_tok, wide, B, S, H, group, counter, scale * 1.4426950408889634f, scale, causal, wait_byte);
+  flash_bwd_kernel<D><<<grid, kThreads, C::kSmem, s>>>(maps, nl2, ndl, in_step, out_step, B, S, H, group, counter, scale * 1.4426950408889634f, scale, causal, wait_byte);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -162,8 +162,8 @@ template <int DQK, int DV>
 __global__ void __launch_bounds__(ffwd::kThreads, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmKs, const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ O,
-                 long long o_tok_stride, int o_wide, float* __restrict__ lse, const ffwd::Seq* __restrict__ seqs, int B, int max_q, int H, float scale_log2, int causal,
-                 unsigned char* wait_byte, long long* __restrict__ trace) {
+                 long long o_tok_stride, int o_wide, float* __restrict__ lse, const ffwd::Seq* __restrict__ seqs, int B, int max_q, int H,
+                 int head_step, float scale_log2, int causal, unsigned char* wait_byte, long long* __restrict__ trace) {
   using namespace ffwd;
   using C = Cfg<DQK, DV>;
   constexpr int kOwn = DQK > 128 ? 2 : DQK / 64;         // panels of K that belong to the head; the last of three is shared by all
@@ -292,7 +292,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           mbar_expect_tx(&bar_kfull[ks], C::kQTile);
           ++nk;
 #pragma unroll
-          for (int p = 0; p < kOwn; ++p) tma_load_4d(sK + p * kPanel, &tmK, &bar_kfull[ks], 64 * p, head, row, bc);
+          for (int p = 0; p < kOwn; ++p) tma_load_4d(sK + p * kPanel, &tmK, &bar_kfull[ks], 64 * p, head + head_step, row, bc);
           if (kOwn < DQK / 64) tma_load_4d(sK + kOwn * kPanel, &tmKs, &bar_kfull[ks], 0, 0, row, bc);
           if (j == 0 && validB) {
             if (!(ok = load_q(1, nB))) break;
@@ -302,7 +302,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           mbar_expect_tx(&bar_vfull[vs], C::kVTile);
           ++nv;
 #pragma unroll
-          for (int p = 0; p < DV / 64; ++p) tma_load_4d(sV + p * kPanel, &tmV, &bar_vfull[vs], 64 * p, head, row, bc);
+          for (int p = 0; p < DV / 64; ++p) tma_load_4d(sV + p * kPanel, &tmV, &bar_vfull[vs], 64 * p, head + 2 * head_step, row, bc);
         }
       }
       // Copies still in flight when a wait ran out land before the CTA's shared memory is given back.
@@ -503,7 +503,8 @@ static long long* flash_trace_buffer() {
 // Persistent launch: one CTA per SM over a heavy-first item list.
 template <int DQK, int DV>
 static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& ks, const CUtensorMap& v, void* o,
-                            long long o_tok_stride, float* lse, const ffwd::Seq* seqs, int B, int max_q, int H, float scale, int causal, cudaStream_t s) {
+                            long long o_tok_stride, float* lse, const ffwd::Seq* seqs, int B, int max_q, int H, int head_step, float scale, int causal,
+                            cudaStream_t s) {
   using namespace ffwd;
   using C = Cfg<DQK, DV>;
   const cudaError_t e = allow_smem(flash_fwd_kernel<DQK, DV>, C::kSmem);
@@ -515,7 +516,7 @@ static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CU
   if (wait_byte == nullptr) return static_cast<int>(cudaErrorMemoryAllocation);
   const int wide = o_tok_stride % 16 == 0 && (reinterpret_cast<uintptr_t>(o) & 31) == 0;
   flash_fwd_kernel<DQK, DV><<<grid, kThreads, C::kSmem, s>>>(q, k, ks, v, (__nv_bfloat16*)o, o_tok_stride, wide, lse, seqs, B, max_q, H,
-                                                             scale * 1.4426950408889634f, causal, wait_byte, flash_trace_buffer());
+                                                             head_step, scale * 1.4426950408889634f, causal, wait_byte, flash_trace_buffer());
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -554,15 +555,23 @@ LLMCTL_API int llmctl_flash_attn_fwd(const void* q, const void* k, const void* v
   LLMCTL_REQUIRE(scale > 0.f && (reinterpret_cast<uintptr_t>(o) & 15) == 0);      // q, k, v: the tensor maps check them
   CUtensorMap tq, tk, tv;
   int rc = 0;
-  auto mkmap = [&](CUtensorMap* m, const void* base, long long tok) {
-    if (!rc) rc = get_tmap_4d_bf16(m, base, D, H, S, B, D, tok, static_cast<uint64_t>(S) * tok, 64, 1, ffwd::kRows, 1, 1);
+  auto mkmap = [&](CUtensorMap* m, const void* base, long long tok, int heads) {
+    if (!rc) rc = get_tmap_4d_bf16(m, base, D, heads, S, B, D, tok, static_cast<uint64_t>(S) * tok, 64, 1, ffwd::kRows, 1, 1);
   };
-  mkmap(&tq, q, q_tok_stride);
-  mkmap(&tk, k, k_tok_stride);
-  mkmap(&tv, v, v_tok_stride);
+  // q | k | v side by side in a token, as one projection leaves them, are one tensor of 3 H heads: one map instead of three
+  const long long step = 2ll * H * D;
+  const bool packed = static_cast<const char*>(k) - static_cast<const char*>(q) == step && static_cast<const char*>(v) - static_cast<const char*>(k) == step &&
+                      q_tok_stride == k_tok_stride && q_tok_stride == v_tok_stride;
+  mkmap(&tq, q, q_tok_stride, packed ? 3 * H : H);
+  if (packed) {
+    tk = tv = tq;
+  } else {
+    mkmap(&tk, k, k_tok_stride, H);
+    mkmap(&tv, v, v_tok_stride, H);
+  }
   if (rc) LLMCTL_FAIL(rc, "tensor map Q / K / V");
-  rc = (D == 128 ? flash_fwd_launch<128, 128> : flash_fwd_launch<64, 64>)(tq, tk, tk, tv, o, o_tok_stride, lse, nullptr, B, S, H, scale,
-                                                                          causal, (cudaStream_t)stream);
+  rc = (D == 128 ? flash_fwd_launch<128, 128> : flash_fwd_launch<64, 64>)(tq, tk, tk, tv, o, o_tok_stride, lse, nullptr, B, S, H,
+                                                                          packed ? H : 0, scale, causal, (cudaStream_t)stream);
   if (rc) LLMCTL_FAIL(rc, "flash forward");
   return 0;
 }
@@ -585,7 +594,7 @@ LLMCTL_API int llmctl_latent_prompt_attention(const void* q, long long ldq, long
   if (!rc) rc = get_tmap_4d_bf16(&tv, v, 128, H, key_rows, 1, 128, ld, ld * key_rows, 64, 1, ffwd::kRows, 1, 1);
   if (rc) LLMCTL_FAIL(rc, "tensor map q / k / v");
   rc = flash_fwd_launch<192, 128>(tq, tk, tks, tv, out, static_cast<long long>(ld), nullptr, reinterpret_cast<const ffwd::Seq*>(seqs), B, max_q,
-                                  H, scale, 1, (cudaStream_t)stream);
+                                  H, 0, scale, 1, (cudaStream_t)stream);
   if (rc) LLMCTL_FAIL(rc, "latent prompt attention");
   return 0;
 }

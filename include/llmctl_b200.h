@@ -129,7 +129,8 @@ int llmctl_gemm_skinny_bf16(const void* X, const void* W, void* C, int Mb, int N
  * elements; lse: fp32 [B,H,S] (natural log).  Any S when causal, else a multiple of 128.  Reference: SDPA/eager inside
  * the HF model (engine.py:284); baseline cuDNN SDPA.
  * Forward: 256 queries per work item as two tiles sharing K/V, S/P/O in TMEM, P never leaves TMEM.
- * Backward: a pass for the rows' statistics, then one deterministic kernel over dK/dV items (transposed scores) and dQ items;
+ * Backward: a pass for the rows' statistics, then one deterministic kernel over dK/dV items (transposed scores) and dQ items; every output is
+ * written by TMA stores of whole tiles;
  * scratch: 2*B*H*(S rounded up to 128) + 2 floats.  All pointers at 16-byte boundaries.
  * llmctl_flash_{fwd,bwd}_status: 0 unless a bounded wait ran out since the last clearing call (synchronises the device). */
 int llmctl_flash_fwd_status(int clear);

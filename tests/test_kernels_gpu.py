@@ -478,6 +478,29 @@ def test_flash_attention_edges_of_blocks(cuda_device, B, S, H, D, causal, shift)
             assert (a - b).norm() <= bound, f"{name} head {h}: {((a - b).norm() / b.norm()).item():.2e}"
 
 
+# several items of one to five blocks per CTA, so that tiles, statistics and accumulators are handed on between items of every length and kind
+@pytest.mark.parametrize("B,S,H,D,causal", [(4, 640, 40, 128, True), (4, 520, 70, 64, True), (12, 100, 64, 128, True), (3, 384, 100, 64, False)])
+def test_flash_attention_backward_over_many_items(cuda_device, B, S, H, D, causal):
+    """Gradients against float64 products of a few heads (bounds as above), and again, bit for bit: nothing depends on who takes which item."""
+    from llmctl_b200.ops import attention as attn, native
+    torch.manual_seed(S)
+    q, k, v = (torch.randn(B, S, H, D, device=cuda_device).bfloat16().requires_grad_(True) for _ in range(3))
+    do = torch.randn(B, S, H, D, device=cuda_device).bfloat16()
+    o = attn.attention(q, k, v, causal=causal)
+    got = torch.autograd.grad(o, (q, k, v), do, retain_graph=True)
+    for a, b in zip(got, torch.autograd.grad(o, (q, k, v), do)):
+        assert torch.equal(a, b)
+    assert native.lib().llmctl_flash_bwd_status(1) == 0
+    for h in (0, H // 2, H - 1):
+        qd, kd, vd = (t.detach()[:, :, h].double().requires_grad_(True) for t in (q, k, v))
+        s = qd @ kd.transpose(-1, -2) / math.sqrt(D)
+        if causal:
+            s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device=cuda_device).triu(1), float("-inf"))
+        want = torch.autograd.grad(torch.softmax(s, -1) @ vd, (qd, kd, vd), do[:, :, h].double())
+        for name, a, b in zip(("dq", "dk", "dv"), got, want):
+            assert (a[:, :, h].double() - b).norm() <= 3 * 2.0 ** -9 * b.norm(), f"{name} head {h}"
+
+
 @pytest.mark.parametrize("S,D", [(130, 64), (128, 64), (77, 128), (128, 128)])
 @pytest.mark.parametrize("packed", [False, True])
 def test_flash_attention_gradients_at_odd_addresses(cuda_device, S, D, packed):

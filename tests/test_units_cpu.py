@@ -578,6 +578,82 @@ def test_flash_backward_accumulator_handover_orders_its_barriers(kinds):
 
 
 
+def test_flash_backward_slots_follow_their_hand_backs(tmp_path):
+    """csrc/attention/flash_bwd_slots.cuh against a queue of slots, over runs of items of 1 to 17 blocks: loads and hand-backs are numbered
+    in their stated orders without gaps, a load takes the slot that was handed back first, and what lay there was handed back no later
+    than the hand-back that the load waits for."""
+    import shutil
+    import subprocess
+    root = Path(__file__).resolve().parents[1]
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("needs g++")
+    (tmp_path / "t.cpp").write_text(r"""
+#define __device__
+#define __forceinline__ inline
+#include "attention/flash_bwd_slots.cuh"
+#include <cstdio>
+#include <cstdlib>
+#include <tuple>
+#include <map>
+#include <vector>
+using namespace llmctl::fbwd;
+typedef std::tuple<char, int, int> Tile;                    // r or e, operand, block
+#define CHECK(x) if (!(x)) { printf("line %d\n", __LINE__); return 1; }
+int main() {
+  srand(1);
+  for (int run = 0; run < 200; ++run) {
+    Slots s;
+    std::vector<uint32_t> queue;                            // slots in the order in which they are free
+    for (uint32_t i = 0; i < kTiles; ++i) queue.push_back(i);
+    std::map<uint32_t, uint32_t> free_at;                   // slot -> number of the hand-back that freed it
+    for (int item = 0; item < 40; ++item) {
+      const int n = run % 4 ? 1 + rand() % 4 : 1 + rand() % 17;
+      std::vector<Tile> loads, backs;
+      for (int i = 0; i < n; ++i)
+        for (int w = 0; w < 2; ++w) {
+          if (i == 0) loads.push_back(Tile('r', w, 0));
+          loads.push_back(Tile('e', w, i));
+        }
+      for (int i = 0; i < n; ++i) {
+        if (n == 1) { backs.push_back(Tile('r', 0, 0)); backs.push_back(Tile('r', 1, 0)); }
+        backs.push_back(Tile('e', 1, i));
+        if (i == n - 2) backs.push_back(Tile('r', 0, 0));
+        backs.push_back(Tile('e', 0, i));
+        if (i == n - 2) backs.push_back(Tile('r', 1, 0));
+      }
+      auto slot = [&](Tile t) { return std::get<0>(t) == 'r' ? s.res(std::get<1>(t)) : s.streamed(std::get<1>(t), std::get<2>(t)); };
+      size_t back = 0;
+      for (size_t j = 0; j < loads.size(); ++j) {
+        const Tile t = loads[j];
+        const uint32_t l = s.base + j;
+        CHECK((std::get<0>(t) == 'r' ? s.load_res(std::get<1>(t)) : s.load_streamed(std::get<1>(t), std::get<2>(t))) == l)
+        while (queue.size() <= l) {                         // this item's own hand-backs, in order
+          free_at[slot(backs[back])] = s.base + back;
+          queue.push_back(slot(backs[back++]));
+        }
+        CHECK(slot(t) == queue[l])
+        CHECK(l < kTiles || free_at[slot(t)] <= l - kTiles)
+      }
+      for (size_t j = 0; j < backs.size(); ++j) {
+        const Tile t = backs[j];
+        CHECK((std::get<0>(t) == 'r' ? s.given_res(std::get<1>(t), n) : s.given_streamed(std::get<1>(t), std::get<2>(t), n)) == s.base + j)
+        if (j >= back) {
+          free_at[slot(t)] = s.base + j;
+          queue.push_back(slot(t));
+        }
+      }
+      s.next(n);
+    }
+  }
+  return 0;
+}
+""")
+    subprocess.run([gxx, "-std=c++17", "-I", str(root / "csrc"), str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t")], check=True)
+    r = subprocess.run([str(tmp_path / "t")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+
+
 def test_shared_memory_limits_are_raised_and_never_lowered(tmp_path):
     """csrc/common/smem_limit.h with the runtime's two calls replaced: threads that ask for unlike sizes of one kernel leave the largest in
     place, a device counts by itself, and a call that was refused is asked again."""
