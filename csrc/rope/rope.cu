@@ -55,6 +55,7 @@ LLMCTL_API int llmctl_rope_inplace(void* x, long long row_stride, int n_tokens, 
                                    const int* positions, int seq_len, float sign, void* stream) {
   LLMCTL_BEGIN();
   LLMCTL_REQUIRE(head_dim % 16 == 0 && row_stride % 8 == 0 && seq_len > 0);
+  LLMCTL_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15) == 0);
   const long long total = static_cast<long long>(n_tokens) * n_heads * (head_dim / 16);
   if (total == 0) return 0;
   long long blocks = (total + 255) / 256;

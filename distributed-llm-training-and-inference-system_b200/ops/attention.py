@@ -114,9 +114,10 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
     if _native_ok(q, k, v, causal):
         return native.apply(_FlashAttnFn, q, k, v, scale, causal)
-    if _native_built(q) and _native_shape(q, k, v, causal) and k.dtype == v.dtype == q.dtype and (q.shape[-1] == 64 or q.shape[1] % 128):
-        # other strides or an odd address: head_dim 64 and ragged lengths (gpt-125m, every serving prefill) are always copied for
-        # the kernel, whole 128-wide tiles are left to the library
+    if (_native_built(q) and _native_shape(q, k, v, causal) and k.dtype == v.dtype == q.dtype
+            and (q.shape[-1] == 64 or q.shape[1] % 128 or any(t.data_ptr() % 16 for t in (q, k, v)))):
+        # other strides: head_dim 64 and ragged lengths (gpt-125m, every serving prefill) are always copied for the kernel, whole
+        # 128-wide tiles are left to the library.  Odd addresses are always copied: the library reads 16-byte units as well.
         q, k, v = (t.clone(memory_format=torch.contiguous_format) for t in (q, k, v))
         return native.apply(_FlashAttnFn, q, k, v, scale, causal)
     return _sdpa(q, k, v, causal, scale)
@@ -243,10 +244,10 @@ def rope_attention_packed(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tenso
         use_native = _native_ok(v5[:, :, 0], v5[:, :, 1], v5[:, :, 2]) and \
             (native.has_symbol("llmctl_flash_attn_bwd") or not torch.is_grad_enabled())
         pos = None if positions is None else positions.to(torch.int32)
-        # views the kernel only takes after a copy (an odd address at head_dim 64 or a ragged length) go through the composed
+        # views the kernels only take after a copy (an odd address) go through the composed
         # ops below, where attention() makes it, instead of dropping to the library inside the fused node
         paddable = (not use_native and cfg.attention == "native" and native.has_symbol("llmctl_flash_attn_bwd")
-                    and (head_dim == 64 or (head_dim == 128 and seq % 128 != 0)))
+                    and (head_dim == 64 or (head_dim == 128 and (seq % 128 != 0 or qkv.data_ptr() % 16 != 0))))
         if not paddable:
             return native.apply(_RopeAttnPackedFn, qkv, cos, sin, batch, seq, heads, head_dim, pos, scale, use_native)
     qkv = ops.rope_packed(qkv, cos, sin, 2 * heads, head_dim, seq, positions)

@@ -478,6 +478,25 @@ def test_flash_attention_edges_of_blocks(cuda_device, B, S, H, D, causal, shift)
             assert (a - b).norm() <= bound, f"{name} head {h}: {((a - b).norm() / b.norm()).item():.2e}"
 
 
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_whole_tiles_at_odd_addresses_are_copied(cuda_device, which):
+    """Heads of 128 and whole 128-token tiles where one of q, k and v begins at an odd address: the kernels run on copies, and nothing else
+    (the library's attention reads 16-byte units at the address that it is given)."""
+    from llmctl_b200.ops import attention as attn, native
+    torch.manual_seed(which)
+    qkv = [torch.randn(2 * 128 * 3 * 128 + 1, device=cuda_device).bfloat16()[int(i == which):][:2 * 128 * 3 * 128].view(2, 128, 3, 128).detach().requires_grad_(True)
+           for i in range(3)]
+    do = torch.randn(2, 128, 3, 128, device=cuda_device).bfloat16()
+    before = native.launch_count
+    o = attn.attention(*qkv)
+    got = (o.detach(), *torch.autograd.grad(o, qkv, do))
+    assert native.launch_count == before + 3
+    whole = [t.detach().clone().requires_grad_(True) for t in qkv]
+    o = attn.attention(*whole)
+    for a, b in zip(got, (o.detach(), *torch.autograd.grad(o, whole, do))):
+        assert torch.equal(a, b)
+
+
 # several items of one to five blocks per CTA, so that tiles, statistics and accumulators are handed on between items of every length and kind
 @pytest.mark.parametrize("B,S,H,D,causal", [(4, 640, 40, 128, True), (4, 520, 70, 64, True), (12, 100, 64, 128, True), (3, 384, 100, 64, False)])
 def test_flash_attention_backward_over_many_items(cuda_device, B, S, H, D, causal):
