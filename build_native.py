@@ -2,6 +2,7 @@
 """Build the native libraries in-tree.
 
   libllmctl_b200.so : every sm_100a CUDA kernel behind a C ABI (include/llmctl_b200.h)
+  llmctl_ops.so     : the operators' host side (checks, allocation, launch, autograd nodes) as a Python extension over libtorch
   libllmctl_host.so : C++ host runtime (KV block manager, batch scheduler, ...), no CUDA needed
 
 Sources are compiled one translation unit per nvcc/g++ process (in parallel) and only when the
@@ -99,6 +100,27 @@ def _compile(cmd: list[str], src: Path, obj: Path, verbose: bool) -> tuple[Path,
     return obj, (r.stdout + r.stderr) if verbose else ""
 
 
+def _build_operators(force: bool, hdr_m: float, verbose: bool) -> Path:
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(find_nvcc() or "/usr/local/cuda/bin/nvcc").resolve().parents[1]
+    src, obj, lib = CSRC / "torch" / "ops.cpp", OBJDIR / "torch" / "ops.o", LIBDIR / "llmctl_ops.so"
+    if not force and lib.exists() and lib.stat().st_mtime > max(src.stat().st_mtime, hdr_m):
+        return lib
+    cxx = os.environ.get("CXX", "g++")
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             "-I", str(ROOT / "include"), "-I", str(root / "include"), "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"),
+             "-I", str(cuda / "include"), "-I", sysconfig.get_paths()["include"]]
+    _compile([cxx, *flags, "-c", str(src), "-o", str(obj)], src, obj, verbose)
+    link = [cxx, "-shared", "-o", str(lib), str(obj), "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-ldl"]
+    r = subprocess.run(link, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"link failed: {src}\n{' '.join(link)}\n{r.stdout}\n{r.stderr}")
+    return lib
+
+
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False, jobs: int | None = None,
           components=None) -> dict:
     LIBDIR.mkdir(parents=True, exist_ok=True)
@@ -141,6 +163,9 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False, 
                 raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
             manifest.write_text("\n".join(sorted(wanted)))
         out["kernels"] = str(lib)
+
+    # ---- host side of the operators: a Python extension over libtorch ----
+    out["operators"] = str(_build_operators(force, hdr_m, verbose))
 
     # ---- host C++ ----
     cpp_srcs = sorted(p for p in (CSRC / "host").glob("*.cpp"))

@@ -1,0 +1,578 @@
+// Host side of the operators that a layer is made of: checks, allocation, launch and autograd nodes in C++, as a Python extension over
+// libtorch.  The kernels are those of libllmctl_b200.so, through its C ABI.
+//
+// What it is for: a launch costs the driver 4.5 us, but an operator of the Python modules (ops/functional.py, ops/attention.py,
+// ops/serving.py) cost 16-17 us without gradients and 22-60 us with them, so that a small model, a decoding step or a layer's backward waited
+// for Python (12 layers of width 768: 2340 us for 760 us of kernels).  Every function here takes plain tensors in the layouts that its
+// kernel reads and returns None for anything else (subclasses, dispatch or function modes, functorch, tracing, forward-mode gradients, other
+// types, strides, addresses): the Python operator then goes its own way, as it does for CPU tensors.
+//
+// Reference: none (the reference has no native layer).
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+
+#include <atomic>
+#include <initializer_list>
+
+#include "llmctl_b200.h"
+
+namespace {
+
+using at::Tensor;
+
+// ---------------------------------------------------------------------------------------------------------------------------------
+// the kernel library
+// ---------------------------------------------------------------------------------------------------------------------------------
+#define LLMCTL_ENTRIES(X)                                                                                                         \
+  X(llmctl_rmsnorm_fwd) X(llmctl_rmsnorm_bwd) X(llmctl_rope_inplace) X(llmctl_gemm_bf16) X(llmctl_gemm_swiglu_bf16)               \
+  X(llmctl_gemm_swiglu_bwd_bf16) X(llmctl_gemm_skinny_bf16) X(llmctl_flash_attn_fwd) X(llmctl_flash_attn_bwd) X(llmctl_kv_append) \
+  X(llmctl_paged_attn_decode) X(llmctl_paged_attn_scratch_elems)
+struct Entries {
+#define X(name) decltype(&::name) name = nullptr;
+  LLMCTL_ENTRIES(X)
+#undef X
+  const volatile uint32_t* waits = nullptr;      // != 0: a bounded wait of a kernel ran out (csrc/common/wait_status.h)
+  void* (*wait_word)() = nullptr;
+} lib;                                           // entries that a partial build leaves out stay null
+
+PyObject* native_error = nullptr;                // ops.native.NativeError
+PyObject* check_waits = nullptr;                 // ops.native.check_waits
+std::atomic<long long> launches{0};
+
+// Whether an entry can be called: it is there and no wait has run out (the Python operator reports that one).
+template <typename F>
+bool ready(F* f) {
+  if (f == nullptr) return false;
+  if (lib.waits == nullptr) {
+    if (lib.wait_word == nullptr) return false;
+    lib.waits = static_cast<const volatile uint32_t*>(lib.wait_word());
+  }
+  return lib.waits != nullptr && *lib.waits == 0;
+}
+
+struct Failed {                                  // of a call into the kernel library, thrown without the GIL
+  const char* name;
+  int rc;
+};
+void done(const char* name, int rc, int kernels = 1) {
+  launches.fetch_add(kernels, std::memory_order_relaxed);
+  if (rc != 0) throw Failed{name, rc};
+}
+void set_failed(const Failed& f) { PyErr_Format(native_error, "%s failed with cudaError %d", f.name, f.rc); }
+
+// Body of an autograd node's backward: errors become the Python exceptions that the Python operators raise.
+template <typename Body>
+torch::autograd::variable_list node_body(const char* name, bool there, Body&& body) {
+  try {
+    if (there) return body();
+  } catch (const Failed& f) {
+    pybind11::gil_scoped_acquire gil;
+    set_failed(f);
+    python_error e;
+    e.persist();
+    throw e;
+  }
+  pybind11::gil_scoped_acquire gil;
+  PyObject* r = PyObject_CallFunction(check_waits, "s", name);
+  if (r != nullptr) PyErr_Format(native_error, "%s is not in the library", name);
+  Py_XDECREF(r);
+  python_error e;
+  e.persist();
+  throw e;
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------------
+// what the functions take
+// ---------------------------------------------------------------------------------------------------------------------------------
+// Nothing wants to see or replace the operators: no mode, transform or trace is active.
+bool quiet() {
+  return c10::impl::TorchDispatchModeTLS::stack_len() == 0 && at::impl::PythonTorchFunctionTLS::stack_len() == 0 &&
+         !c10::impl::tls_local_dispatch_key_set().included_.has_any(
+             c10::DispatchKeySet({c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::FuncTorchDynamicLayerBackMode, c10::DispatchKey::Functionalize})) &&
+         !torch::jit::tracer::isTracing();
+}
+bool is_plain(const Tensor& t) {
+  return t.is_cuda() && t.layout() == at::kStrided && !t.is_nested() &&
+         !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                                   c10::DispatchKey::Functionalize, c10::DispatchKey::ZeroTensor, c10::DispatchKey::Negative,
+                                                   c10::DispatchKey::Conjugate})) &&
+         !torch::autograd::isFwGradDefined(t);
+}
+bool bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16; }
+bool unit16(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0; }
+// an operand of the GEMMs: rows of whole 16-byte units
+bool is_matrix(const Tensor& t) { return bf16(t) && t.dim() == 2 && t.stride(1) == 1 && t.stride(0) % 8 == 0 && unit16(t); }
+bool recorded(std::initializer_list<const Tensor*> ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : ts)
+    if (t->requires_grad()) return true;
+  return false;
+}
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+Tensor empty_like_on(const Tensor& t, at::IntArrayRef size, at::ScalarType type) { return at::empty(size, t.options().dtype(type).requires_grad(false)); }
+Tensor new_bf16(const Tensor& t, at::IntArrayRef size) { return empty_like_on(t, size, at::kBFloat16); }
+Tensor new_f32(const Tensor& t, at::IntArrayRef size) { return empty_like_on(t, size, at::kFloat); }
+void* data(const Tensor& t) { return t.data_ptr(); }
+const void* cdata(const Tensor& t) { return t.const_data_ptr(); }
+
+// Arguments of a call.  A tensor argument is a torch.Tensor or Parameter itself; `ok` turns false for anything else.
+struct Args {
+  PyObject* const* a;
+  Py_ssize_t n;
+  bool ok = true;
+  Tensor tensor(int i) {
+    if (!THPVariable_CheckExact(a[i])) {
+      ok = false;
+      return Tensor();
+    }
+    Tensor t = THPVariable_Unpack(a[i]);
+    if (!is_plain(t)) ok = false;
+    return t;
+  }
+  Tensor optional(int i) { return a[i] == Py_None ? Tensor() : tensor(i); }
+  long long integer(int i) {
+    const long long v = PyLong_AsLongLong(a[i]);
+    if (v == -1 && PyErr_Occurred()) throw python_error();
+    return v;
+  }
+  double number(int i) {
+    const double v = PyFloat_AsDouble(a[i]);
+    if (v == -1.0 && PyErr_Occurred()) throw python_error();
+    return v;
+  }
+};
+
+// Runs `body` without the GIL.
+template <typename Body>
+auto without_gil(Body&& body) {
+  pybind11::gil_scoped_release released;
+  return body();
+}
+
+template <typename Body>
+PyObject* call(PyObject* const* a, Py_ssize_t n, Py_ssize_t want, Body&& body) {
+  HANDLE_TH_ERRORS
+  if (n != want) {
+    PyErr_Format(PyExc_TypeError, "takes %zd arguments (%zd given)", want, n);
+    return nullptr;
+  }
+  try {
+    Args args{a, n};
+    return body(args);
+  } catch (const Failed& f) {
+    set_failed(f);
+    return nullptr;
+  }
+  END_HANDLE_TH_ERRORS
+}
+PyObject* none() { Py_RETURN_NONE; }
+PyObject* pair(const Tensor& a, PyObject* b) {
+  PyObject* x = THPVariable_Wrap(a);
+  PyObject* r = x == nullptr || b == nullptr ? nullptr : PyTuple_Pack(2, x, b);
+  Py_XDECREF(x);
+  Py_XDECREF(b);
+  return r;
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------------
+// RMS norm
+// ---------------------------------------------------------------------------------------------------------------------------------
+struct NormOut {
+  Tensor y, h, rstd;
+};
+NormOut norm_fwd(const Tensor& x, const Tensor& residual, const Tensor& w, double eps, bool keep) {
+  const int64_t cols = x.size(-1), rows = x.numel() / cols;
+  NormOut r{new_bf16(x, x.sizes()), residual.defined() ? new_bf16(x, x.sizes()) : x, keep ? new_f32(x, {rows}) : Tensor()};
+  done("llmctl_rmsnorm_fwd", lib.llmctl_rmsnorm_fwd(cdata(x), residual.defined() ? cdata(residual) : nullptr, cdata(w), residual.defined() ? data(r.h) : nullptr, data(r.y),
+                                                    keep ? static_cast<float*>(data(r.rstd)) : nullptr, static_cast<int>(rows), static_cast<int>(cols),
+                                                    static_cast<float>(eps), stream()));
+  return r;
+}
+
+constexpr int kNormBwdCtas = 148 * 4;
+
+// y = rmsnorm(x + residual) * w, and h = x + residual where there is a residual.
+struct RmsNorm : torch::autograd::Function<RmsNorm> {
+  static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& residual, const Tensor& w,
+                                               double eps) {
+    NormOut r = norm_fwd(x, residual.value_or(Tensor()), w, eps, true);
+    ctx->save_for_backward({r.h, w, r.rstd});
+    ctx->saved_data["residual"] = residual.has_value();
+    if (residual.has_value()) return {r.y, r.h};
+    return {r.y};
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    return node_body("llmctl_rmsnorm_bwd", ready(lib.llmctl_rmsnorm_bwd), [&]() -> torch::autograd::variable_list {
+      const auto saved = ctx->get_saved_variables();
+      const Tensor &h = saved[0], &w = saved[1], &rstd = saved[2];
+      const bool residual = ctx->saved_data["residual"].toBool();
+      const int64_t cols = h.size(-1), rows = h.numel() / cols;
+      const Tensor dy = grads[0].contiguous(), dres = residual ? grads[1].contiguous() : Tensor();
+      Tensor dx = new_bf16(h, h.sizes()), dw = new_f32(h, {cols});
+      const int ctas = static_cast<int>(rows < kNormBwdCtas ? rows : kNormBwdCtas);
+      Tensor scratch = new_f32(h, {ctas * cols});
+      done("llmctl_rmsnorm_bwd", lib.llmctl_rmsnorm_bwd(cdata(dy), cdata(h), cdata(w), static_cast<const float*>(cdata(rstd)), residual ? cdata(dres) : nullptr, data(dx),
+                                                        static_cast<float*>(data(dw)), static_cast<float*>(data(scratch)), ctas, static_cast<int>(rows),
+                                                        static_cast<int>(cols), 0, stream()), 2);
+      return {dx, residual ? dx : Tensor(), dw.to(w.scalar_type()), Tensor()};
+    });
+  }
+};
+
+// rmsnorm(x, residual or None, w, eps) -> (y, h)
+PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 4, [&](Args& args) -> PyObject* {
+    const Tensor x = args.tensor(0), residual = args.optional(1), w = args.tensor(2);
+    const double eps = args.number(3);
+    if (!args.ok || !quiet() || !ready(lib.llmctl_rmsnorm_fwd) || !bf16(x) || !bf16(w) || x.dim() < 1 || x.numel() == 0 || !x.is_contiguous() || w.dim() != 1 ||
+        w.size(0) != x.size(-1) || !w.is_contiguous() || !unit16(x) || !unit16(w))
+      return none();
+    if (residual.defined() && (!bf16(residual) || !residual.is_contiguous() || residual.sizes() != x.sizes() || !unit16(residual))) return none();
+    const bool grad = residual.defined() ? recorded({&x, &residual, &w}) : recorded({&x, &w});
+    Tensor y, h;
+    without_gil([&] {
+      if (grad) {
+        const auto out = RmsNorm::apply(x, residual.defined() ? std::optional<Tensor>(residual) : std::nullopt, w, eps);
+        y = out[0];
+        if (residual.defined()) h = out[1];
+      } else {
+        NormOut r = norm_fwd(x, residual, w, eps, false);
+        y = r.y;
+        h = r.h;
+      }
+    });
+    if (residual.defined()) return pair(y, THPVariable_Wrap(h));
+    Py_INCREF(a[0]);
+    return pair(y, a[0]);
+  });
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------------
+// GEMMs
+// ---------------------------------------------------------------------------------------------------------------------------------
+void gemm(const Tensor& a, const Tensor& b, const Tensor& c, bool a_mn, bool b_mn, bool accumulate, int tile_n, int max_ctas) {
+  const int64_t M = c.size(0), N = c.size(1), K = a_mn ? a.size(0) : a.size(1);
+  done("llmctl_gemm_bf16", lib.llmctl_gemm_bf16(cdata(a), cdata(b), data(c), static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), a.stride(0), b.stride(0),
+                                                c.stride(0), a_mn, b_mn, c.scalar_type() == at::kFloat, accumulate, tile_n, max_ctas, stream()));
+}
+
+// gemm(a, b, a_mn, b_mn, out or None, fp32, accumulate, tile_n, max_ctas) -> out
+PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 9, [&](Args& args) -> PyObject* {
+    const Tensor x = args.tensor(0), y = args.tensor(1);
+    Tensor out = args.optional(4);
+    const bool a_mn = args.integer(2), b_mn = args.integer(3), fp32 = args.integer(5), accumulate = args.integer(6);
+    const int tile_n = static_cast<int>(args.integer(7)), max_ctas = static_cast<int>(args.integer(8));
+    if (!args.ok || !quiet() || !ready(lib.llmctl_gemm_bf16) || !bf16(x) || !bf16(y) || x.dim() != 2 || y.dim() != 2 || x.stride(1) != 1 || y.stride(1) != 1) return none();
+    const int64_t M = x.size(a_mn ? 1 : 0), N = y.size(b_mn ? 1 : 0);
+    if (x.size(a_mn ? 0 : 1) != y.size(b_mn ? 0 : 1)) return none();
+    if (out.defined() ? out.dim() != 2 || out.size(0) != M || out.size(1) != N || out.stride(1) != 1 || (out.scalar_type() != at::kFloat && !bf16(out)) : accumulate)
+      return none();
+    without_gil([&] {
+      if (!out.defined()) out = empty_like_on(x, {M, N}, fp32 ? at::kFloat : at::kBFloat16);
+      gemm(x, y, out, a_mn, b_mn, accumulate, tile_n, max_ctas);
+    });
+    return THPVariable_Wrap(out);
+  });
+}
+
+// rows of the last dimension as a matrix for the GEMMs, or undefined
+Tensor as_rows(const Tensor& x) {
+  if (x.dim() == 2) return is_matrix(x) ? x : Tensor();
+  if (x.dim() < 1 || !x.is_contiguous()) return Tensor();
+  const Tensor r = x.view({-1, x.size(-1)});
+  return is_matrix(r) ? r : Tensor();
+}
+Tensor as_shape_of(const Tensor& y, const Tensor& x) {
+  if (x.dim() == 2) return y;
+  auto size = x.sizes().vec();
+  size.back() = y.size(1);
+  return y.view(size);
+}
+
+// linear(x, w, tile_n, workspace or None, counters) -> x @ w.T where no gradient is recorded; few rows take the decode GEMM if there is a workspace
+PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 5, [&](Args& args) -> PyObject* {
+    const Tensor x = args.tensor(0), w = args.tensor(1);
+    const int tile_n = static_cast<int>(args.integer(2));
+    if (!args.ok || !quiet() || !is_matrix(w) || x.numel() == 0 || recorded({&x, &w})) return none();
+    const Tensor rows = as_rows(x);
+    if (!rows.defined() || rows.size(1) != w.size(1)) return none();
+    const bool skinny = a[3] != Py_None;
+    if (skinny ? !ready(lib.llmctl_gemm_skinny_bf16) : !ready(lib.llmctl_gemm_bf16) || w.size(0) % 8) return none();
+    const Tensor ws = skinny ? args.tensor(3) : Tensor(), counters = skinny ? args.tensor(4) : Tensor();
+    if (!args.ok) return none();
+    Tensor y = without_gil([&] {
+      Tensor out = new_bf16(x, {rows.size(0), w.size(0)});
+      if (skinny)
+        done("llmctl_gemm_skinny_bf16",
+             lib.llmctl_gemm_skinny_bf16(cdata(rows), cdata(w), data(out), static_cast<int>(rows.size(0)), static_cast<int>(w.size(0)), static_cast<int>(w.size(1)),
+                                         rows.stride(0), w.stride(0), out.stride(0), static_cast<float*>(data(ws)), ws.numel(),
+                                         static_cast<unsigned int*>(data(counters)), static_cast<int>(counters.numel()), 0, stream()));
+      else
+        gemm(rows, w, out, false, false, false, tile_n, 0);
+      return as_shape_of(out, x);
+    });
+    return THPVariable_Wrap(y);
+  });
+}
+
+// gemm_swiglu(x, w, keep) -> (swiglu(x @ w.T), the product before or None)
+PyObject* py_gemm_swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 3, [&](Args& args) -> PyObject* {
+    const Tensor x = args.tensor(0), w = args.tensor(1);
+    const bool keep = args.integer(2);
+    if (!args.ok || !quiet() || !ready(lib.llmctl_gemm_swiglu_bf16) || !is_matrix(x) || !is_matrix(w) || x.size(1) != w.size(1) || w.size(0) % 16) return none();
+    Tensor act, gu;
+    without_gil([&] {
+      const int64_t M = x.size(0), F = w.size(0) / 2;
+      act = new_bf16(x, {M, F});
+      if (keep) gu = new_bf16(x, {M, 2 * F});
+      done("llmctl_gemm_swiglu_bf16", lib.llmctl_gemm_swiglu_bf16(cdata(x), cdata(w), keep ? data(gu) : nullptr, data(act), static_cast<int>(M), static_cast<int>(F),
+                                                                  static_cast<int>(x.size(1)), x.stride(0), w.stride(0), 2 * F, F, stream()));
+    });
+    if (keep) return pair(act, THPVariable_Wrap(gu));
+    Py_INCREF(Py_None);
+    return pair(act, Py_None);
+  });
+}
+
+// mlp(x, w_up, w_down, tile_n) -> swiglu(x @ w_up.T) @ w_down.T where no gradient is recorded
+PyObject* py_mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 4, [&](Args& args) -> PyObject* {
+    const Tensor x = args.tensor(0), up = args.tensor(1), down = args.tensor(2);
+    const int least = static_cast<int>(args.integer(3));
+    if (!args.ok || !quiet() || !ready(lib.llmctl_gemm_swiglu_bf16) || !ready(lib.llmctl_gemm_bf16) || !is_matrix(up) || !is_matrix(down) || x.numel() == 0 ||
+        recorded({&x, &up, &down}) || up.size(0) % 16 || down.size(0) % 8 || down.size(1) != up.size(0) / 2)
+      return none();
+    const Tensor rows = as_rows(x);
+    if (!rows.defined() || rows.size(1) != up.size(1) || rows.size(0) <= least) return none();
+    Tensor y = without_gil([&] {
+      const int64_t M = rows.size(0), F = up.size(0) / 2;
+      Tensor act = new_bf16(x, {M, F}), out = new_bf16(x, {M, down.size(0)});
+      done("llmctl_gemm_swiglu_bf16", lib.llmctl_gemm_swiglu_bf16(cdata(rows), cdata(up), nullptr, data(act), static_cast<int>(M), static_cast<int>(F),
+                                                                  static_cast<int>(rows.size(1)), rows.stride(0), up.stride(0), 2 * F, F, stream()));
+      gemm(act, down, out, false, false, false, 0, 0);
+      return as_shape_of(out, x);
+    });
+    return THPVariable_Wrap(y);
+  });
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------------
+// attention
+// ---------------------------------------------------------------------------------------------------------------------------------
+struct AttnOut {
+  Tensor o, lse;
+};
+// q, k, v: [B, S, H, D] as attention_ok takes them
+bool attention_ok(const Tensor& q, const Tensor& k, const Tensor& v, bool causal) {
+  if (q.dim() != 4 || !bf16(q)) return false;
+  const int64_t B = q.size(0), S = q.size(1), H = q.size(2), D = q.size(3);
+  if ((D != 64 && D != 128) || B < 1 || S < 1 || H < 1 || (!causal && S % 128)) return false;
+  for (const Tensor* t : {&q, &k, &v})
+    if (t->dim() != 4 || !bf16(*t) || t->sizes() != q.sizes() || t->stride(3) != 1 || t->stride(2) != D || (B > 1 && t->stride(0) != S * t->stride(1)) ||
+        t->stride(1) % 8 || !unit16(*t))
+      return false;
+  return true;
+}
+AttnOut attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal, bool keep) {
+  const int64_t B = q.size(0), S = q.size(1), H = q.size(2), D = q.size(3);
+  AttnOut r{new_bf16(q, {B, S, H, D}), keep ? new_f32(q, {B, H, S}) : Tensor()};
+  done("llmctl_flash_attn_fwd", lib.llmctl_flash_attn_fwd(cdata(q), cdata(k), cdata(v), data(r.o), keep ? static_cast<float*>(data(r.lse)) : nullptr, static_cast<int>(B),
+                                                          static_cast<int>(S), static_cast<int>(H), static_cast<int>(D), q.stride(1), k.stride(1), v.stride(1),
+                                                          H * D, static_cast<float>(scale), causal, stream()));
+  return r;
+}
+// dq | dk | dv, packed like the projection that made q | k | v, so that the weight gradient that follows sees one tensor
+Tensor attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& grad, double scale, bool causal) {
+  const int64_t B = q.size(0), S = q.size(1), H = q.size(2), D = q.size(3);
+  Tensor d_o = grad.contiguous();
+  if (!unit16(d_o)) d_o = d_o.clone();
+  Tensor d = new_bf16(q, {B, S, 3, H, D});
+  Tensor scratch = new_f32(q, {2 * B * H * ((S + 127) / 128 * 128) + 2});
+  char* at = static_cast<char*>(data(d));
+  done("llmctl_flash_attn_bwd", lib.llmctl_flash_attn_bwd(cdata(q), cdata(k), cdata(v), cdata(o), cdata(d_o), static_cast<const float*>(cdata(lse)), at, at + 2 * H * D,
+                                                          at + 4 * H * D, static_cast<float*>(data(scratch)), static_cast<int>(B), static_cast<int>(S),
+                                                          static_cast<int>(H), static_cast<int>(D), q.stride(1), k.stride(1), v.stride(1), H * D, 3 * H * D,
+                                                          static_cast<float>(scale), causal, stream()), 2);
+  return d;
+}
+
+struct FlashAttention : torch::autograd::Function<FlashAttention> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal) {
+    AttnOut r = attn_fwd(q, k, v, scale, causal, true);
+    ctx->save_for_backward({q, k, v, r.o, r.lse});
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["causal"] = causal;
+    return r.o;
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    return node_body("llmctl_flash_attn_bwd", ready(lib.llmctl_flash_attn_bwd), [&]() -> torch::autograd::variable_list {
+      const auto s = ctx->get_saved_variables();
+      const Tensor d = attn_bwd(s[0], s[1], s[2], s[3], s[4], grads[0], ctx->saved_data["scale"].toDouble(), ctx->saved_data["causal"].toBool());
+      return {d.select(2, 0), d.select(2, 1), d.select(2, 2), Tensor(), Tensor()};
+    });
+  }
+};
+
+// attention(q, k, v, scale, causal) -> [B, S, H, D]
+PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 5, [&](Args& args) -> PyObject* {
+    const Tensor q = args.tensor(0), k = args.tensor(1), v = args.tensor(2);
+    const double scale = args.number(3);
+    const bool causal = args.integer(4);
+    if (!args.ok || !quiet() || !ready(lib.llmctl_flash_attn_fwd) || !lib.llmctl_flash_attn_bwd || !attention_ok(q, k, v, causal)) return none();
+    const bool grad = recorded({&q, &k, &v});
+    Tensor o = without_gil([&] { return grad ? FlashAttention::apply(q, k, v, scale, causal) : attn_fwd(q, k, v, scale, causal, false).o; });
+    return THPVariable_Wrap(o);
+  });
+}
+
+// The first 2 H heads of packed rows q | k | v, rotated in place.
+void rope(const Tensor& x, const Tensor& cos, const Tensor& sin, const Tensor& positions, int64_t S, int64_t heads, int64_t D, float sign) {
+  done("llmctl_rope_inplace", lib.llmctl_rope_inplace(data(x), x.stride(0), static_cast<int>(x.size(0)), static_cast<int>(heads), static_cast<int>(D),
+                                                      static_cast<const float*>(cdata(cos)), static_cast<const float*>(cdata(sin)),
+                                                      positions.defined() ? static_cast<const int*>(cdata(positions)) : nullptr, static_cast<int>(S), sign, stream()));
+}
+struct Packed {
+  Tensor q, k, v;
+};
+Packed unpack(const Tensor& qkv, int64_t B, int64_t S, int64_t H, int64_t D) {
+  const Tensor v5 = qkv.detach().view({B, S, 3, H, D});
+  return {v5.select(2, 0), v5.select(2, 1), v5.select(2, 2)};
+}
+
+struct RopeAttention : torch::autograd::Function<RopeAttention> {
+  // rotates qkv in place: the product that made it keeps no copy of its output
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& qkv, const Tensor& cos, const Tensor& sin, const std::optional<Tensor>& positions,
+                        int64_t B, int64_t S, int64_t H, int64_t D, double scale) {
+    rope(qkv, cos, sin, positions.value_or(Tensor()), S, 2 * H, D, 1.f);
+    const Packed p = unpack(qkv, B, S, H, D);
+    AttnOut r = attn_fwd(p.q, p.k, p.v, scale, true, true);
+    ctx->save_for_backward({qkv.detach(), r.o, r.lse, cos, sin, positions.value_or(Tensor())});
+    ctx->saved_data["sizes"] = std::vector<int64_t>{B, S, H, D};
+    ctx->saved_data["scale"] = scale;
+    return r.o.view({B * S, H * D});
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    return node_body("llmctl_flash_attn_bwd", ready(lib.llmctl_flash_attn_bwd), [&]() -> torch::autograd::variable_list {
+      const auto s = ctx->get_saved_variables();
+      const auto z = ctx->saved_data["sizes"].toIntVector();
+      const int64_t B = z[0], S = z[1], H = z[2], D = z[3];
+      const Packed p = unpack(s[0], B, S, H, D);
+      const Tensor d = attn_bwd(p.q, p.k, p.v, s[1], s[2], grads[0].reshape({B, S, H, D}), ctx->saved_data["scale"].toDouble(), true).view({B * S, 3 * H * D});
+      rope(d, s[3], s[4], s[5], S, 2 * H, D, -1.f);
+      return {d, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    });
+  }
+};
+
+// rope_attention(qkv, cos, sin, positions or None, B, S, H, D, scale) -> [B * S, H * D]
+PyObject* py_rope_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 9, [&](Args& args) -> PyObject* {
+    const Tensor qkv = args.tensor(0), cos = args.tensor(1), sin = args.tensor(2), positions = args.optional(3);
+    const int64_t B = args.integer(4), S = args.integer(5), H = args.integer(6), D = args.integer(7);
+    const double scale = args.number(8);
+    if (!args.ok || !quiet() || !ready(lib.llmctl_rope_inplace) || !ready(lib.llmctl_flash_attn_fwd) || !lib.llmctl_flash_attn_bwd || !bf16(qkv) || qkv.dim() != 2 ||
+        !qkv.is_contiguous() || B < 1 || S < 1 || H < 1 || (D != 64 && D != 128) || qkv.size(0) != B * S || qkv.size(1) != 3 * H * D || !unit16(qkv) ||
+        cos.scalar_type() != at::kFloat || sin.scalar_type() != at::kFloat || !cos.is_contiguous() || !sin.is_contiguous() || cos.requires_grad() || sin.requires_grad())
+      return none();
+    if (positions.defined() && (positions.scalar_type() != at::kInt || !positions.is_contiguous() || positions.numel() != B * S)) return none();
+    if (qkv.is_leaf() && qkv.requires_grad()) return none();
+    const bool grad = recorded({&qkv});
+    Tensor o = without_gil([&] {
+      if (grad) return RopeAttention::apply(qkv, cos, sin, positions.defined() ? std::optional<Tensor>(positions) : std::nullopt, B, S, H, D, scale);
+      if (!qkv.is_inference()) qkv.unsafeGetTensorImpl()->bump_version();
+      rope(qkv, cos, sin, positions, S, 2 * H, D, 1.f);
+      const Packed p = unpack(qkv, B, S, H, D);
+      return attn_fwd(p.q, p.k, p.v, scale, true, false).o.view({B * S, H * D});
+    });
+    return THPVariable_Wrap(o);
+  });
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------------
+// paged cache
+// ---------------------------------------------------------------------------------------------------------------------------------
+// kv_append(qkv, k_cache, v_cache, slots, heads, head_dim) -> True
+PyObject* py_kv_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 6, [&](Args& args) -> PyObject* {
+    const Tensor qkv = args.tensor(0), k = args.tensor(1), v = args.tensor(2), slots = args.tensor(3);
+    const int64_t H = args.integer(4), D = args.integer(5), hd = H * D;
+    if (!args.ok || !quiet() || !ready(lib.llmctl_kv_append) || !bf16(qkv) || !bf16(k) || !bf16(v) || qkv.dim() != 2 || qkv.stride(1) != 1 || slots.scalar_type() != at::kLong)
+      return none();
+    without_gil([&] {
+      done("llmctl_kv_append", lib.llmctl_kv_append(cdata(qkv), qkv.stride(0), static_cast<int>(hd), static_cast<int>(2 * hd), data(k), data(v),
+                                                    static_cast<const long long*>(cdata(slots)), static_cast<int>(qkv.size(0)), static_cast<int>(H), static_cast<int>(D), stream()));
+    });
+    Py_RETURN_TRUE;
+  });
+}
+
+// paged_decode(q, k_cache, v_cache, tables, lens, max_context, splits, scale) -> out
+PyObject* py_paged_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 8, [&](Args& args) -> PyObject* {
+    const Tensor q = args.tensor(0), k = args.tensor(1), v = args.tensor(2), tables = args.tensor(3), lens = args.tensor(4);
+    const int context = static_cast<int>(args.integer(5)), splits = static_cast<int>(args.integer(6));
+    const double scale = args.number(7);
+    if (!args.ok || !quiet() || !ready(lib.llmctl_paged_attn_decode) || !lib.llmctl_paged_attn_scratch_elems || !bf16(q) || !bf16(k) || !bf16(v) || q.dim() != 3 || k.dim() != 4 ||
+        tables.dim() != 2 || tables.scalar_type() != at::kInt || lens.scalar_type() != at::kInt)
+      return none();
+    Tensor o = without_gil([&] {
+      const int B = static_cast<int>(q.size(0)), H = static_cast<int>(q.size(1)), D = static_cast<int>(q.size(2));
+      const long long need = lib.llmctl_paged_attn_scratch_elems(B, H, D, splits);
+      Tensor scratch = need ? new_f32(q, {need}) : Tensor(), out = new_bf16(q, q.sizes());
+      done("llmctl_paged_attn_decode", lib.llmctl_paged_attn_decode(cdata(q), q.stride(0), cdata(k), cdata(v), static_cast<const int*>(cdata(tables)), static_cast<int>(tables.size(1)),
+                                                                    static_cast<const int*>(cdata(lens)), data(out), out.stride(0), need ? static_cast<float*>(data(scratch)) : nullptr, B, H, D,
+                                                                    static_cast<int>(k.size(1)), context, splits, static_cast<float>(scale), stream()), need ? 2 : 1);
+      return out;
+    });
+    return THPVariable_Wrap(o);
+  });
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------------
+// the module
+// ---------------------------------------------------------------------------------------------------------------------------------
+// bind(path of the loaded kernel library, NativeError, check_waits)
+PyObject* py_bind(PyObject*, PyObject* args) {
+  const char* path;
+  PyObject *error, *waits;
+  if (!PyArg_ParseTuple(args, "sOO", &path, &error, &waits)) return nullptr;
+  void* so = dlopen(path, RTLD_NOW | RTLD_NOLOAD);
+  if (so == nullptr) {
+    PyErr_Format(PyExc_RuntimeError, "%s is not loaded", path);
+    return nullptr;
+  }
+#define X(name) lib.name = reinterpret_cast<decltype(lib.name)>(dlsym(so, #name));
+  LLMCTL_ENTRIES(X)
+#undef X
+  lib.wait_word = reinterpret_cast<void* (*)()>(dlsym(so, "llmctl_wait_status_word"));
+  Py_INCREF(error);
+  Py_INCREF(waits);
+  native_error = error;
+  check_waits = waits;
+  Py_RETURN_NONE;
+}
+PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(launches.load(std::memory_order_relaxed)); }
+
+#define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&py_##name)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {{"bind", py_bind, METH_VARARGS, nullptr}, {"launches", py_launches, METH_NOARGS, nullptr}, FAST(rmsnorm), FAST(gemm), FAST(linear), FAST(gemm_swiglu),
+                         FAST(mlp), FAST(attention), FAST(rope_attention), FAST(kv_append), FAST(paged_decode), {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "llmctl_ops", "Host side of the operators (csrc/torch/ops.cpp)", -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_llmctl_ops() { return PyModule_Create(&module); }

@@ -112,6 +112,10 @@ def _sdpa(q, k, v, causal, scale):
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = True,
               scale: Optional[float] = None) -> torch.Tensor:
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
+    if kernel_config().attention == "native":
+        o = native.fast.attention(q, k, v, scale, causal)
+        if o is not None:
+            return o
     if _native_ok(q, k, v, causal):
         return native.apply(_FlashAttnFn, q, k, v, scale, causal)
     if (_native_built(q) and _native_shape(q, k, v, causal) and k.dtype == v.dtype == q.dtype
@@ -238,6 +242,10 @@ def rope_attention_packed(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tenso
     from . import functional as ops
     scale = scale if scale is not None else 1.0 / math.sqrt(head_dim)
     cfg = kernel_config()
+    if cfg.elementwise == "native" and cfg.attention == "native":
+        o = native.fast.rope_attention(qkv, cos, sin, None if positions is None else positions.to(torch.int32), batch, seq, heads, head_dim, scale)
+        if o is not None:
+            return o
     if (qkv.is_cuda and qkv.dtype == torch.bfloat16 and cfg.elementwise == "native" and qkv.dim() == 2
             and qkv.stride(1) == 1 and not qkv.is_leaf and head_dim % 16 == 0):
         v5 = qkv.view(batch, seq, 3, heads, head_dim)

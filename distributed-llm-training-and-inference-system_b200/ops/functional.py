@@ -137,6 +137,10 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5,
             residual: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """Returns ``(y, h)`` with ``h = x + residual`` (``h is x`` when no residual) and
     ``y = h * rsqrt(mean(h^2) + eps) * w``."""
+    if _cfg.elementwise == "native":
+        r = native.fast.rmsnorm(x, residual, w, eps)
+        if r is not None:
+            return r
     if _use_native(x, "elementwise"):
         y, h = native.apply(_RMSNormFn, x, residual, w, eps)
         return (y, h) if residual is not None else (y, x)
@@ -312,6 +316,10 @@ def gemm_raw(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool
     ``a_mn=False``: a is [M,K]; ``a_mn=True``: a is [K,M].  ``b_mn=False``: b is [N,K]; else [K,N].
     ``b_gate`` (K8): ``b`` lives in a ZeRO-3 gather buffer that is still being filled; the kernel waits per tile for the
     arrival flags of the weight rows it loads (keys: flags, epoch, off, slab)."""
+    if b_gate is None:
+        r = native.fast.gemm(a, b, a_mn, b_mn, out, out_dtype == torch.float32, accumulate, tile_n or _cfg.gemm_tile_n, max_ctas)
+        if r is not None:
+            return r
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.is_cuda
     assert a.stride(1) == 1 and b.stride(1) == 1
     if a_mn:
@@ -419,6 +427,11 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
 def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """``x @ w.T`` (no bias).  x: [..., K], w: [N, K]."""
     gate = getattr(w, "_k8_gate", None)
+    if gate is None and _cfg.gemm == "native" and x.is_cuda:
+        ws = _skinny_workspace(x.device) if _cfg.skinny_gemm and x.numel() <= SKINNY_MAX_ROWS * x.shape[-1] else (None, None)
+        y = native.fast.linear(x, w, _cfg.gemm_tile_n, *ws)
+        if y is not None:
+            return y
     if gate is not None and not (_use_native(x, "gemm") and w.dtype == torch.bfloat16 and x.reshape(-1, x.shape[-1]).shape[0] > SKINNY_MAX_ROWS
                                  and w.shape[0] % 8 == 0):
         w._k8_gate = None          # not the gated GEMM path: wait for the whole unit first
@@ -455,6 +468,9 @@ def _wgrad(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor) -> Optional[torch
 
 
 def _gemm_swiglu(x: torch.Tensor, w: torch.Tensor, keep: bool) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
+    r = native.fast.gemm_swiglu(x, w, keep)
+    if r is not None:
+        return r
     M, K = x.shape
     Fd = w.shape[0] // 2
     act = torch.empty(M, Fd, dtype=x.dtype, device=x.device)
@@ -543,6 +559,11 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 def swiglu_mlp(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor) -> torch.Tensor:
     """``swiglu(x @ w_up.T) @ w_down.T``.  Where a gradient will be asked for and the width allows, the backward of the activation runs
     inside the product that precedes it; everything else composes ``linear_swiglu`` and ``linear``."""
+    if (_cfg.gemm == "native" and _cfg.elementwise == "native" and _cfg.gemm_tile_n == 0 and getattr(w_up, "_k8_gate", None) is None
+            and getattr(w_down, "_k8_gate", None) is None):
+        y = native.fast.mlp(x, w_up, w_down, SKINNY_MAX_ROWS)
+        if y is not None:
+            return y
     fused = w_down.shape[0] >= SWIGLU_BWD_COLS and torch.is_grad_enabled() and (x.requires_grad or w_up.requires_grad)
     x2 = _swiglu_rows(x, w_up) if fused else None
     if (x2 is None or w_down.dtype != torch.bfloat16 or getattr(w_down, "_k8_gate", None) is not None or w_down.shape[0] % 8

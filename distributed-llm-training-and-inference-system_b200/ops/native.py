@@ -10,6 +10,7 @@ Reference parity: the reference has no native layer.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import threading
 from pathlib import Path
 from typing import Optional
@@ -23,8 +24,39 @@ _LIB_PATH = _LIB_DIR / "libllmctl_b200.so"
 _lock = threading.Lock()
 _lib: Optional[ctypes.CDLL] = None
 
-#: number of native kernel launches issued through this module (bench.py reports it)
-launch_count = 0
+_OPS_PATH = _LIB_DIR / "llmctl_ops.so"
+_launches = 0
+
+
+class _NoOps:
+    """Stands in for the extension until the kernel library is loaded on a machine with a GPU: takes nothing."""
+
+    def __getattr__(self, name):
+        return _nothing
+
+    @staticmethod
+    def launches() -> int:
+        return 0
+
+
+def _nothing(*args):
+    return None
+
+
+#: the operators' host side (csrc/torch/ops.cpp): each function returns None for what it does not take
+fast = _NoOps()
+
+
+def __getattr__(name: str):
+    # launch_count: number of native kernel launches issued through this module and the extension (bench.py reports it)
+    if name == "launch_count":
+        return _launches + fast.launches()
+    raise AttributeError(name)
+
+
+def count_launches(n: int) -> None:
+    global _launches
+    _launches += n
 
 c_void_p, c_int, c_ll, c_float = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 
@@ -78,8 +110,21 @@ def lib() -> ctypes.CDLL:
                 continue
             fn.restype = _RESULTS.get(name, c_int)
             fn.argtypes = argtypes
+        if torch.cuda.is_available() and not _nvtx.KERNEL_RANGES:        # ranges around launches are made in `call`
+            _load_ops()
         _lib = l
     return _lib
+
+
+def _load_ops():
+    global fast
+    if not _OPS_PATH.exists():
+        raise RuntimeError(f"operator extension not found at {_OPS_PATH}; run `python build_native.py` (or __graft_entry__.build())")
+    spec = importlib.util.spec_from_file_location("llmctl_ops", _OPS_PATH)
+    ops = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(ops)
+    ops.bind(str(_LIB_PATH), NativeError, check_waits)
+    fast = ops
 
 
 def register_signature(name: str, argtypes: list, restype=c_int) -> None:
@@ -206,7 +251,7 @@ _KERNELS_PER_CALL = {"llmctl_rmsnorm_bwd": 2, "llmctl_layernorm_bwd": 3, "llmctl
 
 def call(name: str, *args) -> None:
     """Invoke a C entry point and raise on a non-zero status."""
-    global launch_count
+    global _launches
     if not _wait_bound:
         _bind_waits()
     if _wait_word.value:
@@ -217,6 +262,6 @@ def call(name: str, *args) -> None:
             rc = fn(*args)
     else:
         rc = fn(*args)
-    launch_count += _KERNELS_PER_CALL.get(name, 1)
+    _launches += _KERNELS_PER_CALL.get(name, 1)
     if rc != 0:
         raise NativeError(f"{name} failed with cudaError {rc}")

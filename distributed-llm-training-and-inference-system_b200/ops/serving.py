@@ -24,6 +24,8 @@ def kv_append(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, s
     slot_mapping: int64 [T] (negative = skip)."""
     hd = heads * head_dim
     if qkv.is_cuda:
+        if native.fast.kv_append(qkv, k_cache, v_cache, slot_mapping, heads, head_dim) is not None:
+            return
         native.call("llmctl_kv_append", qkv.data_ptr(), qkv.stride(0), hd, 2 * hd, k_cache.data_ptr(),
                     v_cache.data_ptr(), slot_mapping.data_ptr(), qkv.shape[0], heads, head_dim, native.stream_ptr())
         return
@@ -70,6 +72,10 @@ def paged_attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     if q.is_cuda:
         ns = num_splits or _launch_splits(B, H, D, max_context, block_size)
+        if scratch is None:
+            out = native.fast.paged_decode(q, k_cache, v_cache, block_tables, context_lens, max_context, ns, scale)
+            if out is not None:
+                return out
         need = native.lib().llmctl_paged_attn_scratch_elems(B, H, D, ns)
         if need and (scratch is None or scratch.numel() < need):
             scratch = torch.empty(need, dtype=torch.float32, device=q.device)
@@ -79,7 +85,7 @@ def paged_attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
                     out.stride(0), native.ptr(scratch), B, H, D, block_size, int(max_context), ns, float(scale),
                     native.stream_ptr())
         if need:
-            native.launch_count += 1        # the merge kernel
+            native.count_launches(1)        # the merge kernel
         return out
     out = torch.zeros(B, H, D, dtype=q.dtype)
     for b in range(B):

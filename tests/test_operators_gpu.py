@@ -1,0 +1,305 @@
+"""The operators' host side in C++ (csrc/torch/ops.cpp) against the Python operators that it stands in front of: the same kernels, so the
+same bits, launches, gradients and refusals over the layouts that either takes."""
+import contextlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def ops(cuda_device):
+    from llmctl_b200.ops import functional, native
+    native.lib()
+    assert not isinstance(native.fast, native._NoOps)
+    return functional
+
+
+@contextlib.contextmanager
+def python_operators():
+    from llmctl_b200.ops import native
+    # what the extension has counted so far stays in launch_count
+    fast, native.fast = native.fast, native._NoOps()
+    native.count_launches(fast.launches())
+    try:
+        yield
+    finally:
+        native.fast = fast
+        native.count_launches(-fast.launches())
+
+
+def _same(a, b):
+    if isinstance(a, (tuple, list)):
+        assert len(a) == len(b)
+        for x, y in zip(a, b):
+            _same(x, y)
+    else:
+        assert a.shape == b.shape and a.dtype == b.dtype and torch.equal(a, b)
+
+
+def _both(run):
+    """``run()`` (which makes its own inputs) on either side: outputs and launches."""
+    from llmctl_b200.ops import native
+    n = native.launch_count
+    got = run()
+    n = native.launch_count - n
+    with python_operators():
+        m = native.launch_count
+        want = run()
+        m = native.launch_count - m
+    _same(got, want)
+    assert n == m
+    return got
+
+
+def _randn(*shape, seed=0, shift=0):
+    """bf16 normals; ``shift``: elements past a 16-byte boundary."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    n = 1
+    for s in shape:
+        n *= s
+    return torch.randn(n + shift, device="cuda", generator=g).bfloat16()[shift:].view(*shape)
+
+
+@pytest.mark.parametrize("shape", [(1, 64), (37, 768), (2, 5, 2048), (64,)])
+@pytest.mark.parametrize("form", ["plain", "residual", "strided", "odd"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_rmsnorm(ops, shape, form, grad):
+    if form == "odd" and shape != (37, 768):
+        pytest.skip("one size is enough")
+
+    def run():
+        x = _randn(*shape, shift=8 if form == "odd" else 0)
+        if form == "strided":
+            x = torch.stack([x, x], -1)[..., 0]
+        r = _randn(*shape, seed=1) if form != "plain" else None
+        w = (1 + _randn(shape[-1], seed=2)).requires_grad_(grad)
+        leaves = [w]
+        for t in (x, r):
+            if t is not None and grad:
+                leaves.append(t.requires_grad_(True))
+        y, h = ops.rmsnorm(x, w, 1e-5, r)
+        assert r is not None or h is x
+        if not grad:
+            assert not y.requires_grad
+            return y, h
+        dy, dh = _randn(*shape, seed=3), _randn(*shape, seed=4)
+        outs, grads = ((y, h), (dy, dh)) if r is not None else ((y,), (dy,))
+        one = torch.autograd.grad(y, leaves, dy, retain_graph=True)        # the other output's gradient is missing
+        return (y.detach(), h.detach(), *one, *torch.autograd.grad(outs, leaves, grads))
+    _both(run)
+
+
+@pytest.mark.parametrize("shape,n", [((1, 64), 8), ((32, 256), 64), ((33, 256), 64), ((2, 50, 128), 24), ((300, 72), 40), ((2, 3, 64), 20)])
+@pytest.mark.parametrize("form", ["plain", "columns", "odd", "transposed"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_linear(ops, shape, n, form, grad):
+    def run():
+        K = shape[-1]
+        if form == "columns":
+            x = _randn(*shape[:-1], 2 * K)[..., K:]
+        elif form == "transposed":
+            x = _randn(K, *shape[:-1]).movedim(0, -1)
+        else:
+            x = _randn(*shape, shift=1 if form == "odd" else 0)
+        w = _randn(n, K, seed=1).requires_grad_(grad)
+        x = x.detach().requires_grad_(grad)
+        y = ops.linear(x, w)
+        if not grad:
+            return y
+        return (y.detach(), *torch.autograd.grad(y, (x, w), _randn(*y.shape, seed=2)))
+    _both(run)
+
+
+@pytest.mark.parametrize("rows,width,ffn", [(1, 64, 64), (32, 128, 64), (33, 128, 64), (200, 1024, 256), (130, 256, 96)])
+@pytest.mark.parametrize("grad", [False, True])
+def test_mlp(ops, rows, width, ffn, grad):
+    def run():
+        x, up, down = _randn(rows, width), _randn(2 * ffn, width, seed=1), _randn(width, ffn, seed=2)
+        leaves = [t.requires_grad_(grad) for t in (x, up, down)]
+        y = ops.swiglu_mlp(*leaves)
+        return (y.detach(), *torch.autograd.grad(y, leaves, _randn(rows, width, seed=3))) if grad else y
+    _both(run)
+
+
+@pytest.mark.parametrize("B,S,H,D", [(1, 1, 1, 64), (2, 128, 3, 128), (2, 77, 2, 64), (1, 300, 2, 128)])
+@pytest.mark.parametrize("form", ["packed", "apart", "odd", "heads first", "fp32"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_attention(ops, B, S, H, D, form, grad):
+    if form in ("fp32", "heads first") and grad:
+        pytest.skip("the library's, whose gradients differ from run to run")
+    def run():
+        if form == "packed":
+            q, k, v = _randn(B, S, 3, H, D).unbind(2)
+        elif form == "heads first":
+            q, k, v = (_randn(B, H, S, D, seed=i).transpose(1, 2) for i in range(3))
+        else:
+            q, k, v = (_randn(B, S, H, D, seed=i, shift=1 if form == "odd" and i == 1 else 0) for i in range(3))
+        if form == "fp32":
+            q, k, v = q.float(), k.float(), v.float()
+        leaves = [t.detach().requires_grad_(grad) for t in (q, k, v)]
+        o = ops.attention(*leaves, causal=True)
+        return (o.detach(), *torch.autograd.grad(o, leaves, _randn(B, S, H, D, seed=5).to(o.dtype))) if grad else o
+    _both(run)
+
+
+@pytest.mark.parametrize("B,S,H,D", [(1, 1, 1, 64), (2, 128, 3, 128), (2, 77, 2, 64)])
+@pytest.mark.parametrize("form", ["plain", "positions", "odd", "leaf"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_rope_attention(ops, B, S, H, D, form, grad):
+    from llmctl_b200.ops.attention import rope_attention_packed
+    cos, sin = ops.rope_tables(D, 2 * S, device="cuda")
+
+    def run():
+        leaf = _randn(B * S, 3 * H * D, shift=1 if form == "odd" else 0).requires_grad_(grad)
+        x = leaf if form == "leaf" else torch.empty(B * S * 3 * H * D + 8, dtype=torch.bfloat16, device="cuda")[(1 if form == "odd" else 0):][:leaf.numel()].view_as(leaf).copy_(leaf)
+        p = torch.randperm(2 * S, generator=torch.Generator().manual_seed(1))[:S].repeat(B).cuda() if form == "positions" else None
+        before = x._version
+        o = rope_attention_packed(x, cos, sin, B, S, H, D, positions=p)
+        if grad:
+            return (o.detach(), *torch.autograd.grad(o, leaf, _randn(B * S, H * D, seed=5)))
+        assert (x._version > before) == (form != "odd")                    # rotated in place, and autograd is told; a copy where it cannot be
+        return o, x
+    _both(run)
+
+
+@pytest.mark.parametrize("B,H,D,context", [(1, 12, 64, 300), (3, 4, 128, 70), (16, 8, 128, 900)])
+def test_paged_decode(ops, B, H, D, context):
+    from llmctl_b200.ops import serving
+
+    def run():
+        pages = (context + 15) // 16
+        k, v = _randn(B * pages, 16, H, D, seed=1), _randn(B * pages, 16, H, D, seed=2)
+        tables = torch.randperm(B * pages, generator=torch.Generator().manual_seed(3)).view(B, pages).int().cuda()
+        lens = torch.tensor([max(1, context - 13 * i) for i in range(B)], dtype=torch.int32, device="cuda")
+        at = lens.long() - 1
+        slots = tables.gather(1, (at // 16)[:, None])[:, 0].long() * 16 + at % 16
+        slots[B // 2] = -1 if B > 1 else slots[B // 2]
+        qkv = _randn(B, 3 * H * D)
+        serving.kv_append(qkv, k, v, slots, H, D)
+        return serving.paged_attention_decode(qkv[:, :H * D].reshape(B, H, D), k, v, tables, lens, context), k, v
+    _both(run)
+
+
+def test_saved_tensor_hooks_see_what_is_kept(ops):
+    """Offloading and checkpointing pack what a backward will need and unpack it there."""
+    packed, unpacked = [], []
+
+    def pack(t):
+        packed.append(t)
+        return len(packed) - 1
+
+    def unpack(i):
+        unpacked.append(i)
+        return packed[i]
+    q, k, v = (_randn(1, 130, 2, 64, seed=i).requires_grad_(True) for i in range(3))
+    w = (1 + _randn(64, seed=4)).requires_grad_(True)
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        y, _ = ops.rmsnorm(ops.attention(q, k, v), w)
+    assert len(packed) >= 8
+    y.sum().backward()
+    assert sorted(unpacked) == list(range(len(packed))) and q.grad.abs().sum() > 0
+
+
+def test_transforms_modes_and_subclasses_go_to_the_python_operators(ops):
+    """What wants to see the operators or replace their tensors finds the Python ones, which record or refuse it as before."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from llmctl_b200.ops import native
+    x, w = _randn(40, 64), _randn(64, seed=1)
+
+    class Mine(torch.Tensor):
+        pass
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+    assert native.fast.rmsnorm(x, None, w, 1e-5) is not None
+    assert native.fast.rmsnorm(x.as_subclass(Mine), None, w, 1e-5) is None
+    assert native.fast.rmsnorm(torch.nn.Parameter(x), None, w, 1e-5) is not None
+    with Mode():
+        assert native.fast.rmsnorm(x, None, w, 1e-5) is None
+    with torch.device("cuda"):
+        assert native.fast.rmsnorm(x, None, w, 1e-5) is None
+    seen = []
+    torch.func.grad(lambda t: (seen.append(native.fast.rmsnorm(t, None, w, 1e-5)), t.float().sum())[1])(x)
+    torch.vmap(lambda t: (seen.append(native.fast.rmsnorm(t, None, w, 1e-5)), t)[1])(x)
+    torch.vmap(lambda t: (seen.append(native.fast.rmsnorm(x, None, w, 1e-5)), t)[1])(x)
+    with torch.autograd.forward_ad.dual_level():
+        seen.append(native.fast.rmsnorm(torch.autograd.forward_ad.make_dual(x, x), None, w, 1e-5))
+    assert seen == [None] * 4
+    with torch.inference_mode():
+        y, _ = ops.rmsnorm(x, w)
+        assert y.is_inference()
+    for bad in (x.float(), x.cpu(), x.half(), x.t(), x[:, :32], 3, None):
+        assert native.fast.rmsnorm(bad, None, w, 1e-5) is None
+
+
+def test_errors_are_the_python_operators_errors(ops):
+    """A call that the kernel library refuses raises NativeError from the forward; a wait that ran out is raised before the next launch, in a
+    forward and in a backward."""
+    from llmctl_b200.ops import native
+    x = _randn(40, 12).requires_grad_(True)                                # 12 columns: not whole 16-byte units
+    for grad in (False, True):
+        with torch.set_grad_enabled(grad), pytest.raises(native.NativeError):
+            ops.rmsnorm(x, _randn(12, seed=1))
+    x, w = _randn(40, 64).requires_grad_(True), _randn(64, seed=1)
+    y, _ = ops.rmsnorm(x, w)
+    native.register_signature("llmctl_wait_status_report", [native.c_int, native.c_void_p])
+
+    def run_out():
+        assert native.lib().llmctl_wait_status_report(0, native.stream_ptr()) == 0
+        torch.cuda.synchronize()
+    run_out()
+    with pytest.raises(native.NativeError, match="flash attention forward"):
+        ops.rmsnorm(x, w)
+    run_out()
+    with pytest.raises(native.NativeError, match="flash attention forward"):
+        torch.autograd.grad(y, x, torch.ones_like(y), retain_graph=True)
+    torch.autograd.grad(y, x, torch.ones_like(y))
+
+
+def test_layers_run_on_several_threads_and_streams(ops):
+    """Forward and backward of a few operators on four threads, each on its own stream, against one thread's."""
+    import threading
+    def run(seed):
+        x, w = _randn(300, 128, seed=seed).requires_grad_(True), _randn(384, 128, seed=1)
+        y, _ = ops.rmsnorm(x, _randn(128, seed=2))
+        o = ops.attention(*ops.linear(y, w).view(1, 300, 3, 2, 64).unbind(2))
+        return o.detach(), torch.autograd.grad(o, x, _randn(*o.shape, seed=3))[0]
+    want = [run(i) for i in range(4)]
+    torch.cuda.synchronize()
+    got = [None] * 4
+
+    def work(i):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            for _ in range(20):
+                got[i] = run(i)
+            s.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    _same(got, want)
+
+
+def test_capture(ops):
+    """A captured layer replays with new inputs."""
+    x, w = _randn(64, 128), _randn(384, 128, seed=1)
+    n = 1 + _randn(128, seed=2)
+    cos, sin = ops.rope_tables(64, 64, device="cuda")
+    from llmctl_b200.ops.attention import rope_attention_packed
+
+    def layer(t):
+        with torch.no_grad():
+            return rope_attention_packed(ops.linear(ops.rmsnorm(t, n)[0], w), cos, sin, 1, 64, 2, 64)
+    layer(x)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = layer(x)
+    x.copy_(_randn(64, 128, seed=9))
+    g.replay()
+    assert torch.equal(out, layer(x))
