@@ -39,6 +39,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
+#include "../common/dependent.cuh"
 #include "../common/wait_status.h"
 #include "flash_bwd_slots.cuh"
 
@@ -89,6 +90,8 @@ __global__ void __launch_bounds__(256)
 flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO, long long tok_stride,
                       const float* __restrict__ lse, float* __restrict__ nl2, float* __restrict__ ndl, int S, int Sp, int H,
                       int chunks, int* __restrict__ counter) {
+  wait_for_previous(O, dO, lse, nl2, ndl, counter);
+  release_dependents();
   if (blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;       // the item counter of the kernel that follows
   constexpr int kLanes = D / 8, kGroups = 256 / kLanes, kRows = 4;
   const int g = threadIdx.x / kLanes, li = threadIdx.x % kLanes;
@@ -191,6 +194,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bar.tmem;
+  wait_for_previous();                 // what is read comes by bulk copies and an atomic
   // A waiter of an mbarrier sees only the parity of its phase, so no barrier may complete its next phase before everyone has passed the
   // wait for this one.  acc[a] (product finished) is therefore committed only after accfree[a] (read out) of the use before has been
   // waited for.  acc[0] is used by dKV items alone, acc[1] by every item, each side counting them.
@@ -275,6 +279,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
         if (!ok) break;
         sl.next(it.n);
       }
+      release_dependents();
       // Copies still in flight when a wait ran out land before the CTA's shared memory is given back.
       if (!ok) {
         int none = 0;
@@ -597,8 +602,9 @@ static int flash_bwd_launch(const void* q, const void* k, const void* v, const v
   const int group = static_cast<int>(fit < 1 ? 1 : fit < B * H ? fit : B * H);
   constexpr int kPrepRows = 256 / (D / 8) * 4;
   const int chunks = (Sp + kPrepRows - 1) / kPrepRows;
-  flash_bwd_prep_kernel<D><<<chunks * B * H, 256, 0, s>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, o_tok, lse, nl2, ndl, S, Sp,
-                                                          H, chunks, counter);
+  cudaError_t e = launch_dependent(flash_bwd_prep_kernel<D>, chunks * B * H, 256, 0, s, (const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, o_tok, lse, nl2,
+                                   ndl, S, Sp, H, chunks, counter);
+  if (e != cudaSuccess) return static_cast<int>(e);
   int rc = 0;
   auto mkmap = [&](CUtensorMap* m, const void* base, long long tok, int heads) {
     if (!rc) rc = get_tmap_4d_bf16(m, base, D, heads, S, B, D, tok, static_cast<uint64_t>(S) * tok, 64, 1, kBlk, 1, 1);
@@ -623,11 +629,11 @@ static int flash_bwd_launch(const void* q, const void* k, const void* v, const v
   if (rc) return rc;
   unsigned char* const wait_byte = wait_report(kWaitFlashBackward);
   if (wait_byte == nullptr) return static_cast<int>(cudaErrorMemoryAllocation);
-  const cudaError_t e = allow_smem(flash_bwd_kernel<D>, C::kSmem);
+  e = allow_smem(flash_bwd_kernel<D>, C::kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int n_items = 2 * nblk * B * H, grid = n_items < kNumSMs ? n_items : kNumSMs;
-  flash_bwd_kernel<D><<<grid, kThreads, C::kSmem, s>>>(maps, nl2, ndl, in_step, out_step, B, S, H, group, counter, scale * 1.4426950408889634f, scale, causal, wait_byte);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_dependent(flash_bwd_kernel<D>, grid, kThreads, C::kSmem, s, maps, nl2, ndl, in_step, out_step, B, S, H, group, counter,
+                                           scale * 1.4426950408889634f, scale, causal, wait_byte));
 }
 
 }  // namespace llmctl

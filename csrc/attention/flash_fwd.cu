@@ -9,6 +9,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
+#include "../common/dependent.cuh"
 #include "../common/wait_status.h"
 
 namespace llmctl {
@@ -212,6 +213,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
+  if constexpr (DQK > 128)
+    wait_for_previous(seqs);
+  else
+    wait_for_previous();               // the outputs are stored to, not read
   volatile int* abort = &abort_flag;
 
   // optional event log of CTA 0 (LLMCTL_FLASH_TRACE): per role 127 x (code, clock) pairs after a count word.
@@ -305,6 +310,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           for (int p = 0; p < DV / 64; ++p) tma_load_4d(sV + p * kPanel, &tmV, &bar_vfull[vs], 64 * p, head + 2 * head_step, row, bc);
         }
       }
+      release_dependents();
       // Copies still in flight when a wait ran out land before the CTA's shared memory is given back.
       if (*abort) {
         int none = 0;
@@ -515,9 +521,8 @@ static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CU
   unsigned char* const wait_byte = wait_report(kWaitFlashForward);
   if (wait_byte == nullptr) return static_cast<int>(cudaErrorMemoryAllocation);
   const int wide = o_tok_stride % 16 == 0 && (reinterpret_cast<uintptr_t>(o) & 31) == 0;
-  flash_fwd_kernel<DQK, DV><<<grid, kThreads, C::kSmem, s>>>(q, k, ks, v, (__nv_bfloat16*)o, o_tok_stride, wide, lse, seqs, B, max_q, H,
-                                                             head_step, scale * 1.4426950408889634f, causal, wait_byte, flash_trace_buffer());
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_dependent(flash_fwd_kernel<DQK, DV>, grid, kThreads, C::kSmem, s, q, k, ks, v, (__nv_bfloat16*)o, o_tok_stride, wide, lse, seqs,
+                                           B, max_q, H, head_step, scale * 1.4426950408889634f, causal, wait_byte, flash_trace_buffer()));
 }
 
 }  // namespace llmctl

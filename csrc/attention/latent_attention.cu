@@ -26,6 +26,7 @@
 //                             products on the tensor cores (mma.sync m16n8k16, fp32 accumulation; softmax, masks
 //                             and the running maximum / sum stay fp32); other sizes and fp32 run the FMA kernel.
 // Reference: none (the reference re-runs the HF model over the whole sequence, reference llmctl/serve/server.py:199-204).
+#include "../common/dependent.cuh"
 #include "../common/dtype.cuh"
 #include "../common/mma_sync.cuh"
 #include "../rope/rope_interleaved.cuh"
@@ -79,6 +80,8 @@ latent_kv_write_vec_kernel(const __nv_bfloat16* __restrict__ d, long long ld, in
                            const __nv_bfloat16* __restrict__ wkv, __nv_bfloat16* __restrict__ cq, __nv_bfloat16* __restrict__ cache,
                            const long long* __restrict__ slots, const int* __restrict__ positions, const float* __restrict__ freq,
                            float mult, float eps, int tokens) {
+  wait_for_previous(d, wq, wkv, cq, cache, slots, positions, freq);
+  release_dependents();
   const int lane = threadIdx.x & 31;
   const long long tok = blockIdx.x * 4ll + (threadIdx.x >> 5);
   if (tok >= tokens) return;
@@ -291,6 +294,8 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 latent_attention_merge_kernel(const float* __restrict__ partial, T* __restrict__ out, int R, int nsplit, int H,
                               const T* __restrict__ head_gate, long long gate_ld) {
+  wait_for_previous(partial, out, head_gate);
+  release_dependents();
   const long long base = blockIdx.x;   // token * H + head
   const float* p = partial + base * nsplit * (R + 2);
   extern __shared__ float wsplit[];    // [nsplit]: exp(m_s - max m) / sum, 0 for empty splits
@@ -381,6 +386,8 @@ latent_attention_tc_kernel(const TQ* __restrict__ ql, long long ql_st, long long
                            const float* __restrict__ sinks, int window, const __nv_bfloat16* __restrict__ head_gate, long long gate_ld) {
   constexpr int kR = 16 * MT, kWarps = 8 * MT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  wait_for_previous(ql, q, cache, block_tables, tiles, positions, freq, out, partial, sinks, head_gate);
+  release_dependents();
   const int D = R + dr, Dp = D + 8;
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_raw);      // [kR][Dp]
   __nv_bfloat16* Ks0 = Qs + kR * Dp;                                    // [stages][kTcKeys][Dp]
@@ -608,10 +615,11 @@ static int launch_latent_attention_tc(const TQ* ql, long long ql_st, long long q
     auto kern = latent_attention_tc_kernel<NT, MT, TQ>;                                                              \
     cudaError_t e = allow_smem(kern, static_cast<int>(smem)); \
     if (e != cudaSuccess) return static_cast<int>(e);                                                                \
-    kern<<<grid, 256 * MT, smem, s>>>(ql, ql_st, ql_sh, (const __nv_bfloat16*)q, ldq, dn, (const __nv_bfloat16*)cache, \
-                                      block_tables, max_blocks, block_size, tiles, positions, freq, mult, scale,     \
-                                      H, R, dr, heads_per_tile, keys_per_split, stages, (__nv_bfloat16*)out, partial, sinks, window, \
-                                      (const __nv_bfloat16*)head_gate, gate_ld); \
+    e = launch_dependent(kern, grid, 256 * MT, smem, s, ql, ql_st, ql_sh, (const __nv_bfloat16*)q, ldq, dn, (const __nv_bfloat16*)cache, \
+                         block_tables, max_blocks, block_size, tiles, positions, freq, mult, scale,                  \
+                         H, R, dr, heads_per_tile, keys_per_split, stages, (__nv_bfloat16*)out, partial, sinks, window, \
+                         (const __nv_bfloat16*)head_gate, gate_ld);                                                  \
+    if (e != cudaSuccess) return static_cast<int>(e);                                                                \
   } while (0)
 #define LAUNCH_TC_NT(MT)          \
   do {                            \
@@ -625,8 +633,8 @@ static int launch_latent_attention_tc(const TQ* ql, long long ql_st, long long q
 #undef LAUNCH_TC_NT
 #undef LAUNCH_TC
   if (splits > 1)
-    latent_attention_merge_kernel<__nv_bfloat16><<<tokens * H, 128, splits * sizeof(float), s>>>(partial, (__nv_bfloat16*)out, R, splits, H,
-                                                                                                 (const __nv_bfloat16*)head_gate, gate_ld);
+    return static_cast<int>(launch_dependent(latent_attention_merge_kernel<__nv_bfloat16>, tokens * H, 128, splits * sizeof(float), s, partial, (__nv_bfloat16*)out, R,
+                                             splits, H, (const __nv_bfloat16*)head_gate, gate_ld));
   return 0;
 }
 
@@ -643,9 +651,9 @@ LLMCTL_API int llmctl_latent_kv_write(const void* d, long long ld, int Q, int R,
   const uintptr_t at = reinterpret_cast<uintptr_t>(d) | reinterpret_cast<uintptr_t>(wq) | reinterpret_cast<uintptr_t>(wkv) |
                        reinterpret_cast<uintptr_t>(cq) | reinterpret_cast<uintptr_t>(cache);
   if (!is_fp32 && Q % 8 == 0 && R % 8 == 0 && dr % 8 == 0 && ld % 8 == 0 && (at & 15) == 0 && Q <= 256 * kWriteUnits && R <= 256 * kWriteUnits) {
-    latent_kv_write_vec_kernel<<<(tokens + 3) / 4, 128, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)d, ld, Q, R, dr, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wkv, (__nv_bfloat16*)cq, (__nv_bfloat16*)cache,
-        slots, positions, freq, mult, eps, tokens);
+    LLMCTL_CHECK(launch_dependent(latent_kv_write_vec_kernel, (tokens + 3) / 4, 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d, ld, Q, R, dr,
+                                  (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wkv, (__nv_bfloat16*)cq, (__nv_bfloat16*)cache, slots, positions, freq, mult, eps,
+                                  tokens));
     LLMCTL_RETURN_LAST();
   }
   LLMCTL_DISPATCH_DTYPE(is_fp32, T, (latent_kv_write_kernel<T><<<tokens, 128, 0, (cudaStream_t)stream>>>(

@@ -12,6 +12,7 @@
 // Reference: none (the reference has no model code).
 #include "../common/dtype.cuh"
 #include "../common/util.cuh"
+#include "../common/dependent.cuh"
 #include "../rope/rope_interleaved.cuh"
 
 namespace llmctl {
@@ -24,6 +25,8 @@ latent_prompt_prepare_kernel(__nv_bfloat16* __restrict__ q, long long ldq, int t
                              const __nv_bfloat16* __restrict__ cache, int R, const int* __restrict__ block_tables, int max_blocks,
                              int block_size, const int4* __restrict__ seqs, int B, int key_rows, __nv_bfloat16* __restrict__ c_out,
                              __nv_bfloat16* __restrict__ kr_out) {
+  wait_for_previous(q, positions, freq, cache, block_tables, seqs, c_out, kr_out);
+  release_dependents();
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * kPrepWarps + (threadIdx.x >> 5);
   if (w < tokens) {
@@ -86,8 +89,8 @@ LLMCTL_API int llmctl_latent_prompt_prepare(void* q, long long ldq, int tokens, 
   const long long warps = static_cast<long long>(tokens) + key_rows;
   if (warps == 0) return 0;
   LLMCTL_REQUIRE(warps < (1ll << 31));
-  latent_prompt_prepare_kernel<<<static_cast<unsigned>((warps + kPrepWarps - 1) / kPrepWarps), 32 * kPrepWarps, 0, (cudaStream_t)stream>>>(
-      (__nv_bfloat16*)q, ldq, tokens, H, dn, dr, positions, freq, mult, (const __nv_bfloat16*)cache, R, block_tables, max_blocks, block_size,
-      reinterpret_cast<const int4*>(seqs), B, key_rows, (__nv_bfloat16*)c_out, (__nv_bfloat16*)kr_out);
+  LLMCTL_CHECK(launch_dependent(latent_prompt_prepare_kernel, static_cast<unsigned>((warps + kPrepWarps - 1) / kPrepWarps), 32 * kPrepWarps, 0, (cudaStream_t)stream,
+                                (__nv_bfloat16*)q, ldq, tokens, H, dn, dr, positions, freq, mult, (const __nv_bfloat16*)cache, R, block_tables, max_blocks, block_size,
+                                reinterpret_cast<const int4*>(seqs), B, key_rows, (__nv_bfloat16*)c_out, (__nv_bfloat16*)kr_out));
   LLMCTL_RETURN_LAST();
 }

@@ -24,6 +24,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
+#include "../common/dependent.cuh"
 
 namespace llmctl {
 using namespace ptx;
@@ -81,6 +82,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
+  wait_for_previous(C, workspace, counters);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -103,6 +105,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           ++tile;
         }
       }
+      release_dependents();
     }
   } else if (warp == 1) {
     // the whole warp walks the loop, one elected lane issues (descriptors stay in uniform registers, see gemm_tcgen05.cu)
@@ -272,12 +275,12 @@ LLMCTL_API int llmctl_gemm_skinny_bf16(const void* X, const void* W, void* C, in
   cudaStream_t s = (cudaStream_t)stream;
   if (MB == 16) {
     LLMCTL_CHECK(allow_smem(gemm_skinny_kernel<16>, skinny::Cfg<16>::kSmem));
-    gemm_skinny_kernel<16><<<grid, skinny::kThreads, skinny::Cfg<16>::kSmem, s>>>(
-        tw, tx, (__nv_bfloat16*)C, ldc, Mb, N, num_kb, n_tiles, static_cast<int>(L), max_slots, workspace, counters);
+    LLMCTL_CHECK(launch_dependent(gemm_skinny_kernel<16>, grid, skinny::kThreads, skinny::Cfg<16>::kSmem, s, tw, tx, (__nv_bfloat16*)C, ldc, Mb, N,
+                                  num_kb, n_tiles, static_cast<int>(L), max_slots, workspace, counters));
   } else {
     LLMCTL_CHECK(allow_smem(gemm_skinny_kernel<32>, skinny::Cfg<32>::kSmem));
-    gemm_skinny_kernel<32><<<grid, skinny::kThreads, skinny::Cfg<32>::kSmem, s>>>(
-        tw, tx, (__nv_bfloat16*)C, ldc, Mb, N, num_kb, n_tiles, static_cast<int>(L), max_slots, workspace, counters);
+    LLMCTL_CHECK(launch_dependent(gemm_skinny_kernel<32>, grid, skinny::kThreads, skinny::Cfg<32>::kSmem, s, tw, tx, (__nv_bfloat16*)C, ldc, Mb, N,
+                                  num_kb, n_tiles, static_cast<int>(L), max_slots, workspace, counters));
   }
   LLMCTL_RETURN_LAST();
 }

@@ -18,6 +18,7 @@
 // (reference llmctl/cli/commands/hw.py:317-337, llmctl/plugins/autotuning.py:89-114).
 // Baseline to beat: cuBLASLt bf16 (MEASURED_PEAKS.json).
 #include "../comm/symm.cuh"
+#include "../common/dependent.cuh"
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
 
@@ -50,6 +51,7 @@ struct GemmGate {
   const int* grp_tile_expert;
   const int* grp_num_tiles;
   int grp_experts;
+  __host__ __device__ bool waits() const { return flags != nullptr || b_flags != nullptr; }
 };
 // Row of B where the tile's N range starts, or -1 if this tile-row block holds no rows (grouped mode only).
 __device__ __forceinline__ int grouped_b_row(const GemmGate& g, int m_blk, int n0, int N) {
@@ -376,6 +378,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
+  wait_for_previous(C);
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -421,6 +424,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           }
         }
       }
+      if (!gate.waits()) release_dependents();       // the last loads are on their way
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
@@ -580,6 +584,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
+  wait_for_previous(C);
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
@@ -622,6 +627,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           }
         }
       }
+      if (!gate.waits()) release_dependents();       // the last loads are on their way
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) ------------------------------
@@ -711,6 +717,15 @@ static int num_sms() {
   return g_num_sms;
 }
 
+// A GEMM that waits for flags of other streams' kernels is launched, and lets others be launched, the ordinary way (dependent.cuh, rule 3).
+template <typename Kernel, typename OutT>
+static cudaError_t launch_gemm_kernel(Kernel kern, int grid, int smem, cudaStream_t s, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, OutT* C,
+                                      long long ldc, int M, int N, int K, int beta, const GemmGate& gate, const SwigluMaps& sw) {
+  if (!gate.waits()) return launch_dependent(kern, grid, kGemmThreads, smem, s, tmA, tmB, tmC, C, ldc, M, N, K, beta, gate, sw);
+  kern<<<grid, kGemmThreads, smem, s>>>(tmA, tmB, tmC, C, ldc, M, N, K, beta, gate, sw);
+  return cudaGetLastError();
+}
+
 template <int BN, bool A_MN, bool B_MN, typename OutT>
 static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                        long long ldb, long long ldc, int beta, int max_ctas, cudaStream_t s, GemmGate gate) {
@@ -737,7 +752,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   int grid = num_sms();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (tiles < grid) grid = tiles;
-  kern<<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate, SwigluMaps{});
+  LLMCTL_CHECK(launch_gemm_kernel(kern, grid, Cfg::kSmemBytes, s, tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate, SwigluMaps{}));
   LLMCTL_RETURN_LAST();
 }
 
@@ -780,7 +795,7 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
   if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
   if (pairs < 1) pairs = 1;
   if (tiles < pairs) pairs = tiles;
-  kern<<<2 * pairs, kGemmThreads, Cfg::kSmemBytes, s>>>(tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate, SwigluMaps{});
+  LLMCTL_CHECK(launch_gemm_kernel(kern, 2 * pairs, Cfg::kSmemBytes, s, tmA, tmB, tmC, (OutT*)C, ldc, M, N, K, beta, gate, SwigluMaps{}));
   LLMCTL_RETURN_LAST();
 }
 
@@ -815,12 +830,12 @@ static int launch_swiglu(const void* X, const void* W, void* GU, void* ACT, int 
     auto kern = gemm2_tcgen05_kernel<256, false, false, __nv_bfloat16, Gated::kForward>;
     LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256, Gated::kForward>::kSmemBytes));
     const int pairs = tiles < num_sms() / 2 ? tiles : num_sms() / 2;
-    kern<<<2 * pairs, kGemmThreads, Gemm2Cfg<256, Gated::kForward>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0, GemmGate{}, sw);
+    LLMCTL_CHECK(launch_gemm_kernel(kern, 2 * pairs, Gemm2Cfg<256, Gated::kForward>::kSmemBytes, s, tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0, GemmGate{}, sw));
   } else {
     auto kern = gemm_tcgen05_kernel<128, false, false, __nv_bfloat16, Gated::kForward>;
     LLMCTL_CHECK(allow_smem(kern, GemmCfg<128, Gated::kForward>::kSmemBytes));
-    kern<<<tiles < num_sms() ? tiles : num_sms(), kGemmThreads, GemmCfg<128, Gated::kForward>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact, M, F, K, 0,
-                                                                                            GemmGate{}, sw);
+    LLMCTL_CHECK(launch_gemm_kernel(kern, tiles < num_sms() ? tiles : num_sms(), GemmCfg<128, Gated::kForward>::kSmemBytes, s, tmA, tmW, tmA, (__nv_bfloat16*)ACT, ldact,
+                                    M, F, K, 0, GemmGate{}, sw));
   }
   LLMCTL_RETURN_LAST();
 }
@@ -847,11 +862,11 @@ static int launch_swiglu_bwd(const void* DY, const void* W, const void* GU, void
   if constexpr (kPair) {
     auto kern = gemm2_tcgen05_kernel<256, false, true, __nv_bfloat16, Gated::kBackward>;
     LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256, Gated::kBackward>::kSmemBytes));
-    kern<<<2 * grid, kGemmThreads, Gemm2Cfg<256, Gated::kBackward>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw);
+    LLMCTL_CHECK(launch_gemm_kernel(kern, 2 * grid, Gemm2Cfg<256, Gated::kBackward>::kSmemBytes, s, tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw));
   } else {
     auto kern = gemm_tcgen05_kernel<kBN, false, true, __nv_bfloat16, Gated::kBackward>;
     LLMCTL_CHECK(allow_smem(kern, GemmCfg<kBN, Gated::kBackward>::kSmemBytes));
-    kern<<<grid, kGemmThreads, GemmCfg<kBN, Gated::kBackward>::kSmemBytes, s>>>(tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw);
+    LLMCTL_CHECK(launch_gemm_kernel(kern, grid, GemmCfg<kBN, Gated::kBackward>::kSmemBytes, s, tmA, tmW, tmA, (__nv_bfloat16*)DGU, ldgu, M, F, K, 0, GemmGate{}, sw));
   }
   LLMCTL_RETURN_LAST();
 }

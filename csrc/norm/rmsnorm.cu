@@ -8,6 +8,7 @@
 //           HBM.  h = x (+ residual) ; y = h * rsqrt(mean(h^2)+eps) * w.
 // Backward: persistent CTAs loop over rows; dw/db partial sums stay in registers and are flushed once
 //           per CTA into a scratch [grid, cols] fp32 buffer which a second kernel column-reduces.
+#include "../common/dependent.cuh"
 #include "../common/util.cuh"
 
 namespace llmctl {
@@ -19,6 +20,8 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 __nv_bfloat16* __restrict__ h_out, __nv_bfloat16* __restrict__ y,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols,
                 float eps) {
+  wait_for_previous(x, residual, w, b, h_out, y, mean_out, rstd_out);
+  release_dependents();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -122,6 +125,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                 __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial,
                 float* __restrict__ db_partial, int rows, int cols) {
+  wait_for_previous(dy, h, w, mean_in, rstd_in, dres, dx, dw_partial, db_partial);
+  release_dependents();
   __shared__ float red[32];
   const int nvec = cols >> 3;
   float wreg[kVec][8];
@@ -239,6 +244,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
 // Column-reduce the [nparts, cols] fp32 partials; writes (or accumulates into) an fp32 gradient.
 __global__ void colsum_kernel(const float* __restrict__ partial, float* __restrict__ out, int nparts,
                               int cols, int accumulate) {
+  wait_for_previous(partial, out);
+  release_dependents();
   // blockDim = (32, 8): 32 consecutive columns x 8 row-slices
   __shared__ float tile[8][33];
   const int col = blockIdx.x * 32 + threadIdx.x;
@@ -265,10 +272,10 @@ static int launch_fwd(const void* x, const void* residual, const void* w, const 
   const int per_lane = (nvec + 31) / 32;
   dim3 block(128), grid((rows + 3) / 4);
 #define LAUNCH(MV)                                                                              \
-  norm_fwd_kernel<MV, kLN><<<grid, block, 0, s>>>(                                             \
+  LLMCTL_CHECK(launch_dependent(norm_fwd_kernel<MV, kLN>, grid, block, 0, s,                   \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)w,        \
       (const __nv_bfloat16*)b, (__nv_bfloat16*)h_out, (__nv_bfloat16*)y, mean, rstd, rows, cols, \
-      eps)
+      eps))
   if (per_lane <= 4) LAUNCH(4);
   else if (per_lane <= 8) LAUNCH(8);
   else if (per_lane <= 16) LAUNCH(16);
@@ -291,17 +298,17 @@ static int launch_bwd(const void* dy, const void* h, const void* w, const float*
   float* dwp = scratch;
   float* dbp = kLN ? scratch + static_cast<size_t>(scratch_rows) * cols : nullptr;
 #define LAUNCH(KV)                                                                            \
-  norm_bwd_kernel<KV, kLN><<<grid, 256, 0, s>>>(                                               \
+  LLMCTL_CHECK(launch_dependent(norm_bwd_kernel<KV, kLN>, grid, 256, 0, s,                     \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, mean, rstd, \
-      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dwp, dbp, rows, cols)
+      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dwp, dbp, rows, cols))
   if (kv <= 1) LAUNCH(1);
   else if (kv <= 2) LAUNCH(2);
   else if (kv <= 3) LAUNCH(3);
   else LAUNCH(4);
 #undef LAUNCH
   dim3 b2(32, 8), g2((cols + 31) / 32);
-  colsum_kernel<<<g2, b2, 0, s>>>(dwp, dw, grid, cols, accumulate);
-  if (kLN && db != nullptr) colsum_kernel<<<g2, b2, 0, s>>>(dbp, db, grid, cols, accumulate);
+  LLMCTL_CHECK(launch_dependent(colsum_kernel, g2, b2, 0, s, dwp, dw, grid, cols, accumulate));
+  if (kLN && db != nullptr) LLMCTL_CHECK(launch_dependent(colsum_kernel, g2, b2, 0, s, dbp, db, grid, cols, accumulate));
   LLMCTL_RETURN_LAST();
 }
 

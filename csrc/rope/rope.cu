@@ -6,6 +6,7 @@
 // (reference llmctl/runtime/engine.py:284); config keys rope.base / rope.scaling come from
 // reference configs/models/llama-7b.json:11-14.  The cos/sin table is built by the caller so
 // "linear"/"su" scaling only changes the table, not the kernel.
+#include "../common/dependent.cuh"
 #include "../common/util.cuh"
 
 namespace llmctl {
@@ -15,6 +16,8 @@ __global__ void __launch_bounds__(256)
 rope_kernel(__nv_bfloat16* __restrict__ x, long long row_stride, int n_tokens, int n_heads,
             int head_dim, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
             const int* __restrict__ positions, int seq_len, float sign) {
+  wait_for_previous(x, cos_t, sin_t, positions);
+  release_dependents();
   const int half = head_dim >> 1;
   const int vec_per_head = half >> 3;
   const long long total = static_cast<long long>(n_tokens) * n_heads * vec_per_head;
@@ -60,8 +63,7 @@ LLMCTL_API int llmctl_rope_inplace(void* x, long long row_stride, int n_tokens, 
   if (total == 0) return 0;
   long long blocks = (total + 255) / 256;
   if (blocks > kNumSMs * 16) blocks = kNumSMs * 16;
-  rope_kernel<<<static_cast<int>(blocks), 256, 0, (cudaStream_t)stream>>>(
-      (__nv_bfloat16*)x, row_stride, n_tokens, n_heads, head_dim, cos_t, sin_t, positions, seq_len,
-      sign);
+  LLMCTL_CHECK(launch_dependent(rope_kernel, static_cast<int>(blocks), 256, 0, (cudaStream_t)stream, (__nv_bfloat16*)x, row_stride, n_tokens,
+                                n_heads, head_dim, cos_t, sin_t, positions, seq_len, sign));
   LLMCTL_RETURN_LAST();
 }

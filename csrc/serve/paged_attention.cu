@@ -15,6 +15,7 @@
 // only claims the feature).
 #include "../common/ptx.cuh"
 #include "../common/util.cuh"
+#include "../common/dependent.cuh"
 
 namespace llmctl {
 
@@ -25,6 +26,8 @@ __global__ void __launch_bounds__(128)
 kv_append_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int k_off, int v_off,
                  __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
                  const long long* __restrict__ slot_mapping, int row_elems) {
+  wait_for_previous(qkv, k_cache, v_cache, slot_mapping);
+  release_dependents();
   const int tok = blockIdx.x;
   const long long slot = slot_mapping[tok];
   if (slot < 0) return;  // padded token
@@ -74,6 +77,8 @@ paged_attn_decode_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride
   constexpr int kRowsPerWarp = 32 / kLanesPerRow;
   extern __shared__ __align__(16) uint8_t ring[];
   __shared__ float s_out[kHeadDim + 2];
+  wait_for_previous(q, k_cache, v_cache, block_tables, context_lens, partial, out);
+  release_dependents();
   // heads vary fastest in launch order: the CTAs of all heads of one (sequence, split) are co-resident and walk
   // the same token rows together, so each [heads x head_dim] cache row is fetched from DRAM as one burst
   const int head = blockIdx.x, split = blockIdx.y, b = blockIdx.z;
@@ -242,6 +247,8 @@ template <int kHeadDim>
 __global__ void __launch_bounds__(kHeadDim)
 paged_attn_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out,
                         long long out_stride, int heads, int nsplit) {
+  wait_for_previous(partial, out);
+  release_dependents();
   const int head = blockIdx.x, b = blockIdx.y;
   const float* p = partial + (static_cast<long long>(b) * heads + head) * nsplit * (kHeadDim + 2);
   float gm = -INFINITY;
@@ -266,9 +273,8 @@ LLMCTL_API int llmctl_kv_append(const void* qkv, long long row_stride, int k_off
   LLMCTL_BEGIN();
   LLMCTL_REQUIRE((heads * head_dim) % 8 == 0 && row_stride % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0);
   if (num_tokens == 0) return 0;
-  kv_append_kernel<<<num_tokens, 128, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)qkv, row_stride, k_off, v_off, (__nv_bfloat16*)k_cache,
-      (__nv_bfloat16*)v_cache, slot_mapping, heads * head_dim);
+  LLMCTL_CHECK(launch_dependent(kv_append_kernel, num_tokens, 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)qkv, row_stride, k_off, v_off,
+                                (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, slot_mapping, heads * head_dim));
   LLMCTL_RETURN_LAST();
 }
 
@@ -315,13 +321,15 @@ LLMCTL_API int llmctl_paged_attn_decode(const void* q, long long q_stride, const
     cfg.blockDim = dim3(128, 1, 1);
     cfg.dynamicSmemBytes = kDecodeSmem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 1;
-    at[0].val.clusterDim.y = static_cast<unsigned>(num_splits);
-    at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 1;
+    at[1].val.clusterDim.y = static_cast<unsigned>(num_splits);
+    at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = cluster ? 1 : 0;
+    cfg.numAttrs = cluster ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache,
                               block_tables, max_blocks_per_seq, context_lens, scratch, heads, block_size, shift, per, scale_log2,
                               (__nv_bfloat16*)out, out_stride);
@@ -330,9 +338,9 @@ LLMCTL_API int llmctl_paged_attn_decode(const void* q, long long q_stride, const
   else LLMCTL_CHECK(cluster ? launch(paged_attn_decode_kernel<64, true>) : launch(paged_attn_decode_kernel<64, false>));
   if (!cluster) {
     if (head_dim == 128)
-      paged_attn_merge_kernel<128><<<dim3(heads, batch), 128, 0, s>>>(scratch, (__nv_bfloat16*)out, out_stride, heads, num_splits);
+      LLMCTL_CHECK(launch_dependent(paged_attn_merge_kernel<128>, dim3(heads, batch), 128, 0, s, scratch, (__nv_bfloat16*)out, out_stride, heads, num_splits));
     else
-      paged_attn_merge_kernel<64><<<dim3(heads, batch), 64, 0, s>>>(scratch, (__nv_bfloat16*)out, out_stride, heads, num_splits);
+      LLMCTL_CHECK(launch_dependent(paged_attn_merge_kernel<64>, dim3(heads, batch), 64, 0, s, scratch, (__nv_bfloat16*)out, out_stride, heads, num_splits));
   }
   LLMCTL_RETURN_LAST();
 }

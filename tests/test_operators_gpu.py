@@ -303,3 +303,48 @@ def test_capture(ops):
     x.copy_(_randn(64, 128, seed=9))
     g.replay()
     assert torch.equal(out, layer(x))
+
+
+@pytest.mark.parametrize("rows,width,heads", [(1, 128, 2), (33, 256, 2), (700, 768, 12)])
+def test_kernels_begin_when_those_before_have_ended(ops, rows, width, heads):
+    """A chain of operators whose kernels are launched beside the end of the one before (csrc/common/dependent.cuh), some of them in place or over
+    memory that the one before has just let go of, against the same chain with the device waited for after each."""
+    from llmctl_b200.ops import serving
+    from llmctl_b200.ops.attention import rope_attention_packed
+    D = width // heads
+    cos, sin = ops.rope_tables(D, rows, device="cuda")
+    n, qkv, out, up, down = (1 + _randn(width, seed=1), _randn(3 * width, width, seed=2) * width ** -0.5, _randn(width, width, seed=3) * width ** -0.5,
+                             _randn(4 * width, width, seed=4) * width ** -0.5, _randn(width, 2 * width, seed=5) * width ** -0.5)
+
+    def chain(wait):
+        def then(*t):
+            if wait:
+                torch.cuda.synchronize()
+            return t if len(t) > 1 else t[0]
+        x, r = _randn(rows, width), _randn(rows, width, seed=6)
+        k, v = (torch.zeros(rows, 16, heads, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        tables = torch.arange(rows, device="cuda", dtype=torch.int32).view(rows, 1)
+        with torch.no_grad():
+            for i in range(12):
+                y, r = then(*ops.rmsnorm(x, n, residual=r))
+                p = then(ops.linear(y, qkv))
+                if D in (64, 128):
+                    serving.kv_append(p, k, v, torch.arange(rows, device="cuda") * 16 + i, heads, D)
+                    then(k)
+                    y = then(serving.paged_attention_decode(p[:, :width].reshape(rows, heads, D), k, v, tables, torch.full((rows,), i + 1, device="cuda", dtype=torch.int32), 16))
+                    y = then(ops.linear(y.reshape(rows, width), out))
+                    y, r = then(*ops.rmsnorm(y, n, residual=r))
+                    p = then(ops.linear(y, qkv))
+                y = then(ops.linear(then(rope_attention_packed(p, cos, sin, 1, rows, heads, D)), out))
+                y, r = then(*ops.rmsnorm(y, n, residual=r))
+                x = then(ops.swiglu_mlp(y, up, down))
+        leaves = [t.detach().requires_grad_(True) for t in (x, n, qkv, out, up, down)]
+        x = leaves[0]
+        y, r = ops.rmsnorm(x, leaves[1])
+        o = ops.linear(rope_attention_packed(ops.linear(y, leaves[2]), cos, sin, 1, rows, heads, D), leaves[3])
+        y, r = ops.rmsnorm(o, leaves[1], residual=x)
+        y = ops.swiglu_mlp(y, leaves[4], leaves[5])
+        return (y.detach(), k, v, *torch.autograd.grad((y, r), leaves, (_randn(rows, width, seed=7), _randn(rows, width, seed=8))))
+    want = chain(True)
+    for _ in range(3):
+        _same(chain(False), want)
