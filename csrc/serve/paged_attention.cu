@@ -5,14 +5,15 @@
 // kv_block_manager.cpp); token t sits in slot block_table[t / block_size] * block_size + t % block_size.
 //
 // Decode attention is HBM-bound (every K and V byte of the context is read once), so the kernel is built
-// for bytes in flight, not FLOPs: the context is split over CTAs (split-K) so B x H x splits covers the
-// 148 SMs even at batch 1, each half-warp streams one token (16-byte loads) and keeps an online-softmax
+// for bytes in flight and few instructions per byte: the context is split over CTAs (split-K) so B x H x splits covers the
+// 148 SMs even at batch 1, each warp streams groups of 16 tokens through the tensor cores and keeps an online-softmax
 // state in registers.  Where all CTAs fit one wave the (max, sum, acc) triples of up to 8 splits are merged inside a cluster
 // through distributed shared memory, in one launch; otherwise they go through scratch and a second kernel.
 //
 // Reference: the reference has no paged attention — it re-runs the HF model over the whole right-padded
 // sequence every step and throws the cache away (reference llmctl/serve/server.py:199-204; README.md:12,67
 // only claims the feature).
+#include "../common/mma_sync.cuh"
 #include "../common/ptx.cuh"
 #include "../common/util.cuh"
 #include "../common/dependent.cuh"
@@ -49,19 +50,28 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
 
 // ---------------------------------------------------------------------------------------------
 // K12: decode attention.  grid = (heads, splits, batch), block = 128 threads.
-// head_dim = 128: a half-warp (16 lanes x 8 elements) covers one K/V row.  A warp takes every fourth group of 4 rows per lane group;
-// the rows come through a ring in shared memory that every lane fills and reads for itself (16-byte asynchronous copies, four
-// groups deep, no barrier): 64 KB in flight per CTA, three CTAs per SM.  Loads into registers that were all waited for before the
-// arithmetic left HBM idle in between: 16 contexts of up to 4096 (697 MB) took 195 us, now 123 us (5.7 TB/s).
+// A warp takes every fourth group of 16 tokens, whose K and V rows come through a ring of its own in shared memory (16-byte
+// asynchronous copies, no block barrier).  Both products run on the tensor cores (mma.sync m16n8k16) with the tokens, then the head's
+// dimensions, as the 16 rows: the one query fills a column of eight, and the probabilities, which stay fp32, take three of them as the bf16
+// pieces of their 24 bits (high + middle + low, each the rest truncated: exact).  Bound by HBM.  With fp32 FMAs, a token to a
+// half-warp (360 instructions per 16 tokens and head for 190 here), 63% of the issue slots were taken and DRAM was active 66% of the
+// time.  us, FMAs / now: 16 contexts of up to 4096, 32 heads of 128 (697 MB) 125.2 / 110.2 (6.3 TB/s), 32 of them 220.9 / 199.2, 8 of up to 2304
+// 47.5 / 39.6, 4 of up to 700 15.5 / 11.7; 16 of up to 4096, 12 heads of 64 36.3 / 30.7, 64 of 500 17.6 / 13.5, one of 300 3.9 / 3.8.
 // partial layout: [batch, heads, splits, head_dim + 2] fp32 = {acc[head_dim], max, sum}.
 // kCluster: the splits of a (head, sequence) are one cluster and its first CTA writes the output itself.
 // ---------------------------------------------------------------------------------------------
 constexpr int kMaxClusterSplits = 8;         // portable cluster size
-constexpr int kDecodeStages = 4, kDecodeRows = 4;
-constexpr int kDecodeSmem = 128 * kDecodeStages * kDecodeRows * 32;      // a lane's ring: stages x rows x (16 bytes of K + 16 of V)
+constexpr int kDecodeStages = 2;             // of 16 tokens: deeper rings leave fewer CTAs on an SM (3 stages 120 us, 4 199 us)
+constexpr int decode_smem(int head_dim) { return 4 * kDecodeStages * 2 * 16 * head_dim * 2; }
 
 __device__ __forceinline__ void cp_async_16_or_zero(uint32_t dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&a)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&a)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
 }
 
 template <int kHeadDim, bool kCluster>
@@ -73,10 +83,13 @@ paged_attn_decode_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride
                          const int* __restrict__ context_lens, float* __restrict__ partial,
                          int heads, int block_size, int block_shift, int tokens_per_split, float scale_log2,
                          __nv_bfloat16* __restrict__ out, long long out_stride) {
-  constexpr int kLanesPerRow = kHeadDim / 8;          // 16 for D=128, 8 for D=64
-  constexpr int kRowsPerWarp = 32 / kLanesPerRow;
-  extern __shared__ __align__(16) uint8_t ring[];
+  constexpr int kUnits = kHeadDim / 8;                // 16-byte units of a row
+  constexpr int kRowsPerCopy = 32 / kUnits;           // rows that a warp copies at a time
+  constexpr int kTile = 16 * kHeadDim * 2;            // bytes of 16 rows
+  constexpr int kSteps = kHeadDim / 16;
+  extern __shared__ __align__(128) uint8_t ring[];
   __shared__ float s_out[kHeadDim + 2];
+  __shared__ float s_acc[4][kHeadDim], s_m[4], s_l[4];
   wait_for_previous(q, k_cache, v_cache, block_tables, context_lens, partial, out);
   release_dependents();
   // heads vary fastest in launch order: the CTAs of all heads of one (sequence, split) are co-resident and walk
@@ -87,125 +100,151 @@ paged_attn_decode_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride
   const int t0 = split * tokens_per_split;
   const int t1 = min(ctx, t0 + tokens_per_split);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sub = lane / kLanesPerRow;                // which row of the warp's group
-  const int li = lane % kLanesPerRow;                 // 8-element slice of the row
+  const int g = lane >> 2, t = lane & 3;              // fragment coordinates
   const int* bt = block_tables + static_cast<long long>(b) * max_blocks_per_seq;
   const long long row_elems = static_cast<long long>(heads) * kHeadDim;
-  const __nv_bfloat16* kc = k_cache + head * kHeadDim + li * 8;
-  const __nv_bfloat16* vc = v_cache + head * kHeadDim + li * 8;
+  const int unit = lane % kUnits, sub = lane / kUnits;
+  const __nv_bfloat16* kc = k_cache + head * kHeadDim + unit * 8;
+  const __nv_bfloat16* vc = v_cache + head * kHeadDim + unit * 8;
 
-  float qf[8];
-  unpack8(load8(q + b * q_stride + head * kHeadDim + li * 8), qf);
+  // the query as the first column of B
+  uint32_t bq[kSteps][2];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) qf[j] *= scale_log2;
+  for (int ks = 0; ks < kSteps; ++ks) {
+    bq[ks][0] = bq[ks][1] = 0u;
+    if (g == 0) {
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(q + b * q_stride + head * kHeadDim + ks * 16) + t;
+      bq[ks][0] = src[0];
+      bq[ks][1] = src[4];
+    }
+  }
+  float m = -INFINITY, l = 0.f, acc[kSteps][4];
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
 
-  float m = -INFINITY, l = 0.f, acc[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-
-  // group g of this warp: rows t0 + ((g * 4 + warp) * kDecodeRows + u) * kRowsPerWarp + sub, u < kDecodeRows
-  constexpr int kGroupTokens = kDecodeRows * kRowsPerWarp;
-  const int first = t0 + warp * kGroupTokens + sub;
-  const int groups = t1 > t0 ? (t1 - t0 + 4 * kGroupTokens - 1) / (4 * kGroupTokens) : 0;      // uniform over the CTA
-  const uint32_t mine = ptx::smem_u32(ring) + threadIdx.x * 16;
-  constexpr uint32_t kRow = 128 * 16;                 // bytes between a lane's consecutive 16-byte pieces
-  auto token = [&](int g, int u) { return first + g * 4 * kGroupTokens + u * kRowsPerWarp; };
-  auto page_of = [&](int t) { return bt[block_shift >= 0 ? t >> block_shift : t / block_size]; };
-  auto rest_of = [&](int t) { return block_shift >= 0 ? t & (block_size - 1) : t % block_size; };
-  int page[kDecodeRows];                              // pages of the next group to be fetched, looked up a group ahead
-  auto look_up = [&](int g) {
-#pragma unroll
-    for (int u = 0; u < kDecodeRows; ++u) {
-      const int t = token(g, u);
-      page[u] = g < groups && t < t1 ? page_of(t) : 0;
+  // group n of this warp: tokens t0 + (4 n + warp) * 16 ..; rows are stored with their 16-byte units swizzled by row % 8
+  const int groups = t1 > t0 ? (t1 - t0 + 63) / 64 : 0;      // uniform over the CTA
+  const uint32_t mine = ptx::smem_u32(ring) + warp * (kDecodeStages * 2 * kTile);
+  auto first_of = [&](int n) { return t0 + (4 * n + warp) * 16; };
+  int slot = 0;                                       // cache row of token lane % 16 of the next group to be fetched, looked up a group ahead
+  auto look_up = [&](int n) {
+    const int tok = first_of(n) + (lane & 15);
+    slot = 0;
+    if (n < groups && tok < t1) {
+      const int page = bt[block_shift >= 0 ? tok >> block_shift : tok / block_size];
+      slot = page * block_size + (block_shift >= 0 ? tok & (block_size - 1) : tok % block_size);
     }
   };
-  auto fetch = [&](int g) {
-    if (g < groups) {
-      const uint32_t at = mine + (g % kDecodeStages) * (2 * kDecodeRows * kRow);
+  auto fetch = [&](int n) {
+    if (n < groups) {
+      const int valid = t1 - first_of(n);
+      const uint32_t at = mine + (n % kDecodeStages) * (2 * kTile);
 #pragma unroll
-      for (int u = 0; u < kDecodeRows; ++u) {
-        const int t = token(g, u);
-        const bool valid = t < t1;
-        const long long off = valid ? (static_cast<long long>(page[u]) * block_size + rest_of(t)) * row_elems : 0;
-        cp_async_16_or_zero(at + (2 * u) * kRow, kc + off, valid);
-        cp_async_16_or_zero(at + (2 * u + 1) * kRow, vc + off, valid);
+      for (int i = 0; i < 16 / kRowsPerCopy; ++i) {
+        const int row = i * kRowsPerCopy + sub;
+        const long long off = __shfl_sync(0xffffffffu, slot, row) * row_elems;
+        const uint32_t dst = at + row * (kHeadDim * 2) + ((unit ^ (row & 7)) << 4);
+        cp_async_16_or_zero(dst, kc + off, row < valid);
+        cp_async_16_or_zero(dst + kTile, vc + off, row < valid);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   look_up(0);
 #pragma unroll
-  for (int g = 0; g < kDecodeStages - 1; ++g) {
-    fetch(g);
-    look_up(g + 1);
+  for (int n = 0; n < kDecodeStages - 1; ++n) {
+    fetch(n);
+    look_up(n + 1);
   }
-  // The trip count is uniform across the warp: the shuffles below use the full mask, so a lane whose token
-  // is out of range still executes them (with a masked score) instead of leaving the loop early.
-  for (int g = 0; g < groups; ++g) {
-    fetch(g + kDecodeStages - 1);
-    look_up(g + kDecodeStages);
+  const int krow = lane & 15, kswz = krow & 7;        // K as A: lanes 0-15 address the first eight columns of 16 rows, 16-31 the next
+  const int vrow = (lane & 7) + ((lane >> 4) << 3);   // V transposed as A: columns (dimensions) by lane / 8 % 2, rows (tokens) by lane / 16
+  const uint32_t k_at = mine + krow * (kHeadDim * 2), v_at = mine + kTile + vrow * (kHeadDim * 2);
+  for (int n = 0; n < groups; ++n) {
+    __syncwarp();                                     // the stage that is filled now was read by all lanes a turn ago
+    fetch(n + kDecodeStages - 1);
+    look_up(n + kDecodeStages);
     asm volatile("cp.async.wait_group %0;" ::"n"(kDecodeStages - 1) : "memory");
-    const uint8_t* at = ring + threadIdx.x * 16 + (g % kDecodeStages) * (2 * kDecodeRows * kRow);
-    float sc[kDecodeRows];
+    __syncwarp();
+    const uint32_t stage = (n % kDecodeStages) * (2 * kTile);
+    float sc[2][4] = {};
 #pragma unroll
-    for (int u = 0; u < kDecodeRows; ++u) {
-      float kf[8];
-      unpack8(*reinterpret_cast<const bf16x8*>(at + (2 * u) * kRow), kf);
-      float s = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s += qf[j] * kf[j];
-      sc[u] = s;
+    for (int ks = 0; ks < kSteps; ++ks) {
+      uint32_t a[4];
+      ldmatrix_x4(a, k_at + stage + (((2 * ks + (lane >> 4)) ^ kswz) << 4));
+      mma_bf16_16816(sc[ks & 1], a, bq[ks]);
     }
+    // lanes 4 g hold the scores of tokens g and g + 8
+    const int left = t1 - first_of(n);
+    float x0 = g < left ? (sc[0][0] + sc[1][0]) * scale_log2 : -INFINITY, x1 = g + 8 < left ? (sc[0][2] + sc[1][2]) * scale_log2 : -INFINITY;
+    x0 = __shfl_sync(0xffffffffu, x0, lane & 28);
+    x1 = __shfl_sync(0xffffffffu, x1, lane & 28);
+    float m_new = fmaxf(x0, x1);
 #pragma unroll
-    for (int o = kLanesPerRow / 2; o > 0; o >>= 1)
-#pragma unroll
-      for (int u = 0; u < kDecodeRows; ++u) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o);
-    float m_new = m;
-#pragma unroll
-    for (int u = 0; u < kDecodeRows; ++u) {
-      if (token(g, u) >= t1) sc[u] = -INFINITY;
-      m_new = fmaxf(m_new, sc[u]);
-    }
+    for (int o = 4; o < 32; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
+    m_new = fmaxf(m, m_new);
     const float ref = m_new == -INFINITY ? 0.f : m_new;      // nothing seen yet: every weight below is 0
-    const float corr = exp2f(m - ref);
-    l *= corr;
+    if (m_new != m) {                                 // uniform over the warp
+      const float corr = exp2f(m - ref);
+      l *= corr;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] *= corr;
+      for (int i = 0; i < kSteps; ++i)
 #pragma unroll
-    for (int u = 0; u < kDecodeRows; ++u) {
-      float vf[8];
-      unpack8(*reinterpret_cast<const bf16x8*>(at + (2 * u + 1) * kRow), vf);
-      const float pr = exp2f(sc[u] - ref);
-      l += pr;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += pr * vf[j];
+        for (int e = 0; e < 4; ++e) acc[i][e] *= corr;
+      m = m_new;
     }
-    m = m_new;
+    const float p0 = exp2f(x0 - ref), p1 = exp2f(x1 - ref);
+    l += p0 + p1;
+    // column c of B is the c-th piece of the probabilities
+    uint32_t bp[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float w[2] = {__shfl_sync(0xffffffffu, h ? p1 : p0, 8 * t), __shfl_sync(0xffffffffu, h ? p1 : p0, 8 * t + 4)};
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float high = __uint_as_float(__float_as_uint(w[e]) & 0xffff0000u), rest = w[e] - high;
+        const float middle = __uint_as_float(__float_as_uint(rest) & 0xffff0000u);
+        w[e] = g == 0 ? high : g == 1 ? middle : g == 2 ? rest - middle : 0.f;
+      }
+      bp[h] = __byte_perm(__float_as_uint(w[0]), __float_as_uint(w[1]), 0x7632);
+    }
+#pragma unroll
+    for (int i = 0; i < kSteps; ++i) {
+      uint32_t a[4];
+      ldmatrix_x4_trans(a, v_at + stage + (((2 * i + ((lane >> 3) & 1)) ^ (vrow & 7)) << 4));
+      mma_bf16_16816(acc[i], a, bp);
+    }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();                                    // the ring is idle: it takes the groups' partial states
 
-  // merge the (4 warps x kRowsPerWarp) partial states through shared memory
-  constexpr int ngroups = 4 * kRowsPerWarp;
-  float* s_acc = reinterpret_cast<float*>(ring);      // [ngroups][kHeadDim], then max and sum per group
-  float *s_m = s_acc + ngroups * kHeadDim, *s_l = s_m + ngroups;
-  const int gi = warp * kRowsPerWarp + sub;           // group id
-  if (li == 0) {
-    s_m[gi] = m;
-    s_l[gi] = l;
-  }
+  // The pieces of a dimension: columns 0 and 1 in lanes with t = 0, column 2 in those with t = 1.  A sum that is not finite in its first
+  // piece (an infinity or NaN among the values) is that piece alone: the others multiplied it by zeros.
 #pragma unroll
-  for (int j = 0; j < 8; ++j) s_acc[gi * kHeadDim + li * 8 + j] = acc[j];
+  for (int i = 0; i < kSteps; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float low = __shfl_sync(0xffffffffu, acc[i][2 * h], lane | 1);
+      const float high = acc[i][2 * h];
+      if (t == 0) s_acc[warp][i * 16 + h * 8 + g] = isfinite(high) ? high + (acc[i][2 * h + 1] + low) : high;
+    }
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+  if (lane == 0) {
+    s_m[warp] = m;
+    s_l[warp] = l;
+  }
   __syncthreads();
   if (threadIdx.x < kHeadDim) {
     float gm = -INFINITY;
-    for (int i = 0; i < ngroups; ++i) gm = fmaxf(gm, s_m[i]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) gm = fmaxf(gm, s_m[i]);
     float gl = 0.f, ga = 0.f;
-    for (int i = 0; i < ngroups; ++i) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
       const float w = (s_m[i] == -INFINITY) ? 0.f : exp2f(s_m[i] - gm);
       gl += s_l[i] * w;
-      ga += s_acc[i * kHeadDim + threadIdx.x] * w;
+      ga += s_acc[i][threadIdx.x] * w;
     }
     float* dst = kCluster ? s_out : partial + ((static_cast<long long>(b) * heads + head) * nsplit + split) * (kHeadDim + 2);
     dst[threadIdx.x] = ga;
@@ -314,12 +353,13 @@ LLMCTL_API int llmctl_paged_attn_decode(const void* q, long long q_stride, const
     for (shift = 0; (1 << shift) < block_size; ++shift) {
     }
   auto launch = [&](auto kern) -> cudaError_t {
-    const cudaError_t e = allow_smem(kern, kDecodeSmem);
+    const int smem = decode_smem(head_dim);
+    const cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(heads, num_splits, batch);
     cfg.blockDim = dim3(128, 1, 1);
-    cfg.dynamicSmemBytes = kDecodeSmem;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -36,13 +36,13 @@ def kv_append(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, s
 
 
 def choose_splits(batch: int, heads: int, max_context: int, block_size: int, sms: int = 148) -> int:
-    # Decode attention is a latency-bound stream: each CTA walks block table -> K/V rows -> online softmax in a
-    # dependent chain, so HBM only fills up with ~8 resident CTAs per SM.  Splits are whole KV blocks of >= 64 tokens;
-    # the merge pass costs (head_dim + 2) floats per split, ~3 % of the K/V bytes at 64 tokens per split.
-    # Up to 512 (head, sequence) pairs a CTA walks at most 512 tokens where 8 splits allow it: with longer walks a full batch of unlike
-    # contexts is one and a half waves of CTAs that end at different times (us in ceil(8 sms / pairs) splits / in 8, 32 heads of 128, contexts
-    # from 1 K to 4 K: 16 sequences 154.6 / 140.3).  More pairs fill the waves by themselves, and what each split adds is lost (32 sequences
-    # 242.7 / 246.8, 64: 448 / 472, 256: 1692 / 1912; 64 sequences of up to 2304, 12 heads of 64: 72.9 / 85.0).
+    # Each CTA walks block table -> K/V rows -> online softmax in a dependent chain, so HBM fills up with a few CTAs per SM and many more
+    # to follow.  Splits are whole KV blocks of >= 64 tokens; the merge pass costs (head_dim + 2) floats per split, ~3 % of the K/V bytes at
+    # 64 tokens per split.
+    # Up to 512 (head, sequence) pairs a CTA walks at most 512 tokens where 8 splits allow it, so that a full batch of unlike contexts ends
+    # together; more pairs fill the waves by themselves, and what each split adds is lost (us by splits, contexts from a quarter of the
+    # stated one: 16 sequences of up to 4096, 32 heads of 128 2: 109.0, 8: 110.8, 16: 118.0; 32 of them 2: 200.1, 8: 203.3; 64 1: 374.6, 4: 383.5;
+    # 256 of up to 1500 1: 551.7, 4: 575.2; 64 of up to 2304, 12 heads of 64 1: 55.3, 2: 53.9, 8: 54.3).
     want = max(1, (8 * sms + batch * heads - 1) // (batch * heads), min(8, (max_context + 511) // 512) if batch * heads <= 512 else 1)
     per_split = max(block_size, (64 // block_size) * block_size) if block_size <= 64 else block_size
     return int(max(1, min(want, max(1, max_context // per_split), 256)))
@@ -50,10 +50,10 @@ def choose_splits(batch: int, heads: int, max_context: int, block_size: int, sms
 
 def _launch_splits(batch: int, heads: int, head_dim: int, max_context: int, block_size: int, sms: int = 148) -> int:
     # One launch, merged inside clusters of up to 8 splits, while all CTAs (three per SM) are resident together and none walks
-    # more than 768 tokens (us in the splits of choose_splits with a merge kernel / in one launch: one context of 4096, 32 heads of 128
-    # 23 / 18; 8 of up to 2304, 4 heads 25.6 / 22.6; 4 of up to 700, 32 heads 25.6 / 20.5; 64 of 500, 4 heads 31.7 / 26.7).  Beyond one
-    # wave a single split without a merge kernel pays for the shortest walks only (64 of 500, 12 heads of 64: 39.9 / 37.0; 32 heads of
-    # 128: 68.6 / 75.8 for 32 of them); larger batches and longer contexts take choose_splits.
+    # more than 768 tokens (us in one launch / in the splits of choose_splits with a merge kernel: one context of 4096, 32 heads of 128
+    # 14.5 in 8 / 16.8 in 16; 8 of up to 2304, 4 heads 13.5 / 13.8; 64 of 500, 4 heads 12.6 / 12.3).  Beyond one
+    # wave a single split without a merge kernel pays for the shortest walks only (64 of 500, 12 heads of 64: 13.5 / 14.8; 32 heads of
+    # 128: 65.1 / 62.8); larger batches and longer contexts take choose_splits.
     resident = min(8, 3 * sms // (batch * heads))
     if max_context <= 768 * resident:
         return max(1, min(resident, max_context // 64))

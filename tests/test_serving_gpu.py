@@ -132,3 +132,46 @@ def test_engine_gpu_matches_full_recompute(cuda_device):
             ids.append(t)
     assert agree >= total - 1, f"only {agree}/{total} decode tokens agree with full recompute"
     assert eng.kv.free_blocks == 256
+
+
+@pytest.mark.parametrize("H,D,bs,splits", [(3, 64, 16, 1), (2, 128, 16, 2), (2, 128, 5, 3), (3, 64, 64, 8), (1, 128, 1, 1)])
+def test_paged_decode_around_its_groups(cuda_device, H, D, bs, splits):
+    """Context lengths around the warps' groups of 16 tokens and the CTA's 64, against float64; the output is rounded to bf16 (2^-9), its sum of
+    products in fp32."""
+    from llmctl_b200.ops import serving as sops
+    torch.manual_seed(D + bs)
+    lens = [1, 15, 16, 17, 31, 63, 64, 65, 79, 128, 129, 200, 257]
+    B, ctx = len(lens), 320
+    pages = (ctx + bs - 1) // bs
+    perm = torch.randperm(B * pages).view(B, pages)
+    k, v = (torch.randn(B * pages, bs, H, D, device=cuda_device).bfloat16() for _ in range(2))
+    q = torch.randn(B, H, D, device=cuda_device).bfloat16()
+    out = sops.paged_attention_decode(q, k, v, perm.int().to(cuda_device), torch.tensor(lens, dtype=torch.int32, device=cuda_device), ctx, num_splits=splits)
+    for i, n in enumerate(lens):
+        rows = (perm[i, torch.arange(n) // bs] * bs + torch.arange(n) % bs).to(cuda_device)
+        kk, vv = (t.view(-1, H, D)[rows].double() for t in (k, v))
+        want = torch.einsum("hn,nhd->hd", torch.softmax(torch.einsum("hd,nhd->hn", q[i].double(), kk) * D ** -0.5, -1), vv)
+        assert (out[i].double() - want).norm() <= (2.0 ** -9 + 1e-5) * want.norm(), n
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_paged_decode_with_infinities_and_nan(cuda_device, D):
+    """An infinity or NaN among a head's values reaches its dimension of the output and no other; a context's unused rows reach nothing."""
+    from llmctl_b200.ops import serving as sops
+    torch.manual_seed(D)
+    B, H, n = 6, 2, 100
+    k, v = (torch.randn(B * 7, 16, H, D, device=cuda_device).bfloat16() for _ in range(2))
+    q = torch.randn(B, H, D, device=cuda_device).bfloat16()
+    bt = torch.arange(B * 7, dtype=torch.int32, device=cuda_device).view(B, 7)
+    lens = torch.full((B,), n, dtype=torch.int32, device=cuda_device)
+    plain = sops.paged_attention_decode(q, k, v, bt, lens, 112, num_splits=2)
+    inf = float("inf")
+    v.view(B, 112, H, D)[0, 33, 1, 5] = inf
+    v.view(B, 112, H, D)[1, 34, 0, 6] = float("nan")
+    v.view(B, 112, H, D)[2, 35, 0, 7], v.view(B, 112, H, D)[2, 70, 0, 7] = inf, -inf
+    k.view(B, 112, H, D)[4, n:], v.view(B, 112, H, D)[4, n:] = float("nan"), inf
+    v.view(B, 112, H, D)[5, 99, 1, D - 1] = -inf
+    out = sops.paged_attention_decode(q, k, v, bt, lens, 112, num_splits=2)
+    want = plain.clone()
+    want[0, 1, 5], want[1, 0, 6], want[2, 0, 7], want[5, 1, D - 1] = inf, float("nan"), float("nan"), -inf
+    assert torch.equal(torch.nan_to_num(out, nan=7777.0, posinf=8888.0, neginf=-8888.0), torch.nan_to_num(want, nan=7777.0, posinf=8888.0, neginf=-8888.0))
