@@ -13,7 +13,7 @@ from typing import List, Optional, Sequence as Seq, Tuple
 import numpy as np
 import torch
 
-from ..ops.latent_attention import KEY_ROWS, ROWS_PER_TILE, TILE_WIDTHS
+from ..ops.latent_attention import KEY_ROWS, ROWS_PER_TILE, ROWS_PER_TILE_WIDE, TILE_WIDTHS
 
 
 @dataclass
@@ -91,6 +91,7 @@ class RaggedBatch:
         """Write the description of ``portions`` into the (same) buffers and copy it to the device."""
         tokens, slots, out_rows, positions, tiles, tables, seq_rows, prows, srows = self._h
         block_size = self.block_size
+        self._portions, self._splits = portions, {}
         if self.pad_to is not None:
             assert len(portions) <= self.pad_to[0] and all(len(p.tokens) == 1 for p in portions)
             tokens[:] = 0
@@ -150,5 +151,30 @@ class RaggedBatch:
         """Split the keys of long contexts over CTAs when the tiles alone would leave most SMs idle.  ``span``: most keys a
         tile reads (the longest context unless a window bounds it)."""
         hpt = self.heads_per_tile(heads, rows)
-        ctas = self._tiles[rows].shape[0] * ((heads + hpt - 1) // hpt)
-        return int(max(1, min(2 * self._sms // max(ctas, 1), (self.max_context if span is None else span) // 64)))
+        groups = (heads + hpt - 1) // hpt
+        longest = self.max_context if span is None else span
+        if self.decode_only and rows in (ROWS_PER_TILE, ROWS_PER_TILE_WIDE):
+            key = (rows, groups, longest)
+            if key not in self._splits:
+                self._splits[key] = self._even_splits(self._sms * (2 if rows == ROWS_PER_TILE else 1), groups, longest)
+            return self._splits[key]
+        ctas = self._tiles[rows].shape[0] * groups
+        return int(max(1, min(2 * self._sms // max(ctas, 1), longest // 64)))
+
+    def _even_splits(self, slots: int, groups: int, longest: int) -> int:
+        """Most splits with which all CTAs that have keys to read run at once (two to an SM with 16 rows, one with 32): a sequence's
+        splits are of one length, whole tiles of 64 keys, and those past its end have nothing to do.  A second wave, and half-empty
+        splits, cost more than longer ones (us with the merge, splits by the longest context alone / these: 32 contexts of 2000-4000, 16 heads
+        70.9 in 9 / 65.1 in 12, 32 heads 111.5 in 9 / 91.7 in 5; 4 of 600-1000, 16 heads 24.6 in 15 / 20.6 in 16; 8 of 1000-2000, 32 heads
+        45.8 in 31 / 33.6 in 16; 16 of 150-300, 16 heads 23.6 in 4 / 19.8 in 5)."""
+        if self.pad_to is None:
+            contexts = [min(p.start + len(p.tokens), longest) for p in self._portions]
+        else:                                                   # captured: any of them may be the longest
+            contexts = [longest] * self.pad_to[0]
+        tiles = max(1, -(-sum(contexts) * groups // (64 * slots)))
+        while True:
+            n = -(-longest // (64 * tiles))
+            per = max(64, (-(-longest // n) + 63) // 64 * 64)
+            if n <= 1 or groups * sum(-(-c // per) for c in contexts) <= slots:
+                return max(1, n)
+            tiles += 1

@@ -356,3 +356,29 @@ def test_latent_ranks_of_the_fp32_kernel_keep_it_for_prompts(monkeypatch, R, reb
     assert L.uses_tensor_cores(q.dtype, R, 64) == rebuilds
     assert L.rebuild_pays(q, 128, 64, 128, R, 4, 1024, 1024 * L.REBUILD_PAIRS) == rebuilds
     assert not L.rebuild_pays(q, 128, 64, 128, R, 4, 1024, 1024 * L.REBUILD_PAIRS - 1)
+
+
+@pytest.mark.parametrize("starts,heads", [([4000 - 62 * i for i in range(32)], 16), ([4000 - 62 * i for i in range(32)], 32), ([3000], 16), ([0], 16),
+                                          ([63, 64, 65], 16), ([500] * 300, 16), ([2000, 1], 40)])
+def test_decode_splits_fill_one_wave(starts, heads):
+    """Splits of a decoding batch: whole tiles of 64 keys that cover the longest context, and no more CTAs with keys than run at once unless every
+    context is whole; the next finer cut would have more, or is none."""
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+    b = RaggedBatch([Portion(i, [1], s, [0], list(range(s // 64 + 1))) for i, s in enumerate(starts)], 64, torch.device("cpu"))
+    rows = 32 if heads > 16 else 16
+    groups, slots = -(-heads // b.heads_per_tile(heads, rows)), b._sms * (2 if rows == 16 else 1)
+
+    def ctas(n):
+        per = max(64, (-(-b.max_context // n) + 63) // 64 * 64)
+        assert n * per >= b.max_context
+        return groups * sum(-(-(s + 1) // per) for s in starts)
+    n = b.attention_splits(heads, rows)
+    assert n == 1 or ctas(n) <= slots
+    # finer by whole tiles: the first cut of the same length is n, all shorter ones have too many
+    longest = -(-b.max_context // 64)
+    for tiles in range(1, -(-longest // n)):
+        finer = -(-longest // tiles)
+        assert finer <= n or ctas(finer) > slots or -(-b.max_context // finer) > 64 * tiles
+    assert b.attention_splits(heads, rows) == n
+    b.refill([Portion(0, [1], 0, [0], [0])] * len(starts))
+    assert b.attention_splits(heads, rows, 1) == 1

@@ -381,3 +381,53 @@ def test_greedy_generation_with_replayed_decode_graph(cuda_device, dt):
             if top2[row, 0] - top2[row, 1] > gap:
                 assert tok == int(ref[row].argmax()), f"token {k} of prompt len {len(p)}"
     assert eng.kv.free_blocks == 40
+
+
+@pytest.mark.parametrize("T,Q,R,dr,dt", [(1, 24, 64, 16, torch.bfloat16), (5, 1536, 512, 64, torch.bfloat16), (7, 0, 128, 72, torch.bfloat16),
+                                         (3, 64, 0, 0, torch.bfloat16), (9, 768, 512, 0, torch.bfloat16), (4, 40, 33, 6, torch.float32)])
+def test_latent_write_parts(cuda_device, T, Q, R, dr, dt):
+    """Query and cache parts alone and together, rotated parts of more pairs than a warp has lanes and none, skipped tokens, sizes that take the
+    general kernel; against the PyTorch restatement (norms in fp32, one rounding)."""
+    from llmctl_b200.ops import latent_attention as L
+    torch.manual_seed(Q + R)
+    d, wq, wkv = torch.randn(T, Q + R + dr).to(dt), torch.rand(Q).add(0.5).to(dt), torch.rand(R).add(0.5).to(dt)
+    freq = torch.rand(max(dr // 2, 1))
+    slots = torch.arange(T) * 3
+    if T > 2:
+        slots[1] = -1
+    pos = torch.arange(T, dtype=torch.int32) * 977
+    got = []
+    for dev in ("cpu", "cuda"):
+        cache = torch.zeros(1, 3 * T, R + dr, dtype=dt, device=dev) if R else None
+        cq = L.latent_kv_write(d.to(dev), Q, R, dr, wq.to(dev) if Q else None, wkv.to(dev) if R else None, cache, slots.to(dev), pos.to(dev),
+                               freq.to(dev), 1.25, 1e-5)
+        got.append((cq, cache))
+    eps = 2.0 ** -8 if dt == torch.bfloat16 else 1e-5
+    for a, b in zip(*got):
+        assert (a is None) == (b is None)
+        if a is not None:
+            assert (a.double() - b.cpu().double()).norm() <= eps * a.double().norm() + 1e-12
+
+
+@pytest.mark.parametrize("R,dr,H,splits", [(64, 16, 3, 2), (64, 16, 3, 9), (512, 64, 16, 33), (512, 64, 2, 40), (72, 8, 2, 7), (33, 6, 2, 5)])
+def test_latent_attention_merges_any_number_of_pieces(cuda_device, R, dr, H, splits):
+    """Pieces around the eight that the merge kernel asks for ahead and the 32 that a warp weighs at once, some of them past a context's end, odd
+    widths; against the PyTorch restatement."""
+    from llmctl_b200.ops import latent_attention as L
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+    torch.manual_seed(splits)
+    dt = torch.float32 if R % 8 else torch.bfloat16
+    bs, dn, starts = 32, 8, [64 * splits - 3, 64, 700 % (64 * splits)]
+    pages = [(s + bs) // bs for s in starts]
+    tables = [list(range(sum(pages[:i]), sum(pages[:i + 1]))) for i in range(3)]
+    cache = torch.randn(sum(pages), bs, R + dr).to(dt)
+    ql, q, freq = torch.randn(3, H, R), torch.randn(3, H * (dn + dr)).to(dt), torch.rand(dr // 2)
+    if dt == torch.bfloat16:
+        ql = ql.bfloat16().float()
+    got = []
+    for dev in ("cpu", "cuda"):
+        b = RaggedBatch([Portion(i, [0], s, [0], t) for i, (s, t) in enumerate(zip(starts, tables))], bs, torch.device(dev))
+        got.append(L.latent_attention(ql.to(dev), q.to(dev), dn, cache.to(dev), b.block_tables, b.tiles(), b.positions, freq.to(dev), 1.0, 0.1,
+                                      b.heads_per_tile(H), b.max_context, splits).double().cpu())
+    eps = 1e-2 if dt == torch.bfloat16 else 1e-5          # bf16: rotated queries, probabilities and the output are rounded
+    assert (got[0] - got[1]).norm() <= eps * got[0].norm()
