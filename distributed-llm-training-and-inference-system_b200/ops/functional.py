@@ -632,26 +632,26 @@ class _CrossEntropyFn(torch.autograd.Function):
     ``assume_unit_grad`` the backward hands the buffer on untouched, otherwise it rescales in place."""
 
     @staticmethod
-    def forward(ctx, logits, targets, ignore_index, inv_count, grad_scale, assume_unit_grad):
+    def forward(ctx, logits, targets, ignore_index, grad_scale, assume_unit_grad):
         rows, V = logits.shape
-        loss_rows = torch.empty(rows, dtype=torch.float32, device=logits.device)
+        work = torch.empty(rows + 1, dtype=torch.float32, device=logits.device)
+        loss = torch.empty((), dtype=torch.float32, device=logits.device)
         need_grad = logits.requires_grad
         # The kernel writes through the raw pointer; autograd is deliberately not told (mark_dirty cannot be
         # combined with view inputs).  Safe because the producing GEMM does not keep its output for backward
         # and the documented contract is that the caller never touches `logits` again.
-        native.call("llmctl_cross_entropy_fwd_bwd", logits.data_ptr(), logits.stride(0), targets.data_ptr(),
-                    loss_rows.data_ptr(), None, rows, V, ignore_index, float(grad_scale), inv_count.data_ptr(),
-                    int(need_grad), native.stream_ptr())
+        native.call("llmctl_cross_entropy_mean", logits.data_ptr(), logits.stride(0), targets.data_ptr(),
+                    work.data_ptr(), rows, V, ignore_index, float(grad_scale), int(need_grad), loss.data_ptr(), native.stream_ptr())
         ctx.save_for_backward(logits.detach())
         ctx.assume_unit = assume_unit_grad
-        return (loss_rows.sum() * inv_count).squeeze() * grad_scale
+        return loss
 
     @staticmethod
     def backward(ctx, dloss):
         (grad,) = ctx.saved_tensors
         if not ctx.assume_unit:
             grad = grad.mul_(dloss.to(grad.dtype))
-        return grad, None, None, None, None, None
+        return grad, None, None, None, None
 
 
 def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int = -100,
@@ -664,14 +664,12 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int
     t = targets.reshape(-1)
     # rows of whole 16-byte units at 16-byte boundaries (what is cloned below begins at one)
     if (_use_native(logits2, "elementwise") and V % 8 == 0 and logits2.stride(1) == 1 and logits2.stride(0) % 8 == 0
-            and (not logits2.requires_grad or logits2.data_ptr() % 16 == 0)):
-        cnt = (t != ignore_index).sum().clamp_min(1).to(torch.float32)
-        inv = (1.0 / cnt).reshape(1)
+            and t.dtype == torch.int64 and t.numel() == logits2.shape[0] and t.device == logits2.device and (not logits2.requires_grad or logits2.data_ptr() % 16 == 0)):
         if not logits2.requires_grad:
             logits2 = logits2.clone()
         elif logits2.is_leaf:
             raise RuntimeError("cross_entropy(native) overwrites its input; pass a non-leaf tensor")
-        return _CrossEntropyFn.apply(logits2, t.contiguous(), ignore_index, inv, grad_scale, assume_unit_grad)
+        return _CrossEntropyFn.apply(logits2, t.contiguous(), ignore_index, grad_scale, assume_unit_grad)
     loss = F.cross_entropy(logits2.float(), t, ignore_index=ignore_index)
     return loss * grad_scale if grad_scale != 1.0 else loss
 

@@ -71,6 +71,7 @@ _SIGNATURES = {
     "llmctl_adamw_step": [c_void_p] * 4 + [c_int, c_void_p, c_ll] + [c_float] * 8 + [c_void_p, c_void_p],
     "llmctl_sumsq": [c_void_p, c_int, c_ll, c_void_p, c_int, c_void_p, c_int, c_void_p],
     "llmctl_cross_entropy_fwd_bwd": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_ll, c_float, c_void_p, c_int, c_void_p],
+    "llmctl_cross_entropy_mean": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_ll, c_float, c_int, c_void_p, c_void_p],
     "llmctl_cross_entropy_partial": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_ll, c_void_p],
     "llmctl_cross_entropy_finalize": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_ll, c_ll, c_float, c_void_p, c_void_p],
     "llmctl_gemm_bf16": [c_void_p] * 3 + [c_int] * 3 + [c_ll] * 3 + [c_int] * 6 + [c_void_p],
@@ -245,7 +246,7 @@ def check_waits(context: str = "") -> None:
 
 #: kernels launched per entry point when it is not exactly one
 _KERNELS_PER_CALL = {"llmctl_rmsnorm_bwd": 2, "llmctl_layernorm_bwd": 3, "llmctl_sumsq": 2, "llmctl_rmsnorm_bwd_noalloc": 2,
-                     "llmctl_flash_attn_bwd": 2, "llmctl_rs_sumsq": 2, "llmctl_ag_gemm": 2,
+                     "llmctl_cross_entropy_mean": 3, "llmctl_flash_attn_bwd": 2, "llmctl_rs_sumsq": 2, "llmctl_ag_gemm": 2,
                      "llmctl_comm_watchdog_poll": 0, "llmctl_comm_watchdog_set_timeout_ms": 0}
 
 

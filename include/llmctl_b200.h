@@ -69,6 +69,10 @@ int llmctl_cross_entropy_fwd_bwd(void* logits, long long ld, const long long* ta
                                  float* loss_per_row, float* lse_per_row, int rows, int V,
                                  long long ignore_index, float host_scale, const float* scale_dev,
                                  int write_grad, void* stream);
+/* The mean over rows with another target than ignore_index, times grad_scale (which the gradient takes too, with 1 / count).
+ * work: fp32 [rows + 1] = the rows' losses, 1 / count; loss: fp32 [1]. */
+int llmctl_cross_entropy_mean(void* logits, long long ld, const long long* targets, float* work, int rows, int V, long long ignore_index,
+                              float grad_scale, int write_grad, float* loss, void* stream);
 /* Waits of kernels that ran out (csrc/common/wait_status.h): the host word that they set, one byte per kernel, or NULL; and a kernel that
  * sets byte `which` and does nothing else. */
 void* llmctl_wait_status_word(void);

@@ -176,6 +176,27 @@ def test_cross_entropy_row_lengths(cuda_device, rows, V):
     assert not leaf.grad[::9].any()
 
 
+@pytest.mark.parametrize("rows", [0, 1, 31, 1023, 1024, 1025, 9001])
+def test_cross_entropy_mean(cuda_device, rows):
+    """The mean of the rows' losses: fewer and more rows than the summing block has threads, some or all of them ignored.  A row's loss
+    errs by some 4 units of fp32 of its largest terms (below 16 here), a sum of n numbers by no more than log2(1024) + n / 1024 units."""
+    from llmctl_b200.ops import functional as ops
+    g = torch.Generator(device=cuda_device).manual_seed(rows)
+    base = torch.randn(rows, 64, device=cuda_device, generator=g).bfloat16()
+    t = torch.randint(0, 64, (rows,), device=cuda_device, generator=g)
+    t[::5] = -1
+    for targets, scale in ((t, 0.25), (torch.full_like(t, -1), 1.0)):
+        leaf = base.clone().requires_grad_(True)
+        loss = ops.cross_entropy(leaf * 1.0, targets, ignore_index=-1, grad_scale=scale)
+        loss.backward()
+        ref = base.double().requires_grad_(True)
+        want = scale * F.cross_entropy(ref, targets, ignore_index=-1, reduction="sum") / max(1, int((targets != -1).sum()))
+        want.backward()
+        assert loss.shape == () and loss.dtype == torch.float32
+        assert abs(loss.item() - want.item()) <= 2.0 ** -24 * (4 * 16 + (10 + rows / 1024) * abs(want.item()))
+        assert (leaf.grad.double() - ref.grad).norm() <= 2.0 ** -8.5 * ref.grad.norm()
+
+
 GEMM_SHAPES = [(128, 256, 64), (256, 512, 256), (4096, 4096, 4096), (1000, 2752, 1376), (384, 136, 200),
                (8192, 1024, 512)]
 
