@@ -117,125 +117,94 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   }
 }
 
-// Backward.  blockDim = 256; each thread owns kVec 16-byte column groups: v = i*256 + tid.
-template <int kVec, bool kLayerNorm>
-__global__ void __launch_bounds__(256)
+// Backward.  A CTA takes a row at a time, a thread 16 bytes of it (blockDim = cols / 8 in whole warps).
+// Bound by bytes in flight (three streams read, one written, one block reduction a row): with one 16-byte unit per thread, what is kept
+// across the reduction packed as it was loaded, and one row fetched ahead, 62 registers let 1024 threads stay resident on an SM, 1280 at
+// 640 a CTA.  256 threads with up to four units each needed twice the registers per column (one CTA of 5120 columns per SM).  us of the
+// whole backward before / after (L2 flushed): 8192 x 4096 74.6 / 58.5, 4096 x 5120 72.7 / 47.4, 4096 x 6144 76.8 / 54.5, 512 x 8192
+// 27.3 / 19.4, 8192 x 768 25.5 / 23.5; 2048 columns and small batches alike.
+template <int kThreads, int kCtas, bool kLayerNorm>
+__global__ void __launch_bounds__(kThreads, kCtas)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
                 const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean_in,
                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                 __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial,
                 float* __restrict__ db_partial, int rows, int cols) {
-  wait_for_previous(dy, h, w, mean_in, rstd_in, dres, dx, dw_partial, db_partial);
+  wait_for_previous(dy, h, w, mean_in, rstd_in, dres);     // the others are stored to, not read
   release_dependents();
-  __shared__ float red[32];
-  const int nvec = cols >> 3;
-  float wreg[kVec][8];
-  float dwacc[kVec][8];
-  float dbacc[kLayerNorm ? kVec : 1][8];
+  __shared__ float red[32], red2[32];
+  const int v = threadIdx.x;
+  const bool in = v < (cols >> 3);
+  bf16x8 wv;
+  float dwacc[8], dbacc[kLayerNorm ? 8 : 1];
+  if (in) wv = load8(w + v * 8);
 #pragma unroll
-  for (int i = 0; i < kVec; ++i) {
-    const int v = i * 256 + threadIdx.x;
-    if (v < nvec) unpack8(load8(w + v * 8), wreg[i]);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      dwacc[i][j] = 0.f;
-      if (kLayerNorm) dbacc[i][j] = 0.f;
-    }
+  for (int j = 0; j < 8; ++j) {
+    dwacc[j] = 0.f;
+    if (kLayerNorm) dbacc[j] = 0.f;
   }
-  // Software pipeline over this CTA's rows: the loads of row r+1 (dy, h) and the residual-gradient load of row r
-  // are issued before the block reduction of row r, so two rows of traffic are in flight per CTA instead of one
-  // load -> reduce -> load -> store chain per row (the kernel ran at 36% of HBM bandwidth when it was serial).
-  bf16x8 ndy[kVec], nh[kVec];
-  {
-    const int row0 = blockIdx.x;
-    if (row0 < rows) {
-      const size_t base0 = static_cast<size_t>(row0) * cols;
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        const int v = i * 256 + threadIdx.x;
-        if (v < nvec) {
-          ndy[i] = load8(dy + base0 + v * 8);
-          nh[i] = load8(h + base0 + v * 8);
-        }
-      }
+  // Software pipeline over this CTA's rows: the loads of row r + 1 are issued before the block reduction of row r, so two rows of traffic
+  // are in flight per CTA instead of one load -> reduce -> load -> store chain per row (36% of HBM bandwidth).
+  bf16x8 ndy, nh, nres;
+  float nrstd = 0.f, nmean = 0.f;
+  auto fetch = [&](int row) {
+    if (row >= rows) return;
+    const size_t at = static_cast<size_t>(row) * cols + v * 8;
+    nrstd = rstd_in[row];
+    if (kLayerNorm) nmean = mean_in[row];
+    if (in) {
+      ndy = load8(dy + at);
+      nh = load8(h + at);
+      if (dres != nullptr) nres = load8(dres + at);
     }
-  }
+  };
+  fetch(blockIdx.x);
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const size_t base = static_cast<size_t>(row) * cols;
-    const float rstd = rstd_in[row];
-    const float mean = kLayerNorm ? mean_in[row] : 0.f;
-    float g[kVec][8], xh[kVec][8];
-    bf16x8 rres[kVec];
+    const float rstd = nrstd, mean = nmean;
+    const bf16x8 res = nres, cdy = ndy, ch = nh;             // kept packed: 12 registers instead of 16 for the two products alone
     float c1 = 0.f, c2 = 0.f;
-    if (dres != nullptr) {
+    if (in) {
+      float d[8], a[8], wf[8];
+      unpack8(cdy, d);
+      unpack8(ch, a);
+      unpack8(wv, wf);
 #pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        const int v = i * 256 + threadIdx.x;
-        if (v < nvec) rres[i] = load8(dres + base + v * 8);
+      for (int j = 0; j < 8; ++j) {
+        const float xh = (a[j] - mean) * rstd, g = d[j] * wf[j];
+        c1 += g * xh;
+        c2 += g;
+        dwacc[j] += d[j] * xh;
+        if (kLayerNorm) dbacc[j] += d[j];
       }
     }
-#pragma unroll
-    for (int i = 0; i < kVec; ++i) {
-      const int v = i * 256 + threadIdx.x;
-      if (v < nvec) {
-        float d[8], a[8];
-        unpack8(ndy[i], d);
-        unpack8(nh[i], a);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          xh[i][j] = (a[j] - mean) * rstd;
-          g[i][j] = d[j] * wreg[i][j];
-          c1 += g[i][j] * xh[i][j];
-          c2 += g[i][j];
-          dwacc[i][j] += d[j] * xh[i][j];
-          if (kLayerNorm) dbacc[i][j] += d[j];
-        }
-      }
-    }
-    {
-      const int nrow = row + gridDim.x;
-      if (nrow < rows) {
-        const size_t nbase = static_cast<size_t>(nrow) * cols;
-#pragma unroll
-        for (int i = 0; i < kVec; ++i) {
-          const int v = i * 256 + threadIdx.x;
-          if (v < nvec) {
-            ndy[i] = load8(dy + nbase + v * 8);
-            nh[i] = load8(h + nbase + v * 8);
-          }
-        }
-      }
-    }
+    fetch(row + gridDim.x);
     c1 = block_sum(c1, red) / cols;
-    if (kLayerNorm) c2 = block_sum(c2, red) / cols; else c2 = 0.f;
+    if (kLayerNorm) c2 = block_sum(c2, red2) / cols; else c2 = 0.f;
+    if (in) {
+      float o[8], d[8], a[8], wf[8];
+      unpack8(cdy, d);
+      unpack8(ch, a);
+      unpack8(wv, wf);
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) {
-      const int v = i * 256 + threadIdx.x;
-      if (v < nvec) {
-        float o[8];
+      for (int j = 0; j < 8; ++j) o[j] = rstd * (d[j] * wf[j] - (a[j] - mean) * rstd * c1 - c2);
+      if (dres != nullptr) {
+        float r[8];
+        unpack8(res, r);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rstd * (g[i][j] - xh[i][j] * c1 - c2);
-        if (dres != nullptr) {
-          float r[8];
-          unpack8(rres[i], r);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += r[j];
-        }
-        store8(dx + base + v * 8, pack8(o));
+        for (int j = 0; j < 8; ++j) o[j] += r[j];
       }
+      store8(dx + static_cast<size_t>(row) * cols + v * 8, pack8(o));
     }
   }
-#pragma unroll
-  for (int i = 0; i < kVec; ++i) {
-    const int v = i * 256 + threadIdx.x;
-    if (v < nvec) {
-      float* p = dw_partial + static_cast<size_t>(blockIdx.x) * cols + v * 8;
-      *reinterpret_cast<float4*>(p) = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
-      *reinterpret_cast<float4*>(p + 4) = make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]);
-      if (kLayerNorm && db_partial != nullptr) {
+  if (in) {
+    float* p = dw_partial + static_cast<size_t>(blockIdx.x) * cols + v * 8;
+    *reinterpret_cast<float4*>(p) = make_float4(dwacc[0], dwacc[1], dwacc[2], dwacc[3]);
+    *reinterpret_cast<float4*>(p + 4) = make_float4(dwacc[4], dwacc[5], dwacc[6], dwacc[7]);
+    if constexpr (kLayerNorm) {
+      if (db_partial != nullptr) {
         float* q = db_partial + static_cast<size_t>(blockIdx.x) * cols + v * 8;
-        *reinterpret_cast<float4*>(q) = make_float4(dbacc[i][0], dbacc[i][1], dbacc[i][2], dbacc[i][3]);
-        *reinterpret_cast<float4*>(q + 4) = make_float4(dbacc[i][4], dbacc[i][5], dbacc[i][6], dbacc[i][7]);
+        *reinterpret_cast<float4*>(q) = make_float4(dbacc[0], dbacc[1], dbacc[2], dbacc[3]);
+        *reinterpret_cast<float4*>(q + 4) = make_float4(dbacc[4], dbacc[5], dbacc[6], dbacc[7]);
       }
     }
   }
@@ -295,19 +264,25 @@ static int launch_bwd(const void* dy, const void* h, const void* w, const float*
                       cudaStream_t s) {
   LLMCTL_REQUIRE(cols % 8 == 0 && cols <= 8192 && scratch_rows >= 1);
   if (rows == 0) return 0;
-  const int nvec = cols / 8;
-  const int kv = (nvec + 255) / 256;
+  const int threads = (cols / 8 + 31) / 32 * 32;
   int grid = scratch_rows < rows ? scratch_rows : rows;
   float* dwp = scratch;
   float* dbp = kLN ? scratch + static_cast<size_t>(scratch_rows) * cols : nullptr;
-#define LAUNCH(KV)                                                                            \
-  LLMCTL_CHECK(launch_dependent(norm_bwd_kernel<KV, kLN>, grid, 256, 0, s,                     \
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, mean, rstd, \
-      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dwp, dbp, rows, cols))
-  if (kv <= 1) LAUNCH(1);
-  else if (kv <= 2) LAUNCH(2);
-  else if (kv <= 3) LAUNCH(3);
-  else LAUNCH(4);
+#define LAUNCH(T, N)                                                                            \
+  do {                                                                                          \
+    if (grid > (N) * kNumSMs) grid = (N) * kNumSMs;                                             \
+    LLMCTL_CHECK(launch_dependent(norm_bwd_kernel<T, N, kLN>, grid, threads, 0, s,              \
+        (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, mean, rstd, \
+        (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dwp, dbp, rows, cols));                 \
+  } while (0)
+  // N: the CTAs that an SM holds at the registers left to them.  More only make a second wave and more partials: 4096 x 5120 takes 47.9 us
+  // with 296 CTAs, 54.2 with 444, 50.1 with 592; 512 x 8192 19.3 with 148, 25.6 with 592.  Below 1024 columns the threads are few and four
+  // CTAs may use all the registers they like (4096 x 768: 17.3, 19.3 held to 64).  LayerNorm's second sum has no room in 48 registers.
+  if (threads <= 128) LAUNCH(128, 4);
+  else if (threads <= 256) LAUNCH(256, 4);
+  else if (threads <= 512) LAUNCH(512, 2);
+  else if (threads <= 640) LAUNCH(640, kLN ? 1 : 2);
+  else LAUNCH(1024, 1);
 #undef LAUNCH
   dim3 b2(32, kSumSlices), g2((cols + 31) / 32);
   LLMCTL_CHECK(launch_dependent(colsum_kernel, g2, b2, 0, s, dwp, dw, grid, cols, accumulate));

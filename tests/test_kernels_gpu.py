@@ -132,6 +132,32 @@ def test_sumsq(cuda_device):
     assert abs(out.item() - ref.item()) / ref.item() < 1e-4
 
 
+# both sides of every line of the backward (128 | 256 | 512 | 640 | 1024 threads of 8 columns), fewer and more rows than CTAs
+@pytest.mark.parametrize("rows,cols", [(1, 8), (700, 264), (1500, 1024), (601, 1032), (1300, 2048), (150, 2056), (800, 4096), (297, 4104), (600, 5120),
+                                       (149, 5128), (5, 8184), (400, 8192)])
+@pytest.mark.parametrize("layer,with_res", [(False, True), (False, False), (True, True)])
+def test_norm_backward_row_lengths(cuda_device, rows, cols, layer, with_res):
+    """Gradients against float64 from the same inputs: dx is rounded to bf16 once (2^-9 a number), the weights' sums are fp32 and rounded
+    to bf16 at the end; x + r is rounded to bf16 before the norm, which the reference does too."""
+    from llmctl_b200.ops import functional as ops
+    g = torch.Generator(device=cuda_device).manual_seed(rows + cols)
+    rand = lambda *s: torch.randn(*s, device=cuda_device, generator=g).bfloat16()      # noqa: E731
+    x, r, w, b, dy, dh = rand(rows, cols), rand(rows, cols), rand(cols), rand(cols), rand(rows, cols), rand(rows, cols)
+    leaves = [t.clone().requires_grad_(True) for t in (x, w, b)]
+    res = r if with_res else None
+    y, h = ops.layernorm(*leaves, 1e-5, res) if layer else ops.rmsnorm(*leaves[:2], 1e-5, res)
+    torch.autograd.backward([y, h] if with_res else [y], [dy, dh] if with_res else [dy])
+    want = [t.double().requires_grad_(True) for t in (x + r if with_res else x, w, b)]
+    hd = want[0] * 1
+    yd = F.layer_norm(hd, (cols,), want[1], want[2], 1e-5) if layer else hd * (hd.pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt() * want[1]
+    torch.autograd.backward([yd, hd] if with_res else [yd], [dy.double(), dh.double()] if with_res else [dy.double()])
+    for a, e in list(zip(leaves, want))[:3 if layer else 2]:
+        bound = 2.0 ** -8 * e.grad.norm()
+        if not with_res and rows * cols <= 8:       # dx of one short row is a difference of near numbers: fp32 of its terms
+            bound = bound + 2.0 ** -20 * dy.double().norm() * w.double().norm()
+        assert (a.grad.double() - e.grad).norm() <= bound
+
+
 @pytest.mark.parametrize("rows,V", [(128, 32000), (1024, 32768), (64, 4096), (32, 50304)])
 def test_cross_entropy(cuda_device, rows, V):
     from llmctl_b200.ops import functional as ops
