@@ -89,7 +89,8 @@ def rebuild_pays(q: torch.Tensor, dn: int, dr: int, dv: int, R: int, heads: int,
     ``REBUILD_PAIRS`` visible (query, key) pairs per rebuilt row.  A pair costs a head 1088 products at the absorbed kernel's rate or 320 at four times that
     rate, a rebuilt row 131072 at five times that rate: the line is near 26 pairs a row.  Layer of 16 heads, us absorbed / rebuilt: one prompt of
     48 tokens 74.4 / 74.6, 64 (16 pairs a row) 72.9 / 74.7, 80 (25 pairs) 76.7 / 74.7, 128 97.2 / 74.8, 512 218 / 85, 2 x 2048 937 / 179;
-    behind 4000 cached tokens 24 tokens 181 / 136, 128 232 / 140, 512 519 / 161."""
+    behind 4000 cached tokens 24 tokens 181 / 136, 128 232 / 140, 512 519 / 161 (launches that overlap took 10-20 us off either side
+    since: 2 x 2048 rebuilt 156)."""
     return (q.is_cuda and q.dtype == torch.bfloat16 and (dn, dr, dv) == (128, 64, 128) and uses_tensor_cores(q.dtype, R, dr)
             and q.stride(1) == 1 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and key_rows > 0 and pairs >= REBUILD_PAIRS * key_rows
             and 2 * key_rows * (heads * (dn + dv) + R + dr) <= REBUILD_BYTES and native.has_symbol("llmctl_latent_prompt_attention"))
