@@ -53,6 +53,12 @@ namespace llmctl {
 
 constexpr int kNumSMs = 148;
 
+// Whether kernels may read or write whole 16-byte units at these addresses (null: not used).
+template <typename... P>
+inline bool aligned16(P... p) {
+  return ((uintptr_t(0) | ... | reinterpret_cast<uintptr_t>(p)) & 15) == 0;
+}
+
 struct __align__(16) bf16x8 {
   __nv_bfloat162 v[4];
 };

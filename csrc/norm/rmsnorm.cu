@@ -240,6 +240,7 @@ static int launch_fwd(const void* x, const void* residual, const void* w, const 
                       cudaStream_t s) {
   LLMCTL_REQUIRE(cols % 8 == 0 && cols <= 8192 && rows >= 0);
   if (rows == 0) return 0;
+  LLMCTL_REQUIRE(aligned16(x, residual, w, b, h_out, y));
   const int nvec = cols / 8;
   const int per_lane = (nvec + 31) / 32;
   dim3 block(128), grid((rows + 3) / 4);
@@ -264,6 +265,7 @@ static int launch_bwd(const void* dy, const void* h, const void* w, const float*
                       cudaStream_t s) {
   LLMCTL_REQUIRE(cols % 8 == 0 && cols <= 8192 && scratch_rows >= 1);
   if (rows == 0) return 0;
+  LLMCTL_REQUIRE(aligned16(dy, h, w, dres, dx, scratch));
   const int threads = (cols / 8 + 31) / 32 * 32;
   int grid = scratch_rows < rows ? scratch_rows : rows;
   float* dwp = scratch;
@@ -378,6 +380,11 @@ LLMCTL_API int llmctl_rmsnorm_bwd_noalloc(const void* dy, const void* h, const v
              "llmctl_rmsnorm_bwd_noalloc: cols=%d rows=%d not supported: cols must be a positive multiple of 8 "
              "and at most %d (the built-in scratch holds %d x %d floats)",
              cols, rows, kNoAllocMaxCols, kNoAllocCtas, kNoAllocMaxCols);
+    fprintf(stderr, "[llmctl] %s\n", g_noalloc_err);
+    return static_cast<int>(cudaErrorInvalidValue);
+  }
+  if (rows > 0 && !aligned16(dy, h, w, dres, dx)) {
+    snprintf(g_noalloc_err, sizeof(g_noalloc_err), "llmctl_rmsnorm_bwd_noalloc: dy, h, w, dres and dx must lie on 16-byte boundaries");
     fprintf(stderr, "[llmctl] %s\n", g_noalloc_err);
     return static_cast<int>(cudaErrorInvalidValue);
   }

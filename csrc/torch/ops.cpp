@@ -111,6 +111,11 @@ bool is_plain(const Tensor& t) {
 }
 bool bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16; }
 bool unit16(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0; }
+// contiguous from a 16-byte boundary, as the kernels read it
+Tensor whole_units(const Tensor& t) {
+  const Tensor c = t.contiguous();
+  return unit16(c) ? c : c.clone();
+}
 // an operand of the GEMMs: rows of whole 16-byte units
 bool is_matrix(const Tensor& t) { return bf16(t) && t.dim() == 2 && t.stride(1) == 1 && t.stride(0) % 8 == 0 && unit16(t); }
 bool recorded(std::initializer_list<const Tensor*> ts) {
@@ -215,10 +220,10 @@ struct RmsNorm : torch::autograd::Function<RmsNorm> {
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     return node_body("llmctl_rmsnorm_bwd", ready(lib.llmctl_rmsnorm_bwd), [&]() -> torch::autograd::variable_list {
       const auto saved = ctx->get_saved_variables();
-      const Tensor &h = saved[0], &w = saved[1], &rstd = saved[2];
+      const Tensor h = whole_units(saved[0]), w = whole_units(saved[1]), &rstd = saved[2];
       const bool residual = ctx->saved_data["residual"].toBool();
       const int64_t cols = h.size(-1), rows = h.numel() / cols;
-      const Tensor dy = grads[0].contiguous(), dres = residual ? grads[1].contiguous() : Tensor();
+      const Tensor dy = whole_units(grads[0]), dres = residual ? whole_units(grads[1]) : Tensor();
       Tensor dx = new_bf16(h, h.sizes()), dw = new_f32(h, {cols});
       const int ctas = static_cast<int>(rows < kNormBwdCtas ? rows : kNormBwdCtas);
       Tensor scratch = new_f32(h, {ctas * cols});
@@ -398,8 +403,7 @@ AttnOut attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, double scale
 // dq | dk | dv, packed like the projection that made q | k | v, so that the weight gradient that follows sees one tensor
 Tensor attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& grad, double scale, bool causal) {
   const int64_t B = q.size(0), S = q.size(1), H = q.size(2), D = q.size(3);
-  Tensor d_o = grad.contiguous();
-  if (!unit16(d_o)) d_o = d_o.clone();
+  const Tensor d_o = whole_units(grad);
   Tensor d = new_bf16(q, {B, S, 3, H, D});
   Tensor scratch = new_f32(q, {2 * B * H * ((S + 127) / 128 * 128) + 2});
   char* at = static_cast<char*>(data(d));

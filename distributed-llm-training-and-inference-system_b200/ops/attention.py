@@ -18,7 +18,7 @@ import torch
 import torch.nn.functional as F
 
 from . import native
-from .functional import kernel_config
+from .functional import _whole_units, kernel_config
 
 c_void_p, c_int, c_ll, c_float = native.c_void_p, native.c_int, native.c_ll, native.c_float
 
@@ -59,12 +59,6 @@ def _native_ok(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool =
 def _stats_scratch(B: int, S: int, H: int, device: torch.device) -> torch.Tensor:
     """Scratch of the backward: two numbers per (head, query), sequences rounded up to whole tiles, and the item counter (in two words)."""
     return torch.empty(2 * B * H * ((S + 127) // 128 * 128) + 2, dtype=torch.float32, device=device)
-
-
-def _whole_units(t: torch.Tensor) -> torch.Tensor:
-    """``t`` contiguous from a 16-byte boundary, as the backward kernels read it."""
-    t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 class _FlashAttnFn(torch.autograd.Function):

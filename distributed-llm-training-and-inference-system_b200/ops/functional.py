@@ -77,6 +77,12 @@ def _scratch(device: torch.device, nfloats: int, tag: str = "") -> torch.Tensor:
     return buf
 
 
+def _whole_units(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous from a 16-byte boundary, as the kernels read it."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 _NORM_BWD_CTAS = 148 * 4
 
 
@@ -90,13 +96,10 @@ class _RMSNormFn(torch.autograd.Function):
     def forward(ctx, x, residual, w, eps):
         shape = x.shape
         cols = shape[-1]
-        x2 = x.reshape(-1, cols)
-        x2 = x2 if x2.is_contiguous() else x2.contiguous()
+        x2 = _whole_units(x.reshape(-1, cols))
         rows = x2.shape[0]
-        r2 = None
-        if residual is not None:
-            r2 = residual.reshape(-1, cols)
-            r2 = r2 if r2.is_contiguous() else r2.contiguous()
+        r2 = None if residual is None else _whole_units(residual.reshape(-1, cols))
+        w = _whole_units(w)
         y = torch.empty_like(x2)
         h = torch.empty_like(x2) if r2 is not None else x2
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
@@ -116,12 +119,8 @@ class _RMSNormFn(torch.autograd.Function):
     def backward(ctx, dy, dh):
         h, w, rstd = ctx.saved_tensors
         rows, cols = h.shape
-        dy2 = dy.reshape(rows, cols)
-        dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
-        dres = None
-        if dh is not None and ctx.has_res:
-            dres = dh.reshape(rows, cols)
-            dres = dres if dres.is_contiguous() else dres.contiguous()
+        dy2 = _whole_units(dy.reshape(rows, cols))
+        dres = _whole_units(dh.reshape(rows, cols)) if dh is not None and ctx.has_res else None
         dx = torch.empty_like(h)
         dw = torch.empty(cols, dtype=torch.float32, device=h.device)
         nct = min(_NORM_BWD_CTAS, rows)
@@ -155,14 +154,15 @@ class _LayerNormFn(torch.autograd.Function):
     def forward(ctx, x, residual, w, b, eps):
         shape = x.shape
         cols = shape[-1]
-        x2 = x.reshape(-1, cols).contiguous()
+        x2 = _whole_units(x.reshape(-1, cols))
         rows = x2.shape[0]
-        r2 = residual.reshape(-1, cols).contiguous() if residual is not None else None
+        r2 = _whole_units(residual.reshape(-1, cols)) if residual is not None else None
+        w, b2 = _whole_units(w), None if b is None else _whole_units(b)
         y = torch.empty_like(x2)
         h = torch.empty_like(x2) if r2 is not None else x2
         mean = torch.empty(rows, dtype=torch.float32, device=x.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        native.call("llmctl_layernorm_fwd", x2.data_ptr(), native.ptr(r2), w.data_ptr(), native.ptr(b),
+        native.call("llmctl_layernorm_fwd", x2.data_ptr(), native.ptr(r2), w.data_ptr(), native.ptr(b2),
                     h.data_ptr() if r2 is not None else None, y.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
                     rows, cols, float(eps), native.stream_ptr())
         ctx.save_for_backward(h, w, mean, rstd)
@@ -177,8 +177,8 @@ class _LayerNormFn(torch.autograd.Function):
     def backward(ctx, dy, dh):
         h, w, mean, rstd = ctx.saved_tensors
         rows, cols = h.shape
-        dy2 = dy.reshape(rows, cols).contiguous()
-        dres = dh.reshape(rows, cols).contiguous() if (dh is not None and ctx.has_res) else None
+        dy2 = _whole_units(dy.reshape(rows, cols))
+        dres = _whole_units(dh.reshape(rows, cols)) if (dh is not None and ctx.has_res) else None
         dx = torch.empty_like(h)
         dw = torch.empty(cols, dtype=torch.float32, device=h.device)
         db = torch.empty(cols, dtype=torch.float32, device=h.device)

@@ -17,7 +17,8 @@ extern "C" {
 #endif
 
 /* ---- K3 norms.  Reference: ATen rms_norm/layer_norm inside HF modules (engine.py:284). ---- */
-/* h = x (+ residual); y = h * rsqrt(mean(h^2) + eps) * w.  h_out/residual/rstd may be NULL. */
+/* h = x (+ residual); y = h * rsqrt(mean(h^2) + eps) * w.  h_out/residual/rstd may be NULL.  The norms' bf16 operands and their
+ * scratch lie on 16-byte boundaries (else cudaErrorInvalidValue). */
 int llmctl_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* h_out, void* y,
                        float* rstd, int rows, int cols, float eps, void* stream);
 /* dx = d(norm)/dh (+ dres); dw (fp32) (+)= sum_rows dy * xhat.

@@ -70,10 +70,11 @@ def test_rmsnorm(ops, shape, form, grad):
         pytest.skip("one size is enough")
 
     def run():
-        x = _randn(*shape, shift=8 if form == "odd" else 0)
+        odd = 1 if form == "odd" else 0
+        x = _randn(*shape, shift=odd)
         if form == "strided":
             x = torch.stack([x, x], -1)[..., 0]
-        r = _randn(*shape, seed=1) if form != "plain" else None
+        r = _randn(*shape, seed=1, shift=odd) if form != "plain" else None
         w = (1 + _randn(shape[-1], seed=2)).requires_grad_(grad)
         leaves = [w]
         for t in (x, r):
@@ -84,11 +85,31 @@ def test_rmsnorm(ops, shape, form, grad):
         if not grad:
             assert not y.requires_grad
             return y, h
-        dy, dh = _randn(*shape, seed=3), _randn(*shape, seed=4)
+        dy, dh = _randn(*shape, seed=3, shift=odd), _randn(*shape, seed=4, shift=odd)
         outs, grads = ((y, h), (dy, dh)) if r is not None else ((y,), (dy,))
         one = torch.autograd.grad(y, leaves, dy, retain_graph=True)        # the other output's gradient is missing
         return (y.detach(), h.detach(), *one, *torch.autograd.grad(outs, leaves, grads))
     _both(run)
+
+
+@pytest.mark.parametrize("layer", [False, True])
+@pytest.mark.parametrize("odd", ["x", "residual", "w", "b", "dy", "dh"])
+def test_norms_at_odd_addresses(ops, layer, odd):
+    """Operands and gradients that begin inside a 16-byte unit are copied: the same bits as from whole units, on either side."""
+    if odd == "b" and not layer:
+        pytest.skip("no bias")
+
+    def run(odd):
+        def t(name, *shape, seed):
+            v, at = _randn(*shape, seed=seed), 1 if name == odd else 0
+            return torch.empty(v.numel() + 1, device="cuda", dtype=v.dtype)[at:][:v.numel()].view(shape).copy_(v).requires_grad_(name not in ("dy", "dh"))
+        leaves = [t("x", 37, 768, seed=0), t("residual", 37, 768, seed=1), t("w", 768, seed=2)] + ([t("b", 768, seed=3)] if layer else [])
+        if layer:
+            y, h = ops.layernorm(leaves[0], leaves[2], leaves[3], residual=leaves[1])
+        else:
+            y, h = ops.rmsnorm(leaves[0], leaves[2], residual=leaves[1])
+        return (y.detach(), h.detach(), *torch.autograd.grad((y, h), leaves, (t("dy", 37, 768, seed=4), t("dh", 37, 768, seed=5))))
+    _same(_both(lambda: run(odd)), run(""))
 
 
 @pytest.mark.parametrize("shape,n", [((1, 64), 8), ((32, 256), 64), ((33, 256), 64), ((2, 50, 128), 24), ((300, 72), 40), ((2, 3, 64), 20)])
