@@ -306,9 +306,10 @@ Tensor as_shape_of(const Tensor& y, const Tensor& x) {
   return y.view(size);
 }
 
-// linear(x, w, tile_n, workspace or None, counters) -> x @ w.T where no gradient is recorded; few rows take the decode GEMM if there is a workspace
+// linear(x, w, tile_n, workspace or None) -> x @ w.T where no gradient is recorded; few rows take the decode GEMM, whose partials and tickets
+// workspace(x) returns
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return call(a, n, 5, [&](Args& args) -> PyObject* {
+  return call(a, n, 4, [&](Args& args) -> PyObject* {
     const Tensor x = args.tensor(0), w = args.tensor(1);
     const int tile_n = static_cast<int>(args.integer(2));
     if (!args.ok || !quiet() || !is_matrix(w) || x.numel() == 0 || recorded({&x, &w})) return none();
@@ -316,8 +317,14 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!rows.defined() || rows.size(1) != w.size(1)) return none();
     const bool skinny = a[3] != Py_None;
     if (skinny ? !ready(lib.llmctl_gemm_skinny_bf16) : !ready(lib.llmctl_gemm_bf16) || w.size(0) % 8) return none();
-    const Tensor ws = skinny ? args.tensor(3) : Tensor(), counters = skinny ? args.tensor(4) : Tensor();
-    if (!args.ok) return none();
+    Tensor ws, counters;
+    if (skinny) {
+      PyObject* pair = PyObject_CallOneArg(a[3], a[0]);
+      if (pair == nullptr) throw python_error();
+      ws = THPVariable_Unpack(PyTuple_GET_ITEM(pair, 0));
+      counters = THPVariable_Unpack(PyTuple_GET_ITEM(pair, 1));
+      Py_DECREF(pair);
+    }
     Tensor y = without_gil([&] {
       Tensor out = new_bf16(x, {rows.size(0), w.size(0)});
       if (skinny)

@@ -400,14 +400,14 @@ _skinny_ws: dict = {}
 SKINNY_MAX_ROWS = 32
 
 
-def _skinny_workspace(device: torch.device):
+def _skinny_workspace(x: torch.Tensor):
     """Per-device split-K scratch of the skinny GEMM (fp32 partials + zeroed ticket counters).  Calls are serialised
     by the stream they run on; the decode engine uses one stream."""
-    key = (device.index if device.index is not None else torch.cuda.current_device())
+    key = x.device.index
     ws = _skinny_ws.get(key)
     if ws is None:
-        ws = _skinny_ws[key] = (torch.empty(8 << 20, dtype=torch.float32, device=device),
-                                torch.zeros(4096, dtype=torch.int32, device=device))
+        ws = _skinny_ws[key] = (torch.empty(8 << 20, dtype=torch.float32, device=x.device),
+                                torch.zeros(4096, dtype=torch.int32, device=x.device))
     return ws
 
 
@@ -418,7 +418,7 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
     assert M <= SKINNY_MAX_ROWS and w.shape[1] == K and x.stride(1) == 1 and w.stride(1) == 1
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
-    ws, cnt = _skinny_workspace(x.device)
+    ws, cnt = _skinny_workspace(x)
     native.call("llmctl_gemm_skinny_bf16", x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), w.stride(0),
                 out.stride(0), ws.data_ptr(), ws.numel(), cnt.data_ptr(), cnt.numel(), splits, native.stream_ptr())
     return out
@@ -428,8 +428,7 @@ def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """``x @ w.T`` (no bias).  x: [..., K], w: [N, K]."""
     gate = getattr(w, "_k8_gate", None)
     if gate is None and _cfg.gemm == "native" and x.is_cuda:
-        ws = _skinny_workspace(x.device) if _cfg.skinny_gemm and x.numel() <= SKINNY_MAX_ROWS * x.shape[-1] else (None, None)
-        y = native.fast.linear(x, w, _cfg.gemm_tile_n, *ws)
+        y = native.fast.linear(x, w, _cfg.gemm_tile_n, _skinny_workspace if _cfg.skinny_gemm and x.numel() <= SKINNY_MAX_ROWS * x.shape[-1] else None)
         if y is not None:
             return y
     if gate is not None and not (_use_native(x, "gemm") and w.dtype == torch.bfloat16 and x.reshape(-1, x.shape[-1]).shape[0] > SKINNY_MAX_ROWS

@@ -133,6 +133,19 @@ def test_linear(ops, shape, n, form, grad):
     _both(run)
 
 
+def test_linear_makes_the_decode_workspace_where_it_runs(ops, monkeypatch):
+    """Calls that the decode GEMM does not take ask for none of its memory."""
+    monkeypatch.setattr(ops, "_skinny_ws", {})
+    x, w = _randn(4, 64), _randn(48, 64, seed=1)
+    ops.linear(x.float(), w.float())
+    ops.linear(_randn(40, 64), w)
+    ops.linear(x, w.detach().requires_grad_(True))
+    ops.linear(x, _randn(48, 64, shift=1))
+    assert not ops._skinny_ws
+    ops.linear(x, w)
+    assert len(ops._skinny_ws) == 1
+
+
 @pytest.mark.parametrize("rows,width,ffn", [(1, 64, 64), (32, 128, 64), (33, 128, 64), (200, 1024, 256), (130, 256, 96)])
 @pytest.mark.parametrize("grad", [False, True])
 def test_mlp(ops, rows, width, ffn, grad):
