@@ -236,36 +236,66 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
 using namespace llmctl;
 
+namespace llmctl {
+namespace skinny {
+// k blocks per CTA and the floats of scratch that its pieces of tiles take
+struct Plan {
+  int MB, n_tiles, num_kb;
+  long long total, L;
+  Plan(int Mb, int N, int K, int splits) {
+    MB = Mb <= 16 ? 16 : 32;
+    n_tiles = (N + kBM - 1) / kBM;
+    num_kb = (K + kBK - 1) / kBK;
+    total = static_cast<long long>(n_tiles) * num_kb;
+    // `splits` > 0 forces num_kb / splits (tests); otherwise an even share of all SMs, but never less than 8 blocks (128 KB of weights) so
+    // small layers are not shredded
+    if (splits > 0) {
+      L = (num_kb + splits - 1) / splits;
+    } else {
+      L = (total + kNumSMs - 1) / kNumSMs;
+      if (L < 8) L = 8;
+    }
+  }
+  long long slots() const { return (num_kb + L - 1) / L + 1; }
+  long long scratch() const { return n_tiles * slots() * MB * kBM; }
+};
+}  // namespace skinny
+}  // namespace llmctl
+
+// Floats of `workspace` with which llmctl_gemm_skinny_bf16 splits K as it would like to.
+LLMCTL_API long long llmctl_gemm_skinny_scratch_elems(int Mb, int N, int K, int splits) {
+  if (Mb < 1 || Mb > 32 || N < 1 || K < 1) return 0;
+  return skinny::Plan(Mb, N, K, splits).scratch();
+}
+
+// The id of the capture that the stream is part of, 0 if it is not being captured.
+LLMCTL_API unsigned long long llmctl_stream_capture_id(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id) != cudaSuccess || status != cudaStreamCaptureStatusActive) return 0;
+  return id;
+}
+
 // C[Mb, N] (bf16, row stride ldc) = X[Mb, K] (row stride ldx) . W[N, K]^T (row stride ldw), 1 <= Mb <= 32.
 // workspace: fp32 scratch for split-K partials (workspace_elems floats); counters: n_counters zero-initialised
 // uint32 tickets (>= ceil(N/128)), left zero again on return.  One call at a time per (workspace, counters)
-// pair: calls on the same stream are fine, concurrent streams need their own pair.  splits <= 0 picks it.
+// pair: calls on the same stream are fine, concurrent streams need their own pair, and so does a graph that is replayed
+// beside other work.  splits <= 0 picks it.
 LLMCTL_API int llmctl_gemm_skinny_bf16(const void* X, const void* W, void* C, int Mb, int N, int K, long long ldx,
                                        long long ldw, long long ldc, float* workspace, long long workspace_elems,
                                        unsigned int* counters, int n_counters, int splits, void* stream) {
   LLMCTL_BEGIN();
   LLMCTL_REQUIRE(Mb >= 1 && Mb <= 32 && N >= 1 && K >= 8 && K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0);
-  const int MB = Mb <= 16 ? 16 : 32;
-  const int n_tiles = (N + skinny::kBM - 1) / skinny::kBM;
-  const int num_kb = (K + skinny::kBK - 1) / skinny::kBK;
-  const long long total = static_cast<long long>(n_tiles) * num_kb;
+  skinny::Plan plan(Mb, N, K, splits);
+  const int MB = plan.MB, n_tiles = plan.n_tiles, num_kb = plan.num_kb;
   const bool have_ws = workspace != nullptr && counters != nullptr && n_counters >= n_tiles;
-  // k blocks per CTA: `splits` > 0 forces num_kb / splits (tests); otherwise an even share of all SMs, but
-  // never less than 8 blocks (128 KB of weights) so small layers are not shredded
-  long long L;
-  if (splits > 0) {
-    L = (num_kb + splits - 1) / splits;
-  } else {
-    L = (total + kNumSMs - 1) / kNumSMs;
-    if (L < 8) L = 8;
-  }
-  auto slots_for = [&](long long l) { return (num_kb + l - 1) / l + 1; };
-  if (!have_ws || static_cast<long long>(n_tiles) * slots_for(L) * MB * skinny::kBM > workspace_elems) {
+  if (!have_ws || plan.scratch() > workspace_elems) {
     // no (or too little) scratch: whole tiles per CTA, no fix-up needed
     const long long tiles_per_cta = (n_tiles + kNumSMs - 1) / kNumSMs;
-    L = tiles_per_cta * num_kb;
+    plan.L = tiles_per_cta * num_kb;
   }
-  const int max_slots = static_cast<int>(slots_for(L));
+  const long long L = plan.L, total = plan.total;
+  const int max_slots = static_cast<int>(plan.slots());
   const unsigned grid = static_cast<unsigned>((total + L - 1) / L);
   CUtensorMap tw, tx;
   int rc = get_tmap_2d_bf16(&tw, W, N, K, ldw, skinny::kBM, skinny::kBK, 1);

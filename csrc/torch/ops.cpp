@@ -36,7 +36,7 @@ using at::Tensor;
 // ---------------------------------------------------------------------------------------------------------------------------------
 #define LLMCTL_ENTRIES(X)                                                                                                         \
   X(llmctl_rmsnorm_fwd) X(llmctl_rmsnorm_bwd) X(llmctl_rope_inplace) X(llmctl_gemm_bf16) X(llmctl_gemm_swiglu_bf16)               \
-  X(llmctl_gemm_swiglu_bwd_bf16) X(llmctl_gemm_skinny_bf16) X(llmctl_flash_attn_fwd) X(llmctl_flash_attn_bwd) X(llmctl_kv_append) \
+  X(llmctl_gemm_swiglu_bwd_bf16) X(llmctl_gemm_skinny_bf16) X(llmctl_gemm_skinny_scratch_elems) X(llmctl_flash_attn_fwd) X(llmctl_flash_attn_bwd) X(llmctl_kv_append) \
   X(llmctl_paged_attn_decode) X(llmctl_paged_attn_scratch_elems)
 struct Entries {
 #define X(name) decltype(&::name) name = nullptr;
@@ -307,7 +307,7 @@ Tensor as_shape_of(const Tensor& y, const Tensor& x) {
 }
 
 // linear(x, w, tile_n, workspace or None) -> x @ w.T where no gradient is recorded; few rows take the decode GEMM, whose partials and tickets
-// workspace(x) returns
+// workspace(x, floats of partials) returns
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return call(a, n, 4, [&](Args& args) -> PyObject* {
     const Tensor x = args.tensor(0), w = args.tensor(1);
@@ -316,10 +316,11 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor rows = as_rows(x);
     if (!rows.defined() || rows.size(1) != w.size(1)) return none();
     const bool skinny = a[3] != Py_None;
-    if (skinny ? !ready(lib.llmctl_gemm_skinny_bf16) : !ready(lib.llmctl_gemm_bf16) || w.size(0) % 8) return none();
+    if (skinny ? !ready(lib.llmctl_gemm_skinny_bf16) || !lib.llmctl_gemm_skinny_scratch_elems : !ready(lib.llmctl_gemm_bf16) || w.size(0) % 8) return none();
     Tensor ws, counters;
     if (skinny) {
-      PyObject* pair = PyObject_CallOneArg(a[3], a[0]);
+      PyObject* pair = PyObject_CallFunction(a[3], "OL", a[0], lib.llmctl_gemm_skinny_scratch_elems(static_cast<int>(rows.size(0)), static_cast<int>(w.size(0)),
+                                                                                                     static_cast<int>(w.size(1)), 0));
       if (pair == nullptr) throw python_error();
       ws = THPVariable_Unpack(PyTuple_GET_ITEM(pair, 0));
       counters = THPVariable_Unpack(PyTuple_GET_ITEM(pair, 1));

@@ -14,6 +14,7 @@ can attribute speed-ups.
 """
 from __future__ import annotations
 
+import threading
 from dataclasses import dataclass
 from typing import Optional, Tuple
 
@@ -396,18 +397,41 @@ class _LinearFn(torch.autograd.Function):
         return dx, dw
 
 
-_skinny_ws: dict = {}
 SKINNY_MAX_ROWS = 32
+_SKINNY_ELEMS = 8 << 20         # most floats of partials: beyond, the kernel gives whole tiles to its CTAs
+_SKINNY_TICKETS = 4096
+_SKINNY_STREAMS = 16
+_skinny_ws: dict = {}           # (device, stream) -> (partials, tickets), oldest first
+_skinny_captures: dict = {}     # (device, stream) -> (capture, tickets)
+_skinny_lock = threading.Lock()
 
 
-def _skinny_workspace(x: torch.Tensor):
-    """Per-device split-K scratch of the skinny GEMM (fp32 partials + zeroed ticket counters).  Calls are serialised
-    by the stream they run on; the decode engine uses one stream."""
-    key = x.device.index
+def _skinny_workspace(x: torch.Tensor, elems: int):
+    """Split-K scratch of the skinny GEMM for a call on the current stream: at least ``elems`` fp32 partials (or too few, beyond
+    ``_SKINNY_ELEMS``) and zeroed tickets.  Calls on one stream follow one another and share a pair, kept for the last ``_SKINNY_STREAMS``
+    streams that asked; what is dropped goes back to its stream's pool behind that stream's work.  A captured call may be replayed beside
+    anything, another graph of the same stream too: its partials come from the graph's pool, and the tickets of a capture are zeroed by
+    the graph itself."""
+    elems = min(max(elems, 1), _SKINNY_ELEMS)
+    stream = native.stream_ptr()
+    key = (x.device.index, stream)
+    if torch.cuda.is_current_stream_capturing():
+        capture = native.lib().llmctl_stream_capture_id(stream)
+        with _skinny_lock:
+            made = _skinny_captures.get(key)
+            if made is None or made[0] != capture:
+                made = _skinny_captures[key] = (capture, torch.zeros(_SKINNY_TICKETS, dtype=torch.int32, device=x.device))
+        return torch.empty(elems, dtype=torch.float32, device=x.device), made[1]
     ws = _skinny_ws.get(key)
-    if ws is None:
-        ws = _skinny_ws[key] = (torch.empty(8 << 20, dtype=torch.float32, device=x.device),
-                                torch.zeros(4096, dtype=torch.int32, device=x.device))
+    if ws is None or ws[0].numel() < elems:
+        with _skinny_lock:
+            ws = _skinny_ws.pop(key, None)
+            if ws is None or ws[0].numel() < elems:
+                tickets = torch.zeros(_SKINNY_TICKETS, dtype=torch.int32, device=x.device) if ws is None else ws[1]
+                ws = (torch.empty(min(_SKINNY_ELEMS, -(-elems >> 20) << 20), dtype=torch.float32, device=x.device), tickets)
+            while len(_skinny_ws) >= _SKINNY_STREAMS:
+                del _skinny_ws[next(iter(_skinny_ws))]
+            _skinny_ws[key] = ws
     return ws
 
 
@@ -418,7 +442,7 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
     assert M <= SKINNY_MAX_ROWS and w.shape[1] == K and x.stride(1) == 1 and w.stride(1) == 1
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
-    ws, cnt = _skinny_workspace(x)
+    ws, cnt = _skinny_workspace(x, native.lib().llmctl_gemm_skinny_scratch_elems(M, N, K, splits))
     native.call("llmctl_gemm_skinny_bf16", x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), w.stride(0),
                 out.stride(0), ws.data_ptr(), ws.numel(), cnt.data_ptr(), cnt.numel(), splits, native.stream_ptr())
     return out

@@ -78,9 +78,12 @@ _SIGNATURES = {
     "llmctl_gemm_bf16_bgated": [c_void_p] * 3 + [c_int] * 3 + [c_ll] * 3 + [c_int] * 6 + [c_void_p, ctypes.c_uint, c_ll, c_ll, c_void_p],
     "llmctl_gemm_swiglu_bf16": [c_void_p] * 4 + [c_int] * 3 + [c_ll] * 4 + [c_void_p],
     "llmctl_gemm_swiglu_bwd_bf16": [c_void_p] * 4 + [c_int] * 3 + [c_ll] * 3 + [c_void_p],
+    "llmctl_gemm_skinny_scratch_elems": [c_int] * 4,
+    "llmctl_stream_capture_id": [c_void_p],
     "llmctl_gemm_skinny_bf16": [c_void_p] * 3 + [c_int] * 3 + [c_ll] * 3 + [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p],
 }
-_RESULTS: dict = {}         # result types by name; int for the rest
+# result types by name; int for the rest
+_RESULTS: dict = {"llmctl_gemm_skinny_scratch_elems": c_ll, "llmctl_stream_capture_id": ctypes.c_ulonglong}
 
 
 def library_path() -> Path:

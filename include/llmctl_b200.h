@@ -124,11 +124,16 @@ int llmctl_gemm_swiglu_bwd_bf16(const void* DY, const void* W, const void* GU, v
 
 /* ---- K0s skinny (decode) GEMM: C[Mb,N] = X[Mb,K] W[N,K]^T, 1 <= Mb <= 32.  Swap-AB (UMMA M = 128 weight rows,
  * N = 16/32 token rows), split-K over CTAs with a deterministic in-kernel fix-up.  workspace: fp32 scratch;
- * counters: >= ceil(N/128) zeroed uint32 tickets (left zero on return); one call at a time per pair.
+ * counters: >= ceil(N/128) zeroed uint32 tickets (left zero on return); one call at a time per pair: a stream's calls may share one,
+ * streams that run beside each other and graphs that are replayed need their own.
+ * llmctl_gemm_skinny_scratch_elems: floats of workspace with which K is split freely; with fewer, CTAs take whole tiles.
+ * llmctl_stream_capture_id: the capture that a stream is part of, or 0.
  * Reference: cuBLAS inside the HF model (server.py:199-204). */
 int llmctl_gemm_skinny_bf16(const void* X, const void* W, void* C, int Mb, int N, int K, long long ldx,
                             long long ldw, long long ldc, float* workspace, long long workspace_elems,
                             unsigned int* counters, int n_counters, int splits, void* stream);
+long long llmctl_gemm_skinny_scratch_elems(int Mb, int N, int K, int splits);
+unsigned long long llmctl_stream_capture_id(void* stream);
 
 /* ---- K6 causal flash attention, head_dim 64 or 128, bf16.  q/k/v/o: [B,S,H,D] views with token strides in
  * elements; lse: fp32 [B,H,S] (natural log).  Any S when causal, else a multiple of 128.  Reference: SDPA/eager inside

@@ -319,6 +319,54 @@ def test_layers_run_on_several_threads_and_streams(ops):
     _same(got, want)
 
 
+def test_decode_products_on_several_threads_and_streams(ops):
+    """Products of few rows on four threads, each on its own stream, against one thread's: each stream has partials and tickets of its own."""
+    import threading
+    ws = [_randn(n, 4096, seed=100 + n) for n in (264, 1000)]
+    xs = [_randn(5, 4096, seed=i) for i in range(4)]
+    want = [[ops.linear(x, w) for w in ws] for x in xs]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            outs = [ops.linear(xs[i], w) for _ in range(100) for w in ws]
+            s.synchronize()
+            bad.extend(n for n, o in enumerate(outs) if not torch.equal(o, want[i][n % 2]))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
+def test_captured_decode_products_replay_beside_others(ops):
+    """Two graphs of products of few rows, captured one after the other, replayed on two streams at once and beside products on a third."""
+    ws = [_randn(n, 4096, seed=100 + n) for n in (264, 1000)]
+    xs = [_randn(5, 4096, seed=i) for i in range(3)]
+    want = [[ops.linear(x, w) for w in ws] for x in xs]
+    torch.cuda.synchronize()
+    graphs, outs = [], []
+    for x in xs[:2]:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append([ops.linear(x, w) for _ in range(8) for w in ws])
+        graphs.append(g)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    for _ in range(20):
+        for s, g in zip(streams, graphs):
+            with torch.cuda.stream(s):
+                g.replay()
+        with torch.cuda.stream(streams[2]):
+            eager = [ops.linear(xs[2], w) for _ in range(8) for w in ws]
+    torch.cuda.synchronize()
+    for got, exact in zip([*outs, eager], want):
+        for n, o in enumerate(got):
+            assert torch.equal(o, exact[n % 2])
+
+
 def test_capture(ops):
     """A captured layer replays with new inputs."""
     x, w = _randn(64, 128), _randn(384, 128, seed=1)

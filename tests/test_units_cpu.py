@@ -826,3 +826,46 @@ def test_norm_entries_refuse_odd_addresses(name, operands, tail):
         at = [1 << 20] * len(operands)
         at[odd] += 2
         assert fn(*at, *tail) == 1, operands[odd]
+
+
+def test_decode_gemm_scratch_belongs_to_a_stream(monkeypatch):
+    """Partials and tickets of the decode GEMM: one pair per stream, grown where a call needs more, a bounded number of streams; captured calls take
+    partials of their own and one set of zeroed tickets per capture."""
+    from llmctl_b200.ops import functional as ops, native
+    now = {"stream": 1, "capture": 0}
+
+    class Lib:
+        @staticmethod
+        def llmctl_stream_capture_id(stream):
+            return now["capture"]
+    monkeypatch.setattr(ops, "_skinny_ws", {})
+    monkeypatch.setattr(ops, "_skinny_captures", {})
+    monkeypatch.setattr(native, "stream_ptr", lambda: now["stream"])
+    monkeypatch.setattr(native, "lib", lambda: Lib)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: now["capture"] != 0)
+    x = torch.empty(2, 8)
+
+    def ask(stream, elems, capture=0):
+        now.update(stream=stream, capture=capture)
+        return ops._skinny_workspace(x, elems)
+    a, b = ask(1, 1000), ask(2, 1000)
+    assert ask(1, 2000)[0] is a[0] and ask(1, 2000)[1] is a[1]
+    assert a[0] is not b[0] and a[1] is not b[1] and not a[1].any() and a[1].dtype == torch.int32
+    grown = ask(1, (1 << 20) + 1)
+    assert grown[0].numel() > 1 << 20 and grown[1] is a[1] and ask(1, 5)[0] is grown[0]
+    assert ask(1, 1 << 40)[0].numel() == ops._SKINNY_ELEMS                     # too few: the kernel takes whole tiles
+    first, again, other, elsewhere = ask(1, 1000, 7), ask(1, 1000, 7), ask(1, 1000, 8), ask(2, 1000, 8)
+    assert first[1] is again[1] and first[0] is not again[0]
+    assert len({id(t[1]) for t in (first, other, elsewhere, grown, b)}) == 5
+    assert ask(1, 1000)[1] is a[1] and ask(2, 1000)[1] is b[1]
+    for stream in range(3, 40):
+        ask(stream, 10)
+    assert len(ops._skinny_ws) == ops._SKINNY_STREAMS and (x.device.index, 39) in ops._skinny_ws and (x.device.index, 1) not in ops._skinny_ws
+
+
+@pytest.mark.parametrize("M,N,K,splits,elems", [(1, 128, 64, 0, 1 * 2 * 16 * 128), (17, 129, 4096, 0, 2 * 9 * 32 * 128), (16, 4096, 4096, 4, 32 * 5 * 16 * 128),
+                                                (32, 12288, 4096, 0, 96 * 3 * 32 * 128)])
+def test_decode_gemm_scratch_size(M, N, K, splits, elems):
+    """tiles x (most CTAs that share one) x rows of the tile's width x 128."""
+    from llmctl_b200.ops import native
+    assert native.lib().llmctl_gemm_skinny_scratch_elems(M, N, K, splits) == elems
