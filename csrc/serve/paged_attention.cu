@@ -312,6 +312,7 @@ LLMCTL_API int llmctl_kv_append(const void* qkv, long long row_stride, int k_off
   LLMCTL_BEGIN();
   LLMCTL_REQUIRE((heads * head_dim) % 8 == 0 && row_stride % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0);
   if (num_tokens == 0) return 0;
+  LLMCTL_REQUIRE(aligned16(qkv, k_cache, v_cache));
   LLMCTL_CHECK(launch_dependent(kv_append_kernel, num_tokens, 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)qkv, row_stride, k_off, v_off,
                                 (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, slot_mapping, heads * head_dim));
   LLMCTL_RETURN_LAST();
@@ -343,6 +344,7 @@ LLMCTL_API int llmctl_paged_attn_decode(const void* q, long long q_stride, const
   const bool cluster = decode_in_clusters(batch, heads, num_splits);
   LLMCTL_REQUIRE(num_splits >= 1 && block_size >= 1 && q_stride % 8 == 0 && (cluster || scratch != nullptr));
   if (batch == 0) return 0;
+  LLMCTL_REQUIRE(aligned16(k_cache, v_cache) && (reinterpret_cast<uintptr_t>(q) & 3) == 0);       // queries are read in pairs
   cudaStream_t s = (cudaStream_t)stream;
   int per = (max_context + num_splits - 1) / num_splits;
   per = ((per + block_size - 1) / block_size) * block_size;  // whole blocks per split

@@ -518,12 +518,16 @@ PyObject* py_rope_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // ---------------------------------------------------------------------------------------------------------------------------------
 // paged cache
 // ---------------------------------------------------------------------------------------------------------------------------------
+// a cache of whole rows of heads x head_dim
+bool is_cache(const Tensor& t, int64_t row) { return bf16(t) && t.is_contiguous() && unit16(t) && t.numel() % row == 0; }
+
 // kv_append(qkv, k_cache, v_cache, slots, heads, head_dim) -> True
 PyObject* py_kv_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return call(a, n, 6, [&](Args& args) -> PyObject* {
     const Tensor qkv = args.tensor(0), k = args.tensor(1), v = args.tensor(2), slots = args.tensor(3);
     const int64_t H = args.integer(4), D = args.integer(5), hd = H * D;
-    if (!args.ok || !quiet() || !ready(lib.llmctl_kv_append) || !bf16(qkv) || !bf16(k) || !bf16(v) || qkv.dim() != 2 || qkv.stride(1) != 1 || slots.scalar_type() != at::kLong)
+    if (!args.ok || !quiet() || !ready(lib.llmctl_kv_append) || H < 1 || D < 1 || hd % 8 || !is_matrix(qkv) || qkv.size(1) < 3 * hd || !is_cache(k, hd) || !is_cache(v, hd) ||
+        slots.scalar_type() != at::kLong || !slots.is_contiguous() || slots.numel() < qkv.size(0))
       return none();
     without_gil([&] {
       done("llmctl_kv_append", lib.llmctl_kv_append(cdata(qkv), qkv.stride(0), static_cast<int>(hd), static_cast<int>(2 * hd), data(k), data(v),
@@ -539,8 +543,13 @@ PyObject* py_paged_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor q = args.tensor(0), k = args.tensor(1), v = args.tensor(2), tables = args.tensor(3), lens = args.tensor(4);
     const int context = static_cast<int>(args.integer(5)), splits = static_cast<int>(args.integer(6));
     const double scale = args.number(7);
-    if (!args.ok || !quiet() || !ready(lib.llmctl_paged_attn_decode) || !lib.llmctl_paged_attn_scratch_elems || !bf16(q) || !bf16(k) || !bf16(v) || q.dim() != 3 || k.dim() != 4 ||
-        tables.dim() != 2 || tables.scalar_type() != at::kInt || lens.scalar_type() != at::kInt)
+    if (!args.ok || !quiet() || !ready(lib.llmctl_paged_attn_decode) || !lib.llmctl_paged_attn_scratch_elems || !bf16(q) || q.dim() != 3 || q.numel() == 0 || q.stride(2) != 1 ||
+        q.stride(1) != q.size(2) || !unit16(q))
+      return none();
+    const int64_t row = q.size(1) * q.size(2);
+    if (k.dim() != 4 || k.size(2) != q.size(1) || k.size(3) != q.size(2) || v.sizes() != k.sizes() || !is_cache(k, row) || !is_cache(v, row)) return none();
+    if (tables.dim() != 2 || tables.scalar_type() != at::kInt || !tables.is_contiguous() || tables.size(0) < q.size(0) || lens.scalar_type() != at::kInt || !lens.is_contiguous() ||
+        lens.numel() < q.size(0))
       return none();
     Tensor o = without_gil([&] {
       const int B = static_cast<int>(q.size(0)), H = static_cast<int>(q.size(1)), D = static_cast<int>(q.size(2));

@@ -18,6 +18,16 @@ native.register_signature("llmctl_paged_attn_scratch_elems", [c_int, c_int, c_in
 native.register_signature("llmctl_sample", [c_void_p, c_int, c_ll, c_int, c_int] + [c_void_p] * 6 + [c_void_p])
 
 
+def _check(ok: bool, what: str) -> None:
+    if not ok:
+        raise ValueError(what)
+
+
+def _check_cache(cache: torch.Tensor, like: torch.Tensor, row: int) -> None:
+    _check(cache.is_cuda and cache.dtype == like.dtype and cache.is_contiguous() and cache.data_ptr() % 16 == 0 and cache.numel() % row == 0,
+           f"a cache is contiguous rows of {row} {like.dtype} numbers on the GPU, from a 16-byte boundary")
+
+
 def kv_append(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, slot_mapping: torch.Tensor,
               heads: int, head_dim: int) -> None:
     """qkv: [T, 3*heads*head_dim] (post-RoPE); caches: [blocks, block_size, heads, head_dim];
@@ -26,6 +36,13 @@ def kv_append(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, s
     if qkv.is_cuda:
         if native.fast.kv_append(qkv, k_cache, v_cache, slot_mapping, heads, head_dim) is not None:
             return
+        _check(qkv.dim() == 2 and qkv.dtype.itemsize == 2 and qkv.shape[1] >= 3 * hd > 0, f"qkv: 16-bit rows of at least {3 * hd} numbers")
+        _check_cache(k_cache, qkv, hd)
+        _check_cache(v_cache, qkv, hd)
+        _check(slot_mapping.is_cuda and slot_mapping.dtype == torch.int64 and slot_mapping.numel() >= qkv.shape[0], "slot_mapping: int64 on the GPU, one per row")
+        slot_mapping = slot_mapping.contiguous()
+        if qkv.stride(1) != 1 or qkv.data_ptr() % 16:
+            qkv = qkv.clone(memory_format=torch.contiguous_format)
         native.call("llmctl_kv_append", qkv.data_ptr(), qkv.stride(0), hd, 2 * hd, k_cache.data_ptr(),
                     v_cache.data_ptr(), slot_mapping.data_ptr(), qkv.shape[0], heads, head_dim, native.stream_ptr())
         return
@@ -76,8 +93,18 @@ def paged_attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
             out = native.fast.paged_decode(q, k_cache, v_cache, block_tables, context_lens, max_context, ns, scale)
             if out is not None:
                 return out
+        _check(q.dtype == torch.bfloat16, "q: bfloat16")
+        _check_cache(k_cache, q, H * D)
+        _check_cache(v_cache, q, H * D)
+        _check(k_cache.shape == v_cache.shape, "k_cache and v_cache: of one shape")
+        _check(block_tables.is_cuda and block_tables.dtype == torch.int32 and block_tables.dim() == 2 and block_tables.shape[0] >= B,
+               "block_tables: int32 on the GPU, a row per sequence")
+        _check(context_lens.is_cuda and context_lens.dtype == torch.int32 and context_lens.numel() >= B, "context_lens: int32 on the GPU, one per sequence")
+        block_tables, context_lens = block_tables.contiguous(), context_lens.contiguous()
+        if q.stride(2) != 1 or q.stride(1) != D or q.data_ptr() % 16:
+            q = q.clone(memory_format=torch.contiguous_format)
         need = native.lib().llmctl_paged_attn_scratch_elems(B, H, D, ns)
-        if need and (scratch is None or scratch.numel() < need):
+        if need and (scratch is None or scratch.numel() < need or scratch.dtype != torch.float32 or not scratch.is_contiguous()):
             scratch = torch.empty(need, dtype=torch.float32, device=q.device)
         out = torch.empty(B, H, D, dtype=q.dtype, device=q.device)
         native.call("llmctl_paged_attn_decode", q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),

@@ -99,7 +99,8 @@ int llmctl_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K,
                      int tile_n, int max_ctas, void* stream);
 
 /* ---- K13 / K12 paged KV cache.  Reference: none (server.py:199-204 recomputes the whole sequence). ----
- * caches: [num_blocks, block_size, heads, head_dim] bf16; slot = block * block_size + offset. */
+ * caches: [num_blocks, block_size, heads, head_dim] bf16; slot = block * block_size + offset.  qkv and the caches lie on 16-byte
+ * boundaries, q on a 4-byte one (else cudaErrorInvalidValue). */
 int llmctl_kv_append(const void* qkv, long long row_stride, int k_off, int v_off, void* k_cache,
                      void* v_cache, const long long* slot_mapping, int num_tokens, int heads,
                      int head_dim, void* stream);

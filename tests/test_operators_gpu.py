@@ -216,6 +216,59 @@ def test_paged_decode(ops, B, H, D, context):
     _both(run)
 
 
+def _cache_call(B=3, H=2, D=64):
+    """Arguments of an append and of a decode over three sequences."""
+    k, v = _randn(3 * B, 16, H, D, seed=1), _randn(3 * B, 16, H, D, seed=2)
+    tables = torch.randperm(3 * B, generator=torch.Generator().manual_seed(3)).view(B, 3).int().cuda()
+    lens = torch.tensor([40, 7, 17], dtype=torch.int32, device="cuda")
+    slots = torch.tensor([5, -1, 40], device="cuda")
+    return {"qkv": _randn(B, 3 * H * D), "k": k, "v": v, "slots": slots, "tables": tables, "lens": lens, "q": _randn(B, H, D, seed=4)}
+
+
+def _at_odd_address(t):
+    return torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)[1:].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("name,form", [
+    ("qkv", _at_odd_address), ("qkv", lambda t: t.t().contiguous().t()), ("slots", lambda t: torch.stack([t, t], 1)[:, 0]), ("slots", lambda t: t.repeat(2)),
+    ("qkv", lambda t: torch.cat([t, t], 1)), ("q", _at_odd_address), ("q", lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)), ("q", lambda t: t.transpose(0, 1).contiguous().transpose(0, 1)),
+    ("tables", lambda t: torch.cat([t, t], 1)[:, :3]), ("tables", lambda t: t.t().contiguous().t()), ("tables", lambda t: t.repeat(2, 1)), ("lens", lambda t: torch.stack([t, t], 1)[:, 0])])
+def test_cache_operators_copy_other_layouts(ops, name, form):
+    """Views that the kernels do not read where they lie give what their copies give."""
+    from llmctl_b200.ops import serving
+
+    def run(form):
+        c = _cache_call()
+        c[name] = form(c[name])
+        serving.kv_append(c["qkv"], c["k"], c["v"], c["slots"], 2, 64)
+        return serving.paged_attention_decode(c["q"], c["k"], c["v"], c["tables"], c["lens"], 48), c["k"], c["v"]
+    _same(_both(lambda: run(form)), run(lambda t: t))
+
+
+@pytest.mark.parametrize("name,form", [
+    ("qkv", lambda t: t[:, :383]), ("qkv", lambda t: t.float()), ("k", _at_odd_address), ("v", lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)), ("k", lambda t: t.cpu()),
+    ("k", lambda t: t.float()), ("slots", lambda t: t[:2]), ("slots", lambda t: t.int()), ("slots", lambda t: t.cpu())])
+def test_append_refuses_what_it_cannot_write(ops, name, form):
+    from llmctl_b200.ops import serving
+    c = _cache_call()
+    c[name] = form(c[name])
+    for operators in (contextlib.nullcontext, python_operators):
+        with operators(), pytest.raises(ValueError):
+            serving.kv_append(c["qkv"], c["k"], c["v"], c["slots"], 2, 64)
+
+
+@pytest.mark.parametrize("name,form", [
+    ("q", lambda t: t.half()), ("k", _at_odd_address), ("v", lambda t: t[:4]), ("v", lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)), ("k", lambda t: t.cpu()), ("k", lambda t: t.half()),
+    ("tables", lambda t: t[:2]), ("tables", lambda t: t.long()), ("tables", lambda t: t.cpu()), ("lens", lambda t: t[:2]), ("lens", lambda t: t.long()), ("lens", lambda t: t.cpu())])
+def test_decode_refuses_what_it_cannot_read(ops, name, form):
+    from llmctl_b200.ops import serving
+    c = _cache_call()
+    c[name] = form(c[name])
+    for operators in (contextlib.nullcontext, python_operators):
+        with operators(), pytest.raises(ValueError):
+            serving.paged_attention_decode(c["q"], c["k"], c["v"], c["tables"], c["lens"], 48)
+
+
 def test_saved_tensor_hooks_see_what_is_kept(ops):
     """Offloading and checkpointing pack what a backward will need and unpack it there."""
     packed, unpacked = [], []

@@ -869,3 +869,16 @@ def test_decode_gemm_scratch_size(M, N, K, splits, elems):
     """tiles x (most CTAs that share one) x rows of the tile's width x 128."""
     from llmctl_b200.ops import native
     assert native.lib().llmctl_gemm_skinny_scratch_elems(M, N, K, splits) == elems
+
+
+def test_cache_entries_refuse_odd_addresses():
+    """As above for the append to the paged cache (packed rows, both caches) and the decode over it (queries read in pairs, both caches)."""
+    from llmctl_b200.ops import native
+    lib = native.ctypes.CDLL(str(native.library_path()))
+    p, i, ll, f = native.c_void_p, native.c_int, native.c_ll, native.c_float
+    lib.llmctl_kv_append.argtypes = [p, ll, i, i, p, p, p, i, i, i, p]
+    lib.llmctl_paged_attn_decode.argtypes = [p, ll, p, p, p, i, p, p, ll, p, i, i, i, i, i, i, f, p]
+    at = 1 << 20
+    for odd in ((2, 0, 0), (0, 2, 0), (0, 0, 8)):
+        assert lib.llmctl_kv_append(at + odd[0], 384, 128, 256, at + odd[1], at + odd[2], at, 2, 2, 64, None) == 1
+        assert lib.llmctl_paged_attn_decode(at + odd[0], 128, at + odd[1], at + odd[2], at, 4, at, at, 128, None, 2, 2, 64, 16, 64, 1, 0.125, None) == 1
