@@ -149,6 +149,7 @@ flash_bwd_kernel(const __grid_constant__ fbwd::Maps maps, const float* __restric
   Bars& bar = *reinterpret_cast<Bars*>(smem + C::kBarsAt);
   const uint32_t smem_base = smem_u32(smem);
   if (smem_base & 1023u) {             // the swizzled tiles would not line up (uniform over the grid)
+    wait_for_previous();
     if (threadIdx.x == 0) {
       atomicCAS(&g_status, 0u, 16u);
       report_wait(wait_byte);

@@ -882,3 +882,26 @@ def test_cache_entries_refuse_odd_addresses():
     for odd in ((2, 0, 0), (0, 2, 0), (0, 0, 8)):
         assert lib.llmctl_kv_append(at + odd[0], 384, 128, 256, at + odd[1], at + odd[2], at, 2, 2, 64, None) == 1
         assert lib.llmctl_paged_attn_decode(at + odd[0], 128, at + odd[1], at + odd[2], at, 4, at, at, 128, None, 2, 2, 64, 16, 64, 1, 0.125, None) == 1
+
+
+def test_dependent_kernels_wait_before_they_leave():
+    """csrc/common/dependent.cuh, rule 1: a kernel that is launched beside the end of the one before it waits for that one on every way out
+    and before it lets its own dependents in, or the order of the stream is lost for those behind it."""
+    import re
+    seen = []
+    for path in sorted((Path(__file__).resolve().parents[1] / "csrc").rglob("*.cu")):
+        text = path.read_text()
+        bodies = {}
+        for m in re.finditer(r"__global__ void (?:__\w+__\([^)]*\) )*\s*(\w+)\(", re.sub(r"\s*\n\s*", lambda m: " " * len(m.group()), text)):
+            bodies[m.group(1)] = text[text.index(") {", m.end()):text.index("\n}", m.end())]
+        launched = set(re.findall(r"launch_dependent\((\w+_kernel)\b", text))
+        for name, body in bodies.items():
+            wait = re.search(r"\bwait_for_previous\(", body)
+            if wait is None:
+                assert name not in launched, f"{path.name}: {name}"
+                continue
+            seen.append(name)
+            for leaving in (r"\breturn;", r"\brelease_dependents\("):
+                first = re.search(leaving, body)
+                assert first is None or wait.start() < first.start(), f"{path.name}: {name}: {first.group()} before the wait"
+    assert len(seen) >= 18 and {"flash_bwd_kernel", "gemm2_tcgen05_kernel", "norm_bwd_kernel", "paged_attn_decode_kernel"} <= set(seen), seen
