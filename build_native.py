@@ -2,7 +2,8 @@
 """Build the native libraries in-tree.
 
   libllmctl_b200.so : every sm_100a CUDA kernel behind a C ABI (include/llmctl_b200.h)
-  llmctl_ops.so     : the operators' host side (checks, allocation, launch, autograd nodes) as a Python extension over libtorch
+  llmctl_ops.so     : the operators' host side (checks, allocation, launch, autograd nodes) as a Python extension over libtorch; left out
+                      where PyTorch or the Python headers are missing, and where only components of the kernel library are asked for
   libllmctl_host.so : C++ host runtime (KV block manager, batch scheduler, ...), no CUDA needed
 
 Sources are compiled one translation unit per nvcc/g++ process (in parallel) and only when the
@@ -100,6 +101,30 @@ def _compile(cmd: list[str], src: Path, obj: Path, verbose: bool) -> tuple[Path,
     return obj, (r.stdout + r.stderr) if verbose else ""
 
 
+def _operators_stamp() -> str:
+    """What the extension over libtorch is built for; ops/native.py loads no other."""
+    import sysconfig
+
+    import torch
+    return f"{torch.__version__} {sysconfig.get_config_var('SOABI')}"
+
+
+def _operators_missing() -> str | None:
+    """What the extension cannot be built for want of."""
+    import importlib.util
+    import sysconfig
+    if importlib.util.find_spec("torch") is None:
+        return "PyTorch"
+    if not Path(sysconfig.get_paths()["include"], "Python.h").exists():
+        return "the Python headers"
+    return None
+
+
+def _operators_current(lib: Path, src: Path, hdr_m: float) -> bool:
+    stamp = lib.with_suffix(".built")
+    return lib.exists() and lib.stat().st_mtime > max(src.stat().st_mtime, hdr_m) and stamp.exists() and stamp.read_text() == _operators_stamp()
+
+
 def _build_operators(force: bool, hdr_m: float, verbose: bool) -> Path:
     import sysconfig
 
@@ -107,7 +132,7 @@ def _build_operators(force: bool, hdr_m: float, verbose: bool) -> Path:
     root = Path(torch.__file__).resolve().parent
     cuda = Path(find_nvcc() or "/usr/local/cuda/bin/nvcc").resolve().parents[1]
     src, obj, lib = CSRC / "torch" / "ops.cpp", OBJDIR / "torch" / "ops.o", LIBDIR / "llmctl_ops.so"
-    if not force and lib.exists() and lib.stat().st_mtime > max(src.stat().st_mtime, hdr_m):
+    if not force and _operators_current(lib, src, hdr_m):
         return lib
     cxx = os.environ.get("CXX", "g++")
     flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
@@ -118,11 +143,14 @@ def _build_operators(force: bool, hdr_m: float, verbose: bool) -> Path:
     r = subprocess.run(link, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed: {src}\n{' '.join(link)}\n{r.stdout}\n{r.stderr}")
+    lib.with_suffix(".built").write_text(_operators_stamp())
     return lib
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False, jobs: int | None = None,
-          components=None) -> dict:
+          components=None, operators: bool | None = None) -> dict:
+    """``operators``: whether the extension over libtorch is built too; by default with the whole library, and where it is there already (its calls
+    follow the library's)."""
     LIBDIR.mkdir(parents=True, exist_ok=True)
     hdr_m = _newest_header_mtime()
     nvcc = find_nvcc()
@@ -165,7 +193,11 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False, 
         out["kernels"] = str(lib)
 
     # ---- host side of the operators: a Python extension over libtorch ----
-    out["operators"] = str(_build_operators(force, hdr_m, verbose))
+    if operators is None:
+        operators = not components or "all" in components or (LIBDIR / "llmctl_ops.so").exists()
+    if operators:
+        missing = _operators_missing()
+        out["operators"] = f"left out for want of {missing}" if missing else str(_build_operators(force, hdr_m, verbose))
 
     # ---- host C++ ----
     cpp_srcs = sorted(p for p in (CSRC / "host").glob("*.cpp"))

@@ -11,7 +11,9 @@ from __future__ import annotations
 
 import ctypes
 import importlib.util
+import sysconfig
 import threading
+import warnings
 from pathlib import Path
 from typing import Optional
 
@@ -120,13 +122,23 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
-def _load_ops():
+def _load_ops() -> None:
+    """Take the operators' host side in C++ into use.  Where there is none for this PyTorch the Python operators launch the same kernels, at 10-50 us
+    more of host time each, which is said once."""
     global fast
-    if not _OPS_PATH.exists():
-        raise RuntimeError(f"operator extension not found at {_OPS_PATH}; run `python build_native.py` (or __graft_entry__.build())")
-    spec = importlib.util.spec_from_file_location("llmctl_ops", _OPS_PATH)
-    ops = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(ops)
+    built = _OPS_PATH.with_suffix(".built")
+    here = f"{torch.__version__} {sysconfig.get_config_var('SOABI')}"
+    try:
+        if not _OPS_PATH.exists():
+            raise ImportError("not built")
+        if not built.exists() or built.read_text() != here:          # built for another PyTorch it might load and misread every tensor
+            raise ImportError(f"built for {built.read_text() if built.exists() else 'another PyTorch'}, this is {here}")
+        spec = importlib.util.spec_from_file_location("llmctl_ops", _OPS_PATH)
+        ops = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(ops)
+    except (ImportError, OSError) as e:
+        warnings.warn(f"{_OPS_PATH.name} is not used ({e}): operators take their checks and launches through Python; run `python build_native.py`", RuntimeWarning)
+        return
     ops.bind(str(_LIB_PATH), NativeError, check_waits)
     fast = ops
 
@@ -155,10 +167,13 @@ def _function(name: str):
 
 
 def has_symbol(name: str) -> bool:
+    """Whether the kernel library is built and has this entry.  One that is there and does not load raises."""
+    if _lib is None and not available():
+        return False
     try:
         _function(name)
         return True
-    except (AttributeError, RuntimeError):
+    except AttributeError:
         return False
 
 

@@ -905,3 +905,71 @@ def test_dependent_kernels_wait_before_they_leave():
                 first = re.search(leaving, body)
                 assert first is None or wait.start() < first.start(), f"{path.name}: {name}: {first.group()} before the wait"
     assert len(seen) >= 18 and {"flash_bwd_kernel", "gemm2_tcgen05_kernel", "norm_bwd_kernel", "paged_attn_decode_kernel"} <= set(seen), seen
+
+
+def test_operator_extension_is_not_a_condition(monkeypatch, tmp_path):
+    """An extension that is missing, of another PyTorch or no library at all leaves the Python operators in place, and says so."""
+    import sysconfig
+    from llmctl_b200.ops import native
+    path, here = tmp_path / "llmctl_ops.so", f"{torch.__version__} {sysconfig.get_config_var('SOABI')}"
+    monkeypatch.setattr(native, "_OPS_PATH", path)
+    monkeypatch.setattr(native, "fast", native._NoOps())
+    for content, built, why in ((None, None, "not built"), ("x", None, "another PyTorch"), ("x", "1.0 cpython-2", "1.0 cpython-2"), ("x", here, "")):
+        if content is not None:
+            path.write_text(content)
+        if built is not None:
+            path.with_suffix(".built").write_text(built)
+        with pytest.warns(RuntimeWarning, match=why):
+            native._load_ops()
+        assert native.fast.rmsnorm(1, 2) is None and native.fast.launches() == 0
+
+
+def test_has_symbol_tells_a_missing_entry_from_a_library_that_does_not_load(monkeypatch):
+    from llmctl_b200.ops import native
+    monkeypatch.setattr(native, "_lib", None)
+    monkeypatch.setattr(native, "_functions", {})
+
+    def failing(error):
+        def lib():
+            raise error
+        return lib
+    for built in (True, False):
+        monkeypatch.setattr(native, "available", lambda: built)
+        for error in (OSError("no loader"), RuntimeError("not this one")):
+            monkeypatch.setattr(native, "lib", failing(error))
+            if built:
+                with pytest.raises(type(error)):
+                    native.has_symbol("llmctl_rmsnorm_fwd")
+            else:
+                assert not native.has_symbol("llmctl_rmsnorm_fwd")
+    monkeypatch.setattr(native, "available", lambda: True)
+    monkeypatch.setattr(native, "lib", lambda: type("Library", (), {"llmctl_rmsnorm_fwd": 1}))
+    assert native.has_symbol("llmctl_rmsnorm_fwd") and not native.has_symbol("llmctl_rmsnorm_bwd")
+
+
+def test_build_of_the_operator_extension(monkeypatch, tmp_path):
+    """It is built with the whole library and where it was built before, not for a part of the kernels, and again for another PyTorch."""
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("build_native_under_test", Path(__file__).resolve().parents[1] / "build_native.py")
+    b = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(b)
+    lib, src = tmp_path / "llmctl_ops.so", tmp_path / "ops.cpp"
+    monkeypatch.setattr(b, "LIBDIR", tmp_path)
+    monkeypatch.setattr(b, "CSRC", tmp_path)
+    monkeypatch.setattr(b, "_component_sources", lambda components: [])
+    monkeypatch.setattr(b, "_build_operators", lambda *a: lib)
+    assert "operators" not in b.build(components=["serve"]) and "operators" not in b.build(operators=False)
+    assert b.build()["operators"] == b.build(components=["all"])["operators"] == b.build(components=["serve"], operators=True)["operators"] == str(lib)
+    monkeypatch.setattr(b, "_operators_missing", lambda: "PyTorch")
+    assert "PyTorch" in b.build()["operators"]
+    src.write_text("")
+    lib.write_text("")
+    assert "operators" in b.build(components=["serve"])
+    now = src.stat().st_mtime
+    import os
+    os.utime(lib, (now + 10, now + 10))
+    assert not b._operators_current(lib, src, now)
+    lib.with_suffix(".built").write_text(b._operators_stamp())
+    assert b._operators_current(lib, src, now) and not b._operators_current(lib, src, now + 20)
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert not b._operators_current(lib, src, now)
