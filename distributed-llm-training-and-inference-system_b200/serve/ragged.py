@@ -171,10 +171,24 @@ class RaggedBatch:
             contexts = [min(p.start + len(p.tokens), longest) for p in self._portions]
         else:                                                   # captured: any of them may be the longest
             contexts = [longest] * self.pad_to[0]
-        tiles = max(1, -(-sum(contexts) * groups // (64 * slots)))
-        while True:
-            n = -(-longest // (64 * tiles))
-            per = max(64, (-(-longest // n) + 63) // 64 * 64)
-            if n <= 1 or groups * sum(-(-c // per) for c in contexts) <= slots:
-                return max(1, n)
-            tiles += 1
+        if groups * len(contexts) > slots:                      # whole contexts are more than one wave already
+            return 1
+
+        def cut(tiles: int) -> int:                             # splits of at most `tiles` tiles
+            return -(-longest // (64 * tiles))
+
+        def fits(tiles: int) -> bool:
+            per = max(64, (-(-longest // cut(tiles)) + 63) // 64 * 64)
+            return groups * sum([-(-c // per) for c in contexts]) <= slots
+        # longer splits are fewer CTAs and whole contexts fit: the shortest that fit, near the even share as a rule
+        lo = tiles = max(1, -(-sum(contexts) * groups // (64 * slots)))
+        most, step = -(-longest // 64), 1
+        while tiles < most and not fits(tiles):
+            lo, tiles, step = tiles + 1, min(most, tiles + step), 2 * step
+        while lo < tiles:
+            mid = (lo + tiles) // 2
+            if fits(mid):
+                tiles = mid
+            else:
+                lo = mid + 1
+        return max(1, cut(tiles))

@@ -382,3 +382,38 @@ def test_decode_splits_fill_one_wave(starts, heads):
     assert b.attention_splits(heads, rows) == n
     b.refill([Portion(0, [1], 0, [0], [0])] * len(starts))
     assert b.attention_splits(heads, rows, 1) == 1
+
+
+def test_decode_splits_are_found_in_few_steps():
+    """Against the search that tries one tile after the other, over batches of unlike contexts; and what the search costs, in sums over the batch:
+    one long context among many short ones has thousands of lengths to try."""
+    import random
+    import sys
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+
+    def one_by_one(contexts, slots, groups, longest):
+        tiles = max(1, -(-sum(contexts) * groups // (64 * slots)))
+        while True:
+            n = -(-longest // (64 * tiles))
+            per = max(64, (-(-longest // n) + 63) // 64 * 64)
+            if n <= 1 or groups * sum(-(-c // per) for c in contexts) <= slots:
+                return max(1, n)
+            tiles += 1
+    r, b = random.Random(1), RaggedBatch.__new__(RaggedBatch)
+    b.pad_to = None
+    for _ in range(500):
+        hi = r.choice([1, 64, 65, 500, 4000, 20000])
+        starts = [r.randrange(hi) for _ in range(r.choice([1, 2, 8, 32, 100, 300]))]
+        b._portions = [Portion(0, [1], s, [0], []) for s in starts]
+        longest = r.choice([max(starts) + 1, max(1, max(starts) // 2), max(starts) + 100])
+        groups, slots = r.choice([1, 2, 3, 8]), r.choice([148, 296])
+        assert b._even_splits(slots, groups, longest) == one_by_one([min(s + 1, longest) for s in starts], slots, groups, longest)
+    for short, groups, want in ((255, 4, 1), (140, 1, 8)):
+        b._portions = [Portion(0, [1], s, [0], []) for s in [99] * short + [131071]]
+        sums = []
+        sys.setprofile(lambda frame, event, arg: sums.append(1) if event == "c_call" and arg is sum else None)
+        try:
+            got = b._even_splits(148, groups, 131072)
+        finally:
+            sys.setprofile(None)
+        assert got == want and len(sums) <= 32
