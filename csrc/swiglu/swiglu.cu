@@ -64,6 +64,7 @@ LLMCTL_API int llmctl_swiglu_fwd(const void* gate_up, void* out, int M, int F, l
   LLMCTL_REQUIRE(F % 8 == 0 && ld_gu % 8 == 0 && ld_gu >= 2LL * F);
   const long long total = static_cast<long long>(M) * (F / 8);
   if (total == 0) return 0;
+  LLMCTL_REQUIRE(aligned16(gate_up, out));
   long long blocks = (total + 255) / 256;
   if (blocks > kNumSMs * 16) blocks = kNumSMs * 16;
   swiglu_fwd_kernel<<<static_cast<int>(blocks), 256, 0, (cudaStream_t)stream>>>(
@@ -77,6 +78,7 @@ LLMCTL_API int llmctl_swiglu_bwd(const void* dout, const void* gate_up, void* d_
   LLMCTL_REQUIRE(F % 8 == 0 && ld_gu % 8 == 0 && ld_gu >= 2LL * F);
   const long long total = static_cast<long long>(M) * (F / 8);
   if (total == 0) return 0;
+  LLMCTL_REQUIRE(aligned16(dout, gate_up, d_gate_up));
   long long blocks = (total + 255) / 256;
   if (blocks > kNumSMs * 16) blocks = kNumSMs * 16;
   swiglu_bwd_kernel<<<static_cast<int>(blocks), 256, 0, (cudaStream_t)stream>>>(

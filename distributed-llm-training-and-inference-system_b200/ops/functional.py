@@ -288,8 +288,8 @@ class _SwiGLUFn(torch.autograd.Function):
     def backward(ctx, dout):
         (gu,) = ctx.saved_tensors
         M, F2 = gu.shape
-        dout = dout.contiguous()
-        dgu = torch.empty(M, F2, dtype=gu.dtype, device=gu.device)
+        dout = _whole_units(dout)
+        dgu = torch.empty_strided(gu.shape, gu.stride(), dtype=gu.dtype, device=gu.device)      # the kernel's one row stride is that of both
         native.call("llmctl_swiglu_bwd", dout.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, F2 // 2, gu.stride(0),
                     native.stream_ptr())
         return dgu
@@ -300,8 +300,8 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     if _use_native(gate_up, "elementwise") and gate_up.shape[-1] % 16 == 0:
         shape = gate_up.shape
         g2 = gate_up.reshape(-1, shape[-1])
-        if g2.stride(1) != 1 or g2.stride(0) % 8:
-            g2 = g2.contiguous()
+        if g2.stride(1) != 1 or g2.stride(0) % 8 or g2.data_ptr() % 16:
+            g2 = _whole_units(g2)
         return native.apply(_SwiGLUFn, g2).view(*shape[:-1], shape[-1] // 2)
     g, u = gate_up.chunk(2, dim=-1)
     return (F.silu(g.float()) * u.float()).to(gate_up.dtype)
@@ -379,7 +379,7 @@ class _LinearFn(torch.autograd.Function):
     def backward(ctx, dy):
         x, w = ctx.saved_tensors
         if not _gemm_ok(dy):
-            dy = dy.contiguous()
+            dy = _whole_units(dy)
         dx = dw = None
         if ctx.needs_input_grad[0]:
             dx = gemm_raw(dy, w, b_mn=True)          # [M,N] x [N,K]  (w stored [N,K] = "K x N" MN-major)
@@ -516,7 +516,7 @@ class _LinearSwiGLUFn(torch.autograd.Function):
     def backward(ctx, dact):
         x, w, gu = ctx.saved_tensors
         M, F2 = gu.shape
-        dact = dact.contiguous()
+        dact = _whole_units(dact)
         dgu = torch.empty_like(gu)
         native.call("llmctl_swiglu_bwd", dact.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, F2 // 2, gu.stride(0), native.stream_ptr())
         dx = gemm_raw(dgu, w, b_mn=True) if ctx.needs_input_grad[0] else None
@@ -543,7 +543,7 @@ class _SwiGLUMLPFn(torch.autograd.Function):
     def backward(ctx, dy):
         x, w_up, w_down, gu, act = ctx.saved_tensors
         if not _gemm_ok(dy):
-            dy = dy.contiguous()
+            dy = _whole_units(dy)
         dx = dw_up = dgu = None
         if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
             M, F2 = gu.shape
@@ -613,11 +613,11 @@ class _SwiGLULinearFn(torch.autograd.Function):
         gu, w = ctx.saved_tensors
         M, F2 = gu.shape
         if not _gemm_ok(dy):
-            dy = dy.contiguous()
+            dy = _whole_units(dy)
         act = torch.empty(M, F2 // 2, dtype=gu.dtype, device=gu.device)          # recompute
         native.call("llmctl_swiglu_fwd", gu.data_ptr(), act.data_ptr(), M, F2 // 2, gu.stride(0), native.stream_ptr())
         dact = gemm_raw(dy, w, b_mn=True)
-        dgu = torch.empty_like(gu)
+        dgu = torch.empty_strided(gu.shape, gu.stride(), dtype=gu.dtype, device=gu.device)
         native.call("llmctl_swiglu_bwd", dact.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, F2 // 2, gu.stride(0),
                     native.stream_ptr())
         dw = None

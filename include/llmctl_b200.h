@@ -50,7 +50,7 @@ int llmctl_rope_inplace(void* x, long long row_stride, int n_tokens, int n_heads
                         const float* cos_t, const float* sin_t, const int* positions, int seq_len,
                         float sign, void* stream);
 
-/* ---- K5 SwiGLU on packed [M, 2F] gate|up.  Reference: ATen silu + mul. ---- */
+/* ---- K5 SwiGLU on packed [M, 2F] gate|up, all on 16-byte boundaries; d_gate_up has gate_up's row stride.  Reference: ATen silu + mul. ---- */
 int llmctl_swiglu_fwd(const void* gate_up, void* out, int M, int F, long long ld_gu, void* stream);
 int llmctl_swiglu_bwd(const void* dout, const void* gate_up, void* d_gate_up, int M, int F,
                       long long ld_gu, void* stream);

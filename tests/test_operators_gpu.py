@@ -157,6 +157,34 @@ def test_mlp(ops, rows, width, ffn, grad):
     _both(run)
 
 
+@pytest.mark.parametrize("form", ["odd", "gaps", "odd gradient"])
+@pytest.mark.parametrize("op", ["swiglu", "swiglu_linear", "linear_swiglu", "linear", "mlp"])
+def test_gated_layers_on_other_layouts(ops, op, form):
+    """Inputs and gradients that begin inside a 16-byte unit, and rows with gaps between them, against whole units back to back: the same bits, and
+    nothing is written outside of the gradient."""
+    rows, width = 50, 128
+    down, up = _randn(64, width // 2, seed=1), _randn(width, width, seed=2)
+    w = {"swiglu_linear": [down], "linear_swiglu": [up], "linear": [up], "mlp": [up, _randn(1024, width // 2, seed=3)]}.get(op, [])
+    call = {"swiglu": ops.swiglu, "swiglu_linear": ops.swiglu_linear, "linear_swiglu": ops.linear_swiglu, "linear": ops.linear, "mlp": ops.swiglu_mlp}[op]
+
+    def laid_out(t, how):
+        if how == "odd":
+            return torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)[1:].view(t.shape).copy_(t)
+        return torch.cat([t, t], 1)[:, :t.shape[1]] if how == "gaps" else t
+
+    def run(form):
+        leaves = [laid_out(_randn(rows, width), form).detach().requires_grad_(True)] + [t.detach().requires_grad_(True) for t in w]
+        y = call(*leaves)
+        grads = torch.autograd.grad(y, leaves, laid_out(_randn(*y.shape, seed=4), "odd" if form == "odd gradient" else ""))
+        return (y.detach(), *grads)
+    got, want = run(form), run("")
+    if form == "odd" and op in ("linear", "linear_swiglu", "mlp", "swiglu_linear"):         # products of such inputs are the library's
+        for a, b in zip(got, want):
+            assert (a.float() - b.float()).norm() <= 2.0 ** -7 * b.float().norm()
+    else:
+        _same(got, want)
+
+
 @pytest.mark.parametrize("B,S,H,D", [(1, 1, 1, 64), (2, 128, 3, 128), (2, 77, 2, 64), (1, 300, 2, 128)])
 @pytest.mark.parametrize("form", ["packed", "apart", "odd", "heads first", "fp32"])
 @pytest.mark.parametrize("grad", [False, True])

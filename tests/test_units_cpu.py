@@ -815,13 +815,15 @@ def test_decode_splits_by_pairs_of_head_and_sequence(batch, heads, dim, context,
     ("llmctl_rmsnorm_bwd_noalloc", ["dy", "h", "w", None, "dres", "dx", None], (4, 64, 0, None)),
     ("llmctl_layernorm_fwd", ["x", "residual", "w", "b", "h", "y", None, None], (4, 64, 1e-5, None)),
     ("llmctl_layernorm_bwd", ["dy", "h", "w", None, None, "dres", "dx", None, None, "scratch"], (4, 4, 64, 0, None)),
+    ("llmctl_swiglu_fwd", ["gate_up", "out"], (4, 64, 128, None)),
+    ("llmctl_swiglu_bwd", ["dout", "gate_up", "d_gate_up"], (4, 64, 128, None)),
 ])
-def test_norm_entries_refuse_odd_addresses(name, operands, tail):
+def test_entries_refuse_odd_addresses(name, operands, tail):
     """An operand that the kernels read or write in 16-byte units and that begins inside one is an invalid value (1), told before anything is
     launched."""
     from llmctl_b200.ops import native
     fn = getattr(native.ctypes.CDLL(str(native.library_path())), name)
-    fn.argtypes = [native.c_void_p] * len(operands) + [native.c_float if isinstance(v, float) else native.c_void_p if v is None else native.c_int for v in tail]
+    fn.argtypes = [native.c_void_p] * len(operands) + [native.c_float if isinstance(v, float) else native.c_void_p if v is None else native.c_ll for v in tail]
     for odd in (i for i, operand in enumerate(operands) if operand):
         at = [1 << 20] * len(operands)
         at[odd] += 2
