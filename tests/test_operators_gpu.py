@@ -511,3 +511,75 @@ def test_kernels_begin_when_those_before_have_ended(ops, rows, width, heads):
     want = chain(True)
     for _ in range(3):
         _same(chain(False), want)
+
+
+@contextlib.contextmanager
+def waiting_operators():
+    """Every kernel of the library is waited for before the next one is launched."""
+    from llmctl_b200.ops import native
+    call = native.call
+
+    def call_and_wait(*args):
+        call(*args)
+        torch.cuda.synchronize()
+    native.call = call_and_wait
+    try:
+        with python_operators():
+            yield
+    finally:
+        native.call = call
+
+
+# prompts: cache write, keys and values rebuilt, attention over them; decoding: cache write, attention in splits and their merge, or in one piece
+@pytest.mark.parametrize("starts,tokens,heads", [([0, 0], 300, 4), ([130], 200, 4), ([700, 333, 64], 1, 16), ([2000], 1, 32), ([5, 40], 1, 16)])
+def test_latent_kernels_begin_when_those_before_have_ended(ops, starts, tokens, heads):
+    """Latent-attention layers one after the other over one cache, whose kernels are launched beside the end of the one before, against the same
+    with each kernel waited for."""
+    from llmctl_b200.models.mixers import LatentAttention, LatentAttentionSpec
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+    R, dr, dn, dv, page, Q, W = 512, 64, 128, 128, 64, 256, 512
+    spec = LatentAttentionSpec(heads=heads, dim=dn, rot_dim=dr, vdim=dv, kv_rank=R, q_rank=Q, scale=(dn + dr) ** -0.5, rot_base=10000.0)
+    layers = []
+    for i in range(2):
+        layers.append(LatentAttention(W, spec, 1e-5, torch.bfloat16, "cuda"))
+        with torch.no_grad():
+            for j, (name, w) in enumerate(layers[i].named_parameters()):
+                w.copy_(_randn(*w.shape, seed=10 * i + j) * (1.0 if w.dim() == 1 else 2 * w.shape[-1] ** -0.5))
+    pages = [(s + tokens + page - 1) // page for s in starts]
+    tables = [list(range(sum(pages[:i]), sum(pages[:i + 1]))) for i in range(len(starts))]
+    batch = RaggedBatch([Portion(i, [1] * tokens, s, [tokens - 1], t) for i, (s, t) in enumerate(zip(starts, tables))], page, torch.device("cuda"))
+
+    def run():
+        h = _randn(len(starts) * tokens, W, seed=1)
+        caches = [_randn(sum(pages), page, R + dr, seed=2 + i) for i in range(2)]
+        with torch.no_grad():
+            for i in range(8):
+                h = layers[i % 2](h, batch, caches[i % 2])
+                h = ops.rmsnorm(h, layers[0].kv_norm)[0]           # 512 weights: the width of the layer
+        return h, *caches
+    with waiting_operators():
+        want = run()
+    assert all(t.isfinite().all() for t in want)
+    for _ in range(3):
+        _same(run(), want)
+
+
+@pytest.mark.parametrize("rows,V", [(40, 64), (300, 32000), (1100, 4096)])
+def test_loss_kernels_begin_when_those_before_have_ended(ops, rows, V):
+    """The product before a loss, the loss's three kernels and the gradients behind it, several times over the same memory, as above."""
+    w, t = _randn(V, 128, seed=1) * 0.1, torch.randint(0, V, (rows,), generator=torch.Generator().manual_seed(2)).cuda()
+    t[::7] = -100
+
+    def run():
+        x, out = _randn(rows, 128), []
+        for _ in range(6):
+            x, leaf = x.detach().requires_grad_(True), w.detach().requires_grad_(True)
+            loss = ops.cross_entropy(ops.linear(x, leaf), t, assume_unit_grad=True)
+            dx, dw = torch.autograd.grad(loss, (x, leaf))
+            out += [loss.detach(), dx, dw]
+            x = x.detach() - dx * rows
+        return out
+    with waiting_operators():
+        want = run()
+    for _ in range(3):
+        _same(run(), want)
