@@ -307,7 +307,7 @@ Tensor as_shape_of(const Tensor& y, const Tensor& x) {
 }
 
 // linear(x, w, tile_n, workspace or None) -> x @ w.T where no gradient is recorded; few rows take the decode GEMM, whose partials and tickets
-// workspace(x, floats of partials) returns
+// workspace(x, floats of partials, stream) returns
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return call(a, n, 4, [&](Args& args) -> PyObject* {
     const Tensor x = args.tensor(0), w = args.tensor(1);
@@ -319,8 +319,8 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (skinny ? !ready(lib.llmctl_gemm_skinny_bf16) || !lib.llmctl_gemm_skinny_scratch_elems : !ready(lib.llmctl_gemm_bf16) || w.size(0) % 8) return none();
     Tensor ws, counters;
     if (skinny) {
-      PyObject* pair = PyObject_CallFunction(a[3], "OL", a[0], lib.llmctl_gemm_skinny_scratch_elems(static_cast<int>(rows.size(0)), static_cast<int>(w.size(0)),
-                                                                                                     static_cast<int>(w.size(1)), 0));
+      PyObject* pair = PyObject_CallFunction(a[3], "OLN", a[0], lib.llmctl_gemm_skinny_scratch_elems(static_cast<int>(rows.size(0)), static_cast<int>(w.size(0)),
+                                                                                                      static_cast<int>(w.size(1)), 0), PyLong_FromVoidPtr(stream()));
       if (pair == nullptr) throw python_error();
       ws = THPVariable_Unpack(PyTuple_GET_ITEM(pair, 0));
       counters = THPVariable_Unpack(PyTuple_GET_ITEM(pair, 1));

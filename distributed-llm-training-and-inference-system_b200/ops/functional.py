@@ -406,33 +406,40 @@ _skinny_captures: dict = {}     # (device, stream) -> (capture, tickets)
 _skinny_lock = threading.Lock()
 
 
-def _skinny_workspace(x: torch.Tensor, elems: int):
-    """Split-K scratch of the skinny GEMM for a call on the current stream: at least ``elems`` fp32 partials (or too few, beyond
-    ``_SKINNY_ELEMS``) and zeroed tickets.  Calls on one stream follow one another and share a pair, kept for the last ``_SKINNY_STREAMS``
-    streams that asked; what is dropped goes back to its stream's pool behind that stream's work.  A captured call may be replayed beside
-    anything, another graph of the same stream too: its partials come from the graph's pool, and the tickets of a capture are zeroed by
-    the graph itself."""
-    elems = min(max(elems, 1), _SKINNY_ELEMS)
-    stream = native.stream_ptr()
-    key = (x.device.index, stream)
+def _skinny_workspace(x: torch.Tensor, elems: int, stream: Optional[int] = None):
+    """Split-K scratch of the skinny GEMM for a call on the current stream (its handle, where the caller has it at hand): at least ``elems`` fp32
+    partials (or too few, beyond ``_SKINNY_ELEMS``) and zeroed tickets.  Calls on one stream follow one another and share a pair, kept for the
+    last ``_SKINNY_STREAMS`` streams that asked; what is dropped goes back to its stream's pool behind that stream's work.  A captured call
+    may be replayed beside anything, another graph of the same stream too: its partials come from the graph's pool, and the tickets of a
+    capture are zeroed by the graph itself."""
+    key = (x.get_device(), native.stream_ptr() if stream is None else stream)
     if torch.cuda.is_current_stream_capturing():
-        capture = native.lib().llmctl_stream_capture_id(stream)
-        with _skinny_lock:
-            made = _skinny_captures.get(key)
-            if made is None or made[0] != capture:
-                made = _skinny_captures[key] = (capture, torch.zeros(_SKINNY_TICKETS, dtype=torch.int32, device=x.device))
-        return torch.empty(elems, dtype=torch.float32, device=x.device), made[1]
+        return _captured_skinny_workspace(x, elems, key)
     ws = _skinny_ws.get(key)
-    if ws is None or ws[0].numel() < elems:
-        with _skinny_lock:
-            ws = _skinny_ws.pop(key, None)
-            if ws is None or ws[0].numel() < elems:
-                tickets = torch.zeros(_SKINNY_TICKETS, dtype=torch.int32, device=x.device) if ws is None else ws[1]
-                ws = (torch.empty(min(_SKINNY_ELEMS, -(-elems >> 20) << 20), dtype=torch.float32, device=x.device), tickets)
-            while len(_skinny_ws) >= _SKINNY_STREAMS:
-                del _skinny_ws[next(iter(_skinny_ws))]
-            _skinny_ws[key] = ws
+    if ws is None or ws[0].numel() < elems and ws[0].numel() < _SKINNY_ELEMS:
+        ws = _grown_skinny_workspace(x, elems, key)
     return ws
+
+
+def _grown_skinny_workspace(x: torch.Tensor, elems: int, key):
+    with _skinny_lock:
+        ws = _skinny_ws.pop(key, None)
+        if ws is None or ws[0].numel() < elems:
+            tickets = torch.zeros(_SKINNY_TICKETS, dtype=torch.int32, device=x.device) if ws is None else ws[1]
+            ws = (torch.empty(min(_SKINNY_ELEMS, max(1, -(-elems >> 20)) << 20), dtype=torch.float32, device=x.device), tickets)
+        while len(_skinny_ws) >= _SKINNY_STREAMS:
+            del _skinny_ws[next(iter(_skinny_ws))]
+        _skinny_ws[key] = ws
+    return ws
+
+
+def _captured_skinny_workspace(x: torch.Tensor, elems: int, key):
+    capture = native.lib().llmctl_stream_capture_id(key[1])
+    with _skinny_lock:
+        made = _skinny_captures.get(key)
+        if made is None or made[0] != capture:
+            made = _skinny_captures[key] = (capture, torch.zeros(_SKINNY_TICKETS, dtype=torch.int32, device=x.device))
+    return torch.empty(max(1, min(elems, _SKINNY_ELEMS)), dtype=torch.float32, device=x.device), made[1]
 
 
 def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, splits: int = 0) -> torch.Tensor:

@@ -862,7 +862,8 @@ def test_decode_gemm_scratch_belongs_to_a_stream(monkeypatch):
     assert ask(1, 1000)[1] is a[1] and ask(2, 1000)[1] is b[1]
     for stream in range(3, 40):
         ask(stream, 10)
-    assert len(ops._skinny_ws) == ops._SKINNY_STREAMS and (x.device.index, 39) in ops._skinny_ws and (x.device.index, 1) not in ops._skinny_ws
+    assert len(ops._skinny_ws) == ops._SKINNY_STREAMS and (x.get_device(), 39) in ops._skinny_ws and (x.get_device(), 1) not in ops._skinny_ws
+    assert ops._skinny_workspace(x, 10, 39)[1] is ask(39, 10)[1]
 
 
 @pytest.mark.parametrize("M,N,K,splits,elems", [(1, 128, 64, 0, 1 * 2 * 16 * 128), (17, 129, 4096, 0, 2 * 9 * 32 * 128), (16, 4096, 4096, 4, 32 * 5 * 16 * 128),
