@@ -434,7 +434,7 @@ LLMCTL_API int llmctl_cross_entropy_fwd_bwd(void* logits, long long ld, const lo
 // The mean over the rows whose target is not ignore_index, times grad_scale, with the gradient's 1 / count.  Bound by launches: three
 // here, where the count, its reciprocal and the mean took ten of the library's around the rows' kernel.  us per call before / after:
 // 64 x 4096 76 / 26, 300 x 32000 72 / 26, 1024 x 32000 75 / 40, 4096 x 32000 148 / 116 (the rows' kernel alone 112).  One block each: 4096
-// targets are eight loads in flight per thread, and a fixed order of the sum.
+// targets are four loads in flight per thread, 8192 and more eight, and the sum has a fixed order.
 // work: fp32 [rows + 1], loss: fp32 [1].
 LLMCTL_API int llmctl_cross_entropy_mean(void* logits, long long ld, const long long* targets, float* work, int rows, int V, long long ignore_index,
                                          float grad_scale, int write_grad, float* loss, void* stream) {

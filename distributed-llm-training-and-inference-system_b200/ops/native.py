@@ -2,8 +2,7 @@
 
 The library is plain nvcc output with no torch dependency; tensors cross the boundary as raw device
 pointers plus the current CUDA stream.  Loading is lazy.  On a machine with a GPU the library MUST be
-present — ``lib()`` raises instead of letting callers fall back silently (the round-end driver records
-which ``.so`` files were actually loaded).
+present — ``lib()`` raises instead of letting callers fall back silently.
 
 Reference parity: the reference has no native layer.
 """

@@ -56,10 +56,11 @@ def choose_splits(batch: int, heads: int, max_context: int, block_size: int, sms
     # Each CTA walks block table -> K/V rows -> online softmax in a dependent chain, so HBM fills up with a few CTAs per SM and many more
     # to follow.  Splits are whole KV blocks of >= 64 tokens; the merge pass costs (head_dim + 2) floats per split, ~3 % of the K/V bytes at
     # 64 tokens per split.
-    # Up to 512 (head, sequence) pairs a CTA walks at most 512 tokens where 8 splits allow it, so that a full batch of unlike contexts ends
-    # together; more pairs fill the waves by themselves, and what each split adds is lost (us by splits, contexts from a quarter of the
-    # stated one: 16 sequences of up to 4096, 32 heads of 128 2: 109.0, 8: 110.8, 16: 118.0; 32 of them 2: 200.1, 8: 203.3; 64 1: 374.6, 4: 383.5;
-    # 256 of up to 1500 1: 551.7, 4: 575.2; 64 of up to 2304, 12 heads of 64 1: 55.3, 2: 53.9, 8: 54.3).
+    # Up to 512 (head, sequence) pairs a CTA walks at most 512 tokens where 8 splits allow it; more pairs fill the waves by themselves, and
+    # what each split adds is lost.  Around the line the splits differ by 2% either way (us by splits, contexts from a quarter of the stated
+    # one: 16 sequences of up to 4096, 32 heads of 128 2: 109.0, 8: 110.8, 16: 118.0; 32 of them 2: 200.1, 8: 203.3; 64 1: 374.6, 4: 383.5; 256 of up
+    # to 1500 1: 551.7, 4: 575.2; 64 of up to 2304, 12 heads of 64 1: 55.3, 2: 53.9, 8: 54.3); it was drawn for a kernel that took a quarter
+    # longer, whose full batches of unlike contexts gained 10% by 8 splits.
     want = max(1, (8 * sms + batch * heads - 1) // (batch * heads), min(8, (max_context + 511) // 512) if batch * heads <= 512 else 1)
     per_split = max(block_size, (64 // block_size) * block_size) if block_size <= 64 else block_size
     return int(max(1, min(want, max(1, max_context // per_split), 256)))
