@@ -69,7 +69,10 @@ _scratch_cache: dict = {}
 
 
 def _scratch(device: torch.device, nfloats: int, tag: str = "") -> torch.Tensor:
-    """Per-(device, stream, tag) fp32 scratch buffer, grown geometrically and reused across calls."""
+    """Per-(device, stream, tag) fp32 scratch buffer, grown and reused across calls; a captured call, which may be replayed beside anything, has
+    one of its own from the graph's pool."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(max(nfloats, 1), dtype=torch.float32, device=device)
     key = (device.index, native.stream_ptr(), tag)
     buf = _scratch_cache.get(key)
     if buf is None or buf.numel() < nfloats:

@@ -448,6 +448,33 @@ def test_captured_decode_products_replay_beside_others(ops):
             assert torch.equal(o, exact[n % 2])
 
 
+@pytest.mark.parametrize("norm", ["rmsnorm", "layernorm"])
+def test_captured_norm_backwards_replay_beside_others(ops, norm):
+    """Two captured backwards, replayed on two streams at once: the weights' partial sums of each lie in memory of its own."""
+    ins = [(_randn(600, 768, seed=i), (1 + _randn(768, seed=10)), _randn(600, 768, seed=20 + i)) for i in range(2)]
+
+    def run(x, w, dy):
+        x, w = x.detach().requires_grad_(True), w.detach().requires_grad_(True)
+        return torch.autograd.grad(getattr(ops, norm)(x, w)[0], (x, w), dy)
+    want = [run(*i) for i in ins]
+    torch.cuda.synchronize()
+    graphs, outs = [], []
+    for i in ins:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append([run(*i) for _ in range(8)])
+        graphs.append(g)
+    streams = [torch.cuda.Stream() for _ in graphs]
+    for _ in range(10):
+        for s, g in zip(streams, graphs):
+            with torch.cuda.stream(s):
+                g.replay()
+    torch.cuda.synchronize()
+    for got, exact in zip(outs, want):
+        for o in got:
+            _same(o, exact)
+
+
 def test_capture(ops):
     """A captured layer replays with new inputs."""
     x, w = _randn(64, 128), _randn(384, 128, seed=1)

@@ -976,3 +976,19 @@ def test_build_of_the_operator_extension(monkeypatch, tmp_path):
     assert b._operators_current(lib, src, now) and not b._operators_current(lib, src, now + 20)
     monkeypatch.setattr(torch, "__version__", "0.0.1")
     assert not b._operators_current(lib, src, now)
+
+
+def test_scratch_of_a_captured_call_is_its_own(monkeypatch):
+    """Graphs captured on one stream may be replayed beside each other: they share no buffer, with each other or with that stream's calls."""
+    from llmctl_b200.ops import functional as ops, native
+    capturing = [False]
+    monkeypatch.setattr(ops, "_scratch_cache", {})
+    monkeypatch.setattr(native, "stream_ptr", lambda: 1)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    kept = ops._scratch(torch.device("cpu"), 100, "norm")
+    assert ops._scratch(torch.device("cpu"), 50, "norm") is kept and ops._scratch(torch.device("cpu"), 50, "other") is not kept
+    capturing[0] = True
+    a, b = ops._scratch(torch.device("cpu"), 100, "norm"), ops._scratch(torch.device("cpu"), 100, "norm")
+    assert a is not kept and b is not kept and a is not b
+    capturing[0] = False
+    assert ops._scratch(torch.device("cpu"), 100, "norm") is kept
