@@ -6,7 +6,7 @@
         bench.py --gpus N --steps K --warmup W
     python bench.py --impl reference ...      # the unmodified reference from baseline/_ref (see baseline/)
 
-Metric / config follow BASELINE.json ("train tokens/sec, GPT-7B, 1/2/4/8 B200").  Workload shape mirrors the
+Metric / config: train tokens/sec of GPT-7B on 1/2/4/8 B200.  Workload shape mirrors the
 reference's own training step: micro-batch 8 sequences x 512 tokens per GPU (reference
 llmctl/runtime/engine.py:41 ``batch_size=8`` and :163 ``max_length=512``), AdamW(0.9, 0.95), global-norm
 clipping at 1.0, bf16 compute with fp32 master weights, synthetic tokens, random-init weights.  N>1 is data
@@ -318,7 +318,7 @@ def measure(args, K: int, W: int, with_e2e: bool = True, min_timed_s: float = 0.
     return res
 
 
-#: BASELINE.json configurations #2-#4, measured after the headline arm of an 8-GPU run (same process group)
+#: GPT-7B with TP + SP and with ZeRO-3, GPT-13B with TP x PP, measured after the headline arm of an 8-GPU run (same process group)
 EXTRA_ARMS_8 = {
     "tp8-sp": dict(model="gpt-7b", tp=8, pp=1, sp=True, zero_stage=None, micro_batch=8, seq_len=512, grad_accum=None),
     "dp8-zero3": dict(model="gpt-7b", tp=1, pp=1, sp=False, zero_stage=3, micro_batch=8, seq_len=512, grad_accum=None),

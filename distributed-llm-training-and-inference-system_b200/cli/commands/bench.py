@@ -112,7 +112,7 @@ def e2e(
     kernels: str = typer.Option("native", "--kernels", help="native | baseline (cuBLAS + SDPA + ATen + NCCL all-reduce, eager)"),
     out: Optional[Path] = typer.Option(None, "--out"),
 ):
-    """Serving benchmark: p50 TTFT and decode tokens/s (BASELINE.json config #5: GPT-7B TP=8, 2k prompt / 256 decode:
+    """Serving benchmark: p50 TTFT and decode tokens/s (GPT-7B TP=8, 2k prompt / 256 decode:
     ``torchrun --nproc-per-node 8 -m llmctl_b200.cli.main bench e2e --tp 8``)."""
     import os
     import torch

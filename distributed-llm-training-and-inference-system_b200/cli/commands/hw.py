@@ -5,7 +5,7 @@ Surface of reference llmctl/cli/commands/hw.py:133-345 (``probe --emit --format 
 interconnect/limits``).  The reference fills ``[limits]`` with A100 constants (312 TFLOP/s, 1935 GB/s,
 600/32 GB/s: hw.py:179-184) and benchmarks numpy on the CPU; here, when GPUs are present, the limits are
 measured: bf16 GEMM FLOP/s (tcgen05 kernel and cuBLAS), HBM copy bandwidth, per-pair P2P bandwidth and
-NVLS/multicast availability (BASELINE.json item 4).  ``detected_at`` holds a timestamp (the reference
+NVLS/multicast availability.  ``detected_at`` holds a timestamp (the reference
 stores the cwd there: hw.py:173).
 """
 from __future__ import annotations

@@ -3,7 +3,7 @@
 Same surface as reference llmctl/cli/commands/init.py:53-264 (options ``--template --size --name
 --output-dir --force``; 10 directories; ``configs/models/<template>-<size>.json``, ``configs/default.toml``,
 ``configs/data/example.toml``, ``scripts/train.sh`` (0755), ``README.md``).  Additions: the ``125m`` size
-(BASELINE.json config #1) and an error — instead of a silently missing model file — for an unknown
+(small enough for a CPU) and an error — instead of a silently missing model file — for an unknown
 template/size pair (reference init.py:95).
 """
 from __future__ import annotations

@@ -1,7 +1,6 @@
 """Token datasets and the host->device input pipeline.
 
-* ``SyntheticTokenDataset`` — deterministic pseudo-random token stream of a named shape (
-  "Inputs are synthetic data of the named shape"); sample ``i`` depends only on ``(seed, i)`` so any rank
+* ``SyntheticTokenDataset`` — deterministic pseudo-random token stream of a named shape; sample ``i`` depends only on ``(seed, i)`` so any rank
   / any resume point reproduces it.
 * ``MMapTokenDataset`` — flat binary token file (uint16/uint32/int32) memory-mapped and cut into
   fixed-length windows; ``build_token_file`` / ``index`` create one from text/jsonl (``llmctl admin index``).

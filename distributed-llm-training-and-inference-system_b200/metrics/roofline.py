@@ -1,4 +1,4 @@
-"""Roofline reporting (BASELINE.json item 5): achieved fraction of the measured peaks.
+"""Roofline reporting: achieved fraction of the measured peaks.
 
 Denominators come from ``MEASURED_PEAKS.json`` at the repo root (driver-measured copy bandwidth and
 cuBLAS bf16 throughput on this pool's B200s); the fallback numbers are the ones stated in

@@ -1,8 +1,8 @@
 """Model definition schema (the reference's model JSON) and built-in presets.
 
 Reference: reference configs/models/llama-7b.json:1-24 and the templates in reference
-llmctl/cli/commands/init.py:16-51 (gpt-7b, gpt-13b, llama-7b).  ``gpt-125m`` is added because
-BASELINE.json config #1 needs a ~125M preset that the reference does not ship.
+llmctl/cli/commands/init.py:16-51 (gpt-7b, gpt-13b, llama-7b).  ``gpt-125m`` is added for
+runs on CPU: the reference ships no preset of that size.
 """
 from __future__ import annotations
 

@@ -2,7 +2,7 @@
 
 Activations cross a stage boundary as one ``[tokens(/tp), hidden]`` bf16 tensor (the residual stream is
 folded: ``x + residual``) over ``torch.distributed`` point-to-point — NCCL on GPUs (kept on NCCL p2p by
-design, BASELINE.json), gloo on CPU.
+design), gloo on CPU.
 
 Every exchange is ONE paired group (this stage's send together with the receive it needs next).  In 1F1B the tensor
 a stage waits for is always the one its neighbour produces last, so there is no independent copy to hide: what is

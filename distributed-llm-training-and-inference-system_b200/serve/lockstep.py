@@ -11,7 +11,7 @@ and a pickled payload only when something was admitted or cancelled.  An idle le
 followers never run into the collective timeout.
 
 Reference: ``llmctl serve`` is a single process around one HF model (reference llmctl/serve/server.py:253-407,
-llmctl/cli/commands/serve.py:16-61); BASELINE.json configuration #5 asks for it at TP = 8.
+llmctl/cli/commands/serve.py:16-61); GPT-7B is served at TP = 8.
 """
 from __future__ import annotations
 

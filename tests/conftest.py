@@ -20,5 +20,5 @@ def cuda_device():
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from llmctl_b200.ops import native
-    native.lib()  # fail loudly if the extension is missing on a GPU box
+    native.lib()  # fail loudly if the library is missing on a machine with a GPU
     return torch.device("cuda", 0)

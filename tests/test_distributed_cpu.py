@@ -1,4 +1,4 @@
-"""CPU/gloo multi-process plumbing (BASELINE.json config #1): PP=2 1F1B, ZeRO-1/2/3, TP(+SP) — every
+"""CPU/gloo multi-process plumbing: PP=2 1F1B, ZeRO-1/2/3, TP(+SP) — every
 configuration must reproduce the single-process loss trajectory from identical initial weights."""
 import os
 import tempfile
