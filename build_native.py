@@ -102,7 +102,7 @@ def _compile(cmd: list[str], src: Path, obj: Path, verbose: bool) -> tuple[Path,
 
 
 def _operators_stamp() -> str:
-    """What the extension over libtorch is built for; ops/native.py loads no other."""
+    """What the extension over libtorch is built for; it refuses to be imported elsewhere."""
     import sysconfig
 
     import torch
@@ -136,6 +136,7 @@ def _build_operators(force: bool, hdr_m: float, verbose: bool) -> Path:
         return lib
     cxx = os.environ.get("CXX", "g++")
     flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             f'-DLLMCTL_TORCH_VERSION="{torch.__version__}"',
              "-I", str(ROOT / "include"), "-I", str(root / "include"), "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"),
              "-I", str(cuda / "include"), "-I", sysconfig.get_paths()["include"]]
     _compile([cxx, *flags, "-c", str(src), "-o", str(obj)], src, obj, verbose)

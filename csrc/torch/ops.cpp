@@ -23,6 +23,7 @@
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
+#include <cstdio>
 #include <initializer_list>
 
 #include "llmctl_b200.h"
@@ -596,4 +597,18 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "llmctl_ops", "Host side of the ope
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_llmctl_ops() { return PyModule_Create(&module); }
+// Under another PyTorch or Python than it was built for it might misread every tensor: it refuses to be imported there.
+PyMODINIT_FUNC PyInit_llmctl_ops() {
+  PyObject* torch = PyImport_ImportModule("torch");
+  PyObject* version = torch == nullptr ? nullptr : PyObject_GetAttrString(torch, "__version__");
+  Py_XDECREF(torch);
+  if (version == nullptr) return nullptr;
+  int major = 0, minor = 0;
+  sscanf(Py_GetVersion(), "%d.%d", &major, &minor);
+  const bool same = PyUnicode_Check(version) && PyUnicode_CompareWithASCIIString(version, LLMCTL_TORCH_VERSION) == 0 && major == PY_MAJOR_VERSION &&
+                    minor == PY_MINOR_VERSION;
+  if (!same) PyErr_Format(PyExc_ImportError, "built for PyTorch %s and Python %d.%d, this is PyTorch %S and Python %d.%d", LLMCTL_TORCH_VERSION, PY_MAJOR_VERSION,
+                          PY_MINOR_VERSION, version, major, minor);
+  Py_DECREF(version);
+  return same ? PyModule_Create(&module) : nullptr;
+}

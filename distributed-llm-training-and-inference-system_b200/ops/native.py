@@ -10,7 +10,6 @@ from __future__ import annotations
 
 import ctypes
 import importlib.util
-import sysconfig
 import threading
 import warnings
 from pathlib import Path
@@ -125,13 +124,9 @@ def _load_ops() -> None:
     """Take the operators' host side in C++ into use.  Where there is none for this PyTorch the Python operators launch the same kernels, at 10-50 us
     more of host time each, which is said once."""
     global fast
-    built = _OPS_PATH.with_suffix(".built")
-    here = f"{torch.__version__} {sysconfig.get_config_var('SOABI')}"
     try:
         if not _OPS_PATH.exists():
             raise ImportError("not built")
-        if not built.exists() or built.read_text() != here:          # built for another PyTorch it might load and misread every tensor
-            raise ImportError(f"built for {built.read_text() if built.exists() else 'another PyTorch'}, this is {here}")
         spec = importlib.util.spec_from_file_location("llmctl_ops", _OPS_PATH)
         ops = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(ops)

@@ -911,20 +911,24 @@ def test_dependent_kernels_wait_before_they_leave():
 
 
 def test_operator_extension_is_not_a_condition(monkeypatch, tmp_path):
-    """An extension that is missing, of another PyTorch or no library at all leaves the Python operators in place, and says so."""
-    import sysconfig
+    """An extension that is missing, no library at all or of another PyTorch leaves the Python operators in place, and says so."""
+    import sys
     from llmctl_b200.ops import native
-    path, here = tmp_path / "llmctl_ops.so", f"{torch.__version__} {sysconfig.get_config_var('SOABI')}"
-    monkeypatch.setattr(native, "_OPS_PATH", path)
+    built = native._OPS_PATH
+    monkeypatch.setattr(native, "_OPS_PATH", tmp_path / "llmctl_ops.so")
     monkeypatch.setattr(native, "fast", native._NoOps())
-    for content, built, why in ((None, None, "not built"), ("x", None, "another PyTorch"), ("x", "1.0 cpython-2", "1.0 cpython-2"), ("x", here, "")):
-        if content is not None:
-            path.write_text(content)
-        if built is not None:
-            path.with_suffix(".built").write_text(built)
+
+    def left_out(why):
         with pytest.warns(RuntimeWarning, match=why):
             native._load_ops()
         assert native.fast.rmsnorm(1, 2) is None and native.fast.launches() == 0
+    left_out("not built")
+    native._OPS_PATH.write_text("x")
+    left_out("not used")
+    if built.exists():
+        monkeypatch.setattr(native, "_OPS_PATH", built)
+        monkeypatch.setattr(torch, "__version__", "0.0.1")
+        left_out(f"this is PyTorch 0.0.1 and Python 3.{sys.version_info[1]}")
 
 
 def test_has_symbol_tells_a_missing_entry_from_a_library_that_does_not_load(monkeypatch):
