@@ -654,6 +654,43 @@ int main() {
     assert r.returncode == 0, r.stdout
 
 
+def test_division_by_a_launch_constant(tmp_path):
+    """csrc/common/fast_div.h against the machine's division: divisors and numbers at and around powers of two, the ends of their ranges,
+    and a spread of others."""
+    import shutil
+    import subprocess
+    root = Path(__file__).resolve().parents[1]
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("needs g++")
+    (tmp_path / "t.cpp").write_text(r"""
+#include "common/fast_div.h"
+#include <cstdio>
+#include <random>
+#include <vector>
+int main() {
+  std::mt19937 g(1);
+  std::vector<uint32_t> some = {1, 3, 5, 7, 11, 40, 148, 185, 641, 65537, 0x7fffffffu};
+  for (int b = 0; b < 31; ++b)
+    for (int e = -1; e <= 1; ++e) some.push_back((1u << b) + e);
+  for (int i = 0; i < 2000; ++i) some.push_back(g() >> (1 + g() % 30));
+  for (uint32_t d : some) {
+    if (d == 0) continue;
+    const llmctl::FastDiv f(d);
+    for (uint32_t n : some) {
+      uint32_t rem;
+      const uint32_t q = f.divide(n, rem);
+      if (q != n / d || rem != n % d) { printf("%u / %u = %u rest %u\n", n, d, q, rem); return 1; }
+    }
+  }
+  return 0;
+}
+""")
+    subprocess.run([gxx, "-O1", "-std=c++17", "-I", str(root / "csrc"), str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t")], check=True)
+    r = subprocess.run([str(tmp_path / "t")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+
+
 def test_shared_memory_limits_are_raised_and_never_lowered(tmp_path):
     """csrc/common/smem_limit.h with the runtime's two calls replaced: threads that ask for unlike sizes of one kernel leave the largest in
     place, a device counts by itself, and a call that was refused is asked again."""
