@@ -370,12 +370,11 @@ latent_attention_merge_kernel(const float* __restrict__ partial, T* __restrict__
   }
 }
 
-// Used by the tcgen05 kernel's launcher (latent_attention_t5.cu) for split contexts.
+// Used by the launchers of the tcgen05 kernels (latent_attention_t5.cu, latent_decode.cu) for split contexts.
 int launch_latent_attention_merge_bf16(const float* partial, void* out, int R, int splits, int rows, int H, const void* head_gate,
                                        long long gate_ld, cudaStream_t s) {
-  latent_attention_merge_kernel<__nv_bfloat16><<<rows, 128, 0, s>>>(partial, (__nv_bfloat16*)out, R, splits, H,
-                                                                                         (const __nv_bfloat16*)head_gate, gate_ld);
-  return 0;
+  return static_cast<int>(launch_dependent(latent_attention_merge_kernel<__nv_bfloat16>, rows, 128, 0, s, partial, (__nv_bfloat16*)out, R, splits, H,
+                                           (const __nv_bfloat16*)head_gate, gate_ld));
 }
 
 template <typename T>

@@ -219,9 +219,11 @@ class LatentAttention(nn.Module):
             rows = lops.rows_per_tile(q.dtype, s.kv_rank, s.rot_dim, q.is_cuda, s.heads if batch.decode_only else lops.ROWS_PER_TILE_WIDE)
         hpt = batch.heads_per_tile(s.heads, rows)
         span = lops.key_span(batch.max_context, s.window, rows // hpt)
+        one_token = batch.decode_only and lops.uses_tcgen05_decode(q.dtype, s.kv_rank, s.rot_dim, cache.shape[1], q.is_cuda)
         ol = lops.latent_attention(ql, q, s.dim, cache, batch.block_tables, batch.tiles(rows), batch.positions,
                                    self.rot_freq, self.rot_mult, s.scale, hpt, batch.max_context,
-                                   batch.attention_splits(s.heads, rows, span), rows=rows, sinks=self.sink, window=s.window,
+                                   batch.attention_splits(s.heads, rows, span, 1 if one_token else None), rows=rows, sinks=self.sink,
+                                   window=s.window, one_token=one_token,
                                    head_gate=d[:, self.gate_at:self.gate_at + s.heads] if s.head_gate else None)
         o = torch.empty(T, s.heads * s.vdim, dtype=ol.dtype, device=ol.device)          # the product lands head by head in place
         with torch.no_grad():

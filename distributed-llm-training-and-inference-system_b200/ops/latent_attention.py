@@ -32,6 +32,11 @@ native.register_signature("llmctl_latent_attention_t5", [c_void_p, c_int, c_ll, 
                                                           c_void_p])
 native._KERNELS_PER_CALL["llmctl_latent_attention_t5"] = 2
 
+native.register_signature("llmctl_latent_decode_ok", [c_int, c_int, c_int])
+native.register_signature("llmctl_latent_decode", [c_void_p, c_ll, c_ll, c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
+                                                    c_void_p, c_void_p, c_float, c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                                    c_void_p, c_int, c_void_p, c_ll, c_void_p])
+
 native.register_signature("llmctl_latent_prompt_prepare", [c_void_p, c_ll, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p,
                                                             c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p])
 native.register_signature("llmctl_latent_prompt_attention", [c_void_p, c_ll, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_void_p, c_int, c_int,
@@ -60,6 +65,14 @@ def uses_tcgen05(dtype: torch.dtype, R: int, dr: int, block_size: int, cuda: boo
     if not (cuda and dtype == torch.bfloat16 and native.has_symbol("llmctl_latent_attention_t5")):
         return False
     return bool(native.lib().llmctl_latent_attention_t5_ok(int(R), int(dr), int(block_size)))
+
+
+def uses_tcgen05_decode(dtype: torch.dtype, R: int, dr: int, block_size: int, cuda: bool) -> bool:
+    """bf16 on a GPU with whole blocks of 128 latent dimensions, whole 64-column panels and pages of whole 32-key boxes: single decoded tokens
+    run csrc/attention/latent_decode.cu, which has the cache rows as the long side of its products."""
+    if not (cuda and dtype == torch.bfloat16 and native.has_symbol("llmctl_latent_decode")):
+        return False
+    return bool(native.lib().llmctl_latent_decode_ok(int(R), int(dr), int(block_size)))
 
 
 def tcgen05_status(clear: bool = True) -> int:
@@ -151,14 +164,15 @@ def latent_attention(ql: torch.Tensor, q: torch.Tensor, dn: int, cache: torch.Te
                      tiles: torch.Tensor, positions: torch.Tensor, freq: torch.Tensor, mult: float, scale: float,
                      heads_per_tile: int, max_context: int, splits: int = 1, tensor_cores: bool = True,
                      rows: int = ROWS_PER_TILE, sinks: Optional[torch.Tensor] = None, window: int = 0,
-                     head_gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+                     head_gate: Optional[torch.Tensor] = None, one_token: bool = False) -> torch.Tensor:
     """ql: [T, H, R] absorbed queries (any token / head strides; fp32, or bf16 where ``uses_tensor_cores``); q: [T, H * (dn + dr)] raw queries (the rope part of each head is rotated
     here); tiles: int32 [n, 4] = (first token row, tokens, block-table row, 0) with tokens * heads_per_tile <=
     ``rows`` (16, or 32 where ``rows_per_tile`` says so), all tokens of a tile in one sequence with growing positions.  Returns [T, H, R] in q's type:
     softmax(scale * (ql . c + rot(qr) . kr)) c over cache positions 0..position of each token.  ``sinks``: fp32 [H] or None;
     ``exp(sinks[h])`` (not scaled) joins the softmax denominator of head h: a key without a value.  ``window`` > 0: a token
     sees itself and the ``window - 1`` tokens before it.  ``head_gate``: [T, H] pre-sigmoid in q's type (a view with unit
-    column stride) or None; the output of a head is multiplied by its sigmoid."""
+    column stride) or None; the output of a head is multiplied by its sigmoid.  ``one_token``: every tile holds one token (a decoding
+    batch), which ``uses_tcgen05_decode`` has a kernel for."""
     T, H, R = ql.shape
     D = cache.shape[-1]
     dr = D - R
@@ -182,6 +196,15 @@ def latent_attention(ql: torch.Tensor, q: torch.Tensor, dn: int, cache: torch.Te
                         block_tables.shape[1], block_size, tiles.data_ptr(), tiles.shape[0], T, positions.data_ptr(),
                         freq.data_ptr(), float(mult), float(scale), H, R, dr, heads_per_tile, splits, per, native.ptr(qfull),
                         out.data_ptr(), native.ptr(partial), native.ptr(sinks), int(window), native.ptr(head_gate),
+                        head_gate.stride(0) if head_gate is not None else 0, native.stream_ptr())
+            return out
+        if (one_token and tensor_cores and ql.dtype == torch.bfloat16 and heads_per_tile <= ROWS_PER_TILE_WIDE and ql.stride(0) % 8 == 0
+                and ql.stride(1) % 8 == 0 and ql.data_ptr() % 16 == 0 and cache.data_ptr() % 16 == 0
+                and uses_tcgen05_decode(q.dtype, R, dr, block_size, True)):
+            native.call("llmctl_latent_decode", ql.data_ptr(), ql.stride(0), ql.stride(1), q.data_ptr(), q.stride(0), dn, cache.data_ptr(),
+                        cache.shape[0] * block_size, block_tables.data_ptr(), block_tables.shape[1], block_size, tiles.data_ptr(), tiles.shape[0], T,
+                        positions.data_ptr(), freq.data_ptr(), float(mult), float(scale), H, R, dr, heads_per_tile, splits, per, out.data_ptr(),
+                        native.ptr(partial), native.ptr(sinks), int(window), native.ptr(head_gate),
                         head_gate.stride(0) if head_gate is not None else 0, native.stream_ptr())
             return out
         native.call("llmctl_latent_attention", ql.data_ptr(), int(ql.dtype == torch.bfloat16), ql.stride(0), ql.stride(1),

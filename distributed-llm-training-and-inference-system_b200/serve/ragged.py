@@ -147,16 +147,18 @@ class RaggedBatch:
         up to ``rows`` heads when every sequence decodes."""
         return min(heads, rows) if self.decode_only else 1
 
-    def attention_splits(self, heads: int, rows: int = ROWS_PER_TILE, span: Optional[int] = None) -> int:
+    def attention_splits(self, heads: int, rows: int = ROWS_PER_TILE, span: Optional[int] = None, per_sm: Optional[int] = None) -> int:
         """Split the keys of long contexts over CTAs when the tiles alone would leave most SMs idle.  ``span``: most keys a
-        tile reads (the longest context unless a window bounds it)."""
+        tile reads (the longest context unless a window bounds it); ``per_sm``: CTAs of the decoding kernel that an SM holds, where
+        ``rows`` does not say it."""
         hpt = self.heads_per_tile(heads, rows)
         groups = (heads + hpt - 1) // hpt
         longest = self.max_context if span is None else span
         if self.decode_only and rows in (ROWS_PER_TILE, ROWS_PER_TILE_WIDE):
-            key = (rows, groups, longest)
+            per_sm = per_sm or (2 if rows == ROWS_PER_TILE else 1)
+            key = (per_sm, groups, longest)
             if key not in self._splits:
-                self._splits[key] = self._even_splits(self._sms * (2 if rows == ROWS_PER_TILE else 1), groups, longest)
+                self._splits[key] = self._even_splits(self._sms * per_sm, groups, longest)
             return self._splits[key]
         ctas = self._tiles[rows].shape[0] * groups
         return int(max(1, min(2 * self._sms // max(ctas, 1), longest // 64)))

@@ -283,6 +283,13 @@ int llmctl_latent_attention_t5(const void* ql, int ql_bf16, long long ql_st, lon
                                const float* freq, float mult, float scale, int H, int R, int dr, int heads_per_tile,
                                int splits, int keys_per_split, void* qfull, void* out, float* partial, const float* sinks, int window,
                                const void* head_gate, long long gate_ld, void* stream);
+/* Single decoded tokens on tcgen05 with the cache rows as the long side (csrc/attention/latent_decode.cu): sizes that qualify, and the launch.
+ * tiles of one token, up to 32 heads per tile, bf16 absorbed queries in rows that begin at 16-byte boundaries. */
+int llmctl_latent_decode_ok(int R, int dr, int block_size);
+int llmctl_latent_decode(const void* ql, long long ql_st, long long ql_sh, const void* q, long long ldq, int dn, const void* cache, long long cache_rows,
+                         const int* block_tables, int max_blocks, int block_size, const int* tiles, int ntiles, int tokens, const int* positions,
+                         const float* freq, float mult, float scale, int H, int R, int dr, int heads_per_tile, int splits, int keys_per_split, void* out,
+                         float* partial, const float* sinks, int window, const void* head_gate, long long gate_ld, void* stream);
 int llmctl_moe_tile_rows(void);
 /* correction: fp32 [E] added to the scores for the CHOICE only, or null; n_groups > 1: only experts of the keep_groups
  * best groups (of E / n_groups neighbours each) can be chosen, a group's score being its best (group_best 1) or the sum of

@@ -149,6 +149,51 @@ def test_latent_attention_tcgen05(cuda_device, H, dn, dr, R, bs):
             close(out, ref, dt, 4)
 
 
+@pytest.mark.parametrize("contexts,H,dr,R,bs,splits,window,sink,gate", [
+    ([1, 64, 65, 300], 16, 64, 512, 64, 1, 0, False, False),          # one key, whole tiles, one key more; two stages
+    ([1, 63, 128, 700, 129], 16, 64, 512, 64, 3, 0, False, True),     # splits past the short contexts
+    ([200, 31], 5, 0, 128, 32, 1, 0, True, False),                    # fewer heads than columns, four stages, pages of 32
+    ([1000, 97], 32, 64, 512, 64, 5, 0, True, True),                  # 32 columns
+    ([500, 33, 64], 40, 64, 256, 96, 2, 100, True, False),            # two groups of heads, window not at a tile, pages of 96
+    ([2000], 17, 64, 384, 64, 2, 64, False, True)])
+def test_latent_decode_tcgen05(cuda_device, contexts, H, dr, R, bs, splits, window, sink, gate):
+    """Single tokens on the tcgen05 kernel against the PyTorch restatement in fp32, with NaN in every cache row that no token may see.  bf16
+    queries are equal on both sides; probabilities and outputs are rounded to bf16: 2^-9 each, with a factor of 2 on their sum."""
+    from llmctl_b200.ops import latent_attention as L, native
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+    torch.manual_seed(len(contexts) + H)
+    dn = 8
+    pages = [(c + bs - 1) // bs for c in contexts]
+    perm, at, tables = torch.randperm(sum(pages) + 1).tolist(), 0, []
+    for n in pages:
+        tables.append(perm[at:at + n])
+        at += n
+    cache = torch.full((sum(pages) + 1, bs, R + dr), float("nan"), dtype=torch.bfloat16)
+    for c, t in zip(contexts, tables):
+        for j in range(c):
+            cache[t[j // bs], j % bs] = torch.randn(R + dr).bfloat16()
+    T = len(contexts)
+    ql, q = torch.randn(H, T, R).bfloat16(), torch.randn(T, H * (dn + dr)).bfloat16()
+    freq, sinks = torch.rand(max(dr // 2, 1)), torch.randn(H) if sink else None
+    gates = torch.randn(T, H).bfloat16() if gate else None
+    portions = [Portion(i, [0], c - 1, [0], t) for i, (c, t) in enumerate(zip(contexts, tables))]
+    got = []
+    for dev in ("cpu", "cuda"):
+        b = RaggedBatch(portions, bs, torch.device(dev))
+        mv = lambda t: None if t is None else t.to(dev)       # noqa: E731
+        before = native.launch_count
+        rows = L.ROWS_PER_TILE_WIDE if H > 16 else L.ROWS_PER_TILE
+        got.append(L.latent_attention((ql if dev == "cuda" else ql.float()).to(dev).transpose(0, 1), mv(q), dn, mv(cache), b.block_tables, b.tiles(rows), b.positions,
+                                      mv(freq), 1.0, 0.1, b.heads_per_tile(H, rows), b.max_context, splits, rows=rows, sinks=mv(sinks), window=window,
+                                      head_gate=mv(gates), one_token=True))
+        assert dev == "cpu" or native.launch_count > before
+    want, have = got[0].float(), got[1].float().cpu()
+    assert torch.isfinite(have).all()
+    for i in range(T):
+        err = (have[i] - want[i]).norm() / want[i].norm()
+        assert err < 2 * 2 * 2 ** -9, (contexts[i], float(err))
+
+
 # (tokens, position of the first) of the batch's portions: one prompt around the 128-key and 256-query blocks, portions behind earlier
 # keys at positions that are and are not multiples of 128, unlike lengths side by side, a single token among them
 @pytest.mark.parametrize("portions", [[(64, 0)], [(127, 0)], [(128, 0)], [(129, 0)], [(257, 0)], [(700, 0)], [(300, 128)], [(300, 1)],
