@@ -6,6 +6,8 @@
 // Reference: HF modules choose SDPA/eager attention behind `self.model(**batch)` (reference
 // llmctl/runtime/engine.py:284); the reference's tuner times a naive softmax(QK^T)V (reference
 // llmctl/plugins/autotuning.py:149-188).  Baseline to beat: cuDNN / flash-attn SDPA.
+#include <math.h>
+
 #include "../common/ptx.cuh"
 #include "../common/tma_host.h"
 #include "../common/util.cuh"
@@ -166,7 +168,11 @@ __device__ __forceinline__ void softmax_block(uint32_t tS, uint32_t tO, int q, i
 // item's Q tiles as soon as the last Q K^T of the current one has retired, and the MMA warp starts the next
 // item's Q K^T while the softmax warpgroups are still normalising and storing O of the current one (O goes
 // from registers straight to global memory, so no staging buffer blocks the Q prefetch).
-template <int DQK, int DV>
+//
+// kSplit: an item is one tile of 128 queries whose keys the two softmax warpgroups share, A the first half of the key blocks, B the rest
+// (with the diagonal); every K/V tile then serves one of them.  Both accumulators lie in the same lanes of TMEM, so each warpgroup puts half of the
+// columns together.  For grids whose longest item decides: its chain of blocks is half as long (see split_keys).
+template <int DQK, int DV, bool kSplit>
 __global__ void __launch_bounds__(ffwd::kThreads, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmKs, const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ O,
@@ -180,6 +186,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __shared__ uint64_t bar_s[2], bar_p0[2], bar_p1[2], bar_o[2], bar_ofree[2];
   __shared__ uint32_t tmem_base_smem;
   __shared__ int abort_flag;
+  __shared__ float2 half_ml[kSplit ? 2 : 1][kRows];      // reference and sum of a row over each half of the keys
+  __shared__ uint64_t bar_half[2];
+  constexpr int kItemRows = kSplit ? kRows : 2 * kRows;
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));      // layout: Q_A, Q_B, K ring, V ring
@@ -193,7 +202,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_init(&bar_p0[i], 4);
       mbar_init(&bar_p1[i], 4);
       mbar_init(&bar_o[i], 1);
-      mbar_init(&bar_ofree[i], 4);
+      mbar_init(&bar_half[i], 4);
+      mbar_init(&bar_ofree[i], kSplit ? 8 : 4);
     }
     for (int i = 0; i < C::kKStages; ++i) {
       mbar_init(&bar_kfull[i], 1);
@@ -246,7 +256,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // False: a shorter sequence of the batch has no such block.
   auto decode = [&](int item, int& q0, int& head, int& b, Seq& sq) {
     uint32_t rem, h;
-    q0 = (order.nqb - 1 - static_cast<int>(order.per_qb.divide(item, rem))) * 2 * kRows;
+    q0 = (order.nqb - 1 - static_cast<int>(order.per_qb.divide(item, rem))) * kItemRows;
     b = static_cast<int>(order.heads.divide(rem, h));
     head = static_cast<int>(h);
     if (seqs != nullptr)
@@ -257,6 +267,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   };
   // key blocks of tile t of an item; a tile past the end of its sequence has none
   auto blocks = [&](const Seq& sq, int q0, int t) {
+    if constexpr (kSplit) {
+      const int all = static_cast<int>((sq.start + sq.n + kRows - 1u) / kRows);
+      const int n = causal ? min(all, static_cast<int>((sq.start + q0 + kRows - 1u) / kRows) + 1) : all;
+      return (n + 1 - t) >> 1;
+    }
     const int qt = q0 + t * kRows;
     if (qt >= sq.n) return 0;
     const int all = static_cast<int>((sq.start + sq.n + kRows - 1u) / kRows);
@@ -278,9 +293,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         int q0, head, b;
         Seq sq;
         if (!decode(item, q0, head, b, sq)) continue;
-        const int nblk = max(blocks(sq, q0, 0), blocks(sq, q0, 1));
+        const int nblk_a = blocks(sq, q0, 0), nblk = kSplit ? nblk_a + blocks(sq, q0, 1) : max(nblk_a, blocks(sq, q0, 1));
         const int bc = seqs != nullptr ? 0 : b;          // batch coordinate of the maps
-        const bool validB = q0 + kRows < sq.n;
+        const bool validB = !kSplit && q0 + kRows < sq.n;
         ev(3, 40);
         auto load_q = [&](int t, uint32_t done) {
           if (!mbar_wait_bounded(&bar_qfree[t], (done & 1u) ^ 1u, abort)) return false;      // the previous item's last Q K^T has retired
@@ -294,7 +309,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         ++nA;
         for (int j = 0; j < nblk; ++j, ++g) {
           const uint32_t ks = g % C::kKStages, vs = g % C::kVStages;
-          const int row = sq.k_row + j * kRows;
+          const int row = sq.k_row + (kSplit ? (j & 1 ? nblk_a : 0) + (j >> 1) : j) * kRows;
           uint8_t* sK = smem + C::kKAt + ks * C::kQTile;
           uint8_t* sV = smem + C::kVAt + vs * C::kVTile;
           if (!(ok = mbar_wait_bounded(&bar_kempty[ks], ((g / C::kKStages) & 1u) ^ 1u, abort))) break;
@@ -354,10 +369,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int nblk_t0 = blocks(sq, q0, 0), nblk_t1 = blocks(sq, q0, 1);
       const int nblk = max(nblk_t0, nblk_t1);
       auto issue_qk = [&](int t, int j, bool release_k, bool last) {
-        const uint32_t g = g0 + j, st = g % C::kKStages;
+        const uint32_t g = kSplit ? g0 + 2 * j + t : g0 + j, st = g % C::kKStages;
         wait(&bar_kfull[st], (g / C::kKStages) & 1u);
         tc_fence_after();
-        const uint64_t qd = make_smem_desc(smem_base + t * C::kQTile, 16, 1024, 2);
+        const uint64_t qd = make_smem_desc(smem_base + (kSplit ? 0 : t * C::kQTile), 16, 1024, 2);
         const uint64_t kd = make_smem_desc(smem_base + C::kKAt + st * C::kQTile, 16, 1024, 2);
         if (elect_one()) {
 #pragma unroll
@@ -366,14 +381,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             umma_ss<1>(tmem_base + t * 128, qd + off, kd + off, idesc_qk, ks != 0 ? 1u : 0u);
           }
           umma_commit<1>(&bar_s[t]);
-          if (release_k) umma_commit<1>(&bar_kempty[st]);
-          if (last) umma_commit<1>(&bar_qfree[t]);       // last use of this item's Q_t
+          if (kSplit || release_k) umma_commit<1>(&bar_kempty[st]);
+          if (kSplit ? t == (nblk_t1 > 0 && nblk_t1 == nblk_t0 ? 1 : 0) && j + 1 == nblk_t0 : last) umma_commit<1>(&bar_qfree[kSplit ? 0 : t]);      // last use of this item's Q_t
         }
       };
       // P V of tile t and block j, then Q K^T of its block j + 1
       auto step = [&](int t, int j, int mine, int other, uint32_t nQ, uint32_t nP) {
-        const uint32_t vs = (g0 + j) % C::kVStages;
-        wait(&bar_vfull[vs], ((g0 + j) / C::kVStages) & 1u);
+        const uint32_t g = kSplit ? g0 + 2 * j + t : g0 + j, vs = g % C::kVStages;
+        wait(&bar_vfull[vs], (g / C::kVStages) & 1u);
         wait(&bar_p0[t], nP & 1u);                       // first half of P_t(j) is in TMEM, O_t rescaled if needed
         if (j == 0 && nQ > 0) wait(&bar_ofree[t], (nQ - 1) & 1u);                    // previous item's O_t was read out
         tc_fence_after();
@@ -391,7 +406,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
           for (int ks = kRows / 32; ks < kRows / 16; ++ks)
             umma_ts<1>(tOt, tP + ks * 8, vd + ks * (2048 >> 4), idesc_pv, 1u);
-          if (t == 1 || j >= other) umma_commit<1>(&bar_vempty[vs]);    // last reader of V(j)
+          if (kSplit || t == 1 || j >= other) umma_commit<1>(&bar_vempty[vs]);    // last reader of V(j)
           if (j + 1 == mine) umma_commit<1>(&bar_o[t]);
         }
         if (j + 1 < mine) issue_qk(t, j + 1, t == 1 || j + 1 >= other, j + 2 == mine);
@@ -399,14 +414,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       wait(&bar_q[0], nQ0 & 1u);
       issue_qk(0, 0, nblk_t1 == 0, nblk_t0 == 1);
       if (nblk_t1 > 0) {
-        wait(&bar_q[1], nQ1 & 1u);
+        if (!kSplit) wait(&bar_q[1], nQ1 & 1u);
         issue_qk(1, 0, true, nblk_t1 == 1);
       }
       for (int j = 0; j < nblk; ++j) {
         if (j < nblk_t0) step(0, j, nblk_t0, nblk_t1, nQ0, nP0++);
         if (j < nblk_t1) step(1, j, nblk_t1, nblk_t0, nQ1, nP1++);
       }
-      g0 += nblk;
+      g0 += kSplit ? nblk_t0 + nblk_t1 : nblk;
       ++nQ0;
       if (nblk_t1 > 0) ++nQ1;
     }
@@ -421,21 +436,21 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t tS = tmem_base + t * 128 + lane_off;
     const uint32_t tOt = tmem_base + 256 + t * 128 + lane_off;
     uint32_t nS = 0;                               // S tiles consumed so far (bar_s phase)
-    uint32_t nO = 0;                               // items finished by this tile (bar_o phase)
+    uint32_t nO = 0, nOb = 0;                      // items finished by this tile (bar_o phase); split items with a second half
     for (int item, r = 0; next_item(r, item); ++r) {
       int q0, head, b;
       Seq sq;
       if (!decode(item, q0, head, b, sq)) continue;
       const int nb = blocks(sq, q0, t);
-      if (nb == 0) continue;                       // tile B past the end of the sequence: nobody touches its barriers
-      const int qt0 = q0 + t * kRows;
+      if (!kSplit && nb == 0) continue;            // tile B past the end of the sequence: nobody touches its barriers
+      const int qt0 = kSplit ? q0 : q0 + t * kRows, first_block = kSplit && t == 1 ? blocks(sq, q0, 0) : 0;
       float m_ref = -INFINITY, l0 = 0.f, l1 = 0.f;
       for (int j = 0; j < nb; ++j, ++nS) {
         mbar_wait_or_abort(&bar_s[t], nS & 1u, abort);
         __syncwarp();
         tc_fence_after();
         if (q == 0 && lane == 0) ev(t, 1);
-        const int off = sq.start + qt0 - j * kRows;      // the tile's first row sees the block's columns up to this one
+        const int off = sq.start + qt0 - (first_block + j) * kRows;      // the tile's first row sees the block's columns up to this one
         if (causal && off < kRows - 1)
           softmax_block<true, DV>(tS, tOt, q, lane, off, j == 0, scale_log2, m_ref, l0, l1, &bar_p0[t], &bar_p1[t]);
         else
@@ -443,24 +458,58 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (q == 0 && lane == 0) ev(t, 2);
       }
       // ---- epilogue: O / l -> bf16 -> global (row per thread, whole 32-byte sectors), LSE ----
-      mbar_wait_or_abort(&bar_o[t], nO & 1u, abort);
+      float l = l0 + l1, by[2] = {1.f, 1.f};
+      const bool both = kSplit && blocks(sq, q0, 1) > 0;
+      if constexpr (kSplit) {
+        // bar_ofree: the other warpgroup has read what stands there from the item before (and has passed its wait for this barrier's phase)
+        if (nO > 0) mbar_wait_or_abort(&bar_ofree[0], (nO - 1) & 1u, abort);
+        half_ml[t][row] = make_float2(m_ref, l);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_half[t]);
+        mbar_wait_or_abort(&bar_half[1 - t], nO & 1u, abort);
+        const float2 other = half_ml[1 - t][row];
+        const float m = fmaxf(m_ref, other.x);             // A's half has a visible key for every row
+        by[t] = ex2_approx(m_ref - m);
+        by[1 - t] = ex2_approx(other.x - m);
+        l = l * by[t] + other.y * by[1 - t];
+        m_ref = m;
+        if (both) mbar_wait_or_abort(&bar_o[1], nOb++ & 1u, abort);
+      }
+      mbar_wait_or_abort(&bar_o[kSplit ? 0 : t], nO & 1u, abort);
       __syncwarp();
       ++nO;
       tc_fence_after();
-      const float l = l0 + l1;
       const float inv_l = 1.f / l;
+      constexpr int kChunks = kSplit ? DV / 64 : DV / 32;  // of 32 columns, that this warpgroup stores
+      const int c0 = kSplit ? t * kChunks : 0;
+      const uint32_t tOa = kSplit ? tmem_base + 256 + lane_off : tOt;
       const bool real = qt0 + row < sq.n;
       const long long tok = seqs != nullptr ? sq.q_row + qt0 + row : static_cast<long long>(b) * max_q + qt0 + row;
-      __nv_bfloat16* orow = O + tok * o_tok_stride + head * DV;
+      __nv_bfloat16* orow = O + tok * o_tok_stride + head * DV + c0 * 32;
 #pragma unroll
-      for (int c = 0; c < DV / 32; ++c) {
+      for (int c = 0; c < kChunks; ++c) {
         uint32_t r[32];
-        tmem_ld_x32(tOt + c * 32, r);
-        tmem_ld_wait();
-        if (c == DV / 32 - 1) {                    // O_t is in registers: the next item's P V may overwrite it
+        tmem_ld_x32(tOa + (c0 + c) * 32, r);
+        if constexpr (kSplit) {
+          uint32_t r1[32];
+          if (both) tmem_ld_x32(tOa + 128 + (c0 + c) * 32, r1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            float x = __uint_as_float(r[e]) * by[0];
+            if (both) x += __uint_as_float(r1[e]) * by[1];
+            r[e] = __float_as_uint(x);
+          }
+        } else {
+          tmem_ld_wait();
+        }
+        if (c == kChunks - 1) {                    // O_t is in registers: the next item's P V may overwrite it
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&bar_ofree[t]);
+          if (lane == 0) {
+            mbar_arrive(&bar_ofree[kSplit ? 0 : t]);
+            if (both) mbar_arrive(&bar_ofree[1]);
+          }
         }
         if (!real) continue;
 #pragma unroll
@@ -478,7 +527,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
       }
-      if (lse != nullptr && real)
+      if (lse != nullptr && real && (!kSplit || t == 0))
         lse[(static_cast<long long>(b) * H + head) * max_q + qt0 + row] = (m_ref + log2f(l)) * 0.6931471805599453f;
       if (q == 0 && lane == 0) ev(t, 3);
     }
@@ -510,22 +559,37 @@ static long long* flash_trace_buffer() {
   return buf;
 }
 
+// Whether items of one tile whose keys are split (kSplit) are the better ones: by the steps (a block of both warpgroups, 1.5 us at D = 128) of the
+// busiest CTA, which is the longest item's where the others do not fill the SMs, and 1.7 steps for each of its items; split items are twice as
+// many and read the keys twice as often, so they must be a fifth ahead.  us, pairs of tiles / split (sequences x tokens x heads x size):
+// 1 x 129 x 12 x 64 6.6 / 4.8, 1 x 300 x 12 x 64 6.9 / 5.9, 1 x 777 x 12 x 64 12.9 / 9.0, 1 x 2000 x 12 x 64 27.7 / 17.0, 1 x 4000 x 12 x 64 51.5 / 45.1,
+// 2 x 1024 x 12 x 64 16.2 / 11.5, 1 x 1500 x 16 x 128 24.8 / 16.4, 2 x 700 x 16 x 128 14.9 / 13.6; left as pairs:
+// 1 x 600 x 32 x 128 12.8 / 11.2, 1 x 1200 x 32 x 128 21.9 / 22.5, 1 x 1000 x 40 x 128 19.1 / 21.2, 4 x 333 x 16 x 128 9.0 / 11.7, 1 x 1777 x 32 x 128 29.2 / 34.8, 8 x 512 x 32 x 128 34.0 / 45.0.
+static bool split_keys(int B, int S, int H, int causal) {
+  const double heads = static_cast<double>(B) * H, n = (S + ffwd::kRows - 1) / ffwd::kRows, half = ceil(n / 2), odd = 2 * half - n;
+  if (n < 2) return false;
+  auto cost = [&](double longest, double steps, double items) { return fmax(longest, heads * steps / kNumSMs) + 1.7 * ceil(heads * items / kNumSMs); };
+  const double pairs = cost(n, causal ? half * (half + 1) - odd : half * n, half);
+  return 1.2 * cost(half, causal ? half * (half + 1) - odd * half : half * n, n) < pairs;
+}
+
 // Persistent launch: one CTA per SM over a heavy-first item list.
-template <int DQK, int DV>
+template <int DQK, int DV, bool kSplit = false>
 static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& ks, const CUtensorMap& v, void* o,
                             long long o_tok_stride, float* lse, const ffwd::Seq* seqs, int B, int max_q, int H, int head_step, float scale, int causal,
                             cudaStream_t s) {
   using namespace ffwd;
   using C = Cfg<DQK, DV>;
-  const cudaError_t e = allow_smem(flash_fwd_kernel<DQK, DV>, C::kSmem);
+  const cudaError_t e = allow_smem(flash_fwd_kernel<DQK, DV, kSplit>, C::kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  const long long nqb = (max_q + 2 * kRows - 1) / (2 * kRows), n_items = nqb * H * B;
+  constexpr int kItemRows = kSplit ? kRows : 2 * kRows;
+  const long long nqb = (max_q + kItemRows - 1) / kItemRows, n_items = nqb * H * B;
   if (n_items >= (1ll << 31) - 2 * kNumSMs) return static_cast<int>(cudaErrorInvalidValue);
   const int grid = n_items < kNumSMs ? static_cast<int>(n_items) : kNumSMs;
   unsigned char* const wait_byte = wait_report(kWaitFlashForward);
   if (wait_byte == nullptr) return static_cast<int>(cudaErrorMemoryAllocation);
   const int wide = o_tok_stride % 16 == 0 && (reinterpret_cast<uintptr_t>(o) & 31) == 0;
-  return static_cast<int>(launch_dependent(flash_fwd_kernel<DQK, DV>, grid, kThreads, C::kSmem, s, q, k, ks, v, (__nv_bfloat16*)o, o_tok_stride, wide, lse, seqs,
+  return static_cast<int>(launch_dependent(flash_fwd_kernel<DQK, DV, kSplit>, grid, kThreads, C::kSmem, s, q, k, ks, v, (__nv_bfloat16*)o, o_tok_stride, wide, lse, seqs,
                                            Order{static_cast<int>(n_items), static_cast<int>(nqb), FastDiv(H * B), FastDiv(H)}, max_q, H, head_step, scale * 1.4426950408889634f, causal, wait_byte, flash_trace_buffer()));
 }
 
@@ -579,7 +643,8 @@ LLMCTL_API int llmctl_flash_attn_fwd(const void* q, const void* k, const void* v
     mkmap(&tv, v, v_tok_stride, H);
   }
   if (rc) LLMCTL_FAIL(rc, "tensor map Q / K / V");
-  rc = (D == 128 ? flash_fwd_launch<128, 128> : flash_fwd_launch<64, 64>)(tq, tk, tk, tv, o, o_tok_stride, lse, nullptr, B, S, H,
+  const bool split = split_keys(B, S, H, causal);
+  rc = (D == 128 ? (split ? flash_fwd_launch<128, 128, true> : flash_fwd_launch<128, 128>) : split ? flash_fwd_launch<64, 64, true> : flash_fwd_launch<64, 64>)(tq, tk, tk, tv, o, o_tok_stride, lse, nullptr, B, S, H,
                                                                           packed ? H : 0, scale, causal, (cudaStream_t)stream);
   if (rc) LLMCTL_FAIL(rc, "flash forward");
   return 0;

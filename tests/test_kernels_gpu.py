@@ -525,6 +525,33 @@ def test_flash_attention_edges_of_blocks(cuda_device, B, S, H, D, causal, shift)
             assert (a - b).norm() <= bound, f"{name} head {h}: {((a - b).norm() / b.norm()).item():.2e}"
 
 
+# Keys split between the two warpgroups: one block and two (the second half has one or none), odd and even counts, a ragged end, more tiles
+# than SMs, no mask.
+@pytest.mark.parametrize("B,S,H,D,causal", [(1, 129, 2, 64, True), (1, 256, 3, 128, True), (1, 385, 3, 64, True), (2, 600, 2, 128, True), (1, 2000, 12, 64, True),
+                                            (1, 1500, 16, 128, True), (1, 640, 2, 64, False), (2, 768, 2, 128, False)])
+def test_flash_attention_split_keys(cuda_device, B, S, H, D, causal):
+    """Output against float64 (P and the output are rounded to bf16: 2 x 2^-9 in the 2-norm) and the log-sum-exp against float64 sums of exact
+    products (fp32 sums of up to S terms and the approximate exponential: 1e-5 of the largest)."""
+    from llmctl_b200.ops import attention as attn, native
+    torch.manual_seed(S)
+    qkv = torch.randn(B, S, 3, H, D, device=cuda_device).bfloat16()
+    q, k, v = (qkv[:, :, i] for i in range(3))
+    o, lse = torch.empty(B, S, H, D, dtype=torch.bfloat16, device=cuda_device), torch.empty(B, H, S, device=cuda_device)
+    native.call("llmctl_flash_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B, S, H, D, q.stride(1), k.stride(1),
+                v.stride(1), o.stride(1), 1.0 / math.sqrt(D), int(causal), native.stream_ptr())
+    assert native.lib().llmctl_flash_fwd_status(1) == 0
+    with torch.no_grad():
+        assert torch.equal(attn.attention(q, k, v, causal=causal), o)
+    for h in range(H):
+        s = q[:, :, h].double() @ k[:, :, h].double().transpose(-1, -2) / math.sqrt(D)
+        if causal:
+            s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device=cuda_device).triu(1), float("-inf"))
+        want = torch.softmax(s, -1) @ v[:, :, h].double()
+        assert (o[:, :, h].double() - want).norm() <= 2 * 2.0 ** -9 * want.norm()
+        exact = torch.logsumexp(s, -1)
+        assert (lse[:, h].double() - exact).abs().max() <= 1e-5 * exact.abs().max().clamp(min=1)
+
+
 @pytest.mark.parametrize("which", [0, 1, 2])
 def test_whole_tiles_at_odd_addresses_are_copied(cuda_device, which):
     """Heads of 128 and whole 128-token tiles where one of q, k and v begins at an odd address: the kernels run on copies, and nothing else
