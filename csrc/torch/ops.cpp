@@ -20,6 +20,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
@@ -37,8 +38,8 @@ using at::Tensor;
 // ---------------------------------------------------------------------------------------------------------------------------------
 #define LLMCTL_ENTRIES(X)                                                                                                         \
   X(llmctl_rmsnorm_fwd) X(llmctl_rmsnorm_bwd) X(llmctl_rope_inplace) X(llmctl_gemm_bf16) X(llmctl_gemm_swiglu_bf16)               \
-  X(llmctl_gemm_swiglu_bwd_bf16) X(llmctl_gemm_skinny_bf16) X(llmctl_gemm_skinny_scratch_elems) X(llmctl_flash_attn_fwd) X(llmctl_flash_attn_bwd) X(llmctl_kv_append) \
-  X(llmctl_paged_attn_decode) X(llmctl_paged_attn_scratch_elems)
+  X(llmctl_gemm_swiglu_bwd_bf16) X(llmctl_swiglu_bwd) X(llmctl_gemm_skinny_bf16) X(llmctl_gemm_skinny_scratch_elems) X(llmctl_flash_attn_fwd) X(llmctl_flash_attn_bwd) X(llmctl_kv_append) \
+  X(llmctl_paged_attn_decode) X(llmctl_paged_attn_scratch_elems) X(llmctl_latent_kv_write) X(llmctl_latent_decode)
 struct Entries {
 #define X(name) decltype(&::name) name = nullptr;
   LLMCTL_ENTRIES(X)
@@ -49,6 +50,7 @@ struct Entries {
 
 PyObject* native_error = nullptr;                // ops.native.NativeError
 PyObject* check_waits = nullptr;                 // ops.native.check_waits
+PyObject* buffered_wgrad = nullptr;              // ops.functional._wgrad
 std::atomic<long long> launches{0};
 
 // Whether an entry can be called: it is there and no wait has run out (the Python operator reports that one).
@@ -307,13 +309,172 @@ Tensor as_shape_of(const Tensor& y, const Tensor& x) {
   return y.view(size);
 }
 
-// linear(x, w, tile_n, workspace or None) -> x @ w.T where no gradient is recorded; few rows take the decode GEMM, whose partials and tickets
+// dyT x of a weight; where the weight has a buffer for its gradient (main_grad, looked up now: it may come and go between the passes) through the
+// Python operator, which accumulates into it, and nothing is returned.
+Tensor wgrad(const Tensor& dy, const Tensor& x, const Tensor& w, int tile_n) {
+  {
+    pybind11::gil_scoped_acquire gil;
+    PyObject *o = THPVariable_Wrap(w), *dict = PyObject_GenericGetDict(o, nullptr);
+    PyObject* buffer = dict == nullptr ? nullptr : PyDict_GetItemString(dict, "main_grad");
+    const bool buffered = buffer != nullptr && buffer != Py_None;
+    PyErr_Clear();
+    Py_XDECREF(dict);
+    PyObject* r = nullptr;
+    if (buffered) {
+      PyObject *a = THPVariable_Wrap(dy), *b = THPVariable_Wrap(x);
+      r = PyObject_CallFunctionObjArgs(buffered_wgrad, a, b, o, nullptr);
+      Py_XDECREF(a);
+      Py_XDECREF(b);
+    }
+    Py_DECREF(o);
+    if (buffered) {
+      if (r == nullptr) {
+        python_error e;
+        e.persist();
+        throw e;
+      }
+      Tensor out = r == Py_None ? Tensor() : THPVariable_Unpack(r);
+      Py_DECREF(r);
+      return out;
+    }
+  }
+  Tensor dw = new_bf16(w, w.sizes());
+  gemm(dy, x, dw, true, true, false, tile_n, 0);
+  return dw;
+}
+Tensor dgrad(const Tensor& dy, const Tensor& w, int tile_n) {
+  Tensor dx = new_bf16(dy, {dy.size(0), w.size(1)});
+  gemm(dy, w, dx, false, true, false, tile_n, 0);
+  return dx;
+}
+
+// Nodes of the products: saved tensors and a lock, as autograd's own nodes have them.
+struct Products : torch::autograd::Node {
+  std::vector<torch::autograd::SavedVariable> saved;
+  int tile_n = 0;
+  void keep(std::initializer_list<const Tensor*> ts) {
+    saved.reserve(ts.size());
+    for (const Tensor* t : ts) saved.emplace_back(*t, false);
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    for (auto& t : saved) t.reset_data();
+  }
+  // the gradient as an operand
+  static Tensor rows(const Tensor& g) { return is_matrix(g) ? g : whole_units(g); }
+};
+template <typename T>
+std::shared_ptr<T> new_node(torch::autograd::edge_list&& next, int tile_n) {
+  std::shared_ptr<T> node(new T(), torch::autograd::deleteNode);
+  node->set_next_edges(std::move(next));
+  node->tile_n = tile_n;
+  return node;
+}
+
+struct LinearNode final : Products {
+  static Tensor record(const Tensor& x, const Tensor& w, int tile_n) {
+    auto node = new_node<LinearNode>(torch::autograd::collect_next_edges(x, w), tile_n);
+    node->keep({&x, &w});
+    Tensor y = new_bf16(x, {x.size(0), w.size(0)});
+    gemm(x, w, y, false, false, false, tile_n, 0);
+    torch::autograd::set_history(y, node);
+    return y;
+  }
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    if (!grads[0].defined()) return {Tensor(), Tensor()};
+    return node_body("llmctl_gemm_bf16", ready(lib.llmctl_gemm_bf16), [&]() -> torch::autograd::variable_list {
+      const Tensor x = saved[0].unpack(), w = saved[1].unpack();
+      at::AutoDispatchBelowADInplaceOrView below;
+      const Tensor dy = rows(grads[0]);
+      Tensor dx, dw;
+      if (task_should_compute_output(0)) dx = dgrad(dy, w, tile_n);
+      if (task_should_compute_output(1)) dw = wgrad(dy, x, w, tile_n);
+      return {dx, dw};
+    });
+  }
+  std::string name() const override { return "LinearBackward"; }
+};
+
+// act = swiglu(x @ w.T) and the product before
+std::pair<Tensor, Tensor> up_and_activate(const Tensor& x, const Tensor& w, bool keep) {
+  const int64_t M = x.size(0), F = w.size(0) / 2;
+  Tensor act = new_bf16(x, {M, F}), gu = keep ? new_bf16(x, {M, 2 * F}) : Tensor();
+  done("llmctl_gemm_swiglu_bf16", lib.llmctl_gemm_swiglu_bf16(cdata(x), cdata(w), keep ? data(gu) : nullptr, data(act), static_cast<int>(M), static_cast<int>(F),
+                                                              static_cast<int>(x.size(1)), x.stride(0), w.stride(0), 2 * F, F, stream()));
+  return {act, gu};
+}
+
+struct LinearSwigluNode final : Products {
+  static Tensor record(const Tensor& x, const Tensor& w) {
+    auto node = new_node<LinearSwigluNode>(torch::autograd::collect_next_edges(x, w), 0);
+    const auto [act, gu] = up_and_activate(x, w, true);
+    node->keep({&x, &w, &gu});
+    torch::autograd::set_history(act, node);
+    return act;
+  }
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    if (!grads[0].defined()) return {Tensor(), Tensor()};
+    return node_body("llmctl_swiglu_bwd", ready(lib.llmctl_swiglu_bwd) && lib.llmctl_gemm_bf16, [&]() -> torch::autograd::variable_list {
+      const Tensor x = saved[0].unpack(), w = saved[1].unpack(), gu = saved[2].unpack();
+      at::AutoDispatchBelowADInplaceOrView below;
+      const Tensor dact = whole_units(grads[0]);
+      Tensor dgu = new_bf16(gu, gu.sizes()), dx, dw;
+      done("llmctl_swiglu_bwd", lib.llmctl_swiglu_bwd(cdata(dact), cdata(gu), data(dgu), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2), gu.stride(0), ::stream()));
+      if (task_should_compute_output(0)) dx = dgrad(dgu, w, 0);
+      if (task_should_compute_output(1)) dw = wgrad(dgu, x, w, 0);
+      return {dx, dw};
+    });
+  }
+  std::string name() const override { return "LinearSwigluBackward"; }
+};
+
+// swiglu(x @ up.T) @ down.T: the gradient of the product of the two halves goes straight into theirs
+struct SwigluMlpNode final : Products {
+  static Tensor record(const Tensor& x, const Tensor& up, const Tensor& down) {
+    auto node = new_node<SwigluMlpNode>(torch::autograd::collect_next_edges(x, up, down), 0);
+    const auto [act, gu] = up_and_activate(x, up, true);
+    node->keep({&x, &up, &down, &gu, &act});
+    Tensor y = new_bf16(x, {x.size(0), down.size(0)});
+    gemm(act, down, y, false, false, false, 0, 0);
+    torch::autograd::set_history(y, node);
+    return y;
+  }
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
+    return node_body("llmctl_gemm_swiglu_bwd_bf16", ready(lib.llmctl_gemm_swiglu_bwd_bf16) && lib.llmctl_gemm_bf16, [&]() -> torch::autograd::variable_list {
+      const Tensor x = saved[0].unpack(), up = saved[1].unpack(), down = saved[2].unpack(), gu = saved[3].unpack(), act = saved[4].unpack();
+      at::AutoDispatchBelowADInplaceOrView below;
+      const Tensor dy = rows(grads[0]);
+      Tensor dgu, dx, d_up, d_down;
+      if (task_should_compute_output(0) || task_should_compute_output(1)) {
+        dgu = new_bf16(gu, gu.sizes());
+        done("llmctl_gemm_swiglu_bwd_bf16",
+             lib.llmctl_gemm_swiglu_bwd_bf16(cdata(dy), cdata(down), cdata(gu), data(dgu), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2),
+                                             static_cast<int>(dy.size(1)), dy.stride(0), down.stride(0), gu.stride(0), ::stream()));
+      }
+      if (task_should_compute_output(2)) d_down = wgrad(dy, act, down, 0);
+      if (task_should_compute_output(0)) dx = dgrad(dgu, up, 0);
+      if (task_should_compute_output(1)) d_up = wgrad(dgu, x, up, 0);
+      return {dx, d_up, d_down};
+    });
+  }
+  std::string name() const override { return "SwigluMlpBackward"; }
+};
+
+// linear(x, w, tile_n, workspace or None) -> x @ w.T; where no gradient is recorded few rows take the decode GEMM, whose partials and tickets
 // workspace(x, floats of partials, stream) returns
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return call(a, n, 4, [&](Args& args) -> PyObject* {
     const Tensor x = args.tensor(0), w = args.tensor(1);
     const int tile_n = static_cast<int>(args.integer(2));
-    if (!args.ok || !quiet() || !is_matrix(w) || x.numel() == 0 || recorded({&x, &w})) return none();
+    if (!args.ok || !quiet() || !is_matrix(w) || x.numel() == 0) return none();
+    if (recorded({&x, &w})) {
+      if (!ready(lib.llmctl_gemm_bf16) || !is_matrix(x) || x.size(1) != w.size(1) || w.size(0) % 8 || w.size(1) % 8) return none();
+      return THPVariable_Wrap(without_gil([&] { return LinearNode::record(x, w, tile_n); }));
+    }
     const Tensor rows = as_rows(x);
     if (!rows.defined() || rows.size(1) != w.size(1)) return none();
     const bool skinny = a[3] != Py_None;
@@ -349,35 +510,35 @@ PyObject* py_gemm_swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool keep = args.integer(2);
     if (!args.ok || !quiet() || !ready(lib.llmctl_gemm_swiglu_bf16) || !is_matrix(x) || !is_matrix(w) || x.size(1) != w.size(1) || w.size(0) % 16) return none();
     Tensor act, gu;
-    without_gil([&] {
-      const int64_t M = x.size(0), F = w.size(0) / 2;
-      act = new_bf16(x, {M, F});
-      if (keep) gu = new_bf16(x, {M, 2 * F});
-      done("llmctl_gemm_swiglu_bf16", lib.llmctl_gemm_swiglu_bf16(cdata(x), cdata(w), keep ? data(gu) : nullptr, data(act), static_cast<int>(M), static_cast<int>(F),
-                                                                  static_cast<int>(x.size(1)), x.stride(0), w.stride(0), 2 * F, F, stream()));
-    });
+    without_gil([&] { std::tie(act, gu) = up_and_activate(x, w, keep); });
     if (keep) return pair(act, THPVariable_Wrap(gu));
     Py_INCREF(Py_None);
     return pair(act, Py_None);
   });
 }
 
-// mlp(x, w_up, w_down, tile_n) -> swiglu(x @ w_up.T) @ w_down.T where no gradient is recorded
+// mlp(x, w_up, w_down, least, fused) -> swiglu(x @ w_up.T) @ w_down.T for more than `least` rows; where a gradient is recorded as one node if the
+// down-projection has at least `fused` rows (and the product before it needs a gradient), else as two
 PyObject* py_mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return call(a, n, 4, [&](Args& args) -> PyObject* {
+  return call(a, n, 5, [&](Args& args) -> PyObject* {
     const Tensor x = args.tensor(0), up = args.tensor(1), down = args.tensor(2);
-    const int least = static_cast<int>(args.integer(3));
+    const int least = static_cast<int>(args.integer(3)), fused = static_cast<int>(args.integer(4));
     if (!args.ok || !quiet() || !ready(lib.llmctl_gemm_swiglu_bf16) || !ready(lib.llmctl_gemm_bf16) || !is_matrix(up) || !is_matrix(down) || x.numel() == 0 ||
-        recorded({&x, &up, &down}) || up.size(0) % 16 || down.size(0) % 8 || down.size(1) != up.size(0) / 2)
+        up.size(0) % 16 || down.size(0) % 8 || down.size(1) != up.size(0) / 2)
       return none();
+    if (recorded({&x, &up, &down})) {
+      if (!ready(lib.llmctl_gemm_swiglu_bwd_bf16) || !ready(lib.llmctl_swiglu_bwd) || !is_matrix(x) || x.size(1) != up.size(1) || x.size(0) <= least || up.size(1) % 8) return none();
+      return THPVariable_Wrap(without_gil([&] {
+        const bool first = x.requires_grad() || up.requires_grad();
+        if (first && down.size(0) >= fused) return SwigluMlpNode::record(x, up, down);
+        return LinearNode::record(first ? LinearSwigluNode::record(x, up) : up_and_activate(x, up, false).first, down, 0);
+      }));
+    }
     const Tensor rows = as_rows(x);
     if (!rows.defined() || rows.size(1) != up.size(1) || rows.size(0) <= least) return none();
     Tensor y = without_gil([&] {
-      const int64_t M = rows.size(0), F = up.size(0) / 2;
-      Tensor act = new_bf16(x, {M, F}), out = new_bf16(x, {M, down.size(0)});
-      done("llmctl_gemm_swiglu_bf16", lib.llmctl_gemm_swiglu_bf16(cdata(rows), cdata(up), nullptr, data(act), static_cast<int>(M), static_cast<int>(F),
-                                                                  static_cast<int>(rows.size(1)), rows.stride(0), up.stride(0), 2 * F, F, stream()));
-      gemm(act, down, out, false, false, false, 0, 0);
+      Tensor out = new_bf16(x, {rows.size(0), down.size(0)});
+      gemm(up_and_activate(rows, up, false).first, down, out, false, false, false, 0, 0);
       return as_shape_of(out, x);
     });
     return THPVariable_Wrap(y);
@@ -423,21 +584,43 @@ Tensor attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor&
   return d;
 }
 
-struct FlashAttention : torch::autograd::Function<FlashAttention> {
-  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal) {
+// A node of its own: torch::autograd::Function looks its arguments up by name, and wraps and checks them in ways that this operator, which returns
+// one new tensor, has no use for (forward and backward of a small call 72 us; the engine alone takes 29).
+struct FlashAttention final : torch::autograd::Node {
+  torch::autograd::SavedVariable q, k, v, o, lse;
+  double scale = 0;
+  bool causal = true;
+
+  static Tensor record(const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal) {
+    std::shared_ptr<FlashAttention> node(new FlashAttention(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
+    node->q = {q, false};
+    node->k = {k, false};
+    node->v = {v, false};
+    node->scale = scale;
+    node->causal = causal;
     AttnOut r = attn_fwd(q, k, v, scale, causal, true);
-    ctx->save_for_backward({q, k, v, r.o, r.lse});
-    ctx->saved_data["scale"] = scale;
-    ctx->saved_data["causal"] = causal;
+    torch::autograd::set_history(r.o, node);
+    node->o = {r.o, true};
+    node->lse = {r.lse, false};
     return r.o;
   }
-  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
     return node_body("llmctl_flash_attn_bwd", ready(lib.llmctl_flash_attn_bwd), [&]() -> torch::autograd::variable_list {
-      const auto s = ctx->get_saved_variables();
-      const Tensor d = attn_bwd(s[0], s[1], s[2], s[3], s[4], grads[0], ctx->saved_data["scale"].toDouble(), ctx->saved_data["causal"].toBool());
-      return {d.select(2, 0), d.select(2, 1), d.select(2, 2), Tensor(), Tensor()};
+      const auto self = getptr();
+      const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), o_ = o.unpack(self), lse_ = lse.unpack();
+      at::AutoDispatchBelowADInplaceOrView below;
+      const Tensor d = attn_bwd(q_, k_, v_, o_, lse_, grads[0], scale, causal);
+      return {d.select(2, 0), d.select(2, 1), d.select(2, 2)};
     });
   }
+  void release_variables() override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    for (auto* t : {&q, &k, &v, &o, &lse}) t->reset_data();
+  }
+  std::string name() const override { return "FlashAttentionBackward"; }
 };
 
 // attention(q, k, v, scale, causal) -> [B, S, H, D]
@@ -448,7 +631,7 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool causal = args.integer(4);
     if (!args.ok || !quiet() || !ready(lib.llmctl_flash_attn_fwd) || !lib.llmctl_flash_attn_bwd || !attention_ok(q, k, v, causal)) return none();
     const bool grad = recorded({&q, &k, &v});
-    Tensor o = without_gil([&] { return grad ? FlashAttention::apply(q, k, v, scale, causal) : attn_fwd(q, k, v, scale, causal, false).o; });
+    Tensor o = without_gil([&] { return grad ? FlashAttention::record(q, k, v, scale, causal) : attn_fwd(q, k, v, scale, causal, false).o; });
     return THPVariable_Wrap(o);
   });
 }
@@ -516,6 +699,46 @@ PyObject* py_rope_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// block(x, residual or None, norm1, qkv, out, norm2, up, down, cos, sin, positions or None, B, S, H, D, eps, scale, tile_n, least) -> (y, residual): a
+// decoder layer (RMS norms, packed projection, rotation, causal attention, gated MLP) where no gradient is recorded, as one call.  Layer by
+// layer from Python 12 of them cost 62 us each, as long as their kernels at 777 tokens of width 768.
+PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 19, [&](Args& args) -> PyObject* {
+    const Tensor x = args.tensor(0), residual = args.optional(1), n1 = args.tensor(2), qkv = args.tensor(3), out = args.tensor(4), n2 = args.tensor(5), up = args.tensor(6),
+                 down = args.tensor(7), cos = args.tensor(8), sin = args.tensor(9), positions = args.optional(10);
+    const int64_t B = args.integer(11), S = args.integer(12), H = args.integer(13), D = args.integer(14);
+    const double eps = args.number(15), scale = args.number(16);
+    const int tile_n = static_cast<int>(args.integer(17)), least = static_cast<int>(args.integer(18));
+    if (!args.ok || at::GradMode::is_enabled() || !quiet() || !ready(lib.llmctl_rmsnorm_fwd) || !ready(lib.llmctl_gemm_bf16) || !ready(lib.llmctl_rope_inplace) ||
+        !ready(lib.llmctl_flash_attn_fwd) || !ready(lib.llmctl_gemm_swiglu_bf16))
+      return none();
+    if (!bf16(x) || x.dim() != 2 || !x.is_contiguous() || !unit16(x) || B < 1 || S < 1 || H < 1 || (D != 64 && D != 128) || x.size(0) != B * S || x.size(0) <= least) return none();
+    const int64_t T = x.size(0), W = x.size(1), F = down.dim() == 2 ? down.size(1) : 0;
+    auto weight = [&](const Tensor& w, int64_t rows, int64_t cols) { return is_matrix(w) && w.size(0) == rows && w.size(1) == cols && rows % 8 == 0; };
+    auto norm = [&](const Tensor& w) { return bf16(w) && w.dim() == 1 && w.size(0) == W && w.is_contiguous() && unit16(w); };
+    if (F < 8 || F % 8 || W % 8 || !norm(n1) || !norm(n2) || !weight(qkv, 3 * H * D, W) || !weight(out, W, H * D) || !weight(up, 2 * F, W) || !weight(down, W, F)) return none();
+    if (residual.defined() && (!bf16(residual) || !residual.is_contiguous() || residual.sizes() != x.sizes() || !unit16(residual))) return none();
+    if (cos.scalar_type() != at::kFloat || sin.scalar_type() != at::kFloat || !cos.is_contiguous() || !sin.is_contiguous()) return none();
+    if (positions.defined() && (positions.scalar_type() != at::kInt || !positions.is_contiguous() || positions.numel() != T)) return none();
+    Tensor y, r;
+    without_gil([&] {
+      auto linear = [&](const Tensor& in, const Tensor& w) {
+        Tensor to = new_bf16(in, {T, w.size(0)});
+        gemm(in, w, to, false, false, false, tile_n, 0);
+        return to;
+      };
+      const NormOut first = norm_fwd(x, residual, n1, eps, false);
+      const Tensor p = linear(first.y, qkv);
+      rope(p, cos, sin, positions, S, 2 * H, D, 1.f);
+      const Packed z = unpack(p, B, S, H, D);
+      const NormOut second = norm_fwd(linear(attn_fwd(z.q, z.k, z.v, scale, true, false).o.view({T, H * D}), out), first.h, n2, eps, false);
+      y = linear(up_and_activate(second.y, up, false).first, down);
+      r = second.h;
+    });
+    return pair(y, THPVariable_Wrap(r));
+  });
+}
+
 // ---------------------------------------------------------------------------------------------------------------------------------
 // paged cache
 // ---------------------------------------------------------------------------------------------------------------------------------
@@ -566,13 +789,85 @@ PyObject* py_paged_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------------
+// latent attention
+// ---------------------------------------------------------------------------------------------------------------------------------
+bool is_indices(const Tensor& t, at::ScalarType type, int64_t least) { return t.scalar_type() == type && t.is_contiguous() && t.numel() >= least; }
+
+// latent_kv_write(d, Q, R, dr, wq or None, wkv or None, cache or None, slots, positions, freq, mult, eps) -> the normed query latent, or True without one
+PyObject* py_latent_kv_write(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 12, [&](Args& args) -> PyObject* {
+    const Tensor d = args.tensor(0), wq = args.optional(4), wkv = args.optional(5), cache = args.optional(6), slots = args.tensor(7), positions = args.tensor(8),
+                 freq = args.tensor(9);
+    const int64_t Q = args.integer(1), R = args.integer(2), dr = args.integer(3);
+    const double mult = args.number(10), eps = args.number(11);
+    if (!args.ok || !quiet() || !ready(lib.llmctl_latent_kv_write) || !bf16(d) || d.dim() != 2 || d.numel() == 0 || d.stride(1) != 1 || Q < 0 || R < 0 || dr < 0 || Q + R < 1 ||
+        d.size(1) < Q + R + dr || recorded({&d}))
+      return none();
+    auto norm = [&](const Tensor& w, int64_t size) { return size == 0 || (w.defined() && bf16(w) && w.dim() == 1 && w.size(0) == size && w.is_contiguous()); };
+    if (!norm(wq, Q) || !norm(wkv, R) || (R > 0 && (!cache.defined() || !bf16(cache) || !cache.is_contiguous() || cache.dim() != 3 || cache.size(2) != R + dr)) ||
+        !is_indices(slots, at::kLong, d.size(0)) || !is_indices(positions, at::kInt, d.size(0)) || !is_indices(freq, at::kFloat, dr / 2))
+      return none();
+    auto at = [](const Tensor& t) { return t.defined() ? cdata(t) : nullptr; };
+    Tensor cq;
+    without_gil([&] {
+      if (Q > 0) cq = new_bf16(d, {d.size(0), Q});
+      done("llmctl_latent_kv_write", lib.llmctl_latent_kv_write(cdata(d), d.stride(0), static_cast<int>(Q), static_cast<int>(R), static_cast<int>(dr), at(wq), at(wkv),
+                                                                Q > 0 ? data(cq) : nullptr, R > 0 ? data(cache) : nullptr, static_cast<const long long*>(cdata(slots)),
+                                                                static_cast<const int*>(cdata(positions)), static_cast<const float*>(cdata(freq)), static_cast<float>(mult),
+                                                                static_cast<float>(eps), static_cast<int>(d.size(0)), 0, stream()));
+    });
+    if (Q == 0) Py_RETURN_TRUE;
+    return THPVariable_Wrap(cq);
+  });
+}
+
+// latent_decode(q, dn, w_uk, w_uv, cache, tables, tiles, positions, freq, mult, scale, heads_per_tile, splits, keys_per_split, sinks or None, window,
+// gate or None) -> [T, heads * dv]: absorbed queries, attention over the cache, values, for tokens whose kernel is llmctl_latent_decode
+PyObject* py_latent_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return call(a, n, 17, [&](Args& args) -> PyObject* {
+    const Tensor q = args.tensor(0), uk = args.tensor(2), uv = args.tensor(3), cache = args.tensor(4), tables = args.tensor(5), tiles = args.tensor(6),
+                 positions = args.tensor(7), freq = args.tensor(8), sinks = args.optional(14), gate = args.optional(16);
+    const int64_t dn = args.integer(1), splits = args.integer(12), per = args.integer(13);
+    const double mult = args.number(9), scale = args.number(10);
+    const int hpt = static_cast<int>(args.integer(11)), window = static_cast<int>(args.integer(15));
+    if (!args.ok || !quiet() || !ready(lib.llmctl_latent_decode) || !bf16(q) || q.dim() != 2 || q.numel() == 0 || q.stride(1) != 1 || !bf16(uk) || !bf16(uv) || uk.dim() != 3 ||
+        uv.dim() != 3 || recorded({&q, &uk, &uv}) || !bf16(cache) || cache.dim() != 3 || !cache.is_contiguous() || !unit16(cache))
+      return none();
+    const int64_t T = q.size(0), H = uk.size(0), R = uk.size(2), D = cache.size(2), dr = D - R, dv = uv.size(1);
+    if (dr < 0 || uk.size(1) != dn || q.size(1) < H * (dn + dr) || uv.size(0) != H || uv.size(2) != R || hpt < 1 || hpt > 32 || splits < 1 || tables.dim() != 2 ||
+        !is_indices(tables, at::kInt, 1) || !is_indices(tiles, at::kInt, 4) || !is_indices(positions, at::kInt, T) || !is_indices(freq, at::kFloat, dr / 2))
+      return none();
+    if (sinks.defined() && !is_indices(sinks, at::kFloat, H)) return none();
+    if (gate.defined() && (!bf16(gate) || gate.dim() != 2 || gate.size(0) != T || gate.size(1) != H || gate.stride(1) != 1)) return none();
+    Tensor o = without_gil([&] {
+      at::AutoDispatchBelowADInplaceOrView below;
+      const Tensor ql = at::bmm(q.as_strided({H, T, dn}, {dn + dr, q.stride(0), 1}), uk);            // [H, T, R]
+      Tensor ol = new_bf16(q, {T, H, R}), out = new_bf16(q, {T, H * dv});
+      Tensor partial = splits > 1 ? new_f32(q, {T * H * splits * (R + 2)}) : Tensor();
+      done("llmctl_latent_decode",
+           lib.llmctl_latent_decode(cdata(ql), ql.stride(1), ql.stride(0), cdata(q), q.stride(0), static_cast<int>(dn), cdata(cache), cache.size(0) * cache.size(1),
+                                    static_cast<const int*>(cdata(tables)), static_cast<int>(tables.size(1)), static_cast<int>(cache.size(1)), static_cast<const int*>(cdata(tiles)),
+                                    static_cast<int>(tiles.size(0)), static_cast<int>(T), static_cast<const int*>(cdata(positions)), static_cast<const float*>(cdata(freq)),
+                                    static_cast<float>(mult), static_cast<float>(scale), static_cast<int>(H), static_cast<int>(R), static_cast<int>(dr), hpt, static_cast<int>(splits),
+                                    static_cast<int>(per), data(ol), splits > 1 ? static_cast<float*>(data(partial)) : nullptr,
+                                    sinks.defined() ? static_cast<const float*>(cdata(sinks)) : nullptr, window, gate.defined() ? cdata(gate) : nullptr,
+                                    gate.defined() ? gate.stride(0) : 0, stream()), splits > 1 ? 2 : 1);
+      Tensor by_head = out.as_strided({H, T, dv}, {dv, H * dv, 1});                                   // the product lands head by head in place
+      at::bmm_out(by_head, ol.transpose(0, 1), uv.transpose(1, 2));
+      return out;
+    });
+    return THPVariable_Wrap(o);
+  });
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------------
 // the module
 // ---------------------------------------------------------------------------------------------------------------------------------
-// bind(path of the loaded kernel library, NativeError, check_waits)
+// bind(path of the loaded kernel library, NativeError, check_waits, gradient of a weight with a buffer for it)
 PyObject* py_bind(PyObject*, PyObject* args) {
   const char* path;
-  PyObject *error, *waits;
-  if (!PyArg_ParseTuple(args, "sOO", &path, &error, &waits)) return nullptr;
+  PyObject *error, *waits, *wgrad;
+  if (!PyArg_ParseTuple(args, "sOOO", &path, &error, &waits, &wgrad)) return nullptr;
   void* so = dlopen(path, RTLD_NOW | RTLD_NOLOAD);
   if (so == nullptr) {
     PyErr_Format(PyExc_RuntimeError, "%s is not loaded", path);
@@ -584,15 +879,17 @@ PyObject* py_bind(PyObject*, PyObject* args) {
   lib.wait_word = reinterpret_cast<void* (*)()>(dlsym(so, "llmctl_wait_status_word"));
   Py_INCREF(error);
   Py_INCREF(waits);
+  Py_INCREF(wgrad);
   native_error = error;
   check_waits = waits;
+  buffered_wgrad = wgrad;
   Py_RETURN_NONE;
 }
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(launches.load(std::memory_order_relaxed)); }
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"bind", py_bind, METH_VARARGS, nullptr}, {"launches", py_launches, METH_NOARGS, nullptr}, FAST(rmsnorm), FAST(gemm), FAST(linear), FAST(gemm_swiglu),
-                         FAST(mlp), FAST(attention), FAST(rope_attention), FAST(kv_append), FAST(paged_decode), {nullptr, nullptr, 0, nullptr}};
+                         FAST(mlp), FAST(attention), FAST(rope_attention), FAST(block), FAST(kv_append), FAST(paged_decode), FAST(latent_kv_write), FAST(latent_decode), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "llmctl_ops", "Host side of the operators (csrc/torch/ops.cpp)", -1, methods};
 
 }  // namespace

@@ -101,11 +101,29 @@ class Block(nn.Module):
         self.norm2 = Norm(cfg, dtype, device)
         self.mlp = MLP(cfg, dtype, device)
 
+    def _plain(self) -> bool:
+        """Whether the layer is what ``ops.decoder_block`` computes: the modules that stand here, on one rank, with nothing that wants to see
+        their calls."""
+        n1, n2, attn, mlp = self.norm1, self.norm2, self.attn, self.mlp
+        return (type(n1) is Norm and type(n2) is Norm and type(attn) is Attention and type(mlp) is MLP and n1.kind == n2.kind == "rmsnorm"
+                and n1.eps == n2.eps and mlp.gated and tpl.untouched(n1, _NORM) and tpl.untouched(n2, _NORM) and tpl.untouched(attn, _ATTENTION)
+                and tpl.untouched(mlp, _MLP) and tpl.runs_plain(attn.qkv) and tpl.runs_plain(attn.out) and tpl.runs_plain(mlp.up)
+                and tpl.runs_plain(mlp.down))
+
     def forward(self, x, residual, rope_cos, rope_sin, batch: int, seq: int, positions=None):
+        if x.is_cuda and not torch.is_grad_enabled() and x.shape[0] > ops.SKINNY_MAX_ROWS and self._plain():
+            attn, mlp = self.attn, self.mlp
+            done = ops.decoder_block(x, residual, self.norm1.weight, attn.qkv.weight, attn.out.weight, self.norm2.weight, mlp.up.weight, mlp.down.weight,
+                                     rope_cos, rope_sin, positions, batch, seq, attn.heads_local, attn.head_dim, self.norm1.eps)
+            if done is not None:
+                return done
         y, residual = self.norm1(x, residual)
         a = self.attn(y, (rope_cos, rope_sin), batch, seq, positions)
         y, residual = self.norm2(a, residual)
         return self.mlp(y), residual
+
+
+_NORM, _ATTENTION, _MLP = Norm.forward, Attention.forward, MLP.forward
 
 
 class GPTModel(nn.Module):

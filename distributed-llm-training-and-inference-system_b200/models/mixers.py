@@ -200,6 +200,16 @@ class LatentAttention(nn.Module):
                 o = lops.latent_prompt_attention(q, s.dim, cache, batch.block_tables, batch.seqs, batch.key_rows, batch.max_tokens,
                                                  batch.positions, self.rot_freq, self.rot_mult, s.scale, self.w_uk, self.w_uv)
             return self._project(o, d)
+        one_token = batch.decode_only and lops.uses_tcgen05_decode(q.dtype, s.kv_rank, s.rot_dim, cache.shape[1], q.is_cuda)
+        gate = d[:, self.gate_at:self.gate_at + s.heads] if s.head_gate else None
+        if one_token:
+            rows = lops.rows_per_tile(q.dtype, s.kv_rank, s.rot_dim, True, s.heads)
+            hpt = batch.heads_per_tile(s.heads, rows)
+            span = lops.key_span(batch.max_context, s.window, rows // hpt)
+            o = lops.latent_decode(q, s.dim, self.w_uk, self.w_uv, cache, batch.block_tables, batch.tiles(rows), batch.positions, self.rot_freq,
+                                   self.rot_mult, s.scale, hpt, span, batch.attention_splits(s.heads, rows, span, 1), self.sink, s.window, gate)
+            if o is not None:
+                return self._project(o, d)
         qn = q.unflatten(1, (s.heads, s.dim + s.rot_dim))[:, :, :s.dim].transpose(0, 1) # [H, T, dn], a view
         # absorbed queries ql[t, h] = Uk_h^T qn[t, h]: fp32, except that the tensor-core attention kernel takes them
         # in bf16 (it multiplies in bf16 anyway); the kernel reads the [H, T, R] product through its strides
@@ -219,12 +229,10 @@ class LatentAttention(nn.Module):
             rows = lops.rows_per_tile(q.dtype, s.kv_rank, s.rot_dim, q.is_cuda, s.heads if batch.decode_only else lops.ROWS_PER_TILE_WIDE)
         hpt = batch.heads_per_tile(s.heads, rows)
         span = lops.key_span(batch.max_context, s.window, rows // hpt)
-        one_token = batch.decode_only and lops.uses_tcgen05_decode(q.dtype, s.kv_rank, s.rot_dim, cache.shape[1], q.is_cuda)
         ol = lops.latent_attention(ql, q, s.dim, cache, batch.block_tables, batch.tiles(rows), batch.positions,
                                    self.rot_freq, self.rot_mult, s.scale, hpt, batch.max_context,
                                    batch.attention_splits(s.heads, rows, span, 1 if one_token else None), rows=rows, sinks=self.sink,
-                                   window=s.window, one_token=one_token,
-                                   head_gate=d[:, self.gate_at:self.gate_at + s.heads] if s.head_gate else None)
+                                   window=s.window, one_token=one_token, head_gate=gate)
         o = torch.empty(T, s.heads * s.vdim, dtype=ol.dtype, device=ol.device)          # the product lands head by head in place
         with torch.no_grad():
             torch.bmm(ol.transpose(0, 1), self.w_uv.transpose(1, 2), out=o.view(T, s.heads, s.vdim).transpose(0, 1))

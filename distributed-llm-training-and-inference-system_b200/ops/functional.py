@@ -594,7 +594,7 @@ def swiglu_mlp(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor) -> tor
     inside the product that precedes it; everything else composes ``linear_swiglu`` and ``linear``."""
     if (_cfg.gemm == "native" and _cfg.elementwise == "native" and _cfg.gemm_tile_n == 0 and getattr(w_up, "_k8_gate", None) is None
             and getattr(w_down, "_k8_gate", None) is None):
-        y = native.fast.mlp(x, w_up, w_down, SKINNY_MAX_ROWS)
+        y = native.fast.mlp(x, w_up, w_down, SKINNY_MAX_ROWS, SWIGLU_BWD_COLS)
         if y is not None:
             return y
     fused = w_down.shape[0] >= SWIGLU_BWD_COLS and torch.is_grad_enabled() and (x.requires_grad or w_up.requires_grad)
@@ -603,6 +603,19 @@ def swiglu_mlp(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor) -> tor
             or not _gemm_ok(w_down)):
         return linear(linear_swiglu(x, w_up), w_down)
     return native.apply(_SwiGLUMLPFn, x2, w_up, w_down).view(*x.shape[:-1], w_down.shape[0])
+
+
+def decoder_block(x: torch.Tensor, residual: Optional[torch.Tensor], norm1: torch.Tensor, qkv: torch.Tensor, out: torch.Tensor, norm2: torch.Tensor,
+                  up: torch.Tensor, down: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, positions: Optional[torch.Tensor], batch: int, seq: int,
+                  heads: int, head_dim: int, eps: float):
+    """A decoder layer without gradients, as one call: ``y, r = rmsnorm(x, residual)``, packed projection, rotation, causal attention and output
+    projection, ``y, r = rmsnorm(., r)``, gated MLP.  Returns (y, r), or None where the operators' extension does not take it (the operators
+    that the layer is made of then do the same)."""
+    if (_cfg.gemm != "native" or _cfg.elementwise != "native" or _cfg.attention != "native" or _cfg.gemm_tile_n != 0
+            or any(getattr(w, "_k8_gate", None) is not None for w in (qkv, out, up, down))):
+        return None
+    return native.fast.block(x, residual, norm1, qkv, out, norm2, up, down, cos, sin, None if positions is None else positions.to(torch.int32), batch, seq, heads,
+                             head_dim, eps, head_dim ** -0.5, 0, SKINNY_MAX_ROWS)
 
 
 class _SwiGLULinearFn(torch.autograd.Function):

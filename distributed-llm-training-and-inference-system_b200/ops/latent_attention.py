@@ -9,6 +9,7 @@ sigmoid gate per (token, head).  CPU tensors run a PyTorch restatement.
 Reference: none — the reference has no attention code (reference llmctl/serve/server.py:199-204)."""
 from __future__ import annotations
 
+from functools import lru_cache
 from typing import Optional
 
 import torch
@@ -70,9 +71,22 @@ def uses_tcgen05(dtype: torch.dtype, R: int, dr: int, block_size: int, cuda: boo
 def uses_tcgen05_decode(dtype: torch.dtype, R: int, dr: int, block_size: int, cuda: bool) -> bool:
     """bf16 on a GPU with whole blocks of 128 latent dimensions, whole 64-column panels and pages of whole 32-key boxes: single decoded tokens
     run csrc/attention/latent_decode.cu, which has the cache rows as the long side of its products."""
-    if not (cuda and dtype == torch.bfloat16 and native.has_symbol("llmctl_latent_decode")):
-        return False
-    return bool(native.lib().llmctl_latent_decode_ok(int(R), int(dr), int(block_size)))
+    return cuda and dtype == torch.bfloat16 and native.has_symbol("llmctl_latent_decode") and _decode_sizes(R, dr, block_size)
+
+
+@lru_cache(maxsize=256)
+def _decode_sizes(R: int, dr: int, block_size: int) -> bool:
+    return bool(native.lib().llmctl_latent_decode_ok(R, dr, block_size))
+
+
+def latent_decode(q: torch.Tensor, dn: int, w_uk: torch.Tensor, w_uv: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tensor,
+                  tiles: torch.Tensor, positions: torch.Tensor, freq: torch.Tensor, mult: float, scale: float, heads_per_tile: int, span: int,
+                  splits: int, sinks: Optional[torch.Tensor], window: int, head_gate: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """Queries [T, H * (dn + dr)] -> heads [T, H * dv] of a decoding batch without gradients, absorbed queries, attention and values in one call;
+    None where the operators' extension does not take it (``latent_attention`` and the products around it then do the same)."""
+    per = max(64, (-(-span // splits) + 63) // 64 * 64)
+    return native.fast.latent_decode(q, dn, w_uk, w_uv, cache, block_tables, tiles, positions, freq, mult, scale, heads_per_tile, splits, per, sinks, window,
+                                     head_gate)
 
 
 def tcgen05_status(clear: bool = True) -> int:
@@ -140,6 +154,9 @@ def latent_kv_write(d: torch.Tensor, Q: int, R: int, dr: int, wq: Optional[torch
     ``cache`` ([blocks, block_size, R + dr]) at ``slots`` (int64 [T], negative = skip)."""
     T = d.shape[0]
     if d.is_cuda:
+        done = native.fast.latent_kv_write(d, Q, R, dr, wq, wkv, cache, slots, positions, freq, mult, eps)
+        if done is not None:
+            return done if Q else None
         assert d.stride(1) == 1
         cq = torch.empty(T, Q, dtype=d.dtype, device=d.device) if Q else None
         native.call("llmctl_latent_kv_write", d.data_ptr(), d.stride(0), Q, R, dr, native.ptr(wq), native.ptr(wkv), native.ptr(cq),

@@ -133,8 +133,14 @@ def _load_ops() -> None:
     except (ImportError, OSError) as e:
         warnings.warn(f"{_OPS_PATH.name} is not used ({e}): operators take their checks and launches through Python; run `python build_native.py`", RuntimeWarning)
         return
-    ops.bind(str(_LIB_PATH), NativeError, check_waits)
+    ops.bind(str(_LIB_PATH), NativeError, check_waits, _buffered_wgrad)
     fast = ops
+
+
+def _buffered_wgrad(dy, x, w):
+    """The gradient of a weight that has a buffer for it, for the extension's nodes."""
+    from .functional import _wgrad
+    return _wgrad(dy, x, w)
 
 
 def register_signature(name: str, argtypes: list, restype=c_int) -> None:

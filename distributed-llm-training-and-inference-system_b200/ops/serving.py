@@ -3,6 +3,7 @@ the native kernels; CPU tensors run a plain PyTorch restatement (used by the CPU
 from __future__ import annotations
 
 import math
+from functools import lru_cache
 from typing import Optional
 
 import torch
@@ -66,6 +67,7 @@ def choose_splits(batch: int, heads: int, max_context: int, block_size: int, sms
     return int(max(1, min(want, max(1, max_context // per_split), 256)))
 
 
+@lru_cache(maxsize=4096)
 def _launch_splits(batch: int, heads: int, head_dim: int, max_context: int, block_size: int, sms: int = 148) -> int:
     # One launch, merged inside clusters of up to 8 splits, while all CTAs (three per SM) are resident together and none walks
     # more than 768 tokens (us in one launch / in the splits of choose_splits with a merge kernel: one context of 4096, 32 heads of 128

@@ -204,14 +204,20 @@ def runs_plain(layer: nn.Module) -> bool:
     """Whether calling ``layer`` is ``ops.linear(x, layer.weight)`` and nothing else, so that a fused caller may take its weight and pass
     it by: one rank, one of the two layers above with the methods that stand there (a subclass, an instance or a module put in its place
     may do more), and no hook on it or on all modules that would want to see the call."""
+    own = _OWN.get(type(layer))
+    return (own is not None and untouched(layer, own[0]) and getattr(type(layer), "finish", None) is own[1] and "finish" not in layer.__dict__
+            and get_state().tp == 1)
+
+
+def untouched(layer: nn.Module, forward) -> bool:
+    """Whether calling ``layer`` is calling ``forward`` on it and nothing else: the class has that method, the instance none of its own, and no
+    hook on it or on all modules wants to see the call."""
     t, d = type(layer), layer.__dict__
-    own = _OWN.get(t)
-    return (own is not None and t.forward is own[0] and getattr(t, "finish", None) is own[1] and t.__call__ is _CALL
-            and not ("forward" in d or "finish" in d or d.get("_compiled_call_impl")
+    return (t.forward is forward and t.__call__ is _CALL
+            and not ("forward" in d or d.get("_compiled_call_impl")
                      or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
                      or _every._global_forward_hooks or _every._global_forward_pre_hooks
-                     or _every._global_backward_hooks or _every._global_backward_pre_hooks)
-            and get_state().tp == 1)
+                     or _every._global_backward_hooks or _every._global_backward_pre_hooks))
 
 
 class VocabParallelEmbedding(nn.Module):

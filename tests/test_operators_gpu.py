@@ -610,3 +610,100 @@ def test_loss_kernels_begin_when_those_before_have_ended(ops, rows, V):
         want = run()
     for _ in range(3):
         _same(run(), want)
+
+
+@pytest.mark.parametrize("wants", ["x", "w", "up", "down", "x w up down"])
+@pytest.mark.parametrize("width", [128, 1024])          # two nodes for the gated layer, one
+def test_products_make_the_gradients_that_are_asked_for(ops, wants, width):
+    """linear and the gated layer with some of their inputs recorded; a second pass through a graph that is given up is refused."""
+    def run():
+        t = {"x": _randn(130, 64), "w": _randn(64, 64, seed=1), "up": _randn(192, 64, seed=2), "down": _randn(width, 96, seed=3)}
+        wanted = [t[n].requires_grad_(True) for n in wants.split()]
+        y = ops.swiglu_mlp(ops.linear(t["x"], t["w"]), t["up"], t["down"])
+        dy = _randn(130, width, seed=4)
+        first = torch.autograd.grad(y, wanted, dy, retain_graph=True)
+        again = torch.autograd.grad(y, wanted, dy)
+        _same(first, again)
+        with pytest.raises(RuntimeError):
+            torch.autograd.grad(y, wanted, dy)
+        return (y.detach(), *first)
+    _both(run)
+
+
+def test_weights_with_gradient_buffers(ops):
+    """A buffer that is there when the backward runs takes the gradient, fresh or added to, and its owner is told; it need not be there before."""
+    def run():
+        x, told = _randn(130, 64).requires_grad_(True), []
+        ws = [_randn(64, 64, seed=1), _randn(256, 64, seed=2), _randn(1024, 128, seed=3)]
+        ws = [torch.nn.Parameter(w) for w in ws]
+        y = ops.swiglu_mlp(ops.linear(x, ws[0]), ws[1], ws[2])
+        for i, w in enumerate(ws):
+            w.main_grad = torch.ones(w.shape, device="cuda")
+            w._main_grad_fresh = i == 1
+            w._grad_ready_cb = lambda p: told.append([p is w for w in ws].index(True))
+        y.backward(_randn(130, 1024, seed=4))
+        assert all(w.grad is None for w in ws) and told == [2, 1, 0] and not any(w._main_grad_fresh for w in ws)
+        return (x.grad, *(w.main_grad for w in ws))
+    _both(run)
+
+
+@pytest.mark.parametrize("B,S,heads,dim", [(1, 33, 2, 64), (2, 130, 2, 128), (1, 600, 12, 64)])
+@pytest.mark.parametrize("form", ["plain", "first", "positions", "hook", "few"])
+def test_block_without_gradients(ops, B, S, heads, dim, form):
+    """A decoder layer as one call against the operators that it is made of; a layer whose parts are watched, or of few rows, is not taken."""
+    from llmctl_b200.models.config import ModelConfig
+    from llmctl_b200.models.gpt import GPTModel
+    from llmctl_b200.ops import native
+    S = 20 if form == "few" else S
+    B = 1 if form == "few" else B
+    torch.manual_seed(1)
+    W = heads * dim
+    m = GPTModel(ModelConfig(name="t", layers=1, hidden=W, ffn=2 * W, heads=heads, head_dim=dim, vocab_size=128, max_position_embeddings=1024), device="cuda")
+    blk, (cos, sin) = m.blocks[0], m.rope_tables(torch.device("cuda"))
+    x, r = _randn(B * S, W), None if form == "first" else _randn(B * S, W, seed=1)
+    positions = torch.arange(B * S, device="cuda") % S + 3 if form == "positions" else None
+    seen, calls = [], []
+    if form == "hook":
+        blk.attn.out.register_forward_hook(lambda *a: seen.append(1))
+    block = native.fast.block
+
+    class Counted:
+        def __getattr__(self, name):
+            return (lambda *a: (calls.append(1), block(*a))[1]) if name == "block" else getattr(fast, name)
+    fast, native.fast = native.fast, Counted()
+    try:
+        with torch.no_grad():
+            got = blk(x, r, cos, sin, B, S, positions)
+    finally:
+        native.fast = fast
+    assert len(calls) == (form not in ("hook", "few"))
+    with python_operators(), torch.no_grad():
+        want = blk(x, r, cos, sin, B, S, positions)
+    _same(got, want)
+    assert len(seen) == (2 if form == "hook" else 0)
+
+
+@pytest.mark.parametrize("starts,width,heads,q_rank,parts", [([0], 256, 16, 128, {}), ([500, 77, 64], 256, 32, 128, {"sink": True}), ([130, 900], 256, 5, 0, {}),
+                                                          ([300, 40], 128, 40, 64, {"head_gate": True, "window": 100}), ([70], 128, 8, 64, {"out_gate": True})])
+def test_latent_layer_decodes(ops, starts, width, heads, q_rank, parts):
+    """A decoding latent-attention layer through the extension against the Python operators around the same kernels."""
+    from llmctl_b200.models.mixers import LatentAttention, LatentAttentionSpec
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+    torch.manual_seed(len(starts))
+    spec = LatentAttentionSpec(heads=heads, dim=32, rot_dim=64, vdim=24, kv_rank=128, q_rank=q_rank, scale=0.1, rot_base=10000.0, **parts)
+    layer = LatentAttention(width, spec, 1e-5, torch.bfloat16, "cuda")
+    with torch.no_grad():
+        for name, p in layer.named_parameters():
+            p.copy_(torch.randn(p.shape, device="cuda") * (0.1 if p.dim() > 1 else 1.0))
+    pages = [(s + 64) // 64 for s in starts]
+    tables = [list(range(sum(pages[:i]), sum(pages[:i + 1]))) for i in range(len(starts))]
+    h, rows = _randn(len(starts), width), _randn(sum(pages), 64, 192, seed=1)
+
+    def run():
+        cache = rows.clone()
+        batch = RaggedBatch([Portion(i, [0], s, [0], t) for i, (s, t) in enumerate(zip(starts, tables))], 64, torch.device("cuda"))
+        with torch.no_grad():
+            return layer(h, batch, cache), cache
+    with python_operators():
+        want = run()
+    _same(run(), want)
