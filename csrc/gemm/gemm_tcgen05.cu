@@ -704,6 +704,168 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   }
 }
 
+// ================================================================================================
+// Split K: a cluster of `splits` CTAs computes one 128 x 64 tile, each over its share of the k-blocks, and each sums and stores its share of the
+// columns: the others' partial sums come into its shared memory (distributed shared memory, over the operand ring, which is idle by
+// then) and are added in the order of the ranks.  For problems with fewer tiles than SMs, which a CTA that walks all of K alone leaves waiting:
+// the products of a few rows with a vocabulary's or an MLP's long side.
+// ================================================================================================
+constexpr int kSplitBN = 64, kMaxSplits = 8;
+template <int kStages>
+struct SplitCfg {
+  static constexpr int kABytes = kBM * kBK * 2, kStageBytes = kABytes + kSplitBN * kBK * 2;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024;
+};
+// Columns go to the CTAs in units of 8.
+__device__ __forceinline__ int first_unit(int rank, int splits) { return kSplitBN / 8 * rank / splits; }
+__device__ __forceinline__ int unit_owner(int u, int splits) { return ((u + 1) * splits - 1) / (kSplitBN / 8); }
+
+template <int kStages, bool A_MN, bool B_MN, typename OutT>
+__global__ void __launch_bounds__(kGemmThreads, kStages <= 4 ? 2 : 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OutT* __restrict__ C, long long ldc, int M, int N, int K,
+                  int beta, int splits) {
+  using Cfg = SplitCfg<kStages>;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t bar_full[kStages], bar_empty[kStages], bar_done;
+  __shared__ uint32_t tmem_base_smem;
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_ctarank()), tile = blockIdx.x / splits;
+  const int num_m = (M + kBM - 1) / kBM, num_n = (N + kSplitBN - 1) / kSplitBN, num_kb = (K + kBK - 1) / kBK;
+  int m_blk, n_blk;
+  tile_to_mn(tile, num_m, num_n, m_blk, n_blk);
+  const int m0 = m_blk * kBM, n0 = n_blk * kSplitBN;
+  const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * rank / splits), kb1 = static_cast<int>(static_cast<long long>(num_kb) * (rank + 1) / splits);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&bar_full[i], 1);
+      mbar_init(&bar_empty[i], 1);
+    }
+    mbar_init(&bar_done, 1);
+    fence_mbar_init();
+    prefetch_tmap(&tmA);
+    prefetch_tmap(&tmB);
+  }
+  if (warp == 1) tmem_alloc<1>(&tmem_base_smem, kSplitBN);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_smem;
+  wait_for_previous(C);
+  float acc[kSplitBN];
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+        const int stage = i % kStages;
+        mbar_wait(&bar_empty[stage], ((i / kStages) & 1u) ^ 1u);
+        uint8_t *sA = smem + stage * Cfg::kStageBytes, *sB = sA + Cfg::kABytes;
+        mbar_expect_tx(&bar_full[stage], Cfg::kStageBytes);
+        const int k0 = kb * kBK;
+        if (!A_MN) {
+          tma_load_2d(sA, &tmA, &bar_full[stage], k0, m0);
+        } else {
+          tma_load_2d(sA, &tmA, &bar_full[stage], m0, k0);
+          tma_load_2d(sA + 8192, &tmA, &bar_full[stage], m0 + 64, k0);
+        }
+        if (!B_MN) tma_load_2d(sB, &tmB, &bar_full[stage], k0, n0); else tma_load_2d(sB, &tmB, &bar_full[stage], n0, k0);
+      }
+      release_dependents();
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    constexpr uint32_t idesc = make_idesc_bf16(kBM, kSplitBN, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      mbar_wait(&bar_full[stage], phase);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t a_addr = smem_base + stage * Cfg::kStageBytes;
+      const uint64_t da = A_MN ? make_smem_desc(a_addr, 8192, 1024, 2) : make_smem_desc(a_addr, 16, 1024, 2);
+      const uint64_t db = B_MN ? make_smem_desc(a_addr + Cfg::kABytes, 8192, 1024, 2) : make_smem_desc(a_addr + Cfg::kABytes, 16, 1024, 2);
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < kBK / 16; ++k)
+          umma_ss<1>(tmem_base, da + ((A_MN ? k * 2048 : k * 32) >> 4), db + ((B_MN ? k * 2048 : k * 32) >> 4), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+        umma_commit<1>(&bar_empty[stage]);
+        if (kb + 1 == kb1) umma_commit<1>(&bar_done);
+      }
+      if (++stage == kStages) {
+        stage = 0;
+        phase ^= 1u;
+      }
+    }
+    __syncwarp();
+  } else {
+    mbar_wait(&bar_done, 0u);
+    __syncwarp();
+    tc_fence_after();
+    uint32_t r[kSplitBN];
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    tmem_ld_x32(t_row, r);
+    tmem_ld_x32(t_row + 32, r + 32);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < kSplitBN; ++i) acc[i] = __uint_as_float(r[i]);
+  }
+  const int row = (warp & 3) * 32 + lane;
+  cluster_sync();                      // every CTA's loads have landed and been multiplied: the rings may be written over
+  if (warp >= 2) {
+#pragma unroll
+    for (int u = 0; u < kSplitBN / 8; ++u) {
+      const int to = unit_owner(u, splits), first = first_unit(to, splits), width = (first_unit(to + 1, splits) - first) * 8;
+      const uint32_t at = mapa_u32(smem_base + ((rank * kBM + row) * width + (u - first) * 8) * 4, to);
+      st_cluster_v4(at, make_float4(acc[8 * u], acc[8 * u + 1], acc[8 * u + 2], acc[8 * u + 3]));
+      st_cluster_v4(at + 16, make_float4(acc[8 * u + 4], acc[8 * u + 5], acc[8 * u + 6], acc[8 * u + 7]));
+    }
+  }
+  cluster_sync();
+  if (warp >= 2 && m0 + row < M) {
+    const int first = first_unit(rank, splits), last = first_unit(rank + 1, splits), width = (last - first) * 8;
+    const float* mine = reinterpret_cast<const float*>(smem) + row * width;
+    for (int u = first; u < last; ++u) {
+      const int col = n0 + u * 8;
+      if (col >= N) break;
+      float f[8] = {};
+      for (int src = 0; src < splits; ++src) {
+        const float4* p = reinterpret_cast<const float4*>(mine + src * kBM * width + (u - first) * 8);
+        const float4 x = p[0], y = p[1];
+        f[0] += x.x; f[1] += x.y; f[2] += x.z; f[3] += x.w;
+        f[4] += y.x; f[5] += y.y; f[6] += y.z; f[7] += y.w;
+      }
+      OutT* dst = C + static_cast<long long>(m0 + row) * ldc + col;
+      if constexpr (sizeof(OutT) == 2) {
+        if (beta) {
+          float old[8];
+          unpack8(load8(dst), old);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] += old[e];
+        }
+        store8(dst, pack8(f));
+      } else {
+        float4* to = reinterpret_cast<float4*>(dst);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float4 v = make_float4(f[4 * h], f[4 * h + 1], f[4 * h + 2], f[4 * h + 3]);
+          if (beta) {
+            const float4 o = to[h];
+            v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+          }
+          to[h] = v;
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc<1>(tmem_base, kSplitBN);
+  }
+}
+
 static int g_num_sms = 0;
 static int num_sms() {
   if (g_num_sms == 0) {
@@ -766,6 +928,47 @@ static int dispatch_layout(int a_mn, int b_mn, const void* A, const void* B, voi
   return launch_gemm<BN, true, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
 }
 
+
+template <int kStages, bool A_MN, bool B_MN, typename OutT>
+static int launch_split_stages(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C, int M, int N, int K, long long ldc, int beta, int tiles, int splits,
+                               cudaStream_t s) {
+  auto kern = gemm_split_kernel<kStages, A_MN, B_MN, OutT>;
+  LLMCTL_CHECK(allow_smem(kern, SplitCfg<kStages>::kSmemBytes));
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim = {static_cast<unsigned>(splits), 1, 1};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = tiles * splits;
+  cfg.blockDim = kGemmThreads;
+  cfg.dynamicSmemBytes = SplitCfg<kStages>::kSmemBytes;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  LLMCTL_CHECK(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, (OutT*)C, ldc, M, N, K, beta, splits));
+  LLMCTL_RETURN_LAST();
+}
+template <bool A_MN, bool B_MN, typename OutT>
+static int launch_split(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int beta, int splits,
+                        cudaStream_t s) {
+  CUtensorMap tmA, tmB;
+  int rc = A_MN ? get_tmap_2d_bf16(&tmA, A, K, M, lda, kBK, 64, 1) : get_tmap_2d_bf16(&tmA, A, M, K, lda, kBM, kBK, 1);
+  if (!rc) rc = B_MN ? get_tmap_2d_bf16(&tmB, B, K, N, ldb, kBK, 64, 1) : get_tmap_2d_bf16(&tmB, B, N, K, ldb, kSplitBN, kBK, 1);
+  if (rc) LLMCTL_FAIL(rc, "tensor maps");
+  const int tiles = ((M + kBM - 1) / kBM) * ((N + kSplitBN - 1) / kSplitBN);
+  // one CTA to an SM has all of its shared memory for loads in flight; beyond one wave two share it
+  return tiles * splits <= num_sms() ? launch_split_stages<8, A_MN, B_MN, OutT>(tmA, tmB, C, M, N, K, ldc, beta, tiles, splits, s)
+                                     : launch_split_stages<4, A_MN, B_MN, OutT>(tmA, tmB, C, M, N, K, ldc, beta, tiles, splits, s);
+}
+template <typename OutT>
+static int dispatch_split(int a_mn, int b_mn, const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int beta,
+                          int splits, cudaStream_t s) {
+  if (!a_mn && !b_mn) return launch_split<false, false, OutT>(A, B, C, M, N, K, lda, ldb, ldc, beta, splits, s);
+  if (!a_mn && b_mn) return launch_split<false, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, beta, splits, s);
+  if (a_mn && !b_mn) return launch_split<true, false, OutT>(A, B, C, M, N, K, lda, ldb, ldc, beta, splits, s);
+  return launch_split<true, true, OutT>(A, B, C, M, N, K, lda, ldb, ldc, beta, splits, s);
+}
 
 template <int PBN, bool A_MN, bool B_MN, typename OutT>
 static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
@@ -882,8 +1085,33 @@ static int one_wave_tile(int M, int N) {
   return rows * ((N + 127) / 128) <= sms ? 128 : 0;
 }
 
+// CTAs that share the K of each 128 x 64 tile (gemm_split_kernel), 1 where that does not pay: fewer tiles than SMs, and a K whose blocks, 0.2 us
+// each for a CTA alone on its SM and 0.32 for two, outweigh the cluster's launch and exchange.  Clusters of 4 and 8 leave SMs of a GPC over: 128 CTAs
+// of them are resident one to an SM.  us, one CTA a tile / split (operands from HBM): 64 x 768 x 32000 98 / 19 (8), 200 x 768 98 / 31 (4), 500 x 768
+// 100 / 48 (4), 1000 x 768 104 / 83 (2), 500 x 2048 101 / 88 (2), 200 x 2048 x 11264 37 / 23, x 5632 20.1 / 15.3, 500 x 768 x 4096 15.8 / 12.9, 768 x 768 x 3000
+// of M-major operands 14.0 / 12.4; left alone: 200 x 2048 x 2048 9.5 / 9.9, 300 x 768 x 2048 9.3 / 9.4, 777 x 768 x 2048 9.6 / 13.9, 500 x 2048 x 5632 20.5 / 22.9.
+static int split_count(int M, int N, int K) {
+  const long long tiles = static_cast<long long>((M + kBM - 1) / kBM) * ((N + kSplitBN - 1) / kSplitBN), sms = num_sms();
+  if (tiles > sms) return 1;
+  const double blocks = (K + kBK - 1) / kBK;
+  double least = 0.87 * (2.7 + 0.2 * blocks);
+  int best = 1;
+  for (int splits = 2; splits <= kMaxSplits && 8 * splits <= blocks; splits *= 2) {
+    const long long ctas = tiles * splits;
+    if (ctas > 2 * sms) break;
+    const bool alone = splits == 2 ? ctas <= sms : ctas <= sms * 128 / 148;
+    const double us = (splits == 8 ? 2. : 0.) + (alone ? 6. + 0.2 * blocks / splits : 9.5 + 0.32 * blocks / splits);
+    if (us < least) {
+      least = us;
+      best = splits;
+    }
+  }
+  return best;
+}
+
 // D[M,N] = op(A) op(B) (+ D if beta).  a_mn / b_mn select the operand storage (see file header).
-// out_fp32: D is fp32 (else bf16).  tile_n: 0 = auto, 64 / 128 / 192 / 256 (1-CTA tiles), 2 = 256x256 CTA-pair tile, 3 = 256x128 CTA-pair tile.  max_ctas: 0 = all SMs
+// out_fp32: D is fp32 (else bf16).  tile_n: 0 = auto, 64 / 128 / 192 / 256 (1-CTA tiles), 2 = 256x256 CTA-pair tile, 3 = 256x128 CTA-pair tile, -2 .. -8 = 128x64 tiles
+// whose K that many CTAs share.  max_ctas: 0 = all SMs
 // (a smaller value leaves SMs free for a concurrent communication kernel).
 static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, int K,
                           long long lda, long long ldb, long long ldc, int a_mn, int b_mn,
@@ -901,8 +1129,16 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
   // Beyond one wave operand traffic from L2 sets the pace and the 256 x 256 CTA-pair tile moves least of it (4096 x 2048 x 2048:
   // 26.7 / 33.1 / 49.0, 4096 x 11264 x 2048: 130 / 181 / 276); 128 x 192 and pair 256 x 128 never win by more than a few per cent
   // and stay selectable (tile_n = 192 / 3).  Gated operands arrive slab by slab and keep the pair tile.
+  if (tile_n == 0 && !g.waits() && g.grp_tile_expert == nullptr && max_ctas == 0) {
+    const int splits = split_count(M, N, K);
+    if (splits > 1) tile_n = -splits;
+  }
   if (tile_n == 0 && g.flags == nullptr && g.b_flags == nullptr && max_ctas == 0) tile_n = one_wave_tile(M, N);
   if (tile_n == 0 && M > 128 && N > 128) tile_n = 2;
+  if (tile_n < 0) {
+    LLMCTL_REQUIRE(tile_n >= -kMaxSplits && -tile_n <= (K + kBK - 1) / kBK && !g.waits() && g.grp_tile_expert == nullptr && max_ctas == 0);
+    return (out_fp32 ? dispatch_split<float> : dispatch_split<__nv_bfloat16>)(a_mn, b_mn, A, B, C, M, N, K, lda, ldb, ldc, beta, -tile_n, s);
+  }
   if (tile_n == 2) {   // 2-CTA pair tile 256 x 256 (cta_group::2)
     if (out_fp32) return dispatch_layout2<256, float>(a_mn, b_mn, A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);
     return dispatch_layout2<256, __nv_bfloat16>(a_mn, b_mn, A, B, C, M, N, K, lda, ldb, ldc, beta, max_ctas, s, g);

@@ -492,6 +492,34 @@ def test_flash_attention_head_dim_64_uses_the_native_kernel(cuda_device):
         _close(qkv.grad[:, :, i], ref_in.grad[:, :, i], 4e-2, 4e-2, name)
 
 
+# K shared by a cluster: every number of CTAs (uneven shares of K and of the 64 columns), one k-block each, ragged tiles, all layouts, two CTAs
+# to an SM (100 tiles), and sizes for which it is chosen.
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn,splits", [
+    (1, 8, 128, 0, 0, 2), (100, 72, 200, 0, 0, 3), (136, 200, 1000, 0, 1, 4), (200, 136, 1000, 1, 0, 5), (128, 64, 448, 1, 1, 7), (264, 72, 4104, 1, 1, 8),
+    (640, 1280, 264, 0, 0, 4), (300, 768, 1000, 0, 1, 6), (200, 768, 32000, 0, 1, 0), (64, 2048, 5632, 0, 0, 0), (768, 768, 3000, 1, 1, 0)])
+def test_gemm_split_k(cuda_device, M, N, K, a_mn, b_mn, splits):
+    """Against float64: fp32 sums of K exact products rounded to bf16 (2^-9 in the 2-norm, and as much again for the sums), and added to
+    what fp32 outputs hold (2^-16)."""
+    from llmctl_b200.ops import native
+    torch.manual_seed(M + N)
+    a = torch.randn(K, M, device=cuda_device).bfloat16() if a_mn else torch.randn(M, K, device=cuda_device).bfloat16()
+    b = torch.randn(K, N, device=cuda_device).bfloat16() if b_mn else torch.randn(N, K, device=cuda_device).bfloat16()
+    want = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+
+    def product(out, beta):
+        native.call("llmctl_gemm_bf16", a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0), a_mn, b_mn,
+                    int(out.dtype == torch.float32), beta, -splits, 0, native.stream_ptr())
+        return out.double()
+    err = product(torch.full((M, N), float("nan"), device=cuda_device, dtype=torch.bfloat16), 0) - want
+    assert err.norm() <= 2 * 2.0 ** -9 * want.norm()
+    old = torch.randn(M, N, device=cuda_device)
+    err = product(old.clone(), 1) - (want + old)
+    assert err.norm() <= 2.0 ** -16 * (want + old).norm()
+    old = old.bfloat16()
+    err = product(old.clone(), 1) - (want + old)
+    assert err.norm() <= 2 * 2.0 ** -9 * (want + old).norm()
+
+
 # Lengths around the 128-row blocks and the 256-query items, more items than SMs (256 x 3 blocks), several head groups of the
 # backward's item order (S = 2048: 16 heads of 128 to a group), non-causal whole blocks, views at an odd address (copied first).
 @pytest.mark.parametrize("B,S,H,D,causal,shift", [
