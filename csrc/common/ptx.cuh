@@ -240,7 +240,10 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t smem_addr, uint32_t cta) {
   return remote;
 }
 
-// 16 bytes into another CTA's shared memory (an address from mapa_u32).
+// 8 or 16 bytes into another CTA's shared memory (an address from mapa_u32).
+__device__ __forceinline__ void st_cluster_v2(uint32_t at, float2 v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(at), "f"(v.x), "f"(v.y) : "memory");
+}
 __device__ __forceinline__ void st_cluster_v4(uint32_t at, float4 v) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }

@@ -232,12 +232,153 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
 }
 
+// A layer whose tiles of weight rows are few is no stream but a latency: launch, first bytes, and the way of the pieces through the workspace (store,
+// fence, ticket, and their sum by one CTA), 6-10 us for any few MB of weights.  Here a cluster of S CTAs takes a tile's K, a share each, and every CTA sums and
+// stores MB / S of the token rows, whose partial sums come through distributed shared memory (over the operand ring, idle by then) and are
+// added in the order of the ranks: no workspace, no ticket.
+template <int MB, int S>
+__global__ void __launch_bounds__(skinny::kThreads, 1)
+gemm_skinny_cluster_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, __nv_bfloat16* __restrict__ C, long long ldc, int Mb, int N,
+                           int num_kb) {
+  using namespace skinny;
+  using C_ = Cfg<MB>;
+  constexpr int kOwn = MB / S;               // token rows that a CTA sums and stores
+  static_assert(kOwn >= 2 && (S * kBM * kOwn + 32) * 4 <= C_::kStages * C_::kStageBytes, "exchange");
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t bar_full[C_::kStages], bar_empty[C_::kStages], bar_done;
+  __shared__ uint32_t tmem_base_smem;
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_ctarank()), tile = blockIdx.x / S;
+  const int kb0 = num_kb * rank / S, kb1 = num_kb * (rank + 1) / S;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < C_::kStages; ++i) {
+      mbar_init(&bar_full[i], 1);
+      mbar_init(&bar_empty[i], 1);
+    }
+    mbar_init(&bar_done, 1);
+    fence_mbar_init();
+    prefetch_tmap(&tmW);
+    prefetch_tmap(&tmX);
+  }
+  if (warp == 1) tmem_alloc<1>(&tmem_base_smem, 32);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_smem;
+  wait_for_previous(C);
+  float acc[MB];
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+        const int stage = i % C_::kStages;
+        mbar_wait(&bar_empty[stage], ((i / C_::kStages) & 1u) ^ 1u);
+        uint8_t* sW = smem + stage * C_::kStageBytes;
+        mbar_expect_tx(&bar_full[stage], C_::kStageBytes);
+        tma_load_2d(sW, &tmW, &bar_full[stage], kb * kBK, tile * kBM);   // rows past N read as zero
+        tma_load_2d(sW + kWBytes, &tmX, &bar_full[stage], kb * kBK, 0);  // rows past Mb read as zero
+      }
+      release_dependents();
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    constexpr uint32_t idesc = make_idesc_bf16(kBM, MB, 0u, 0u);
+    for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+      const int stage = i % C_::kStages;
+      mbar_wait(&bar_full[stage], (i / C_::kStages) & 1u);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t w_addr = smem_base + stage * C_::kStageBytes;
+      const uint64_t dw = make_smem_desc(w_addr, 16, 1024, 2), dx = make_smem_desc(w_addr + kWBytes, 16, 1024, 2);
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < kBK / 16; ++k) umma_ss<1>(tmem_base, dw + k * 2, dx + k * 2, idesc, (i | k) != 0 ? 1u : 0u);
+        umma_commit<1>(&bar_empty[stage]);
+        if (kb + 1 == kb1) umma_commit<1>(&bar_done);
+      }
+    }
+    __syncwarp();
+  } else {
+    mbar_wait(&bar_done, 0u);
+    __syncwarp();
+    tc_fence_after();
+    uint32_t r[MB];
+    const uint32_t taddr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    if constexpr (MB == 16) tmem_ld_x16(taddr, r); else tmem_ld_x32(taddr, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int m = 0; m < MB; ++m) acc[m] = __uint_as_float(r[m]);
+  }
+  const int row = (warp & 3) * 32 + lane;
+  cluster_sync();                      // every CTA's loads have landed and been multiplied: the rings may be written over
+  if (warp >= 2) {
+#pragma unroll
+    for (int to = 0; to < S; ++to) {
+      const uint32_t at = mapa_u32(smem_base + (rank * kBM + row) * kOwn * 4, to);
+#pragma unroll
+      for (int m = 0; m < kOwn; m += (kOwn >= 4 ? 4 : 2)) {
+        const float* v = acc + to * kOwn + m;
+        if constexpr (kOwn >= 4) st_cluster_v4(at + m * 4, make_float4(v[0], v[1], v[2], v[3])); else st_cluster_v2(at + m * 4, make_float2(v[0], v[1]));
+      }
+    }
+  }
+  cluster_sync();
+  const int n = tile * kBM + row;
+  if (warp >= 2 && n < N) {
+    const float* mine = reinterpret_cast<const float*>(smem) + row * kOwn;
+    float sum[kOwn] = {};
+#pragma unroll
+    for (int src = 0; src < S; ++src)
+#pragma unroll
+      for (int m = 0; m < kOwn; ++m) sum[m] += mine[src * kBM * kOwn + m];
+#pragma unroll
+    for (int m = 0; m < kOwn; ++m)
+      if (rank * kOwn + m < Mb) C[(rank * kOwn + m) * ldc + n] = __float2bfloat16(sum[m]);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc<1>(tmem_base, 32);
+  }
+}
+
+template <int MB, int S>
+static int launch_skinny_cluster(const CUtensorMap& tw, const CUtensorMap& tx, __nv_bfloat16* C, long long ldc, int Mb, int N, int num_kb, int n_tiles, cudaStream_t s) {
+  auto kern = gemm_skinny_cluster_kernel<MB, S>;
+  LLMCTL_CHECK(allow_smem(kern, skinny::Cfg<MB>::kSmem));
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim = {S, 1, 1};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = n_tiles * S;
+  cfg.blockDim = skinny::kThreads;
+  cfg.dynamicSmemBytes = skinny::Cfg<MB>::kSmem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  LLMCTL_CHECK(cudaLaunchKernelEx(&cfg, kern, tw, tx, C, ldc, Mb, N, num_kb));
+  LLMCTL_RETURN_LAST();
+}
+
 }  // namespace llmctl
 
 using namespace llmctl;
 
 namespace llmctl {
 namespace skinny {
+// CTAs of a cluster that share a tile's K, 0: the stream of all SMs (gemm_skinny_kernel).  As many as are resident together, one to an SM and whole
+// clusters to a GPC: 96 CTAs in eights, 128 in fours (2048 x 2048: 16 tiles in eights 7.9 us, in fours 4.9).  us, stream / clusters, 32 rows (1 row),
+// weights from HBM: 768 x 768 9.0 / 3.5 (6.5 / 3.1), 1344 x 2048 9.1 / 4.5 (6.2 / 4.0), 2048 x 5632 15.0 / 8.8 (9.7 / 7.8), 4096 x 4096 14.8 / 9.5
+// (10.6 / 8.4), 4096 x 11008 23.7 / 18.0 (18.8 / 16.8), 6144 x 2048 13.0 / 8.4 (9.5 / 7.4), 8192 x 2048 13.5 / 9.4; beyond 64 tiles the stream fills the SMs better.
+static int cluster_size(int n_tiles, int num_kb) {
+  const int fit = n_tiles <= 12 ? 8 : n_tiles <= 32 ? 4 : n_tiles <= 64 ? 2 : 0;
+  return fit <= num_kb ? fit : 0;
+}
 // k blocks per CTA and the floats of scratch that its pieces of tiles take
 struct Plan {
   int MB, n_tiles, num_kb;
@@ -303,6 +444,12 @@ LLMCTL_API int llmctl_gemm_skinny_bf16(const void* X, const void* W, void* C, in
   rc = get_tmap_2d_bf16(&tx, X, Mb, K, ldx, MB, skinny::kBK, 1);
   if (rc) LLMCTL_FAIL(rc, "tensor map X");
   cudaStream_t s = (cudaStream_t)stream;
+  const int cluster = splits > 0 ? 0 : skinny::cluster_size(n_tiles, num_kb);
+  if (cluster) {
+    const auto launch = MB == 16 ? (cluster == 8 ? launch_skinny_cluster<16, 8> : cluster == 4 ? launch_skinny_cluster<16, 4> : launch_skinny_cluster<16, 2>)
+                                 : (cluster == 8 ? launch_skinny_cluster<32, 8> : cluster == 4 ? launch_skinny_cluster<32, 4> : launch_skinny_cluster<32, 2>);
+    return launch(tw, tx, (__nv_bfloat16*)C, ldc, Mb, N, num_kb, n_tiles, s);
+  }
   if (MB == 16) {
     LLMCTL_CHECK(allow_smem(gemm_skinny_kernel<16>, skinny::Cfg<16>::kSmem));
     LLMCTL_CHECK(launch_dependent(gemm_skinny_kernel<16>, grid, skinny::kThreads, skinny::Cfg<16>::kSmem, s, tw, tx, (__nv_bfloat16*)C, ldc, Mb, N,

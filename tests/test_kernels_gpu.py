@@ -262,6 +262,22 @@ def test_gemm_skinny(cuda_device, M, N, K, splits):
         assert torch.equal(ops.linear(x, w), out1) or splits != 0
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 8, 512), (17, 1000, 520), (32, 1536, 4096), (16, 1544, 2048), (5, 4096, 256), (9, 4104, 136), (32, 8192, 128), (15, 8200, 128),
+                                   (3, 104, 448), (2, 2048, 64)])
+def test_gemm_skinny_clusters(cuda_device, M, N, K):
+    """Decode GEMM where a cluster shares a tile's K (eights, fours and pairs to either side of their lines, shares of one block and uneven ones, too
+    few blocks for a cluster) against float64: fp32 sums rounded to bf16, 2 x 2^-9 in the 2-norm; equal bits in a second call, and no writes past
+    the rows that there are."""
+    from llmctl_b200.ops import functional as ops
+    torch.manual_seed(N)
+    x, w = torch.randn(M, K, device=cuda_device).bfloat16(), torch.randn(N, K, device=cuda_device).bfloat16()
+    out = torch.full((M + 1, N), 7.0, device=cuda_device, dtype=torch.bfloat16)
+    ops.gemm_skinny(x, w, out=out[:M])
+    want = x.double() @ w.double().t()
+    assert (out[:M].double() - want).norm() <= 2 * 2.0 ** -9 * want.norm() and (out[M] == 7).all()
+    assert torch.equal(ops.gemm_skinny(x, w), out[:M])
+
+
 def test_gemm_fp32_accumulate(cuda_device):
     from llmctl_b200.ops import functional as ops
     torch.manual_seed(7)
