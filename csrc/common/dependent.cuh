@@ -10,7 +10,7 @@
 //
 // Persistent kernels release theirs when the last loads are under way, so that a waiting dependent does not take the place that a
 // communication kernel could have beside them; short ones at once.
-// Rules: (1) no global access before wait_for_previous(), and no CTA without it; (2) TMEM is allocated before release_dependents(), so
+// Rules: (1) no global access before wait_for_previous() but prefetches into L2, which return nothing (ptx.cuh), and no CTA without it; (2) TMEM is allocated before release_dependents(), so
 // that a dependent's allocation never stands before one that the kernel it waits for still has to make; (3) kernels that wait for flags
 // which kernels of other streams or GPUs set release nothing early: a waiting dependent would take the room that those kernels need.
 #pragma once

@@ -82,6 +82,16 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
+  if (warp == 0 && lane == 0) {        // the first weights on their way to L2 beside the end of the kernel before
+    int tile = static_cast<int>(begin / num_kb), kb = static_cast<int>(begin % num_kb);
+    for (int i = 0; i < C_::kStages && begin + i < end; ++i) {
+      tma_prefetch_2d(&tmW, kb * kBK, tile * kBM);
+      if (++kb == num_kb) {
+        kb = 0;
+        ++tile;
+      }
+    }
+  }
   wait_for_previous(C, workspace, counters);
 
   if (warp == 0) {
@@ -268,6 +278,8 @@ gemm_skinny_cluster_kernel(const __grid_constant__ CUtensorMap tmW, const __grid
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
+  if (warp == 0 && lane == 0)          // the first weights on their way to L2 beside the end of the kernel before
+    for (int kb = kb0; kb < kb1 && kb < kb0 + C_::kStages; ++kb) tma_prefetch_2d(&tmW, kb * kBK, tile * kBM);
   wait_for_previous(C);
   float acc[MB];
   if (warp == 0) {
