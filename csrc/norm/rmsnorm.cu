@@ -9,6 +9,7 @@
 // Backward: persistent CTAs loop over rows; dw/db partial sums stay in registers and are flushed once
 //           per CTA into a scratch [grid, cols] fp32 buffer which a second kernel column-reduces.
 #include "../common/dependent.cuh"
+#include "../common/dtype.cuh"
 #include "../common/util.cuh"
 
 namespace llmctl {
@@ -214,9 +215,11 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
 // nparts is at most a few hundred: 32 slices of rows with eight loads in flight each leave three rounds of 592 partials, where eight slices
 // walked 74 rows one by one.  us of the whole backward, 8 slices / 32 (L2 flushed): 4096 x 2048 31.7 / 23.4, 4096 x 768 24.4 / 17.4,
 // 777 x 768 16.2 / 11.3, 8192 x 4096 78.8 / 74.6.
+// A bf16 gradient is rounded here: a conversion of its own was a launch of 2 us for a few KB.
 constexpr int kSumSlices = 32;
+template <typename T>
 __global__ void __launch_bounds__(32 * kSumSlices)
-colsum_kernel(const float* __restrict__ partial, float* __restrict__ out, int nparts, int cols, int accumulate) {
+colsum_kernel(const float* __restrict__ partial, T* __restrict__ out, int nparts, int cols, int accumulate) {
   wait_for_previous(partial, out);
   release_dependents();
   // 32 consecutive columns x kSumSlices slices of rows
@@ -231,7 +234,7 @@ colsum_kernel(const float* __restrict__ partial, float* __restrict__ out, int np
   __syncthreads();
   const int mine = blockIdx.x * 32 + threadIdx.y;               // warp y sums column y of the tile
   const float t = warp_sum(tile[threadIdx.x][threadIdx.y]);
-  if (threadIdx.x == 0 && mine < cols) out[mine] = accumulate ? out[mine] + t : t;
+  if (threadIdx.x == 0 && mine < cols) out[mine] = from_f32<T>(accumulate ? to_f32(out[mine]) + t : t);
 }
 
 template <bool kLN>
@@ -258,9 +261,9 @@ static int launch_fwd(const void* x, const void* residual, const void* w, const 
   LLMCTL_RETURN_LAST();
 }
 
-template <bool kLN>
+template <bool kLN, typename T = float>
 static int launch_bwd(const void* dy, const void* h, const void* w, const float* mean,
-                      const float* rstd, const void* dres, void* dx, float* dw, float* db,
+                      const float* rstd, const void* dres, void* dx, T* dw, T* db,
                       float* scratch, int scratch_rows, int rows, int cols, int accumulate,
                       cudaStream_t s) {
   LLMCTL_REQUIRE(cols % 8 == 0 && cols <= 8192 && scratch_rows >= 1);
@@ -287,8 +290,8 @@ static int launch_bwd(const void* dy, const void* h, const void* w, const float*
   else LAUNCH(1024, 1);
 #undef LAUNCH
   dim3 b2(32, kSumSlices), g2((cols + 31) / 32);
-  LLMCTL_CHECK(launch_dependent(colsum_kernel, g2, b2, 0, s, dwp, dw, grid, cols, accumulate));
-  if (kLN && db != nullptr) LLMCTL_CHECK(launch_dependent(colsum_kernel, g2, b2, 0, s, dbp, db, grid, cols, accumulate));
+  LLMCTL_CHECK(launch_dependent(colsum_kernel<T>, g2, b2, 0, s, dwp, dw, grid, cols, accumulate));
+  if (kLN && db != nullptr) LLMCTL_CHECK(launch_dependent(colsum_kernel<T>, g2, b2, 0, s, dbp, db, grid, cols, accumulate));
   LLMCTL_RETURN_LAST();
 }
 
@@ -308,8 +311,15 @@ LLMCTL_API int llmctl_rmsnorm_bwd(const void* dy, const void* h, const void* w, 
                                   int scratch_rows, int rows, int cols, int accumulate,
                                   void* stream) {
   LLMCTL_BEGIN();
-  return launch_bwd<false>(dy, h, w, nullptr, rstd, dres, dx, dw, nullptr, scratch, scratch_rows,
+  return launch_bwd<false>(dy, h, w, nullptr, rstd, dres, dx, dw, static_cast<float*>(nullptr), scratch, scratch_rows,
                            rows, cols, accumulate, (cudaStream_t)stream);
+}
+// The same with the weight's gradient in bf16, rounded from its fp32 sum.
+LLMCTL_API int llmctl_rmsnorm_bwd_bf16w(const void* dy, const void* h, const void* w, const float* rstd, const void* dres, void* dx, void* dw, float* scratch,
+                                        int scratch_rows, int rows, int cols, void* stream) {
+  LLMCTL_BEGIN();
+  return launch_bwd<false, __nv_bfloat16>(dy, h, w, nullptr, rstd, dres, dx, (__nv_bfloat16*)dw, nullptr, scratch, scratch_rows, rows, cols, 0,
+                                          (cudaStream_t)stream);
 }
 LLMCTL_API int llmctl_layernorm_fwd(const void* x, const void* residual, const void* w,
                                     const void* b, void* h_out, void* y, float* mean, float* rstd,
@@ -411,6 +421,6 @@ LLMCTL_API int llmctl_rmsnorm_bwd_noalloc(const void* dy, const void* h, const v
     }
     scratch = g_noalloc_scratch_addr[dev];
   }
-  return launch_bwd<false>(dy, h, w, nullptr, rstd, dres, dx, dw, nullptr, scratch, kNoAllocCtas, rows, cols,
+  return launch_bwd<false>(dy, h, w, nullptr, rstd, dres, dx, dw, static_cast<float*>(nullptr), scratch, kNoAllocCtas, rows, cols,
                            accumulate, (cudaStream_t)stream);
 }

@@ -7,27 +7,25 @@
 // reference configs/models/llama-7b.json:11-14.  The cos/sin table is built by the caller so
 // "linear"/"su" scaling only changes the table, not the kernel.
 #include "../common/dependent.cuh"
+#include "../common/fast_div.h"
 #include "../common/util.cuh"
 
 namespace llmctl {
 
-// One thread rotates 8 pairs: elements [d0, d0+8) of the first half with the matching second half.
+// One thread rotates 8 pairs: elements [d0, d0+8) of the first half with the matching second half.  Bound by the two passes over the rows; with three
+// 64-bit divisions for each thread's place it took 2.8 us for 777 x 24 heads of 64, now 2.5 (1500 x 32 of 128 6.0 / 5.5, 4096 x 32 of 128 12.3 / 12.0).
 __global__ void __launch_bounds__(256)
-rope_kernel(__nv_bfloat16* __restrict__ x, long long row_stride, int n_tokens, int n_heads,
+rope_kernel(__nv_bfloat16* __restrict__ x, long long row_stride, uint32_t total, FastDiv per_token, FastDiv per_head, FastDiv seq,
             int head_dim, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-            const int* __restrict__ positions, int seq_len, float sign) {
+            const int* __restrict__ positions, int tok0, float sign) {
   wait_for_previous(x, cos_t, sin_t, positions);
   release_dependents();
   const int half = head_dim >> 1;
-  const int vec_per_head = half >> 3;
-  const long long total = static_cast<long long>(n_tokens) * n_heads * vec_per_head;
-  for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
-       idx += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int vh = static_cast<int>(idx % vec_per_head);
-    const long long th = idx / vec_per_head;
-    const int head = static_cast<int>(th % n_heads);
-    const int tok = static_cast<int>(th / n_heads);
-    const int pos = positions ? positions[tok] : (tok % seq_len);
+  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    uint32_t unit, vh, at;
+    const int tok = tok0 + static_cast<int>(per_token.divide(idx, unit)), head = static_cast<int>(per_head.divide(unit, vh));
+    seq.divide(tok, at);
+    const int pos = positions ? positions[tok] : static_cast<int>(at);
     __nv_bfloat16* p = x + tok * row_stride + static_cast<long long>(head) * head_dim + vh * 8;
     float a[8], b[8], c[8], s[8], oa[8], ob[8];
     unpack8(load8(p), a);
@@ -59,11 +57,17 @@ LLMCTL_API int llmctl_rope_inplace(void* x, long long row_stride, int n_tokens, 
   LLMCTL_BEGIN();
   LLMCTL_REQUIRE(head_dim % 16 == 0 && row_stride % 8 == 0 && seq_len > 0);
   LLMCTL_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15) == 0);
-  const long long total = static_cast<long long>(n_tokens) * n_heads * (head_dim / 16);
-  if (total == 0) return 0;
-  long long blocks = (total + 255) / 256;
-  if (blocks > kNumSMs * 16) blocks = kNumSMs * 16;
-  LLMCTL_CHECK(launch_dependent(rope_kernel, static_cast<int>(blocks), 256, 0, (cudaStream_t)stream, (__nv_bfloat16*)x, row_stride, n_tokens,
-                                n_heads, head_dim, cos_t, sin_t, positions, seq_len, sign));
+  const long long per_token = static_cast<long long>(n_heads) * (head_dim / 16);
+  if (per_token == 0 || n_tokens == 0) return 0;
+  LLMCTL_REQUIRE(n_heads > 0 && head_dim > 0 && n_tokens > 0 && per_token < (1 << 30));
+  const long long most = (1 << 30) / per_token;              // tokens of a launch: its units are counted in 31 bits
+  for (long long tok0 = 0; tok0 < n_tokens; tok0 += most) {
+    const long long tokens = n_tokens - tok0 < most ? n_tokens - tok0 : most, total = tokens * per_token;
+    long long blocks = (total + 255) / 256;
+    if (blocks > kNumSMs * 16) blocks = kNumSMs * 16;
+    LLMCTL_CHECK(launch_dependent(rope_kernel, static_cast<int>(blocks), 256, 0, (cudaStream_t)stream, (__nv_bfloat16*)x, row_stride,
+                                  static_cast<uint32_t>(total), FastDiv(static_cast<uint32_t>(per_token)), FastDiv(head_dim / 16), FastDiv(seq_len),
+                                  head_dim, cos_t, sin_t, positions, static_cast<int>(tok0), sign));
+  }
   LLMCTL_RETURN_LAST();
 }

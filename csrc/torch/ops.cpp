@@ -37,7 +37,7 @@ using at::Tensor;
 // the kernel library
 // ---------------------------------------------------------------------------------------------------------------------------------
 #define LLMCTL_ENTRIES(X)                                                                                                         \
-  X(llmctl_rmsnorm_fwd) X(llmctl_rmsnorm_bwd) X(llmctl_rope_inplace) X(llmctl_gemm_bf16) X(llmctl_gemm_swiglu_bf16)               \
+  X(llmctl_rmsnorm_fwd) X(llmctl_rmsnorm_bwd_bf16w) X(llmctl_rope_inplace) X(llmctl_gemm_bf16) X(llmctl_gemm_swiglu_bf16)               \
   X(llmctl_gemm_swiglu_bwd_bf16) X(llmctl_swiglu_bwd) X(llmctl_gemm_skinny_bf16) X(llmctl_gemm_skinny_scratch_elems) X(llmctl_flash_attn_fwd) X(llmctl_flash_attn_bwd) X(llmctl_kv_append) \
   X(llmctl_paged_attn_decode) X(llmctl_paged_attn_scratch_elems) X(llmctl_latent_kv_write) X(llmctl_latent_decode)
 struct Entries {
@@ -221,19 +221,19 @@ struct RmsNorm : torch::autograd::Function<RmsNorm> {
     return {r.y};
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
-    return node_body("llmctl_rmsnorm_bwd", ready(lib.llmctl_rmsnorm_bwd), [&]() -> torch::autograd::variable_list {
+    return node_body("llmctl_rmsnorm_bwd_bf16w", ready(lib.llmctl_rmsnorm_bwd_bf16w), [&]() -> torch::autograd::variable_list {
       const auto saved = ctx->get_saved_variables();
       const Tensor h = whole_units(saved[0]), w = whole_units(saved[1]), &rstd = saved[2];
       const bool residual = ctx->saved_data["residual"].toBool();
       const int64_t cols = h.size(-1), rows = h.numel() / cols;
       const Tensor dy = whole_units(grads[0]), dres = residual ? whole_units(grads[1]) : Tensor();
-      Tensor dx = new_bf16(h, h.sizes()), dw = new_f32(h, {cols});
+      Tensor dx = new_bf16(h, h.sizes()), dw = new_bf16(w, {cols});
       const int ctas = static_cast<int>(rows < kNormBwdCtas ? rows : kNormBwdCtas);
       Tensor scratch = new_f32(h, {ctas * cols});
-      done("llmctl_rmsnorm_bwd", lib.llmctl_rmsnorm_bwd(cdata(dy), cdata(h), cdata(w), static_cast<const float*>(cdata(rstd)), residual ? cdata(dres) : nullptr, data(dx),
-                                                        static_cast<float*>(data(dw)), static_cast<float*>(data(scratch)), ctas, static_cast<int>(rows),
-                                                        static_cast<int>(cols), 0, stream()), 2);
-      return {dx, residual ? dx : Tensor(), dw.to(w.scalar_type()), Tensor()};
+      done("llmctl_rmsnorm_bwd_bf16w", lib.llmctl_rmsnorm_bwd_bf16w(cdata(dy), cdata(h), cdata(w), static_cast<const float*>(cdata(rstd)), residual ? cdata(dres) : nullptr,
+                                                                    data(dx), data(dw), static_cast<float*>(data(scratch)), ctas, static_cast<int>(rows),
+                                                                    static_cast<int>(cols), stream()), 2);
+      return {dx, residual ? dx : Tensor(), dw, Tensor()};
     });
   }
 };

@@ -23,6 +23,8 @@ int llmctl_rmsnorm_fwd(const void* x, const void* residual, const void* w, void*
                        float* rstd, int rows, int cols, float eps, void* stream);
 /* dx = d(norm)/dh (+ dres); dw (fp32) (+)= sum_rows dy * xhat.
  * scratch: fp32 [scratch_rows * cols]; scratch_rows CTAs are used (1..rows). */
+int llmctl_rmsnorm_bwd_bf16w(const void* dy, const void* h, const void* w, const float* rstd, const void* dres, void* dx, void* dw, float* scratch,
+                             int scratch_rows, int rows, int cols, void* stream);      /* dw in bf16 */
 int llmctl_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd,
                        const void* dres, void* dx, float* dw, float* scratch, int scratch_rows,
                        int rows, int cols, int accumulate, void* stream);
