@@ -101,8 +101,9 @@ constexpr int kGemmThreads = 192;
 // CTAs fitted, where their registers allow two; beside a gated activation's 196-209 registers they allow one.
 constexpr int kOutBox = 32 * 128;
 constexpr int kSmShared = 228 * 1024, kNeighbourShared = 1280;      // of an SM; of such a CTA (static, the reserved KB, rounded up)
-enum class Gated { kNone, kForward, kBackward };
-constexpr int out_bufs(Gated g) { return g == Gated::kNone ? 1 : 2; }
+enum class Gated { kNone, kForward, kBackward, kRotate };       // what the epilogue does besides storing
+constexpr bool plain_output(Gated g) { return g == Gated::kNone || g == Gated::kRotate; }
+constexpr int out_bufs(Gated g) { return plain_output(g) ? 1 : 2; }
 
 template <int BN, Gated kGated = Gated::kNone>
 struct GemmCfg {
@@ -237,7 +238,49 @@ struct SwigluMaps {
   int keep;                  // gate and up are stored
   const __nv_bfloat16* gu;   // backward: gate | up as the forward left them; `gate` and `up` take their gradients
   long long ldgu;
+  // rotation (kRotate): tables [positions][32], position of each row or null (row % seq), columns that are rotated
+  const float *cos, *sin;
+  const int* positions;
+  int seq, rotated;
 };
+
+// Rotation of heads of 64 on their way out (llmctl_gemm_rope_bf16): a chunk of 64 columns is a head, and a lane holds its row of it, halves and all.
+// The product is rounded to bf16 before it is rotated, as it would be between two kernels.  The row's angles are asked for before
+// the accumulator is waited for.
+struct Angles {
+  float c[32], s[32];
+  __device__ __forceinline__ void load(const SwigluMaps& sw, int row, int M) {
+    if (row >= M) return;
+    const long long at = static_cast<long long>(sw.positions != nullptr ? sw.positions[row] : row % sw.seq) * 32;
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      *reinterpret_cast<float4*>(c + i) = *reinterpret_cast<const float4*>(sw.cos + at + i);
+      *reinterpret_cast<float4*>(s + i) = *reinterpret_cast<const float4*>(sw.sin + at + i);
+    }
+  }
+};
+template <int BN>
+__device__ __forceinline__ void rotate_epilogue(uint32_t t_row, OutStage<1>& out, const CUtensorMap* tmC, const Angles& angles, int rotated, int row0, int n0,
+                                                int M, int N, int lane) {
+#pragma unroll 1
+  for (int c = 0; c < BN / 64; ++c) {
+    uint32_t r[64];
+    tmem_ld_x32(t_row + c * 64, r);
+    tmem_ld_x32(t_row + c * 64 + 32, r + 32);
+    tmem_ld_wait();
+    const int col = n0 + c * 64;
+    if (row0 >= M || col >= N) continue;               // uniform over the warp
+    if (col < rotated) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float a = __bfloat162float(__float2bfloat16(__uint_as_float(r[i]))), b = __bfloat162float(__float2bfloat16(__uint_as_float(r[i + 32])));
+        r[i] = __float_as_uint(__fmaf_rn(a, angles.c[i], -__fmul_rn(b, angles.s[i])));            // rounded as in rope.cu
+        r[i + 32] = __float_as_uint(__fmaf_rn(b, angles.c[i], __fmul_rn(a, angles.s[i])));
+      }
+    }
+    stage_box(out, tmC, col, row0, lane, [&](int e) { return pack_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])); });
+  }
+}
 template <int BN>
 __device__ __forceinline__ void swiglu_epilogue(uint32_t t_row, OutStage<2>& out, const SwigluMaps& maps, int row0, int f0,
                                                 int M, int F, int lane) {
@@ -338,7 +381,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate,
                     const __grid_constant__ SwigluMaps sw) {
   using Cfg = GemmCfg<BN, kGated>;
-  static_assert(Cfg::kSmemBytes + 1280 + (kGated == Gated::kNone ? 2 : 1) * kNeighbourShared <= kSmShared, "no room for the kernels beside this one");
+  static_assert(Cfg::kSmemBytes + 1280 + (plain_output(kGated) ? 2 : 1) * kNeighbourShared <= kSmShared, "no room for the kernels beside this one");
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[Cfg::kStages];
   __shared__ uint64_t bar_empty[Cfg::kStages];
@@ -480,14 +523,18 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int m0 = mb_ * kBM;
       const int n0 = nb_ * kCols;
       if (grouped_b_row(gate, mb_, n0, N) < 0) continue;
+      [[maybe_unused]] Angles angles;
+      if constexpr (kGated == Gated::kRotate) angles.load(sw, m0 + q * 32 + lane, M);
       mbar_wait(&bar_tfull[acc], aphase);
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
-      out.begin(smem + Cfg::kOutAt, smem, q, BN / 64, kGated == Gated::kNone && tile + static_cast<int>(gridDim.x) >= num_tiles);
+      out.begin(smem + Cfg::kOutAt, smem, q, BN / 64, plain_output(kGated) && tile + static_cast<int>(gridDim.x) >= num_tiles);
       if constexpr (kSwiglu)
         swiglu_epilogue<BN>(t_row, out, sw, m0 + q * 32, n0, M, N, lane);
       else if constexpr (kGated == Gated::kBackward)
         swiglu_bwd_epilogue<BN>(t_row, out.at, sw, m0 + q * 32, n0, M, N, lane);
+      else if constexpr (kGated == Gated::kRotate)
+        rotate_epilogue<BN>(t_row, out, &tmC, angles, sw.rotated, m0 + q * 32, n0, M, N, lane);
       else
         gemm_epilogue<BN, OutT>(t_row, out, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
@@ -539,7 +586,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                      const __grid_constant__ CUtensorMap tmC, OutT* __restrict__ C, long long ldc, int M, int N, int K, int beta, const GemmGate gate,
                     const __grid_constant__ SwigluMaps sw) {
   using Cfg = Gemm2Cfg<PBN, kGated>;
-  static_assert(Cfg::kSmemBytes + 1280 + (kGated == Gated::kNone ? 2 : 1) * kNeighbourShared <= kSmShared, "no room for the kernels beside this one");
+  static_assert(Cfg::kSmemBytes + 1280 + (plain_output(kGated) ? 2 : 1) * kNeighbourShared <= kSmShared, "no room for the kernels beside this one");
   constexpr int BN = Cfg::kBN;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[Cfg::kStages];
@@ -677,14 +724,18 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       mb_ = gate_perm(gate, mb_);
       const int m0 = mb_ * (2 * kBM) + static_cast<int>(cta_rank) * kBM;
       const int n0 = nb_ * kCols;
+      [[maybe_unused]] Angles angles;
+      if constexpr (kGated == Gated::kRotate) angles.load(sw, m0 + q * 32 + lane, M);
       mbar_wait(&bar_tfull[acc], aphase);
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
-      out.begin(smem + Cfg::kOutAt, smem, q, BN / 64, kGated == Gated::kNone && tile + num_pairs >= num_tiles);
+      out.begin(smem + Cfg::kOutAt, smem, q, BN / 64, plain_output(kGated) && tile + num_pairs >= num_tiles);
       if constexpr (kSwiglu)
         swiglu_epilogue<BN>(t_row, out, sw, m0 + q * 32, n0, M, N, lane);
       else if constexpr (kGated == Gated::kBackward)
         swiglu_bwd_epilogue<BN>(t_row, out.at, sw, m0 + q * 32, n0, M, N, lane);
+      else if constexpr (kGated == Gated::kRotate)
+        rotate_epilogue<BN>(t_row, out, &tmC, angles, sw.rotated, m0 + q * 32, n0, M, N, lane);
       else
         gemm_epilogue<BN, OutT>(t_row, out, &tmC, C, ldc, m0 + q * 32, n0, M, N, beta, lane);
       tc_fence_before();
@@ -1045,6 +1096,30 @@ static int launch_swiglu(const void* X, const void* W, void* GU, void* ACT, int 
 
 // kBN: 64 or 128 (one CTA), 256 (CTA pair).
 template <int kBN>
+static int launch_rotate(const void* X, const void* W, void* C, int M, int N, int K, long long ldx, long long ldw, long long ldc, const SwigluMaps& sw, cudaStream_t s) {
+  constexpr bool kPair = kBN == 256;
+  constexpr int kRows = (kPair ? 2 : 1) * kBM;
+  CUtensorMap tmA, tmW, tmC;
+  int rc = get_tmap_2d_bf16(&tmA, X, M, K, ldx, kBM, kBK, 1);
+  if (!rc) rc = get_tmap_2d_bf16(&tmW, W, N, K, ldw, kPair ? kBN / 2 : kBN, kBK, 1);
+  if (!rc) rc = get_tmap_2d_bf16(&tmC, C, M, N, ldc, 32, 64, 1);
+  if (rc) LLMCTL_FAIL(rc, "tensor maps");
+  const int tiles = ((M + kRows - 1) / kRows) * ((N + kBN - 1) / kBN), most = kPair ? num_sms() / 2 : num_sms();
+  const int grid = tiles < most ? tiles : most;
+  if constexpr (kPair) {
+    auto kern = gemm2_tcgen05_kernel<256, false, false, __nv_bfloat16, Gated::kRotate>;
+    LLMCTL_CHECK(allow_smem(kern, Gemm2Cfg<256, Gated::kRotate>::kSmemBytes));
+    LLMCTL_CHECK(launch_gemm_kernel(kern, 2 * grid, Gemm2Cfg<256, Gated::kRotate>::kSmemBytes, s, tmA, tmW, tmC, (__nv_bfloat16*)C, ldc, M, N, K, 0, GemmGate{}, sw));
+  } else {
+    auto kern = gemm_tcgen05_kernel<kBN, false, false, __nv_bfloat16, Gated::kRotate>;
+    LLMCTL_CHECK(allow_smem(kern, GemmCfg<kBN, Gated::kRotate>::kSmemBytes));
+    LLMCTL_CHECK(launch_gemm_kernel(kern, grid, GemmCfg<kBN, Gated::kRotate>::kSmemBytes, s, tmA, tmW, tmC, (__nv_bfloat16*)C, ldc, M, N, K, 0, GemmGate{}, sw));
+  }
+  LLMCTL_RETURN_LAST();
+}
+
+// kBN: 64 or 128 (one CTA), 256 (CTA pair).
+template <int kBN>
 static int launch_swiglu_bwd(const void* DY, const void* W, const void* GU, void* DGU, int M, int F, int K, long long lddy, long long ldw,
                              long long ldgu, cudaStream_t s) {
   constexpr bool kPair = kBN == 256;
@@ -1206,6 +1281,26 @@ LLMCTL_API int llmctl_gemm_swiglu_bwd_bf16(const void* DY, const void* W, const 
   const int bn = one_wave_tile(M, F);
   auto launch = bn == 64 ? launch_swiglu_bwd<64> : bn == 128 || M <= 128 || F <= 128 ? launch_swiglu_bwd<128> : launch_swiglu_bwd<256>;
   return launch(DY, W, GU, DGU, M, F, K, lddy, ldw, ldgu, (cudaStream_t)stream);
+}
+
+// C[M, N] = X W^T with the first `rotated` columns, heads of 64, rotated as llmctl_rope_inplace does (sign 1; cos, sin: [positions, 32]): a packed
+// projection and its rotation in one launch, without the pass over q and k between them.  Tiles by the rule of llmctl_gemm_bf16.
+// us of 12 layers of width 768 without gradients, two launches / one: 777 tokens 668 / 653, 2000 tokens 893 / 870, 100 tokens (host) 623 / 590.
+LLMCTL_API int llmctl_gemm_rope_bf16(const void* X, const void* W, void* C, int M, int N, int K, long long ldx, long long ldw, long long ldc, const float* cos_t,
+                                     const float* sin_t, const int* positions, int seq_len, int rotated, void* stream) {
+  LLMCTL_BEGIN();
+  LLMCTL_REQUIRE(M > 0 && N > 0 && K > 0 && N % 64 == 0 && rotated % 64 == 0 && rotated >= 0 && rotated <= N && ldx % 8 == 0 && ldw % 8 == 0 && ldc % 8 == 0 && ldc >= N &&
+                 seq_len > 0 && cos_t != nullptr && sin_t != nullptr);
+  LLMCTL_REQUIRE(aligned16(X, W, C, cos_t, sin_t));
+  SwigluMaps sw{};
+  sw.cos = cos_t;
+  sw.sin = sin_t;
+  sw.positions = positions;
+  sw.seq = seq_len;
+  sw.rotated = rotated;
+  const int bn = one_wave_tile(M, N);
+  const auto launch = bn == 64 ? launch_rotate<64> : bn == 128 || M <= 128 ? launch_rotate<128> : launch_rotate<256>;
+  return launch(X, W, C, M, N, K, ldx, ldw, ldc, sw, (cudaStream_t)stream);
 }
 
 // Grouped GEMM for mixture-of-experts layers: C[r, :] = A[r, :] W[expert(r)]^T over `max_tiles` blocks of 128 rows of A

@@ -39,8 +39,8 @@ rope_kernel(__nv_bfloat16* __restrict__ x, long long row_stride, uint32_t total,
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float sj = s[j] * sign;
-      oa[j] = a[j] * c[j] - b[j] * sj;
-      ob[j] = b[j] * c[j] + a[j] * sj;
+      oa[j] = __fmaf_rn(a[j], c[j], -__fmul_rn(b[j], sj));      // spelt out: the projection's epilogue rounds alike
+      ob[j] = __fmaf_rn(b[j], c[j], __fmul_rn(a[j], sj));
     }
     store8(p, pack8(oa));
     store8(p + half, pack8(ob));

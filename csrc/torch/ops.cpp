@@ -37,7 +37,7 @@ using at::Tensor;
 // the kernel library
 // ---------------------------------------------------------------------------------------------------------------------------------
 #define LLMCTL_ENTRIES(X)                                                                                                         \
-  X(llmctl_rmsnorm_fwd) X(llmctl_rmsnorm_bwd_bf16w) X(llmctl_rope_inplace) X(llmctl_gemm_bf16) X(llmctl_gemm_swiglu_bf16)               \
+  X(llmctl_rmsnorm_fwd) X(llmctl_rmsnorm_bwd_bf16w) X(llmctl_rope_inplace) X(llmctl_gemm_rope_bf16) X(llmctl_gemm_bf16) X(llmctl_gemm_swiglu_bf16)               \
   X(llmctl_gemm_swiglu_bwd_bf16) X(llmctl_swiglu_bwd) X(llmctl_gemm_skinny_bf16) X(llmctl_gemm_skinny_scratch_elems) X(llmctl_flash_attn_fwd) X(llmctl_flash_attn_bwd) X(llmctl_kv_append) \
   X(llmctl_paged_attn_decode) X(llmctl_paged_attn_scratch_elems) X(llmctl_latent_kv_write) X(llmctl_latent_decode)
 struct Entries {
@@ -728,8 +728,17 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
         return to;
       };
       const NormOut first = norm_fwd(x, residual, n1, eps, false);
-      const Tensor p = linear(first.y, qkv);
-      rope(p, cos, sin, positions, S, 2 * H, D, 1.f);
+      Tensor p;
+      if (D == 64 && lib.llmctl_gemm_rope_bf16 && unit16(cos) && unit16(sin)) {
+        p = new_bf16(x, {T, 3 * H * D});
+        done("llmctl_gemm_rope_bf16",
+             lib.llmctl_gemm_rope_bf16(cdata(first.y), cdata(qkv), data(p), static_cast<int>(T), static_cast<int>(3 * H * D), static_cast<int>(W), W, qkv.stride(0), 3 * H * D,
+                                       static_cast<const float*>(cdata(cos)), static_cast<const float*>(cdata(sin)),
+                                       positions.defined() ? static_cast<const int*>(cdata(positions)) : nullptr, static_cast<int>(S), static_cast<int>(2 * H * D), stream()));
+      } else {
+        p = linear(first.y, qkv);
+        rope(p, cos, sin, positions, S, 2 * H, D, 1.f);
+      }
       const Packed z = unpack(p, B, S, H, D);
       const NormOut second = norm_fwd(linear(attn_fwd(z.q, z.k, z.v, scale, true, false).o.view({T, H * D}), out), first.h, n2, eps, false);
       y = linear(up_and_activate(second.y, up, false).first, down);

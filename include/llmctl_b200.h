@@ -48,6 +48,8 @@ int llmctl_layernorm_bwd(const void* dy, const void* h, const void* w, const flo
                          void* stream);
 
 /* ---- K4 RoPE (rotate-half), in place; sign=+1 forward, -1 backward.  Reference: HF rotary. ---- */
+int llmctl_gemm_rope_bf16(const void* X, const void* W, void* C, int M, int N, int K, long long ldx, long long ldw, long long ldc, const float* cos_t,
+                          const float* sin_t, const int* positions, int seq_len, int rotated, void* stream);      /* X W^T, heads of 64 rotated */
 int llmctl_rope_inplace(void* x, long long row_stride, int n_tokens, int n_heads, int head_dim,
                         const float* cos_t, const float* sin_t, const int* positions, int seq_len,
                         float sign, void* stream);

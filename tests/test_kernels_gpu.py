@@ -536,6 +536,27 @@ def test_gemm_split_k(cuda_device, M, N, K, a_mn, b_mn, splits):
     assert err.norm() <= 2 * 2.0 ** -9 * (want + old).norm()
 
 
+@pytest.mark.parametrize("M,heads,K,seq", [(1, 1, 64, 1), (33, 3, 200, 11), (130, 12, 768, 130), (777, 12, 768, 259), (777, 20, 136, 777), (2000, 12, 72, 500), (4100, 16, 64, 1025)])
+@pytest.mark.parametrize("form", ["plain", "positions", "one part"])
+def test_gemm_with_rotation(cuda_device, M, heads, K, seq, form):
+    """The packed projection with its rotation (one wave of either narrow tile, pair tiles, ragged rows) against the product and the rotation after it:
+    the same bits."""
+    from llmctl_b200.ops import functional as ops, native
+    torch.manual_seed(M)
+    N = 3 * heads * 64
+    x, w = torch.randn(M, K, device=cuda_device).bfloat16(), torch.randn(N, K, device=cuda_device).bfloat16()
+    cos, sin = torch.randn(2048, 32, device=cuda_device), torch.randn(2048, 32, device=cuda_device)
+    positions = torch.randint(0, 2048, (M,), device=cuda_device, dtype=torch.int32) if form == "positions" else None
+    parts = heads if form == "one part" else 2 * heads
+    got = torch.full((M, N), float("nan"), device=cuda_device, dtype=torch.bfloat16)
+    native.register_signature("llmctl_gemm_rope_bf16", [native.c_void_p] * 3 + [native.c_int] * 3 + [native.c_ll] * 3 + [native.c_void_p] * 3 + [native.c_int] * 2 + [native.c_void_p])
+    native.call("llmctl_gemm_rope_bf16", x.data_ptr(), w.data_ptr(), got.data_ptr(), M, N, K, K, K, N, cos.data_ptr(), sin.data_ptr(), native.ptr(positions), seq,
+                parts * 64, native.stream_ptr())
+    want = ops.gemm_raw(x, w, tile_n=128)
+    native.call("llmctl_rope_inplace", want.data_ptr(), N, M, parts, 64, cos.data_ptr(), sin.data_ptr(), native.ptr(positions), seq, 1.0, native.stream_ptr())
+    assert torch.equal(got, want)
+
+
 # Lengths around the 128-row blocks and the 256-query items, more items than SMs (256 x 3 blocks), several head groups of the
 # backward's item order (S = 2048: 16 heads of 128 to a group), non-causal whole blocks, views at an odd address (copied first).
 @pytest.mark.parametrize("B,S,H,D,causal,shift", [
