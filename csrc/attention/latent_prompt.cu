@@ -30,18 +30,28 @@ latent_prompt_prepare_kernel(__nv_bfloat16* __restrict__ q, long long ldq, int t
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * kPrepWarps + (threadIdx.x >> 5);
   if (w < tokens) {
-    // ---- rotate: lane = coordinate pair; all heads of the token ----
+    // ---- rotate: lane = coordinate pair; all heads of the token, kAhead of them asked for before the first is stored (a head is stored where
+    // the next might be read, so the loads do not move up by themselves and the heads of a token were a chain).  A layer over two prompts of 2048
+    // tokens, 16 heads: 141.4 -> 140.6 us, three runs of each within 0.4 ----
+    constexpr int kAhead = 16;
     __nv_bfloat16* row = q + w * ldq + dn;
-    const float pos = static_cast<float>(positions[w]);
     for (int i = lane; i < dr / 2; i += 32) {
-      float s, c;
-      sincosf(pos * freq[i], &s, &c);
-      s *= mult;
-      c *= mult;
-      for (int h = 0; h < H; ++h) {
-        __nv_bfloat162* at = reinterpret_cast<__nv_bfloat162*>(row + h * (dn + dr) + 2 * i);
-        const float2 v = __bfloat1622float2(*at);
-        *at = __floats2bfloat162_rn(v.x * c - v.y * s, v.y * c + v.x * s);
+      float s = 0.f, c = 0.f;
+      for (int h0 = 0; h0 < H; h0 += kAhead) {
+        __nv_bfloat162 x[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+          if (h0 + u < H) x[u] = *reinterpret_cast<const __nv_bfloat162*>(row + (h0 + u) * (dn + dr) + 2 * i);
+        if (h0 == 0) {
+          sincosf(static_cast<float>(positions[w]) * freq[i], &s, &c);
+          s *= mult;
+          c *= mult;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const float2 v = __bfloat1622float2(x[u]);
+          if (h0 + u < H) *reinterpret_cast<__nv_bfloat162*>(row + (h0 + u) * (dn + dr) + 2 * i) = __floats2bfloat162_rn(v.x * c - v.y * s, v.y * c + v.x * s);
+        }
       }
     }
     return;
