@@ -12,6 +12,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/autocast_mode.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
@@ -23,6 +24,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
+#include <array>
 #include <atomic>
 #include <cstdio>
 #include <initializer_list>
@@ -351,10 +353,20 @@ Tensor dgrad(const Tensor& dy, const Tensor& w, int tile_n) {
 // Nodes of the products: saved tensors and a lock, as autograd's own nodes have them.
 struct Products : torch::autograd::Node {
   std::vector<torch::autograd::SavedVariable> saved;
+  std::vector<std::array<int64_t, 2>> sizes;
   int tile_n = 0;
   void keep(std::initializer_list<const Tensor*> ts) {
     saved.reserve(ts.size());
-    for (const Tensor* t : ts) saved.emplace_back(*t, false);
+    for (const Tensor* t : ts) {
+      saved.emplace_back(*t, false);
+      sizes.push_back({t->size(0), t->size(1)});
+    }
+  }
+  // a hook on saved tensors may give back anything: what the kernels cannot read is refused
+  Tensor operand(size_t i) {
+    Tensor t = saved[i].unpack();
+    TORCH_CHECK(t.is_cuda() && is_matrix(t) && t.size(0) == sizes[i][0] && t.size(1) == sizes[i][1], name(), ": a saved matrix came back as ", t.scalar_type(), " of sizes ", t.sizes(), " on ", t.device());
+    return t;
   }
   void release_variables() override {
     std::lock_guard<std::mutex> hold(mutex_);
@@ -384,7 +396,7 @@ struct LinearNode final : Products {
     std::lock_guard<std::mutex> hold(mutex_);
     if (!grads[0].defined()) return {Tensor(), Tensor()};
     return node_body("llmctl_gemm_bf16", ready(lib.llmctl_gemm_bf16), [&]() -> torch::autograd::variable_list {
-      const Tensor x = saved[0].unpack(), w = saved[1].unpack();
+      const Tensor x = operand(0), w = operand(1);
       at::AutoDispatchBelowADInplaceOrView below;
       const Tensor dy = rows(grads[0]);
       Tensor dx, dw;
@@ -417,7 +429,7 @@ struct LinearSwigluNode final : Products {
     std::lock_guard<std::mutex> hold(mutex_);
     if (!grads[0].defined()) return {Tensor(), Tensor()};
     return node_body("llmctl_swiglu_bwd", ready(lib.llmctl_swiglu_bwd) && lib.llmctl_gemm_bf16, [&]() -> torch::autograd::variable_list {
-      const Tensor x = saved[0].unpack(), w = saved[1].unpack(), gu = saved[2].unpack();
+      const Tensor x = operand(0), w = operand(1), gu = operand(2);
       at::AutoDispatchBelowADInplaceOrView below;
       const Tensor dact = whole_units(grads[0]);
       Tensor dgu = new_bf16(gu, gu.sizes()), dx, dw;
@@ -445,7 +457,7 @@ struct SwigluMlpNode final : Products {
     std::lock_guard<std::mutex> hold(mutex_);
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
     return node_body("llmctl_gemm_swiglu_bwd_bf16", ready(lib.llmctl_gemm_swiglu_bwd_bf16) && lib.llmctl_gemm_bf16, [&]() -> torch::autograd::variable_list {
-      const Tensor x = saved[0].unpack(), up = saved[1].unpack(), down = saved[2].unpack(), gu = saved[3].unpack(), act = saved[4].unpack();
+      const Tensor x = operand(0), up = operand(1), down = operand(2), gu = operand(3), act = operand(4);
       at::AutoDispatchBelowADInplaceOrView below;
       const Tensor dy = rows(grads[0]);
       Tensor dgu, dx, d_up, d_down;
@@ -611,6 +623,9 @@ struct FlashAttention final : torch::autograd::Node {
     return node_body("llmctl_flash_attn_bwd", ready(lib.llmctl_flash_attn_bwd), [&]() -> torch::autograd::variable_list {
       const auto self = getptr();
       const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), o_ = o.unpack(self), lse_ = lse.unpack();
+      TORCH_CHECK(q_.is_cuda() && k_.is_cuda() && v_.is_cuda() && o_.is_cuda() && attention_ok(q_, k_, v_, causal) && bf16(o_) && o_.is_contiguous() && unit16(o_) && o_.sizes() == q_.sizes() && lse_.is_cuda() &&
+                      lse_.scalar_type() == at::kFloat && lse_.is_contiguous() && lse_.numel() == q_.size(0) * q_.size(1) * q_.size(2) && grads[0].sizes() == q_.sizes(),
+                  "FlashAttentionBackward: saved tensors came back in other forms");
       at::AutoDispatchBelowADInplaceOrView below;
       const Tensor d = attn_bwd(q_, k_, v_, o_, lse_, grads[0], scale, causal);
       return {d.select(2, 0), d.select(2, 1), d.select(2, 2)};
@@ -840,7 +855,7 @@ PyObject* py_latent_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const double mult = args.number(9), scale = args.number(10);
     const int hpt = static_cast<int>(args.integer(11)), window = static_cast<int>(args.integer(15));
     if (!args.ok || !quiet() || !ready(lib.llmctl_latent_decode) || !bf16(q) || q.dim() != 2 || q.numel() == 0 || q.stride(1) != 1 || !bf16(uk) || !bf16(uv) || uk.dim() != 3 ||
-        uv.dim() != 3 || recorded({&q, &uk, &uv}) || !bf16(cache) || cache.dim() != 3 || !cache.is_contiguous() || !unit16(cache))
+        uv.dim() != 3 || recorded({&q, &uk, &uv}) || at::autocast::is_autocast_enabled(at::kCUDA) || !bf16(cache) || cache.dim() != 3 || !cache.is_contiguous() || !unit16(cache))
       return none();
     const int64_t T = q.size(0), H = uk.size(0), R = uk.size(2), D = cache.size(2), dr = D - R, dv = uv.size(1);
     if (dr < 0 || uk.size(1) != dn || q.size(1) < H * (dn + dr) || uv.size(0) != H || uv.size(2) != R || hpt < 1 || hpt > 32 || splits < 1 || tables.dim() != 2 ||

@@ -317,6 +317,23 @@ def test_saved_tensor_hooks_see_what_is_kept(ops):
     assert sorted(unpacked) == list(range(len(packed))) and q.grad.abs().sum() > 0
 
 
+@pytest.mark.parametrize("form", ["fp32", "cpu", "columns", "part"])
+@pytest.mark.parametrize("call", ["linear", "mlp", "two products", "attention"])
+def test_saved_tensors_that_come_back_in_other_forms_are_refused(ops, form, call):
+    """A hook may give back anything: what the kernels would read wrongly, or out of range, is an error before any launch."""
+    def unpack(t):
+        return {"fp32": t.float, "cpu": t.cpu, "columns": lambda: t.transpose(0, 1).contiguous().transpose(0, 1), "part": lambda: t[:-1]}[form]()
+    x, up, down = (_randn(*size, seed=i).requires_grad_(True) for i, size in enumerate([(40, 64), (256, 64), (64 if call == "two products" else 4096, 128)]))
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        if call == "attention":
+            y = ops.attention(*(_randn(2, 130, 2, 64, seed=i).requires_grad_(True) for i in range(3)))
+        else:
+            y = ops.linear(x, up) if call == "linear" else ops.swiglu_mlp(x, up, down)
+    with pytest.raises(RuntimeError):
+        y.sum().backward()
+    torch.cuda.synchronize()
+
+
 def test_transforms_modes_and_subclasses_go_to_the_python_operators(ops):
     """What wants to see the operators or replace their tensors finds the Python ones, which record or refuse it as before."""
     from torch.utils._python_dispatch import TorchDispatchMode
