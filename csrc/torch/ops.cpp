@@ -429,9 +429,9 @@ struct LinearSwigluNode final : Products {
     std::lock_guard<std::mutex> hold(mutex_);
     if (!grads[0].defined()) return {Tensor(), Tensor()};
     return node_body("llmctl_swiglu_bwd", ready(lib.llmctl_swiglu_bwd) && lib.llmctl_gemm_bf16, [&]() -> torch::autograd::variable_list {
-      const Tensor x = operand(0), w = operand(1), gu = operand(2);
+      const Tensor x = operand(0), w = operand(1);
       at::AutoDispatchBelowADInplaceOrView below;
-      const Tensor dact = whole_units(grads[0]);
+      const Tensor gu = whole_units(operand(2)), dact = whole_units(grads[0]);      // the kernel's one row stride is that of gu and of its gradient
       Tensor dgu = new_bf16(gu, gu.sizes()), dx, dw;
       done("llmctl_swiglu_bwd", lib.llmctl_swiglu_bwd(cdata(dact), cdata(gu), data(dgu), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2), gu.stride(0), ::stream()));
       if (task_should_compute_output(0)) dx = dgrad(dgu, w, 0);
@@ -457,9 +457,9 @@ struct SwigluMlpNode final : Products {
     std::lock_guard<std::mutex> hold(mutex_);
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
     return node_body("llmctl_gemm_swiglu_bwd_bf16", ready(lib.llmctl_gemm_swiglu_bwd_bf16) && lib.llmctl_gemm_bf16, [&]() -> torch::autograd::variable_list {
-      const Tensor x = operand(0), up = operand(1), down = operand(2), gu = operand(3), act = operand(4);
+      const Tensor x = operand(0), up = operand(1), down = operand(2), act = operand(4);
       at::AutoDispatchBelowADInplaceOrView below;
-      const Tensor dy = rows(grads[0]);
+      const Tensor gu = whole_units(operand(3)), dy = rows(grads[0]);               // the kernel's one row stride is that of gu and of its gradient
       Tensor dgu, dx, d_up, d_down;
       if (task_should_compute_output(0) || task_should_compute_output(1)) {
         dgu = new_bf16(gu, gu.sizes());

@@ -526,8 +526,8 @@ class _LinearSwiGLUFn(torch.autograd.Function):
     def backward(ctx, dact):
         x, w, gu = ctx.saved_tensors
         M, F2 = gu.shape
-        dact = _whole_units(dact)
-        dgu = torch.empty_like(gu)
+        gu, dact = _whole_units(gu), _whole_units(dact)         # a hook on saved tensors may give back rows with gaps
+        dgu = torch.empty_like(gu)                              # the kernel's one row stride is that of both
         native.call("llmctl_swiglu_bwd", dact.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, F2 // 2, gu.stride(0), native.stream_ptr())
         dx = gemm_raw(dgu, w, b_mn=True) if ctx.needs_input_grad[0] else None
         dw = _wgrad(dgu, x, w) if ctx.needs_input_grad[1] else None
@@ -557,7 +557,8 @@ class _SwiGLUMLPFn(torch.autograd.Function):
         dx = dw_up = dgu = None
         if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
             M, F2 = gu.shape
-            dgu = torch.empty_like(gu)
+            gu = _whole_units(gu)                               # a hook on saved tensors may give back rows with gaps
+            dgu = torch.empty_like(gu)                          # the kernel's one row stride is that of both
             native.call("llmctl_gemm_swiglu_bwd_bf16", dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, F2 // 2, dy.shape[1],
                         dy.stride(0), w_down.stride(0), gu.stride(0), native.stream_ptr())
         dw_down = _wgrad(dy, act, w_down) if ctx.needs_input_grad[2] else None

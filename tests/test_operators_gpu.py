@@ -334,6 +334,20 @@ def test_saved_tensors_that_come_back_in_other_forms_are_refused(ops, form, call
     torch.cuda.synchronize()
 
 
+@pytest.mark.parametrize("extension", [True, False])
+@pytest.mark.parametrize("call", ["linear", "mlp", "two products"])
+def test_saved_rows_that_come_back_with_gaps_give_the_same_gradients(ops, extension, call):
+    """The layout that a hook may change without being refused: rows of whole 16-byte units with something between them."""
+    def run(unpack):
+        leaves = [_randn(*size, seed=i).requires_grad_(True) for i, size in enumerate([(40, 64), (256, 64), (64 if call == "two products" else 4096, 128)])]
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            y = ops.linear(*leaves[:2]) if call == "linear" else ops.swiglu_mlp(*leaves)
+        y.backward(_randn(*y.shape, seed=4))
+        return [t.grad for t in leaves[:2 if call == "linear" else 3]]
+    with contextlib.nullcontext() if extension else python_operators():
+        _same(run(lambda t: torch.cat([t, t[:, :8]], 1)[:, :t.shape[1]]), run(lambda t: t))
+
+
 def test_transforms_modes_and_subclasses_go_to_the_python_operators(ops):
     """What wants to see the operators or replace their tensors finds the Python ones, which record or refuse it as before."""
     from torch.utils._python_dispatch import TorchDispatchMode

@@ -654,6 +654,26 @@ int main() {
     assert r.returncode == 0, r.stdout
 
 
+@pytest.mark.parametrize("node", ["_LinearSwiGLUFn", "_SwiGLUMLPFn"])
+def test_gated_backwards_write_within_their_gradient(monkeypatch, node):
+    """gate | up that comes back from a hook on saved tensors as rows with gaps: the kernels have one row stride for it and for its gradient."""
+    from types import SimpleNamespace
+    from llmctl_b200.ops import functional as ops
+    from llmctl_b200.ops import native
+    rows, width, cols = 6, 16, 24
+    gu = torch.zeros(rows, 2 * width + 8, dtype=torch.bfloat16)[:, :2 * width]
+    x, up, down, act = (torch.zeros(*s, dtype=torch.bfloat16) for s in ((rows, 8), (2 * width, 8), (cols, width), (rows, width)))
+    stride, operands = {}, []
+    monkeypatch.setattr(native, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(native, "call", lambda name, *a: stride.update(gate_up=a[5] if name == "llmctl_swiglu_bwd" else a[9]))
+    monkeypatch.setattr(ops, "gemm_raw", lambda a, b, **k: operands.append(a))
+    monkeypatch.setattr(ops, "_wgrad", lambda *a: None)
+    ctx = SimpleNamespace(needs_input_grad=[True] * 3, saved_tensors=(x, up, gu) if node == "_LinearSwiGLUFn" else (x, up, down, gu, act))
+    getattr(ops, node).backward(ctx, act if node == "_LinearSwiGLUFn" else torch.zeros(rows, cols, dtype=torch.bfloat16))
+    (dgu,) = operands
+    assert dgu.stride(0) == stride["gate_up"] and dgu.untyped_storage().nbytes() >= 2 * ((rows - 1) * stride["gate_up"] + 2 * width)
+
+
 def test_division_by_a_launch_constant(tmp_path):
     """csrc/common/fast_div.h against the machine's division: divisors and numbers at and around powers of two, the ends of their ranges,
     and a spread of others."""
