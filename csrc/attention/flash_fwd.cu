@@ -6,6 +6,7 @@
 // Reference: HF modules choose SDPA/eager attention behind `self.model(**batch)` (reference
 // llmctl/runtime/engine.py:284); the reference's tuner times a naive softmax(QK^T)V (reference
 // llmctl/plugins/autotuning.py:149-188).  Baseline to beat: cuDNN / flash-attn SDPA.
+#include <float.h>
 #include <math.h>
 
 #include "../common/ptx.cuh"
@@ -444,7 +445,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int nb = blocks(sq, q0, t);
       if (!kSplit && nb == 0) continue;            // tile B past the end of the sequence: nobody touches its barriers
       const int qt0 = kSplit ? q0 : q0 + t * kRows, first_block = kSplit && t == 1 ? blocks(sq, q0, 0) : 0;
-      float m_ref = -INFINITY, l0 = 0.f, l1 = 0.f;
+      // a half's reference starts finite: scores of -inf, all that a row may see of it, then weigh nothing instead of being no number
+      float m_ref = kSplit ? -FLT_MAX : -INFINITY, l0 = 0.f, l1 = 0.f;
       for (int j = 0; j < nb; ++j, ++nS) {
         mbar_wait_or_abort(&bar_s[t], nS & 1u, abort);
         __syncwarp();
@@ -468,7 +470,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (lane == 0) mbar_arrive(&bar_half[t]);
         mbar_wait_or_abort(&bar_half[1 - t], nO & 1u, abort);
         const float2 other = half_ml[1 - t][row];
-        const float m = fmaxf(m_ref, other.x);             // A's half has a visible key for every row
+        const float m = fmaxf(m_ref, other.x);
         by[t] = ex2_approx(m_ref - m);
         by[1 - t] = ex2_approx(other.x - m);
         l = l * by[t] + other.y * by[1 - t];

@@ -617,6 +617,24 @@ def test_flash_attention_split_keys(cuda_device, B, S, H, D, causal):
         assert (lse[:, h].double() - exact).abs().max() <= 1e-5 * exact.abs().max().clamp(min=1)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("keys", [slice(512, None), slice(0, 512), slice(600, 700)])
+def test_flash_attention_scores_of_minus_infinity(cuda_device, D, keys):
+    """Keys whose scores are -inf weigh nothing, also where they are all that a row sees of one half of the keys (blocks of 128: 0 to 3 and 4 to 6 of
+    the last rows); a row that sees no other has no result.  Bound as above."""
+    from llmctl_b200.ops import attention as attn
+    torch.manual_seed(1)
+    q, k, v = (torch.randn(1, 777, 12, D, device=cuda_device).bfloat16() for _ in range(3))
+    q[..., 0] = q[..., 0].abs() + 0.1
+    k[:, keys, :, 0] = float("-inf")
+    got = attn.attention(q, k, v).double()
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) / math.sqrt(D)
+    s = s.masked_fill(torch.ones(777, 777, dtype=torch.bool, device=cuda_device).triu(1), float("-inf"))
+    want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v.double())
+    assert torch.equal(got.isnan(), want.isnan())
+    assert (got - want).nan_to_num().norm() <= 2 * 2.0 ** -9 * want.nan_to_num().norm()
+
+
 @pytest.mark.parametrize("which", [0, 1, 2])
 def test_whole_tiles_at_odd_addresses_are_copied(cuda_device, which):
     """Heads of 128 and whole 128-token tiles where one of q, k and v begins at an odd address: the kernels run on copies, and nothing else
