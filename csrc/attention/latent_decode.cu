@@ -23,6 +23,8 @@
 // CTA to an SM (two: 39 -> 43).
 // Every wait is bounded, as in latent_attention_t5.cu.
 // Reference: none (the reference has no model code).
+#include <float.h>
+
 #include "../common/dependent.cuh"
 #include "../common/dtype.cuh"
 #include "../common/mma_sync.cuh"
@@ -294,10 +296,11 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __nv_bfloat1
 
       const float scale_log2 = scale * kLog2e;
       const int key = quad * 16 + lane;                   // of the tile; lanes 16 .. 31 have none
-      // a sink is a key without a value: it is the head's first reference, and its term of the sum
+      // a sink is a key without a value: it is the head's first reference, and its term of the sum.  References start finite, so that scores of -inf,
+      // where a head has seen no other, weigh nothing instead of being no number.
       const bool sink = sinks != nullptr && split == 0;
       float __align__(16) ref[N];
-      float sum[N], my_ref = sink && lane % N < nh ? sinks[h0 + lane % N] * kLog2e : -INFINITY;       // of the lane's own head
+      float sum[N], my_ref = sink && lane % N < nh ? fmaxf(sinks[h0 + lane % N] * kLog2e, -FLT_MAX) : -FLT_MAX;       // of the lane's own head
 #pragma unroll
       for (int h = 0; h < N; ++h) {
         ref[h] = __shfl_sync(0xffffffffu, my_ref, h);
@@ -330,7 +333,7 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __nv_bfloat1
           const float m = fmaxf(my_ref, fmaxf(fmaxf(warp_row[0][head], warp_row[1][head]), fmaxf(warp_row[2][head], warp_row[3][head])));
           if (lane < N) {
             new_ref[w][head] = m;
-            new_alpha[w][head] = my_ref == -INFINITY ? 0.f : ex2_approx(my_ref - m);
+            new_alpha[w][head] = ex2_approx(my_ref - m);
           }
           my_ref = m;
           if (n > 0) mbar_wait_or_abort(&bar_pv[(n - 1) & 1], ((n - 1) >> 1) & 1u, abort);

@@ -194,6 +194,32 @@ def test_latent_decode_tcgen05(cuda_device, contexts, H, dr, R, bs, splits, wind
         assert err < 2 * 2 * 2 ** -9, (contexts[i], float(err))
 
 
+@pytest.mark.parametrize("one_token", [False, True])
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("keys", [slice(0, 64), slice(0, 130), slice(70, 200), slice(0, 200)])
+@pytest.mark.parametrize("sink", [None, 0.5, float("-inf")])
+def test_latent_decode_scores_of_minus_infinity(cuda_device, one_token, splits, keys, sink):
+    """Keys whose scores are -inf (a rotated coordinate of -inf; nothing is rotated) weigh nothing, whole tiles and splits of them, as on the
+    general kernel; with no other key nothing is seen.  Bound as above."""
+    from llmctl_b200.ops import latent_attention as L, native
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+    torch.manual_seed(2)
+    H, dn, dr, R, bs, n = 16, 8, 64, 128, 64, 200
+    cache, ql, q = torch.randn(4, bs, R + dr).bfloat16().cuda(), torch.randn(1, H, R).bfloat16().cuda(), torch.randn(1, H, dn + dr).bfloat16().cuda()
+    q[..., dn] = 1.0
+    cache.view(-1, R + dr)[keys, R] = float("-inf")
+    sinks = None if sink is None else torch.full((H,), sink, device="cuda")
+    b = RaggedBatch([Portion(0, [0], n - 1, [0], [0, 1, 2, 3])], bs, torch.device("cuda"))
+    got = L.latent_attention(ql, q.view(1, -1), dn, cache, b.block_tables, b.tiles(16), b.positions, torch.zeros(dr // 2, device="cuda"), 1.0, 0.1, 16, b.max_context,
+                             splits, sinks=sinks, one_token=one_token)[0].double()
+    k = cache.view(-1, R + dr)[:n].double()
+    s = torch.cat([ql[0].double(), q[0, :, dn:].double()], 1) @ k.T * 0.1
+    extra = torch.full((H, 1), float("-inf") if sink is None else sink, dtype=torch.float64, device="cuda")
+    want = torch.softmax(torch.cat([s, extra], 1), 1)[:, :n].nan_to_num() @ k[:, :R]
+    assert (got - want).norm() <= 2 * 2 * 2 ** -9 * want.norm()
+    assert native.lib().llmctl_latent_attention_t5_status(1) == 0
+
+
 # (tokens, position of the first) of the batch's portions: one prompt around the 128-key and 256-query blocks, portions behind earlier
 # keys at positions that are and are not multiples of 128, unlike lengths side by side, a single token among them
 @pytest.mark.parametrize("portions", [[(64, 0)], [(127, 0)], [(128, 0)], [(129, 0)], [(257, 0)], [(700, 0)], [(300, 128)], [(300, 1)],
