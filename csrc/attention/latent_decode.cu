@@ -14,7 +14,8 @@
 //   warp 1      MMA issuer
 //   warps 2-5   assemble Q (absorbed part | rotated part) in shared memory, then turn S^T into P^T: a key per thread, all its heads; a running
 //               reference per head that moves only when a score outgrows it by 2^8 (one vote per tile instead of maxima over keys,
-//               which lie in different threads), probabilities in bf16, their sums in fp32
+//               which lie in different threads), probabilities in bf16, their sums in fp32 over what was rounded: a key that decides alone
+//               then weighs 1, wherever the reference stands
 // TMEM: S^T two buffers of N columns (64 rows: lanes 32q + 0 .. 15 of quadrant q), O^T R / 128 blocks of N columns.
 //
 // Bound by HBM: two stages in flight and 27 / 46 clocks for each of a tile's 36 / 16 products leave 3350 clocks a tile, 6.2 TB/s over 148 CTAs.
@@ -370,9 +371,12 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __nv_bfloat1
             for (int e = 0; e < 8; ++e) {
               const int h = g * 8 + e;
               f[e] = seen ? ex2_approx(__uint_as_float(s[h]) - ref[h]) : 0.f;
-              sum[h] += f[e];
             }
-            *reinterpret_cast<bf16x8*>(dst + g * 1024) = pack8(f);
+            const bf16x8 p = pack8(f);
+            *reinterpret_cast<bf16x8*>(dst + g * 1024) = p;
+            unpack8(p, f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum[g * 8 + e] += f[e];
           }
         }
         // Rows past the last key: nothing that the cache holds there may meet a probability of zero.

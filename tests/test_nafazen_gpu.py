@@ -220,6 +220,29 @@ def test_latent_decode_scores_of_minus_infinity(cuda_device, one_token, splits, 
     assert native.lib().llmctl_latent_attention_t5_status(1) == 0
 
 
+@pytest.mark.parametrize("one_token", [False, True])
+@pytest.mark.parametrize("splits", [1, 2])
+def test_latent_decode_of_a_key_that_decides_behind_the_reference(cuda_device, one_token, splits):
+    """A key of weight 0.992 in the second tile whose probability lies between two bf16 numbers (128.47 of the first tile's largest): what its
+    rounding takes off has to leave the sum as well.  The output's rounding alone is 2^-9 in the 2-norm; the key's would add 0.0037."""
+    import math
+    from llmctl_b200.ops import latent_attention as L
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+    torch.manual_seed(3)
+    H, dn, dr, R, bs, n = 16, 8, 64, 128, 64, 65
+    cache, ql, q = torch.randn(2, bs, R + dr).bfloat16().cuda(), torch.zeros(1, H, R).bfloat16().cuda(), torch.zeros(1, H * (dn + dr)).bfloat16().cuda()
+    ql[..., 0] = 1.0
+    first = cache.view(-1, R + dr)[:n, 0]
+    first[:] = -16.0
+    first[0], first[64] = 0.0, 1.0
+    b = RaggedBatch([Portion(0, [0], n - 1, [0], [0, 1])], bs, torch.device("cuda"))
+    got = L.latent_attention(ql, q, dn, cache, b.block_tables, b.tiles(16), b.positions, torch.zeros(dr // 2, device="cuda"), 1.0, math.log(128.47), 16,
+                             b.max_context, splits, one_token=one_token)[0].double()
+    k = cache.view(-1, R + dr)[:n, :R].double()
+    want = torch.softmax(k[:, 0] * math.log(128.47), 0) @ k
+    assert (got - want).norm() <= 2 ** -9 * want.norm() * H ** 0.5
+
+
 # (tokens, position of the first) of the batch's portions: one prompt around the 128-key and 256-query blocks, portions behind earlier
 # keys at positions that are and are not multiples of 128, unlike lengths side by side, a single token among them
 @pytest.mark.parametrize("portions", [[(64, 0)], [(127, 0)], [(128, 0)], [(129, 0)], [(257, 0)], [(700, 0)], [(300, 128)], [(300, 1)],
