@@ -22,6 +22,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include <array>
@@ -350,62 +351,132 @@ Tensor dgrad(const Tensor& dy, const Tensor& w, int tile_n) {
   return dx;
 }
 
-// Nodes of the products: saved tensors and a lock, as autograd's own nodes have them.
-struct Products : torch::autograd::Node {
+// A recorded operator as a node of its own: torch::autograd::Function looks its arguments up by name, and wraps and checks them in ways that
+// operators which return one new tensor have no use for (forward and backward of a small attention 72 us; the engine alone takes 29).  `T` says
+// what its backward needs (kEntry, there()) and is
+//   static variable_list gradients(const Numbers&, const Tensor& grad, const variable_list& saved, unsigned wants)
+// with a bit of `wants` for each gradient that is asked for.  Nothing else may enter: compiled autograd calls it with tensors of its own, and
+// for any call whose numbers and `wants` are the same.
+namespace compiled = torch::dynamo::autograd;
+template <typename T, typename Numbers>
+struct Recorded : torch::autograd::Node {
   std::vector<torch::autograd::SavedVariable> saved;
-  std::vector<std::array<int64_t, 2>> sizes;
-  int tile_n = 0;
-  void keep(std::initializer_list<const Tensor*> ts) {
-    saved.reserve(ts.size());
-    for (const Tensor* t : ts) {
-      saved.emplace_back(*t, false);
-      sizes.push_back({t->size(0), t->size(1)});
-    }
+  int output = -1;                                 // which of them is what the forward returned
+  Numbers numbers;
+
+  static std::shared_ptr<T> make(torch::autograd::edge_list&& next, Numbers numbers) {
+    std::shared_ptr<T> node(new T(), torch::autograd::deleteNode);
+    node->set_next_edges(std::move(next));
+    node->numbers = std::move(numbers);
+    return node;
   }
-  // a hook on saved tensors may give back anything: what the kernels cannot read is refused
-  Tensor operand(size_t i) {
-    Tensor t = saved[i].unpack();
-    TORCH_CHECK(t.is_cuda() && is_matrix(t) && t.size(0) == sizes[i][0] && t.size(1) == sizes[i][1], name(), ": a saved matrix came back as ", t.scalar_type(), " of sizes ", t.sizes(), " on ", t.device());
-    return t;
+  torch::autograd::variable_list kept() {
+    torch::autograd::variable_list ts;
+    ts.reserve(saved.size());
+    for (size_t i = 0; i < saved.size(); ++i) ts.push_back(static_cast<int>(i) == output ? saved[i].unpack(getptr()) : saved[i].unpack());
+    return ts;
+  }
+  unsigned wants() const {
+    unsigned bits = 0;
+    for (uint32_t i = 0; i < num_outputs(); ++i) bits |= static_cast<unsigned>(task_should_compute_output(i)) << i;
+    return bits;
+  }
+  static torch::autograd::variable_list run(const Numbers& numbers, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
+    return node_body(T::kEntry, T::there(), [&] { return T::gradients(numbers, grad, kept, wants); });
+  }
+
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    if (!grads[0].defined()) return torch::autograd::variable_list(num_outputs());
+    return run(numbers, grads[0], kept(), wants());
   }
   void release_variables() override {
     std::lock_guard<std::mutex> hold(mutex_);
     for (auto& t : saved) t.reset_data();
   }
-  // the gradient as an operand
-  static Tensor rows(const Tensor& g) { return is_matrix(g) ? g : whole_units(g); }
+  void compiled_args(compiled::CompiledNodeArgs& args) const override {
+    for (size_t i = 0; i < saved.size(); ++i) args.collect(saved[i], static_cast<int>(i) == output);
+    numbers.collect(args);
+    args.collect(static_cast<int64_t>(wants()));
+  }
+  torch::autograd::variable_list apply_with_saved(const torch::autograd::variable_list& grads, compiled::SwapSavedVariables& swap) override {
+    for (auto& t : saved) swap.before(t);
+    compiled::PackedArgs packed;
+    std::vector<at::TypePtr> schema;
+    for (const Tensor& t : kept()) {
+      packed.pack(t);
+      schema.push_back(compiled::IValuePacker<Tensor>::packed_type());
+    }
+    const size_t outputs = num_outputs(), n = saved.size();
+    auto later = [numbers = numbers, wants = wants(), outputs, n](const torch::autograd::variable_list& grads, const std::vector<c10::IValue>& stack) {
+      compiled::PackedArgs packed(stack);
+      torch::autograd::variable_list kept;
+      for (size_t i = 0; i < n; ++i) kept.push_back(packed.unpack<Tensor>());
+      return grads[0].defined() ? run(numbers, grads[0], kept, wants) : torch::autograd::variable_list(outputs);
+    };
+    const auto& compiler = compiled::getPyCompilerInterface();
+    const std::string id = compiler->bind_function(swap.get_py_compiler(), name(), later, schema, /*is_custom_function=*/true, /*is_traceable=*/false);
+    const auto metadata = compiled::IValuePacker<std::vector<std::optional<torch::autograd::InputMetadata>>>::pack(compiled::get_input_metadata(next_edges()));
+    auto out = compiler->call_function(swap.get_py_compiler(), "apply_functional", id, grads, packed.vec(), metadata);
+    for (auto& t : saved) swap.after(t);
+    return out;
+  }
+};
+
+struct ProductNumbers {
+  int tile_n = 0;
+  std::vector<std::array<int64_t, 2>> sizes;       // of the saved matrices
+  void collect(compiled::CompiledNodeArgs& args) const {
+    args.collect(static_cast<int64_t>(tile_n));
+    for (const auto& s : sizes) {
+      args.collect(s[0]);
+      args.collect(s[1]);
+    }
+  }
 };
 template <typename T>
-std::shared_ptr<T> new_node(torch::autograd::edge_list&& next, int tile_n) {
-  std::shared_ptr<T> node(new T(), torch::autograd::deleteNode);
-  node->set_next_edges(std::move(next));
-  node->tile_n = tile_n;
-  return node;
-}
+struct Product : Recorded<T, ProductNumbers> {
+  void keep(std::initializer_list<const Tensor*> ts) {
+    this->saved.reserve(ts.size());
+    for (const Tensor* t : ts) {
+      this->saved.emplace_back(*t, false);
+      this->numbers.sizes.push_back({t->size(0), t->size(1)});
+    }
+  }
+  // a hook on saved tensors may give back anything: what the kernels cannot read is refused
+  static void check(const ProductNumbers& numbers, const torch::autograd::variable_list& kept) {
+    for (size_t i = 0; i < kept.size(); ++i) {
+      const Tensor& t = kept[i];
+      TORCH_CHECK(t.is_cuda() && is_matrix(t) && t.size(0) == numbers.sizes[i][0] && t.size(1) == numbers.sizes[i][1], T::kName, ": a saved matrix came back as ",
+                  t.scalar_type(), " of sizes ", t.sizes(), " on ", t.device());
+    }
+  }
+  // the gradient as an operand
+  static Tensor rows(const Tensor& g) { return is_matrix(g) ? g : whole_units(g); }
+  std::string name() const override { return T::kName; }
+};
 
-struct LinearNode final : Products {
+struct LinearNode final : Product<LinearNode> {
+  static constexpr const char *kName = "LinearBackward", *kEntry = "llmctl_gemm_bf16";
+  static bool there() { return ready(lib.llmctl_gemm_bf16); }
   static Tensor record(const Tensor& x, const Tensor& w, int tile_n) {
-    auto node = new_node<LinearNode>(torch::autograd::collect_next_edges(x, w), tile_n);
+    auto node = make(torch::autograd::collect_next_edges(x, w), {tile_n, {}});
     node->keep({&x, &w});
     Tensor y = new_bf16(x, {x.size(0), w.size(0)});
     gemm(x, w, y, false, false, false, tile_n, 0);
     torch::autograd::set_history(y, node);
     return y;
   }
-  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
-    std::lock_guard<std::mutex> hold(mutex_);
-    if (!grads[0].defined()) return {Tensor(), Tensor()};
-    return node_body("llmctl_gemm_bf16", ready(lib.llmctl_gemm_bf16), [&]() -> torch::autograd::variable_list {
-      const Tensor x = operand(0), w = operand(1);
-      at::AutoDispatchBelowADInplaceOrView below;
-      const Tensor dy = rows(grads[0]);
-      Tensor dx, dw;
-      if (task_should_compute_output(0)) dx = dgrad(dy, w, tile_n);
-      if (task_should_compute_output(1)) dw = wgrad(dy, x, w, tile_n);
-      return {dx, dw};
-    });
+  static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
+    check(z, kept);
+    const Tensor &x = kept[0], &w = kept[1];
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor dy = rows(grad);
+    Tensor dx, dw;
+    if (wants & 1) dx = dgrad(dy, w, z.tile_n);
+    if (wants & 2) dw = wgrad(dy, x, w, z.tile_n);
+    return {dx, dw};
   }
-  std::string name() const override { return "LinearBackward"; }
 };
 
 // act = swiglu(x @ w.T) and the product before
@@ -417,35 +488,35 @@ std::pair<Tensor, Tensor> up_and_activate(const Tensor& x, const Tensor& w, bool
   return {act, gu};
 }
 
-struct LinearSwigluNode final : Products {
+struct LinearSwigluNode final : Product<LinearSwigluNode> {
+  static constexpr const char *kName = "LinearSwigluBackward", *kEntry = "llmctl_swiglu_bwd";
+  static bool there() { return ready(lib.llmctl_swiglu_bwd) && lib.llmctl_gemm_bf16; }
   static Tensor record(const Tensor& x, const Tensor& w) {
-    auto node = new_node<LinearSwigluNode>(torch::autograd::collect_next_edges(x, w), 0);
+    auto node = make(torch::autograd::collect_next_edges(x, w), {});
     const auto [act, gu] = up_and_activate(x, w, true);
     node->keep({&x, &w, &gu});
     torch::autograd::set_history(act, node);
     return act;
   }
-  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
-    std::lock_guard<std::mutex> hold(mutex_);
-    if (!grads[0].defined()) return {Tensor(), Tensor()};
-    return node_body("llmctl_swiglu_bwd", ready(lib.llmctl_swiglu_bwd) && lib.llmctl_gemm_bf16, [&]() -> torch::autograd::variable_list {
-      const Tensor x = operand(0), w = operand(1);
-      at::AutoDispatchBelowADInplaceOrView below;
-      const Tensor gu = whole_units(operand(2)), dact = whole_units(grads[0]);      // the kernel's one row stride is that of gu and of its gradient
-      Tensor dgu = new_bf16(gu, gu.sizes()), dx, dw;
-      done("llmctl_swiglu_bwd", lib.llmctl_swiglu_bwd(cdata(dact), cdata(gu), data(dgu), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2), gu.stride(0), ::stream()));
-      if (task_should_compute_output(0)) dx = dgrad(dgu, w, 0);
-      if (task_should_compute_output(1)) dw = wgrad(dgu, x, w, 0);
-      return {dx, dw};
-    });
+  static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
+    check(z, kept);
+    const Tensor &x = kept[0], &w = kept[1];
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor gu = whole_units(kept[2]), dact = whole_units(grad);           // the kernel's one row stride is that of gu and of its gradient
+    Tensor dgu = new_bf16(gu, gu.sizes()), dx, dw;
+    done("llmctl_swiglu_bwd", lib.llmctl_swiglu_bwd(cdata(dact), cdata(gu), data(dgu), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2), gu.stride(0), ::stream()));
+    if (wants & 1) dx = dgrad(dgu, w, 0);
+    if (wants & 2) dw = wgrad(dgu, x, w, 0);
+    return {dx, dw};
   }
-  std::string name() const override { return "LinearSwigluBackward"; }
 };
 
 // swiglu(x @ up.T) @ down.T: the gradient of the product of the two halves goes straight into theirs
-struct SwigluMlpNode final : Products {
+struct SwigluMlpNode final : Product<SwigluMlpNode> {
+  static constexpr const char *kName = "SwigluMlpBackward", *kEntry = "llmctl_gemm_swiglu_bwd_bf16";
+  static bool there() { return ready(lib.llmctl_gemm_swiglu_bwd_bf16) && lib.llmctl_gemm_bf16; }
   static Tensor record(const Tensor& x, const Tensor& up, const Tensor& down) {
-    auto node = new_node<SwigluMlpNode>(torch::autograd::collect_next_edges(x, up, down), 0);
+    auto node = make(torch::autograd::collect_next_edges(x, up, down), {});
     const auto [act, gu] = up_and_activate(x, up, true);
     node->keep({&x, &up, &down, &gu, &act});
     Tensor y = new_bf16(x, {x.size(0), down.size(0)});
@@ -453,27 +524,23 @@ struct SwigluMlpNode final : Products {
     torch::autograd::set_history(y, node);
     return y;
   }
-  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
-    std::lock_guard<std::mutex> hold(mutex_);
-    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
-    return node_body("llmctl_gemm_swiglu_bwd_bf16", ready(lib.llmctl_gemm_swiglu_bwd_bf16) && lib.llmctl_gemm_bf16, [&]() -> torch::autograd::variable_list {
-      const Tensor x = operand(0), up = operand(1), down = operand(2), act = operand(4);
-      at::AutoDispatchBelowADInplaceOrView below;
-      const Tensor gu = whole_units(operand(3)), dy = rows(grads[0]);               // the kernel's one row stride is that of gu and of its gradient
-      Tensor dgu, dx, d_up, d_down;
-      if (task_should_compute_output(0) || task_should_compute_output(1)) {
-        dgu = new_bf16(gu, gu.sizes());
-        done("llmctl_gemm_swiglu_bwd_bf16",
-             lib.llmctl_gemm_swiglu_bwd_bf16(cdata(dy), cdata(down), cdata(gu), data(dgu), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2),
-                                             static_cast<int>(dy.size(1)), dy.stride(0), down.stride(0), gu.stride(0), ::stream()));
-      }
-      if (task_should_compute_output(2)) d_down = wgrad(dy, act, down, 0);
-      if (task_should_compute_output(0)) dx = dgrad(dgu, up, 0);
-      if (task_should_compute_output(1)) d_up = wgrad(dgu, x, up, 0);
-      return {dx, d_up, d_down};
-    });
+  static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
+    check(z, kept);
+    const Tensor &x = kept[0], &up = kept[1], &down = kept[2], &act = kept[4];
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor gu = whole_units(kept[3]), dy = rows(grad);                    // the kernel's one row stride is that of gu and of its gradient
+    Tensor dgu, dx, d_up, d_down;
+    if (wants & 3) {
+      dgu = new_bf16(gu, gu.sizes());
+      done("llmctl_gemm_swiglu_bwd_bf16",
+           lib.llmctl_gemm_swiglu_bwd_bf16(cdata(dy), cdata(down), cdata(gu), data(dgu), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2),
+                                           static_cast<int>(dy.size(1)), dy.stride(0), down.stride(0), gu.stride(0), ::stream()));
+    }
+    if (wants & 4) d_down = wgrad(dy, act, down, 0);
+    if (wants & 1) dx = dgrad(dgu, up, 0);
+    if (wants & 2) d_up = wgrad(dgu, x, up, 0);
+    return {dx, d_up, d_down};
   }
-  std::string name() const override { return "SwigluMlpBackward"; }
 };
 
 // linear(x, w, tile_n, workspace or None) -> x @ w.T; where no gradient is recorded few rows take the decode GEMM, whose partials and tickets
@@ -596,44 +663,37 @@ Tensor attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor&
   return d;
 }
 
-// A node of its own: torch::autograd::Function looks its arguments up by name, and wraps and checks them in ways that this operator, which returns
-// one new tensor, has no use for (forward and backward of a small call 72 us; the engine alone takes 29).
-struct FlashAttention final : torch::autograd::Node {
-  torch::autograd::SavedVariable q, k, v, o, lse;
+struct AttentionNumbers {
   double scale = 0;
   bool causal = true;
-
+  void collect(compiled::CompiledNodeArgs& args) const {
+    args.collect(scale);
+    args.collect(causal);
+  }
+};
+struct FlashAttention final : Recorded<FlashAttention, AttentionNumbers> {
+  static constexpr const char* kEntry = "llmctl_flash_attn_bwd";
+  static bool there() { return ready(lib.llmctl_flash_attn_bwd); }
   static Tensor record(const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal) {
-    std::shared_ptr<FlashAttention> node(new FlashAttention(), torch::autograd::deleteNode);
-    node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
-    node->q = {q, false};
-    node->k = {k, false};
-    node->v = {v, false};
-    node->scale = scale;
-    node->causal = causal;
+    auto node = make(torch::autograd::collect_next_edges(q, k, v), {scale, causal});
+    node->saved.reserve(5);
+    for (const Tensor* t : {&q, &k, &v}) node->saved.emplace_back(*t, false);
     AttnOut r = attn_fwd(q, k, v, scale, causal, true);
     torch::autograd::set_history(r.o, node);
-    node->o = {r.o, true};
-    node->lse = {r.lse, false};
+    node->output = 3;
+    node->saved.emplace_back(r.o, true);
+    node->saved.emplace_back(r.lse, false);
     return r.o;
   }
-  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
-    std::lock_guard<std::mutex> hold(mutex_);
-    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
-    return node_body("llmctl_flash_attn_bwd", ready(lib.llmctl_flash_attn_bwd), [&]() -> torch::autograd::variable_list {
-      const auto self = getptr();
-      const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), o_ = o.unpack(self), lse_ = lse.unpack();
-      TORCH_CHECK(q_.is_cuda() && k_.is_cuda() && v_.is_cuda() && o_.is_cuda() && attention_ok(q_, k_, v_, causal) && bf16(o_) && o_.is_contiguous() && unit16(o_) && o_.sizes() == q_.sizes() && lse_.is_cuda() &&
-                      lse_.scalar_type() == at::kFloat && lse_.is_contiguous() && lse_.numel() == q_.size(0) * q_.size(1) * q_.size(2) && grads[0].sizes() == q_.sizes(),
-                  "FlashAttentionBackward: saved tensors came back in other forms");
-      at::AutoDispatchBelowADInplaceOrView below;
-      const Tensor d = attn_bwd(q_, k_, v_, o_, lse_, grads[0], scale, causal);
-      return {d.select(2, 0), d.select(2, 1), d.select(2, 2)};
-    });
-  }
-  void release_variables() override {
-    std::lock_guard<std::mutex> hold(mutex_);
-    for (auto* t : {&q, &k, &v, &o, &lse}) t->reset_data();
+  static torch::autograd::variable_list gradients(const AttentionNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned) {
+    const Tensor &q = kept[0], &k = kept[1], &v = kept[2], &o = kept[3], &lse = kept[4];
+    TORCH_CHECK(q.is_cuda() && k.is_cuda() && v.is_cuda() && o.is_cuda() && attention_ok(q, k, v, z.causal) && bf16(o) && o.is_contiguous() && unit16(o) &&
+                    o.sizes() == q.sizes() && lse.is_cuda() && lse.scalar_type() == at::kFloat && lse.is_contiguous() &&
+                    lse.numel() == q.size(0) * q.size(1) * q.size(2) && grad.sizes() == q.sizes(),
+                "FlashAttentionBackward: saved tensors came back in other forms");
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor d = attn_bwd(q, k, v, o, lse, grad, z.scale, z.causal);
+    return {d.select(2, 0), d.select(2, 1), d.select(2, 2)};
   }
   std::string name() const override { return "FlashAttentionBackward"; }
 };

@@ -348,6 +348,44 @@ def test_saved_rows_that_come_back_with_gaps_give_the_same_gradients(ops, extens
         _same(run(lambda t: torch.cat([t, t[:, :8]], 1)[:, :t.shape[1]]), run(lambda t: t))
 
 
+@pytest.mark.parametrize("wants", ["first", "others", "all"])
+@pytest.mark.parametrize("call", ["linear", "mlp", "two products", "attention", "rotated", "norm"])
+def test_compiled_autograd(ops, call, wants):
+    """A backward that is traced (and run as it was traced, for two lengths) makes the gradients that the engine makes."""
+    import torch._dynamo.compiled_autograd as compiled
+    from llmctl_b200.ops import attention as attn
+    cos, sin = (torch.randn(256, 32, device="cuda", generator=torch.Generator(device="cuda").manual_seed(i)) for i in range(2))
+
+    def run(rows, traced):
+        sizes = {"linear": [(rows, 64), (128, 64)], "mlp": [(rows, 64), (256, 64), (1024, 128)], "two products": [(rows, 64), (256, 64), (64, 128)],
+                 "attention": [(1, rows, 2, 64)] * 3, "rotated": [(rows, 64), (384, 64)], "norm": [(rows, 64), (64,)]}[call]
+        leaves = [_randn(*z, seed=i).requires_grad_(wants == "all" or (wants == "first") == (i == 0)) for i, z in enumerate(sizes)]
+        y = {"linear": ops.linear, "mlp": ops.swiglu_mlp, "two products": ops.swiglu_mlp, "attention": attn.attention, "norm": lambda x, w: ops.rmsnorm(x, w)[0],
+             "rotated": lambda x, w: attn.rope_attention_packed(ops.linear(x, w), cos, sin, 1, rows, 2, 64)}[call](*leaves)
+        with compiled._enable(lambda graph: torch.compile(graph, backend="eager")) if traced else contextlib.nullcontext():
+            y.backward(_randn(*y.shape, seed=7))
+        return [t.grad for t in leaves if t.requires_grad]
+    torch._dynamo.reset()
+    for rows in (40, 40, 130):
+        _same(run(rows, True), run(rows, False))
+
+
+def test_compiled_autograd_of_weights_with_gradient_buffers(ops):
+    """A traced backward leaves the gradient in the weight's buffer and tells its owner, as the engine's does."""
+    import torch._dynamo.compiled_autograd as compiled
+
+    def run(traced):
+        x, w, told = _randn(130, 64).requires_grad_(True), torch.nn.Parameter(_randn(64, 64, seed=1)), []
+        w.main_grad, w._main_grad_fresh, w._grad_ready_cb = torch.ones(w.shape, device="cuda"), False, lambda p: told.append(p is w)
+        y = ops.linear(x, w)
+        with compiled._enable(lambda graph: torch.compile(graph, backend="eager")) if traced else contextlib.nullcontext():
+            y.backward(_randn(130, 64, seed=4))
+        assert w.grad is None and told == [True]
+        return x.grad, w.main_grad
+    torch._dynamo.reset()
+    _same(run(True), run(False))
+
+
 def test_transforms_modes_and_subclasses_go_to_the_python_operators(ops):
     """What wants to see the operators or replace their tensors finds the Python ones, which record or refuse it as before."""
     from torch.utils._python_dispatch import TorchDispatchMode
