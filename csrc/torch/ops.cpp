@@ -313,7 +313,8 @@ Tensor as_shape_of(const Tensor& y, const Tensor& x) {
 }
 
 // dyT x of a weight; where the weight has a buffer for its gradient (main_grad, looked up now: it may come and go between the passes) through the
-// Python operator, which accumulates into it, and nothing is returned.
+// Python operator, which accumulates into it and tells its owner, and nothing is returned.  What the owner runs then is a program's own: no
+// dispatch key may be left out around it.
 Tensor wgrad(const Tensor& dy, const Tensor& x, const Tensor& w, int tile_n) {
   {
     pybind11::gil_scoped_acquire gil;
@@ -341,11 +342,13 @@ Tensor wgrad(const Tensor& dy, const Tensor& x, const Tensor& w, int tile_n) {
       return out;
     }
   }
+  at::AutoDispatchBelowADInplaceOrView below;
   Tensor dw = new_bf16(w, w.sizes());
   gemm(dy, x, dw, true, true, false, tile_n, 0);
   return dw;
 }
 Tensor dgrad(const Tensor& dy, const Tensor& w, int tile_n) {
+  at::AutoDispatchBelowADInplaceOrView below;
   Tensor dx = new_bf16(dy, {dy.size(0), w.size(1)});
   gemm(dy, w, dx, false, true, false, tile_n, 0);
   return dx;
@@ -386,9 +389,13 @@ struct Recorded : torch::autograd::Node {
   }
 
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
-    std::lock_guard<std::mutex> hold(mutex_);
     if (!grads[0].defined()) return torch::autograd::variable_list(num_outputs());
-    return run(numbers, grads[0], kept(), wants());
+    torch::autograd::variable_list ts;
+    {
+      std::lock_guard<std::mutex> hold(mutex_);
+      ts = kept();
+    }
+    return run(numbers, grads[0], ts, wants());
   }
   void release_variables() override {
     std::lock_guard<std::mutex> hold(mutex_);
@@ -452,7 +459,10 @@ struct Product : Recorded<T, ProductNumbers> {
     }
   }
   // the gradient as an operand
-  static Tensor rows(const Tensor& g) { return is_matrix(g) ? g : whole_units(g); }
+  static Tensor rows(const Tensor& g) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return is_matrix(g) ? g : whole_units(g);
+  }
   std::string name() const override { return T::kName; }
 };
 
@@ -469,9 +479,7 @@ struct LinearNode final : Product<LinearNode> {
   }
   static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
     check(z, kept);
-    const Tensor &x = kept[0], &w = kept[1];
-    at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor dy = rows(grad);
+    const Tensor &x = kept[0], &w = kept[1], dy = rows(grad);
     Tensor dx, dw;
     if (wants & 1) dx = dgrad(dy, w, z.tile_n);
     if (wants & 2) dw = wgrad(dy, x, w, z.tile_n);
@@ -500,11 +508,14 @@ struct LinearSwigluNode final : Product<LinearSwigluNode> {
   }
   static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
     check(z, kept);
-    const Tensor &x = kept[0], &w = kept[1];
-    at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor gu = whole_units(kept[2]), dact = whole_units(grad);           // the kernel's one row stride is that of gu and of its gradient
-    Tensor dgu = new_bf16(gu, gu.sizes()), dx, dw;
-    done("llmctl_swiglu_bwd", lib.llmctl_swiglu_bwd(cdata(dact), cdata(gu), data(dgu), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2), gu.stride(0), ::stream()));
+    const Tensor &x = kept[0], &w = kept[1], dgu = [&] {
+      at::AutoDispatchBelowADInplaceOrView below;
+      const Tensor gu = whole_units(kept[2]), dact = whole_units(grad);         // the kernel's one row stride is that of gu and of its gradient
+      Tensor d = new_bf16(gu, gu.sizes());
+      done("llmctl_swiglu_bwd", lib.llmctl_swiglu_bwd(cdata(dact), cdata(gu), data(d), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2), gu.stride(0), ::stream()));
+      return d;
+    }();
+    Tensor dx, dw;
     if (wants & 1) dx = dgrad(dgu, w, 0);
     if (wants & 2) dw = wgrad(dgu, x, w, 0);
     return {dx, dw};
@@ -526,11 +537,11 @@ struct SwigluMlpNode final : Product<SwigluMlpNode> {
   }
   static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
     check(z, kept);
-    const Tensor &x = kept[0], &up = kept[1], &down = kept[2], &act = kept[4];
-    at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor gu = whole_units(kept[3]), dy = rows(grad);                    // the kernel's one row stride is that of gu and of its gradient
+    const Tensor &x = kept[0], &up = kept[1], &down = kept[2], &act = kept[4], dy = rows(grad);
     Tensor dgu, dx, d_up, d_down;
     if (wants & 3) {
+      at::AutoDispatchBelowADInplaceOrView below;
+      const Tensor gu = whole_units(kept[3]);                                   // the kernel's one row stride is that of gu and of its gradient
       dgu = new_bf16(gu, gu.sizes());
       done("llmctl_gemm_swiglu_bwd_bf16",
            lib.llmctl_gemm_swiglu_bwd_bf16(cdata(dy), cdata(down), cdata(gu), data(dgu), static_cast<int>(gu.size(0)), static_cast<int>(gu.size(1) / 2),

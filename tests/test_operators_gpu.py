@@ -716,6 +716,24 @@ def test_weights_with_gradient_buffers(ops):
     _both(run)
 
 
+@pytest.mark.parametrize("call", ["linear", "mlp", "two products"])
+def test_owners_of_gradient_buffers_run_as_anywhere(ops, call):
+    """What is told of a finished gradient may update tensors in place, which their versions show, and record a graph."""
+    leaves = [torch.nn.Parameter(_randn(*z, seed=i)) for i, z in enumerate([(130, 64), (256, 64), (64 if call == "two products" else 1024, 128)])]
+    seen = []
+
+    def told(p):
+        t, before = torch.zeros(1, device="cuda"), torch.zeros(1, device="cuda", requires_grad=True)
+        t.add_(1)
+        with torch.enable_grad():
+            seen.append((t._version, (before * 2).requires_grad))
+    for w in leaves[1:]:
+        w.main_grad, w._grad_ready_cb = torch.zeros(w.shape, device="cuda"), told
+    y = ops.linear(*leaves[:2]) if call == "linear" else ops.swiglu_mlp(*leaves)
+    y.backward(_randn(*y.shape, seed=4))
+    assert seen == [(1, True)] * (1 if call == "linear" else 2)
+
+
 @pytest.mark.parametrize("B,S,heads,dim", [(1, 33, 2, 64), (2, 130, 2, 128), (1, 600, 12, 64)])
 @pytest.mark.parametrize("form", ["plain", "first", "positions", "hook", "few"])
 def test_block_without_gradients(ops, B, S, heads, dim, form):
