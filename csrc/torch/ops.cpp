@@ -213,6 +213,12 @@ NormOut norm_fwd(const Tensor& x, const Tensor& residual, const Tensor& w, doubl
 
 constexpr int kNormBwdCtas = 148 * 4;
 
+// A hook on saved tensors may give back anything: what has another type, size or device than what was kept is refused before a kernel reads it as that.
+void came_back(const char* node, const Tensor& t, at::ScalarType type, at::IntArrayRef sizes, const Tensor& grad) {
+  TORCH_CHECK(t.scalar_type() == type && t.sizes() == sizes && t.device() == grad.device() && is_plain(t), node, ": a saved tensor came back as ", t.scalar_type(),
+              " of sizes ", t.sizes(), " on ", t.device());
+}
+
 // y = rmsnorm(x + residual) * w, and h = x + residual where there is a residual.
 struct RmsNorm : torch::autograd::Function<RmsNorm> {
   static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& residual, const Tensor& w,
@@ -226,9 +232,12 @@ struct RmsNorm : torch::autograd::Function<RmsNorm> {
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     return node_body("llmctl_rmsnorm_bwd_bf16w", ready(lib.llmctl_rmsnorm_bwd_bf16w), [&]() -> torch::autograd::variable_list {
       const auto saved = ctx->get_saved_variables();
-      const Tensor h = whole_units(saved[0]), w = whole_units(saved[1]), &rstd = saved[2];
+      const int64_t cols = grads[0].size(-1), rows = grads[0].numel() / cols;
+      came_back("RmsNormBackward", saved[0], at::kBFloat16, grads[0].sizes(), grads[0]);
+      came_back("RmsNormBackward", saved[1], at::kBFloat16, {cols}, grads[0]);
+      came_back("RmsNormBackward", saved[2], at::kFloat, {rows}, grads[0]);
+      const Tensor h = whole_units(saved[0]), w = whole_units(saved[1]), rstd = whole_units(saved[2]);
       const bool residual = ctx->saved_data["residual"].toBool();
-      const int64_t cols = h.size(-1), rows = h.numel() / cols;
       const Tensor dy = whole_units(grads[0]), dres = residual ? whole_units(grads[1]) : Tensor();
       Tensor dx = new_bf16(h, h.sizes()), dw = new_bf16(w, {cols});
       const int ctas = static_cast<int>(rows < kNormBwdCtas ? rows : kNormBwdCtas);
@@ -451,10 +460,10 @@ struct Product : Recorded<T, ProductNumbers> {
     }
   }
   // a hook on saved tensors may give back anything: what the kernels cannot read is refused
-  static void check(const ProductNumbers& numbers, const torch::autograd::variable_list& kept) {
+  static void check(const ProductNumbers& numbers, const torch::autograd::variable_list& kept, const Tensor& grad) {
     for (size_t i = 0; i < kept.size(); ++i) {
       const Tensor& t = kept[i];
-      TORCH_CHECK(t.is_cuda() && is_matrix(t) && t.size(0) == numbers.sizes[i][0] && t.size(1) == numbers.sizes[i][1], T::kName, ": a saved matrix came back as ",
+      TORCH_CHECK(t.device() == grad.device() && is_matrix(t) && t.size(0) == numbers.sizes[i][0] && t.size(1) == numbers.sizes[i][1], T::kName, ": a saved matrix came back as ",
                   t.scalar_type(), " of sizes ", t.sizes(), " on ", t.device());
     }
   }
@@ -478,7 +487,7 @@ struct LinearNode final : Product<LinearNode> {
     return y;
   }
   static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
-    check(z, kept);
+    check(z, kept, grad);
     const Tensor &x = kept[0], &w = kept[1], dy = rows(grad);
     Tensor dx, dw;
     if (wants & 1) dx = dgrad(dy, w, z.tile_n);
@@ -507,7 +516,7 @@ struct LinearSwigluNode final : Product<LinearSwigluNode> {
     return act;
   }
   static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
-    check(z, kept);
+    check(z, kept, grad);
     const Tensor &x = kept[0], &w = kept[1], dgu = [&] {
       at::AutoDispatchBelowADInplaceOrView below;
       const Tensor gu = whole_units(kept[2]), dact = whole_units(grad);         // the kernel's one row stride is that of gu and of its gradient
@@ -536,7 +545,7 @@ struct SwigluMlpNode final : Product<SwigluMlpNode> {
     return y;
   }
   static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
-    check(z, kept);
+    check(z, kept, grad);
     const Tensor &x = kept[0], &up = kept[1], &down = kept[2], &act = kept[4], dy = rows(grad);
     Tensor dgu, dx, d_up, d_down;
     if (wants & 3) {
@@ -698,8 +707,9 @@ struct FlashAttention final : Recorded<FlashAttention, AttentionNumbers> {
   }
   static torch::autograd::variable_list gradients(const AttentionNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned) {
     const Tensor &q = kept[0], &k = kept[1], &v = kept[2], &o = kept[3], &lse = kept[4];
-    TORCH_CHECK(q.is_cuda() && k.is_cuda() && v.is_cuda() && o.is_cuda() && attention_ok(q, k, v, z.causal) && bf16(o) && o.is_contiguous() && unit16(o) &&
-                    o.sizes() == q.sizes() && lse.is_cuda() && lse.scalar_type() == at::kFloat && lse.is_contiguous() &&
+    const auto here = grad.device();
+    TORCH_CHECK(q.device() == here && k.device() == here && v.device() == here && o.device() == here && attention_ok(q, k, v, z.causal) && bf16(o) &&
+                    o.is_contiguous() && unit16(o) && o.sizes() == q.sizes() && lse.device() == here && lse.scalar_type() == at::kFloat && lse.is_contiguous() &&
                     lse.numel() == q.size(0) * q.size(1) * q.size(2) && grad.sizes() == q.sizes(),
                 "FlashAttentionBackward: saved tensors came back in other forms");
     at::AutoDispatchBelowADInplaceOrView below;
@@ -745,6 +755,7 @@ struct RopeAttention : torch::autograd::Function<RopeAttention> {
     AttnOut r = attn_fwd(p.q, p.k, p.v, scale, true, true);
     ctx->save_for_backward({qkv.detach(), r.o, r.lse, cos, sin, positions.value_or(Tensor())});
     ctx->saved_data["sizes"] = std::vector<int64_t>{B, S, H, D};
+    ctx->saved_data["tables"] = std::vector<int64_t>{cos.numel(), sin.numel()};
     ctx->saved_data["scale"] = scale;
     return r.o.view({B * S, H * D});
   }
@@ -753,9 +764,22 @@ struct RopeAttention : torch::autograd::Function<RopeAttention> {
       const auto s = ctx->get_saved_variables();
       const auto z = ctx->saved_data["sizes"].toIntVector();
       const int64_t B = z[0], S = z[1], H = z[2], D = z[3];
-      const Packed p = unpack(s[0], B, S, H, D);
-      const Tensor d = attn_bwd(p.q, p.k, p.v, s[1], s[2], grads[0].reshape({B, S, H, D}), ctx->saved_data["scale"].toDouble(), true).view({B * S, 3 * H * D});
-      rope(d, s[3], s[4], s[5], S, 2 * H, D, -1.f);
+      const char* node = "RopeAttentionBackward";
+      came_back(node, s[0], at::kBFloat16, {B * S, 3 * H * D}, grads[0]);
+      came_back(node, s[1], at::kBFloat16, {B, S, H, D}, grads[0]);
+      came_back(node, s[2], at::kFloat, {B, H, S}, grads[0]);
+      const auto tables = ctx->saved_data["tables"].toIntVector();
+      for (int i = 0; i < 2; ++i) {
+        came_back(node, s[3 + i], at::kFloat, s[3 + i].sizes(), grads[0]);
+        TORCH_CHECK(s[3 + i].numel() == tables[i], node, ": a table came back with ", s[3 + i].numel(), " numbers");
+      }
+      if (s[5].defined()) {
+        came_back(node, s[5], at::kInt, s[5].sizes(), grads[0]);
+        TORCH_CHECK(s[5].numel() == B * S, node, ": ", s[5].numel(), " positions came back");
+      }
+      const Packed p = unpack(whole_units(s[0]), B, S, H, D);
+      const Tensor d = attn_bwd(p.q, p.k, p.v, whole_units(s[1]), whole_units(s[2]), grads[0].reshape({B, S, H, D}), ctx->saved_data["scale"].toDouble(), true).view({B * S, 3 * H * D});
+      rope(d, whole_units(s[3]), whole_units(s[4]), s[5].defined() ? whole_units(s[5]) : s[5], S, 2 * H, D, -1.f);
       return {d, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     });
   }

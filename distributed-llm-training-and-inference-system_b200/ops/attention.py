@@ -46,8 +46,10 @@ def _native_shape(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: boo
 
 def _native_ok(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = True) -> bool:
     """The kernels read these views where they lie: heads side by side in a token, whole 16-byte units, sequences back to back."""
-    if not (_native_built(q) and _native_shape(q, k, v, causal)):
-        return False
+    return _native_built(q) and _native_shape(q, k, v, causal) and _native_layout(q, k, v)
+
+
+def _native_layout(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
     B, S, H, D = q.shape
     for t in (q, k, v):
         if (t.dtype != q.dtype or t.stride(3) != 1 or t.stride(2) != D or (B > 1 and t.stride(0) != S * t.stride(1))
@@ -70,16 +72,18 @@ class _FlashAttnFn(torch.autograd.Function):
         native.call("llmctl_flash_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
                     B, S, H, D, q.stride(1), k.stride(1), v.stride(1), o.stride(1), float(scale), int(causal),
                     native.stream_ptr())
-        ctx.save_for_backward(q, k, v, o, lse)
+        native.keep(ctx, q, k, v, o, lse)
         ctx.scale, ctx.causal = scale, causal
         return o
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v, o, lse = ctx.saved_tensors
+        q, k, v, o, lse = native.kept(ctx)
         if native.has_symbol("llmctl_flash_attn_bwd"):
             B, S, H, D = q.shape
-            do = _whole_units(do)
+            if not _native_layout(q, k, v):
+                q, k, v = (t.clone(memory_format=torch.contiguous_format) for t in (q, k, v))
+            o, lse, do = _whole_units(o), _whole_units(lse), _whole_units(do)
             # dq|dk|dv packed like the forward's qkv so the following wgrad GEMM sees one tensor
             dqkv = torch.empty(B, S, 3, H, D, dtype=q.dtype, device=q.device)
             dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
@@ -183,12 +187,12 @@ class _RopeAttnPackedFn(torch.autograd.Function):
                         B, S, H, D, q.stride(1), k.stride(1), v.stride(1), o.stride(1), float(scale), 1,
                         native.stream_ptr())
             ctx.lib_saved = None
-            ctx.save_for_backward(qkv.detach(), o, lse, cos, sin, positions if positions is not None else torch.empty(0))
+            native.keep(ctx, qkv.detach(), o, lse, cos, sin, positions if positions is not None else torch.empty(0))
             out = o
         else:
             o_bhsd, saved = _lib_attention_fwd(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), scale, True)
             ctx.lib_saved = (saved[0],) + tuple(x for x in saved[1:])
-            ctx.save_for_backward(qkv.detach(), o_bhsd, saved[1], cos, sin,
+            native.keep(ctx, qkv.detach(), o_bhsd, saved[1], cos, sin,
                                   positions if positions is not None else torch.empty(0))
             out = o_bhsd.transpose(1, 2)
         ctx.meta = (B, S, H, D, positions is not None, scale, use_native)
@@ -196,16 +200,19 @@ class _RopeAttnPackedFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, do):
-        qkv, o, lse, cos, sin, positions = ctx.saved_tensors
+        qkv, o, lse, cos, sin, positions = native.kept(ctx)
         B, S, H, D, has_pos, scale, use_native = ctx.meta
         T = B * S
+        if qkv.stride(1) != 1 or qkv.stride(0) % 8 or qkv.data_ptr() % 16:
+            qkv = _whole_units(qkv)
+        cos, sin, positions = _whole_units(cos), _whole_units(sin), _whole_units(positions)
         v5 = qkv.view(B, S, 3, H, D)
         q, k, v = v5[:, :, 0], v5[:, :, 1], v5[:, :, 2]
         dqkv = torch.empty(T, 3 * H * D, dtype=qkv.dtype, device=qkv.device)
         d5 = dqkv.view(B, S, 3, H, D)
         do4 = do.reshape(B, S, H, D)
         if use_native and native.has_symbol("llmctl_flash_attn_bwd"):
-            do4 = _whole_units(do4)
+            o, lse, do4 = _whole_units(o), _whole_units(lse), _whole_units(do4)
             scratch = _stats_scratch(B, S, H, qkv.device)
             native.call("llmctl_flash_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do4.data_ptr(),
                         lse.data_ptr(), d5[:, :, 0].data_ptr(), d5[:, :, 1].data_ptr(), d5[:, :, 2].data_ptr(),

@@ -110,7 +110,7 @@ class _RMSNormFn(torch.autograd.Function):
         native.call("llmctl_rmsnorm_fwd", x2.data_ptr(), native.ptr(r2), w.data_ptr(),
                     h.data_ptr() if r2 is not None else None, y.data_ptr(), rstd.data_ptr(),
                     rows, cols, float(eps), native.stream_ptr())
-        ctx.save_for_backward(h, w, rstd)
+        native.keep(ctx, h, w, rstd)
         ctx.has_res = residual is not None
         ctx.shape = shape
         if residual is None:
@@ -121,7 +121,7 @@ class _RMSNormFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy, dh):
-        h, w, rstd = ctx.saved_tensors
+        h, w, rstd = (_whole_units(t) for t in native.kept(ctx))
         rows, cols = h.shape
         dy2 = _whole_units(dy.reshape(rows, cols))
         dres = _whole_units(dh.reshape(rows, cols)) if dh is not None and ctx.has_res else None
@@ -169,7 +169,7 @@ class _LayerNormFn(torch.autograd.Function):
         native.call("llmctl_layernorm_fwd", x2.data_ptr(), native.ptr(r2), w.data_ptr(), native.ptr(b2),
                     h.data_ptr() if r2 is not None else None, y.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
                     rows, cols, float(eps), native.stream_ptr())
-        ctx.save_for_backward(h, w, mean, rstd)
+        native.keep(ctx, h, w, mean, rstd)
         ctx.has_res, ctx.has_bias, ctx.shape = residual is not None, b is not None, shape
         if residual is None:
             h_ret = y.new_empty(0)
@@ -179,7 +179,7 @@ class _LayerNormFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy, dh):
-        h, w, mean, rstd = ctx.saved_tensors
+        h, w, mean, rstd = (_whole_units(t) for t in native.kept(ctx))
         rows, cols = h.shape
         dy2 = _whole_units(dy.reshape(rows, cols))
         dres = _whole_units(dh.reshape(rows, cols)) if (dh is not None and ctx.has_res) else None
@@ -244,13 +244,13 @@ class _RopeFn(torch.autograd.Function):
         native.call("llmctl_rope_inplace", x.data_ptr(), x.stride(0), x.shape[0], n_rot_heads, head_dim,
                     cos.data_ptr(), sin.data_ptr(), native.ptr(positions), seq_len, 1.0, native.stream_ptr())
         ctx.mark_dirty(x)
-        ctx.save_for_backward(cos, sin, positions if positions is not None else torch.empty(0))
+        native.keep(ctx, cos, sin, positions if positions is not None else torch.empty(0))
         ctx.meta = (n_rot_heads, head_dim, seq_len, positions is not None)
         return x
 
     @staticmethod
     def backward(ctx, dout):
-        cos, sin, positions = ctx.saved_tensors
+        cos, sin, positions = (_whole_units(t) for t in native.kept(ctx))
         n_rot, hd, seq_len, has_pos = ctx.meta
         dx = dout.clone(memory_format=torch.contiguous_format)   # never rotate a possibly shared grad in place
         native.call("llmctl_rope_inplace", dx.data_ptr(), dx.stride(0), dx.shape[0], n_rot, hd,
@@ -277,6 +277,11 @@ def rope_packed(x: torch.Tensor, cos, sin, n_rot_heads: int, head_dim: int, seq_
 # ------------------------------------------------------------------------------------------------
 # SwiGLU (K5)
 # ------------------------------------------------------------------------------------------------
+def _gate_up_rows(gu: torch.Tensor) -> torch.Tensor:
+    """``gu`` where it lies if its rows are whole 16-byte units, else a copy."""
+    return gu if gu.stride(1) == 1 and gu.stride(0) % 8 == 0 and gu.data_ptr() % 16 == 0 else _whole_units(gu)
+
+
 class _SwiGLUFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gu):
@@ -284,12 +289,12 @@ class _SwiGLUFn(torch.autograd.Function):
         Fd = F2 // 2
         out = torch.empty(M, Fd, dtype=gu.dtype, device=gu.device)
         native.call("llmctl_swiglu_fwd", gu.data_ptr(), out.data_ptr(), M, Fd, gu.stride(0), native.stream_ptr())
-        ctx.save_for_backward(gu)
+        native.keep(ctx, gu)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        (gu,) = ctx.saved_tensors
+        gu = _gate_up_rows(*native.kept(ctx))
         M, F2 = gu.shape
         dout = _whole_units(dout)
         dgu = torch.empty_strided(gu.shape, gu.stride(), dtype=gu.dtype, device=gu.device)      # the kernel's one row stride is that of both
@@ -303,9 +308,7 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     if _use_native(gate_up, "elementwise") and gate_up.shape[-1] % 16 == 0:
         shape = gate_up.shape
         g2 = gate_up.reshape(-1, shape[-1])
-        if g2.stride(1) != 1 or g2.stride(0) % 8 or g2.data_ptr() % 16:
-            g2 = _whole_units(g2)
-        return native.apply(_SwiGLUFn, g2).view(*shape[:-1], shape[-1] // 2)
+        return native.apply(_SwiGLUFn, _gate_up_rows(g2)).view(*shape[:-1], shape[-1] // 2)
     g, u = gate_up.chunk(2, dim=-1)
     return (F.silu(g.float()) * u.float()).to(gate_up.dtype)
 
@@ -375,12 +378,12 @@ class _LinearFn(torch.autograd.Function):
             gate["after"]()
         else:
             y = gemm_raw(x, w)
-        ctx.save_for_backward(x, w)
+        native.keep(ctx, x, w)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, w = ctx.saved_tensors
+        x, w = native.kept(ctx)
         if not _gemm_ok(dy):
             dy = _whole_units(dy)
         dx = dw = None
@@ -519,12 +522,12 @@ class _LinearSwiGLUFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w):
         act, gu = _gemm_swiglu(x, w, any(ctx.needs_input_grad))
-        ctx.save_for_backward(x, w, gu)
+        native.keep(ctx, x, w, gu)
         return act
 
     @staticmethod
     def backward(ctx, dact):
-        x, w, gu = ctx.saved_tensors
+        x, w, gu = native.kept(ctx)
         M, F2 = gu.shape
         gu, dact = _whole_units(gu), _whole_units(dact)         # a hook on saved tensors may give back rows with gaps
         dgu = torch.empty_like(gu)                              # the kernel's one row stride is that of both
@@ -546,12 +549,12 @@ class _SwiGLUMLPFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w_up, w_down):
         act, gu = _gemm_swiglu(x, w_up, True)
-        ctx.save_for_backward(x, w_up, w_down, gu, act)
+        native.keep(ctx, x, w_up, w_down, gu, act)
         return gemm_raw(act, w_down)
 
     @staticmethod
     def backward(ctx, dy):
-        x, w_up, w_down, gu, act = ctx.saved_tensors
+        x, w_up, w_down, gu, act = native.kept(ctx)
         if not _gemm_ok(dy):
             dy = _whole_units(dy)
         dx = dw_up = dgu = None
@@ -629,12 +632,13 @@ class _SwiGLULinearFn(torch.autograd.Function):
         act = torch.empty(M, F2 // 2, dtype=gu.dtype, device=gu.device)
         native.call("llmctl_swiglu_fwd", gu.data_ptr(), act.data_ptr(), M, F2 // 2, gu.stride(0), native.stream_ptr())
         y = gemm_raw(act, w)
-        ctx.save_for_backward(gu, w)
+        native.keep(ctx, gu, w)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        gu, w = ctx.saved_tensors
+        gu, w = native.kept(ctx)
+        gu = _gate_up_rows(gu)
         M, F2 = gu.shape
         if not _gemm_ok(dy):
             dy = _whole_units(dy)

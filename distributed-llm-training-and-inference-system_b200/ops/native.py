@@ -227,6 +227,22 @@ def apply(fn, *args):
     return fn.forward(_NoContext(), *args)
 
 
+def keep(ctx, *tensors) -> None:
+    """``ctx.save_for_backward`` of tensors that a backward will hand to a kernel (``kept``)."""
+    ctx.save_for_backward(*tensors)
+    ctx.kept_as = tuple(None if t is None else (t.shape, t.dtype, t.device) for t in tensors)
+
+
+def kept(ctx):
+    """``ctx.saved_tensors``.  A hook on saved tensors may give back anything: what has another size, type or device than what was kept is
+    refused before a kernel reads it as that."""
+    tensors = ctx.saved_tensors
+    for t, form in zip(tensors, ctx.kept_as):
+        if form is not None and (t.shape, t.dtype, t.device) != form:
+            raise RuntimeError(f"a saved tensor came back as {t.dtype} of sizes {list(t.shape)} on {t.device}")
+    return tensors
+
+
 class NativeError(RuntimeError):
     pass
 

@@ -334,6 +334,39 @@ def test_saved_tensors_that_come_back_in_other_forms_are_refused(ops, form, call
     torch.cuda.synchronize()
 
 
+@pytest.mark.parametrize("form", ["fp32", "cpu", "part", "gaps", "reversed"])
+@pytest.mark.parametrize("call", ["norm", "sum and norm", "layer norm", "rotated attention", "rotated attention at positions", "rotation", "gated"])
+@pytest.mark.parametrize("extension", [True, False])
+def test_saved_tensors_of_norms_and_rotations(ops, extension, call, form):
+    """Other types, devices and sizes are an error before any launch, other layouts are copied: the same gradients."""
+    from llmctl_b200.ops import attention as attn
+    cos, sin = (torch.rand(256, 32, device="cuda", generator=torch.Generator(device="cuda").manual_seed(i)) for i in range(2))
+    at = torch.arange(130, device="cuda", dtype=torch.int32) + 5
+
+    def spread(t):            # a copy whose numbers lie two apart, or in the other order of the dimensions
+        if form == "gaps":
+            return torch.stack([t, t], -1)[..., 0]
+        return t.permute(*reversed(range(t.dim()))).contiguous().permute(*reversed(range(t.dim())))
+
+    def run(unpack):
+        x, r, w, b = (_randn(*z, seed=i).requires_grad_(True) for i, z in enumerate([(130, 384), (130, 384), (384,), (384,)]))
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            y = {"norm": lambda: ops.rmsnorm(x, w)[0], "sum and norm": lambda: ops.rmsnorm(x, w, residual=r)[0], "layer norm": lambda: ops.layernorm(x, w, b)[0],
+                 "rotated attention": lambda: attn.rope_attention_packed(x * 1, cos, sin, 1, 130, 2, 64),
+                 "rotated attention at positions": lambda: attn.rope_attention_packed(x * 1, cos, sin, 1, 130, 2, 64, at),
+                 "rotation": lambda: ops.rope_packed(x * 1, cos, sin, 4, 64, 130), "gated": lambda: ops.swiglu(x)}[call]()
+        y.backward(_randn(*y.shape, seed=9))
+        return [t.grad for t in (x, r, w, b) if t.grad is not None]
+    with contextlib.nullcontext() if extension else python_operators():
+        if form in ("gaps", "reversed"):
+            _same(run(spread), run(lambda t: t))
+        else:
+            other = {"fp32": lambda t: t.double() if t.dtype == torch.float32 else t.float(), "cpu": torch.Tensor.cpu, "part": lambda t: t[:-1]}[form]
+            with pytest.raises(RuntimeError):
+                run(lambda t: other(t) if t.is_cuda and t.is_floating_point() else t)
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("extension", [True, False])
 @pytest.mark.parametrize("call", ["linear", "mlp", "two products"])
 def test_saved_rows_that_come_back_with_gaps_give_the_same_gradients(ops, extension, call):

@@ -1,5 +1,6 @@
 """Unit tests the reference never had: planner, config schemas, health thresholds, autotuner,
 plugin registry, checkpoint GC, LR schedule, export re-sharding, roofline."""
+import contextlib
 import json
 import math
 import time
@@ -668,10 +669,47 @@ def test_gated_backwards_write_within_their_gradient(monkeypatch, node):
     monkeypatch.setattr(native, "call", lambda name, *a: stride.update(gate_up=a[5] if name == "llmctl_swiglu_bwd" else a[9]))
     monkeypatch.setattr(ops, "gemm_raw", lambda a, b, **k: operands.append(a))
     monkeypatch.setattr(ops, "_wgrad", lambda *a: None)
-    ctx = SimpleNamespace(needs_input_grad=[True] * 3, saved_tensors=(x, up, gu) if node == "_LinearSwiGLUFn" else (x, up, down, gu, act))
+    saved = (x, up, gu) if node == "_LinearSwiGLUFn" else (x, up, down, gu, act)
+    ctx = SimpleNamespace(needs_input_grad=[True] * 3, saved_tensors=saved, kept_as=tuple((t.shape, t.dtype, t.device) for t in saved))
     getattr(ops, node).backward(ctx, act if node == "_LinearSwiGLUFn" else torch.zeros(rows, cols, dtype=torch.bfloat16))
     (dgu,) = operands
     assert dgu.stride(0) == stride["gate_up"] and dgu.untyped_storage().nbytes() >= 2 * ((rows - 1) * stride["gate_up"] + 2 * width)
+
+
+@pytest.mark.parametrize("form", ["wider", "part", "as it was"])
+@pytest.mark.parametrize("call", ["rmsnorm", "rmsnorm and sum", "layernorm", "rotation", "swiglu", "swiglu and product", "product", "product and swiglu", "mlp",
+                                  "attention", "rotation and attention"])
+def test_backwards_refuse_saved_tensors_of_other_forms(monkeypatch, call, form):
+    """What a hook on saved tensors gives back is looked at before any kernel is called: its address says nothing of its type and size."""
+    from llmctl_b200.ops import attention as attn
+    from llmctl_b200.ops import functional as ops
+    from llmctl_b200.ops import native
+    calls = []
+    monkeypatch.setattr(native, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(native, "has_symbol", lambda name: True)
+    monkeypatch.setattr(native, "call", lambda name, *a: calls.append(name))
+    monkeypatch.setattr(ops, "_scratch", lambda device, n, name: torch.zeros(n))
+
+    def product(a, b, *, a_mn=False, b_mn=False, **k):
+        calls.append("product")
+        return torch.zeros(a.shape[int(a_mn)], b.shape[int(b_mn)], dtype=a.dtype)
+    monkeypatch.setattr(ops, "gemm_raw", product)
+    z = lambda *s: torch.zeros(*s, dtype=torch.bfloat16, requires_grad=True)                # noqa: E731
+    table = torch.zeros(8, 32)
+    run = {"rmsnorm": lambda: ops._RMSNormFn.apply(z(6, 16), None, z(16), 1e-5)[0], "rmsnorm and sum": lambda: ops._RMSNormFn.apply(z(6, 16), z(6, 16), z(16), 1e-5)[0],
+           "layernorm": lambda: ops._LayerNormFn.apply(z(6, 16), None, z(16), z(16), 1e-5)[0],
+           "rotation": lambda: ops._RopeFn.apply(z(6, 128) * 1, table, table, 2, 64, 6, None), "swiglu": lambda: ops._SwiGLUFn.apply(z(6, 32)),
+           "swiglu and product": lambda: ops._SwiGLULinearFn.apply(z(6, 32), z(8, 16)), "product": lambda: ops._LinearFn.apply(z(6, 16), z(8, 16)),
+           "product and swiglu": lambda: ops._LinearSwiGLUFn.apply(z(6, 16), z(32, 16)), "mlp": lambda: ops._SwiGLUMLPFn.apply(z(6, 16), z(32, 16), z(8, 16)),
+           "attention": lambda: attn._FlashAttnFn.apply(z(2, 6, 1, 64), z(2, 6, 1, 64), z(2, 6, 1, 64), 1.0, True),
+           "rotation and attention": lambda: attn._RopeAttnPackedFn.apply(z(6, 192) * 1, table, table, 1, 6, 1, 64, None, 1.0, True)}[call]
+    unpack = {"wider": torch.Tensor.double, "part": lambda t: t[:-1], "as it was": lambda t: t}[form]
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        y = run()
+    calls.clear()
+    with contextlib.nullcontext() if form == "as it was" else pytest.raises(RuntimeError, match="came back"):
+        y.backward(torch.zeros_like(y))
+    assert bool(calls) == (form == "as it was")
 
 
 def test_division_by_a_launch_constant(tmp_path):
