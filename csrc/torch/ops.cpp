@@ -837,20 +837,29 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
         gemm(in, w, to, false, false, false, tile_n, 0);
         return to;
       };
-      const NormOut first = norm_fwd(x, residual, n1, eps, false);
-      Tensor p;
-      if (D == 64 && lib.llmctl_gemm_rope_bf16 && unit16(cos) && unit16(sin)) {
-        p = new_bf16(x, {T, 3 * H * D});
-        done("llmctl_gemm_rope_bf16",
-             lib.llmctl_gemm_rope_bf16(cdata(first.y), cdata(qkv), data(p), static_cast<int>(T), static_cast<int>(3 * H * D), static_cast<int>(W), W, qkv.stride(0), 3 * H * D,
-                                       static_cast<const float*>(cdata(cos)), static_cast<const float*>(cdata(sin)),
-                                       positions.defined() ? static_cast<const int*>(cdata(positions)) : nullptr, static_cast<int>(S), static_cast<int>(2 * H * D), stream()));
-      } else {
-        p = linear(first.y, qkv);
-        rope(p, cos, sin, positions, S, 2 * H, D, 1.f);
-      }
-      const Packed z = unpack(p, B, S, H, D);
-      const NormOut second = norm_fwd(linear(attn_fwd(z.q, z.k, z.v, scale, true, false).o.view({T, H * D}), out), first.h, n2, eps, false);
+      // what the layer's operators would have given back by then is given back: a projection is three rows wide
+      NormOut first = norm_fwd(x, residual, n1, eps, false);
+      Tensor o = [&] {
+        Tensor p;
+        if (D == 64 && lib.llmctl_gemm_rope_bf16 && unit16(cos) && unit16(sin)) {
+          p = new_bf16(x, {T, 3 * H * D});
+          done("llmctl_gemm_rope_bf16",
+               lib.llmctl_gemm_rope_bf16(cdata(first.y), cdata(qkv), data(p), static_cast<int>(T), static_cast<int>(3 * H * D), static_cast<int>(W), W, qkv.stride(0), 3 * H * D,
+                                         static_cast<const float*>(cdata(cos)), static_cast<const float*>(cdata(sin)),
+                                         positions.defined() ? static_cast<const int*>(cdata(positions)) : nullptr, static_cast<int>(S), static_cast<int>(2 * H * D), stream()));
+        } else {
+          p = linear(first.y, qkv);
+          rope(p, cos, sin, positions, S, 2 * H, D, 1.f);
+        }
+        first.y.reset();
+        const Packed z = unpack(p, B, S, H, D);
+        return attn_fwd(z.q, z.k, z.v, scale, true, false).o.view({T, H * D});
+      }();
+      Tensor a = linear(o, out);
+      o.reset();
+      const NormOut second = norm_fwd(a, first.h, n2, eps, false);
+      a.reset();
+      first.h.reset();
       y = linear(up_and_activate(second.y, up, false).first, down);
       r = second.h;
     });

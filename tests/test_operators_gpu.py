@@ -803,6 +803,31 @@ def test_block_without_gradients(ops, B, S, heads, dim, form):
     assert len(seen) == (2 if form == "hook" else 0)
 
 
+@pytest.mark.parametrize("dim", [64, 128])
+def test_block_holds_no_more_than_its_operators(ops, dim):
+    """The most memory that a layer holds as one call, and layer by layer through the extension."""
+    from llmctl_b200.models.config import ModelConfig
+    from llmctl_b200.models.gpt import GPTModel
+    heads = 1024 // dim
+    m = GPTModel(ModelConfig(name="t", layers=1, hidden=1024, ffn=1024, heads=heads, head_dim=dim, vocab_size=128, max_position_embeddings=4096), device="cuda")
+    blk, (cos, sin) = m.blocks[0], m.rope_tables(torch.device("cuda"))
+    x, r = _randn(4096, 1024), _randn(4096, 1024, seed=1)
+
+    def most():
+        with torch.no_grad():
+            blk(x, r, cos, sin, 1, 4096)
+            torch.cuda.synchronize()
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            y = blk(x, r, cos, sin, 1, 4096)
+        torch.cuda.synchronize()
+        del y
+        return torch.cuda.max_memory_allocated() - before
+    whole = most()
+    blk._plain = lambda: False
+    assert whole <= most()
+
+
 @pytest.mark.parametrize("starts,width,heads,q_rank,parts", [([0], 256, 16, 128, {}), ([500, 77, 64], 256, 32, 128, {"sink": True}), ([130, 900], 256, 5, 0, {}),
                                                           ([300, 40], 128, 40, 64, {"head_gate": True, "window": 100}), ([70], 128, 8, 64, {"out_gate": True})])
 def test_latent_layer_decodes(ops, starts, width, heads, q_rank, parts):
