@@ -15,6 +15,7 @@
 #include "../common/dependent.cuh"
 #include "../common/fast_div.h"
 #include "../common/wait_status.h"
+#include "flash_split.h"
 
 namespace llmctl {
 using namespace ptx;
@@ -561,20 +562,6 @@ static long long* flash_trace_buffer() {
   return buf;
 }
 
-// Whether items of one tile whose keys are split (kSplit) are the better ones: by the steps (a block of both warpgroups, 1.5 us at D = 128) of the
-// busiest CTA, which is the longest item's where the others do not fill the SMs, and 1.7 steps for each of its items; split items are twice as
-// many and read the keys twice as often, so they must be a fifth ahead.  us, pairs of tiles / split (sequences x tokens x heads x size):
-// 1 x 129 x 12 x 64 6.6 / 4.8, 1 x 300 x 12 x 64 6.9 / 5.9, 1 x 777 x 12 x 64 12.9 / 9.0, 1 x 2000 x 12 x 64 27.7 / 17.0, 1 x 4000 x 12 x 64 51.5 / 45.1,
-// 2 x 1024 x 12 x 64 16.2 / 11.5, 1 x 1500 x 16 x 128 24.8 / 16.4, 2 x 700 x 16 x 128 14.9 / 13.6; left as pairs:
-// 1 x 600 x 32 x 128 12.8 / 11.2, 1 x 1200 x 32 x 128 21.9 / 22.5, 1 x 1000 x 40 x 128 19.1 / 21.2, 4 x 333 x 16 x 128 9.0 / 11.7, 1 x 1777 x 32 x 128 29.2 / 34.8, 8 x 512 x 32 x 128 34.0 / 45.0.
-static bool split_keys(int B, int S, int H, int causal) {
-  const double heads = static_cast<double>(B) * H, n = (S + ffwd::kRows - 1) / ffwd::kRows, half = ceil(n / 2), odd = 2 * half - n;
-  if (n < 2) return false;
-  auto cost = [&](double longest, double steps, double items) { return fmax(longest, heads * steps / kNumSMs) + 1.7 * ceil(heads * items / kNumSMs); };
-  const double pairs = cost(n, causal ? half * (half + 1) - odd : half * n, half);
-  return 1.2 * cost(half, causal ? half * (half + 1) - odd * half : half * n, n) < pairs;
-}
-
 // Persistent launch: one CTA per SM over a heavy-first item list.
 template <int DQK, int DV, bool kSplit = false>
 static int flash_fwd_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& ks, const CUtensorMap& v, void* o,
@@ -645,7 +632,7 @@ LLMCTL_API int llmctl_flash_attn_fwd(const void* q, const void* k, const void* v
     mkmap(&tv, v, v_tok_stride, H);
   }
   if (rc) LLMCTL_FAIL(rc, "tensor map Q / K / V");
-  const bool split = split_keys(B, S, H, causal);
+  const bool split = split_keys(B * H, (S + ffwd::kRows - 1) / ffwd::kRows, D, causal, kNumSMs);
   rc = (D == 128 ? (split ? flash_fwd_launch<128, 128, true> : flash_fwd_launch<128, 128>) : split ? flash_fwd_launch<64, 64, true> : flash_fwd_launch<64, 64>)(tq, tk, tk, tv, o, o_tok_stride, lse, nullptr, B, S, H,
                                                                           packed ? H : 0, scale, causal, (cudaStream_t)stream);
   if (rc) LLMCTL_FAIL(rc, "flash forward");

@@ -749,6 +749,29 @@ int main() {
     assert r.returncode == 0, r.stdout
 
 
+def test_items_of_the_attention_forward(tmp_path):
+    """csrc/attention/flash_split.h takes the items that were measured to be at least 3% faster, from operands in L2 and in memory alike, at the sizes
+    on either side of its lines."""
+    import shutil
+    import subprocess
+    root = Path(__file__).resolve().parents[1]
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("needs g++")
+    # (head size, mask, heads): (key blocks where single tiles won, where pairs won)
+    won = {(64, 1, 12): ([2, 3, 8, 16, 24, 32], []), (64, 1, 16): ([2, 3, 9, 16, 24], [32]), (64, 1, 24): ([2, 3, 7, 13, 14], [20, 24]),
+           (64, 1, 32): ([2, 4, 5, 7, 9], [12, 20]), (64, 1, 48): ([2, 3, 4], [5, 8, 20]), (64, 1, 96): ([], [4, 6, 8]),
+           (128, 1, 16): ([2, 3, 9, 16, 20], [32]), (128, 1, 20): ([2, 5, 10, 14], [20, 24]), (128, 1, 32): ([2, 4, 5, 6, 7, 8], [12, 14, 20]),
+           (128, 1, 40): ([2, 4], [5, 7, 8, 10, 20]), (128, 1, 64): ([2], [3, 4, 8]), (128, 1, 80): ([], [2, 4, 8]), (128, 1, 128): ([], [2, 3, 4, 8]),
+           (64, 0, 12): ([2, 4, 8, 12], [16]), (64, 0, 16): ([2, 4, 8], [10, 12]), (128, 0, 16): ([2, 4, 8], [10, 12]), (128, 0, 40): ([2, 3, 7], [4, 5, 6]),
+           (128, 0, 128): ([], [2, 3, 4])}
+    (tmp_path / "t.cpp").write_text("#include \"attention/flash_split.h\"\n#include <cstdio>\nint main() {\n" + "".join(
+        f'  printf("%d", llmctl::split_keys({heads}, {n}, {dim}, {mask}, 148));\n' for (dim, mask, heads), sides in won.items() for n in sides[0] + sides[1]) + "}\n")
+    subprocess.run([gxx, "-O1", "-std=c++17", "-I", str(root / "csrc"), str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t")], check=True)
+    got = subprocess.run([str(tmp_path / "t")], capture_output=True, text=True).stdout
+    assert got == "".join("1" * len(a) + "0" * len(b) for a, b in won.values())
+
+
 def test_shared_memory_limits_are_raised_and_never_lowered(tmp_path):
     """csrc/common/smem_limit.h with the runtime's two calls replaced: threads that ask for unlike sizes of one kernel leave the largest in
     place, a device counts by itself, and a call that was refused is asked again."""
