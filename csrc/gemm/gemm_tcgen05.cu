@@ -1163,8 +1163,9 @@ static int one_wave_tile(int M, int N) {
 // CTAs that share the K of each 128 x 64 tile (gemm_split_kernel), 1 where that does not pay: fewer tiles than SMs, and a K whose blocks, 0.2 us
 // each for a CTA alone on its SM and 0.32 for two, outweigh the cluster's launch and exchange.  Clusters of 4 and 8 leave SMs of a GPC over: 128 CTAs
 // of them are resident one to an SM.  us, one CTA a tile / split (operands from HBM): 64 x 768 x 32000 98 / 19 (8), 200 x 768 98 / 31 (4), 500 x 768
-// 100 / 48 (4), 1000 x 768 104 / 83 (2), 500 x 2048 101 / 88 (2), 200 x 2048 x 11264 37 / 23, x 5632 20.1 / 15.3, 500 x 768 x 4096 15.8 / 12.9, 768 x 768 x 3000
-// of M-major operands 14.0 / 12.4; left alone: 200 x 2048 x 2048 9.5 / 9.9, 300 x 768 x 2048 9.3 / 9.4, 777 x 768 x 2048 9.6 / 13.9, 500 x 2048 x 5632 20.5 / 22.9.
+// 100 / 48 (4), 1000 x 768 104 / 83 (2), 500 x 2048 101 / 88 (2), 200 x 2048 x 11264 37 / 23, x 5632 20.1 / 15.3, 500 x 768 x 4096 15.8 / 12.9;
+// left alone: 200 x 2048 x 2048 9.5 / 9.9, 300 x 768 x 2048 9.3 / 9.4, 777 x 768 x 2048 9.6 / 13.9, 500 x 2048 x 5632 20.5 / 22.9, and, though it would win,
+// 768 x 768 x 3000 of M-major operands 14.0 / 12.4.  fp32 sums of another order: the bits of a product depend on its number of rows.
 static int split_count(int M, int N, int K) {
   const long long tiles = static_cast<long long>((M + kBM - 1) / kBM) * ((N + kSplitBN - 1) / kSplitBN), sms = num_sms();
   if (tiles > sms) return 1;
@@ -1284,7 +1285,8 @@ LLMCTL_API int llmctl_gemm_swiglu_bwd_bf16(const void* DY, const void* W, const 
 }
 
 // C[M, N] = X W^T with the first `rotated` columns, heads of 64, rotated as llmctl_rope_inplace does (sign 1; cos, sin: [positions, 32]): a packed
-// projection and its rotation in one launch, without the pass over q and k between them.  Tiles by the rule of llmctl_gemm_bf16.
+// projection and its rotation in one launch, without the pass over q and k between them.  Tiles by the one-wave and pair rule of
+// llmctl_gemm_bf16; no K shared by a cluster, which that entry tries first and takes for no packed projection (N = 3 K has too many tiles).
 // us of 12 layers of width 768 without gradients, two launches / one: 777 tokens 668 / 653, 2000 tokens 893 / 870, 100 tokens (host) 623 / 590.
 LLMCTL_API int llmctl_gemm_rope_bf16(const void* X, const void* W, void* C, int M, int N, int K, long long ldx, long long ldw, long long ldc, const float* cos_t,
                                      const float* sin_t, const int* positions, int seq_len, int rotated, void* stream) {

@@ -536,6 +536,24 @@ def test_gemm_split_k(cuda_device, M, N, K, a_mn, b_mn, splits):
     assert err.norm() <= 2 * 2.0 ** -9 * (want + old).norm()
 
 
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn,chosen", [(200, 768, 32000, 0, 1, 4), (64, 2048, 5632, 0, 0, 4), (768, 768, 4000, 1, 1, 2), (500, 768, 32000, 0, 1, 4),
+                                                    (768, 768, 3000, 1, 1, 1), (200, 2048, 2048, 0, 0, 1), (500, 2048, 5632, 0, 0, 1)])
+def test_gemm_split_k_is_chosen(cuda_device, M, N, K, a_mn, b_mn, chosen):
+    """On either side of the rule's line: the bits of the number of CTAs that it gives a tile, whose sums no other order leaves alike."""
+    from llmctl_b200.ops import native
+    torch.manual_seed(1)
+    a = torch.randn(*((K, M) if a_mn else (M, K)), device=cuda_device).bfloat16()
+    b = torch.randn(*((K, N) if b_mn else (N, K)), device=cuda_device).bfloat16()
+
+    def product(tile):
+        out = torch.empty(M, N, device=cuda_device)
+        native.call("llmctl_gemm_bf16", a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0), a_mn, b_mn, 1, 0, tile, 0,
+                    native.stream_ptr())
+        return out
+    for splits in (1, 2, 4, 8):
+        assert torch.equal(product(0), product(64 if splits == 1 else -splits)) == (splits == chosen), splits
+
+
 @pytest.mark.parametrize("M,heads,K,seq", [(1, 1, 64, 1), (33, 3, 200, 11), (130, 12, 768, 130), (777, 12, 768, 259), (777, 20, 136, 777), (2000, 12, 72, 500), (4100, 16, 64, 1025)])
 @pytest.mark.parametrize("form", ["plain", "positions", "one part"])
 def test_gemm_with_rotation(cuda_device, M, heads, K, seq, form):
