@@ -18,8 +18,8 @@
 //               then weighs 1, wherever the reference stands
 // TMEM: S^T two buffers of N columns (64 rows: lanes 32q + 0 .. 15 of quadrant q), O^T R / 128 blocks of N columns.
 //
-// Bound by HBM: two stages in flight and 27 / 46 clocks for each of a tile's 36 / 16 products leave 3350 clocks a tile, 6.2 TB/s over 148 CTAs.
-// With the merge of split contexts, us, mma.sync kernel of latent_attention.cu / this one: 32 contexts of 2000-4000, 16 heads 65 / 39, 32 heads 92 / 42
+// Bound by a CTA's chain from tile to tile (copy, scores, softmax, values, the stage handed back) with no more than two stages to hide it: about 3 TB/s,
+// 35-38% of DRAM's peak; a tile's products alone are 36 of 27 and 16 of 46 clocks.  With the merge of split contexts, us, mma.sync kernel of latent_attention.cu / this one: 32 contexts of 2000-4000, 16 heads 65 / 39, 32 heads 92 / 42
 // (112 MB: 17 at the rate of a copy); 32 of 500-1000, 16 heads 31 / 19; 8 of 1000-2000 28 / 14; one of 300 18.4 / 9.9, 32 heads 21 / 12.  Splits for one
 // CTA to an SM (two: 39 -> 43).
 // Every wait is bounded, as in latent_attention_t5.cu.

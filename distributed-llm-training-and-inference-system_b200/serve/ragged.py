@@ -164,11 +164,12 @@ class RaggedBatch:
         return int(max(1, min(2 * self._sms // max(ctas, 1), longest // 64)))
 
     def _even_splits(self, slots: int, groups: int, longest: int) -> int:
-        """Most splits with which all CTAs that have keys to read run at once (two to an SM with 16 rows, one with 32): a sequence's
-        splits are of one length, whole tiles of 64 keys, and those past its end have nothing to do.  A second wave, and half-empty
-        splits, cost more than longer ones (us with the merge, splits by the longest context alone / these: 32 contexts of 2000-4000, 16 heads
-        70.9 in 9 / 65.1 in 12, 32 heads 111.5 in 9 / 91.7 in 5; 4 of 600-1000, 16 heads 24.6 in 15 / 20.6 in 16; 8 of 1000-2000, 32 heads
-        45.8 in 31 / 33.6 in 16; 16 of 150-300, 16 heads 23.6 in 4 / 19.8 in 5)."""
+        """Most splits with which all CTAs that have keys to read run at once (``slots`` of them; the decoding kernel of
+        csrc/attention/latent_decode.cu has one to an SM, the kernel of other layouts two with 16 rows and one with 32): a sequence's splits
+        are of one length, whole tiles of 64 keys, and those past its end have nothing to do.  A second wave, and half-empty splits, cost
+        more than longer ones (us with the merge on the kernel of other layouts, splits by the longest context alone / these: 32 contexts of
+        2000-4000, 16 heads 70.9 in 9 / 65.1 in 12, 32 heads 111.5 in 9 / 91.7 in 5; 4 of 600-1000, 16 heads 24.6 in 15 / 20.6 in 16; 8 of
+        1000-2000, 32 heads 45.8 in 31 / 33.6 in 16; 16 of 150-300, 16 heads 23.6 in 4 / 19.8 in 5)."""
         if self.pad_to is None:
             contexts = [min(p.start + len(p.tokens), longest) for p in self._portions]
         else:                                                   # captured: any of them may be the longest

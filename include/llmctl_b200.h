@@ -23,11 +23,12 @@ int llmctl_rmsnorm_fwd(const void* x, const void* residual, const void* w, void*
                        float* rstd, int rows, int cols, float eps, void* stream);
 /* dx = d(norm)/dh (+ dres); dw (fp32) (+)= sum_rows dy * xhat.
  * scratch: fp32 [scratch_rows * cols]; scratch_rows CTAs are used (1..rows). */
-int llmctl_rmsnorm_bwd_bf16w(const void* dy, const void* h, const void* w, const float* rstd, const void* dres, void* dx, void* dw, float* scratch,
-                             int scratch_rows, int rows, int cols, void* stream);      /* dw in bf16 */
 int llmctl_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd,
                        const void* dres, void* dx, float* dw, float* scratch, int scratch_rows,
                        int rows, int cols, int accumulate, void* stream);
+/* The same with dw in bf16, rounded from its fp32 sum. */
+int llmctl_rmsnorm_bwd_bf16w(const void* dy, const void* h, const void* w, const float* rstd, const void* dres, void* dx, void* dw, float* scratch,
+                             int scratch_rows, int rows, int cols, void* stream);
 /* RMSNorm backward for callers that cannot allocate device memory (a host runtime whose arena already owns the
  * whole device budget, or a latency-bound loop that must stay away from cudaMalloc's driver lock).  Same math
  * as llmctl_rmsnorm_bwd; the dw partials live in a 2 MiB array built into the library (held on every GPU that
@@ -48,11 +49,12 @@ int llmctl_layernorm_bwd(const void* dy, const void* h, const void* w, const flo
                          void* stream);
 
 /* ---- K4 RoPE (rotate-half), in place; sign=+1 forward, -1 backward.  Reference: HF rotary. ---- */
-int llmctl_gemm_rope_bf16(const void* X, const void* W, void* C, int M, int N, int K, long long ldx, long long ldw, long long ldc, const float* cos_t,
-                          const float* sin_t, const int* positions, int seq_len, int rotated, void* stream);      /* X W^T, heads of 64 rotated */
 int llmctl_rope_inplace(void* x, long long row_stride, int n_tokens, int n_heads, int head_dim,
                         const float* cos_t, const float* sin_t, const int* positions, int seq_len,
                         float sign, void* stream);
+/* C[M, N] = X W^T whose first `rotated` columns, heads of 64, are rotated on their way out (sign +1). */
+int llmctl_gemm_rope_bf16(const void* X, const void* W, void* C, int M, int N, int K, long long ldx, long long ldw, long long ldc, const float* cos_t,
+                          const float* sin_t, const int* positions, int seq_len, int rotated, void* stream);
 
 /* ---- K5 SwiGLU on packed [M, 2F] gate|up, all on 16-byte boundaries; d_gate_up has gate_up's row stride.  Reference: ATen silu + mul. ---- */
 int llmctl_swiglu_fwd(const void* gate_up, void* out, int M, int F, long long ld_gu, void* stream);
