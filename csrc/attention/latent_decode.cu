@@ -49,7 +49,8 @@ constexpr int kWindowAlign = 32;             // a window's first key tile starts
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.f;
 constexpr int fixed_smem(int panels, int N) { return panels * N * 128 + 2 * N * 128 + 1024; }      // Q, P, alignment
-constexpr int kSmemMost = 225 * 1024;
+constexpr int smem_most(int ctas) { return (ctas == 1 ? 225 : 110) * 1024; }      // dynamic, of a CTA, where an SM has to hold that many
+constexpr int stages_in(int bytes, int panels, int N) { return (bytes - fixed_smem(panels, N)) / (panels * kPanel); }
 
 // A stage of nine panels (four 128-wide blocks of the latent, the rotated part) is handed back in three parts, as the value products of its blocks end, and
 // loaded again part by part; other tiles in one.  A layer, 32 tokens behind 4000: 16 heads 70.1 -> 69.1 us, 32 heads 84.5 -> 83.7.  Scores that also
@@ -98,9 +99,10 @@ __device__ __forceinline__ void tmem_ld(uint32_t at, uint32_t* r) {
 
 // Grid: (tokens, groups of heads_per_tile heads, splits).  kPanels: 64-column panels of a cache row, 9 for latents of 512 with 64 rotated
 // dimensions, or 0 for what R and dr say.  With 9 the products unroll and their descriptors are constants away from one register (32 contexts of
-// 2000-4000 from stages that are not loaded: 34.6 us in loops, 28.5 unrolled).
-template <int N, int kPanels>
-__global__ void __launch_bounds__(ldec::kThreads, 1)
+// 2000-4000 from stages that are not loaded: 34.6 us in loops, 28.5 unrolled).  kCtas: CTAs that an SM has to hold; the registers of 32 heads are as
+// many as one may have, and a few have to be spilled for two.
+template <int N, int kPanels, int kCtas>
+__global__ void __launch_bounds__(ldec::kThreads, kCtas)
 latent_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __nv_bfloat16* __restrict__ ql, long long ql_st, long long ql_sh,
                      const __nv_bfloat16* __restrict__ q, long long ldq, int dn, const int* __restrict__ block_tables, int max_blocks, int block_size,
                      const int* __restrict__ tiles, const int* __restrict__ positions, const float* __restrict__ freq, float mult, float scale,
@@ -437,18 +439,18 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __nv_bfloat1
   }
 }
 
-template <int N, int kPanels>
+template <int N, int kPanels, int kCtas = 1>
 static int launch_latent_decode(const CUtensorMap& tmK, const void* ql, long long ql_st, long long ql_sh, const void* q, long long ldq, int dn,
                                 const int* block_tables, int max_blocks, int block_size, const int* tiles, int ntiles, const int* positions,
                                 const float* freq, float mult, float scale, int H, int R, int dr, int heads_per_tile, int splits, int keys_per_split,
                                 int box_rows, void* out, float* partial, const float* sinks, int window, const void* head_gate, long long gate_ld,
                                 cudaStream_t s) {
   using namespace ldec;
-  const int panels = (R + dr) >> 6, room = (kSmemMost - fixed_smem(panels, N)) / (panels * kPanel);
+  const int panels = (R + dr) >> 6, room = stages_in(smem_most(kCtas), panels, N);
   const int stages = room < kMaxStages ? room : kMaxStages, smem = fixed_smem(panels, N) + stages * panels * kPanel;
   unsigned char* const wait_byte = wait_report(kWaitLatentAttention);
   if (wait_byte == nullptr) return static_cast<int>(cudaErrorMemoryAllocation);
-  auto kern = latent_decode_kernel<N, kPanels>;
+  auto kern = latent_decode_kernel<N, kPanels, kCtas>;
   const cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const dim3 grid(ntiles, (H + heads_per_tile - 1) / heads_per_tile, splits);
@@ -484,8 +486,13 @@ LLMCTL_API int llmctl_latent_decode(const void* ql, long long ql_st, long long q
   int rc = get_tmap_2d_bf16(&tmK, cache, cache_rows, R + dr, R + dr, box_rows, 64, 1);
   if (rc) LLMCTL_FAIL(rc, "tensor map of the cache");
   const bool usual = R == 512 && dr == 64;
-  rc = (heads_per_tile <= 16 ? (usual ? launch_latent_decode<16, 9> : launch_latent_decode<16, 0>)
-                             : (usual ? launch_latent_decode<32, 9> : launch_latent_decode<32, 0>))(tmK, ql, ql_st, ql_sh, q, ldq, dn, block_tables, max_blocks, block_size, tiles,
+  // More CTAs than SMs (many tokens, or one long context beside short ones, whose splits are mostly empty): two to an SM where both have stages
+  // enough.  A layer, us, mma.sync kernel / one / two: 32 heads of 128 + 64 columns, 200 contexts of 100 43.1 / 46.3 / 38.7, one of 8000 beside 30 of 50
+  // 93.6 / 119 / 81; 16 heads of 256 + 64, the same 40.6 / 40.0 / 33.2 and 171 / 90.7 / 66.4.  Up to 148 CTAs one each is as fast, and spills nothing.
+  const long long ctas = static_cast<long long>(ntiles) * ((H + heads_per_tile - 1) / heads_per_tile) * splits;
+  auto two = [&](int N, int stages) { return ctas > kNumSMs && ldec::stages_in(ldec::smem_most(2), (R + dr) / 64, N) >= stages; };
+  rc = (heads_per_tile <= 16 ? (usual ? launch_latent_decode<16, 9> : two(16, 2) ? launch_latent_decode<16, 0, 2> : launch_latent_decode<16, 0>)
+                             : (usual ? launch_latent_decode<32, 9> : two(32, 3) ? launch_latent_decode<32, 0, 2> : launch_latent_decode<32, 0>))(tmK, ql, ql_st, ql_sh, q, ldq, dn, block_tables, max_blocks, block_size, tiles,
                                                                                   ntiles, positions, freq, mult, scale, H, R, dr, heads_per_tile, splits,
                                                                                   keys_per_split, box_rows, out, partial, sinks, window, head_gate, gate_ld,
                                                                                   (cudaStream_t)stream);

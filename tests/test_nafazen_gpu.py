@@ -220,6 +220,26 @@ def test_latent_decode_scores_of_minus_infinity(cuda_device, one_token, splits, 
     assert native.lib().llmctl_latent_attention_t5_status(1) == 0
 
 
+# more CTAs than SMs, two to an SM where their stages fit (32 heads up to 192 columns, 16 up to 320): many tokens, one long context beside short ones
+@pytest.mark.parametrize("contexts", [[100] * 160, [3000] + [50] * 30, [1]])
+@pytest.mark.parametrize("H,dr,R", [(32, 64, 128), (32, 0, 128), (64, 64, 128), (32, 64, 256), (16, 64, 256), (5, 0, 256), (16, 64, 384), (16, 64, 512)])
+def test_latent_decode_of_many_ctas(cuda_device, contexts, H, dr, R):
+    """Against the general kernel, which rounds the same things to bf16.  Bound as above."""
+    from llmctl_b200.ops import latent_attention as L
+    from llmctl_b200.serve.ragged import Portion, RaggedBatch
+    torch.manual_seed(R + H)
+    T, bs, dn = len(contexts), 64, 8
+    pages = [(c + bs - 1) // bs for c in contexts]
+    tables = [list(range(sum(pages[:i]), sum(pages[:i + 1]))) for i in range(T)]
+    cache, ql, q = torch.randn(sum(pages), bs, R + dr).bfloat16().cuda(), torch.randn(T, H, R).bfloat16().cuda(), torch.randn(T, H * (dn + dr)).bfloat16().cuda()
+    b = RaggedBatch([Portion(i, [0], c - 1, [0], t) for i, (c, t) in enumerate(zip(contexts, tables))], bs, torch.device("cuda"))
+    rows = L.ROWS_PER_TILE_WIDE if H > 16 else L.ROWS_PER_TILE
+    hpt = b.heads_per_tile(H, rows)
+    got, want = (L.latent_attention(ql, q, dn, cache, b.block_tables, b.tiles(rows), b.positions, torch.rand(max(dr // 2, 1), generator=torch.Generator().manual_seed(1)).cuda(),
+                                    1.0, 0.1, hpt, b.max_context, b.attention_splits(H, rows, None, 1), rows=rows, one_token=one).double() for one in (True, False))
+    assert ((got - want).flatten(1).norm(dim=1) <= 2 * 2 * 2 ** -9 * want.flatten(1).norm(dim=1)).all()
+
+
 @pytest.mark.parametrize("one_token", [False, True])
 @pytest.mark.parametrize("splits", [1, 2])
 def test_latent_decode_of_a_key_that_decides_behind_the_reference(cuda_device, one_token, splits):
