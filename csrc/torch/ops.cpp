@@ -366,13 +366,15 @@ Tensor dgrad(const Tensor& dy, const Tensor& w, int tile_n) {
 // A recorded operator as a node of its own: torch::autograd::Function looks its arguments up by name, and wraps and checks them in ways that
 // operators which return one new tensor have no use for (forward and backward of a small attention 72 us; the engine alone takes 29).  `T` says
 // what its backward needs (kEntry, there()) and is
-//   static variable_list gradients(const Numbers&, const Tensor& grad, const variable_list& saved, unsigned wants)
-// with a bit of `wants` for each gradient that is asked for.  Nothing else may enter: compiled autograd calls it with tensors of its own, and
+//   static variable_list gradients(const Numbers&, const Tensor& grad, Kept saved, unsigned wants)
+// with a bit of `wants` for each gradient that is asked for, unless kAllAtOnce.  Nothing else may enter: compiled autograd calls it with tensors of its own, and
 // for any call whose numbers and `wants` are the same.
 namespace compiled = torch::dynamo::autograd;
+using Kept = c10::ArrayRef<Tensor>;
+constexpr unsigned kMostKept = 5;
 template <typename T, typename Numbers>
 struct Recorded : torch::autograd::Node {
-  std::vector<torch::autograd::SavedVariable> saved;
+  c10::SmallVector<torch::autograd::SavedVariable, kMostKept> saved;
   int output = -1;                                 // which of them is what the forward returned
   Numbers numbers;
 
@@ -382,24 +384,24 @@ struct Recorded : torch::autograd::Node {
     node->numbers = std::move(numbers);
     return node;
   }
-  torch::autograd::variable_list kept() {
-    torch::autograd::variable_list ts;
-    ts.reserve(saved.size());
+  c10::SmallVector<Tensor, kMostKept> kept() {
+    c10::SmallVector<Tensor, kMostKept> ts;
     for (size_t i = 0; i < saved.size(); ++i) ts.push_back(static_cast<int>(i) == output ? saved[i].unpack(getptr()) : saved[i].unpack());
     return ts;
   }
   unsigned wants() const {
     unsigned bits = 0;
-    for (uint32_t i = 0; i < num_outputs(); ++i) bits |= static_cast<unsigned>(task_should_compute_output(i)) << i;
+    if constexpr (!T::kAllAtOnce)
+      for (uint32_t i = 0; i < num_outputs(); ++i) bits |= static_cast<unsigned>(task_should_compute_output(i)) << i;
     return bits;
   }
-  static torch::autograd::variable_list run(const Numbers& numbers, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
+  static torch::autograd::variable_list run(const Numbers& numbers, const Tensor& grad, Kept kept, unsigned wants) {
     return node_body(T::kEntry, T::there(), [&] { return T::gradients(numbers, grad, kept, wants); });
   }
 
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
     if (!grads[0].defined()) return torch::autograd::variable_list(num_outputs());
-    torch::autograd::variable_list ts;
+    c10::SmallVector<Tensor, kMostKept> ts;
     {
       std::lock_guard<std::mutex> hold(mutex_);
       ts = kept();
@@ -426,7 +428,7 @@ struct Recorded : torch::autograd::Node {
     const size_t outputs = num_outputs(), n = saved.size();
     auto later = [numbers = numbers, wants = wants(), outputs, n](const torch::autograd::variable_list& grads, const std::vector<c10::IValue>& stack) {
       compiled::PackedArgs packed(stack);
-      torch::autograd::variable_list kept;
+      c10::SmallVector<Tensor, kMostKept> kept;
       for (size_t i = 0; i < n; ++i) kept.push_back(packed.unpack<Tensor>());
       return grads[0].defined() ? run(numbers, grads[0], kept, wants) : torch::autograd::variable_list(outputs);
     };
@@ -452,15 +454,15 @@ struct ProductNumbers {
 };
 template <typename T>
 struct Product : Recorded<T, ProductNumbers> {
+  static constexpr bool kAllAtOnce = false;
   void keep(std::initializer_list<const Tensor*> ts) {
-    this->saved.reserve(ts.size());
     for (const Tensor* t : ts) {
       this->saved.emplace_back(*t, false);
       this->numbers.sizes.push_back({t->size(0), t->size(1)});
     }
   }
   // a hook on saved tensors may give back anything: what the kernels cannot read is refused
-  static void check(const ProductNumbers& numbers, const torch::autograd::variable_list& kept, const Tensor& grad) {
+  static void check(const ProductNumbers& numbers, Kept kept, const Tensor& grad) {
     for (size_t i = 0; i < kept.size(); ++i) {
       const Tensor& t = kept[i];
       TORCH_CHECK(t.device() == grad.device() && is_matrix(t) && t.size(0) == numbers.sizes[i][0] && t.size(1) == numbers.sizes[i][1], T::kName, ": a saved matrix came back as ",
@@ -486,7 +488,7 @@ struct LinearNode final : Product<LinearNode> {
     torch::autograd::set_history(y, node);
     return y;
   }
-  static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
+  static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, Kept kept, unsigned wants) {
     check(z, kept, grad);
     const Tensor &x = kept[0], &w = kept[1], dy = rows(grad);
     Tensor dx, dw;
@@ -515,7 +517,7 @@ struct LinearSwigluNode final : Product<LinearSwigluNode> {
     torch::autograd::set_history(act, node);
     return act;
   }
-  static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
+  static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, Kept kept, unsigned wants) {
     check(z, kept, grad);
     const Tensor &x = kept[0], &w = kept[1], dgu = [&] {
       at::AutoDispatchBelowADInplaceOrView below;
@@ -544,7 +546,7 @@ struct SwigluMlpNode final : Product<SwigluMlpNode> {
     torch::autograd::set_history(y, node);
     return y;
   }
-  static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned wants) {
+  static torch::autograd::variable_list gradients(const ProductNumbers& z, const Tensor& grad, Kept kept, unsigned wants) {
     check(z, kept, grad);
     const Tensor &x = kept[0], &up = kept[1], &down = kept[2], &act = kept[4], dy = rows(grad);
     Tensor dgu, dx, d_up, d_down;
@@ -693,10 +695,10 @@ struct AttentionNumbers {
 };
 struct FlashAttention final : Recorded<FlashAttention, AttentionNumbers> {
   static constexpr const char* kEntry = "llmctl_flash_attn_bwd";
+  static constexpr bool kAllAtOnce = true;
   static bool there() { return ready(lib.llmctl_flash_attn_bwd); }
   static Tensor record(const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal) {
     auto node = make(torch::autograd::collect_next_edges(q, k, v), {scale, causal});
-    node->saved.reserve(5);
     for (const Tensor* t : {&q, &k, &v}) node->saved.emplace_back(*t, false);
     AttnOut r = attn_fwd(q, k, v, scale, causal, true);
     torch::autograd::set_history(r.o, node);
@@ -705,7 +707,7 @@ struct FlashAttention final : Recorded<FlashAttention, AttentionNumbers> {
     node->saved.emplace_back(r.lse, false);
     return r.o;
   }
-  static torch::autograd::variable_list gradients(const AttentionNumbers& z, const Tensor& grad, const torch::autograd::variable_list& kept, unsigned) {
+  static torch::autograd::variable_list gradients(const AttentionNumbers& z, const Tensor& grad, Kept kept, unsigned) {
     const Tensor &q = kept[0], &k = kept[1], &v = kept[2], &o = kept[3], &lse = kept[4];
     const auto here = grad.device();
     TORCH_CHECK(q.device() == here && k.device() == here && v.device() == here && o.device() == here && attention_ok(q, k, v, z.causal) && bf16(o) &&
